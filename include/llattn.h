@@ -151,6 +151,64 @@ int llattn_mamba2_final_state(const void* k, const void* v, const float* g, floa
 int llattn_mamba2_step(float* states, const void* q, const void* k, const void* v, const float* g, const void* lambda, void* o,
                        int B, int H, int G, int K, int V, int L, int carry_level, void* stream);
 
+/* ---- Prompts of any length and decode steps on LEVEL-MAJOR states: fp32, stored (B,H,L,K,V), one contiguous K x V block per
+ * level of a head (the tensor a caller sees can still have the shape (B,H,K,V,L)).  A step then moves only the levels that
+ * hold tokens.
+ *
+ * llattn_mamba2_layer_step: hselective_state_update (hattention/mamba_apis.py:407-566) in one launch.  q, k (B,G,K), x (B,H,V),
+ * dt (B,H), dl (B,H,L) bf16; Lp (H,L), D (H), dt_bias (H) fp32 or bf16 by their flags, the last two may be NULL; A (H) fp32.
+ *     dt = softplus(dt + dt_bias), v = x dt, g = A dt, lambda = f(Lp, dl), the step of llattn_mamba2_step, y = o + D x
+ * with the rounding of the reference's torch operators; y bf16, fp32 with an fp32 D.  dt == NULL: x is v and g (B,H) fp32 is
+ * given; Lp == NULL: dl is lambda.  `live`: bit l is set when level l holds tokens before the step (counts > 0); levels
+ * whose bit is clear are taken as zero and not read.  carry_level as in llattn_mamba2_step.  V % 16 == 0, V <= 256, K <= 1024.
+ * llattn_gdn_layer_step: the one-token call of chunk_h_gated_delta_rule (hattention/gated_delta_rule_apis.py:93-132).  q, k
+ * (B,G,K) raw; with l2norm != 0 they are normalised (q scaled) first; lambda_mul != 0: lambda is multiplied by it and rounded to
+ * bf16.  V % 16 == 0, K <= 256.
+ * Both launch on `device`, which `stream` belongs to. */
+int llattn_mamba2_layer_step(float* states, const void* q, const void* k, const void* x, const void* dt, const float* g,
+                             const void* dl, const void* Lp, int lp_is_f32, const void* D, int d_is_f32, const void* dt_bias,
+                             int bias_is_f32, const float* A, void* y, int B, int H, int G, int K, int V, int L, unsigned live,
+                             int carry_level, int lambda_mode, int dt_softplus, int device, void* stream);
+int llattn_gdn_layer_step(float* states, const void* q, const void* k, const void* v, const void* beta, const float* g,
+                          const void* lambda, void* o, int B, int H, int G, int K, int V, int L, unsigned live, int carry_level,
+                          int l2norm, float scale, float lambda_mul, int device, void* stream);
+
+/* Prompts: the chunkwise kernels run on tensors of Tp >= T tokens whose last Tp - T tokens are zero (they leave the states as
+ * they are), so that no token of a ragged prompt is stepped.  Together these replace hattention_prefill (hattention/kernel.py:
+ * 469-560) and the torch operators of the layer around it (hattention/mamba_apis.py:346-399).
+ *   pad_tokens: n <= 8 tensors (B,T,...) of src_bytes[i] per token copied to (B,Tp,...) of dst_bytes[i] >= src_bytes[i]
+ *   mamba2_prompt_prep: llattn_mamba2_prep_fwd writing v, g, lambda (L_out >= L columns) Tp tokens long, and, where q_pad and
+ *     k_pad are given, q and k; dt_bias (may be NULL) and Lp are fp32 or bf16 by their flags
+ *   mamba2_prompt_residual: y (B,T,H,P) = o (B,Tp,H,P) + D x; y and D are fp32 (y_is_f32 != 0) or bf16; D may be NULL
+ *   mamba2_prompt_states: the level states after T tokens, level-major, every level written; k, v, g are Tp tokens long.  With the
+ *     workspace of the forward call on them (may be NULL) the levels that hold whole 512-token segments are sums of its summaries.
+ *   gdn_prompt_prep: l2norm of q (scaled) and k, one per head, K_out >= K columns wide (at most 128), Tp tokens long, and, each where
+ *     its pointer is given, v (as consecutive slices (B,Tp,H,v_slice)), beta and g, lambda (times lambda_mul unless 0, L_out columns)
+ *   gdn_prefill_slice: llattn_gdn_prefill writing the inter-chunk levels of value columns first_col .. first_col + V - 1 into
+ *     level-major states (B,H,state_levels,state_rows,state_cols); other levels are left alone
+ *   gdn_prompt_states: advances those levels by the tokens of the last chunk and writes the levels inside it, so that every level of
+ *     the v_cols columns from first_col is as of token T - 1; kn (B,Tp,H,128), v (B,Tp,H,v_cols); T is in the last 64 tokens of Tp */
+int llattn_pad_tokens(int n, const void* const* src, void* const* dst, const int* src_bytes, const int* dst_bytes, int B, int T, int Tp,
+                      void* stream);
+int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
+                              const void* Lp, int lp_is_f32, const void* q, const void* k, void* v, float* g, void* lambda, void* q_pad,
+                              void* k_pad, int B, int T, int Tp, int H, int G, int K, int P, int L, int L_out, int lambda_mode,
+                              void* stream);
+int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, void* y, int y_is_f32, int B, int T, int Tp, int H, int P,
+                                  void* stream);
+int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, float* states, const void* fwd_workspace,
+                                size_t fwd_workspace_bytes, int B, int T, int Tp, int H, int G, int K, int V, int L, void* stream);
+int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
+                           void* qn, void* kn, void* v_pad, void* beta_pad, float* g_pad, void* lambda_pad,
+                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int v_slice, int L, int L_out, float scale,
+                           float lambda_mul, void* stream);
+int llattn_gdn_prefill_slice(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
+                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int state_cols, int first_col,
+                             int state_levels, void* workspace, size_t workspace_bytes,
+                             int B, int T, int H, int K, int V, int L, void* stream);
+int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, const float* g, float* states, int B, int T, int Tp, int H,
+                             int K, int V, int v_cols, int first_col, int L, void* stream);
+
 /* Log-linear Gated DeltaNet forward.  Replaces hattention.chunkwise_hgdn.chunkwise_fwd
  * (hattention/chunkwise_hgdn.py:566-788) with output_final_state=False.  q and k are per head,
  * (B,T,H,K), and must already be L2-normalised (q also scaled) as the reference's autograd

@@ -77,6 +77,22 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
     return c.off;
 }
 
+}  // namespace
+
+namespace llattn {
+int mamba2_fwd_workspace_segments(const void* ws, size_t bytes, int B, int T, int H, int G, int K, int V, const float** F, const float** D) {
+    Mamba2Params p = {};
+    p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V;
+    if (bytes < setup(p, nullptr, false) || ((uintptr_t)ws & 255)) return LLATTN_ERR_WORKSPACE;
+    setup(p, const_cast<void*>(ws), false);
+    *F = p.seg_F;
+    *D = p.seg_D;
+    return 0;
+}
+}  // namespace llattn
+
+namespace {
+
 // Scratch for llattn_mamba2_fwd_static.  The array lives in the library's device image: every GPU
 // that loads the library carries these bytes until the process exits.  In host code the symbol is
 // only a handle; the device address is obtained once per device with cudaGetSymbolAddress.
@@ -279,7 +295,24 @@ size_t llattn_gdn_fwd_keep_workspace_bytes(int B, int T, int H, int K, int V, in
 
 static int gdn_fwd_impl(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                         void* o, float* g_cum, void* Aw, void* Au, void* workspace, size_t workspace_bytes,
-                        int B, int T, int H, int K, int V, int L, void* stream, bool keep, float* final_states = nullptr);
+                        int B, int T, int H, int K, int V, int L, void* stream, bool keep,
+                        const llattn::GdnStateOut& final_states = llattn::GdnStateOut{});
+
+int llattn_gdn_prefill_slice(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
+                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int state_cols, int first_col,
+                             int state_levels, void* workspace, size_t workspace_bytes,
+                             int B, int T, int H, int K, int V, int L, void* stream) {
+    if (!states) return LLATTN_ERR_NULL;
+    if (state_rows <= 0 || state_rows > K || first_col < 0 || first_col + V > state_cols || state_levels > L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    llattn::GdnStateOut out;
+    out.p = states + first_col;
+    out.rows = state_rows;
+    out.col = 1;
+    out.row = state_cols;
+    out.level = (long)state_rows * state_cols;
+    out.bh = out.level * state_levels;
+    return gdn_fwd_impl(q, k, v, beta, g, lambda, o, g_cum, Aw, Au, workspace, workspace_bytes, B, T, H, K, V, L, stream, false, out);
+}
 
 int llattn_gdn_prefill(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                        void* o, float* g_cum, void* Aw, void* Au, float* states, void* workspace, size_t workspace_bytes,
@@ -289,7 +322,14 @@ int llattn_gdn_prefill(const void* q, const void* k, const void* v, const void* 
     if (rc != 0) return rc;
     cudaError_t e = cudaMemsetAsync(states, 0, (size_t)B * H * K * V * L * sizeof(float), (cudaStream_t)stream);
     if (e != cudaSuccess) return (int)e;
-    return gdn_fwd_impl(q, k, v, beta, g, lambda, o, g_cum, Aw, Au, workspace, workspace_bytes, B, T, H, K, V, L, stream, false, states);
+    llattn::GdnStateOut out;
+    out.p = states;
+    out.rows = K;
+    out.col = L;
+    out.row = (long)V * L;
+    out.level = 1;
+    out.bh = (long)K * V * L;
+    return gdn_fwd_impl(q, k, v, beta, g, lambda, o, g_cum, Aw, Au, workspace, workspace_bytes, B, T, H, K, V, L, stream, false, out);
 }
 
 int llattn_gdn_fwd(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
@@ -306,7 +346,7 @@ int llattn_gdn_fwd_keep(const void* q, const void* k, const void* v, const void*
 
 static int gdn_fwd_impl(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                         void* o, float* g_cum, void* Aw, void* Au, void* workspace, size_t workspace_bytes,
-                        int B, int T, int H, int K, int V, int L, void* stream, bool keep, float* final_states) {
+                        int B, int T, int H, int K, int V, int L, void* stream, bool keep, const llattn::GdnStateOut& final_states) {
     int rc = gdn_check(B, T, H, K, V, L);
     if (rc != 0) return rc;
     if (!q || !k || !v || !beta || !g || !lambda || !o || !g_cum || !Aw || !Au) return LLATTN_ERR_NULL;

@@ -491,11 +491,12 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const GdnParams p) {
                 }
             }
         }
-        if (OUT && c == p.NT - 1 && p.final_states != nullptr) {
+        if (OUT && c == p.NT - 1 && p.final_states.p != nullptr) {
             // prefill hand-off: the level states every token of the last chunk starts from.  Level 7 + lv holds the block
             // of 2^lv chunks for each set bit lv of c (the binary-indexed tree as it stands before this chunk); the
             // caller steps the last chunk's tokens through the decode kernel, which fills levels 0..6.
-            float* dst = p.final_states + ((long)b * p.H + h) * KD * p.V * p.L;
+            const GdnStateOut& fs = p.final_states;
+            float* dst = fs.p + ((long)b * p.H + h) * fs.bh + INTRA_LEVELS * fs.level;
 #pragma unroll
             for (int lv = 0; lv < GDN_MAXLEV; ++lv) {
                 if (lv < nlev && ((c >> lv) & 1)) {
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const GdnParams p) {
                             for (int e = 0; e < 4; ++e) {
                                 const int row = warp * 16 * MT + mt * 16 + lr + (e >> 1) * 8;
                                 const int col = vs * GDN_VS + nt * 8 + lc2 + (e & 1);
-                                dst[((long)row * p.V + col) * p.L + INTRA_LEVELS + lv] = M[lv][mt][nt][e];
+                                if (row < fs.rows) dst[row * fs.row + col * fs.col + lv * fs.level] = M[lv][mt][nt][e];
                             }
                 }
             }

@@ -350,18 +350,20 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
             stage_ut((c + 1) & 1);                                   // u of chunk c + 1 (needed only if that chunk has a transition)
             fetch_u(c + 2);
         }
-        if (OUT && c == NT - 1 && p.final_states != nullptr) {
+        if (OUT && c == NT - 1 && p.final_states.p != nullptr) {
             // prefill hand-off: the level states every token of the last chunk starts from.  Level 7 + lv holds the block
             // of 2^lv chunks for each set bit lv of c (the binary-indexed tree as it stands before this chunk); the
             // caller steps the last chunk's tokens through the decode kernel, which fills levels 0..6.
-            float* dst = p.final_states + (((long)b * p.H + h) * gtc::KD + row) * (long)p.V * p.L;
+            const GdnStateOut& fs = p.final_states;
+            float* dst = fs.p + ((long)b * p.H + h) * fs.bh + row * fs.row + INTRA_LEVELS * fs.level;
 #pragma unroll 1
             for (uint32_t m = live; m; m &= m - 1) {
                 const int lv = __ffs(m) - 1;
                 float v[16];
                 umma::tmem_ld16(tM + lv * gtc::VS, v);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) dst[(long)(col0 + j) * p.L + INTRA_LEVELS + lv] = v[j];
+                for (int j = 0; j < 16; ++j)
+                    if (row < fs.rows) dst[(col0 + j) * fs.col + lv * fs.level] = v[j];
             }
         }
         STAMP();

@@ -122,6 +122,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// a per-head parameter that the caller keeps in fp32 or bf16
+__device__ __forceinline__ float load_param(const void* p, int i, bool f32) {
+    return f32 ? reinterpret_cast<const float*>(p)[i] : __bfloat162float(reinterpret_cast<const bf16*>(p)[i]);
+}
+
 // exp(x) for x <= 0 (and 0 for x > 0 never arises in causal positions; callers mask)
 __device__ __forceinline__ float fexp(float x) { return __expf(x); }
 

@@ -11,6 +11,14 @@ namespace llattn {
 constexpr int GDN_VS = 32;          // V columns per CTA of the sequential scans
 constexpr int GDN_MAXLEV = 8;       // inter-chunk levels (T up to 64 * 2^8 = 16384)
 
+// Where the level states before the last chunk go (prefill hand-off): element (b*H + h, level, row, column) at
+// p[bh * .bh + level * .level + row * .row + column * .col]; rows beyond `rows` (padding of narrow keys) are not written.
+struct GdnStateOut {
+    float* p = nullptr;
+    long bh = 0, level = 0, row = 0, col = 0;
+    int rows = 0;
+};
+
 struct GdnParams {
     // inputs (q, k already L2-normalised / scaled by the caller, one q/k per head)
     const __nv_bfloat16* q;      // (B,T,H,K)
@@ -22,7 +30,7 @@ struct GdnParams {
     // outputs
     __nv_bfloat16* o;            // (B,T,H,V)
     float* g_cum;                // (B,T,H)
-    float* final_states;         // optional (B,H,K,V,L) fp32: level states as of the start of the last chunk (prefill hand-off)
+    GdnStateOut final_states;    // optional, fp32: level states as of the start of the last chunk
     __nv_bfloat16* Aw;           // (B,T,H,64)  (I + A)^-1 rows, saved for the backward
     __nv_bfloat16* Au;           // (B,T,H,64)  (I + A*Gamma)^-1 rows
     // scratch written by the chunk preparation, read by the scan

@@ -14,14 +14,19 @@
 //       (levels 0..j are summed into level j); then every level is decayed by exp(g), level 0 becomes
 //       k v^T, and o = q . sum_l lambda_l S_l.  HBM-bound: reads and writes L*K*V floats per head.
 #include "llattn_common.cuh"
+#include "llattn_mamba2.h"
 #include "../../include/llattn.h"
 
 namespace llattn {
 
-template <int KD, int VD>
+// LM: level-major states (B,H,L,K,V), of tensors that are Tp >= T tokens long, and with the segment summaries of the forward
+// call on the same tensors (seg_F, seg_D; null when there is one segment) for the levels that hold whole segments: the sum over
+// a bucket of 2^j segments is then an element-wise pass over 2^j summaries instead of 2^(j+3) products of 64 tokens.
+template <int KD, int VD, bool LM>
 __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v,
                                                                     const float* __restrict__ g, float* __restrict__ states,
-                                                                    int B, int T, int H, int G, int L) {
+                                                                    const float* __restrict__ seg_F, const float* __restrict__ seg_D,
+                                                                    int B, int T, int Tp, int H, int G, int L) {
     constexpr int LDK = KD + PAD, LDV = VD + PAD;
     constexpr int MT = KD / 128;                         // 16-row tiles of the K x V result per warp (8 warps)
     static_assert(KD % 128 == 0 || KD == 64, "K rows are split over the warps");
@@ -43,14 +48,49 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         s0 = (m >> lev) << lev;                          // tokens taken by the higher set bits
         s1 = s0 + (1 << (lev - 1));
     }
-    float* out = states + ((long)(b * H + h) * KD * VD) * L + lev;
+    float* out = states + ((long)(b * H + h) * KD * VD) * L + (LM ? (long)lev * KD * VD : (long)lev);
     if (s1 == s0) {
-        for (int e = tid; e < KD * VD; e += 256) out[(long)e * L] = 0.f;
+        if (LM) {
+            for (int e = tid * 4; e < KD * VD; e += 1024) *reinterpret_cast<float4*>(out + e) = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+            for (int e = tid; e < KD * VD; e += 256) out[(long)e * L] = 0.f;
+        }
+        return;
+    }
+    constexpr int SEG = 512;
+    if (LM && seg_F != nullptr && s1 - s0 >= SEG) {
+        // after the bucket: whole segments up to the one of the last token, then that segment's tokens up to the last one
+        const int r0 = s0 / SEG, r1 = s1 / SEG, rl = m / SEG, NS = (Tp + SEG - 1) / SEG;
+        const float* D = seg_D + (long)(b * H + h) * NS;
+        const float* F = seg_F + (long)(b * H + h) * NS * KD * VD;
+        float part = 0.f;
+        for (int r = r1 + tid; r < rl; r += 256) part += D[r];
+        for (int t = rl * SEG + tid; t <= m; t += 256) part += g[((long)b * Tp + t) * H + h];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
+        if (lane == 0) sRed[warp] = part;
+        __syncthreads();
+        float after = 0.f;
+        for (int w = 0; w < 8; ++w) after += sRed[w];
+        float4 acc[KD * VD / 1024];
+#pragma unroll
+        for (int i = 0; i < KD * VD / 1024; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = r1 - 1; r >= r0; --r) {
+            const float w = fexp(after);
+#pragma unroll
+            for (int i = 0; i < KD * VD / 1024; ++i) {
+                const float4 f = *reinterpret_cast<const float4*>(F + (long)r * KD * VD + i * 1024 + tid * 4);
+                acc[i].x += w * f.x; acc[i].y += w * f.y; acc[i].z += w * f.z; acc[i].w += w * f.w;
+            }
+            after += D[r];
+        }
+#pragma unroll
+        for (int i = 0; i < KD * VD / 1024; ++i) *reinterpret_cast<float4*>(out + i * 1024 + tid * 4) = acc[i];
         return;
     }
     // decay from the end of the bucket to the last token: sum_{r = s1 .. m} g_r
     float part = 0.f;
-    for (int r = s1 + tid; r <= m; r += 256) part += g[((long)b * T + r) * H + h];
+    for (int r = s1 + tid; r <= m; r += 256) part += g[((long)b * Tp + r) * H + h];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
     if (lane == 0) sRed[warp] = part;
@@ -71,8 +111,8 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         // in-tile decay: token a + i gets exp(after + sum_{r = a+i+1 .. e1-1} g_r)
         if (warp == 0) {
             const int i0 = CH - 1 - 2 * lane, i1 = CH - 2 - 2 * lane;      // reversed order
-            float x0 = (i0 + 1 < n) ? g[((long)b * T + a + i0 + 1) * H + h] : 0.f;
-            float x1 = (i1 + 1 < n) ? g[((long)b * T + a + i1 + 1) * H + h] : 0.f;
+            float x0 = (i0 + 1 < n) ? g[((long)b * Tp + a + i0 + 1) * H + h] : 0.f;
+            float x1 = (i1 + 1 < n) ? g[((long)b * Tp + a + i1 + 1) * H + h] : 0.f;
             warp_cumsum64(x0, x1, lane);
             sDec[i0] = (i0 < n) ? fexp(after + x0) : 0.f;
             sDec[i1] = (i1 < n) ? fexp(after + x1) : 0.f;
@@ -80,7 +120,7 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         for (int e = tid; e < CH * (KD / 8); e += 256) {
             const int i = e / (KD / 8), c8 = (e % (KD / 8)) * 8;
             uint4 x = make_uint4(0, 0, 0, 0);
-            if (i < n) x = *reinterpret_cast<const uint4*>(k + (((long)b * T + a + i) * G + grp) * KD + c8);
+            if (i < n) x = *reinterpret_cast<const uint4*>(k + (((long)b * Tp + a + i) * G + grp) * KD + c8);
             *reinterpret_cast<uint4*>(sK + i * LDK + c8) = x;
         }
         __syncthreads();
@@ -88,7 +128,7 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
             const int i = e / (VD / 8), c8 = (e % (VD / 8)) * 8;
             uint4 x = make_uint4(0, 0, 0, 0);
             if (i < n) {
-                x = *reinterpret_cast<const uint4*>(v + (((long)b * T + a + i) * H + h) * VD + c8);
+                x = *reinterpret_cast<const uint4*>(v + (((long)b * Tp + a + i) * H + h) * VD + c8);
                 const float d = sDec[i];
                 uint32_t* xw = reinterpret_cast<uint32_t*>(&x);
 #pragma unroll
@@ -105,7 +145,7 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         float tile = 0.f;
         if (warp == 0) {
             float x = 0.f;
-            for (int i = lane; i < n; i += 32) x += g[((long)b * T + a + i) * H + h];
+            for (int i = lane; i < n; i += 32) x += g[((long)b * Tp + a + i) * H + h];
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
             if (lane == 0) sRed[0] = x;
@@ -120,9 +160,14 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
 #pragma unroll
             for (int nt = 0; nt < VD / 8; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int row = warp * 16 * MTW + mt * 16 + lr + (e >> 1) * 8, col = nt * 8 + lc2 + (e & 1);
-                    out[((long)row * VD + col) * L] = acc[mt][nt][e];
+                for (int e = 0; e < 4; e += 2) {
+                    const int row = warp * 16 * MTW + mt * 16 + lr + (e >> 1) * 8, col = nt * 8 + lc2;
+                    if (LM) {
+                        *reinterpret_cast<float2*>(out + row * VD + col) = make_float2(acc[mt][nt][e], acc[mt][nt][e + 1]);
+                    } else {
+                        out[((long)row * VD + col) * L] = acc[mt][nt][e];
+                        out[((long)row * VD + col + 1) * L] = acc[mt][nt][e + 1];
+                    }
                 }
     }
 }
@@ -191,17 +236,44 @@ __global__ void __launch_bounds__(256) mamba2_step_kernel(float* __restrict__ st
 
 extern "C" {
 
-int llattn_mamba2_final_state(const void* k, const void* v, const float* g, float* states,
-                              int B, int T, int H, int G, int K, int V, int L, void* stream) {
+static int final_state_check(int B, int T, int H, int G, int K, int V, int L) {
     if (B <= 0 || T <= 0 || H <= 0 || G <= 0 || H % G != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!((K == 64 || K == 128) && V == 64) || L <= 0 || L > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (L < 1 + (32 - __builtin_clz((unsigned)(T - 1) | 1u)) && T > 1) return LLATTN_ERR_TOO_FEW_LEVELS;
+    return 0;
+}
+
+int llattn_mamba2_final_state(const void* k, const void* v, const float* g, float* states,
+                              int B, int T, int H, int G, int K, int V, int L, void* stream) {
+    const int rc = final_state_check(B, T, H, G, K, V, L);
+    if (rc != 0) return rc;
     if (!k || !v || !g || !states) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
     dim3 grid(B * H, L);
     cudaStream_t st = (cudaStream_t)stream;
-    if (K == 128) { llattn::mamba2_final_state_kernel<128, 64><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, B, T, H, G, L); LLATTN_LAUNCHED(); }
-    else { llattn::mamba2_final_state_kernel<64, 64><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, B, T, H, G, L); LLATTN_LAUNCHED(); }
+    if (K == 128) llattn::mamba2_final_state_kernel<128, 64, false><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, nullptr, nullptr, B, T, T, H, G, L);
+    else llattn::mamba2_final_state_kernel<64, 64, false><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, nullptr, nullptr, B, T, T, H, G, L);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, float* states, const void* fwd_workspace,
+                                size_t fwd_workspace_bytes, int B, int T, int Tp, int H, int G, int K, int V, int L, void* stream) {
+    const int rc = final_state_check(B, T, H, G, K, V, L);
+    if (rc != 0) return rc;
+    if (Tp < T || Tp % 64 != 0) return LLATTN_ERR_BAD_LENGTH;
+    if (!k || !v || !g || !states) return LLATTN_ERR_NULL;
+    const float *seg_F = nullptr, *seg_D = nullptr;
+    if (fwd_workspace != nullptr) {
+        const int e = llattn::mamba2_fwd_workspace_segments(fwd_workspace, fwd_workspace_bytes, B, Tp, H, G, K, V, &seg_F, &seg_D);
+        if (e != 0) return e;
+    }
+    using bf = __nv_bfloat16;
+    dim3 grid(B * H, L);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (K == 128) llattn::mamba2_final_state_kernel<128, 64, true><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, seg_F, seg_D, B, T, Tp, H, G, L);
+    else llattn::mamba2_final_state_kernel<64, 64, true><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, seg_F, seg_D, B, T, Tp, H, G, L);
+    LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

@@ -1,0 +1,402 @@
+// Prompts of any length: what surrounds the chunkwise kernels when a prompt is not a whole number of chunks.
+//
+// Reference being replaced: hattention_prefill (hattention/kernel.py:469-560), which runs the chunkwise kernels on the whole
+// chunks, steps the remaining tokens one by one and rebuilds the levels inside the last chunk (postprocess_prefill_hstate_,
+// :378-466), and the torch operators around it (hattention/mamba_apis.py:346-399, gated_delta_rule_apis.py:65-92).
+//
+// Here the tensors that the chunkwise kernels read are written Tp >= T tokens long by the pass that prepares them anyway.  A
+// token of zeros (k, v, beta zero, log decay zero) leaves every level state as it is and its output rows are not used, so the
+// chunkwise kernels cover the whole prompt and no token is stepped: a 1000-token prompt of 48 heads is eight launches instead
+// of forty decode steps behind the chunkwise launches.
+#include "llattn_common.cuh"
+#include "../../include/llattn.h"
+
+namespace llattn {
+
+__device__ __forceinline__ float softplus_p(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
+
+// ---- log-linear Mamba-2: the preparation of mamba_prep.cu with the padding of v, g, lambda, q and k in the same launch.
+// LPR lanes per (b, t, h) row of the padded tensors; the blocks behind those of the rows copy q and k (16 bytes a thread).
+template <int LPR>
+__global__ void __launch_bounds__(256) m2_prompt_prep_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dt_raw, const void* __restrict__ dt_bias, int bias_f32,
+                                                             const float* __restrict__ A, const bf16* __restrict__ dl, const void* __restrict__ Lp, int lp_f32,
+                                                             const uint4* __restrict__ q, const uint4* __restrict__ k, bf16* __restrict__ v,
+                                                             float* __restrict__ g, bf16* __restrict__ lam, uint4* __restrict__ qp, uint4* __restrict__ kp,
+                                                             int B, int T, int Tp, int H, int P, int L, int Lo, int mode, int row_blocks, int qk16) {
+    if ((int)blockIdx.x >= row_blocks) {
+        // qk16: 16-byte words of a token of q (and of k)
+        const unsigned e = (blockIdx.x - row_blocks) * 256u + threadIdx.x;
+        const unsigned n = (unsigned)B * Tp * qk16;
+        if (e >= 2u * n) return;
+        const bool is_k = e >= n;
+        const unsigned i = is_k ? e - n : e;
+        const unsigned c = i % qk16, tok = i / qk16, t = tok % Tp, b = tok / Tp;
+        uint4 w = make_uint4(0, 0, 0, 0);
+        if (t < (unsigned)T) w = (is_k ? k : q)[((long)b * T + t) * qk16 + c];
+        (is_k ? kp : qp)[i] = w;
+        return;
+    }
+    const int lane = threadIdx.x % LPR;
+    const unsigned row = (blockIdx.x * 256u + threadIdx.x) / LPR;
+    if (row >= (unsigned)B * Tp * H) return;
+    const int h = row % H;
+    const unsigned tok = row / H, t = tok % Tp, b = tok / Tp;
+    const bool in = t < (unsigned)T;
+    const long src = in ? ((long)b * T + t) * H + h : 0;
+    float dt = 0.f;
+    if (in) {
+        dt = __bfloat162float(dt_raw[src]);
+        if (dt_bias) dt += load_param(dt_bias, h, bias_f32);
+        dt = softplus_p(dt);
+    }
+    if (lane == 0) g[row] = in ? A[h] * dt : 0.f;
+    if (lane * 8 < P) {
+        uint4 out = make_uint4(0, 0, 0, 0);
+        if (in) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(x + src * P + lane * 8);
+            const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&raw);
+            uint32_t* o = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = pack_bf16(__bfloat162float(hx[i].x) * dt, __bfloat162float(hx[i].y) * dt);
+        }
+        *reinterpret_cast<uint4*>(v + (long)row * P + lane * 8) = out;
+    }
+    for (int j = lane; j < Lo; j += LPR) {
+        float r = 0.f;
+        if (in && j < L) {
+            const float lp = load_param(Lp, h * L + j, lp_f32), d = __bfloat162float(dl[src * L + j]);
+            if (mode == 0) r = softplus_p(lp * d);
+            else if (mode == 1) r = __expf(-__expf(lp) * softplus_p(d));
+            else r = lp * d;
+        }
+        lam[(long)row * Lo + j] = __float2bfloat16(r);
+    }
+}
+
+// y = o + D x for the T tokens of x; o is Tp tokens long; y has the dtype of D (bf16 without D).  P / 8 threads a row.
+template <bool F32OUT>
+__global__ void __launch_bounds__(256) m2_prompt_residual_kernel(const bf16* __restrict__ o, const bf16* __restrict__ x, const void* __restrict__ D,
+                                                                 void* __restrict__ y, int B, int T, int Tp, int H, int P) {
+    const unsigned p8 = P / 8;
+    const unsigned e = blockIdx.x * 256u + threadIdx.x;
+    const unsigned row = e / p8, c = (e % p8) * 8;
+    if (row >= (unsigned)B * T * H) return;
+    const unsigned h = row % H, tok = row / H, t = tok % T, b = tok / T;
+    const long at = (long)row * P + c;
+    const uint4 ro = *reinterpret_cast<const uint4*>(o + (((long)b * Tp + t) * H + h) * P + c);
+    uint4 rx = make_uint4(0, 0, 0, 0);
+    if (D) rx = *reinterpret_cast<const uint4*>(x + at);
+    const float d = D ? load_param(D, h, F32OUT) : 0.f;
+    const __nv_bfloat162* ho = reinterpret_cast<const __nv_bfloat162*>(&ro);
+    const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&rx);
+    float r[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        r[2 * i] = __bfloat162float(ho[i].x) + __bfloat162float(hx[i].x) * d;
+        r[2 * i + 1] = __bfloat162float(ho[i].y) + __bfloat162float(hx[i].y) * d;
+    }
+    if (F32OUT) {
+        float* w = reinterpret_cast<float*>(y) + at;
+        *reinterpret_cast<float4*>(w) = make_float4(r[0], r[1], r[2], r[3]);
+        *reinterpret_cast<float4*>(w + 4) = make_float4(r[4], r[5], r[6], r[7]);
+    } else {
+        uint4 out;
+        uint32_t* w = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = pack_bf16(r[2 * i], r[2 * i + 1]);
+        *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(y) + at) = out;
+    }
+}
+
+// ---- token-padded copies of up to eight (B, T, ...) tensors in one launch
+struct PadList {
+    const void* src[8];
+    void* dst[8];
+    int src_bytes[8], dst_bytes[8];     // bytes of a token (the rest of a longer destination row is zero)
+    int unit[8];                        // copy unit: 16, 4 or 2 bytes
+    unsigned first_block[9];
+    int n, B, T, Tp;
+};
+
+__global__ void __launch_bounds__(256) pad_tokens_kernel(const __grid_constant__ PadList l) {
+    int i = 0;
+    while (i + 1 < l.n && blockIdx.x >= l.first_block[i + 1]) ++i;
+    const unsigned per = l.dst_bytes[i] / l.unit[i], real = l.src_bytes[i] / l.unit[i];
+    const unsigned long e = (unsigned long)(blockIdx.x - l.first_block[i]) * 256u + threadIdx.x;
+    if (e >= (unsigned long)l.B * l.Tp * per) return;
+    const unsigned c = (unsigned)(e % per), tok = (unsigned)(e / per), t = tok % l.Tp, b = tok / l.Tp;
+    const bool in = t < (unsigned)l.T && c < real;
+    const unsigned long s = ((unsigned long)b * l.T + t) * real + c;
+    if (l.unit[i] == 16) reinterpret_cast<uint4*>(l.dst[i])[e] = in ? reinterpret_cast<const uint4*>(l.src[i])[s] : make_uint4(0, 0, 0, 0);
+    else if (l.unit[i] == 4) reinterpret_cast<uint32_t*>(l.dst[i])[e] = in ? reinterpret_cast<const uint32_t*>(l.src[i])[s] : 0u;
+    else reinterpret_cast<unsigned short*>(l.dst[i])[e] = in ? reinterpret_cast<const unsigned short*>(l.src[i])[s] : (unsigned short)0;
+}
+
+// ---- Gated DeltaNet: q, k normalised (q scaled), widened to Ko columns and expanded to one per head, lambda scaled, and every
+// tensor padded to Tp tokens, in one launch.  16 lanes per (b, t, h) row.
+struct GdnPrepArgs {
+    const bf16 *q, *k;       // (B,T,G,K)
+    const bf16 *v;           // (B,T,H,V)
+    const bf16* beta;        // (B,T,H)
+    const float* g;          // (B,T,H)
+    const bf16* l;           // (B,T,H,L)
+    bf16 *qn, *kn;           // (B,Tp,H,Ko)
+    bf16 *vp, *bp;           // (B,Tp,H,V) in slices of v_slice columns, (B,Tp,H)
+    float* gp;               // (B,Tp,H)
+    bf16* lp;                // (B,Tp,H,Lo)
+    int B, T, Tp, H, G, K, Ko, V, v_slice, L, Lo;
+    float scale, lam_mul;    // lam_mul = 0: lambda as it is
+};
+
+__global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_constant__ GdnPrepArgs a) {
+    const int lane = threadIdx.x & 15;
+    const unsigned row = blockIdx.x * 16u + (threadIdx.x >> 4);
+    const unsigned rows = (unsigned)a.B * a.Tp * a.H;
+    const bool have = row < rows;
+    const unsigned h = row % a.H, tok = row / a.H, t = tok % a.Tp, b = tok / a.Tp;
+    const bool in = have && t < (unsigned)a.T;
+    const long tr = in ? (long)b * a.T + t : 0;
+    const long src = tr * a.H + h, qsrc = tr * a.G + h / (a.H / a.G);
+    uint4 raw[2];
+    float rstd[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        raw[w] = make_uint4(0, 0, 0, 0);
+        if (in && lane * 8 < a.K) raw[w] = *reinterpret_cast<const uint4*>((w ? a.k : a.q) + qsrc * a.K + lane * 8);
+        const __nv_bfloat162* f = reinterpret_cast<const __nv_bfloat162*>(&raw[w]);
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float x0 = __bfloat162float(f[i].x), x1 = __bfloat162float(f[i].y);
+            ss += x0 * x0 + x1 * x1;
+        }
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+        rstd[w] = rsqrtf(ss + 1e-6f);
+    }
+    if (!have) return;
+    if (lane * 8 < a.Ko) {
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const __nv_bfloat162* f = reinterpret_cast<const __nv_bfloat162*>(&raw[w]);
+            uint4 out;
+            __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&out);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                o[i] = __floats2bfloat162_rn(__bfloat162float(f[i].x) * rstd[w], __bfloat162float(f[i].y) * rstd[w]);
+                if (w == 0) o[i] = __floats2bfloat162_rn(__bfloat162float(o[i].x) * a.scale, __bfloat162float(o[i].y) * a.scale);
+            }
+            *reinterpret_cast<uint4*>((w ? a.kn : a.qn) + (long)row * a.Ko + lane * 8) = out;
+        }
+    }
+    if (a.vp)
+        for (int c = lane * 8; c < a.V; c += 128) {
+            const int s0 = c / a.v_slice * a.v_slice, width = min(a.v_slice, a.V - s0);
+            uint4 w = make_uint4(0, 0, 0, 0);
+            if (in) w = *reinterpret_cast<const uint4*>(a.v + src * a.V + c);
+            *reinterpret_cast<uint4*>(a.vp + (long)rows * s0 + (long)row * width + c - s0) = w;
+        }
+    if (a.lp)
+        for (int j = lane; j < a.Lo; j += 16) {
+            float x = 0.f;
+            if (in && j < a.L) {
+                x = __bfloat162float(a.l[src * a.L + j]);
+                if (a.lam_mul != 0.f) x *= a.lam_mul;
+            }
+            a.lp[(long)row * a.Lo + j] = __float2bfloat16(x);
+        }
+    if (lane == 0 && a.gp) {
+        a.gp[row] = in ? a.g[src] : 0.f;
+        a.bp[row] = in ? a.beta[src] : __float2bfloat16(0.f);
+    }
+}
+
+// ---- Gated DeltaNet: the level states after the last token of a prompt.  The scan over chunks leaves the inter-chunk levels as
+// they stand before the last chunk; the tokens of that chunk advance them, and build the levels inside it.  Every level is
+// independent of the others: level 0 is the last token alone, level j + 1 (for each set bit j of the last token's position in
+// the chunk) starts from zero at the first of its 2^j tokens, takes their writes and then the transitions of the tokens behind
+// them, and the levels of earlier chunks take the transitions of all.  fp32 throughout, as the decode kernel steps.
+// One warp holds four value columns of one level (lane: KR = Ko / 32 state rows), so a token is four dot products over the
+// lanes and no barrier; grid (B*H, levels, V / 32).
+constexpr int TAIL_KD = 128;
+__global__ void __launch_bounds__(256) gdn_tail_states_kernel(const bf16* __restrict__ kn, const bf16* __restrict__ v, const bf16* __restrict__ beta,
+                                                              const float* __restrict__ g, float* __restrict__ states, int T, int Tp, int H,
+                                                              int K, int V, int Vs, int first_col, int L) {
+    constexpr int KR = TAIL_KD / 32;
+    __shared__ __align__(16) bf16 sK[CH * TAIL_KD];
+    __shared__ float sV[CH][33];
+    __shared__ float sB[CH], sD[CH];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int lev = blockIdx.y;
+    const int h = blockIdx.x % H, b = blockIdx.x / H;
+    const int m = T - 1, c0 = m & ~(CH - 1), n = m - c0 + 1;
+    const int col = blockIdx.z * 32 + warp * 4;              // first of this warp's columns in the slice of Vs columns
+    float* S = states + (((long)b * H + h) * L + lev) * (long)K * V + first_col + col;
+    // tokens [s0, s1) of the chunk write to this level; [s1, n) only advance it
+    int s0 = -1, s1 = 0;
+    if (lev == 0) {
+        s0 = n - 1;
+        s1 = n;
+    } else if (lev < INTRA_LEVELS) {
+        if (((m & (CH - 1)) >> (lev - 1)) & 1) {
+            s0 = ((m & (CH - 1)) >> lev) << lev;
+            s1 = s0 + (1 << (lev - 1));
+        }
+    } else if (lev - INTRA_LEVELS < 25 && ((m >> (lev - 1)) & 1)) {
+        s0 = s1 = 0;
+    }
+    float4 s[KR];
+#pragma unroll
+    for (int i = 0; i < KR; ++i) {
+        const int row = lane * KR + i;
+        s[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s0 >= 0 && lev >= INTRA_LEVELS && row < K) s[i] = *reinterpret_cast<const float4*>(S + (long)row * V);
+    }
+    if (s0 >= 0) {
+        const long t0 = (long)b * Tp + c0;
+        for (int e = tid; e < n * (TAIL_KD / 8); e += 256) {
+            const int i = e / (TAIL_KD / 8), c8 = (e % (TAIL_KD / 8)) * 8;
+            *reinterpret_cast<uint4*>(sK + i * TAIL_KD + c8) = *reinterpret_cast<const uint4*>(kn + ((t0 + i) * H + h) * TAIL_KD + c8);
+        }
+        for (int e = tid; e < n * 32; e += 256)
+            sV[e >> 5][e & 31] = __bfloat162float(v[((t0 + (e >> 5)) * H + h) * Vs + blockIdx.z * 32 + (e & 31)]);
+        for (int i = tid; i < n; i += 256) {
+            sB[i] = __bfloat162float(beta[(t0 + i) * H + h]);
+            sD[i] = fexp(g[(t0 + i) * H + h]);
+        }
+        __syncthreads();
+        for (int t = s0; t < n; ++t) {
+            const uint2 raw = *reinterpret_cast<const uint2*>(sK + t * TAIL_KD + lane * KR);
+            const __nv_bfloat162 k01 = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), k23 = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+            const float kr[KR] = {__bfloat162float(k01.x), __bfloat162float(k01.y), __bfloat162float(k23.x), __bfloat162float(k23.y)};
+            float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < KR; ++i) {
+                d.x += kr[i] * s[i].x; d.y += kr[i] * s[i].y; d.z += kr[i] * s[i].z; d.w += kr[i] * s[i].w;
+            }
+#pragma unroll
+            for (int w = 16; w > 0; w >>= 1) {
+                d.x += __shfl_xor_sync(0xffffffffu, d.x, w);
+                d.y += __shfl_xor_sync(0xffffffffu, d.y, w);
+                d.z += __shfl_xor_sync(0xffffffffu, d.z, w);
+                d.w += __shfl_xor_sync(0xffffffffu, d.w, w);
+            }
+            const float dec = sD[t], be = sB[t];
+            float4 w4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (t < s1) w4 = make_float4(sV[t][warp * 4], sV[t][warp * 4 + 1], sV[t][warp * 4 + 2], sV[t][warp * 4 + 3]);
+#pragma unroll
+            for (int i = 0; i < KR; ++i) {
+                const float bk = be * kr[i];
+                s[i].x = dec * (s[i].x - bk * d.x) + bk * w4.x;
+                s[i].y = dec * (s[i].y - bk * d.y) + bk * w4.y;
+                s[i].z = dec * (s[i].z - bk * d.z) + bk * w4.z;
+                s[i].w = dec * (s[i].w - bk * d.w) + bk * w4.w;
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < KR; ++i) {
+        const int row = lane * KR + i;
+        if (row < K) *reinterpret_cast<float4*>(S + (long)row * V) = s[i];
+    }
+}
+
+}  // namespace llattn
+
+extern "C" {
+
+int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl, const void* Lp,
+                              int lp_is_f32, const void* q, const void* k, void* v, float* g, void* lambda, void* q_pad, void* k_pad,
+                              int B, int T, int Tp, int H, int G, int K, int P, int L, int L_out, int lambda_mode, void* stream) {
+    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || G <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (P <= 0 || P > 256 || P % 8 != 0 || (G * K) % 8 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (L <= 0 || L > 64 || L_out < L || L_out > 64 || lambda_mode < 0 || lambda_mode > 2) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!x || !dt_raw || !A || !dl || !Lp || !v || !g || !lambda) return LLATTN_ERR_NULL;
+    if ((q_pad != nullptr) != (k_pad != nullptr) || (q_pad && (!q || !k))) return LLATTN_ERR_NULL;
+    using bf = __nv_bfloat16;
+    const long rows = (long)B * Tp * H;
+    const int lpr = P <= 64 ? 8 : (P <= 128 ? 16 : 32);
+    const int qk16 = G * K / 8;
+    const long copies = q_pad ? 2l * B * Tp * qk16 : 0;
+    if (rows * lpr > 0x7fffff00l || copies > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    const int row_blocks = (int)((rows * lpr + 255) / 256);
+    const unsigned grid = row_blocks + (unsigned)((copies + 255) / 256);
+    cudaStream_t st = (cudaStream_t)stream;
+#define LLATTN_PP(N) llattn::m2_prompt_prep_kernel<N><<<grid, 256, 0, st>>>((const bf*)x, (const bf*)dt_raw, dt_bias, bias_is_f32, A, (const bf*)dl, Lp, lp_is_f32, (const uint4*)q, (const uint4*)k, (bf*)v, g, (bf*)lambda, (uint4*)q_pad, (uint4*)k_pad, B, T, Tp, H, P, L, L_out, lambda_mode, row_blocks, qk16)
+    if (lpr == 8) LLATTN_PP(8);
+    else if (lpr == 16) LLATTN_PP(16);
+    else LLATTN_PP(32);
+#undef LLATTN_PP
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, void* y, int y_is_f32, int B, int T, int Tp, int H, int P, void* stream) {
+    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || P <= 0 || P % 8 != 0 || (long)B * T * H * P > 0x7fffff00l * 8) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!o || !y || (D && !x)) return LLATTN_ERR_NULL;
+    using bf = __nv_bfloat16;
+    const unsigned grid = (unsigned)(((long)B * T * H * (P / 8) + 255) / 256);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (y_is_f32) llattn::m2_prompt_residual_kernel<true><<<grid, 256, 0, st>>>((const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
+    else llattn::m2_prompt_residual_kernel<false><<<grid, 256, 0, st>>>((const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+int llattn_pad_tokens(int n, const void* const* src, void* const* dst, const int* src_bytes, const int* dst_bytes, int B, int T, int Tp,
+                      void* stream) {
+    if (n <= 0 || n > 8 || B <= 0 || T <= 0 || Tp < T || (long)B * Tp > 0x7fffffffl) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    llattn::PadList l = {};
+    l.n = n; l.B = B; l.T = T; l.Tp = Tp;
+    unsigned long blocks = 0;
+    for (int i = 0; i < n; ++i) {
+        if (!src[i] || !dst[i]) return LLATTN_ERR_NULL;
+        if (src_bytes[i] <= 0 || dst_bytes[i] < src_bytes[i]) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+        const size_t all = (size_t)src[i] | (size_t)dst[i] | (size_t)src_bytes[i] | (size_t)dst_bytes[i];
+        l.unit[i] = (all & 15) == 0 ? 16 : ((all & 3) == 0 ? 4 : 2);
+        if (all & 1) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+        l.src[i] = src[i]; l.dst[i] = dst[i]; l.src_bytes[i] = src_bytes[i]; l.dst_bytes[i] = dst_bytes[i];
+        l.first_block[i] = (unsigned)blocks;
+        blocks += ((unsigned long)B * Tp * (dst_bytes[i] / l.unit[i]) + 255) / 256;
+    }
+    if (blocks > 0x7ffffffful) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    l.first_block[n] = (unsigned)blocks;
+    llattn::pad_tokens_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(l);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
+                           void* qn, void* kn, void* v_pad, void* beta_pad, float* g_pad, void* lambda_pad,
+                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int v_slice, int L, int L_out, float scale,
+                           float lambda_mul, void* stream) {
+    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || G <= 0 || H % G != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (K <= 0 || K % 8 != 0 || K_out < K || K_out > 128 || K_out % 8 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (V <= 0 || V % 8 != 0 || v_slice <= 0 || v_slice % 8 != 0 || L <= 0 || L_out < L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if ((long)B * Tp * H > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!q || !k || !qn || !kn || (v_pad && !v) || (lambda_pad && !lambda) || (g_pad && (!g || !beta || !beta_pad))) return LLATTN_ERR_NULL;
+    using bf = __nv_bfloat16;
+    llattn::GdnPrepArgs a{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, (const bf*)lambda, (bf*)qn, (bf*)kn, (bf*)v_pad,
+                          (bf*)beta_pad, g_pad, (bf*)lambda_pad, B, T, Tp, H, G, K, K_out, V, v_slice, L, L_out, scale, lambda_mul};
+    const unsigned grid = (unsigned)(((long)B * Tp * H + 15) / 16);
+    llattn::gdn_prompt_prep_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, const float* g, float* states, int B, int T, int Tp, int H,
+                             int K, int V, int v_cols, int first_col, int L, void* stream) {
+    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || K <= 0 || K > llattn::TAIL_KD) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (v_cols <= 0 || v_cols % 32 != 0 || first_col < 0 || first_col % 4 != 0 || first_col + v_cols > V || V % 4 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (L <= 0 || L > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (T > 1 && L < 1 + (32 - __builtin_clz((unsigned)(T - 1) | 1u))) return LLATTN_ERR_TOO_FEW_LEVELS;
+    if (!kn || !v || !beta || !g || !states) return LLATTN_ERR_NULL;
+    using bf = __nv_bfloat16;
+    dim3 grid(B * H, L, v_cols / 32);
+    llattn::gdn_tail_states_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const bf*)kn, (const bf*)v, (const bf*)beta, g, states, T, Tp, H, K, V,
+                                                                          v_cols, first_col, L);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+}  // extern "C"

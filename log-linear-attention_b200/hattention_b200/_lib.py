@@ -69,6 +69,20 @@ def lib():
     L.llattn_gdn_prefill.argtypes = [_P] * 11 + [_P, ctypes.c_size_t] + [ctypes.c_int] * 6 + [_P]
     L.llattn_gdn_step.restype = ctypes.c_int
     L.llattn_gdn_step.argtypes = [_P] * 8 + [ctypes.c_int] * 6 + [_P]
+    _I, _U, _F = ctypes.c_int, ctypes.c_uint, ctypes.c_float
+    for name, args in {
+        "llattn_mamba2_layer_step": [_P] * 8 + [_I, _P, _I, _P, _I] + [_P] * 2 + [_I] * 6 + [_U] + [_I] * 4 + [_P],
+        "llattn_gdn_layer_step": [_P] * 8 + [_I] * 6 + [_U, _I, _I, _F, _F, _I, _P],
+        "llattn_pad_tokens": [_I] + [_P] * 4 + [_I] * 3 + [_P],
+        "llattn_mamba2_prompt_prep": [_P] * 3 + [_I] + [_P] * 3 + [_I] + [_P] * 7 + [_I] * 10 + [_P],
+        "llattn_mamba2_prompt_residual": [_P] * 4 + [_I] * 6 + [_P],
+        "llattn_mamba2_prompt_states": [_P] * 5 + [ctypes.c_size_t] + [_I] * 8 + [_P],
+        "llattn_gdn_prompt_prep": [_P] * 12 + [_I] * 11 + [_F, _F, _P],
+        "llattn_gdn_prefill_slice": [_P] * 11 + [_I] * 4 + [_P, ctypes.c_size_t] + [_I] * 6 + [_P],
+        "llattn_gdn_prompt_states": [_P] * 5 + [_I] * 9 + [_P],
+    }.items():
+        fn = getattr(L, name)
+        fn.restype, fn.argtypes = _I, args
     L.llattn_l2norm_fwd.restype = ctypes.c_int
     L.llattn_l2norm_fwd.argtypes = [_P, _P, ctypes.c_long, ctypes.c_int, ctypes.c_float, _P]
     L.llattn_l2norm_bwd.restype = ctypes.c_int

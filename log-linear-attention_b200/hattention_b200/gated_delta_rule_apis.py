@@ -6,7 +6,8 @@ from typing import Optional
 import torch
 
 from .base import HStruct, HType
-from .kernel import hattention_kernel, hattention_prefill, hattention_step
+from .kernel import gdn_layer_step, hattention_kernel, hattention_step, prefill
+from .recurrent import is_level_major
 
 SCALE_LAMBDA = True
 
@@ -42,20 +43,33 @@ def chunk_h_gated_delta_rule(
         warnings.warn(f"seq_len ({q.shape[1]}) < num_heads ({q.shape[2]}): inputs may be in head-first format")
     if scale is None:
         scale = k.shape[-1] ** -0.5
+    if output_final_state is not False:
+        lambda_mul = 1.0 / scale if SCALE_LAMBDA else 0.0
+        if initial_state is None:
+            if l.dtype != torch.bfloat16 and SCALE_LAMBDA:
+                l, lambda_mul = l / scale, 0.0
+            return prefill(q=q, k=k, v=v, b=beta, g=g, l=l, scale=scale, head_first=False, level_base=2, htype=HType.WEAK,
+                           hstruct=HStruct.GDELTA, use_qk_l2norm_in_kernel=True, lambda_mul=lambda_mul)
+        if not (q.ndim == 4 and k.ndim == 4 and v.ndim == 4 and beta.ndim == 3 and g.ndim == 3 and l.ndim == 4
+                and q.shape[1] == k.shape[1] == v.shape[1] == beta.shape[1] == g.shape[1] == l.shape[1] == 1):
+            raise ValueError
+        q, k, v, beta, g, l = (x.squeeze(1) for x in (q, k, v, beta, g, l))
+        s = initial_state
+        if (q.dtype == l.dtype == beta.dtype == torch.bfloat16 and g.dtype == s.dtype == torch.float32 and s.base == 2
+                and s.htype == HType.WEAK and s.hstruct == HStruct.GDELTA and v.is_cuda and is_level_major(s.states)):
+            with torch.no_grad():
+                o = gdn_layer_step(s, q.contiguous(), k.contiguous(), v.contiguous(), beta.contiguous(), g.contiguous(), l.contiguous(),
+                                   scale, lambda_mul)
+            return o.unsqueeze(1), s
+        if SCALE_LAMBDA:
+            l = l / scale
+        o, final_state = hattention_step(hstate=s, q=q, k=k, v=v, b=beta, g=g, l=l, scale=scale, level_base=2, htype=HType.WEAK,
+                                         hstruct=HStruct.GDELTA, use_qk_l2norm_in_kernel=True)
+        return o.unsqueeze(1), final_state
+    if initial_state is not None:
+        raise NotImplementedError
     if SCALE_LAMBDA:
         l = l / scale
-    common = dict(scale=scale, level_base=2, htype=HType.WEAK, hstruct=HStruct.GDELTA,
-                  use_qk_l2norm_in_kernel=use_qk_l2norm_in_kernel)
-    if output_final_state is False:
-        if initial_state is not None:
-            raise NotImplementedError
-        o = hattention_kernel(q=q, k=k, v=v, b=beta, g=g, l=l, head_first=False, **common)
-        return o, None
-    if initial_state is None:
-        return hattention_prefill(q=q, k=k, v=v, b=beta, g=g, l=l, head_first=False, **common)
-    if not (q.ndim == 4 and k.ndim == 4 and v.ndim == 4 and beta.ndim == 3 and g.ndim == 3 and l.ndim == 4
-            and q.shape[1] == k.shape[1] == v.shape[1] == beta.shape[1] == g.shape[1] == l.shape[1] == 1):
-        raise ValueError
-    o, final_state = hattention_step(hstate=initial_state, q=q.squeeze(1), k=k.squeeze(1), v=v.squeeze(1), b=beta.squeeze(1),
-                                     g=g.squeeze(1), l=l.squeeze(1), **common)
-    return o.unsqueeze(1), final_state
+    o = hattention_kernel(q=q, k=k, v=v, b=beta, g=g, l=l, scale=scale, head_first=False, level_base=2, htype=HType.WEAK,
+                          hstruct=HStruct.GDELTA, use_qk_l2norm_in_kernel=True)
+    return o, None

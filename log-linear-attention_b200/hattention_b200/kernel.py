@@ -6,8 +6,8 @@ import torch
 
 from .base import HStruct, HType
 from . import _lib
-from .chunkwise import chunkwise_bwd, chunkwise_fwd, final_states
-from .recurrent import HState  # noqa: F401  (re-exported: the reference imports it from both modules)
+from .chunkwise import chunkwise_bwd, chunkwise_fwd
+from .recurrent import HState, is_level_major  # noqa: F401  (HState: the reference imports it from both modules)
 
 
 # Keep the forward call's scratch alive until the backward, which then skips its recomputation: the
@@ -115,8 +115,9 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
                     use_qk_l2norm_in_kernel: bool = False):
     """One decoding step, signature of the reference's `hattention_step` (kernel.py:563-633):
     q, k (B,G,K), v (B,H,V), g (B,H), l (B,H,L)[, b (B,H)] -> (o (B,H,V), hstate).  One CUDA kernel per step for
-    either structure (`llattn_mamba2_step`, `llattn_gdn_step`); for the delta-rule structure q and k are
-    L2-normalised (q also scaled) first, as the reference does when `use_qk_l2norm_in_kernel` is set."""
+    either structure, the l2norm of the delta-rule structure included, which moves only the levels that hold tokens
+    (`llattn_mamba2_layer_step`, `llattn_gdn_layer_step`); states that a caller has stored with the level innermost go
+    through `llattn_mamba2_step` / `llattn_gdn_step`."""
     if not (q.ndim == 3 and k.ndim == 3 and v.ndim == 3 and g.ndim == 2 and l.ndim == 3
             and (b is None or b.ndim == 2) and g.dtype == hstate.dtype and q.dtype == k.dtype == v.dtype == l.dtype
             and hstate.base == level_base and hstate.htype == htype and hstate.hstruct == hstruct):
@@ -126,7 +127,6 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
     B, G, K = k.shape
     _, H, V = v.shape
     L = l.shape[-1]
-    lib = _lib.lib()
     if hstruct == HStruct.MAMBA2:
         if b is not None:
             raise ValueError
@@ -138,10 +138,23 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
         if use_qk_l2norm_in_kernel:
             if scale is None:
                 raise NotImplementedError
-            from .chunkwise_hgdn import l2norm_fwd
-            q, k = l2norm_fwd(q, scale), l2norm_fwd(k)
         elif scale is not None:
             raise NotImplementedError
+    if not v.is_cuda:
+        raise RuntimeError("the decode kernels need CUDA tensors (there is no CPU path)")
+    if is_level_major(hstate.states):
+        q_, k_, v_, l_ = (x.to(torch.bfloat16).contiguous() for x in (q, k, v, l))
+        g_ = g.contiguous()
+        if hstruct == HStruct.MAMBA2:
+            o = mamba2_layer_step(hstate, q_, k_, v_, None, g_, l_)
+        else:
+            o = gdn_layer_step(hstate, q_, k_, v_, b.to(torch.bfloat16).contiguous(), g_, l_, scale if use_qk_l2norm_in_kernel else None)
+        return o.to(v.dtype), hstate
+    lib = _lib.lib()
+    if hstruct == HStruct.GDELTA:
+        if use_qk_l2norm_in_kernel:
+            from .chunkwise_hgdn import l2norm_fwd
+            q, k = l2norm_fwd(q, scale), l2norm_fwd(k)
         if G != H:
             q, k = q.repeat_interleave(H // G, dim=1), k.repeat_interleave(H // G, dim=1)
     carry = hstate.cascade_counts()
@@ -163,15 +176,62 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
     return o.to(v.dtype), hstate
 
 
-@torch.no_grad()
+def mamba2_layer_step(hstate: HState, q, k, x, dt, g, dl, Lp=None, A=None, D=None, dt_bias=None, lambda_mode: int = 2,
+                      dt_softplus: bool = False) -> torch.Tensor:
+    """One launch of `llattn_mamba2_layer_step` on a level-major state: contiguous bf16 q, k, x, dt, dl; fp32 g, A; fp32 or bf16
+    Lp, D, dt_bias.  Without dt, x is v and g the log decay; without Lp, dl is lambda."""
+    B, G, K = k.shape
+    _, H, V = x.shape
+    L = dl.shape[-1]
+    dev = x.device.index
+    f32 = torch.float32
+    y = torch.empty(B, H, V, dtype=f32 if D is not None and D.dtype == f32 else torch.bfloat16, device=x.device)
+    live = hstate.live_levels()
+    carry = hstate.cascade_counts()
+    hstate.counts[0] += 1
+    rc = _lib.lib().llattn_mamba2_layer_step(
+        hstate.states.data_ptr(), q.data_ptr(), k.data_ptr(), x.data_ptr(), None if dt is None else dt.data_ptr(),
+        None if g is None else g.data_ptr(), dl.data_ptr(), None if Lp is None else Lp.data_ptr(), Lp is not None and Lp.dtype == f32,
+        None if D is None else D.data_ptr(), D is not None and D.dtype == f32, None if dt_bias is None else dt_bias.data_ptr(),
+        dt_bias is not None and dt_bias.dtype == f32, None if A is None else A.data_ptr(), y.data_ptr(), B, H, G, K, V, L, live, carry,
+        lambda_mode, dt_softplus, dev, torch._C._cuda_getCurrentRawStream(dev))
+    if rc != 0:
+        _lib.check(rc, "llattn_mamba2_layer_step")
+    return y
+
+
+def gdn_layer_step(hstate: HState, q, k, v, b, g, l, scale: Optional[float] = None, lambda_mul: float = 0.0) -> torch.Tensor:
+    """One launch of `llattn_gdn_layer_step` on a level-major state: contiguous bf16 q, k, v, b, l; fp32 g.  With a scale q and k
+    are normalised (and q scaled) first; lambda_mul != 0 multiplies lambda."""
+    B, G, K = k.shape
+    _, H, V = v.shape
+    dev = v.device.index
+    o = torch.empty(B, H, V, dtype=torch.bfloat16, device=v.device)
+    live = hstate.live_levels()
+    carry = hstate.cascade_counts()
+    hstate.counts[0] += 1
+    rc = _lib.lib().llattn_gdn_layer_step(
+        hstate.states.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), b.data_ptr(), g.data_ptr(), l.data_ptr(), o.data_ptr(),
+        B, H, G, K, V, l.shape[-1], live, carry, scale is not None, scale or 1.0, lambda_mul, dev,
+        torch._C._cuda_getCurrentRawStream(dev))
+    if rc != 0:
+        _lib.check(rc, "llattn_gdn_layer_step")
+    return o
+
+
 def hattention_prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct,
                        chunk_size: Optional[int] = None, use_qk_l2norm_in_kernel: bool = False):
     """Outputs for a prompt and the level states to continue from, signature of the reference's
-    `hattention_prefill` (kernel.py:469-560).  Mamba-2 structure: the largest multiple of the chunk size goes
-    through the chunkwise kernels, its level states come from one kernel (`final_states`), the remaining tokens
-    are stepped.  Delta-rule structure: the chunkwise kernels produce the outputs of the full chunks and the
-    inter-chunk level states as of the start of the last full chunk; that chunk's tokens and the remaining ones
-    are stepped through the decode kernel, which builds the levels inside the chunk."""
+    `hattention_prefill` (kernel.py:469-560).  The whole prompt goes through the chunkwise kernels, on tensors padded
+    with zero tokens where its length is not a number of chunks; the level states come from one more kernel.  Shapes
+    that the chunkwise kernels do not take and that are shorter than a chunk are stepped token by token."""
+    return prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chunk_size, use_qk_l2norm_in_kernel)
+
+
+@torch.no_grad()
+def prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chunk_size: Optional[int] = None,
+            use_qk_l2norm_in_kernel: bool = False, lambda_mul: float = 0.0):
+    """`hattention_prefill`; lambda_mul != 0 (delta-rule structure): lambda is multiplied by it on the way to the kernels."""
     if chunk_size is None:
         chunk_size = 64
     if head_first:
@@ -179,39 +239,36 @@ def hattention_prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, h
     B, T, G, K = k.shape
     _, _, H, V = v.shape
     L = l.shape[-1]
-    T0 = T - (T % chunk_size)
-    o = torch.zeros_like(v)
-    hstate = HState(base=level_base, htype=htype, hstruct=hstruct, shape=(B, H, K, V, L), dtype=torch.float32, device=g.device)
     if hstruct == HStruct.MAMBA2:
         if b is not None:
             raise ValueError
         if use_qk_l2norm_in_kernel or scale is not None:
             raise NotImplementedError
-        if T0 != 0:
-            o0, _, ht = chunkwise_fwd(q[:, :T0], k[:, :T0], v[:, :T0], g[:, :T0], l[:, :T0], head_first, level_base, htype,
-                                      chunk_size, True)
-            o[:, :T0] = o0.to(v.dtype)
-            hstate.states = ht
-            hstate.set_counts_after(T0)
-        first_step = T0
+        chunkwise = T >= chunk_size or (K in (64, 128) and V == 64)
     else:
-        from .chunkwise_hgdn import chunkwise_fwd as chunkwise_fwd_hgdn, l2norm_fwd
         if b is None:
             raise ValueError
         if not use_qk_l2norm_in_kernel or scale is None:
             raise NotImplementedError
-        first_step = 0
-        if T0 != 0:
-            qn, kn = l2norm_fwd(q[:, :T0], scale), l2norm_fwd(k[:, :T0])
-            _, o0, _, _, ht = chunkwise_fwd_hgdn(qn, kn, v[:, :T0], b[:, :T0], g[:, :T0], l[:, :T0], head_first, level_base,
-                                                 htype, chunk_size, True)
-            o[:, :T0] = o0.to(v.dtype)
-            hstate.states = ht
-            first_step = T0 - chunk_size
-            hstate.set_counts_before(first_step)
-    for t in range(first_step, T):
-        ot, hstate = hattention_step(hstate, q[:, t], k[:, t], v[:, t], b[:, t] if b is not None else None, g[:, t].float(),
-                                     l[:, t], scale, level_base, htype, hstruct, use_qk_l2norm_in_kernel)
-        if t >= T0:
-            o[:, t] = ot
+        chunkwise = T >= chunk_size or (K <= 128 and V % 64 == 0 and V <= 384)
+    ragged = T % chunk_size != 0
+    if (ragged or hstruct == HStruct.GDELTA) and not (q.dtype == k.dtype == v.dtype == l.dtype):
+        raise TypeError
+    if chunkwise:
+        if hstruct == HStruct.MAMBA2:
+            from .chunkwise import prompt_forward
+            o, states = prompt_forward(q, k, v, g, l, level_base, htype, chunk_size)
+        else:
+            from .chunkwise_hgdn import prompt_forward
+            o, states = prompt_forward(q, k, v, b, g, l, scale, level_base, htype, chunk_size, lambda_mul)
+        hstate = HState.holding(states, level_base, htype, hstruct)
+        hstate.set_counts_after(T)
+        return o.to(v.dtype), hstate
+    if lambda_mul != 0.0:
+        l = l * lambda_mul
+    o = torch.zeros_like(v)
+    hstate = HState(base=level_base, htype=htype, hstruct=hstruct, shape=(B, H, K, V, L), dtype=torch.float32, device=g.device)
+    for t in range(T):
+        o[:, t], hstate = hattention_step(hstate, q[:, t], k[:, t], v[:, t], b[:, t] if b is not None else None, g[:, t].float(),
+                                          l[:, t], scale, level_base, htype, hstruct, use_qk_l2norm_in_kernel)
     return o, hstate

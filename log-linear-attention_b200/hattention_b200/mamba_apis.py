@@ -7,9 +7,9 @@ import torch
 
 from . import _lib
 from .base import HStruct, HType
-from .chunkwise import chunkwise_bwd, chunkwise_fwd
-from .kernel import KEEP_FORWARD_STATES, hattention_kernel, hattention_prefill, hattention_step
-from .recurrent import HState
+from .chunkwise import chunkwise_bwd, chunkwise_fwd, prompt_forward_padded, prompt_length
+from .kernel import KEEP_FORWARD_STATES, hattention_kernel, hattention_prefill, hattention_step, mamba2_layer_step
+from .recurrent import HState, is_level_major
 
 try:
     from torchtune.modules import RotaryPositionalEmbeddings
@@ -150,6 +150,64 @@ def compute_lambda(L: torch.Tensor, dl: torch.Tensor, lambda_mode: Optional[str]
     raise ValueError
 
 
+_PARAM_DTYPES = (torch.float32, torch.bfloat16)
+
+
+def _fused_inference(tensors, params) -> bool:
+    """Whether the inference kernels take these operands: bf16 CUDA activations, fp32 or bf16 parameters, nothing to differentiate."""
+    if not all(t.dtype == torch.bfloat16 and t.is_cuda for t in tensors) or not all(p is None or p.dtype in _PARAM_DTYPES for p in params):
+        return False
+    return not torch.is_grad_enabled() or not any(t is not None and t.requires_grad for t in (*tensors, *params))
+
+
+def _prompt_is_fused(x, dt, A, B, C, dl, L, D, dt_bias, lambda_mode, level_base, htype, hstruct) -> bool:
+    return (FUSED_PREP and _fused_inference((x, dt, B, C, dl), (A, L, D, dt_bias)) and hstruct == HStruct.MAMBA2
+            and htype == HType.WEAK and level_base == 2 and lambda_mode in _LAMBDA_MODES and L.dim() == 2
+            and x.shape[-1] == 64 and B.shape[-1] in (64, 128) and dl.shape[-1] <= 32)
+
+
+def _prompt(x, dt, A, Bm, Cm, dl, Lp, D, dt_bias, mode: int, level_base: int, htype: HType):
+    """The prompt call of the layer: one pass prepares (and pads) everything the chunkwise kernels read, the chunkwise kernels, the
+    level states, one pass for the D residual."""
+    Bsz, T, H, P = x.shape
+    G, N = Bm.shape[2:]
+    L = dl.shape[-1]
+    Tp = prompt_length(T)
+    Lo = max(L, 7) if T < 64 else L
+    lib = _lib.lib()
+    with torch.no_grad(), torch.cuda.device(x.device):
+        stream = torch.cuda.current_stream().cuda_stream
+        x_, dt_, dl_, q, k = (t.contiguous() for t in (x, dt, dl, Cm, Bm))
+        A_ = A.float().contiguous()
+        Lp_ = Lp.contiguous()
+        bf = dict(dtype=torch.bfloat16, device=x.device)
+        v = torch.empty(Bsz, Tp, H, P, **bf)
+        lam = torch.empty(Bsz, Tp, H, Lo, **bf)
+        g = torch.empty(Bsz, Tp, H, dtype=torch.float32, device=x.device)
+        qp = kp = None
+        if Tp != T:
+            qp, kp = torch.empty(Bsz, Tp, G, N, **bf), torch.empty(Bsz, Tp, G, N, **bf)
+        f32 = torch.float32
+        rc = lib.llattn_mamba2_prompt_prep(
+            x_.data_ptr(), dt_.data_ptr(), _ptr(dt_bias), dt_bias is not None and dt_bias.dtype == f32, A_.data_ptr(), dl_.data_ptr(),
+            Lp_.data_ptr(), Lp_.dtype == f32, q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), lam.data_ptr(), _ptr(qp), _ptr(kp),
+            Bsz, T, Tp, H, G, N, P, L, Lo, mode, stream)
+        _lib.check(rc, "llattn_mamba2_prompt_prep")
+        if Tp != T:
+            q, k = qp, kp
+        o, states = prompt_forward_padded(q, k, v, g, lam, T, L, level_base, htype, 64)
+        if D is not None or (Tp != T and Bsz > 1):
+            y = torch.empty(Bsz, T, H, P, dtype=f32 if D is not None and D.dtype == f32 else torch.bfloat16, device=x.device)
+            rc = lib.llattn_mamba2_prompt_residual(o.data_ptr(), x_.data_ptr(), _ptr(D), y.data_ptr(), y.dtype == f32, Bsz, T, Tp, H, P,
+                                                   stream)
+            _lib.check(rc, "llattn_mamba2_prompt_residual")
+        else:
+            y = o[:, :T]
+    state = HState.holding(states, level_base, htype, HStruct.MAMBA2)
+    state.set_counts_after(T)
+    return y, state
+
+
 def hmamba_chunk_scan_combined(
     x: torch.Tensor,
     dt: torch.Tensor,
@@ -204,6 +262,8 @@ def hmamba_chunk_scan_combined(
         raise ValueError
     if return_final_states:
         # inference: outputs for the prompt and the level states to decode from (mamba_apis.py:381-399)
+        if _prompt_is_fused(x, dt, A, B, C, dl, L, D, dt_bias, lambda_mode, lambda_level_base, lambda_htype, lambda_hstruct):
+            return _prompt(x, dt, A, B, C, dl, L, D, dt_bias, _LAMBDA_MODES[lambda_mode], lambda_level_base, lambda_htype)
         if D is not None:
             D_residual = x * D[None, None, :, None]
         if dt_bias is not None:
@@ -285,11 +345,18 @@ def hselective_state_update(
     if lambda_level_max is None or lambda_level_base is None or lambda_htype is None or lambda_hstruct is None \
             or lambda_level_fixed is None:
         raise ValueError
+    if dt_bias is not None and dt_bias.shape != (nheads,):
+        raise ValueError
+    if (lambda_level_fixed and lambda_level_max == dlambda and lambda_mode in _LAMBDA_MODES and state.base == lambda_level_base
+            and state.htype == lambda_htype and state.hstruct == lambda_hstruct == HStruct.MAMBA2 and state.dtype == torch.float32
+            and _fused_inference((x, dt, B, C, dl), (A, L, D, dt_bias)) and is_level_major(state.states)):
+        y = mamba2_layer_step(state, C.contiguous(), B.contiguous(), x.contiguous(), dt.contiguous(), None, dl.contiguous(), L.contiguous(),
+                              A.float().contiguous(), D if D is None else D.contiguous(), dt_bias if dt_bias is None else dt_bias.contiguous(),
+                              _LAMBDA_MODES[lambda_mode], dt_softplus)
+        return y, state
     if D is not None:
         D_residual = x * D[None, :, None]
     if dt_bias is not None:
-        if dt_bias.shape != (nheads,):
-            raise ValueError
         dt = dt + dt_bias
     if dt_softplus:
         dt = torch.nn.functional.softplus(dt)

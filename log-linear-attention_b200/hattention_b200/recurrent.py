@@ -6,6 +6,26 @@ import torch
 from .base import HStruct, HType
 
 
+def is_level_major(states: torch.Tensor) -> bool:
+    """Whether a (B,H,K,V,L) tensor is stored (B,H,L,K,V): one contiguous K x V block per level of a head."""
+    B, H, K, V, L = states.shape
+    return states.stride() == (H * L * K * V, L * K * V, V, 1, K * V)
+
+
+def level_major_states(shape, device, dtype=torch.float32, zero=False) -> torch.Tensor:
+    """An (uninitialised) (B,H,K,V,L) tensor stored (B,H,L,K,V)."""
+    B, H, K, V, L = shape
+    make = torch.zeros if zero else torch.empty
+    return make((B, H, L, K, V), dtype=dtype, device=device).permute(0, 1, 3, 4, 2)
+
+
+def _zero_states(shape, dtype, device) -> torch.Tensor:
+    # level-major where the decode kernels for that layout take the value width: they move only the levels that hold tokens
+    if len(shape) == 5 and shape[3] % 16 == 0 and torch.device(device).type == "cuda":
+        return level_major_states(shape, device, dtype, zero=True)
+    return torch.zeros(shape, dtype=dtype, device=device)
+
+
 class HState:
     """Level states of one layer for decoding, with the fields of the reference's `HState`
     (hattention/recurrent.py:9-131): `states` (B,H,K,V,L) in `dtype` and one token count per level.
@@ -18,8 +38,27 @@ class HState:
         self.base, self.htype, self.hstruct = base, htype, hstruct
         self.shape, self.dtype, self.device = tuple(shape), dtype, device
         self.max_num_levels = self.shape[-1]
-        self.states = torch.zeros(self.shape, dtype=dtype, device=device)
+        self.states = _zero_states(self.shape, dtype, device)
         self.counts = [0] * self.max_num_levels
+
+    @classmethod
+    def holding(cls, states: torch.Tensor, base: int, htype: HType, hstruct: HStruct) -> "HState":
+        """A state around an existing tensor (B,H,K,V,L), which is adopted as it is; the counts start at zero."""
+        self = cls.__new__(cls)
+        self.base, self.htype, self.hstruct = base, htype, hstruct
+        self.shape, self.dtype, self.device = tuple(states.shape), states.dtype, states.device
+        self.max_num_levels = self.shape[-1]
+        self.states = states
+        self.counts = [0] * self.max_num_levels
+        return self
+
+    def live_levels(self) -> int:
+        """Bit l is set when level l holds tokens."""
+        live = 0
+        for level, count in enumerate(self.counts):
+            if count:
+                live |= 1 << level
+        return live
 
     def cascade_counts(self) -> int:
         """Runs the cascade on the counts; returns the level that receives the merged levels."""
@@ -62,7 +101,7 @@ class HState:
 
     def reset_states(self) -> None:
         """recurrent.py:102-103; the token counts restart with the states."""
-        self.states = torch.zeros_like(self.states)
+        self.states = _zero_states(self.shape, self.dtype, self.device)
         self.counts = [0] * self.max_num_levels
 
     def replace(self, other: "HState") -> None:
