@@ -131,6 +131,30 @@ int llattn_mamba2_prep_bwd(const void* x, const void* dt_raw, const float* dt_bi
                            long rows, int H, int P, int L, int lambda_mode, void* stream);
 int llattn_mamba2_residual(const void* o, const void* x, const float* D, void* y, int y_is_f32, long rows, int H, int P, void* stream);
 
+/* What the mixer does around the scan, in place on the rows of its projection zxbcdtdl (B,T,W), W = 2 H 64 + 2 G N + H + H L:
+ * [z (H 64) | x (H 64) | B (G N) | C (G N) | dt (H) | dl (H L)], bf16.  Replace the split, convolution, preparation, gated norm and
+ * the gradients of all of them in hmamba_split_conv1d_scan_combined (hattention/mamba_apis.py:186-259).
+ *   prep_fwd: (x, B, C) = silu(causal depthwise convolution with four taps); v = x softplus(dt + dt_bias), g = A softplus(...),
+ *        lambda = f(Lp, dl); writes x, v (B,T,H,64), k = B, q = C (B,T,G,N), g, lambda
+ *   prep_bwd: from dv, dq, dk, dg, dlambda of the scan and dy of the norm (for the D residual): every slice of dzx but z's, and
+ *        dconv_w (channels,4), dconv_b, dA, dbias, dLp ACCUMULATED into fp32 buffers the caller has cleared (the
+ *        first two, and dw below, at 16-byte boundaries)
+ *   norm_fwd: out = RMSNorm((o + D x) silu(z)) w, and rstd per token; norm_bwd: dy (gradient of o and of o + D x), the z slice of dzx, and
+ *        dw, dD accumulated
+ * conv_w, conv_b (may be NULL), dt_bias (may be NULL), Lp, D (may be NULL), w are fp32 or bf16 by their flags.  Constraints: heads of 64,
+ * N % 64 == 0, H <= 128, L <= 64. */
+int llattn_mixer_prep_fwd(const void* zx, const void* conv_w, int conv_w_f32, const void* conv_b, int conv_b_f32, const void* dt_bias,
+                          int bias_f32, const float* A, const void* Lp, int lp_f32, void* x, void* v, void* k, void* q, float* g,
+                          void* lambda, int B, int T, int H, int G, int N, int L, int lambda_mode, void* stream);
+int llattn_mixer_prep_bwd(const void* zx, const void* conv_w, int conv_w_f32, const void* conv_b, int conv_b_f32, const void* dt_bias,
+                          int bias_f32, const float* A, const void* Lp, int lp_f32, const void* D, int d_f32, const void* dv, const void* dy,
+                          const void* dq, const void* dk, const float* dg, const float* dlambda, void* dzx, float* dconv_w, float* dconv_b,
+                          float* dA, float* dbias, float* dLp, int B, int T, int H, int G, int N, int L, int lambda_mode, void* stream);
+int llattn_mixer_norm_fwd(const void* o, const void* x, const void* D, int d_f32, const void* zx, int zx_width, const void* w, int w_f32,
+                          void* out, float* rstd, long rows, int H, float eps, void* stream);
+int llattn_mixer_norm_bwd(const void* o, const void* x, const void* D, int d_f32, const void* zx, int zx_width, const void* w, int w_f32,
+                          const void* dn, const float* rstd, void* dy, void* dzx, float* dw, float* dD, long rows, int H, void* stream);
+
 /* Prefill hand-off: the level states after T tokens, states fp32 (B,H,K,V,L), every level written.
  * Level 0 is k_m v_m^T for the last token m = T-1; for each set bit j of m, level j+1 holds the 2^j
  * tokens that follow the buckets of the higher set bits, each decayed to token m; other levels are zero.

@@ -8,148 +8,144 @@
 // Rounding points follow torch's type promotion for bf16 activations with fp32 parameters (the
 // products are fp32 there): dt and g stay fp32, v and lam are rounded once to bf16 (the cast at the
 // kernel boundary, hattention/kernel.py), y = o + D x is fp32 or bf16 as the caller asks.
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-
+#include "rowwise.cuh"
 #include "../../include/llattn.h"
-#include "launch_count.h"
 
 namespace llattn {
 
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
+struct PrepArgs {
+    const __nv_bfloat16 *x, *dt_raw, *dl;      // (rows,P), (rows), (rows,L)
+    const float *dt_bias, *A, *Lp, *D;         // (H) or null, (H), (H,L), (H) or null
+    __nv_bfloat16 *v, *lam;
+    float* g;
+    const __nv_bfloat16 *dv, *dy;
+    const float *dg, *dlam;
+    __nv_bfloat16 *dx, *ddt, *ddl;
+    float *dA, *dbias, *dLp, *dD;
+    int H, P, L, mode;
+    int tokens, run;                           // B T, and how many of them a thread walks
+    int lpr;                                   // lanes of a head, 8 columns each
+    int row_blocks, lam_blocks;                // blocks of the x part and of the lambda part per run; the latter come first
+    int lam8, lam_runs;                        // the lambda columns come in eights; runs of that part
+};
 
-// LPR lanes share one (b,t,h) row; each lane owns 8 consecutive elements of the P-wide row and the
-// lambda columns lane, lane + LPR, ...
-template <int LPR, int MODE>
-__global__ void __launch_bounds__(256) m2_prep_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dt_raw,
-                                                          const float* __restrict__ dt_bias, const float* __restrict__ A,
-                                                          const __nv_bfloat16* __restrict__ dl, const float* __restrict__ Lp,
-                                                          __nv_bfloat16* __restrict__ v, float* __restrict__ g, __nv_bfloat16* __restrict__ lam,
-                                                          long rows, int H, int P, int L) {
-    const int lane = threadIdx.x % LPR;
-    const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
-    if (row >= rows) return;
-    const int h = (int)(row % H);
-    float t = __bfloat162float(dt_raw[row]);
-    if (dt_bias) t += dt_bias[h];
-    const float dt = softplus_f(t);
-    if (lane == 0) g[row] = A[h] * dt;
-    if (lane * 8 < P) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(x + row * P + lane * 8);
-        const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&raw);
-        uint4 out;
-        __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = __floats2bfloat162_rn(__bfloat162float(hx[i].x) * dt, __bfloat162float(hx[i].y) * dt);
-        *reinterpret_cast<uint4*>(v + row * P + lane * 8) = out;
+// Both passes: a group of LPR lanes owns one head and walks `run` tokens, eight columns a lane.  What depends on the (token, head)
+// alone is evaluated once by the group, each lane for one of LPR tokens, and the parameter sums stay in registers over the run.  The
+// loads of a token are not fetched ahead: few registers and many warps keep more bytes in flight than two tokens a thread did
+// (B = 2, T = 16384, 32 heads, L = 15: backward 321 us with a row per group, a shared-memory atomic per lambda column and a token
+// per thread before, 212 us with two tokens in flight and a thread per lambda column).
+template <int LPR>
+__global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_constant__ PrepArgs a) {
+    constexpr int U = 2;
+    const int lam_grid = a.lam_blocks * a.lam_runs;
+    if ((int)blockIdx.x < lam_grid) {
+        const int per = (a.tokens + a.lam_runs - 1) / a.lam_runs, t0 = blockIdx.x / a.lam_blocks * per, t1 = min(a.tokens, t0 + per);
+        const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, 1, a.H * a.L, a.mode};
+        const int block = blockIdx.x % a.lam_blocks;
+        if (a.lam8) lambda_part_fwd<8>(c, a.lam, t0, t1, block, a.lam_blocks);
+        else lambda_part_fwd<1>(c, a.lam, t0, t1, block, a.lam_blocks);
+        return;
     }
-    for (int j = lane; j < L; j += LPR) {
-        const float lp = Lp[h * L + j], d = __bfloat162float(dl[row * L + j]);
-        float r;
-        if (MODE == 0) r = softplus_f(lp * d);
-        else if (MODE == 1) r = __expf(-__expf(lp) * softplus_f(d));
-        else r = lp * d;
-        lam[row * L + j] = __float2bfloat16(r);
+    const int at = blockIdx.x - lam_grid;
+    const int t0 = at / a.row_blocks * a.run, t1 = min(a.tokens, t0 + a.run);
+    const int lane = threadIdx.x % LPR;
+    const int h = at % a.row_blocks * (256 / LPR) + threadIdx.x / LPR;
+    if (h >= a.H) return;                      // whole groups
+    const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u) << (threadIdx.x & 31 & ~(LPR - 1));
+    const bool act = lane * 8 < a.P;
+    const float bias = a.dt_bias ? a.dt_bias[h] : 0.f, A = a.A[h];
+    const long xs = (long)a.H * a.P, off = (long)h * a.P + lane * 8;
+    float dtl = 0.f;
+    for (int t = t0; t < t1; t += U) {
+        Packed<8> c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) c[u].load_if(a.x + (t + u) * xs + off, true, act && t + u < t1);
+        if ((t - t0) % LPR == 0 && t + lane < t1) {
+            dtl = softplus_row(__bfloat162float(a.dt_raw[(long)(t + lane) * a.H + h]) + bias);
+            a.g[(long)(t + lane) * a.H + h] = A * dtl;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (t + u >= t1) break;
+            const float dt = __shfl_sync(group, dtl, (t - t0 + u) % LPR, LPR);
+            float y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = c[u][i] * dt;
+            if (act) store_row<8>(a.v + (t + u) * xs + off, y, true);
+        }
     }
 }
 
-// gradients: dx = dv * dt (+ D * dy), d dt_raw = (sum_p dv x + A dg) sigmoid(dt_raw + bias), d dl, and the
-// parameter sums dA, d dt_bias, dD (H) and dL (H,L) through shared-memory partials and one global atomic
-// per CTA and entry.
-template <int LPR, int MODE>
-__global__ void __launch_bounds__(256) m2_prep_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dt_raw,
-                                                          const float* __restrict__ dt_bias, const float* __restrict__ A,
-                                                          const __nv_bfloat16* __restrict__ dl, const float* __restrict__ Lp,
-                                                          const float* __restrict__ D, const __nv_bfloat16* __restrict__ dv,
-                                                          const float* __restrict__ dg, const float* __restrict__ dlam,
-                                                          const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx,
-                                                          __nv_bfloat16* __restrict__ ddt, __nv_bfloat16* __restrict__ ddl,
-                                                          float* __restrict__ dA, float* __restrict__ dbias, float* __restrict__ dLp,
-                                                          float* __restrict__ dD, long rows, int H, int P, int L) {
-    extern __shared__ float sacc[];            // [H] dA | [H] dbias | [H] dD | [H*L] dL
-    float* sA = sacc;
-    float* sB = sA + H;
-    float* sD = sB + H;
-    float* sL = sD + H;
-    for (int i = threadIdx.x; i < 3 * H + H * L; i += blockDim.x) sacc[i] = 0.f;
-    __syncthreads();
+// gradients: dx = dv * dt (+ D * dy), d dt_raw = (sum_p dv x + A dg) sigmoid(dt_raw + bias), d dl, and the parameter sums dA,
+// d dt_bias, dD (H) and dL (H,L): one global atomic per thread and entry at the end of the run.
+template <int LPR>
+__global__ void __launch_bounds__(256, 4) m2_prep_bwd_kernel(const __grid_constant__ PrepArgs a) {
+    const int lam_grid = a.lam_blocks * a.lam_runs;
+    if ((int)blockIdx.x < lam_grid) {
+        const int per = (a.tokens + a.lam_runs - 1) / a.lam_runs, t0 = blockIdx.x / a.lam_blocks * per, t1 = min(a.tokens, t0 + per);
+        const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, 1, a.H * a.L, a.mode};
+        __shared__ float sums[256 * 8];
+        const int block = blockIdx.x % a.lam_blocks;
+        if (a.lam8) lambda_part_bwd<8>(c, a.dlam, a.ddl, c.dl_stride, a.dLp, t0, t1, block, a.lam_blocks, sums);
+        else lambda_part_bwd<1>(c, a.dlam, a.ddl, c.dl_stride, a.dLp, t0, t1, block, a.lam_blocks, sums);
+        return;
+    }
+    const int at = blockIdx.x - lam_grid;
+    const int t0 = at / a.row_blocks * a.run, t1 = min(a.tokens, t0 + a.run);
     const int lane = threadIdx.x % LPR;
-    const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
-    const bool act = row < rows;
-    const int h = act ? (int)(row % H) : 0;
-    float t = 0.f, dt = 0.f, dot = 0.f, dsum = 0.f;
-    if (act) {
-        t = __bfloat162float(dt_raw[row]);
-        if (dt_bias) t += dt_bias[h];
-        dt = softplus_f(t);
-        if (lane * 8 < P) {
-            const uint4 rx = *reinterpret_cast<const uint4*>(x + row * P + lane * 8);
-            const uint4 rv = *reinterpret_cast<const uint4*>(dv + row * P + lane * 8);
-            uint4 ry = make_uint4(0, 0, 0, 0);
-            const float dcoef = D ? D[h] : 0.f;
-            if (D) ry = *reinterpret_cast<const uint4*>(dy + row * P + lane * 8);
-            const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&rx);
-            const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&rv);
-            const __nv_bfloat162* hy = reinterpret_cast<const __nv_bfloat162*>(&ry);
-            uint4 out;
-            __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&out);
+    const int h = at % a.row_blocks * (256 / LPR) + threadIdx.x / LPR;
+    if (h >= a.H) return;
+    const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u) << (threadIdx.x & 31 & ~(LPR - 1));
+    const bool act = lane * 8 < a.P;
+    const float bias = a.dt_bias ? a.dt_bias[h] : 0.f, A = a.A[h], D = a.D ? a.D[h] : 0.f;
+    const long xs = (long)a.H * a.P, off = (long)h * a.P + lane * 8;
+    float raw = 0.f, dtl = 0.f, dotl = 0.f, sA = 0.f, sB = 0.f, sD = 0.f;
+    for (int t = t0; t < t1; ++t) {
+        Packed<8> cx, cv, cy;
+        cx.load_if(a.x + t * xs + off, true, act);
+        cv.load_if(a.dv + t * xs + off, true, act);
+        cy.load_if(a.dy + t * xs + off, true, act && a.D != nullptr);
+        const int k = (t - t0) % LPR;
+        if (k == 0 && t + lane < t1) {
+            raw = __bfloat162float(a.dt_raw[(long)(t + lane) * a.H + h]) + bias;
+            dtl = softplus_row(raw);
+        }
+        const float dt = __shfl_sync(group, dtl, k, LPR);
+        float y[8], dot = 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float x0 = __bfloat162float(hx[i].x), x1 = __bfloat162float(hx[i].y);
-                const float v0 = __bfloat162float(hv[i].x), v1 = __bfloat162float(hv[i].y);
-                const float y0 = __bfloat162float(hy[i].x), y1 = __bfloat162float(hy[i].y);
-                dot += v0 * x0 + v1 * x1;
-                dsum += y0 * x0 + y1 * x1;
-                o[i] = __floats2bfloat162_rn(v0 * dt + dcoef * y0, v1 * dt + dcoef * y1);
+        for (int i = 0; i < 8; ++i) {
+            const float dv = cv[i], dy = cy[i], xv = cx[i];
+            dot += dv * xv;
+            sD += dy * xv;
+            y[i] = dv * dt + D * dy;
+        }
+        if (act) store_row<8>(a.dx + t * xs + off, y, true);
+#pragma unroll
+        for (int d = LPR / 2; d > 0; d >>= 1) dot += __shfl_xor_sync(group, dot, d);
+        if (k == lane) dotl = dot;
+        if (k == LPR - 1 || t + 1 == t1) {
+            // a block of LPR tokens (or the rest of the run) is complete: one token a lane
+            const int tt = t - k + lane;
+            if (lane <= k) {
+                const float dgv = a.dg[(long)tt * a.H + h];
+                const float d_raw = (dotl + A * dgv) * (raw > 20.f ? 1.f : sigmoid_row(raw));
+                a.ddt[(long)tt * a.H + h] = __float2bfloat16(d_raw);
+                sA += dgv * dtl;
+                sB += d_raw;
             }
-            *reinterpret_cast<uint4*>(dx + row * P + lane * 8) = out;
         }
     }
 #pragma unroll
     for (int d = LPR / 2; d > 0; d >>= 1) {
-        dot += __shfl_xor_sync(0xffffffffu, dot, d);
-        dsum += __shfl_xor_sync(0xffffffffu, dsum, d);
+        sA += __shfl_xor_sync(group, sA, d);
+        sB += __shfl_xor_sync(group, sB, d);
+        sD += __shfl_xor_sync(group, sD, d);
     }
-    if (act) {
-        if (lane == 0) {
-            const float dgv = dg[row];
-            const float d_dt = dot + A[h] * dgv;
-            const float d_raw = d_dt * (t > 20.f ? 1.f : sigmoid_f(t));
-            ddt[row] = __float2bfloat16(d_raw);
-            atomicAdd(&sA[h], dgv * dt);
-            atomicAdd(&sB[h], d_raw);
-            if (D) atomicAdd(&sD[h], dsum);
-        }
-        for (int j = lane; j < L; j += LPR) {
-            const float lp = Lp[h * L + j], d = __bfloat162float(dl[row * L + j]);
-            const float gl = dlam[row * L + j];
-            float g_dl, g_lp;
-            if (MODE == 0) {
-                const float a = lp * d;
-                const float s = a > 20.f ? 1.f : sigmoid_f(a);
-                g_dl = gl * s * lp;
-                g_lp = gl * s * d;
-            } else if (MODE == 1) {
-                const float el = __expf(lp), sp = softplus_f(d);
-                const float r = __expf(-el * sp);
-                g_dl = -gl * r * el * (d > 20.f ? 1.f : sigmoid_f(d));
-                g_lp = -gl * r * el * sp;
-            } else {
-                g_dl = gl * lp;
-                g_lp = gl * d;
-            }
-            ddl[row * L + j] = __float2bfloat16(g_dl);
-            atomicAdd(&sL[h * L + j], g_lp);
-        }
+    if (lane == 0) {
+        atomicAdd(&a.dA[h], sA);
+        if (a.dbias) atomicAdd(&a.dbias[h], sB);
+        if (a.D) atomicAdd(&a.dD[h], sD);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < H; i += blockDim.x) {
-        atomicAdd(&dA[i], sA[i]);
-        if (dbias) atomicAdd(&dbias[i], sB[i]);
-        if (D) atomicAdd(&dD[i], sD[i]);
-    }
-    for (int i = threadIdx.x; i < H * L; i += blockDim.x) atomicAdd(&dLp[i], sL[i]);
 }
 
 template <int LPR, bool F32OUT>
@@ -195,12 +191,21 @@ static int prep_check(long rows, int H, int P, int L, int mode) {
     return 0;
 }
 
-#define LLATTN_PREP_DISPATCH(KERN, LPRV, MODEV, ...)                                              \
-    do {                                                                                          \
-        if (MODEV == 0) KERN<LPRV, 0> __VA_ARGS__;                                                \
-        else if (MODEV == 1) KERN<LPRV, 1> __VA_ARGS__;                                           \
-        else KERN<LPRV, 2> __VA_ARGS__;                                                           \
-    } while (0)
+// Grid of a pass: runs long enough that the sums at their end are cheap, as many as fill the chip
+static unsigned prep_grid(llattn::PrepArgs& a, long rows, int H, int P, int L, int mode, bool backward) {
+    a.H = H; a.P = P; a.L = L; a.mode = mode;
+    a.tokens = (int)(rows / H);
+    a.lpr = llattn::lanes_per_row(P);
+    a.row_blocks = (H * a.lpr + 255) / 256;
+    a.lam8 = H * L % 8 == 0;
+    a.lam_blocks = (H * L / (a.lam8 ? 8 : 1) + 255) / 256;
+    a.run = 64;
+    while (a.run > 8 && (long)a.row_blocks * ((a.tokens + a.run - 1) / a.run) < 148 * 8) a.run /= 2;
+    // forward: eight tokens a thread
+    const int groups = H * L / (a.lam8 ? 8 : 1), per = groups < 256 ? 256 / groups : 1;
+    a.lam_runs = backward ? llattn::lambda_runs(a.tokens, a.lam_blocks) : (a.tokens + 8 * per - 1) / (8 * per);
+    return (unsigned)(a.row_blocks * ((a.tokens + a.run - 1) / a.run) + a.lam_blocks * a.lam_runs);
+}
 
 int llattn_mamba2_prep_fwd(const void* x, const void* dt_raw, const float* dt_bias, const float* A, const void* dl, const float* Lp,
                            void* v, float* g, void* lambda, long rows, int H, int P, int L, int lambda_mode, void* stream) {
@@ -209,14 +214,14 @@ int llattn_mamba2_prep_fwd(const void* x, const void* dt_raw, const float* dt_bi
     if (!x || !dt_raw || !A || !dl || !Lp || !v || !g || !lambda) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
     cudaStream_t st = (cudaStream_t)stream;
-    const int lpr = llattn::lanes_per_row(P);
-    const unsigned blocks = (unsigned)((rows * lpr + 255) / 256);
-#define ARGS_F <<<blocks, 256, 0, st>>>((const bf*)x, (const bf*)dt_raw, dt_bias, A, (const bf*)dl, Lp, (bf*)v, g, (bf*)lambda, rows, H, P, L)
-    if (lpr == 4) LLATTN_PREP_DISPATCH(llattn::m2_prep_fwd_kernel, 4, lambda_mode, ARGS_F);
-    else if (lpr == 8) LLATTN_PREP_DISPATCH(llattn::m2_prep_fwd_kernel, 8, lambda_mode, ARGS_F);
-    else if (lpr == 16) LLATTN_PREP_DISPATCH(llattn::m2_prep_fwd_kernel, 16, lambda_mode, ARGS_F);
-    else LLATTN_PREP_DISPATCH(llattn::m2_prep_fwd_kernel, 32, lambda_mode, ARGS_F);
-#undef ARGS_F
+    llattn::PrepArgs a = {};
+    a.x = (const bf*)x; a.dt_raw = (const bf*)dt_raw; a.dl = (const bf*)dl; a.dt_bias = dt_bias; a.A = A; a.Lp = Lp;
+    a.v = (bf*)v; a.lam = (bf*)lambda; a.g = g;
+    const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, false);
+    if (a.lpr == 4) llattn::m2_prep_fwd_kernel<4><<<grid, 256, 0, st>>>(a);
+    else if (a.lpr == 8) llattn::m2_prep_fwd_kernel<8><<<grid, 256, 0, st>>>(a);
+    else if (a.lpr == 16) llattn::m2_prep_fwd_kernel<16><<<grid, 256, 0, st>>>(a);
+    else llattn::m2_prep_fwd_kernel<32><<<grid, 256, 0, st>>>(a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -232,17 +237,15 @@ int llattn_mamba2_prep_bwd(const void* x, const void* dt_raw, const float* dt_bi
     if (dt_bias && !dbias) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
     cudaStream_t st = (cudaStream_t)stream;
-    const int lpr = llattn::lanes_per_row(P);
-    const unsigned blocks = (unsigned)((rows * lpr + 255) / 256);
-    const size_t sm = (size_t)(3 * H + H * L) * sizeof(float);
-    if (sm > 48 * 1024) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-#define ARGS_B <<<blocks, 256, sm, st>>>((const bf*)x, (const bf*)dt_raw, dt_bias, A, (const bf*)dl, Lp, D, (const bf*)dv, dg, dlambda, \
-                                         (const bf*)dy, (bf*)dx, (bf*)ddt, (bf*)ddl, dA, dt_bias ? dbias : nullptr, dLp, dD, rows, H, P, L)
-    if (lpr == 4) LLATTN_PREP_DISPATCH(llattn::m2_prep_bwd_kernel, 4, lambda_mode, ARGS_B);
-    else if (lpr == 8) LLATTN_PREP_DISPATCH(llattn::m2_prep_bwd_kernel, 8, lambda_mode, ARGS_B);
-    else if (lpr == 16) LLATTN_PREP_DISPATCH(llattn::m2_prep_bwd_kernel, 16, lambda_mode, ARGS_B);
-    else LLATTN_PREP_DISPATCH(llattn::m2_prep_bwd_kernel, 32, lambda_mode, ARGS_B);
-#undef ARGS_B
+    llattn::PrepArgs a = {};
+    a.x = (const bf*)x; a.dt_raw = (const bf*)dt_raw; a.dl = (const bf*)dl; a.dt_bias = dt_bias; a.A = A; a.Lp = Lp; a.D = D;
+    a.dv = (const bf*)dv; a.dg = dg; a.dlam = dlambda; a.dy = (const bf*)dy;
+    a.dx = (bf*)dx; a.ddt = (bf*)ddt; a.ddl = (bf*)ddl; a.dA = dA; a.dbias = dt_bias ? dbias : nullptr; a.dLp = dLp; a.dD = dD;
+    const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, true);
+    if (a.lpr == 4) llattn::m2_prep_bwd_kernel<4><<<grid, 256, 0, st>>>(a);
+    else if (a.lpr == 8) llattn::m2_prep_bwd_kernel<8><<<grid, 256, 0, st>>>(a);
+    else if (a.lpr == 16) llattn::m2_prep_bwd_kernel<16><<<grid, 256, 0, st>>>(a);
+    else llattn::m2_prep_bwd_kernel<32><<<grid, 256, 0, st>>>(a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

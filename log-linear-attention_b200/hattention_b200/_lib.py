@@ -80,6 +80,10 @@ def lib():
         "llattn_gdn_prompt_prep": [_P] * 12 + [_I] * 11 + [_F, _F, _P],
         "llattn_gdn_prefill_slice": [_P] * 11 + [_I] * 4 + [_P, ctypes.c_size_t] + [_I] * 6 + [_P],
         "llattn_gdn_prompt_states": [_P] * 5 + [_I] * 9 + [_P],
+        "llattn_mixer_prep_fwd": [_P] * 2 + [_I, _P, _I, _P, _I] + [_P] * 2 + [_I] + [_P] * 6 + [_I] * 7 + [_P],
+        "llattn_mixer_prep_bwd": [_P] * 2 + [_I, _P, _I, _P, _I] + [_P] * 2 + [_I, _P, _I] + [_P] * 12 + [_I] * 7 + [_P],
+        "llattn_mixer_norm_fwd": [_P] * 3 + [_I, _P, _I, _P, _I] + [_P] * 2 + [ctypes.c_long, _I, _F, _P],
+        "llattn_mixer_norm_bwd": [_P] * 3 + [_I, _P, _I, _P, _I] + [_P] * 6 + [ctypes.c_long, _I, _P],
     }.items():
         fn = getattr(L, name)
         fn.restype, fn.argtypes = _I, args

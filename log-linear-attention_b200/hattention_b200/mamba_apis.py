@@ -374,6 +374,83 @@ def hselective_state_update(
     return out, state
 
 
+class HMambaMixerFunction(torch.autograd.Function):
+    """Everything of the mixer between its two projections as one autograd node: convolution, preparation, chunkwise kernels, D
+    residual and gated norm, on the rows of the input projection in place (mamba_apis.py:186-259 in the reference)."""
+
+    @staticmethod
+    def forward(ctx, zx, conv_w, conv_b, dt_bias, A, Lp, D, norm_w, eps, G, mode, level_base, htype):
+        lib = _lib.lib()
+        Bsz, T, W = zx.shape
+        H, L = Lp.shape
+        dim = H * 64
+        N = (W - 2 * dim - H - H * L) // (2 * G)
+        f32 = torch.float32
+        zx, conv_w, Lp, norm_w = (t.contiguous() for t in (zx, conv_w, Lp, norm_w))
+        conv_b, dt_bias, D = (t if t is None else t.contiguous() for t in (conv_b, dt_bias, D))
+        A_ = A.detach().float().contiguous()
+        is32 = lambda t: t is not None and t.dtype == f32
+        with torch.cuda.device(zx.device):
+            stream = torch.cuda.current_stream().cuda_stream
+            bf = dict(dtype=torch.bfloat16, device=zx.device)
+            x, v = torch.empty(Bsz, T, H, 64, **bf), torch.empty(Bsz, T, H, 64, **bf)
+            k, q = torch.empty(Bsz, T, G, N, **bf), torch.empty(Bsz, T, G, N, **bf)
+            g = torch.empty(Bsz, T, H, dtype=f32, device=zx.device)
+            lam = torch.empty(Bsz, T, H, L, **bf)
+            rc = lib.llattn_mixer_prep_fwd(zx.data_ptr(), conv_w.data_ptr(), is32(conv_w), _ptr(conv_b), is32(conv_b), _ptr(dt_bias),
+                                           is32(dt_bias), A_.data_ptr(), Lp.data_ptr(), is32(Lp), x.data_ptr(), v.data_ptr(),
+                                           k.data_ptr(), q.data_ptr(), g.data_ptr(), lam.data_ptr(), Bsz, T, H, G, N, L, mode, stream)
+            _lib.check(rc, "llattn_mixer_prep_fwd")
+            kept = [] if KEEP_FORWARD_STATES else None
+            o, g_cum, _ = chunkwise_fwd(q=q, k=k, v=v, g=g, l=lam, head_first=False, level_base=level_base, htype=htype, chunk_size=64,
+                                        output_final_state=False, keep_workspace=kept)
+            out = torch.empty(Bsz, T, dim, **bf)
+            rstd = torch.empty(Bsz, T, dtype=f32, device=zx.device)
+            rc = lib.llattn_mixer_norm_fwd(o.data_ptr(), x.data_ptr(), _ptr(D), is32(D), zx.data_ptr(), W, norm_w.data_ptr(), is32(norm_w),
+                                           out.data_ptr(), rstd.data_ptr(), Bsz * T, H, eps, stream)
+            _lib.check(rc, "llattn_mixer_norm_fwd")
+        ctx.save_for_backward(zx, conv_w, conv_b, dt_bias, A_, Lp, D, norm_w, x, v, k, q, g_cum, lam, o, rstd)
+        ctx.fwd_workspace = kept[0] if kept else None
+        ctx.meta = (G, N, mode, level_base, htype, A.dtype)
+        return out
+
+    @staticmethod
+    def backward(ctx, dn):
+        zx, conv_w, conv_b, dt_bias, A_, Lp, D, norm_w, x, v, k, q, g_cum, lam, o, rstd = ctx.saved_tensors
+        G, N, mode, level_base, htype, A_dt = ctx.meta
+        lib = _lib.lib()
+        Bsz, T, W = zx.shape
+        H, L = Lp.shape
+        dim = H * 64
+        f32 = torch.float32
+        is32 = lambda t: t is not None and t.dtype == f32
+        dn = dn.to(torch.bfloat16).contiguous()
+        with torch.cuda.device(zx.device):
+            stream = torch.cuda.current_stream().cuda_stream
+            dzx = torch.empty_like(zx)
+            dy = torch.empty_like(x)
+            # sums over tokens: conv taps and bias, norm weight, A, dt_bias, D, L
+            ch = dim + 2 * G * N
+            acc = torch.zeros(ch * 5 + dim + 3 * H + H * L, dtype=f32, device=zx.device)
+            dcw, dcb, dnw, dA, dbias, dD, dLp = acc.split([ch * 4, ch, dim, H, H, H, H * L])
+            rc = lib.llattn_mixer_norm_bwd(o.data_ptr(), x.data_ptr(), _ptr(D), is32(D), zx.data_ptr(), W, norm_w.data_ptr(), is32(norm_w),
+                                           dn.data_ptr(), rstd.data_ptr(), dy.data_ptr(), dzx.data_ptr(), dnw.data_ptr(), dD.data_ptr(),
+                                           Bsz * T, H, stream)
+            _lib.check(rc, "llattn_mixer_norm_bwd")
+            dq, dk, dv, dg, dlam = chunkwise_bwd(q=q, k=k, v=v, g=g_cum, l=lam, do=dy, head_first=False, level_base=level_base,
+                                                 htype=htype, chunk_size=64, fwd_workspace=ctx.fwd_workspace)
+            ctx.fwd_workspace = None
+            rc = lib.llattn_mixer_prep_bwd(zx.data_ptr(), conv_w.data_ptr(), is32(conv_w), _ptr(conv_b), is32(conv_b), _ptr(dt_bias),
+                                           is32(dt_bias), A_.data_ptr(), Lp.data_ptr(), is32(Lp), _ptr(D), is32(D), dv.data_ptr(),
+                                           dy.data_ptr(), dq.data_ptr(), dk.data_ptr(), dg.data_ptr(), dlam.data_ptr(), dzx.data_ptr(),
+                                           dcw.data_ptr(), dcb.data_ptr(), dA.data_ptr(), dbias.data_ptr(), dLp.data_ptr(),
+                                           Bsz, T, H, G, N, L, mode, stream)
+            _lib.check(rc, "llattn_mixer_prep_bwd")
+        as_ = lambda d, p: None if p is None else d.view(p.shape).to(p.dtype)
+        return (dzx, as_(dcw, conv_w), as_(dcb, conv_b), as_(dbias, dt_bias), dA.to(A_dt), as_(dLp, Lp), as_(dD, D), as_(dnw, norm_w),
+                None, None, None, None, None)
+
+
 def _causal_conv1d_silu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> torch.Tensor:
     """Depthwise causal convolution followed by SiLU on (B, D, T): what causal_conv1d_fn(..., activation="silu")
     computes (call site mamba_apis.py:213-220 in the reference).  Outside the log-linear attention path:
@@ -452,6 +529,14 @@ def hmamba_split_conv1d_scan_combined(
         raise ValueError
     if dt_bias.shape != (nheads,) or A.shape != (nheads,) or L.shape != (nheads, dlambda):
         raise ValueError
+    params = (conv1d_weight, conv1d_bias, dt_bias, L, D, rmsnorm_weight)
+    if (FUSED_PREP and zxbcdtdl.is_cuda and zxbcdtdl.dtype == torch.bfloat16 and all(p is None or p.dtype in _PARAM_DTYPES for p in params)
+            and headdim == 64 and dstate in (64, 128) and nheads <= 128 and conv1d_weight.shape == (dim + 2 * ngroups * dstate, 4)
+            and rmsnorm_weight.shape == (dim,) and lambda_hstruct == HStruct.MAMBA2 and lambda_htype == HType.WEAK
+            and lambda_level_base == 2 and lambda_mode in _LAMBDA_MODES and lambda_level_fixed and lambda_level_max == dlambda):
+        y = HMambaMixerFunction.apply(zxbcdtdl, conv1d_weight, conv1d_bias, dt_bias, A, L, D, rmsnorm_weight, rmsnorm_eps, ngroups,
+                                      _LAMBDA_MODES[lambda_mode], lambda_level_base, lambda_htype)
+        return torch.nn.functional.linear(y, outproj_weight.to(y.dtype), outproj_bias.to(y.dtype) if outproj_bias is not None else None)
     z, xBC, dt, dl = torch.split(zxbcdtdl, [dim, dim + 2 * ngroups * dstate, nheads, nheads * dlambda], dim=-1)
     xBC = _causal_conv1d_silu(xBC.transpose(1, 2), conv1d_weight, conv1d_bias).transpose(1, 2)
     x, Bm, Cm = torch.split(xBC, [dim, ngroups * dstate, ngroups * dstate], dim=-1)
