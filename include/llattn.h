@@ -129,6 +129,14 @@ int llattn_mamba2_prep_bwd(const void* x, const void* dt_raw, const float* dt_bi
                            const float* D, const void* dv, const float* dg, const float* dlambda, const void* dy,
                            void* dx, void* ddt, void* ddl, float* dA, float* dbias, float* dLp, float* dD,
                            long rows, int H, int P, int L, int lambda_mode, void* stream);
+/* The same passes for parameters in the dtype the model keeps them in: dt_bias, Lp, D fp32 or bf16 by their flags. */
+int llattn_mamba2_layer_prep_fwd(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
+                                 const void* Lp, int lp_is_f32, void* v, float* g, void* lambda, long rows, int H, int P, int L,
+                                 int lambda_mode, void* stream);
+int llattn_mamba2_layer_prep_bwd(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
+                                 const void* Lp, int lp_is_f32, const void* D, int d_is_f32, const void* dv, const float* dg,
+                                 const float* dlambda, const void* dy, void* dx, void* ddt, void* ddl, float* dA, float* dbias,
+                                 float* dLp, float* dD, long rows, int H, int P, int L, int lambda_mode, void* stream);
 int llattn_mamba2_residual(const void* o, const void* x, const float* D, void* y, int y_is_f32, long rows, int H, int P, void* stream);
 
 /* What the mixer does around the scan, in place on the rows of its projection zxbcdtdl (B,T,W), W = 2 H 64 + 2 G N + H + H L:
@@ -331,6 +339,12 @@ int llattn_gdn_bwd_kept_bf16dv(const void* q, const void* k, const void* v, cons
  * Constraints: D % 8 == 0, D <= 256. */
 int llattn_l2norm_fwd(const void* x, void* y, long rows, int D, float scale, void* stream);
 int llattn_l2norm_bwd(const void* x, const float* dy, void* dx, long rows, int D, float scale, void* stream);
+
+/* The gradients that leave a Gated DeltaNet backward, in one pass: gq, gk (rows,K) bf16 = l2norm backward of dq, dk (rows,K_in) fp32 at raw
+ * q, k (q with `scale`; K_in >= K, at most 128: padded keys), gbeta (rows) and glambda (rows,L) bf16; lambda_mul != 0: glambda is
+ * rounded, multiplied and rounded again, as the reference's lambda / scale differentiates (gated_delta_rule_apis.py:65-70). */
+int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const float* dk, const float* dbeta, const float* dlambda, void* gq,
+                        void* gk, void* gbeta, void* glambda, long rows, int K, int K_in, int L, float scale, float lambda_mul, void* stream);
 
 /* Diagnostic: one 128 x N x kred bf16 tensor-core product (tcgen05.mma, accumulator in tensor
  * memory) per operand-layout combination used by the kernels: mode 0: D = A B^T with A [128][kred],

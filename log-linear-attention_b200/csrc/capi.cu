@@ -55,24 +55,25 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
     const size_t KV = (size_t)p.K * p.V, BH = (size_t)p.B * p.H;
     Carver c(ws);
     p.err = c.take<int>(64);      // status word first (256 bytes)
-    if (p.NS > 1) {
-        p.seg_F = c.take<float>(BH * p.NS * KV);
-        p.seg_D = c.take<float>(BH * p.NS);
-        p.seg_H0 = c.take<__nv_bfloat16>(BH * p.NS * p.LH * KV);
-        p.o_hi = c.take<__nv_bfloat16>((size_t)p.B * p.T * p.H * p.V);
-    }
     if (backward) {
-        p.g = c.take<float>((size_t)p.B * p.T * p.H);
+        // what a call clears: from the status word up to Zc
         p.dq_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
         p.dk_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
         p.wq = c.take<float>((size_t)p.B * p.T * p.H);
         p.Yseg = c.take<float>(BH * p.NS * (p.LH > 0 ? p.LH : 1));
         p.Zc = c.take<float>(BH * p.NT * p.LZ);
         p.Yc = c.take<float>(BH * p.NT * (llattn::M2_MLOW + 1));
-        if (p.NS > 1) {
-            p.seg_dF = c.take<float>(BH * p.NS * p.LH * KV);
-            p.seg_dHf = c.take<float>(BH * p.NS * KV);
-        }
+        p.g = c.take<float>((size_t)p.B * p.T * p.H);
+    }
+    if (p.NS > 1) {
+        p.seg_F = c.take<float>(BH * p.NS * KV);
+        p.seg_D = c.take<float>(BH * p.NS);
+        p.seg_H0 = c.take<__nv_bfloat16>(BH * p.NS * p.LH * KV);
+        p.o_hi = c.take<__nv_bfloat16>((size_t)p.B * p.T * p.H * p.V);
+    }
+    if (backward && p.NS > 1) {
+        p.seg_dF = c.take<float>(BH * p.NS * p.LH * KV);
+        p.seg_dHf = c.take<float>(BH * p.NS * KV);
     }
     return c.off;
 }
@@ -230,17 +231,19 @@ int llattn_mamba2_bwd_saved(const void* q, const void* k, const void* v, const f
     p.l = (const __nv_bfloat16*)lambda; p.d_o = (const __nv_bfloat16*)d_o;
     p.dv = (__nv_bfloat16*)dv; p.dl = dlambda;
     const size_t nqk = (size_t)B * T * G * K, nbth = (size_t)B * T * H;
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(p.err, 0, sizeof(int), st)) != cudaSuccess) return (int)e;
-    // dq_acc, dk_acc, wq and Yseg are adjacent in the workspace: one clear covers the four
-    if ((e = cudaMemsetAsync(p.dq_acc, 0, (size_t)((unsigned char*)p.Zc - (unsigned char*)p.dq_acc), st)) != cudaSuccess) return (int)e;
-    if ((e = cudaMemsetAsync(dlambda, 0, nbth * L * sizeof(float), st)) != cudaSuccess) return (int)e;
-    llattn::mamba2_uncumsum(g_cum, const_cast<float*>(p.g), (long)B * T, H, st);
+    if ((rc = llattn::mamba2_bwd_init(g_cum, const_cast<float*>(p.g), (long)B * T, H, p.err, (size_t)((unsigned char*)p.Zc - (unsigned char*)p.err),
+                                      dlambda, (long)(nbth * L), st)) != 0)
+        return rc;
     rc = llattn::mamba2_bwd_dispatch(p, st);
     if (rc != 0) return rc;
     if ((rc = llattn::mamba2_dg(p, dg, st)) != 0) return rc;
-    llattn::cast_f32_to_bf16(p.dq_acc, dq, (long)nqk, st);
-    llattn::cast_f32_to_bf16(p.dk_acc, dk, (long)nqk, st);
+    // the accumulators are adjacent (their size is a multiple of 256 bytes); one pass where the results are too
+    if ((unsigned char*)dk == (unsigned char*)dq + nqk * 2) {
+        llattn::cast_f32_to_bf16(p.dq_acc, dq, (long)(2 * nqk), st);
+    } else {
+        llattn::cast_f32_to_bf16(p.dq_acc, dq, (long)nqk, st);
+        llattn::cast_f32_to_bf16(p.dk_acc, dk, (long)nqk, st);
+    }
     return (int)cudaGetLastError();
 }
 

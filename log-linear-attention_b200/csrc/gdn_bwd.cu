@@ -484,7 +484,7 @@ int gdn_bwd_scan_dispatch(const GdnParams& p, cudaStream_t stream) {
     auto kern = gdn_scan_bwd_kernel<128>;
     const size_t sm = ScanBwdSmem<128>::total;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+    if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
     kern<<<p.B * p.H * (p.V / GDN_VS), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -494,7 +494,7 @@ static int launch_levels(const GdnParams& p, cudaStream_t stream) {
     auto kern = gdn_bwd_levels_kernel<KD, VD>;
     const size_t sm = LevSmem<KD, VD>::total;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+    if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
     kern<<<p.B * p.NT * p.H, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

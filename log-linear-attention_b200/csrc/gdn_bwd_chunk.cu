@@ -629,7 +629,7 @@ static int launch_chunk(const GdnParams& p, cudaStream_t stream) {
     auto kern = gdn_bwd_chunk_kernel<KD, VD, FUSED>;
     const size_t sm = ChunkBwdSmem<KD, VD>::total;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+    if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
     kern<<<p.B * p.NT * p.H, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

@@ -616,11 +616,11 @@ int gdn_bwd_levels_tc_dispatch(const GdnParams& p0, cudaStream_t stream) {
     int dev = 0, sms = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+    if ((e = sm_count(&sms, dev)) != cudaSuccess) return (int)e;
     const int nitems = p.B * p.NT * p.H;
     const int grid = nitems < sms ? nitems : sms;
     auto kern = gdn_bwd_levels_tc_kernel;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LevTcSmem::total)) != cudaSuccess) return (int)e;
+    if ((e = allow_smem(kern, LevTcSmem::total)) != cudaSuccess) return (int)e;
     kern<<<grid, glt::NTHREADS, LevTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

@@ -666,14 +666,14 @@ static int launch_gdn_fwd(const GdnParams& p, cudaStream_t stream) {
     } else {
         auto kern = gdn_chunk_prep_kernel<KD, VD, BWD>;
         const size_t sm = PrepSmem<KD, VD>::total;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+        if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
         kern<<<p.B * p.NT * p.H, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
     }
     if (KD == 128 && g_use_tensor_core_path.load()) return gdn_scan_tc_dispatch(p, BWD ? 2 : (KEEP ? 1 : 0), stream);
     {
         auto kern = gdn_scan_kernel<KD, BWD || KEEP, !BWD>;
         const size_t sm = ScanSmem<KD>::total;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+        if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
         kern<<<p.B * p.H * (p.V / GDN_VS), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();

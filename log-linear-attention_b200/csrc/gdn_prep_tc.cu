@@ -624,11 +624,11 @@ static int launch_prep_tc(GdnParams& p, cudaStream_t stream) {
     int dev = 0, sms = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+    if ((e = sm_count(&sms, dev)) != cudaSuccess) return (int)e;
     const int nitems = p.B * p.NT * p.H;
     const int grid = nitems < sms ? nitems : sms;
     auto kern = gdn_chunk_prep_tc_kernel<VD>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PrepTcSmem::total)) != cudaSuccess) return (int)e;
+    if ((e = allow_smem(kern, PrepTcSmem::total)) != cudaSuccess) return (int)e;
     kern<<<grid, gpt::NTHREADS, PrepTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

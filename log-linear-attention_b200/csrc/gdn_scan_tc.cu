@@ -701,7 +701,7 @@ static int launch_scan_tc(GdnParams& p, cudaStream_t stream) {
     if (rc != 0) return rc;
     auto kern = gdn_scan_tc_kernel<SAVE, OUT>;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ScanTcSmem::total)) != cudaSuccess) return (int)e;
+    if ((e = allow_smem(kern, ScanTcSmem::total)) != cudaSuccess) return (int)e;
     kern<<<p.B * p.H * (p.V / gtc::VS), gtc::NTHREADS, ScanTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -722,7 +722,7 @@ int gdn_scan_bwd_tc_dispatch(const GdnParams& p0, cudaStream_t stream) {
     if (rc != 0) return rc;
     auto kern = gdn_scan_bwd_tc_kernel;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ScanBwdTcSmem::total)) != cudaSuccess) return (int)e;
+    if ((e = allow_smem(kern, ScanBwdTcSmem::total)) != cudaSuccess) return (int)e;
     kern<<<p.B * p.H * (p.V / gtc::VS), gtc::NTHREADS, ScanBwdTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

@@ -1,0 +1,709 @@
+// Native host side of the Python package: one call into this module does what a public call needs between its argument checks and its
+// kernels - output and scratch allocation, the C-ABI calls, the autograd nodes.
+//
+// It exists because small calls are bound by the host.  The same work in Python (an autograd.Function, ctypes calls of 20 arguments,
+// context managers) took 100 us for a forward, 250 us for a backward and 15 us for a decode step on the box the kernels are timed on,
+// several times the kernels of a short sequence.
+//
+// Every entry returns None when the operands are not the ones it takes (dtypes, devices, shapes); the Python caller then goes its
+// general way, which also raises the errors.  The kernels are reached through the C ABI of libllattn.so (include/llattn.h), which is
+// loaded from the path that the Python binding uses.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include "../../include/llattn.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Variable;
+using torch::autograd::variable_list;
+
+#define LLATTN_FUNCS(F)                                                                                                             \
+    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved)        \
+    F(llattn_mamba2_layer_prep_fwd) F(llattn_mamba2_layer_prep_bwd) F(llattn_mamba2_layer_step) F(llattn_gdn_layer_step)            \
+    F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mixer_prep_fwd)            \
+    F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
+    F(llattn_gdn_fwd_workspace_bytes) F(llattn_gdn_fwd_keep_workspace_bytes) F(llattn_gdn_fwd) F(llattn_gdn_fwd_keep)                \
+    F(llattn_gdn_prefill_slice) F(llattn_gdn_prompt_states) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
+    F(llattn_gdn_bwd_kept_workspace_bytes) F(llattn_gdn_bwd_kept_bf16dv) F(llattn_gdn_grad_out) F(llattn_workspace_status)
+
+struct Library {
+#define LLATTN_MEMBER(name) decltype(&::name) name = nullptr;
+    LLATTN_FUNCS(LLATTN_MEMBER)
+#undef LLATTN_MEMBER
+} lib;
+
+void bind(const std::string& path) {
+    void* so = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+    TORCH_CHECK(so, "cannot load ", path, ": ", dlerror());
+#define LLATTN_BIND(name)                                                   \
+    lib.name = reinterpret_cast<decltype(lib.name)>(dlsym(so, #name));      \
+    TORCH_CHECK(lib.name, path, " has no " #name);
+    LLATTN_FUNCS(LLATTN_BIND)
+#undef LLATTN_BIND
+}
+
+void check(int rc, const char* what) {
+    if (rc == 0) return;
+    TORCH_CHECK_VALUE(rc > 0, what, ": unsupported arguments (code ", rc, ")");
+    TORCH_CHECK(false, what, ": CUDA error ", rc);
+}
+
+// ------------------------------------------------------------------------------------------ small helpers
+inline bool is(const Tensor& t, at::ScalarType s) { return t.defined() && t.is_cuda() && t.scalar_type() == s; }
+inline bool bf16(const Tensor& t) { return is(t, at::kBFloat16); }
+inline bool f32(const Tensor& t) { return t.defined() && t.scalar_type() == at::kFloat; }
+// a parameter: fp32 or bf16 on the device, or absent
+inline bool param(const Tensor& t) { return !t.defined() || (t.is_cuda() && (t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16)); }
+inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+inline Tensor contiguous(const Tensor& t) { return t.defined() ? t.contiguous() : t; }
+using Maybe = std::optional<Tensor>;     // a tensor that may be absent: autograd functions take no undefined tensors
+inline Tensor of(const Maybe& t) { return t.has_value() ? *t : Tensor(); }
+inline Tensor empty(at::IntArrayRef size, at::ScalarType dt, const Tensor& like) {
+    return at::empty(size, at::TensorOptions().dtype(dt).device(like.device()));
+}
+inline bool wants_grad(std::initializer_list<Tensor> ts) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor& t : ts)
+        if (t.defined() && t.requires_grad()) return true;
+    return false;
+}
+inline bool same_device(std::initializer_list<Tensor> ts) {
+    const Tensor* first = nullptr;
+    for (const Tensor& t : ts) {
+        if (!t.defined()) continue;
+        if (first && t.device() != first->device()) return false;
+        first = &t;
+    }
+    return true;
+}
+inline int ceil_log2(int64_t x) {
+    int l = 0;
+    while ((int64_t(1) << l) < x) ++l;
+    return l;
+}
+inline int bit_length(int64_t x) {
+    int l = 0;
+    while (x) {
+        ++l;
+        x >>= 1;
+    }
+    return l;
+}
+void check_status(const Tensor& ws, void* stream, const char* what) {
+    int status = -1;
+    check(lib.llattn_workspace_status(ws.data_ptr(), &status, stream), "llattn_workspace_status");
+    TORCH_CHECK(status == 0, what, ": a kernel gave up on a bounded wait (status word set); the outputs are not valid");
+}
+// the current stream of t's device, which the guard makes the current one
+struct On {
+    c10::cuda::CUDAGuard guard;
+    void* stream;
+    explicit On(const Tensor& t) : guard(t.device()), stream(at::cuda::getCurrentCUDAStream(t.device().index()).stream()) {}
+};
+
+// ------------------------------------------------------------------------------------------ Mamba-2 chunkwise kernels
+bool mamba2_shape(int64_t T, int64_t H, int64_t G, int64_t N, int64_t P, int64_t L) {
+    return T > 0 && T % 64 == 0 && T <= 524288 && G > 0 && H % G == 0 && (N == 64 || N == 128) && P == 64 && L <= 32 && L >= 7 + ceil_log2(T / 64);
+}
+struct Scan {
+    Tensor o, g_cum, ws;
+};
+// contiguous operands of the checked shape
+Scan mamba2_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, void* stream, bool status) {
+    const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
+    Scan s;
+    s.o = at::empty_like(v);
+    s.g_cum = at::empty_like(g);
+    const size_t n = lib.llattn_mamba2_fwd_workspace_bytes(B, T, H, G, K, V, L);
+    s.ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
+    check(lib.llattn_mamba2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), l.data_ptr(), s.o.data_ptr(), fptr(s.g_cum), s.ws.data_ptr(),
+                                s.ws.numel(), B, T, H, G, K, V, L, stream),
+          "llattn_mamba2_fwd");
+    if (status) check_status(s.ws, stream, "llattn_mamba2_fwd");
+    return s;
+}
+struct ScanGrads {
+    Tensor dq, dk, dv, dg, dl;       // dl fp32
+};
+ScanGrads mamba2_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g_cum, const Tensor& l, const Tensor& d_o, const Tensor& fws,
+                     void* stream, bool status) {
+    const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
+    ScanGrads r;
+    const Tensor qk = empty({2, B, T, G, K}, at::kBFloat16, q);      // side by side: one conversion pass writes both
+    r.dq = qk.select(0, 0);
+    r.dk = qk.select(0, 1);
+    r.dv = at::empty_like(v);
+    r.dg = at::empty_like(g_cum);
+    r.dl = empty(l.sizes(), at::kFloat, l);
+    const size_t n = lib.llattn_mamba2_bwd_workspace_bytes(B, T, H, G, K, V, L);
+    const Tensor ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
+    check(lib.llattn_mamba2_bwd_saved(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g_cum), l.data_ptr(), d_o.data_ptr(), r.dq.data_ptr(),
+                                      r.dk.data_ptr(), r.dv.data_ptr(), fptr(r.dg), fptr(r.dl), ws.data_ptr(), ws.numel(), ptr(fws),
+                                      fws.defined() ? fws.numel() : 0, B, T, H, G, K, V, L, stream),
+          "llattn_mamba2_bwd_saved");
+    if (status) check_status(ws, stream, "llattn_mamba2_bwd_saved");
+    return r;
+}
+
+// ---- hattention_kernel, Mamba-2 structure
+struct Mamba2Kernel : torch::autograd::Function<Mamba2Kernel> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool keep,
+                          bool status) {
+        On on(q);
+        const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
+        Scan s = mamba2_fwd(q_, k_, v_, g_, l_, on.stream, status);
+        if (ctx) {
+            ctx->save_for_backward({q_, k_, v_, s.g_cum, l_, keep ? s.ws : Tensor()});
+            ctx->saved_data["status"] = status;
+        }
+        return s.o;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list d) {
+        const auto s = ctx->get_saved_variables();
+        On on(s[0]);
+        ScanGrads r = mamba2_bwd(s[0], s[1], s[2], s[3], s[4], d[0].to(at::kBFloat16).contiguous(), s[5], on.stream,
+                                 ctx->saved_data["status"].toBool());
+        return {r.dq, r.dk, r.dv, r.dg, r.dl.to(at::kBFloat16), Tensor(), Tensor()};
+    }
+};
+
+py::object hattention_mamba2(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool keep, bool status) {
+    if (!bf16(q) || !bf16(k) || !bf16(v) || !is(g, at::kFloat) || !bf16(l) || k.dim() != 4 || v.dim() != 4 || l.dim() != 4 || q.sizes() != k.sizes() ||
+        !same_device({q, k, v, g, l}))
+        return py::none();
+    const int64_t B = k.size(0), T = k.size(1), H = v.size(2), L = l.size(3);
+    if (v.size(0) != B || v.size(1) != T || g.sizes() != at::IntArrayRef({B, T, H}) || l.sizes() != at::IntArrayRef({B, T, H, L}) ||
+        !mamba2_shape(T, H, k.size(2), k.size(3), v.size(3), L))
+        return py::none();
+    py::gil_scoped_release nogil;
+    Tensor o = wants_grad({q, k, v, g, l}) ? Mamba2Kernel::apply(q, k, v, g, l, keep, status) : Mamba2Kernel::forward(nullptr, q, k, v, g, l, false, status);
+    py::gil_scoped_acquire gil;
+    return py::cast(o);
+}
+
+// ---- the layer call: preparation, chunkwise kernels, D residual
+struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm, const Tensor& dl,
+                          const Tensor& Lp, const Maybe& D, const Maybe& bias, int64_t mode, bool keep, bool status) {
+        On on(x);
+        const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), L = dl.size(3);
+        const Tensor x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), A_ = A.to(at::kFloat).contiguous(), Lp_ = Lp.contiguous(),
+                     D_ = contiguous(of(D)), b_ = contiguous(of(bias)), q = Cm.contiguous(), k = Bm.contiguous();
+        const Tensor v = at::empty_like(x_), g = empty({B, T, H}, at::kFloat, x), lam = at::empty_like(dl_);
+        check(lib.llattn_mamba2_layer_prep_fwd(x_.data_ptr(), dt_.data_ptr(), ptr(b_), f32(b_), fptr(A_), dl_.data_ptr(), Lp_.data_ptr(), f32(Lp_),
+                                               v.data_ptr(), fptr(g), lam.data_ptr(), (long)B * T * H, H, P, L, (int)mode, on.stream),
+              "llattn_mamba2_layer_prep_fwd");
+        Scan s = mamba2_fwd(q, k, v, g, lam, on.stream, status);
+        Tensor y = s.o;
+        if (D_.defined()) {
+            y = empty(x_.sizes(), f32(D_) ? at::kFloat : at::kBFloat16, x);
+            check(lib.llattn_mamba2_prompt_residual(s.o.data_ptr(), x_.data_ptr(), ptr(D_), y.data_ptr(), f32(D_), B, T, T, H, P, on.stream),
+                  "llattn_mamba2_prompt_residual");
+        }
+        if (ctx) {
+            ctx->save_for_backward({x_, dt_, A_, k, q, dl_, Lp_, D_, b_, v, s.g_cum, lam, keep ? s.ws : Tensor()});
+            ctx->saved_data["mode"] = mode;
+            ctx->saved_data["status"] = status;
+            ctx->saved_data["A"] = (int64_t)A.scalar_type();
+        }
+        return y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list d) {
+        const auto s = ctx->get_saved_variables();
+        const Tensor &x = s[0], &dt = s[1], &A = s[2], &k = s[3], &q = s[4], &dl = s[5], &Lp = s[6], &D = s[7], &bias = s[8], &v = s[9], &g_cum = s[10],
+                     &lam = s[11], &ws = s[12];
+        On on(x);
+        const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), L = dl.size(3);
+        const Tensor dy = d[0].to(at::kBFloat16).contiguous();
+        ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool());
+        const Tensor dx = at::empty_like(x), ddt = at::empty_like(dt), ddl = at::empty_like(dl);
+        const Tensor acc = at::zeros({3 * H + H * L}, at::TensorOptions().dtype(at::kFloat).device(x.device()));
+        float* a = fptr(acc);
+        check(lib.llattn_mamba2_layer_prep_bwd(x.data_ptr(), dt.data_ptr(), ptr(bias), f32(bias), fptr(A), dl.data_ptr(), Lp.data_ptr(), f32(Lp), ptr(D),
+                                               f32(D), r.dv.data_ptr(), fptr(r.dg), fptr(r.dl), dy.data_ptr(), dx.data_ptr(), ddt.data_ptr(), ddl.data_ptr(),
+                                               a, a + H, a + 3 * H, a + 2 * H, (long)B * T * H, H, P, L, (int)ctx->saved_data["mode"].toInt(), on.stream),
+              "llattn_mamba2_layer_prep_bwd");
+        // one conversion for all parameters that are kept in bf16
+        const at::ScalarType A_dt = (at::ScalarType)ctx->saved_data["A"].toInt();
+        Tensor half;
+        auto part = [&](int64_t at0, int64_t n, at::ScalarType t) {
+            if (t == at::kFloat) return acc.narrow(0, at0, n);
+            if (!half.defined()) half = acc.to(at::kBFloat16);
+            return t == at::kBFloat16 ? half.narrow(0, at0, n) : acc.narrow(0, at0, n).to(t);
+        };
+        return {dx, ddt, part(0, H, A_dt), r.dk, r.dq, ddl, part(3 * H, (int64_t)H * L, Lp.scalar_type()).view({H, L}),
+                D.defined() ? part(2 * H, H, D.scalar_type()) : Tensor(), bias.defined() ? part(H, H, bias.scalar_type()) : Tensor(), Tensor(), Tensor(),
+                Tensor()};
+    }
+};
+
+bool layer_operands(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm, const Tensor& dl, const Tensor& Lp,
+                    const Tensor& D, const Tensor& bias) {
+    if (!bf16(x) || !bf16(dt) || !bf16(Bm) || !bf16(Cm) || !bf16(dl) || !A.is_cuda() || !A.is_floating_point() || !param(Lp) || !param(D) || !param(bias) ||
+        x.dim() != 4 || Bm.dim() != 4 || dl.dim() != 4 || Lp.dim() != 2 || Cm.sizes() != Bm.sizes() || !same_device({x, dt, A, Bm, Cm, dl, Lp, D, bias}))
+        return false;
+    const int64_t B = x.size(0), T = x.size(1), H = x.size(2), L = dl.size(3);
+    return dt.sizes() == at::IntArrayRef({B, T, H}) && A.sizes() == at::IntArrayRef({H}) && Bm.size(0) == B && Bm.size(1) == T &&
+           dl.sizes() == at::IntArrayRef({B, T, H, L}) && Lp.sizes() == at::IntArrayRef({H, L}) && (!D.defined() || D.sizes() == at::IntArrayRef({H})) &&
+           (!bias.defined() || bias.sizes() == at::IntArrayRef({H})) && x.size(3) == 64 && Bm.size(2) > 0 && H % Bm.size(2) == 0 &&
+           (Bm.size(3) == 64 || Bm.size(3) == 128) && L <= 32 && B * T * H < (int64_t(1) << 28);
+}
+
+py::object mamba2_layer(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm, const Tensor& dl, const Tensor& Lp,
+                        const Maybe& D_, const Maybe& bias_, int64_t mode, bool keep, bool status) {
+    const Tensor D = of(D_), bias = of(bias_);
+    if (!layer_operands(x, dt, A, Bm, Cm, dl, Lp, D, bias) || !mamba2_shape(x.size(1), x.size(2), Bm.size(2), Bm.size(3), x.size(3), dl.size(3)))
+        return py::none();
+    py::gil_scoped_release nogil;
+    Tensor y = wants_grad({x, dt, A, Bm, Cm, dl, Lp, D, bias}) ? Mamba2Layer::apply(x, dt, A, Bm, Cm, dl, Lp, D_, bias_, mode, keep, status)
+                                                              : Mamba2Layer::forward(nullptr, x, dt, A, Bm, Cm, dl, Lp, D_, bias_, mode, false, status);
+    py::gil_scoped_acquire gil;
+    return py::cast(y);
+}
+
+// ---- a prompt of any length: outputs and level states (level-major).  (y, states) or None
+py::object mamba2_prompt(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm, const Tensor& dl, const Tensor& Lp,
+                         const Maybe& D_, const Maybe& bias_, int64_t mode, bool status) {
+    const Tensor D = of(D_), bias = of(bias_);
+    if (!layer_operands(x, dt, A, Bm, Cm, dl, Lp, D, bias) || wants_grad({x, dt, A, Bm, Cm, dl, Lp, D, bias})) return py::none();
+    const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), G = Bm.size(2), N = Bm.size(3), L = dl.size(3);
+    // an even number of chunks, which the tensor-core kernels take
+    const int Tp = T <= 64 ? 64 : (T + 127) / 128 * 128, Lo = T < 64 ? std::max(L, 7) : L;
+    if (T < 1 || L < 1 + bit_length(T - 1) || !mamba2_shape(Tp, H, G, N, P, Lo)) return py::none();
+    Tensor y, states;
+    {
+        py::gil_scoped_release nogil;
+        at::NoGradGuard no_grad;
+        On on(x);
+        const Tensor x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), A_ = A.to(at::kFloat).contiguous(), Lp_ = Lp.contiguous(),
+                     D_c = contiguous(D), b_ = contiguous(bias);
+        Tensor q = Cm.contiguous(), k = Bm.contiguous(), qp, kp;
+        const Tensor v = empty({B, Tp, H, P}, at::kBFloat16, x), g = empty({B, Tp, H}, at::kFloat, x), lam = empty({B, Tp, H, Lo}, at::kBFloat16, x);
+        if (Tp != T) {
+            qp = empty({B, Tp, G, N}, at::kBFloat16, x);
+            kp = at::empty_like(qp);
+        }
+        check(lib.llattn_mamba2_prompt_prep(x_.data_ptr(), dt_.data_ptr(), ptr(b_), f32(b_), fptr(A_), dl_.data_ptr(), Lp_.data_ptr(), f32(Lp_),
+                                            q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), ptr(qp), ptr(kp), B, T, Tp, H, G, N, P, L,
+                                            Lo, (int)mode, on.stream),
+              "llattn_mamba2_prompt_prep");
+        if (Tp != T) {
+            q = qp;
+            k = kp;
+        }
+        Scan s = mamba2_fwd(q, k, v, g, lam, on.stream, status);
+        states = empty({B, H, L, N, P}, at::kFloat, x);
+        check(lib.llattn_mamba2_prompt_states(k.data_ptr(), v.data_ptr(), fptr(g), fptr(states), s.ws.data_ptr(), s.ws.numel(), B, T, Tp, H, G, N, P, L,
+                                              on.stream),
+              "llattn_mamba2_prompt_states");
+        states = states.permute({0, 1, 3, 4, 2});
+        if (D_c.defined() || (Tp != T && B > 1)) {
+            y = empty({B, T, H, P}, D_c.defined() && f32(D_c) ? at::kFloat : at::kBFloat16, x);
+            check(lib.llattn_mamba2_prompt_residual(s.o.data_ptr(), x_.data_ptr(), ptr(D_c), y.data_ptr(), f32(y), B, T, Tp, H, P, on.stream),
+                  "llattn_mamba2_prompt_residual");
+        } else {
+            y = s.o.narrow(1, 0, T);
+        }
+    }
+    return py::make_tuple(y, states);
+}
+
+// ---- the mixer between its projections
+struct Mixer : torch::autograd::Function<Mixer> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& zx, const Tensor& cw, const Maybe& cb, const Tensor& bias, const Tensor& A, const Tensor& Lp,
+                          const Tensor& D, const Tensor& nw, double eps, int64_t G, int64_t mode, bool keep, bool status) {
+        On on(zx);
+        const int B = zx.size(0), T = zx.size(1), W = zx.size(2), H = Lp.size(0), L = Lp.size(1), dim = H * 64, N = (W - 2 * dim - H - H * L) / (2 * G);
+        const Tensor z = zx.contiguous(), cw_ = cw.contiguous(), cb_ = contiguous(of(cb)), b_ = contiguous(bias), A_ = A.to(at::kFloat).contiguous(),
+                     Lp_ = Lp.contiguous(), D_ = contiguous(D), nw_ = nw.contiguous();
+        const Tensor xv = empty({2, B, T, H, 64}, at::kBFloat16, zx), x = xv.select(0, 0), v = xv.select(0, 1);
+        const Tensor kq = empty({2, B, T, G, N}, at::kBFloat16, zx), k = kq.select(0, 0), q = kq.select(0, 1);
+        const Tensor g = empty({B, T, H}, at::kFloat, zx), lam = empty({B, T, H, L}, at::kBFloat16, zx);
+        check(lib.llattn_mixer_prep_fwd(z.data_ptr(), cw_.data_ptr(), f32(cw_), ptr(cb_), f32(cb_), ptr(b_), f32(b_), fptr(A_), Lp_.data_ptr(), f32(Lp_),
+                                        x.data_ptr(), v.data_ptr(), k.data_ptr(), q.data_ptr(), fptr(g), lam.data_ptr(), B, T, H, (int)G, N, L, (int)mode,
+                                        on.stream),
+              "llattn_mixer_prep_fwd");
+        Scan s = mamba2_fwd(q, k, v, g, lam, on.stream, status);
+        const Tensor out = empty({B, T, dim}, at::kBFloat16, zx), rstd = empty({B, T}, at::kFloat, zx);
+        check(lib.llattn_mixer_norm_fwd(s.o.data_ptr(), x.data_ptr(), ptr(D_), f32(D_), z.data_ptr(), W, nw_.data_ptr(), f32(nw_), out.data_ptr(),
+                                        fptr(rstd), (long)B * T, H, (float)eps, on.stream),
+              "llattn_mixer_norm_fwd");
+        if (ctx) {
+            ctx->save_for_backward({z, cw_, cb_, b_, A_, Lp_, D_, nw_, x, v, k, q, s.g_cum, lam, s.o, rstd, keep ? s.ws : Tensor()});
+            ctx->saved_data["mode"] = mode;
+            ctx->saved_data["status"] = status;
+            ctx->saved_data["A"] = (int64_t)A.scalar_type();
+        }
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list d) {
+        const auto s = ctx->get_saved_variables();
+        const Tensor &z = s[0], &cw = s[1], &cb = s[2], &bias = s[3], &A = s[4], &Lp = s[5], &D = s[6], &nw = s[7], &x = s[8], &v = s[9], &k = s[10],
+                     &q = s[11], &g_cum = s[12], &lam = s[13], &o = s[14], &rstd = s[15], &ws = s[16];
+        On on(z);
+        const int B = z.size(0), T = z.size(1), W = z.size(2), H = Lp.size(0), L = Lp.size(1), dim = H * 64, G = k.size(2), N = k.size(3);
+        const Tensor dn = d[0].to(at::kBFloat16).contiguous();
+        const Tensor dzx = at::empty_like(z), dy = empty(x.sizes(), at::kBFloat16, x);
+        // sums over tokens: conv taps and bias, norm weight, A, dt_bias, D, L
+        const int64_t ch = dim + 2 * G * N, at_b = ch * 4, at_n = ch * 5, at_A = at_n + dim, at_dt = at_A + H, at_D = at_dt + H, at_L = at_D + H;
+        const Tensor acc = at::zeros({at_L + (int64_t)H * L}, at::TensorOptions().dtype(at::kFloat).device(z.device()));
+        float* a = fptr(acc);
+        check(lib.llattn_mixer_norm_bwd(o.data_ptr(), x.data_ptr(), ptr(D), f32(D), z.data_ptr(), W, nw.data_ptr(), f32(nw), dn.data_ptr(), fptr(rstd),
+                                        dy.data_ptr(), dzx.data_ptr(), a + at_n, a + at_D, (long)B * T, H, on.stream),
+              "llattn_mixer_norm_bwd");
+        ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool());
+        check(lib.llattn_mixer_prep_bwd(z.data_ptr(), cw.data_ptr(), f32(cw), ptr(cb), f32(cb), ptr(bias), f32(bias), fptr(A), Lp.data_ptr(), f32(Lp), ptr(D),
+                                        f32(D), r.dv.data_ptr(), dy.data_ptr(), r.dq.data_ptr(), r.dk.data_ptr(), fptr(r.dg), fptr(r.dl), dzx.data_ptr(), a,
+                                        a + at_b, a + at_A, a + at_dt, a + at_L, B, T, H, G, N, L, (int)ctx->saved_data["mode"].toInt(), on.stream),
+              "llattn_mixer_prep_bwd");
+        const at::ScalarType A_dt = (at::ScalarType)ctx->saved_data["A"].toInt();
+        Tensor half;
+        auto part = [&](int64_t at0, at::IntArrayRef size, at::ScalarType t) {
+            int64_t n = 1;
+            for (int64_t e : size) n *= e;
+            if (t == at::kFloat) return acc.narrow(0, at0, n).view(size);
+            if (!half.defined()) half = acc.to(at::kBFloat16);
+            return t == at::kBFloat16 ? half.narrow(0, at0, n).view(size) : acc.narrow(0, at0, n).view(size).to(t);
+        };
+        auto grad = [&](const Tensor& p, int64_t at0) { return p.defined() ? part(at0, p.sizes(), p.scalar_type()) : Tensor(); };
+        return {dzx, grad(cw, 0), grad(cb, at_b), grad(bias, at_dt), part(at_A, {H}, A_dt), grad(Lp, at_L), grad(D, at_D), grad(nw, at_n), Tensor(), Tensor(),
+                Tensor(), Tensor(), Tensor()};
+    }
+};
+
+// zxbcdtdl (B,T,W) with the widths already checked -> the normed output (B,T,H 64), or None
+py::object mamba2_mixer(const Tensor& zx, const Tensor& cw, const Maybe& cb_, const Tensor& bias, const Tensor& A, const Tensor& Lp,
+                        const Tensor& D, const Tensor& nw, double eps, int64_t G, int64_t mode, bool keep, bool status) {
+    const Tensor cb = of(cb_);
+    if (!bf16(zx) || !param(cw) || !param(cb) || !param(bias) || !param(Lp) || !param(D) || !param(nw) || !A.is_cuda() || !A.is_floating_point() ||
+        zx.dim() != 3 || Lp.dim() != 2 || !same_device({zx, cw, cb, bias, A, Lp, D, nw}))
+        return py::none();
+    const int64_t T = zx.size(1), H = Lp.size(0), L = Lp.size(1), dim = H * 64, rest = zx.size(2) - 2 * dim - H - H * L;
+    if (G <= 0 || rest <= 0 || rest % (2 * G) != 0) return py::none();
+    const int64_t N = rest / (2 * G), ch = dim + 2 * G * N;
+    if (!mamba2_shape(T, H, G, N, 64, L) || H > 128 || cw.sizes() != at::IntArrayRef({ch, 4}) || (cb.defined() && cb.sizes() != at::IntArrayRef({ch})) ||
+        nw.sizes() != at::IntArrayRef({dim}) || zx.size(0) * T * H >= (int64_t(1) << 28))
+        return py::none();
+    py::gil_scoped_release nogil;
+    Tensor y = wants_grad({zx, cw, cb, bias, A, Lp, D, nw}) ? Mixer::apply(zx, cw, cb_, bias, A, Lp, D, nw, eps, G, mode, keep, status)
+                                                           : Mixer::forward(nullptr, zx, cw, cb_, bias, A, Lp, D, nw, eps, G, mode, false, status);
+    py::gil_scoped_acquire gil;
+    return py::cast(y);
+}
+
+// ------------------------------------------------------------------------------------------ Gated DeltaNet
+constexpr int GDN_K = 128, GDN_SLICE = 128, GDN_V_MAX = 384;     // key width and widest value head of one kernel call; widest head
+
+struct GdnInputs {
+    Tensor qn, kn, v, b, g, l;       // v: slices of at most 128 columns, one behind the other
+    int B, T, H, G, K, V, L;
+    int slices() const { return (V + GDN_SLICE - 1) / GDN_SLICE; }
+    int width(int i) const { return std::min(GDN_SLICE, V - i * GDN_SLICE); }
+    Tensor slice(const Tensor& all, int i) const {       // slice i of a tensor of slices
+        const int64_t n = (int64_t)B * T * H;
+        return all.view({-1}).narrow(0, n * i * GDN_SLICE, n * width(i)).view({B, T, H, width(i)});
+    }
+};
+
+// l2norm of q and k, lambda times its factor, and (T < Tp) padding; b, g and unscaled lambda are used as they are when nothing pads
+GdnInputs gdn_prepare(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, int T, int Tp, int Lo, double scale,
+                      double lam_mul, void* stream) {
+    GdnInputs a;
+    a.B = q.size(0);
+    a.T = Tp;
+    a.G = q.size(2);
+    a.K = q.size(3);
+    a.H = v.size(2);
+    a.V = v.size(3);
+    a.L = l.size(3);
+    const int B = a.B, H = a.H;
+    const bool pad = Tp != T, own_l = pad || lam_mul != 0.0 || Lo != a.L, own_v = pad || a.V > GDN_SLICE;
+    const Tensor qk = empty({2, B, Tp, H, GDN_K}, at::kBFloat16, q);
+    a.qn = qk.select(0, 0);
+    a.kn = qk.select(0, 1);
+    a.v = own_v ? empty({(int64_t)B * Tp * H * a.V}, at::kBFloat16, q) : v;
+    a.b = pad ? empty({B, Tp, H}, at::kBFloat16, q) : b;
+    a.g = pad ? empty({B, Tp, H}, at::kFloat, q) : g;
+    a.l = own_l ? empty({B, Tp, H, Lo}, at::kBFloat16, q) : l;
+    check(lib.llattn_gdn_prompt_prep(q.data_ptr(), k.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g), l.data_ptr(), a.qn.data_ptr(), a.kn.data_ptr(),
+                                     own_v ? a.v.data_ptr() : nullptr, pad ? a.b.data_ptr() : nullptr, pad ? fptr(a.g) : nullptr,
+                                     own_l ? a.l.data_ptr() : nullptr, B, T, Tp, H, a.G, a.K, GDN_K, a.V, GDN_SLICE, a.L, Lo, (float)scale, (float)lam_mul,
+                                     stream),
+          "llattn_gdn_prompt_prep");
+    a.L = Lo;
+    return a;
+}
+
+bool gdn_operands(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l) {
+    if (!bf16(q) || !bf16(k) || !bf16(v) || !bf16(b) || !is(g, at::kFloat) || !bf16(l) || q.dim() != 4 || v.dim() != 4 || l.dim() != 4 ||
+        q.sizes() != k.sizes() || !same_device({q, k, v, b, g, l}))
+        return false;
+    const int64_t B = q.size(0), T = q.size(1), G = q.size(2), K = q.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
+    return v.size(0) == B && v.size(1) == T && b.sizes() == at::IntArrayRef({B, T, H}) && g.sizes() == at::IntArrayRef({B, T, H}) &&
+           l.sizes() == at::IntArrayRef({B, T, H, L}) && T > 0 && G > 0 && H % G == 0 && K <= GDN_K && K % 8 == 0 && V > 0 && V % 64 == 0 && V <= GDN_V_MAX &&
+           L <= 32 && B * T * H < (int64_t(1) << 28);
+}
+
+struct GdnKernel : torch::autograd::Function<GdnKernel> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l,
+                          double scale, double lam_mul, int64_t keep_bytes, bool status) {
+        On on(q);
+        const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), b_ = b.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
+        const int T = q.size(1);
+        GdnInputs a = gdn_prepare(q_, k_, v_, b_, g_, l_, T, T, l.size(3), scale, lam_mul, on.stream);
+        const int B = a.B, H = a.H, n = a.slices();
+        size_t total = 0;
+        for (int i = 0; i < n; ++i) total += lib.llattn_gdn_fwd_keep_workspace_bytes(B, T, H, GDN_K, a.width(i), a.L);
+        const bool keep = ctx != nullptr && (int64_t)total <= keep_bytes;
+        const Tensor g_cum = at::empty_like(g_), A = empty({2, B, T, H, 64}, at::kBFloat16, q), Aw = A.select(0, 0), Au = A.select(0, 1);
+        std::vector<Tensor> parts, kept;
+        for (int i = 0; i < n; ++i) {
+            const int V = a.width(i);
+            const size_t bytes = (keep ? lib.llattn_gdn_fwd_keep_workspace_bytes : lib.llattn_gdn_fwd_workspace_bytes)(B, T, H, GDN_K, V, a.L);
+            const Tensor ws = empty({(int64_t)bytes}, at::kByte, q), o = empty({B, T, H, V}, at::kBFloat16, q), vs = n > 1 ? a.slice(a.v, i) : a.v;
+            check((keep ? lib.llattn_gdn_fwd_keep : lib.llattn_gdn_fwd)(a.qn.data_ptr(), a.kn.data_ptr(), vs.data_ptr(), a.b.data_ptr(), fptr(a.g),
+                                                                       a.l.data_ptr(), o.data_ptr(), fptr(g_cum), Aw.data_ptr(), Au.data_ptr(),
+                                                                       ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
+                  "llattn_gdn_fwd");
+            if (status) check_status(ws, on.stream, "llattn_gdn_fwd");
+            parts.push_back(o);
+            if (keep) kept.push_back(ws);
+        }
+        if (ctx) {
+            variable_list save = {q_, k_, a.v, b_, g_cum, a.l, Aw, Au};
+            if (keep) {
+                save.push_back(a.qn);
+                save.push_back(a.kn);
+                for (const Tensor& w : kept) save.push_back(w);
+            }
+            ctx->save_for_backward(save);
+            ctx->saved_data["V"] = (int64_t)a.V;
+            ctx->saved_data["scale"] = scale;
+            ctx->saved_data["lam_mul"] = lam_mul;
+            ctx->saved_data["status"] = status;
+        }
+        return n == 1 ? parts[0] : at::cat(parts, -1);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list d) {
+        const auto s = ctx->get_saved_variables();
+        On on(s[0]);
+        const Tensor &q = s[0], &k = s[1], &v = s[2], &b = s[3], &g_cum = s[4], &l = s[5], &Aw = s[6], &Au = s[7];
+        const bool kept = s.size() > 8, status = ctx->saved_data["status"].toBool();
+        const double scale = ctx->saved_data["scale"].toDouble(), lam_mul = ctx->saved_data["lam_mul"].toDouble();
+        GdnInputs a;
+        a.B = q.size(0);
+        a.T = q.size(1);
+        a.H = q.size(2);
+        a.K = q.size(3);
+        a.V = (int)ctx->saved_data["V"].toInt();
+        a.L = l.size(3);
+        const int B = a.B, T = a.T, H = a.H, n = a.slices();
+        Tensor qn, kn;
+        if (kept) {
+            qn = s[8];
+            kn = s[9];
+        } else {
+            const Tensor qk = empty({2, B, T, H, GDN_K}, at::kBFloat16, q);
+            qn = qk.select(0, 0);
+            kn = qk.select(0, 1);
+            check(lib.llattn_gdn_prompt_prep(q.data_ptr(), k.data_ptr(), nullptr, nullptr, nullptr, nullptr, qn.data_ptr(), kn.data_ptr(), nullptr, nullptr,
+                                             nullptr, nullptr, B, T, T, H, H, a.K, GDN_K, 64, GDN_SLICE, a.L, a.L, (float)scale, 0.f, on.stream),
+                  "llattn_gdn_prompt_prep");
+        }
+        const Tensor d_o = d[0].to(at::kBFloat16).contiguous();
+        // fp32 gradients of the inputs that all slices share: dq | dk | dbeta | dlambda in one buffer, and dg, which is handed on as it is
+        const int64_t rows = (int64_t)B * T * H, per = rows * (2 * GDN_K + 1 + a.L);
+        Tensor sum, dg;
+        std::vector<Tensor> dvs;
+        for (int i = 0; i < n; ++i) {
+            const int V = a.width(i);
+            const Tensor vs = n > 1 ? a.slice(v, i) : v, dos = n > 1 ? d_o.narrow(3, i * GDN_SLICE, V).contiguous() : d_o;
+            const Tensor out = empty({per}, at::kFloat, q), dgi = empty({B, T, H}, at::kFloat, q);
+            float *dq = fptr(out), *dk = dq + rows * GDN_K, *db = dk + rows * GDN_K, *dl = db + rows;
+            const size_t bytes = (kept ? lib.llattn_gdn_bwd_kept_workspace_bytes : lib.llattn_gdn_bwd_workspace_bytes)(B, T, H, GDN_K, V, a.L);
+            const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
+            Tensor dv = empty({B, T, H, V}, kept ? at::kBFloat16 : at::kFloat, q);
+            if (kept) {
+                const Tensor& fws = s[10 + i];
+                check(lib.llattn_gdn_bwd_kept_bf16dv(qn.data_ptr(), kn.data_ptr(), vs.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(),
+                                                     Au.data_ptr(), dos.data_ptr(), dq, dk, dv.data_ptr(), db, fptr(dgi), dl, fws.data_ptr(), fws.numel(),
+                                                     ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
+                      "llattn_gdn_bwd_kept_bf16dv");
+            } else {
+                check(lib.llattn_gdn_bwd(qn.data_ptr(), kn.data_ptr(), vs.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(), Au.data_ptr(),
+                                         dos.data_ptr(), dq, dk, fptr(dv), db, fptr(dgi), dl, ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
+                      "llattn_gdn_bwd");
+                dv = dv.to(at::kBFloat16);
+            }
+            if (status) check_status(ws, on.stream, "llattn_gdn_bwd");
+            dvs.push_back(dv);
+            if (i == 0) {
+                sum = out;
+                dg = dgi;
+            } else {
+                sum.add_(out);
+                dg.add_(dgi);
+            }
+        }
+        const Tensor gqk = empty({2, B, T, H, a.K}, at::kBFloat16, q), gq = gqk.select(0, 0), gk = gqk.select(0, 1);
+        const Tensor gb = at::empty_like(b), gl = at::empty_like(l);
+        float *dq = fptr(sum), *dk = dq + rows * GDN_K, *db = dk + rows * GDN_K, *dl = db + rows;
+        check(lib.llattn_gdn_grad_out(q.data_ptr(), k.data_ptr(), dq, dk, db, dl, gq.data_ptr(), gk.data_ptr(), gb.data_ptr(), gl.data_ptr(), rows, a.K, GDN_K,
+                                      a.L, (float)scale, (float)lam_mul, on.stream),
+              "llattn_gdn_grad_out");
+        return {gq, gk, n == 1 ? dvs[0] : at::cat(dvs, -1), gb, dg, gl, Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+// hattention_kernel, delta-rule structure: l2norm of q (scaled) and k, lambda times lam_mul unless that is 0
+py::object hattention_gdn(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, double scale, double lam_mul,
+                          int64_t keep_bytes, bool status) {
+    if (!gdn_operands(q, k, v, b, g, l)) return py::none();
+    const int64_t T = q.size(1);
+    if (T % 64 != 0 || T > 16384 || l.size(3) < 7 + ceil_log2(T / 64)) return py::none();
+    const bool grad = wants_grad({q, k, v, b, g, l});
+    if (grad && q.size(2) != v.size(2)) return py::none();
+    py::gil_scoped_release nogil;
+    Tensor o = grad ? GdnKernel::apply(q, k, v, b, g, l, scale, lam_mul, keep_bytes, status)
+                    : GdnKernel::forward(nullptr, q, k, v, b, g, l, scale, lam_mul, 0, status);
+    py::gil_scoped_acquire gil;
+    return py::cast(o);
+}
+
+// a prompt of any length -> (o, level-major states) or None
+py::object gdn_prompt(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, double scale, double lam_mul,
+                      bool status) {
+    if (!gdn_operands(q, k, v, b, g, l)) return py::none();
+    const int T = q.size(1), L = l.size(3), Tp = (T + 63) / 64 * 64, Lo = T < 64 ? std::max(L, 7) : L;
+    if (Tp > 16384 || L < 1 + bit_length(T - 1) || Lo < 7 + ceil_log2(Tp / 64)) return py::none();
+    Tensor o, states;
+    {
+        py::gil_scoped_release nogil;
+        at::NoGradGuard no_grad;
+        On on(q);
+        GdnInputs a = gdn_prepare(q.contiguous(), k.contiguous(), v.contiguous(), b.contiguous(), g.contiguous(), l.contiguous(), T, Tp, Lo, scale, lam_mul,
+                                  on.stream);
+        const int B = a.B, H = a.H, K = a.K, n = a.slices();
+        states = empty({B, H, L, K, a.V}, at::kFloat, q);
+        const Tensor g_cum = at::empty_like(a.g), A = empty({2, B, Tp, H, 64}, at::kBFloat16, q);
+        std::vector<Tensor> parts;
+        for (int i = 0; i < n; ++i) {
+            const int V = a.width(i), c0 = i * GDN_SLICE;
+            const Tensor vs = a.V > GDN_SLICE || Tp != T ? a.slice(a.v, i) : a.v, out = empty({B, Tp, H, V}, at::kBFloat16, q);
+            const size_t bytes = lib.llattn_gdn_fwd_workspace_bytes(B, Tp, H, GDN_K, V, Lo);
+            const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
+            check(lib.llattn_gdn_prefill_slice(a.qn.data_ptr(), a.kn.data_ptr(), vs.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(), out.data_ptr(),
+                                               fptr(g_cum), A.select(0, 0).data_ptr(), A.select(0, 1).data_ptr(), fptr(states), K, a.V, c0, L,
+                                               ws.data_ptr(), bytes, B, Tp, H, GDN_K, V, Lo, on.stream),
+                  "llattn_gdn_prefill_slice");
+            check(lib.llattn_gdn_prompt_states(a.kn.data_ptr(), vs.data_ptr(), a.b.data_ptr(), fptr(a.g), fptr(states), B, T, Tp, H, K, a.V, V, c0, L,
+                                               on.stream),
+                  "llattn_gdn_prompt_states");
+            if (status) check_status(ws, on.stream, "llattn_gdn_prefill_slice");
+            parts.push_back(Tp == T ? out : out.narrow(1, 0, T));
+        }
+        o = n == 1 ? parts[0].contiguous() : at::cat(parts, -1);
+        states = states.permute({0, 1, 3, 4, 2});
+    }
+    return py::make_tuple(o, states);
+}
+
+// ------------------------------------------------------------------------------------------ decode steps
+// Runs the cascade on the token counts (a list of ints, updated in place): the levels that hold tokens before it, as bits, and the
+// level that receives the merged ones.  The new token is counted.
+struct Cascade {
+    unsigned live = 0;
+    int carry = 0;
+};
+Cascade cascade(const py::list& counts, int64_t L) {
+    TORCH_CHECK_VALUE((int64_t)counts.size() == L && L <= 32, "one token count per level");
+    Cascade c;
+    int64_t n[32];
+    for (int64_t i = 0; i < L; ++i) {
+        n[i] = PyLong_AsLongLong(PyList_GET_ITEM(counts.ptr(), i));
+        if (n[i] != 0) c.live |= 1u << i;
+    }
+    int level = 0;
+    while (n[level] == (int64_t(1) << level)) {
+        TORCH_CHECK_VALUE(level + 1 < L, "more tokens than the levels can hold");
+        n[level + 1] += n[level];
+        n[level] = 0;
+        ++level;
+    }
+    TORCH_CHECK_VALUE(n[level] < (int64_t(1) << level), "more tokens in a level than it holds");
+    c.carry = level;
+    n[0] += 1;
+    for (int64_t i = 0; i <= std::min<int64_t>(level, L - 1); ++i) PyList_SetItem(counts.ptr(), i, PyLong_FromLongLong(n[i]));
+    return c;
+}
+bool level_major(const Tensor& s) {
+    if (!is(s, at::kFloat) || s.dim() != 5) return false;
+    const int64_t H = s.size(1), K = s.size(2), V = s.size(3), L = s.size(4);
+    const auto st = s.strides();
+    return V % 16 == 0 && st[0] == H * L * K * V && st[1] == L * K * V && st[2] == V && st[3] == 1 && st[4] == K * V;
+}
+
+// hselective_state_update on a level-major state: y, or None (nothing done)
+py::object mamba2_step(const Tensor& states, const py::list& counts, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm,
+                       const Tensor& dl, const Tensor& Lp, const Maybe& D_, const Maybe& bias_, int64_t mode, bool softplus) {
+    const Tensor D = of(D_), bias = of(bias_);
+    if (!bf16(x) || !bf16(dt) || !bf16(Bm) || !bf16(Cm) || !bf16(dl) || !A.is_cuda() || !A.is_floating_point() || !param(Lp) || !param(D) || !param(bias) ||
+        x.dim() != 3 || Bm.dim() != 3 || dl.dim() != 3 || !level_major(states) || wants_grad({x, dt, A, Bm, Cm, dl, Lp, D, bias}) ||
+        !same_device({states, x, dt, A, Bm, Cm, dl, Lp, D, bias}))
+        return py::none();
+    const int64_t B = x.size(0), H = x.size(1), V = x.size(2), G = Bm.size(1), K = Bm.size(2), L = dl.size(2);
+    if (states.sizes() != at::IntArrayRef({B, H, K, V, L}) || dt.sizes() != at::IntArrayRef({B, H}) || A.sizes() != at::IntArrayRef({H}) || G <= 0 || H % G != 0 ||
+        Bm.size(0) != B || Cm.sizes() != Bm.sizes() || dl.sizes() != at::IntArrayRef({B, H, L}) || Lp.sizes() != at::IntArrayRef({H, L}) ||
+        (D.defined() && D.sizes() != at::IntArrayRef({H})) || (bias.defined() && bias.sizes() != at::IntArrayRef({H})) || V > 256 || K > 1024)
+        return py::none();
+    const Tensor q = Cm.contiguous(), k = Bm.contiguous(), x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), Lp_ = Lp.contiguous(),
+                 A_ = A.to(at::kFloat).contiguous(), D_c = contiguous(D), b_ = contiguous(bias);
+    const Tensor y = empty({B, H, V}, f32(D_c) ? at::kFloat : at::kBFloat16, x);
+    const Cascade c = cascade(counts, L);
+    const int dev = x.device().index();
+    check(lib.llattn_mamba2_layer_step(fptr(states), q.data_ptr(), k.data_ptr(), x_.data_ptr(), dt_.data_ptr(), nullptr, dl_.data_ptr(), Lp_.data_ptr(),
+                                       f32(Lp_), ptr(D_c), f32(D_c), ptr(b_), f32(b_), fptr(A_), y.data_ptr(), B, H, G, K, V, L, c.live, c.carry, (int)mode,
+                                       softplus, dev, at::cuda::getCurrentCUDAStream(dev).stream()),
+          "llattn_mamba2_layer_step");
+    return py::cast(y);
+}
+
+// the one-token call of chunk_h_gated_delta_rule (a token dimension of one in every operand): o (B,1,H,V), or None (nothing done)
+py::object gdn_step(const Tensor& states, const py::list& counts, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g,
+                    const Tensor& l, double scale, double lam_mul) {
+    if (!bf16(q) || !bf16(k) || !bf16(v) || !bf16(b) || !is(g, at::kFloat) || !bf16(l) || q.dim() != 4 || v.dim() != 4 || l.dim() != 4 ||
+        q.sizes() != k.sizes() || !level_major(states) || !same_device({states, q, k, v, b, g, l}))
+        return py::none();
+    const int64_t B = q.size(0), G = q.size(2), K = q.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
+    if (q.size(1) != 1 || v.size(0) != B || v.size(1) != 1 || b.sizes() != at::IntArrayRef({B, 1, H}) || g.sizes() != b.sizes() ||
+        l.sizes() != at::IntArrayRef({B, 1, H, L}) || states.sizes() != at::IntArrayRef({B, H, K, V, L}) || G <= 0 || H % G != 0 || K > 256)
+        return py::none();
+    const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), b_ = b.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
+    const Tensor o = empty({B, 1, H, V}, at::kBFloat16, q);
+    const Cascade c = cascade(counts, L);
+    const int dev = q.device().index();
+    check(lib.llattn_gdn_layer_step(fptr(states), q_.data_ptr(), k_.data_ptr(), v_.data_ptr(), b_.data_ptr(), fptr(g_), l_.data_ptr(), o.data_ptr(), B, H, G, K,
+                                    V, L, c.live, c.carry, 1, (float)scale, (float)lam_mul, dev, at::cuda::getCurrentCUDAStream(dev).stream()),
+          "llattn_gdn_layer_step");
+    return py::cast(o);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.def("bind", &bind);
+    m.def("hattention_mamba2", &hattention_mamba2);
+    m.def("mamba2_layer", &mamba2_layer);
+    m.def("mamba2_prompt", &mamba2_prompt);
+    m.def("mamba2_mixer", &mamba2_mixer);
+    m.def("mamba2_step", &mamba2_step);
+    m.def("hattention_gdn", &hattention_gdn);
+    m.def("gdn_prompt", &gdn_prompt);
+    m.def("gdn_step", &gdn_step);
+}

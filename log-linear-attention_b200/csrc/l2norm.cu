@@ -89,9 +89,84 @@ __global__ void __launch_bounds__(256) l2norm_bwd_kernel(const __nv_bfloat16* __
     }
 }
 
+// The gradients that leave a Gated DeltaNet backward, in one pass over the rows: q and k through the l2norm (and scale), beta and
+// lambda rounded to bf16 (lambda through its factor, rounded before and after it as two operators would).  16 lanes a row; K_in >= K columns of dq, dk are stored (padded keys).
+struct GdnGradOut {
+    const __nv_bfloat16 *q, *k;       // (rows,K)
+    const float *dq, *dk;             // (rows,K_in)
+    const float *db, *dl;             // (rows), (rows,L)
+    __nv_bfloat16 *gq, *gk, *gb, *gl;
+    long rows;
+    int K, K_in, L;
+    float scale, lam_mul;
+};
+
+__global__ void __launch_bounds__(256) gdn_grad_out_kernel(const __grid_constant__ GdnGradOut a) {
+    const int lane = threadIdx.x & 15;
+    const long row = (long)blockIdx.x * 16 + (threadIdx.x >> 4);
+    const bool have = row < a.rows, act = have && lane * 8 < a.K;
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const float scale = w == 0 ? a.scale : 1.f;
+        float f[8] = {}, g[8] = {};
+        float ss = 0.f, dot = 0.f;
+        if (act) {
+            const uint4 raw = *reinterpret_cast<const uint4*>((w == 0 ? a.q : a.k) + row * a.K + lane * 8);
+            const float* d = (w == 0 ? a.dq : a.dk) + row * a.K_in + lane * 8;
+            const float4 g0 = *reinterpret_cast<const float4*>(d), g1 = *reinterpret_cast<const float4*>(d + 4);
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+            g[0] = g0.x * scale; g[1] = g0.y * scale; g[2] = g0.z * scale; g[3] = g0.w * scale;
+            g[4] = g1.x * scale; g[5] = g1.y * scale; g[6] = g1.z * scale; g[7] = g1.w * scale;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                f[2 * i] = __bfloat162float(h[i].x);
+                f[2 * i + 1] = __bfloat162float(h[i].y);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                ss += f[i] * f[i];
+                dot += f[i] * g[i];
+            }
+        }
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) {
+            ss += __shfl_xor_sync(0xffffffffu, ss, d);
+            dot += __shfl_xor_sync(0xffffffffu, dot, d);
+        }
+        if (act) {
+            const float rstd = rsqrtf(ss + 1e-6f), yd = dot * rstd * rstd;
+            uint4 out;
+            __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&out);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                o[i] = __floats2bfloat162_rn((g[2 * i] - f[2 * i] * yd) * rstd, (g[2 * i + 1] - f[2 * i + 1] * yd) * rstd);
+            *reinterpret_cast<uint4*>((w == 0 ? a.gq : a.gk) + row * a.K + lane * 8) = out;
+        }
+    }
+    if (!have) return;
+    if (lane == 15) a.gb[row] = __float2bfloat16(a.db[row]);
+    for (int j = lane; j < a.L; j += 16) {
+        __nv_bfloat16 x = __float2bfloat16(a.dl[row * a.L + j]);
+        if (a.lam_mul != 0.f) x = __float2bfloat16(__bfloat162float(x) * a.lam_mul);
+        a.gl[row * a.L + j] = x;
+    }
+}
+
 }  // namespace llattn
 
 extern "C" {
+
+int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const float* dk, const float* dbeta, const float* dlambda, void* gq,
+                        void* gk, void* gbeta, void* glambda, long rows, int K, int K_in, int L, float scale, float lambda_mul, void* stream) {
+    if (rows <= 0 || K <= 0 || K % 8 != 0 || K_in < K || K_in % 8 != 0 || K_in > 128 || L <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!q || !k || !dq || !dk || !dbeta || !dlambda || !gq || !gk || !gbeta || !glambda) return LLATTN_ERR_NULL;
+    using bf = __nv_bfloat16;
+    llattn::GdnGradOut a{(const bf*)q, (const bf*)k, dq, dk, dbeta, dlambda, (bf*)gq, (bf*)gk, (bf*)gbeta, (bf*)glambda, rows, K, K_in, L, scale,
+                         lambda_mul};
+    llattn::gdn_grad_out_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, (cudaStream_t)stream>>>(a);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
 
 static int l2norm_check(const void* a, const void* b, long rows, int D) {
     if (rows <= 0 || D <= 0 || D > 256 || D % 8 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;

@@ -3,6 +3,8 @@
 #pragma once
 #include <atomic>
 
+#include "launch_cache.h"
+
 namespace llattn {
 extern std::atomic<unsigned long long> g_kernel_launches;
 }

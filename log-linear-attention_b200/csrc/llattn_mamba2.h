@@ -67,7 +67,8 @@ int mamba2_hi_out_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 extern std::atomic<int> g_use_tensor_core_path;   // test hook, see llattn_testing.h
 // segment summaries and decays inside the workspace of a forward call (null when it has one segment only)
 int mamba2_fwd_workspace_segments(const void* ws, size_t bytes, int B, int T, int H, int G, int K, int V, const float** F, const float** D);
-void mamba2_uncumsum(const float* gc, float* g, long BT, int H, cudaStream_t stream);
+// clears acc_bytes (a multiple of 16) at acc and ndl floats at dl, and takes the in-chunk cumulative sum of g apart
+int mamba2_bwd_init(const float* gc, float* g, long BT, int H, void* acc, size_t acc_bytes, float* dl, long ndl, cudaStream_t stream);
 int mamba2_dg(const Mamba2Params& p, float* dg, cudaStream_t stream);
 void cast_f32_to_bf16(const float* src, void* dst, long n, cudaStream_t stream);
 

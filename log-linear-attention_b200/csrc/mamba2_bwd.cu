@@ -949,14 +949,22 @@ __global__ void __launch_bounds__(256) m2_seg_dscan_kernel(const Mamba2Params p,
 // ------------------------------------------------------------------------------------------
 // small elementwise kernels
 // ------------------------------------------------------------------------------------------
-// raw g from its in-chunk inclusive cumulative sum (what the forward returns and autograd saves)
-__global__ void m2_uncumsum_kernel(const float* __restrict__ gc, float* __restrict__ g, long BT, int H) {
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= BT * H) return;
-    const long t = idx / H;
-    float x = gc[idx];
-    if ((t % CH) != 0) x -= gc[idx - H];
-    g[idx] = x;
+// What the backward kernels expect before they start, in one launch (three clears and a small kernel before): the raw g from its in-chunk
+// inclusive cumulative sum (what the forward returns and autograd saves), cleared accumulators and status word, cleared dlambda.
+__global__ void __launch_bounds__(256) m2_bwd_init_kernel(const float* __restrict__ gc, float* __restrict__ g, unsigned n, unsigned H,
+                                                          float4* __restrict__ acc, long acc4, float4* __restrict__ dl, long dl4,
+                                                          float* __restrict__ dl_tail, int ntail) {
+    const long i0 = (long)blockIdx.x * 256 + threadIdx.x, step = (long)gridDim.x * 256;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long i = i0; i < acc4; i += step) acc[i] = z;
+    for (long i = i0; i < dl4; i += step) dl[i] = z;
+    if (i0 < ntail) dl_tail[i0] = 0.f;
+    for (long i = i0; i < n; i += step) {
+        const unsigned t = (unsigned)i / H;
+        float x = gc[i];
+        if ((t % CH) != 0) x -= gc[i - H];
+        g[i] = x;
+    }
 }
 
 // dg for one (batch, head) per CTA.
@@ -1112,11 +1120,6 @@ __global__ void m2_cast_bf16_kernel(const float* __restrict__ src, bf16* __restr
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
-template <typename KernT>
-static cudaError_t set_smem(KernT kern, size_t bytes) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 template <int KD, int VD, int MLOW>
 static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
@@ -1133,12 +1136,12 @@ static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
         } else {
             {
                 auto kern = m2_hi_bwd_q_kernel<KD, VD, MLOW>;
-                if ((e = set_smem(kern, HiBwdSmem<KD, VD>::total)) != cudaSuccess) return (int)e;
+                if ((e = allow_smem(kern, HiBwdSmem<KD, VD>::total)) != cudaSuccess) return (int)e;
                 kern<<<p.B * p.H * (p.NT - SEG), 256, HiBwdSmem<KD, VD>::total, stream>>>(p); LLATTN_LAUNCHED();
             }
             {
                 auto kern = m2_seg_dstate_kernel<KD, VD, MLOW>;
-                if ((e = set_smem(kern, SegDSmem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
+                if ((e = allow_smem(kern, SegDSmem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
                 dim3 grid(p.B * p.H * (p.NS - 1), p.LH);
                 kern<<<grid, 256, SegDSmem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
             }
@@ -1155,7 +1158,7 @@ static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
         if (rc != 0) return rc;
     } else {
         auto kern = m2_bwd_fwdorder_kernel<KD, VD, MLOW>;
-        if ((e = set_smem(kern, Bwd1Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
+        if ((e = allow_smem(kern, Bwd1Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
         kern<<<p.B * p.H * p.NS, 256, Bwd1Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
     }
     if (use_tc) {
@@ -1163,7 +1166,7 @@ static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
         if (rc != 0) return rc;
     } else {
         auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;
-        if ((e = set_smem(kern, Bwd2Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
+        if ((e = allow_smem(kern, Bwd2Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
         kern<<<p.B * p.H * p.NS, 256, Bwd2Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();
@@ -1175,16 +1178,30 @@ int mamba2_bwd_dispatch(Mamba2Params p, cudaStream_t stream) {
     return LLATTN_ERR_UNSUPPORTED_SHAPE;
 }
 
-void mamba2_uncumsum(const float* gc, float* g, long BT, int H, cudaStream_t stream) {
-    const long n = BT * H;
-    m2_uncumsum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(gc, g, BT, H); LLATTN_LAUNCHED();
+int mamba2_bwd_init(const float* gc, float* g, long BT, int H, void* acc, size_t acc_bytes, float* dl, long ndl, cudaStream_t stream) {
+    if (BT * H > 0xffffffffl) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    long dl4 = ndl / 4, tail = ndl % 4;
+    if ((uintptr_t)dl & 15) {
+        const cudaError_t e = cudaMemsetAsync(dl, 0, (size_t)ndl * sizeof(float), stream);
+        if (e != cudaSuccess) return (int)e;
+        dl4 = tail = 0;
+    }
+    const long acc4 = (long)(acc_bytes / 16);
+    long most = BT * H;
+    if (acc4 > most) most = acc4;
+    if (dl4 > most) most = dl4;
+    const long blocks = (most + 255) / 256;
+    m2_bwd_init_kernel<<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream>>>(
+        gc, g, (unsigned)(BT * H), (unsigned)H, (float4*)acc, acc4, (float4*)dl, dl4, dl + dl4 * 4, (int)tail);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
 }
 
 int mamba2_dg(const Mamba2Params& p, float* dg, cudaStream_t stream) {
     dim3 grid(p.B * p.H, (p.NT + 63) / 64);
     const size_t smem = (size_t)(p.NT + p.NS + p.NT * p.LZ + p.NT * (M2_MLOW + 1) + p.NS * (p.LH > 0 ? p.LH : 1) + (size_t)p.LZ * p.NT) * sizeof(float);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(m2_dg_kernel<M2_MLOW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(m2_dg_kernel<M2_MLOW>, smem);
         if (e != cudaSuccess) return (int)e;
     }
     m2_dg_kernel<M2_MLOW><<<grid, 256, smem, stream>>>(p, dg); LLATTN_LAUNCHED();

@@ -1312,7 +1312,7 @@ int mamba2_bwd2_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_f32_box_map(&p.tm_dk, p.dk_acc, BT, p.G, p.K, tc::PT)) != 0) return rc;
     auto kern = m2_bwd_revorder_tc_kernel<M2_MLOW>;
     const size_t sm = Bwd2TcSmem<M2_MLOW>::total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
     kern<<<p.B * p.H * p.NS, tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
@@ -1330,11 +1330,11 @@ int mamba2_bwd1_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_f32_box_map(&p.tm_dk, p.dk_acc, BT, p.G, p.K, tc::PT)) != 0) return rc;
     auto kern = m2_bwd_fwdorder_tc_kernel<M2_MLOW>;
     const size_t sm = Bwd1TcSmem<M2_MLOW>::total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+    if ((e = sm_count(&sms, dev)) != cudaSuccess) return (int)e;
     const int nitems = p.B * p.H * p.NS;
     kern<<<nitems < sms ? nitems : sms, tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();      // persistent: one CTA per SM
     return (int)cudaGetLastError();

@@ -581,7 +581,7 @@ static int launch_states(Mamba2Params p, cudaStream_t stream) {
     } else {
         auto kern = m2_seg_state_kernel<KD, VD, MLOW>;
         size_t sm = SegSmem<KD, VD, MLOW>::total;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+        if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
         kern<<<p.B * p.H * (p.NS - 1), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
     }
     const int KV = KD * VD;
@@ -604,7 +604,7 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
         } else {
             auto kern = m2_hi_out_kernel<KD, VD, MLOW>;
             size_t sm = HiSmem<KD, VD>::total;
-            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+            if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
             kern<<<p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
         }
     }
@@ -614,7 +614,7 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     {
         auto kern = m2_chunk_fwd_kernel<KD, VD, MLOW>;
         size_t sm = FwdSmem<KD, VD, MLOW>::total;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess) return (int)e;
+        if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
         kern<<<p.B * p.H * p.NS, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();

@@ -488,7 +488,7 @@ int mamba2_fwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_panel_map(&p.tm_v, p.v, (long)p.B * p.T, p.H, p.V, tc::PT)) != 0) return rc;
     auto kern = m2_chunk_fwd_tc_kernel<M2_MLOW>;
     const size_t sm = FwdTcSmem<M2_MLOW>::total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
     kern<<<p.B * p.H * p.NS, tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();

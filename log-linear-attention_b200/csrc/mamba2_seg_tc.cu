@@ -689,7 +689,7 @@ int mamba2_seg_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_panel_map(&p.tm_v, p.v, BT, p.H, p.V, tc::PT)) != 0) return rc;
     auto kern = m2_seg_state_tc_kernel<M2_MLOW>;
     const size_t sm = SegStateTcSmem<M2_MLOW>::total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
     kern<<<p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
@@ -705,13 +705,13 @@ int mamba2_hi_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if (p.LH <= 5) {
         auto kern = m2_hi_out_tc_kernel<M2_MLOW, 5>;
         const size_t sm = HiOutTcSmem<M2_MLOW, 5>::total;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_smem(kern, sm);
         if (e != cudaSuccess) return (int)e;
         kern<<<p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
     } else {
         auto kern = m2_hi_out_tc_kernel<M2_MLOW, 8>;
         const size_t sm = HiOutTcSmem<M2_MLOW, 8>::total;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_smem(kern, sm);
         if (e != cudaSuccess) return (int)e;
         kern<<<p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
     }
@@ -728,7 +728,7 @@ int mamba2_hi_bwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_f32_box_map(&p.tm_dq, p.dq_acc, BT, p.G, p.K, tc::PT)) != 0) return rc;
     auto kern = m2_hi_bwd_tc_kernel<M2_MLOW>;
     const size_t sm = HiBwdTcSmem<M2_MLOW>::total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
     // one launch per window of five segment levels (a single one up to T = 16384); dq, the q.dq totals and
     // the per-level outputs of different windows add up or are disjoint

@@ -15,7 +15,9 @@ namespace llattn {
 
 struct PrepArgs {
     const __nv_bfloat16 *x, *dt_raw, *dl;      // (rows,P), (rows), (rows,L)
-    const float *dt_bias, *A, *Lp, *D;         // (H) or null, (H), (H,L), (H) or null
+    const void *dt_bias, *Lp, *D;              // (H) or null, (H,L), (H) or null
+    const float* A;                            // (H)
+    int bias_f32, lp_f32, d_f32;
     __nv_bfloat16 *v, *lam;
     float* g;
     const __nv_bfloat16 *dv, *dy;
@@ -40,7 +42,7 @@ __global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_consta
     const int lam_grid = a.lam_blocks * a.lam_runs;
     if ((int)blockIdx.x < lam_grid) {
         const int per = (a.tokens + a.lam_runs - 1) / a.lam_runs, t0 = blockIdx.x / a.lam_blocks * per, t1 = min(a.tokens, t0 + per);
-        const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, 1, a.H * a.L, a.mode};
+        const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, a.lp_f32, a.H * a.L, a.mode};
         const int block = blockIdx.x % a.lam_blocks;
         if (a.lam8) lambda_part_fwd<8>(c, a.lam, t0, t1, block, a.lam_blocks);
         else lambda_part_fwd<1>(c, a.lam, t0, t1, block, a.lam_blocks);
@@ -53,7 +55,7 @@ __global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_consta
     if (h >= a.H) return;                      // whole groups
     const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u) << (threadIdx.x & 31 & ~(LPR - 1));
     const bool act = lane * 8 < a.P;
-    const float bias = a.dt_bias ? a.dt_bias[h] : 0.f, A = a.A[h];
+    const float bias = a.dt_bias ? load_param(a.dt_bias, h, a.bias_f32) : 0.f, A = a.A[h];
     const long xs = (long)a.H * a.P, off = (long)h * a.P + lane * 8;
     float dtl = 0.f;
     for (int t = t0; t < t1; t += U) {
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(256, 4) m2_prep_bwd_kernel(const __grid_consta
     const int lam_grid = a.lam_blocks * a.lam_runs;
     if ((int)blockIdx.x < lam_grid) {
         const int per = (a.tokens + a.lam_runs - 1) / a.lam_runs, t0 = blockIdx.x / a.lam_blocks * per, t1 = min(a.tokens, t0 + per);
-        const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, 1, a.H * a.L, a.mode};
+        const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, a.lp_f32, a.H * a.L, a.mode};
         __shared__ float sums[256 * 8];
         const int block = blockIdx.x % a.lam_blocks;
         if (a.lam8) lambda_part_bwd<8>(c, a.dlam, a.ddl, c.dl_stride, a.dLp, t0, t1, block, a.lam_blocks, sums);
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(256, 4) m2_prep_bwd_kernel(const __grid_consta
     if (h >= a.H) return;
     const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u) << (threadIdx.x & 31 & ~(LPR - 1));
     const bool act = lane * 8 < a.P;
-    const float bias = a.dt_bias ? a.dt_bias[h] : 0.f, A = a.A[h], D = a.D ? a.D[h] : 0.f;
+    const float bias = a.dt_bias ? load_param(a.dt_bias, h, a.bias_f32) : 0.f, A = a.A[h], D = a.D ? load_param(a.D, h, a.d_f32) : 0.f;
     const long xs = (long)a.H * a.P, off = (long)h * a.P + lane * 8;
     float raw = 0.f, dtl = 0.f, dotl = 0.f, sA = 0.f, sB = 0.f, sD = 0.f;
     for (int t = t0; t < t1; ++t) {
@@ -207,8 +209,9 @@ static unsigned prep_grid(llattn::PrepArgs& a, long rows, int H, int P, int L, i
     return (unsigned)(a.row_blocks * ((a.tokens + a.run - 1) / a.run) + a.lam_blocks * a.lam_runs);
 }
 
-int llattn_mamba2_prep_fwd(const void* x, const void* dt_raw, const float* dt_bias, const float* A, const void* dl, const float* Lp,
-                           void* v, float* g, void* lambda, long rows, int H, int P, int L, int lambda_mode, void* stream) {
+int llattn_mamba2_layer_prep_fwd(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
+                                 const void* Lp, int lp_is_f32, void* v, float* g, void* lambda, long rows, int H, int P, int L,
+                                 int lambda_mode, void* stream) {
     int rc = prep_check(rows, H, P, L, lambda_mode);
     if (rc != 0) return rc;
     if (!x || !dt_raw || !A || !dl || !Lp || !v || !g || !lambda) return LLATTN_ERR_NULL;
@@ -216,6 +219,7 @@ int llattn_mamba2_prep_fwd(const void* x, const void* dt_raw, const float* dt_bi
     cudaStream_t st = (cudaStream_t)stream;
     llattn::PrepArgs a = {};
     a.x = (const bf*)x; a.dt_raw = (const bf*)dt_raw; a.dl = (const bf*)dl; a.dt_bias = dt_bias; a.A = A; a.Lp = Lp;
+    a.bias_f32 = bias_is_f32; a.lp_f32 = lp_is_f32;
     a.v = (bf*)v; a.lam = (bf*)lambda; a.g = g;
     const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, false);
     if (a.lpr == 4) llattn::m2_prep_fwd_kernel<4><<<grid, 256, 0, st>>>(a);
@@ -226,10 +230,15 @@ int llattn_mamba2_prep_fwd(const void* x, const void* dt_raw, const float* dt_bi
     return (int)cudaGetLastError();
 }
 
-int llattn_mamba2_prep_bwd(const void* x, const void* dt_raw, const float* dt_bias, const float* A, const void* dl, const float* Lp,
-                           const float* D, const void* dv, const float* dg, const float* dlambda, const void* dy,
-                           void* dx, void* ddt, void* ddl, float* dA, float* dbias, float* dLp, float* dD,
-                           long rows, int H, int P, int L, int lambda_mode, void* stream) {
+int llattn_mamba2_prep_fwd(const void* x, const void* dt_raw, const float* dt_bias, const float* A, const void* dl, const float* Lp,
+                           void* v, float* g, void* lambda, long rows, int H, int P, int L, int lambda_mode, void* stream) {
+    return llattn_mamba2_layer_prep_fwd(x, dt_raw, dt_bias, 1, A, dl, Lp, 1, v, g, lambda, rows, H, P, L, lambda_mode, stream);
+}
+
+int llattn_mamba2_layer_prep_bwd(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
+                                 const void* Lp, int lp_is_f32, const void* D, int d_is_f32, const void* dv, const float* dg,
+                                 const float* dlambda, const void* dy, void* dx, void* ddt, void* ddl, float* dA, float* dbias,
+                                 float* dLp, float* dD, long rows, int H, int P, int L, int lambda_mode, void* stream) {
     int rc = prep_check(rows, H, P, L, lambda_mode);
     if (rc != 0) return rc;
     if (!x || !dt_raw || !A || !dl || !Lp || !dv || !dg || !dlambda || !dx || !ddt || !ddl || !dA || !dLp) return LLATTN_ERR_NULL;
@@ -239,6 +248,7 @@ int llattn_mamba2_prep_bwd(const void* x, const void* dt_raw, const float* dt_bi
     cudaStream_t st = (cudaStream_t)stream;
     llattn::PrepArgs a = {};
     a.x = (const bf*)x; a.dt_raw = (const bf*)dt_raw; a.dl = (const bf*)dl; a.dt_bias = dt_bias; a.A = A; a.Lp = Lp; a.D = D;
+    a.bias_f32 = bias_is_f32; a.lp_f32 = lp_is_f32; a.d_f32 = d_is_f32;
     a.dv = (const bf*)dv; a.dg = dg; a.dlam = dlambda; a.dy = (const bf*)dy;
     a.dx = (bf*)dx; a.ddt = (bf*)ddt; a.ddl = (bf*)ddl; a.dA = dA; a.dbias = dt_bias ? dbias : nullptr; a.dLp = dLp; a.dD = dD;
     const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, true);
@@ -248,6 +258,14 @@ int llattn_mamba2_prep_bwd(const void* x, const void* dt_raw, const float* dt_bi
     else llattn::m2_prep_bwd_kernel<32><<<grid, 256, 0, st>>>(a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
+}
+
+int llattn_mamba2_prep_bwd(const void* x, const void* dt_raw, const float* dt_bias, const float* A, const void* dl, const float* Lp,
+                           const float* D, const void* dv, const float* dg, const float* dlambda, const void* dy,
+                           void* dx, void* ddt, void* ddl, float* dA, float* dbias, float* dLp, float* dD,
+                           long rows, int H, int P, int L, int lambda_mode, void* stream) {
+    return llattn_mamba2_layer_prep_bwd(x, dt_raw, dt_bias, 1, A, dl, Lp, 1, D, 1, dv, dg, dlambda, dy, dx, ddt, ddl, dA, dbias, dLp, dD, rows, H,
+                                        P, L, lambda_mode, stream);
 }
 
 int llattn_mamba2_residual(const void* o, const void* x, const float* D, void* y, int y_is_f32, long rows, int H, int P, void* stream) {

@@ -123,6 +123,24 @@ def lib():
     return L
 
 
+_host = None
+
+
+def host():
+    """The native host module (csrc/host.cpp), bound to the same library.  Raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("the native host module _host.so is missing: build it with `make -C log-linear-attention_b200/csrc` "
+                               f"(or __graft_entry__.build()): {e}") from e
+        module.bind(_LIB_PATH)
+        _host = module
+    return _host
+
+
 # When set, every Mamba-2 driver call reads its workspace's status word after the launch (one stream
 # synchronisation per call) and raises if a kernel gave up on a bounded wait.  Off by default: the
 # drivers then never synchronise, like the reference's.  The test-suite, the smoke check and the

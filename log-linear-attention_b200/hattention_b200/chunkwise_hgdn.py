@@ -12,7 +12,6 @@ import torch
 
 from . import _lib
 from .base import HType, ceil_log, get_num_levels
-from .recurrent import level_major_states
 
 CHUNK = 64
 
@@ -226,55 +225,20 @@ def chunkwise_bwd(q, k, v, b, g, l, Aw, Au, do, head_first, level_base, htype, c
     return dq, dk, dv, db, dg, dl
 
 
-def prompt_forward(q, k, v, b, g, l, scale, level_base: int, htype: HType, chunk_size: int, lambda_mul: float = 0.0):
+def prompt_forward(q, k, v, b, g, l, scale, head_first, level_base: int, htype: HType, chunk_size: int, lambda_mul: float = 0.0):
     """Outputs (B,T,H,V) and level states (B,H,K,V,L), level-major, after a prompt of any length: q, k raw (normalised here, q also
-    scaled), l multiplied by lambda_mul unless that is 0."""
-    B, T, G, K = k.shape
-    H, V = v.shape[2:]
-    L = l.shape[-1]
-    Tp = -(-T // CHUNK) * CHUNK
-    Lo = max(L, get_num_levels(CHUNK, 2) if T < CHUNK else 0)
-    if 1 + (T - 1).bit_length() > L:
-        raise ValueError("more tokens than the levels can hold")
-    bf = dict(dtype=torch.bfloat16, device=q.device)
-    with torch.cuda.device(q.device):
-        q_, k_, v_, b_, l_ = (x.to(torch.bfloat16).contiguous() for x in (q, k, v, b, l))
-        g_ = g.to(torch.float32).contiguous()
-        qn, kn = torch.empty(B, Tp, H, K_CALL, **bf), torch.empty(B, Tp, H, K_CALL, **bf)
-        vp, bp, lp = torch.empty(B * Tp * H * V, **bf), torch.empty(B, Tp, H, **bf), torch.empty(B, Tp, H, Lo, **bf)
-        gp = torch.empty(B, Tp, H, dtype=torch.float32, device=q.device)
-        slices = _v_slices(V)
-        _check(kn, kn, v, bp, gp, lp, False, level_base, htype, chunk_size)
-        lib = _lib.lib()
-        stream = torch.cuda.current_stream().cuda_stream
-        rc = lib.llattn_gdn_prompt_prep(q_.data_ptr(), k_.data_ptr(), v_.data_ptr(), b_.data_ptr(), g_.data_ptr(), l_.data_ptr(),
-                                        qn.data_ptr(), kn.data_ptr(), vp.data_ptr(), bp.data_ptr(), gp.data_ptr(), lp.data_ptr(),
-                                        B, T, Tp, H, G, K, K_CALL, V, V_SLICE, L, Lo, scale, lambda_mul, stream)
-        _lib.check(rc, "llattn_gdn_prompt_prep")
-        states = level_major_states((B, H, K, V, L), q.device)
-        g_cum = torch.empty_like(gp)
-        Aw, Au = torch.empty(B, Tp, H, CHUNK, **bf), torch.empty(B, Tp, H, CHUNK, **bf)
-        parts = []
-        for s, e in slices:
-            n = e - s
-            vs = vp[B * Tp * H * s:B * Tp * H * e]
-            o = torch.empty(B, Tp, H, n, **bf)
-            nbytes = lib.llattn_gdn_fwd_workspace_bytes(B, Tp, H, K_CALL, n, Lo)
-            if nbytes == 0:
-                raise ValueError("unsupported GDN shape (K at most 128, V a multiple of 64, T <= 16384)")
-            ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
-            rc = lib.llattn_gdn_prefill_slice(qn.data_ptr(), kn.data_ptr(), vs.data_ptr(), bp.data_ptr(), gp.data_ptr(), lp.data_ptr(),
-                                              o.data_ptr(), g_cum.data_ptr(), Aw.data_ptr(), Au.data_ptr(), states.data_ptr(), K, V, s, L,
-                                              ws.data_ptr(), nbytes, B, Tp, H, K_CALL, n, Lo, stream)
-            _lib.check(rc, "llattn_gdn_prefill_slice")
-            rc = lib.llattn_gdn_prompt_states(kn.data_ptr(), vs.data_ptr(), bp.data_ptr(), gp.data_ptr(), states.data_ptr(), B, T, Tp, H,
-                                              K, V, n, s, L, stream)
-            _lib.check(rc, "llattn_gdn_prompt_states")
-            if _lib.CHECK_STATUS:
-                _lib.raise_on_status(ws, stream, "llattn_gdn_prefill_slice")
-            parts.append(o[:, :T])
-        o = parts[0].contiguous() if len(parts) == 1 else torch.cat(parts, dim=-1)
-    return o, states
+    scaled), l multiplied by lambda_mul unless that is 0.  The tensors are padded with zero tokens to whole chunks by the pass that
+    normalises q and k; the scan over chunks leaves the inter-chunk levels, and one kernel advances them by the last chunk's tokens
+    and builds the levels inside it."""
+    bf = torch.bfloat16
+    r = _lib.host().gdn_prompt(q.to(bf), k.to(bf), v.to(bf), b.to(bf), g.to(torch.float32), l.to(bf), scale, lambda_mul, _lib.CHECK_STATUS)
+    if r is None:
+        T = q.shape[1]
+        _check(q[:, :T // CHUNK * CHUNK], k[:, :T // CHUNK * CHUNK], v, b[:, :T // CHUNK * CHUNK], g[:, :T // CHUNK * CHUNK],
+               l[:, :T // CHUNK * CHUNK], head_first, level_base, htype, chunk_size)
+        _v_slices(v.shape[-1])
+        raise ValueError("unsupported GDN prompt (K at most 128 and a multiple of 8, V a multiple of 64, T <= 16384, enough lambda levels)")
+    return r
 
 
 # Largest forward workspace (chunk matrices + level states, bytes) that gdn_forward keeps for the backward

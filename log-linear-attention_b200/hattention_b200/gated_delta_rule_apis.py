@@ -5,9 +5,9 @@ from typing import Optional
 
 import torch
 
+from . import _lib
 from .base import HStruct, HType
-from .kernel import gdn_layer_step, hattention_kernel, hattention_step, prefill
-from .recurrent import is_level_major
+from .kernel import gdn_native, hattention_kernel, hattention_step, prefill
 
 SCALE_LAMBDA = True
 
@@ -53,14 +53,12 @@ def chunk_h_gated_delta_rule(
         if not (q.ndim == 4 and k.ndim == 4 and v.ndim == 4 and beta.ndim == 3 and g.ndim == 3 and l.ndim == 4
                 and q.shape[1] == k.shape[1] == v.shape[1] == beta.shape[1] == g.shape[1] == l.shape[1] == 1):
             raise ValueError
-        q, k, v, beta, g, l = (x.squeeze(1) for x in (q, k, v, beta, g, l))
         s = initial_state
-        if (q.dtype == l.dtype == beta.dtype == torch.bfloat16 and g.dtype == s.dtype == torch.float32 and s.base == 2
-                and s.htype == HType.WEAK and s.hstruct == HStruct.GDELTA and v.is_cuda and is_level_major(s.states)):
-            with torch.no_grad():
-                o = gdn_layer_step(s, q.contiguous(), k.contiguous(), v.contiguous(), beta.contiguous(), g.contiguous(), l.contiguous(),
-                                   scale, lambda_mul)
-            return o.unsqueeze(1), s
+        if s.base == 2 and s.htype == HType.WEAK and s.hstruct == HStruct.GDELTA:
+            o = _lib.host().gdn_step(s.states, s.counts, q, k, v, beta, g, l, scale, lambda_mul)
+            if o is not None:
+                return o, s
+        q, k, v, beta, g, l = (x.squeeze(1) for x in (q, k, v, beta, g, l))
         if SCALE_LAMBDA:
             l = l / scale
         o, final_state = hattention_step(hstate=s, q=q, k=k, v=v, b=beta, g=g, l=l, scale=scale, level_base=2, htype=HType.WEAK,
@@ -68,6 +66,9 @@ def chunk_h_gated_delta_rule(
         return o.unsqueeze(1), final_state
     if initial_state is not None:
         raise NotImplementedError
+    o = gdn_native(q, k, v, beta, g, l, scale, 1.0 / scale if SCALE_LAMBDA else 0.0)
+    if o is not None:
+        return o, None
     if SCALE_LAMBDA:
         l = l / scale
     o = hattention_kernel(q=q, k=k, v=v, b=beta, g=g, l=l, scale=scale, head_first=False, level_base=2, htype=HType.WEAK,

@@ -87,6 +87,13 @@ class HAttentionFunction(torch.autograd.Function):
                 None, None, None, None, None, None, None, None)
 
 
+def gdn_native(q, k, v, b, g, l, scale: float, lambda_mul: float):
+    """The native Gated DeltaNet node (lambda times lambda_mul unless that is 0), or None for operands that it does not take."""
+    from .chunkwise_hgdn import KEEP_WORKSPACE_MAX_BYTES
+    return _lib.host().hattention_gdn(q, k, v, b, g, l, scale, lambda_mul, KEEP_WORKSPACE_MAX_BYTES if KEEP_FORWARD_STATES else -1,
+                                      _lib.CHECK_STATUS)
+
+
 def hattention_kernel(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -106,6 +113,15 @@ def hattention_kernel(
     """o = log-linear attention(q, k, v, g, l[, b]) with gradients; see kernel.py:338-374."""
     if chunk_sizes is None:
         chunk_sizes = (64, 64)
+    if chunkwise and not head_first and level_base == 2 and htype == HType.WEAK and tuple(chunk_sizes) == (64, 64):
+        # bf16 operands of the supported shapes: the native nodes; everything else, errors included, below
+        o = None
+        if hstruct == HStruct.MAMBA2 and b is None and scale is None and not use_qk_l2norm_in_kernel:
+            o = _lib.host().hattention_mamba2(q, k, v, g, l, KEEP_FORWARD_STATES, _lib.CHECK_STATUS)
+        elif hstruct == HStruct.GDELTA and b is not None and scale is not None and use_qk_l2norm_in_kernel:
+            o = gdn_native(q, k, v, b, g, l, scale, 0.0)
+        if o is not None:
+            return o
     return HAttentionFunction.apply(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chunk_sizes,
                                     chunkwise, use_qk_l2norm_in_kernel)
 
@@ -260,7 +276,7 @@ def prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chu
             o, states = prompt_forward(q, k, v, g, l, level_base, htype, chunk_size)
         else:
             from .chunkwise_hgdn import prompt_forward
-            o, states = prompt_forward(q, k, v, b, g, l, scale, level_base, htype, chunk_size, lambda_mul)
+            o, states = prompt_forward(q, k, v, b, g, l, scale, head_first, level_base, htype, chunk_size, lambda_mul)
         hstate = HState.holding(states, level_base, htype, hstruct)
         hstate.set_counts_after(T)
         return o.to(v.dtype), hstate

@@ -5,11 +5,10 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import _lib
+from . import _lib, kernel
 from .base import HStruct, HType
-from .chunkwise import chunkwise_bwd, chunkwise_fwd, prompt_forward_padded, prompt_length
-from .kernel import KEEP_FORWARD_STATES, hattention_kernel, hattention_prefill, hattention_step, mamba2_layer_step
-from .recurrent import HState, is_level_major
+from .kernel import hattention_kernel, hattention_prefill, hattention_step
+from .recurrent import HState
 
 try:
     from torchtune.modules import RotaryPositionalEmbeddings
@@ -17,82 +16,9 @@ except ImportError:          # the reference tolerates a missing torchtune the s
     RotaryPositionalEmbeddings = None
 
 _LAMBDA_MODES = {"positive": 0, "bounded": 1, None: 2}
-# bf16 CUDA activations take the fused element-wise kernels; False keeps the reference's sequence of
-# torch ops around the kernel for every dtype (used by the tests as the cross-check)
+# bf16 CUDA activations take the native nodes (fused element-wise kernels around the scan, csrc/host.cpp); False keeps the reference's
+# sequence of torch ops around the kernel for every dtype (used by the tests as the cross-check)
 FUSED_PREP = True
-
-
-def _ptr(t):
-    return t.data_ptr() if t is not None else None
-
-
-class HMambaCombinedFunction(torch.autograd.Function):
-    """The whole layer call for bf16 CUDA activations as one autograd node: fused element-wise
-    preparation (one pass), the chunkwise kernels, the D residual; backward in the opposite order with
-    one fused pass for every element-wise gradient (mamba_apis.py:346-366, 401-402 in the reference are
-    separate torch ops, each differentiated by autograd)."""
-
-    @staticmethod
-    def forward(ctx, x, dt, A, Bm, Cm, dl, Lp, D, dt_bias, lambda_mode, level_base, htype):
-        lib = _lib.lib()
-        Bsz, T, H, P = x.shape
-        L = dl.shape[-1]
-        rows = Bsz * T * H
-        x_, dt_, dl_ = x.contiguous(), dt.contiguous(), dl.contiguous()
-        A_, Lp_ = A.detach().float().contiguous(), Lp.detach().float().contiguous()
-        D_ = D.detach().float().contiguous() if D is not None else None
-        bias_ = dt_bias.detach().float().contiguous() if dt_bias is not None else None
-        mode = _LAMBDA_MODES[lambda_mode]
-        with torch.cuda.device(x.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            v = torch.empty_like(x_)
-            g = torch.empty(Bsz, T, H, dtype=torch.float32, device=x.device)
-            lam = torch.empty_like(dl_)
-            rc = lib.llattn_mamba2_prep_fwd(x_.data_ptr(), dt_.data_ptr(), _ptr(bias_), A_.data_ptr(), dl_.data_ptr(), Lp_.data_ptr(),
-                                            v.data_ptr(), g.data_ptr(), lam.data_ptr(), rows, H, P, L, mode, stream)
-            _lib.check(rc, "llattn_mamba2_prep_fwd")
-            kept = [] if KEEP_FORWARD_STATES else None
-            o, g_cum, _ = chunkwise_fwd(q=Cm, k=Bm, v=v, g=g, l=lam, head_first=False, level_base=level_base, htype=htype,
-                                        chunk_size=64, output_final_state=False, keep_workspace=kept)
-            if D_ is not None:
-                y_dtype = torch.promote_types(o.dtype, D.dtype)      # fp32 for an fp32 D, as x * D[...] + y gives
-                y = torch.empty(o.shape, dtype=torch.float32 if y_dtype == torch.float32 else torch.bfloat16, device=o.device)
-                rc = lib.llattn_mamba2_residual(o.data_ptr(), x_.data_ptr(), D_.data_ptr(), y.data_ptr(),
-                                                1 if y.dtype == torch.float32 else 0, rows, H, P, stream)
-                _lib.check(rc, "llattn_mamba2_residual")
-            else:
-                y = o
-        ctx.save_for_backward(x_, dt_, A_, Bm, Cm, dl_, Lp_, D_, bias_, v, g_cum, lam)
-        ctx.fwd_workspace = kept[0] if kept else None
-        ctx.meta = (mode, level_base, htype, A.dtype, Lp.dtype, D.dtype if D is not None else None,
-                    dt_bias.dtype if dt_bias is not None else None)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x_, dt_, A_, Bm, Cm, dl_, Lp_, D_, bias_, v, g_cum, lam = ctx.saved_tensors
-        mode, level_base, htype, A_dt, L_dt, D_dt, b_dt = ctx.meta
-        lib = _lib.lib()
-        Bsz, T, H, P = x_.shape
-        L = dl_.shape[-1]
-        rows = Bsz * T * H
-        dy = dy.to(torch.bfloat16).contiguous()
-        dq, dk, dv, dg, dlam = chunkwise_bwd(q=Cm, k=Bm, v=v, g=g_cum, l=lam, do=dy, head_first=False, level_base=level_base,
-                                             htype=htype, chunk_size=64, fwd_workspace=ctx.fwd_workspace)
-        ctx.fwd_workspace = None
-        with torch.cuda.device(x_.device):
-            dx = torch.empty_like(x_)
-            ddt = torch.empty_like(dt_)
-            ddl = torch.empty_like(dl_)
-            acc = torch.zeros(3 * H + H * L, dtype=torch.float32, device=x_.device)
-            dA, dbias, dD, dLp = acc[:H], acc[H:2 * H], acc[2 * H:3 * H], acc[3 * H:].view(H, L)
-            rc = lib.llattn_mamba2_prep_bwd(x_.data_ptr(), dt_.data_ptr(), _ptr(bias_), A_.data_ptr(), dl_.data_ptr(), Lp_.data_ptr(),
-                                            _ptr(D_), dv.data_ptr(), dg.data_ptr(), dlam.data_ptr(), dy.data_ptr(),
-                                            dx.data_ptr(), ddt.data_ptr(), ddl.data_ptr(), dA.data_ptr(), dbias.data_ptr(),
-                                            dLp.data_ptr(), dD.data_ptr(), rows, H, P, L, mode, torch.cuda.current_stream().cuda_stream)
-            _lib.check(rc, "llattn_mamba2_prep_bwd")
-        return (dx, ddt, dA.to(A_dt), dk.to(Bm.dtype), dq.to(Cm.dtype), ddl, dLp.to(L_dt),
-                dD.to(D_dt) if D_ is not None else None, dbias.to(b_dt) if bias_ is not None else None, None, None, None)
 
 
 class LambdaLevelMLP(torch.nn.Module):
@@ -150,62 +76,9 @@ def compute_lambda(L: torch.Tensor, dl: torch.Tensor, lambda_mode: Optional[str]
     raise ValueError
 
 
-_PARAM_DTYPES = (torch.float32, torch.bfloat16)
-
-
-def _fused_inference(tensors, params) -> bool:
-    """Whether the inference kernels take these operands: bf16 CUDA activations, fp32 or bf16 parameters, nothing to differentiate."""
-    if not all(t.dtype == torch.bfloat16 and t.is_cuda for t in tensors) or not all(p is None or p.dtype in _PARAM_DTYPES for p in params):
-        return False
-    return not torch.is_grad_enabled() or not any(t is not None and t.requires_grad for t in (*tensors, *params))
-
-
-def _prompt_is_fused(x, dt, A, B, C, dl, L, D, dt_bias, lambda_mode, level_base, htype, hstruct) -> bool:
-    return (FUSED_PREP and _fused_inference((x, dt, B, C, dl), (A, L, D, dt_bias)) and hstruct == HStruct.MAMBA2
-            and htype == HType.WEAK and level_base == 2 and lambda_mode in _LAMBDA_MODES and L.dim() == 2
-            and x.shape[-1] == 64 and B.shape[-1] in (64, 128) and dl.shape[-1] <= 32)
-
-
-def _prompt(x, dt, A, Bm, Cm, dl, Lp, D, dt_bias, mode: int, level_base: int, htype: HType):
-    """The prompt call of the layer: one pass prepares (and pads) everything the chunkwise kernels read, the chunkwise kernels, the
-    level states, one pass for the D residual."""
-    Bsz, T, H, P = x.shape
-    G, N = Bm.shape[2:]
-    L = dl.shape[-1]
-    Tp = prompt_length(T)
-    Lo = max(L, 7) if T < 64 else L
-    lib = _lib.lib()
-    with torch.no_grad(), torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream().cuda_stream
-        x_, dt_, dl_, q, k = (t.contiguous() for t in (x, dt, dl, Cm, Bm))
-        A_ = A.float().contiguous()
-        Lp_ = Lp.contiguous()
-        bf = dict(dtype=torch.bfloat16, device=x.device)
-        v = torch.empty(Bsz, Tp, H, P, **bf)
-        lam = torch.empty(Bsz, Tp, H, Lo, **bf)
-        g = torch.empty(Bsz, Tp, H, dtype=torch.float32, device=x.device)
-        qp = kp = None
-        if Tp != T:
-            qp, kp = torch.empty(Bsz, Tp, G, N, **bf), torch.empty(Bsz, Tp, G, N, **bf)
-        f32 = torch.float32
-        rc = lib.llattn_mamba2_prompt_prep(
-            x_.data_ptr(), dt_.data_ptr(), _ptr(dt_bias), dt_bias is not None and dt_bias.dtype == f32, A_.data_ptr(), dl_.data_ptr(),
-            Lp_.data_ptr(), Lp_.dtype == f32, q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), lam.data_ptr(), _ptr(qp), _ptr(kp),
-            Bsz, T, Tp, H, G, N, P, L, Lo, mode, stream)
-        _lib.check(rc, "llattn_mamba2_prompt_prep")
-        if Tp != T:
-            q, k = qp, kp
-        o, states = prompt_forward_padded(q, k, v, g, lam, T, L, level_base, htype, 64)
-        if D is not None or (Tp != T and Bsz > 1):
-            y = torch.empty(Bsz, T, H, P, dtype=f32 if D is not None and D.dtype == f32 else torch.bfloat16, device=x.device)
-            rc = lib.llattn_mamba2_prompt_residual(o.data_ptr(), x_.data_ptr(), _ptr(D), y.data_ptr(), y.dtype == f32, Bsz, T, Tp, H, P,
-                                                   stream)
-            _lib.check(rc, "llattn_mamba2_prompt_residual")
-        else:
-            y = o[:, :T]
-    state = HState.holding(states, level_base, htype, HStruct.MAMBA2)
-    state.set_counts_after(T)
-    return y, state
+def _native(lambda_mode, level_base, htype, hstruct) -> bool:
+    """Whether the native nodes cover these options (whether they take the operands, they decide themselves)."""
+    return FUSED_PREP and hstruct == HStruct.MAMBA2 and htype == HType.WEAK and level_base == 2 and lambda_mode in _LAMBDA_MODES
 
 
 def hmamba_chunk_scan_combined(
@@ -262,8 +135,12 @@ def hmamba_chunk_scan_combined(
         raise ValueError
     if return_final_states:
         # inference: outputs for the prompt and the level states to decode from (mamba_apis.py:381-399)
-        if _prompt_is_fused(x, dt, A, B, C, dl, L, D, dt_bias, lambda_mode, lambda_level_base, lambda_htype, lambda_hstruct):
-            return _prompt(x, dt, A, B, C, dl, L, D, dt_bias, _LAMBDA_MODES[lambda_mode], lambda_level_base, lambda_htype)
+        if _native(lambda_mode, lambda_level_base, lambda_htype, lambda_hstruct):
+            r = _lib.host().mamba2_prompt(x, dt, A, B, C, dl, L, D, dt_bias, _LAMBDA_MODES[lambda_mode], _lib.CHECK_STATUS)
+            if r is not None:
+                state = HState.holding(r[1], lambda_level_base, lambda_htype, HStruct.MAMBA2)
+                state.set_counts_after(x.shape[1])
+                return r[0], state
         if D is not None:
             D_residual = x * D[None, None, :, None]
         if dt_bias is not None:
@@ -277,11 +154,11 @@ def hmamba_chunk_scan_combined(
         if D is not None:
             y = y + D_residual
         return y, state
-    bf16_cuda = all(t.is_cuda and t.dtype == torch.bfloat16 for t in (x, dt, B, C, dl))
-    if (FUSED_PREP and bf16_cuda and lambda_hstruct == HStruct.MAMBA2 and lambda_htype == HType.WEAK and lambda_level_base == 2
-            and lambda_mode in _LAMBDA_MODES and x.shape[-1] % 8 == 0 and x.shape[-1] <= 256 and L.dim() == 2):
-        y = HMambaCombinedFunction.apply(x, dt, A, B, C, dl, L, D, dt_bias, lambda_mode, lambda_level_base, lambda_htype)
-        return y, None
+    if _native(lambda_mode, lambda_level_base, lambda_htype, lambda_hstruct):
+        y = _lib.host().mamba2_layer(x, dt, A, B, C, dl, L, D, dt_bias, _LAMBDA_MODES[lambda_mode], kernel.KEEP_FORWARD_STATES,
+                                     _lib.CHECK_STATUS)
+        if y is not None:
+            return y, None
     # other dtypes: the reference's own sequence of torch element-wise ops around the kernel
     if D is not None:
         D_residual = x * D[None, None, :, None]
@@ -328,6 +205,13 @@ def hselective_state_update(
         raise NotImplementedError
     if z is not None:
         raise NotImplementedError
+    if (lambda_level_fixed and lambda_level_max == state.max_num_levels and state.base == lambda_level_base == 2
+            and state.htype == lambda_htype and state.hstruct == lambda_hstruct
+            and _native(lambda_mode, lambda_level_base, lambda_htype, lambda_hstruct)):
+        y = _lib.host().mamba2_step(state.states, state.counts, x, dt, A, B, C, dl, L, D, dt_bias, _LAMBDA_MODES[lambda_mode],
+                                    bool(dt_softplus))
+        if y is not None:
+            return y, state
     if x.dim() != 3 or dt.dim() != 2 or A.dim() != 1 or B.dim() != 3 or C.dim() != 3 or dl.dim() != 3 or L.dim() != 2:
         raise ValueError
     if D is not None and D.dim() != 1:
@@ -347,13 +231,6 @@ def hselective_state_update(
         raise ValueError
     if dt_bias is not None and dt_bias.shape != (nheads,):
         raise ValueError
-    if (lambda_level_fixed and lambda_level_max == dlambda and lambda_mode in _LAMBDA_MODES and state.base == lambda_level_base
-            and state.htype == lambda_htype and state.hstruct == lambda_hstruct == HStruct.MAMBA2 and state.dtype == torch.float32
-            and _fused_inference((x, dt, B, C, dl), (A, L, D, dt_bias)) and is_level_major(state.states)):
-        y = mamba2_layer_step(state, C.contiguous(), B.contiguous(), x.contiguous(), dt.contiguous(), None, dl.contiguous(), L.contiguous(),
-                              A.float().contiguous(), D if D is None else D.contiguous(), dt_bias if dt_bias is None else dt_bias.contiguous(),
-                              _LAMBDA_MODES[lambda_mode], dt_softplus)
-        return y, state
     if D is not None:
         D_residual = x * D[None, :, None]
     if dt_bias is not None:
@@ -372,83 +249,6 @@ def hselective_state_update(
     if D is not None:
         out = out + D_residual
     return out, state
-
-
-class HMambaMixerFunction(torch.autograd.Function):
-    """Everything of the mixer between its two projections as one autograd node: convolution, preparation, chunkwise kernels, D
-    residual and gated norm, on the rows of the input projection in place (mamba_apis.py:186-259 in the reference)."""
-
-    @staticmethod
-    def forward(ctx, zx, conv_w, conv_b, dt_bias, A, Lp, D, norm_w, eps, G, mode, level_base, htype):
-        lib = _lib.lib()
-        Bsz, T, W = zx.shape
-        H, L = Lp.shape
-        dim = H * 64
-        N = (W - 2 * dim - H - H * L) // (2 * G)
-        f32 = torch.float32
-        zx, conv_w, Lp, norm_w = (t.contiguous() for t in (zx, conv_w, Lp, norm_w))
-        conv_b, dt_bias, D = (t if t is None else t.contiguous() for t in (conv_b, dt_bias, D))
-        A_ = A.detach().float().contiguous()
-        is32 = lambda t: t is not None and t.dtype == f32
-        with torch.cuda.device(zx.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            bf = dict(dtype=torch.bfloat16, device=zx.device)
-            x, v = torch.empty(Bsz, T, H, 64, **bf), torch.empty(Bsz, T, H, 64, **bf)
-            k, q = torch.empty(Bsz, T, G, N, **bf), torch.empty(Bsz, T, G, N, **bf)
-            g = torch.empty(Bsz, T, H, dtype=f32, device=zx.device)
-            lam = torch.empty(Bsz, T, H, L, **bf)
-            rc = lib.llattn_mixer_prep_fwd(zx.data_ptr(), conv_w.data_ptr(), is32(conv_w), _ptr(conv_b), is32(conv_b), _ptr(dt_bias),
-                                           is32(dt_bias), A_.data_ptr(), Lp.data_ptr(), is32(Lp), x.data_ptr(), v.data_ptr(),
-                                           k.data_ptr(), q.data_ptr(), g.data_ptr(), lam.data_ptr(), Bsz, T, H, G, N, L, mode, stream)
-            _lib.check(rc, "llattn_mixer_prep_fwd")
-            kept = [] if KEEP_FORWARD_STATES else None
-            o, g_cum, _ = chunkwise_fwd(q=q, k=k, v=v, g=g, l=lam, head_first=False, level_base=level_base, htype=htype, chunk_size=64,
-                                        output_final_state=False, keep_workspace=kept)
-            out = torch.empty(Bsz, T, dim, **bf)
-            rstd = torch.empty(Bsz, T, dtype=f32, device=zx.device)
-            rc = lib.llattn_mixer_norm_fwd(o.data_ptr(), x.data_ptr(), _ptr(D), is32(D), zx.data_ptr(), W, norm_w.data_ptr(), is32(norm_w),
-                                           out.data_ptr(), rstd.data_ptr(), Bsz * T, H, eps, stream)
-            _lib.check(rc, "llattn_mixer_norm_fwd")
-        ctx.save_for_backward(zx, conv_w, conv_b, dt_bias, A_, Lp, D, norm_w, x, v, k, q, g_cum, lam, o, rstd)
-        ctx.fwd_workspace = kept[0] if kept else None
-        ctx.meta = (G, N, mode, level_base, htype, A.dtype)
-        return out
-
-    @staticmethod
-    def backward(ctx, dn):
-        zx, conv_w, conv_b, dt_bias, A_, Lp, D, norm_w, x, v, k, q, g_cum, lam, o, rstd = ctx.saved_tensors
-        G, N, mode, level_base, htype, A_dt = ctx.meta
-        lib = _lib.lib()
-        Bsz, T, W = zx.shape
-        H, L = Lp.shape
-        dim = H * 64
-        f32 = torch.float32
-        is32 = lambda t: t is not None and t.dtype == f32
-        dn = dn.to(torch.bfloat16).contiguous()
-        with torch.cuda.device(zx.device):
-            stream = torch.cuda.current_stream().cuda_stream
-            dzx = torch.empty_like(zx)
-            dy = torch.empty_like(x)
-            # sums over tokens: conv taps and bias, norm weight, A, dt_bias, D, L
-            ch = dim + 2 * G * N
-            acc = torch.zeros(ch * 5 + dim + 3 * H + H * L, dtype=f32, device=zx.device)
-            dcw, dcb, dnw, dA, dbias, dD, dLp = acc.split([ch * 4, ch, dim, H, H, H, H * L])
-            rc = lib.llattn_mixer_norm_bwd(o.data_ptr(), x.data_ptr(), _ptr(D), is32(D), zx.data_ptr(), W, norm_w.data_ptr(), is32(norm_w),
-                                           dn.data_ptr(), rstd.data_ptr(), dy.data_ptr(), dzx.data_ptr(), dnw.data_ptr(), dD.data_ptr(),
-                                           Bsz * T, H, stream)
-            _lib.check(rc, "llattn_mixer_norm_bwd")
-            dq, dk, dv, dg, dlam = chunkwise_bwd(q=q, k=k, v=v, g=g_cum, l=lam, do=dy, head_first=False, level_base=level_base,
-                                                 htype=htype, chunk_size=64, fwd_workspace=ctx.fwd_workspace)
-            ctx.fwd_workspace = None
-            rc = lib.llattn_mixer_prep_bwd(zx.data_ptr(), conv_w.data_ptr(), is32(conv_w), _ptr(conv_b), is32(conv_b), _ptr(dt_bias),
-                                           is32(dt_bias), A_.data_ptr(), Lp.data_ptr(), is32(Lp), _ptr(D), is32(D), dv.data_ptr(),
-                                           dy.data_ptr(), dq.data_ptr(), dk.data_ptr(), dg.data_ptr(), dlam.data_ptr(), dzx.data_ptr(),
-                                           dcw.data_ptr(), dcb.data_ptr(), dA.data_ptr(), dbias.data_ptr(), dLp.data_ptr(),
-                                           Bsz, T, H, G, N, L, mode, stream)
-            _lib.check(rc, "llattn_mixer_prep_bwd")
-        as_ = lambda d, p: None if p is None else d.view(p.shape).to(p.dtype)
-        return (dzx, as_(dcw, conv_w), as_(dcb, conv_b), as_(dbias, dt_bias), dA.to(A_dt), as_(dLp, Lp), as_(dD, D), as_(dnw, norm_w),
-                None, None, None, None, None)
 
 
 def _causal_conv1d_silu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> torch.Tensor:
@@ -529,14 +329,12 @@ def hmamba_split_conv1d_scan_combined(
         raise ValueError
     if dt_bias.shape != (nheads,) or A.shape != (nheads,) or L.shape != (nheads, dlambda):
         raise ValueError
-    params = (conv1d_weight, conv1d_bias, dt_bias, L, D, rmsnorm_weight)
-    if (FUSED_PREP and zxbcdtdl.is_cuda and zxbcdtdl.dtype == torch.bfloat16 and all(p is None or p.dtype in _PARAM_DTYPES for p in params)
-            and headdim == 64 and dstate in (64, 128) and nheads <= 128 and conv1d_weight.shape == (dim + 2 * ngroups * dstate, 4)
-            and rmsnorm_weight.shape == (dim,) and lambda_hstruct == HStruct.MAMBA2 and lambda_htype == HType.WEAK
-            and lambda_level_base == 2 and lambda_mode in _LAMBDA_MODES and lambda_level_fixed and lambda_level_max == dlambda):
-        y = HMambaMixerFunction.apply(zxbcdtdl, conv1d_weight, conv1d_bias, dt_bias, A, L, D, rmsnorm_weight, rmsnorm_eps, ngroups,
-                                      _LAMBDA_MODES[lambda_mode], lambda_level_base, lambda_htype)
-        return torch.nn.functional.linear(y, outproj_weight.to(y.dtype), outproj_bias.to(y.dtype) if outproj_bias is not None else None)
+    if headdim == 64 and lambda_level_fixed and lambda_level_max == dlambda and _native(lambda_mode, lambda_level_base, lambda_htype, lambda_hstruct):
+        # everything between the two projections as one node, on the rows of the first one in place
+        y = _lib.host().mamba2_mixer(zxbcdtdl, conv1d_weight, conv1d_bias, dt_bias, A, L, D, rmsnorm_weight, rmsnorm_eps, ngroups,
+                                     _LAMBDA_MODES[lambda_mode], kernel.KEEP_FORWARD_STATES, _lib.CHECK_STATUS)
+        if y is not None:
+            return torch.nn.functional.linear(y, outproj_weight.to(y.dtype), outproj_bias.to(y.dtype) if outproj_bias is not None else None)
     z, xBC, dt, dl = torch.split(zxbcdtdl, [dim, dim + 2 * ngroups * dstate, nheads, nheads * dlambda], dim=-1)
     xBC = _causal_conv1d_silu(xBC.transpose(1, 2), conv1d_weight, conv1d_bias).transpose(1, 2)
     x, Bm, Cm = torch.split(xBC, [dim, ngroups * dstate, ngroups * dstate], dim=-1)
