@@ -214,12 +214,13 @@ int llattn_gdn_layer_step(float* states, const void* q, const void* k, const voi
  *   mamba2_prompt_residual: y (B,T,H,P) = o (B,Tp,H,P) + D x; y and D are fp32 (y_is_f32 != 0) or bf16; D may be NULL
  *   mamba2_prompt_states: the level states after T tokens, level-major, every level written; k, v, g are Tp tokens long.  With the
  *     workspace of the forward call on them (may be NULL) the levels that hold whole 512-token segments are sums of its summaries.
- *   gdn_prompt_prep: l2norm of q (scaled) and k, one per head, K_out >= K columns wide (at most 128), Tp tokens long, and, each where
- *     its pointer is given, v (as consecutive slices (B,Tp,H,v_slice)), beta and g, lambda (times lambda_mul unless 0, L_out columns)
- *   gdn_prefill_slice: llattn_gdn_prefill writing the inter-chunk levels of value columns first_col .. first_col + V - 1 into
- *     level-major states (B,H,state_levels,state_rows,state_cols); other levels are left alone
- *   gdn_prompt_states: advances those levels by the tokens of the last chunk and writes the levels inside it, so that every level of
- *     the v_cols columns from first_col is as of token T - 1; kn (B,Tp,H,128), v (B,Tp,H,v_cols); T is in the last 64 tokens of Tp */
+ *   gdn_prompt_prep: a value head of V columns as `rep` heads of V / rep columns that share everything else ((B,T,H,V) is (B,T,H rep,V / rep)
+ *     in memory).  One row per part: l2norm of q (scaled) and k, K_out >= K columns wide (at most 128), and, each where its pointer is given,
+ *     v, beta and g, lambda (times lambda_mul unless 0, L_out columns), all Tp tokens long.  q, k have G groups of H / G heads.
+ *   gdn_prefill_parts: llattn_gdn_prefill on H = heads x rep parts, the inter-chunk levels written into level-major states
+ *     (B,H / rep,state_levels,state_rows,rep V); other levels are left alone
+ *   gdn_prompt_states: advances those levels by the tokens of the last chunk and writes the levels inside it, so that every level is as of
+ *     token T - 1; kn (B,Tp,H,128), v (B,Tp,H,V), states (B,H / rep,L,K,rep V); T is in the last 64 tokens of Tp */
 int llattn_pad_tokens(int n, const void* const* src, void* const* dst, const int* src_bytes, const int* dst_bytes, int B, int T, int Tp,
                       void* stream);
 int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
@@ -232,14 +233,13 @@ int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, fl
                                 size_t fwd_workspace_bytes, int B, int T, int Tp, int H, int G, int K, int V, int L, void* stream);
 int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                            void* qn, void* kn, void* v_pad, void* beta_pad, float* g_pad, void* lambda_pad,
-                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int v_slice, int L, int L_out, float scale,
+                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int rep, int L, int L_out, float scale,
                            float lambda_mul, void* stream);
-int llattn_gdn_prefill_slice(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
-                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int state_cols, int first_col,
-                             int state_levels, void* workspace, size_t workspace_bytes,
-                             int B, int T, int H, int K, int V, int L, void* stream);
+int llattn_gdn_prefill_parts(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
+                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int rep, int state_levels,
+                             void* workspace, size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream);
 int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, const float* g, float* states, int B, int T, int Tp, int H,
-                             int K, int V, int v_cols, int first_col, int L, void* stream);
+                             int K, int V, int rep, int L, void* stream);
 
 /* Log-linear Gated DeltaNet forward.  Replaces hattention.chunkwise_hgdn.chunkwise_fwd
  * (hattention/chunkwise_hgdn.py:566-788) with output_final_state=False.  q and k are per head,
@@ -340,11 +340,14 @@ int llattn_gdn_bwd_kept_bf16dv(const void* q, const void* k, const void* v, cons
 int llattn_l2norm_fwd(const void* x, void* y, long rows, int D, float scale, void* stream);
 int llattn_l2norm_bwd(const void* x, const float* dy, void* dx, long rows, int D, float scale, void* stream);
 
-/* The gradients that leave a Gated DeltaNet backward, in one pass: gq, gk (rows,K) bf16 = l2norm backward of dq, dk (rows,K_in) fp32 at raw
- * q, k (q with `scale`; K_in >= K, at most 128: padded keys), gbeta (rows) and glambda (rows,L) bf16; lambda_mul != 0: glambda is
- * rounded, multiplied and rounded again, as the reference's lambda / scale differentiates (gated_delta_rule_apis.py:65-70). */
-int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const float* dk, const float* dbeta, const float* dlambda, void* gq,
-                        void* gk, void* gbeta, void* glambda, long rows, int K, int K_in, int L, float scale, float lambda_mul, void* stream);
+/* The gradients that leave a Gated DeltaNet backward, in one pass: gq, gk (rows,K) bf16 = l2norm backward of dq, dk (K_in >= K columns, at
+ * most 128: padded keys) at raw q, k (q with `scale`), gbeta (rows) and glambda (rows,L) bf16; lambda_mul != 0: glambda is
+ * rounded, multiplied and rounded again, as the reference's lambda / scale differentiates (gated_delta_rule_apis.py:65-70).  The fp32
+ * inputs have `rep` rows for each row of the results, which are summed (parts of a wide value head); gg (rows) takes the sums of dg where
+ * dg is given. */
+int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const float* dk, const float* dbeta, const float* dlambda,
+                        const float* dg, void* gq, void* gk, void* gbeta, void* glambda, float* gg, long rows, int rep, int K, int K_in, int L,
+                        float scale, float lambda_mul, void* stream);
 
 /* Diagnostic: one 128 x N x kred bf16 tensor-core product (tcgen05.mma, accumulator in tensor
  * memory) per operand-layout combination used by the kernels: mode 0: D = A B^T with A [128][kred],

@@ -301,18 +301,19 @@ static int gdn_fwd_impl(const void* q, const void* k, const void* v, const void*
                         int B, int T, int H, int K, int V, int L, void* stream, bool keep,
                         const llattn::GdnStateOut& final_states = llattn::GdnStateOut{});
 
-int llattn_gdn_prefill_slice(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
-                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int state_cols, int first_col,
-                             int state_levels, void* workspace, size_t workspace_bytes,
-                             int B, int T, int H, int K, int V, int L, void* stream) {
+int llattn_gdn_prefill_parts(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
+                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int rep, int state_levels,
+                             void* workspace, size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream) {
     if (!states) return LLATTN_ERR_NULL;
-    if (state_rows <= 0 || state_rows > K || first_col < 0 || first_col + V > state_cols || state_levels > L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (state_rows <= 0 || state_rows > K || rep <= 0 || H % rep != 0 || state_levels > L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     llattn::GdnStateOut out;
-    out.p = states + first_col;
+    out.p = states;
     out.rows = state_rows;
+    out.rep = rep;
+    out.part = V;
     out.col = 1;
-    out.row = state_cols;
-    out.level = (long)state_rows * state_cols;
+    out.row = (long)rep * V;
+    out.level = (long)state_rows * out.row;
     out.bh = out.level * state_levels;
     return gdn_fwd_impl(q, k, v, beta, g, lambda, o, g_cum, Aw, Au, workspace, workspace_bytes, B, T, H, K, V, L, stream, false, out);
 }

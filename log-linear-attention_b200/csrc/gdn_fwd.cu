@@ -496,7 +496,8 @@ __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const GdnParams p) {
             // of 2^lv chunks for each set bit lv of c (the binary-indexed tree as it stands before this chunk); the
             // caller steps the last chunk's tokens through the decode kernel, which fills levels 0..6.
             const GdnStateOut& fs = p.final_states;
-            float* dst = fs.p + ((long)b * p.H + h) * fs.bh + INTRA_LEVELS * fs.level;
+            const long bh = (long)b * p.H + h;
+            float* dst = fs.p + bh / fs.rep * fs.bh + bh % fs.rep * fs.part + INTRA_LEVELS * fs.level;
 #pragma unroll
             for (int lv = 0; lv < GDN_MAXLEV; ++lv) {
                 if (lv < nlev && ((c >> lv) & 1)) {

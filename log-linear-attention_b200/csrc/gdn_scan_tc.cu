@@ -355,7 +355,8 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
             // of 2^lv chunks for each set bit lv of c (the binary-indexed tree as it stands before this chunk); the
             // caller steps the last chunk's tokens through the decode kernel, which fills levels 0..6.
             const GdnStateOut& fs = p.final_states;
-            float* dst = fs.p + ((long)b * p.H + h) * fs.bh + row * fs.row + INTRA_LEVELS * fs.level;
+            const long bh = (long)b * p.H + h;
+            float* dst = fs.p + bh / fs.rep * fs.bh + bh % fs.rep * fs.part + row * fs.row + INTRA_LEVELS * fs.level;
 #pragma unroll 1
             for (uint32_t m = live; m; m &= m - 1) {
                 const int lv = __ffs(m) - 1;

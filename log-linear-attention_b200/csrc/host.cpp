@@ -28,7 +28,7 @@ using torch::autograd::variable_list;
     F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mixer_prep_fwd)            \
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
     F(llattn_gdn_fwd_workspace_bytes) F(llattn_gdn_fwd_keep_workspace_bytes) F(llattn_gdn_fwd) F(llattn_gdn_fwd_keep)                \
-    F(llattn_gdn_prefill_slice) F(llattn_gdn_prompt_states) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
+    F(llattn_gdn_prefill_parts) F(llattn_gdn_prompt_states) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
     F(llattn_gdn_bwd_kept_workspace_bytes) F(llattn_gdn_bwd_kept_bf16dv) F(llattn_gdn_grad_out) F(llattn_workspace_status)
 
 struct Library {
@@ -398,20 +398,22 @@ py::object mamba2_mixer(const Tensor& zx, const Tensor& cw, const Maybe& cb_, co
 }
 
 // ------------------------------------------------------------------------------------------ Gated DeltaNet
-constexpr int GDN_K = 128, GDN_SLICE = 128, GDN_V_MAX = 384;     // key width and widest value head of one kernel call; widest head
+constexpr int GDN_K = 128, GDN_V_MAX = 384;      // key width of the kernels; widest value head
 
 struct GdnInputs {
-    Tensor qn, kn, v, b, g, l;       // v: slices of at most 128 columns, one behind the other
-    int B, T, H, G, K, V, L;
-    int slices() const { return (V + GDN_SLICE - 1) / GDN_SLICE; }
-    int width(int i) const { return std::min(GDN_SLICE, V - i * GDN_SLICE); }
-    Tensor slice(const Tensor& all, int i) const {       // slice i of a tensor of slices
-        const int64_t n = (int64_t)B * T * H;
-        return all.view({-1}).narrow(0, n * i * GDN_SLICE, n * width(i)).view({B, T, H, width(i)});
+    Tensor qn, kn, v, b, g, l;       // one row per part of a value head
+    int B, T, H, G, K, V, L;         // of the caller's tensors (T and L as padded)
+    // A value head is `rep` heads of `width` columns that share q, k, beta, g and lambda: the delta rule acts on every value column
+    // independently.  The kernels take 64 or 128 columns a head; all parts run in one launch.
+    int rep, width;
+    int heads() const { return H * rep; }
+    void split() {
+        width = V % 128 == 0 ? 128 : 64;
+        rep = V / width;
     }
 };
 
-// l2norm of q and k, lambda times its factor, and (T < Tp) padding; b, g and unscaled lambda are used as they are when nothing pads
+// l2norm of q and k, lambda times its factor, the parts of wide heads and (T < Tp) padding; what none of these changes is used as it is
 GdnInputs gdn_prepare(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, int T, int Tp, int Lo, double scale,
                       double lam_mul, void* stream) {
     GdnInputs a;
@@ -421,22 +423,22 @@ GdnInputs gdn_prepare(const Tensor& q, const Tensor& k, const Tensor& v, const T
     a.K = q.size(3);
     a.H = v.size(2);
     a.V = v.size(3);
-    a.L = l.size(3);
-    const int B = a.B, H = a.H;
-    const bool pad = Tp != T, own_l = pad || lam_mul != 0.0 || Lo != a.L, own_v = pad || a.V > GDN_SLICE;
+    a.L = Lo;
+    a.split();
+    const int B = a.B, H = a.heads(), L = l.size(3);
+    const bool pad = Tp != T, own = pad || a.rep > 1, own_l = own || lam_mul != 0.0 || Lo != L;
     const Tensor qk = empty({2, B, Tp, H, GDN_K}, at::kBFloat16, q);
     a.qn = qk.select(0, 0);
     a.kn = qk.select(0, 1);
-    a.v = own_v ? empty({(int64_t)B * Tp * H * a.V}, at::kBFloat16, q) : v;
-    a.b = pad ? empty({B, Tp, H}, at::kBFloat16, q) : b;
-    a.g = pad ? empty({B, Tp, H}, at::kFloat, q) : g;
+    a.v = pad ? empty({B, Tp, H, a.width}, at::kBFloat16, q) : v;
+    a.b = own ? empty({B, Tp, H}, at::kBFloat16, q) : b;
+    a.g = own ? empty({B, Tp, H}, at::kFloat, q) : g;
     a.l = own_l ? empty({B, Tp, H, Lo}, at::kBFloat16, q) : l;
     check(lib.llattn_gdn_prompt_prep(q.data_ptr(), k.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g), l.data_ptr(), a.qn.data_ptr(), a.kn.data_ptr(),
-                                     own_v ? a.v.data_ptr() : nullptr, pad ? a.b.data_ptr() : nullptr, pad ? fptr(a.g) : nullptr,
-                                     own_l ? a.l.data_ptr() : nullptr, B, T, Tp, H, a.G, a.K, GDN_K, a.V, GDN_SLICE, a.L, Lo, (float)scale, (float)lam_mul,
+                                     pad ? a.v.data_ptr() : nullptr, own ? a.b.data_ptr() : nullptr, own ? fptr(a.g) : nullptr,
+                                     own_l ? a.l.data_ptr() : nullptr, B, T, Tp, a.H, a.G, a.K, GDN_K, a.V, a.rep, L, Lo, (float)scale, (float)lam_mul,
                                      stream),
           "llattn_gdn_prompt_prep");
-    a.L = Lo;
     return a;
 }
 
@@ -457,38 +459,26 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
         const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), b_ = b.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
         const int T = q.size(1);
         GdnInputs a = gdn_prepare(q_, k_, v_, b_, g_, l_, T, T, l.size(3), scale, lam_mul, on.stream);
-        const int B = a.B, H = a.H, n = a.slices();
-        size_t total = 0;
-        for (int i = 0; i < n; ++i) total += lib.llattn_gdn_fwd_keep_workspace_bytes(B, T, H, GDN_K, a.width(i), a.L);
-        const bool keep = ctx != nullptr && (int64_t)total <= keep_bytes;
-        const Tensor g_cum = at::empty_like(g_), A = empty({2, B, T, H, 64}, at::kBFloat16, q), Aw = A.select(0, 0), Au = A.select(0, 1);
-        std::vector<Tensor> parts, kept;
-        for (int i = 0; i < n; ++i) {
-            const int V = a.width(i);
-            const size_t bytes = (keep ? lib.llattn_gdn_fwd_keep_workspace_bytes : lib.llattn_gdn_fwd_workspace_bytes)(B, T, H, GDN_K, V, a.L);
-            const Tensor ws = empty({(int64_t)bytes}, at::kByte, q), o = empty({B, T, H, V}, at::kBFloat16, q), vs = n > 1 ? a.slice(a.v, i) : a.v;
-            check((keep ? lib.llattn_gdn_fwd_keep : lib.llattn_gdn_fwd)(a.qn.data_ptr(), a.kn.data_ptr(), vs.data_ptr(), a.b.data_ptr(), fptr(a.g),
-                                                                       a.l.data_ptr(), o.data_ptr(), fptr(g_cum), Aw.data_ptr(), Au.data_ptr(),
-                                                                       ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
-                  "llattn_gdn_fwd");
-            if (status) check_status(ws, on.stream, "llattn_gdn_fwd");
-            parts.push_back(o);
-            if (keep) kept.push_back(ws);
-        }
+        const int B = a.B, H = a.heads(), V = a.width;
+        const size_t keep_need = lib.llattn_gdn_fwd_keep_workspace_bytes(B, T, H, GDN_K, V, a.L);
+        const bool keep = ctx != nullptr && (int64_t)keep_need <= keep_bytes;
+        const Tensor g_cum = at::empty_like(a.g), A = empty({2, B, T, H, 64}, at::kBFloat16, q), Aw = A.select(0, 0), Au = A.select(0, 1);
+        const size_t bytes = keep ? keep_need : lib.llattn_gdn_fwd_workspace_bytes(B, T, H, GDN_K, V, a.L);
+        const Tensor ws = empty({(int64_t)bytes}, at::kByte, q), o = at::empty_like(v_);
+        check((keep ? lib.llattn_gdn_fwd_keep : lib.llattn_gdn_fwd)(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(),
+                                                                   o.data_ptr(), fptr(g_cum), Aw.data_ptr(), Au.data_ptr(), ws.data_ptr(), bytes, B, T, H,
+                                                                   GDN_K, V, a.L, on.stream),
+              "llattn_gdn_fwd");
+        if (status) check_status(ws, on.stream, "llattn_gdn_fwd");
         if (ctx) {
-            variable_list save = {q_, k_, a.v, b_, g_cum, a.l, Aw, Au};
-            if (keep) {
-                save.push_back(a.qn);
-                save.push_back(a.kn);
-                for (const Tensor& w : kept) save.push_back(w);
-            }
+            variable_list save = {q_, k_, v_, a.b, g_cum, a.l, Aw, Au};
+            if (keep) save.insert(save.end(), {a.qn, a.kn, ws});
             ctx->save_for_backward(save);
-            ctx->saved_data["V"] = (int64_t)a.V;
             ctx->saved_data["scale"] = scale;
             ctx->saved_data["lam_mul"] = lam_mul;
             ctx->saved_data["status"] = status;
         }
-        return n == 1 ? parts[0] : at::cat(parts, -1);
+        return o;
     }
     static variable_list backward(AutogradContext* ctx, variable_list d) {
         const auto s = ctx->get_saved_variables();
@@ -501,9 +491,10 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
         a.T = q.size(1);
         a.H = q.size(2);
         a.K = q.size(3);
-        a.V = (int)ctx->saved_data["V"].toInt();
+        a.V = v.size(3);
         a.L = l.size(3);
-        const int B = a.B, T = a.T, H = a.H, n = a.slices();
+        a.split();
+        const int B = a.B, T = a.T, H = a.heads(), V = a.width;
         Tensor qn, kn;
         if (kept) {
             qn = s[8];
@@ -513,51 +504,38 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
             qn = qk.select(0, 0);
             kn = qk.select(0, 1);
             check(lib.llattn_gdn_prompt_prep(q.data_ptr(), k.data_ptr(), nullptr, nullptr, nullptr, nullptr, qn.data_ptr(), kn.data_ptr(), nullptr, nullptr,
-                                             nullptr, nullptr, B, T, T, H, H, a.K, GDN_K, 64, GDN_SLICE, a.L, a.L, (float)scale, 0.f, on.stream),
+                                             nullptr, nullptr, B, T, T, a.H, a.H, a.K, GDN_K, a.V, a.rep, a.L, a.L, (float)scale, 0.f, on.stream),
                   "llattn_gdn_prompt_prep");
         }
         const Tensor d_o = d[0].to(at::kBFloat16).contiguous();
-        // fp32 gradients of the inputs that all slices share: dq | dk | dbeta | dlambda in one buffer, and dg, which is handed on as it is
-        const int64_t rows = (int64_t)B * T * H, per = rows * (2 * GDN_K + 1 + a.L);
-        Tensor sum, dg;
-        std::vector<Tensor> dvs;
-        for (int i = 0; i < n; ++i) {
-            const int V = a.width(i);
-            const Tensor vs = n > 1 ? a.slice(v, i) : v, dos = n > 1 ? d_o.narrow(3, i * GDN_SLICE, V).contiguous() : d_o;
-            const Tensor out = empty({per}, at::kFloat, q), dgi = empty({B, T, H}, at::kFloat, q);
-            float *dq = fptr(out), *dk = dq + rows * GDN_K, *db = dk + rows * GDN_K, *dl = db + rows;
-            const size_t bytes = (kept ? lib.llattn_gdn_bwd_kept_workspace_bytes : lib.llattn_gdn_bwd_workspace_bytes)(B, T, H, GDN_K, V, a.L);
-            const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
-            Tensor dv = empty({B, T, H, V}, kept ? at::kBFloat16 : at::kFloat, q);
-            if (kept) {
-                const Tensor& fws = s[10 + i];
-                check(lib.llattn_gdn_bwd_kept_bf16dv(qn.data_ptr(), kn.data_ptr(), vs.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(),
-                                                     Au.data_ptr(), dos.data_ptr(), dq, dk, dv.data_ptr(), db, fptr(dgi), dl, fws.data_ptr(), fws.numel(),
-                                                     ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
-                      "llattn_gdn_bwd_kept_bf16dv");
-            } else {
-                check(lib.llattn_gdn_bwd(qn.data_ptr(), kn.data_ptr(), vs.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(), Au.data_ptr(),
-                                         dos.data_ptr(), dq, dk, fptr(dv), db, fptr(dgi), dl, ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
-                      "llattn_gdn_bwd");
-                dv = dv.to(at::kBFloat16);
-            }
-            if (status) check_status(ws, on.stream, "llattn_gdn_bwd");
-            dvs.push_back(dv);
-            if (i == 0) {
-                sum = out;
-                dg = dgi;
-            } else {
-                sum.add_(out);
-                dg.add_(dgi);
-            }
+        // fp32 gradients of what the parts of a head share: dq | dk | dbeta | dlambda in one buffer, and dg, which is handed on as it is
+        // where a head has one part
+        const int64_t rows = (int64_t)B * T * a.H, prows = rows * a.rep;
+        const Tensor out = empty({prows * (2 * GDN_K + 1 + a.L)}, at::kFloat, q), dgp = empty({B, T, H}, at::kFloat, q);
+        float *dq = fptr(out), *dk = dq + prows * GDN_K, *db = dk + prows * GDN_K, *dl = db + prows;
+        const size_t bytes = (kept ? lib.llattn_gdn_bwd_kept_workspace_bytes : lib.llattn_gdn_bwd_workspace_bytes)(B, T, H, GDN_K, V, a.L);
+        const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
+        Tensor dv = empty(v.sizes(), kept ? at::kBFloat16 : at::kFloat, q);
+        if (kept) {
+            const Tensor& fws = s[10];
+            check(lib.llattn_gdn_bwd_kept_bf16dv(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(),
+                                                 Au.data_ptr(), d_o.data_ptr(), dq, dk, dv.data_ptr(), db, fptr(dgp), dl, fws.data_ptr(), fws.numel(),
+                                                 ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
+                  "llattn_gdn_bwd_kept_bf16dv");
+        } else {
+            check(lib.llattn_gdn_bwd(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(), Au.data_ptr(),
+                                     d_o.data_ptr(), dq, dk, fptr(dv), db, fptr(dgp), dl, ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
+                  "llattn_gdn_bwd");
+            dv = dv.to(at::kBFloat16);
         }
-        const Tensor gqk = empty({2, B, T, H, a.K}, at::kBFloat16, q), gq = gqk.select(0, 0), gk = gqk.select(0, 1);
-        const Tensor gb = at::empty_like(b), gl = at::empty_like(l);
-        float *dq = fptr(sum), *dk = dq + rows * GDN_K, *db = dk + rows * GDN_K, *dl = db + rows;
-        check(lib.llattn_gdn_grad_out(q.data_ptr(), k.data_ptr(), dq, dk, db, dl, gq.data_ptr(), gk.data_ptr(), gb.data_ptr(), gl.data_ptr(), rows, a.K, GDN_K,
-                                      a.L, (float)scale, (float)lam_mul, on.stream),
+        if (status) check_status(ws, on.stream, "llattn_gdn_bwd");
+        const Tensor gqk = empty({2, B, T, a.H, a.K}, at::kBFloat16, q), gq = gqk.select(0, 0), gk = gqk.select(0, 1);
+        const Tensor gb = empty({B, T, a.H}, at::kBFloat16, q), gl = empty({B, T, a.H, a.L}, at::kBFloat16, q);
+        const Tensor gg = a.rep > 1 ? empty({B, T, a.H}, at::kFloat, q) : dgp;
+        check(lib.llattn_gdn_grad_out(q.data_ptr(), k.data_ptr(), dq, dk, db, dl, a.rep > 1 ? fptr(dgp) : nullptr, gq.data_ptr(), gk.data_ptr(), gb.data_ptr(),
+                                      gl.data_ptr(), fptr(gg), rows, a.rep, a.K, GDN_K, a.L, (float)scale, (float)lam_mul, on.stream),
               "llattn_gdn_grad_out");
-        return {gq, gk, n == 1 ? dvs[0] : at::cat(dvs, -1), gb, dg, gl, Tensor(), Tensor(), Tensor(), Tensor()};
+        return {gq, gk, dv, gb, gg, gl, Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
@@ -589,26 +567,19 @@ py::object gdn_prompt(const Tensor& q, const Tensor& k, const Tensor& v, const T
         On on(q);
         GdnInputs a = gdn_prepare(q.contiguous(), k.contiguous(), v.contiguous(), b.contiguous(), g.contiguous(), l.contiguous(), T, Tp, Lo, scale, lam_mul,
                                   on.stream);
-        const int B = a.B, H = a.H, K = a.K, n = a.slices();
-        states = empty({B, H, L, K, a.V}, at::kFloat, q);
-        const Tensor g_cum = at::empty_like(a.g), A = empty({2, B, Tp, H, 64}, at::kBFloat16, q);
-        std::vector<Tensor> parts;
-        for (int i = 0; i < n; ++i) {
-            const int V = a.width(i), c0 = i * GDN_SLICE;
-            const Tensor vs = a.V > GDN_SLICE || Tp != T ? a.slice(a.v, i) : a.v, out = empty({B, Tp, H, V}, at::kBFloat16, q);
-            const size_t bytes = lib.llattn_gdn_fwd_workspace_bytes(B, Tp, H, GDN_K, V, Lo);
-            const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
-            check(lib.llattn_gdn_prefill_slice(a.qn.data_ptr(), a.kn.data_ptr(), vs.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(), out.data_ptr(),
-                                               fptr(g_cum), A.select(0, 0).data_ptr(), A.select(0, 1).data_ptr(), fptr(states), K, a.V, c0, L,
-                                               ws.data_ptr(), bytes, B, Tp, H, GDN_K, V, Lo, on.stream),
-                  "llattn_gdn_prefill_slice");
-            check(lib.llattn_gdn_prompt_states(a.kn.data_ptr(), vs.data_ptr(), a.b.data_ptr(), fptr(a.g), fptr(states), B, T, Tp, H, K, a.V, V, c0, L,
-                                               on.stream),
-                  "llattn_gdn_prompt_states");
-            if (status) check_status(ws, on.stream, "llattn_gdn_prefill_slice");
-            parts.push_back(Tp == T ? out : out.narrow(1, 0, T));
-        }
-        o = n == 1 ? parts[0].contiguous() : at::cat(parts, -1);
+        const int B = a.B, H = a.heads(), K = a.K, V = a.width;
+        states = empty({B, a.H, L, K, a.V}, at::kFloat, q);
+        const Tensor g_cum = at::empty_like(a.g), A = empty({2, B, Tp, H, 64}, at::kBFloat16, q), out = empty({B, Tp, a.H, a.V}, at::kBFloat16, q);
+        const size_t bytes = lib.llattn_gdn_fwd_workspace_bytes(B, Tp, H, GDN_K, V, Lo);
+        const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
+        check(lib.llattn_gdn_prefill_parts(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(), out.data_ptr(),
+                                           fptr(g_cum), A.select(0, 0).data_ptr(), A.select(0, 1).data_ptr(), fptr(states), K, a.rep, L, ws.data_ptr(), bytes,
+                                           B, Tp, H, GDN_K, V, Lo, on.stream),
+              "llattn_gdn_prefill_parts");
+        check(lib.llattn_gdn_prompt_states(a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), fptr(states), B, T, Tp, H, K, V, a.rep, L, on.stream),
+              "llattn_gdn_prompt_states");
+        if (status) check_status(ws, on.stream, "llattn_gdn_prefill_parts");
+        o = Tp == T ? out : out.narrow(1, 0, T).contiguous();
         states = states.permute({0, 1, 3, 4, 2});
     }
     return py::make_tuple(o, states);

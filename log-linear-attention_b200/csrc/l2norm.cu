@@ -94,8 +94,10 @@ __global__ void __launch_bounds__(256) l2norm_bwd_kernel(const __nv_bfloat16* __
 struct GdnGradOut {
     const __nv_bfloat16 *q, *k;       // (rows,K)
     const float *dq, *dk;             // (rows,K_in)
-    const float *db, *dl;             // (rows), (rows,L)
+    const float *db, *dl, *dg;        // (rows), (rows,L), (rows)
     __nv_bfloat16 *gq, *gk, *gb, *gl;
+    float* gg;                        // (rows), with dg
+    int rep;                          // the fp32 gradients have `rep` rows for each of these (parts of a wide value head), summed here
     long rows;
     int K, K_in, L;
     float scale, lam_mul;
@@ -112,8 +114,13 @@ __global__ void __launch_bounds__(256) gdn_grad_out_kernel(const __grid_constant
         float ss = 0.f, dot = 0.f;
         if (act) {
             const uint4 raw = *reinterpret_cast<const uint4*>((w == 0 ? a.q : a.k) + row * a.K + lane * 8);
-            const float* d = (w == 0 ? a.dq : a.dk) + row * a.K_in + lane * 8;
-            const float4 g0 = *reinterpret_cast<const float4*>(d), g1 = *reinterpret_cast<const float4*>(d + 4);
+            const float* d = (w == 0 ? a.dq : a.dk) + row * a.rep * a.K_in + lane * 8;
+            float4 g0 = *reinterpret_cast<const float4*>(d), g1 = *reinterpret_cast<const float4*>(d + 4);
+            for (int r = 1; r < a.rep; ++r) {
+                const float4 e0 = *reinterpret_cast<const float4*>(d + (long)r * a.K_in), e1 = *reinterpret_cast<const float4*>(d + (long)r * a.K_in + 4);
+                g0.x += e0.x; g0.y += e0.y; g0.z += e0.z; g0.w += e0.w;
+                g1.x += e1.x; g1.y += e1.y; g1.z += e1.z; g1.w += e1.w;
+            }
             const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
             g[0] = g0.x * scale; g[1] = g0.y * scale; g[2] = g0.z * scale; g[3] = g0.w * scale;
             g[4] = g1.x * scale; g[5] = g1.y * scale; g[6] = g1.z * scale; g[7] = g1.w * scale;
@@ -144,9 +151,19 @@ __global__ void __launch_bounds__(256) gdn_grad_out_kernel(const __grid_constant
         }
     }
     if (!have) return;
-    if (lane == 15) a.gb[row] = __float2bfloat16(a.db[row]);
+    if (lane >= 14) {
+        const float* d = (lane == 15 ? a.db : a.dg);
+        if (d != nullptr) {
+            float x = d[row * a.rep];
+            for (int r = 1; r < a.rep; ++r) x += d[row * a.rep + r];
+            if (lane == 15) a.gb[row] = __float2bfloat16(x);
+            else a.gg[row] = x;
+        }
+    }
     for (int j = lane; j < a.L; j += 16) {
-        __nv_bfloat16 x = __float2bfloat16(a.dl[row * a.L + j]);
+        float s = a.dl[row * a.rep * a.L + j];
+        for (int r = 1; r < a.rep; ++r) s += a.dl[(row * a.rep + r) * a.L + j];
+        __nv_bfloat16 x = __float2bfloat16(s);
         if (a.lam_mul != 0.f) x = __float2bfloat16(__bfloat162float(x) * a.lam_mul);
         a.gl[row * a.L + j] = x;
     }
@@ -156,12 +173,13 @@ __global__ void __launch_bounds__(256) gdn_grad_out_kernel(const __grid_constant
 
 extern "C" {
 
-int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const float* dk, const float* dbeta, const float* dlambda, void* gq,
-                        void* gk, void* gbeta, void* glambda, long rows, int K, int K_in, int L, float scale, float lambda_mul, void* stream) {
-    if (rows <= 0 || K <= 0 || K % 8 != 0 || K_in < K || K_in % 8 != 0 || K_in > 128 || L <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (!q || !k || !dq || !dk || !dbeta || !dlambda || !gq || !gk || !gbeta || !glambda) return LLATTN_ERR_NULL;
+int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const float* dk, const float* dbeta, const float* dlambda,
+                        const float* dg, void* gq, void* gk, void* gbeta, void* glambda, float* gg, long rows, int rep, int K, int K_in, int L,
+                        float scale, float lambda_mul, void* stream) {
+    if (rows <= 0 || rep <= 0 || K <= 0 || K % 8 != 0 || K_in < K || K_in % 8 != 0 || K_in > 128 || L <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!q || !k || !dq || !dk || !dbeta || !dlambda || !gq || !gk || !gbeta || !glambda || (dg && !gg)) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
-    llattn::GdnGradOut a{(const bf*)q, (const bf*)k, dq, dk, dbeta, dlambda, (bf*)gq, (bf*)gk, (bf*)gbeta, (bf*)glambda, rows, K, K_in, L, scale,
+    llattn::GdnGradOut a{(const bf*)q, (const bf*)k, dq, dk, dbeta, dlambda, dg, (bf*)gq, (bf*)gk, (bf*)gbeta, (bf*)glambda, gg, rep, rows, K, K_in, L, scale,
                          lambda_mul};
     llattn::gdn_grad_out_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, (cudaStream_t)stream>>>(a);
     LLATTN_LAUNCHED();

@@ -12,11 +12,12 @@ constexpr int GDN_VS = 32;          // V columns per CTA of the sequential scans
 constexpr int GDN_MAXLEV = 8;       // inter-chunk levels (T up to 64 * 2^8 = 16384)
 
 // Where the level states before the last chunk go (prefill hand-off): element (b*H + h, level, row, column) at
-// p[bh * .bh + level * .level + row * .row + column * .col]; rows beyond `rows` (padding of narrow keys) are not written.
+// p[(b*H + h) / rep * .bh + (b*H + h) % rep * .part + level * .level + row * .row + column * .col] (rep heads are the parts of one wide
+// value head); rows beyond `rows` (padding of narrow keys) are not written.
 struct GdnStateOut {
     float* p = nullptr;
-    long bh = 0, level = 0, row = 0, col = 0;
-    int rows = 0;
+    long bh = 0, part = 0, level = 0, row = 0, col = 0;
+    int rows = 0, rep = 1;
 };
 
 struct GdnParams {

@@ -140,20 +140,21 @@ struct GdnPrepArgs {
     const bf16* beta;        // (B,T,H)
     const float* g;          // (B,T,H)
     const bf16* l;           // (B,T,H,L)
-    bf16 *qn, *kn;           // (B,Tp,H,Ko)
-    bf16 *vp, *bp;           // (B,Tp,H,V) in slices of v_slice columns, (B,Tp,H)
-    float* gp;               // (B,Tp,H)
-    bf16* lp;                // (B,Tp,H,Lo)
-    int B, T, Tp, H, G, K, Ko, V, v_slice, L, Lo;
+    // results, one row per part of a head: a value head of V columns is `rep` heads of V / rep columns that share q, k, beta, g, lambda
+    bf16 *qn, *kn;           // (B,Tp,H rep,Ko)
+    bf16 *vp, *bp;           // (B,Tp,H rep,V / rep), (B,Tp,H rep)
+    float* gp;               // (B,Tp,H rep)
+    bf16* lp;                // (B,Tp,H rep,Lo)
+    int B, T, Tp, H, G, K, Ko, V, rep, L, Lo;
     float scale, lam_mul;    // lam_mul = 0: lambda as it is
 };
 
 __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_constant__ GdnPrepArgs a) {
     const int lane = threadIdx.x & 15;
     const unsigned row = blockIdx.x * 16u + (threadIdx.x >> 4);
-    const unsigned rows = (unsigned)a.B * a.Tp * a.H;
+    const unsigned heads = a.H * a.rep, rows = (unsigned)a.B * a.Tp * heads;
     const bool have = row < rows;
-    const unsigned h = row % a.H, tok = row / a.H, t = tok % a.Tp, b = tok / a.Tp;
+    const unsigned hp = row % heads, h = hp / a.rep, part = hp % a.rep, tok = row / heads, t = tok % a.Tp, b = tok / a.Tp;
     const bool in = have && t < (unsigned)a.T;
     const long tr = in ? (long)b * a.T + t : 0;
     const long src = tr * a.H + h, qsrc = tr * a.G + h / (a.H / a.G);
@@ -189,13 +190,14 @@ __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_const
             *reinterpret_cast<uint4*>((w ? a.kn : a.qn) + (long)row * a.Ko + lane * 8) = out;
         }
     }
-    if (a.vp)
-        for (int c = lane * 8; c < a.V; c += 128) {
-            const int s0 = c / a.v_slice * a.v_slice, width = min(a.v_slice, a.V - s0);
+    if (a.vp) {
+        const int width = a.V / a.rep;
+        for (int c = lane * 8; c < width; c += 128) {
             uint4 w = make_uint4(0, 0, 0, 0);
-            if (in) w = *reinterpret_cast<const uint4*>(a.v + src * a.V + c);
-            *reinterpret_cast<uint4*>(a.vp + (long)rows * s0 + (long)row * width + c - s0) = w;
+            if (in) w = *reinterpret_cast<const uint4*>(a.v + src * a.V + part * width + c);
+            *reinterpret_cast<uint4*>(a.vp + (long)row * width + c) = w;
         }
+    }
     if (a.lp)
         for (int j = lane; j < a.Lo; j += 16) {
             float x = 0.f;
@@ -216,12 +218,12 @@ __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_const
 // independent of the others: level 0 is the last token alone, level j + 1 (for each set bit j of the last token's position in
 // the chunk) starts from zero at the first of its 2^j tokens, takes their writes and then the transitions of the tokens behind
 // them, and the levels of earlier chunks take the transitions of all.  fp32 throughout, as the decode kernel steps.
-// One warp holds four value columns of one level (lane: KR = Ko / 32 state rows), so a token is four dot products over the
+// Level-major states of value heads that are processed as `rep` parts of Vs columns.  One warp holds four value columns of one level (lane: KR = Ko / 32 state rows), so a token is four dot products over the
 // lanes and no barrier; grid (B*H, levels, V / 32).
 constexpr int TAIL_KD = 128;
 __global__ void __launch_bounds__(256) gdn_tail_states_kernel(const bf16* __restrict__ kn, const bf16* __restrict__ v, const bf16* __restrict__ beta,
                                                               const float* __restrict__ g, float* __restrict__ states, int T, int Tp, int H,
-                                                              int K, int V, int Vs, int first_col, int L) {
+                                                              int K, int Vs, int rep, int L) {
     constexpr int KR = TAIL_KD / 32;
     __shared__ __align__(16) bf16 sK[CH * TAIL_KD];
     __shared__ float sV[CH][33];
@@ -231,7 +233,9 @@ __global__ void __launch_bounds__(256) gdn_tail_states_kernel(const bf16* __rest
     const int h = blockIdx.x % H, b = blockIdx.x / H;
     const int m = T - 1, c0 = m & ~(CH - 1), n = m - c0 + 1;
     const int col = blockIdx.z * 32 + warp * 4;              // first of this warp's columns in the slice of Vs columns
-    float* S = states + (((long)b * H + h) * L + lev) * (long)K * V + first_col + col;
+    const int V = Vs * rep;                                  // H counts parts of value heads, rep of them in one
+    const long bh = (long)b * H + h;
+    float* S = states + (bh / rep * L + lev) * (long)K * V + bh % rep * Vs + col;
     // tokens [s0, s1) of the chunk write to this level; [s1, n) only advance it
     int s0 = -1, s1 = 0;
     if (lev == 0) {
@@ -368,33 +372,31 @@ int llattn_pad_tokens(int n, const void* const* src, void* const* dst, const int
 
 int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                            void* qn, void* kn, void* v_pad, void* beta_pad, float* g_pad, void* lambda_pad,
-                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int v_slice, int L, int L_out, float scale,
+                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int rep, int L, int L_out, float scale,
                            float lambda_mul, void* stream) {
     if (B <= 0 || T <= 0 || Tp < T || H <= 0 || G <= 0 || H % G != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (K <= 0 || K % 8 != 0 || K_out < K || K_out > 128 || K_out % 8 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (V <= 0 || V % 8 != 0 || v_slice <= 0 || v_slice % 8 != 0 || L <= 0 || L_out < L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if ((long)B * Tp * H > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (V <= 0 || rep <= 0 || V % (8 * rep) != 0 || L <= 0 || L_out < L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if ((long)B * Tp * H * rep > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!q || !k || !qn || !kn || (v_pad && !v) || (lambda_pad && !lambda) || (g_pad && (!g || !beta || !beta_pad))) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
     llattn::GdnPrepArgs a{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, (const bf*)lambda, (bf*)qn, (bf*)kn, (bf*)v_pad,
-                          (bf*)beta_pad, g_pad, (bf*)lambda_pad, B, T, Tp, H, G, K, K_out, V, v_slice, L, L_out, scale, lambda_mul};
-    const unsigned grid = (unsigned)(((long)B * Tp * H + 15) / 16);
+                          (bf*)beta_pad, g_pad, (bf*)lambda_pad, B, T, Tp, H, G, K, K_out, V, rep, L, L_out, scale, lambda_mul};
+    const unsigned grid = (unsigned)(((long)B * Tp * H * rep + 15) / 16);
     llattn::gdn_prompt_prep_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
 int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, const float* g, float* states, int B, int T, int Tp, int H,
-                             int K, int V, int v_cols, int first_col, int L, void* stream) {
-    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || K <= 0 || K > llattn::TAIL_KD) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (v_cols <= 0 || v_cols % 32 != 0 || first_col < 0 || first_col % 4 != 0 || first_col + v_cols > V || V % 4 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (L <= 0 || L > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+                             int K, int V, int rep, int L, void* stream) {
+    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || rep <= 0 || H % rep != 0 || K <= 0 || K > llattn::TAIL_KD) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (V <= 0 || V % 32 != 0 || L <= 0 || L > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (T > 1 && L < 1 + (32 - __builtin_clz((unsigned)(T - 1) | 1u))) return LLATTN_ERR_TOO_FEW_LEVELS;
     if (!kn || !v || !beta || !g || !states) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
-    dim3 grid(B * H, L, v_cols / 32);
-    llattn::gdn_tail_states_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const bf*)kn, (const bf*)v, (const bf*)beta, g, states, T, Tp, H, K, V,
-                                                                          v_cols, first_col, L);
+    dim3 grid(B * H, L, V / 32);
+    llattn::gdn_tail_states_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const bf*)kn, (const bf*)v, (const bf*)beta, g, states, T, Tp, H, K, V, rep, L);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

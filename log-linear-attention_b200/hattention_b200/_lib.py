@@ -74,16 +74,7 @@ def lib():
         "llattn_mamba2_layer_step": [_P] * 8 + [_I, _P, _I, _P, _I] + [_P] * 2 + [_I] * 6 + [_U] + [_I] * 4 + [_P],
         "llattn_gdn_layer_step": [_P] * 8 + [_I] * 6 + [_U, _I, _I, _F, _F, _I, _P],
         "llattn_pad_tokens": [_I] + [_P] * 4 + [_I] * 3 + [_P],
-        "llattn_mamba2_prompt_prep": [_P] * 3 + [_I] + [_P] * 3 + [_I] + [_P] * 7 + [_I] * 10 + [_P],
-        "llattn_mamba2_prompt_residual": [_P] * 4 + [_I] * 6 + [_P],
         "llattn_mamba2_prompt_states": [_P] * 5 + [ctypes.c_size_t] + [_I] * 8 + [_P],
-        "llattn_gdn_prompt_prep": [_P] * 12 + [_I] * 11 + [_F, _F, _P],
-        "llattn_gdn_prefill_slice": [_P] * 11 + [_I] * 4 + [_P, ctypes.c_size_t] + [_I] * 6 + [_P],
-        "llattn_gdn_prompt_states": [_P] * 5 + [_I] * 9 + [_P],
-        "llattn_mixer_prep_fwd": [_P] * 2 + [_I, _P, _I, _P, _I] + [_P] * 2 + [_I] + [_P] * 6 + [_I] * 7 + [_P],
-        "llattn_mixer_prep_bwd": [_P] * 2 + [_I, _P, _I, _P, _I] + [_P] * 2 + [_I, _P, _I] + [_P] * 12 + [_I] * 7 + [_P],
-        "llattn_mixer_norm_fwd": [_P] * 3 + [_I, _P, _I, _P, _I] + [_P] * 2 + [ctypes.c_long, _I, _F, _P],
-        "llattn_mixer_norm_bwd": [_P] * 3 + [_I, _P, _I, _P, _I] + [_P] * 6 + [ctypes.c_long, _I, _P],
     }.items():
         fn = getattr(L, name)
         fn.restype, fn.argtypes = _I, args
