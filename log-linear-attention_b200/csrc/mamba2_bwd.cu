@@ -22,6 +22,7 @@
 // chunkwise.py:1583-1591).
 #include "llattn_common.cuh"
 #include "llattn_mamba2.h"
+#include "side_stream.h"
 
 namespace llattn {
 
@@ -1121,17 +1122,24 @@ __global__ void m2_cast_bf16_kernel(const float* __restrict__ src, bf16* __restr
 // host side
 // ------------------------------------------------------------------------------------------
 template <int KD, int VD, int MLOW>
-static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
+static int launch_fwdorder(const Mamba2Params& p, bool use_tc, cudaStream_t stream) {
+    if (use_tc) return mamba2_bwd1_tc_launch(p, stream);
+    cudaError_t e;
+    auto kern = m2_bwd_fwdorder_kernel<KD, VD, MLOW>;
+    if ((e = allow_smem(kern, Bwd1Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
+    kern<<<p.B * p.H * p.NS, 256, Bwd1Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+template <int KD, int VD, int MLOW>
+static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStream_t stream) {
     cudaError_t e;
     constexpr int SEG = 1 << MLOW;
     const int KV = KD * VD;
     if (p.NS > 1) {
-        // forward high-level states: recomputed unless the caller kept the forward call's workspace
-        int rc = p.reuse_states ? 0 : mamba2_fwd_states_dispatch(p, stream);
-        if (rc != 0) return rc;
         const bool hi_tc = (KD == 128 && VD == 64 && (p.NT % 2) == 0 && p.L <= 20 && p.LH <= 10 && g_use_tensor_core_path.load());
         if (hi_tc) {
-            rc = mamba2_hi_bwd_tc_launch(p, stream);
+            const int rc = mamba2_hi_bwd_tc_launch(p, stream);
             if (rc != 0) return rc;
         } else {
             {
@@ -1152,24 +1160,36 @@ static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
             else { m2_seg_dscan_kernel<MAX_LH_B><<<grid, 256, 0, stream>>>(p, KV); LLATTN_LAUNCHED(); }
         }
     }
-    const bool use_tc = (KD == 128 && VD == 64 && (p.NT % 2) == 0 && p.L <= 20 && g_use_tensor_core_path.load());
-    if (use_tc) {
-        int rc = mamba2_bwd1_tc_launch(p, stream);
-        if (rc != 0) return rc;
-    } else {
-        auto kern = m2_bwd_fwdorder_kernel<KD, VD, MLOW>;
-        if ((e = allow_smem(kern, Bwd1Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
-        kern<<<p.B * p.H * p.NS, 256, Bwd1Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
-    }
-    if (use_tc) {
-        int rc = mamba2_bwd2_tc_launch(p, stream);
-        if (rc != 0) return rc;
-    } else {
-        auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;
-        if ((e = allow_smem(kern, Bwd2Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
-        kern<<<p.B * p.H * p.NS, 256, Bwd2Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
-    }
+    if (use_tc) return mamba2_bwd2_tc_launch(p, stream);
+    auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;
+    if ((e = allow_smem(kern, Bwd2Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
+    kern<<<p.B * p.H * p.NS, 256, Bwd2Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
+}
+
+template <int KD, int VD, int MLOW>
+static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
+    int rc;
+    if (p.NS > 1 && !p.reuse_states) {
+        // forward high-level states: recomputed unless the caller kept the forward call's workspace
+        if ((rc = mamba2_fwd_states_dispatch(p, stream)) != 0) return rc;
+    }
+    const bool use_tc = (KD == 128 && VD == 64 && (p.NT % 2) == 0 && p.L <= 20 && g_use_tensor_core_path.load());
+    // The forward-order pass and the chain high levels -> reverse-order pass only meet in the accumulators they add to.  A pass has one CTA
+    // per (batch, head, segment) and one fits on an SM: below three waves of them the two run side by side (two of 64 CTAs each then
+    // take the time of one), beyond that each fills the chip by itself.
+    if ((long)p.B * p.H * p.NS < 3 * 148) {
+        if (SideStream* side = SideStream::get(stream)) {
+            cudaError_t e;
+            if ((e = side->fork(stream)) != cudaSuccess) return (int)e;
+            rc = launch_fwdorder<KD, VD, MLOW>(p, use_tc, side->stream());
+            const int rc2 = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream);
+            if ((e = side->join(stream)) != cudaSuccess) return (int)e;
+            return rc != 0 ? rc : rc2;
+        }
+    }
+    if ((rc = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream)) != 0) return rc;
+    return launch_fwdorder<KD, VD, MLOW>(p, use_tc, stream);
 }
 
 int mamba2_bwd_dispatch(Mamba2Params p, cudaStream_t stream) {

@@ -33,9 +33,9 @@ struct PrepArgs {
 
 // Both passes: a group of LPR lanes owns one head and walks `run` tokens, eight columns a lane.  What depends on the (token, head)
 // alone is evaluated once by the group, each lane for one of LPR tokens, and the parameter sums stay in registers over the run.  The
-// loads of a token are not fetched ahead: few registers and many warps keep more bytes in flight than two tokens a thread did
-// (B = 2, T = 16384, 32 heads, L = 15: backward 321 us with a row per group, a shared-memory atomic per lambda column and a token
-// per thread before, 212 us with two tokens in flight and a thread per lambda column).
+// loads of a token are not fetched ahead: few registers and many warps keep more bytes in flight (B = 2, T = 16384, 32 heads, L = 15:
+// backward 321 us with a row per group, a shared-memory atomic per lambda column and a token per thread before; 130 us as it is; 136 us
+// with the next token in flight, 212 us with two and a thread per lambda column).
 template <int LPR>
 __global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_constant__ PrepArgs a) {
     constexpr int U = 2;
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_consta
     const int at = blockIdx.x - lam_grid;
     const int t0 = at / a.row_blocks * a.run, t1 = min(a.tokens, t0 + a.run);
     const int lane = threadIdx.x % LPR;
-    const int h = at % a.row_blocks * (256 / LPR) + threadIdx.x / LPR;
+    const int h = at % a.row_blocks * ((int)blockDim.x / LPR) + threadIdx.x / LPR;
     if (h >= a.H) return;                      // whole groups
     const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u) << (threadIdx.x & 31 & ~(LPR - 1));
     const bool act = lane * 8 < a.P;
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256, 4) m2_prep_bwd_kernel(const __grid_consta
     const int at = blockIdx.x - lam_grid;
     const int t0 = at / a.row_blocks * a.run, t1 = min(a.tokens, t0 + a.run);
     const int lane = threadIdx.x % LPR;
-    const int h = at % a.row_blocks * (256 / LPR) + threadIdx.x / LPR;
+    const int h = at % a.row_blocks * ((int)blockDim.x / LPR) + threadIdx.x / LPR;
     if (h >= a.H) return;
     const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1u) << (threadIdx.x & 31 & ~(LPR - 1));
     const bool act = lane * 8 < a.P;
@@ -194,17 +194,20 @@ static int prep_check(long rows, int H, int P, int L, int mode) {
 }
 
 // Grid of a pass: runs long enough that the sums at their end are cheap, as many as fill the chip
-static unsigned prep_grid(llattn::PrepArgs& a, long rows, int H, int P, int L, int mode, bool backward) {
+static unsigned prep_grid(llattn::PrepArgs& a, long rows, int H, int P, int L, int mode, bool backward, int& threads) {
     a.H = H; a.P = P; a.L = L; a.mode = mode;
     a.tokens = (int)(rows / H);
     a.lpr = llattn::lanes_per_row(P);
-    a.row_blocks = (H * a.lpr + 255) / 256;
+    // few heads: smaller CTAs rather than idle threads
+    const int want = (H * a.lpr + 31) / 32 * 32;
+    threads = want < 64 ? 64 : want > 256 ? 256 : want;
+    a.row_blocks = (H * a.lpr + threads - 1) / threads;
     a.lam8 = H * L % 8 == 0;
-    a.lam_blocks = (H * L / (a.lam8 ? 8 : 1) + 255) / 256;
+    a.lam_blocks = (H * L / (a.lam8 ? 8 : 1) + threads - 1) / threads;
     a.run = 64;
-    while (a.run > 8 && (long)a.row_blocks * ((a.tokens + a.run - 1) / a.run) < 148 * 8) a.run /= 2;
+    while (a.run > (backward ? 8 : 4) && (long)a.row_blocks * ((a.tokens + a.run - 1) / a.run) * threads < 148 * 6 * 256) a.run /= 2;
     // forward: eight tokens a thread
-    const int groups = H * L / (a.lam8 ? 8 : 1), per = groups < 256 ? 256 / groups : 1;
+    const int groups = H * L / (a.lam8 ? 8 : 1), per = groups < threads ? threads / groups : 1;
     a.lam_runs = backward ? llattn::lambda_runs(a.tokens, a.lam_blocks) : (a.tokens + 8 * per - 1) / (8 * per);
     return (unsigned)(a.row_blocks * ((a.tokens + a.run - 1) / a.run) + a.lam_blocks * a.lam_runs);
 }
@@ -221,11 +224,12 @@ int llattn_mamba2_layer_prep_fwd(const void* x, const void* dt_raw, const void* 
     a.x = (const bf*)x; a.dt_raw = (const bf*)dt_raw; a.dl = (const bf*)dl; a.dt_bias = dt_bias; a.A = A; a.Lp = Lp;
     a.bias_f32 = bias_is_f32; a.lp_f32 = lp_is_f32;
     a.v = (bf*)v; a.lam = (bf*)lambda; a.g = g;
-    const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, false);
-    if (a.lpr == 4) llattn::m2_prep_fwd_kernel<4><<<grid, 256, 0, st>>>(a);
-    else if (a.lpr == 8) llattn::m2_prep_fwd_kernel<8><<<grid, 256, 0, st>>>(a);
-    else if (a.lpr == 16) llattn::m2_prep_fwd_kernel<16><<<grid, 256, 0, st>>>(a);
-    else llattn::m2_prep_fwd_kernel<32><<<grid, 256, 0, st>>>(a);
+    int threads;
+    const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, false, threads);
+    if (a.lpr == 4) llattn::m2_prep_fwd_kernel<4><<<grid, threads, 0, st>>>(a);
+    else if (a.lpr == 8) llattn::m2_prep_fwd_kernel<8><<<grid, threads, 0, st>>>(a);
+    else if (a.lpr == 16) llattn::m2_prep_fwd_kernel<16><<<grid, threads, 0, st>>>(a);
+    else llattn::m2_prep_fwd_kernel<32><<<grid, threads, 0, st>>>(a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -251,11 +255,12 @@ int llattn_mamba2_layer_prep_bwd(const void* x, const void* dt_raw, const void* 
     a.bias_f32 = bias_is_f32; a.lp_f32 = lp_is_f32; a.d_f32 = d_is_f32;
     a.dv = (const bf*)dv; a.dg = dg; a.dlam = dlambda; a.dy = (const bf*)dy;
     a.dx = (bf*)dx; a.ddt = (bf*)ddt; a.ddl = (bf*)ddl; a.dA = dA; a.dbias = dt_bias ? dbias : nullptr; a.dLp = dLp; a.dD = dD;
-    const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, true);
-    if (a.lpr == 4) llattn::m2_prep_bwd_kernel<4><<<grid, 256, 0, st>>>(a);
-    else if (a.lpr == 8) llattn::m2_prep_bwd_kernel<8><<<grid, 256, 0, st>>>(a);
-    else if (a.lpr == 16) llattn::m2_prep_bwd_kernel<16><<<grid, 256, 0, st>>>(a);
-    else llattn::m2_prep_bwd_kernel<32><<<grid, 256, 0, st>>>(a);
+    int threads;
+    const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, true, threads);
+    if (a.lpr == 4) llattn::m2_prep_bwd_kernel<4><<<grid, threads, 0, st>>>(a);
+    else if (a.lpr == 8) llattn::m2_prep_bwd_kernel<8><<<grid, threads, 0, st>>>(a);
+    else if (a.lpr == 16) llattn::m2_prep_bwd_kernel<16><<<grid, threads, 0, st>>>(a);
+    else llattn::m2_prep_bwd_kernel<32><<<grid, threads, 0, st>>>(a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

@@ -19,14 +19,10 @@
 
 namespace llattn {
 
-// LM: level-major states (B,H,L,K,V), of tensors that are Tp >= T tokens long, and with the segment summaries of the forward
-// call on the same tensors (seg_F, seg_D; null when there is one segment) for the levels that hold whole segments: the sum over
-// a bucket of 2^j segments is then an element-wise pass over 2^j summaries instead of 2^(j+3) products of 64 tokens.
-template <int KD, int VD, bool LM>
+template <int KD, int VD>
 __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v,
                                                                     const float* __restrict__ g, float* __restrict__ states,
-                                                                    const float* __restrict__ seg_F, const float* __restrict__ seg_D,
-                                                                    int B, int T, int Tp, int H, int G, int L) {
+                                                                    int B, int T, int H, int G, int L) {
     constexpr int LDK = KD + PAD, LDV = VD + PAD;
     constexpr int MT = KD / 128;                         // 16-row tiles of the K x V result per warp (8 warps)
     static_assert(KD % 128 == 0 || KD == 64, "K rows are split over the warps");
@@ -48,49 +44,14 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         s0 = (m >> lev) << lev;                          // tokens taken by the higher set bits
         s1 = s0 + (1 << (lev - 1));
     }
-    float* out = states + ((long)(b * H + h) * KD * VD) * L + (LM ? (long)lev * KD * VD : (long)lev);
+    float* out = states + ((long)(b * H + h) * KD * VD) * L + lev;
     if (s1 == s0) {
-        if (LM) {
-            for (int e = tid * 4; e < KD * VD; e += 1024) *reinterpret_cast<float4*>(out + e) = make_float4(0.f, 0.f, 0.f, 0.f);
-        } else {
-            for (int e = tid; e < KD * VD; e += 256) out[(long)e * L] = 0.f;
-        }
-        return;
-    }
-    constexpr int SEG = 512;
-    if (LM && seg_F != nullptr && s1 - s0 >= SEG) {
-        // after the bucket: whole segments up to the one of the last token, then that segment's tokens up to the last one
-        const int r0 = s0 / SEG, r1 = s1 / SEG, rl = m / SEG, NS = (Tp + SEG - 1) / SEG;
-        const float* D = seg_D + (long)(b * H + h) * NS;
-        const float* F = seg_F + (long)(b * H + h) * NS * KD * VD;
-        float part = 0.f;
-        for (int r = r1 + tid; r < rl; r += 256) part += D[r];
-        for (int t = rl * SEG + tid; t <= m; t += 256) part += g[((long)b * Tp + t) * H + h];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
-        if (lane == 0) sRed[warp] = part;
-        __syncthreads();
-        float after = 0.f;
-        for (int w = 0; w < 8; ++w) after += sRed[w];
-        float4 acc[KD * VD / 1024];
-#pragma unroll
-        for (int i = 0; i < KD * VD / 1024; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int r = r1 - 1; r >= r0; --r) {
-            const float w = fexp(after);
-#pragma unroll
-            for (int i = 0; i < KD * VD / 1024; ++i) {
-                const float4 f = *reinterpret_cast<const float4*>(F + (long)r * KD * VD + i * 1024 + tid * 4);
-                acc[i].x += w * f.x; acc[i].y += w * f.y; acc[i].z += w * f.z; acc[i].w += w * f.w;
-            }
-            after += D[r];
-        }
-#pragma unroll
-        for (int i = 0; i < KD * VD / 1024; ++i) *reinterpret_cast<float4*>(out + i * 1024 + tid * 4) = acc[i];
+        for (int e = tid; e < KD * VD; e += 256) out[(long)e * L] = 0.f;
         return;
     }
     // decay from the end of the bucket to the last token: sum_{r = s1 .. m} g_r
     float part = 0.f;
-    for (int r = s1 + tid; r <= m; r += 256) part += g[((long)b * Tp + r) * H + h];
+    for (int r = s1 + tid; r <= m; r += 256) part += g[((long)b * T + r) * H + h];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
     if (lane == 0) sRed[warp] = part;
@@ -111,8 +72,8 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         // in-tile decay: token a + i gets exp(after + sum_{r = a+i+1 .. e1-1} g_r)
         if (warp == 0) {
             const int i0 = CH - 1 - 2 * lane, i1 = CH - 2 - 2 * lane;      // reversed order
-            float x0 = (i0 + 1 < n) ? g[((long)b * Tp + a + i0 + 1) * H + h] : 0.f;
-            float x1 = (i1 + 1 < n) ? g[((long)b * Tp + a + i1 + 1) * H + h] : 0.f;
+            float x0 = (i0 + 1 < n) ? g[((long)b * T + a + i0 + 1) * H + h] : 0.f;
+            float x1 = (i1 + 1 < n) ? g[((long)b * T + a + i1 + 1) * H + h] : 0.f;
             warp_cumsum64(x0, x1, lane);
             sDec[i0] = (i0 < n) ? fexp(after + x0) : 0.f;
             sDec[i1] = (i1 < n) ? fexp(after + x1) : 0.f;
@@ -120,7 +81,7 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         for (int e = tid; e < CH * (KD / 8); e += 256) {
             const int i = e / (KD / 8), c8 = (e % (KD / 8)) * 8;
             uint4 x = make_uint4(0, 0, 0, 0);
-            if (i < n) x = *reinterpret_cast<const uint4*>(k + (((long)b * Tp + a + i) * G + grp) * KD + c8);
+            if (i < n) x = *reinterpret_cast<const uint4*>(k + (((long)b * T + a + i) * G + grp) * KD + c8);
             *reinterpret_cast<uint4*>(sK + i * LDK + c8) = x;
         }
         __syncthreads();
@@ -128,7 +89,7 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
             const int i = e / (VD / 8), c8 = (e % (VD / 8)) * 8;
             uint4 x = make_uint4(0, 0, 0, 0);
             if (i < n) {
-                x = *reinterpret_cast<const uint4*>(v + (((long)b * Tp + a + i) * H + h) * VD + c8);
+                x = *reinterpret_cast<const uint4*>(v + (((long)b * T + a + i) * H + h) * VD + c8);
                 const float d = sDec[i];
                 uint32_t* xw = reinterpret_cast<uint32_t*>(&x);
 #pragma unroll
@@ -145,7 +106,7 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
         float tile = 0.f;
         if (warp == 0) {
             float x = 0.f;
-            for (int i = lane; i < n; i += 32) x += g[((long)b * Tp + a + i) * H + h];
+            for (int i = lane; i < n; i += 32) x += g[((long)b * T + a + i) * H + h];
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
             if (lane == 0) sRed[0] = x;
@@ -160,16 +121,167 @@ __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* 
 #pragma unroll
             for (int nt = 0; nt < VD / 8; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; e += 2) {
-                    const int row = warp * 16 * MTW + mt * 16 + lr + (e >> 1) * 8, col = nt * 8 + lc2;
-                    if (LM) {
-                        *reinterpret_cast<float2*>(out + row * VD + col) = make_float2(acc[mt][nt][e], acc[mt][nt][e + 1]);
-                    } else {
-                        out[((long)row * VD + col) * L] = acc[mt][nt][e];
-                        out[((long)row * VD + col + 1) * L] = acc[mt][nt][e + 1];
-                    }
+                for (int e = 0; e < 4; ++e) {
+                    const int row = warp * 16 * MTW + mt * 16 + lr + (e >> 1) * 8, col = nt * 8 + lc2 + (e & 1);
+                    out[((long)row * VD + col) * L] = acc[mt][nt][e];
                 }
     }
+}
+
+// The same states level-major (B,H,L,K,V), of tensors that are Tp >= T tokens long.  One CTA per (batch, head, level).
+// A bucket is walked in blocks of at most 256 tokens from its end: the decays of a block come from one scan over its 256 values of g, and
+// its 64-token tiles are copied two deep, so that a tile costs one product behind one barrier.  (A tile that fetched its own decays and
+// loaded k, then v, cost three dependent trips to memory: 24 us for a 1000-token prompt of 48 heads, most of it the four tiles of the level
+// that holds 256 tokens.)  With the segment summaries of the forward call on the same tensors (seg_F, seg_D; null when there is one
+// segment) a level of 2^j segments is an element-wise pass over 2^j summaries instead of 2^(j+3) products.
+template <int KD>
+struct PromptStateSmem {
+    static constexpr int LDK = KD + PAD, LDV = 64 + PAD;
+    static constexpr size_t k_off = 0, v_off = 2ull * CH * LDK * 2, dec_off = v_off + 2ull * CH * LDV * 2, red_off = dec_off + 256 * 4, total = red_off + 64;
+};
+
+template <int KD>
+__global__ void __launch_bounds__(256) mamba2_prompt_state_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v, const float* __restrict__ g,
+                                                                  float* __restrict__ states, const float* __restrict__ seg_F,
+                                                                  const float* __restrict__ seg_D, int T, int Tp, int H, int G, int L) {
+    using SM = PromptStateSmem<KD>;
+    constexpr int VD = 64, LDK = SM::LDK, LDV = SM::LDV, KV = KD * VD, SEG = 512;
+    constexpr int MT = KD / 64, NPW = VD / 32;           // a warp: 16 MT rows x 32 columns (4 x 2 warps)
+    extern __shared__ __align__(16) unsigned char smem[];
+    bf16* sK = reinterpret_cast<bf16*>(smem + SM::k_off);
+    bf16* sV = reinterpret_cast<bf16*>(smem + SM::v_off);
+    float* sDec = reinterpret_cast<float*>(smem + SM::dec_off);
+    float* sRed = reinterpret_cast<float*>(smem + SM::red_off);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int lev = blockIdx.y, h = blockIdx.x % H, b = blockIdx.x / H, grp = h / (H / G);
+    const long bh = blockIdx.x;
+    const int m = T - 1;
+    int s0 = 0, s1 = 0;
+    if (lev == 0) {
+        s0 = m;
+        s1 = m + 1;
+    } else if (lev - 1 < 31 && ((m >> (lev - 1)) & 1)) {
+        s0 = (m >> lev) << lev;
+        s1 = s0 + (1 << (lev - 1));
+    }
+    float* out = states + (bh * L + lev) * KV;
+    if (s1 == s0) {
+        for (int e = tid * 4; e < KV; e += 1024) *reinterpret_cast<float4*>(out + e) = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    auto block_sum = [&](float x) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+        if (lane == 0) sRed[warp] = x;
+        __syncthreads();
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += sRed[w];
+        __syncthreads();
+        return t;
+    };
+    const float* gb = g + (long)b * Tp * H + h;
+    if (seg_F != nullptr && s1 - s0 >= SEG) {
+        // behind the bucket: whole segments up to the one of the last token, then that segment's tokens up to the last one
+        const int r0 = s0 / SEG, r1 = s1 / SEG, rl = m / SEG, NS = (Tp + SEG - 1) / SEG;
+        const float *D = seg_D + bh * NS, *F = seg_F + bh * NS * KV;
+        float part = 0.f;
+        for (int r = r1 + tid; r < rl; r += 256) part += D[r];
+        for (int t = rl * SEG + tid; t <= m; t += 256) part += gb[(long)t * H];
+        float after = block_sum(part);
+        float4 acc[KV / 1024];
+#pragma unroll
+        for (int i = 0; i < KV / 1024; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = r1 - 1; r >= r0; --r) {
+            const float w = fexp(after);
+#pragma unroll
+            for (int i = 0; i < KV / 1024; ++i) {
+                const float4 f = *reinterpret_cast<const float4*>(F + (long)r * KV + i * 1024 + tid * 4);
+                acc[i].x += w * f.x; acc[i].y += w * f.y; acc[i].z += w * f.z; acc[i].w += w * f.w;
+            }
+            after += D[r];
+        }
+#pragma unroll
+        for (int i = 0; i < KV / 1024; ++i) *reinterpret_cast<float4*>(out + i * 1024 + tid * 4) = acc[i];
+        return;
+    }
+    const int wr = warp & 3, wc = warp >> 2;
+    float acc[MT][2 * NPW][4];
+    zero_acc(acc);
+    // tokens e1 - 1 downwards in tiles of 64; rows of a tile beyond its tokens are zero
+    uint4 vr[2];
+    auto fetch = [&](int a, int e1, int st) {
+        const int n = e1 - a;
+        for (int e = tid; e < CH * (KD / 8); e += 256) {
+            const int i = e / (KD / 8), c8 = (e % (KD / 8)) * 8;
+            bf16* dst = sK + st * CH * LDK + i * LDK + c8;
+            if (i < n) cp_async16(dst, k + (((long)b * Tp + a + i) * G + grp) * KD + c8);
+            else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+        }
+        cp_async_commit();
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = (tid + u * 256) / (VD / 8), c8 = ((tid + u * 256) % (VD / 8)) * 8;
+            vr[u] = i < n ? *reinterpret_cast<const uint4*>(v + (((long)b * Tp + a + i) * H + h) * VD + c8) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    float part = 0.f;
+    fetch(max(s1 - CH, s0), s1, 0);
+    for (int r = s1 + tid; r <= m; r += 256) part += gb[(long)r * H];
+    float after = block_sum(part);
+    int st = 0;
+    for (int e2 = s1; e2 > s0; e2 -= 256) {
+        const int a2 = max(e2 - 256, s0), n2 = e2 - a2;
+        // token a2 + i of the block: exp(after + sum_{r = a2+i+1 .. e2-1} g_r), by a scan from the end (thread j holds token n2 - 1 - j)
+        const int i = n2 - 1 - tid;
+        float x = (tid >= 1 && i >= 0) ? gb[(long)(a2 + i + 1) * H] : 0.f;
+        const float first = gb[(long)a2 * H];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += t;
+        }
+        if (lane == 31) sRed[warp] = x;
+        __syncthreads();
+        float all = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            if (w < warp) x += sRed[w];
+            all += sRed[w];
+        }
+        if (i >= 0) sDec[i] = fexp(after + x);
+        after += all + first;
+        __syncthreads();
+        for (int e1 = e2; e1 > a2; e1 -= CH) {
+            const int a = max(e1 - CH, s0), n = e1 - a;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int row = (tid + u * 256) / (VD / 8), c8 = ((tid + u * 256) % (VD / 8)) * 8;
+                const float d = row < n ? sDec[a - a2 + row] : 0.f;
+                uint32_t* xw = reinterpret_cast<uint32_t*>(&vr[u]);
+#pragma unroll
+                for (int q4 = 0; q4 < 4; ++q4) {
+                    const __nv_bfloat162 t2 = *reinterpret_cast<const __nv_bfloat162*>(&xw[q4]);
+                    xw[q4] = pack_bf16(__bfloat162float(t2.x) * d, __bfloat162float(t2.y) * d);
+                }
+                *reinterpret_cast<uint4*>(sV + st * CH * LDV + row * LDV + c8) = vr[u];
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+            if (a > s0) fetch(max(a - CH, s0), a, st ^ 1);
+            warp_gemm<MT, NPW, true, true>(acc, sK + st * CH * LDK, LDK, wr * 16 * MT, sV + st * CH * LDV, LDV, wc * 32, CH, lane);
+            st ^= 1;
+        }
+    }
+    const int lr = lane >> 2, lc2 = (lane & 3) * 2;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2 * NPW; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; e += 2)
+                *reinterpret_cast<float2*>(out + (wr * 16 * MT + mt * 16 + lr + (e >> 1) * 8) * VD + wc * 32 + nt * 8 + lc2) =
+                    make_float2(acc[mt][nt][e], acc[mt][nt][e + 1]);
 }
 
 // one decode step for one (batch, head) per CTA; thread t owns column t % VD and rows t / VD, + 256 / VD, ...
@@ -251,8 +363,8 @@ int llattn_mamba2_final_state(const void* k, const void* v, const float* g, floa
     using bf = __nv_bfloat16;
     dim3 grid(B * H, L);
     cudaStream_t st = (cudaStream_t)stream;
-    if (K == 128) llattn::mamba2_final_state_kernel<128, 64, false><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, nullptr, nullptr, B, T, T, H, G, L);
-    else llattn::mamba2_final_state_kernel<64, 64, false><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, nullptr, nullptr, B, T, T, H, G, L);
+    if (K == 128) llattn::mamba2_final_state_kernel<128, 64><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, B, T, H, G, L);
+    else llattn::mamba2_final_state_kernel<64, 64><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, B, T, H, G, L);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -271,8 +383,14 @@ int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, fl
     using bf = __nv_bfloat16;
     dim3 grid(B * H, L);
     cudaStream_t st = (cudaStream_t)stream;
-    if (K == 128) llattn::mamba2_final_state_kernel<128, 64, true><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, seg_F, seg_D, B, T, Tp, H, G, L);
-    else llattn::mamba2_final_state_kernel<64, 64, true><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, seg_F, seg_D, B, T, Tp, H, G, L);
+    auto launch = [&](auto kern, size_t sm) -> cudaError_t {
+        const cudaError_t e = llattn::allow_smem(kern, sm);
+        if (e == cudaSuccess) kern<<<grid, 256, sm, st>>>((const bf*)k, (const bf*)v, g, states, seg_F, seg_D, T, Tp, H, G, L);
+        return e;
+    };
+    const cudaError_t e = K == 128 ? launch(llattn::mamba2_prompt_state_kernel<128>, llattn::PromptStateSmem<128>::total)
+                                   : launch(llattn::mamba2_prompt_state_kernel<64>, llattn::PromptStateSmem<64>::total);
+    if (e != cudaSuccess) return (int)e;
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
