@@ -61,6 +61,7 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
         p.dk_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
         p.wq = c.take<float>((size_t)p.B * p.T * p.H);
         p.Yseg = c.take<float>(BH * p.NS * (p.LH > 0 ? p.LH : 1));
+        p.Xt = c.take<float>(BH * p.NT);
         p.Zc = c.take<float>(BH * p.NT * p.LZ);
         p.Yc = c.take<float>(BH * p.NT * (llattn::M2_MLOW + 1));
         p.g = c.take<float>((size_t)p.B * p.T * p.H);

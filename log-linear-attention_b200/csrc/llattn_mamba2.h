@@ -44,6 +44,7 @@ struct Mamba2Params {
     float* Zc;                   // (B,H,NT,LZ)      reader side: sum_t lambda * dlambda per level
     float* Yc;                   // (B,H,NT,MLOW+1)  contributor side: <KV_c, adjoint state> per low level, + combined high
     float* Yseg;                 // (B,H,NS,LH)      contributor side per segment and high level
+    float* Xt;                   // (B,H,NT)         what reaches the end of each chunk, summed over the levels
     int LZ;                      // MLOW + LH
     int* err;                    // device status word: set to 1 when a bounded wait on the tensor core gave up
     int B, T, H, G, K, V, L;

@@ -872,67 +872,72 @@ __global__ void __launch_bounds__(256, 1) m2_seg_dstate_kernel(const Mamba2Param
 //   for r = NS-1 .. 0 : dHseg[r] = sum_{j: bit j of r clear} dH_j ; then dH_j is zeroed when
 //   r % 2^(j+1) == 0, else decayed by exp(D_r) ; then dF[r][j] is added when bit j of r is set.
 // ------------------------------------------------------------------------------------------
-constexpr int MAX_LH_B = 10;
+// Bound by HBM: it reads the reader summaries of the set bits and F once and writes dH once.  A thread owns two neighbouring elements of the
+// K x V states and walks the segments with the loads of two in flight; the loads are predicated, not branched around, and the number of
+// levels is a template parameter, so that 128-thread CTAs of a whole 65536-token problem (1024 of them) are resident at once.  (Four
+// elements a thread, branches and one instantiation for up to ten levels: 411 us at B = 1, T = 65536, 32 heads.)
+__device__ __forceinline__ float2 ldg2_if(const float* ptr, bool p) {
+    float2 r;
+    asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %3, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n @p ld.global.nc.v2.f32 {%0, %1}, [%2];\n}\n"
+                 : "=&f"(r.x), "=&f"(r.y)
+                 : "l"(ptr), "r"((int)p));
+    return r;
+}
 
-template <int MAXLH>
-__global__ void __launch_bounds__(256) m2_seg_dscan_kernel(const Mamba2Params p, int KV) {
+template <int LH>
+__global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p, int KV) {
     const long bh = blockIdx.y;
-    const int e4 = (blockIdx.x * 256 + threadIdx.x) * 4;
-    if (e4 >= KV) return;
-    const float* dF = p.seg_dF + bh * p.NS * p.LH * KV + e4;
-    const float* F = p.seg_F + bh * p.NS * KV + e4;
+    const int e2 = (blockIdx.x * 128 + threadIdx.x) * 2;
+    if (e2 >= KV) return;                       // whole warps: KV is a multiple of 64
+    const float* dF = p.seg_dF + bh * p.NS * LH * KV + e2;
+    const float* F = p.seg_F + bh * p.NS * KV + e2;
     const float* D = p.seg_D + bh * p.NS;
-    float* dH = p.seg_dHf + bh * p.NS * KV + e4;
-    float* Yseg = p.Yseg + bh * p.NS * p.LH;
+    float* dH = p.seg_dHf + bh * p.NS * KV + e2;
+    float* Yseg = p.Yseg + bh * p.NS * LH;
     const int lane = threadIdx.x & 31;
-    float st[MAXLH][4];
+    float2 st[LH];
 #pragma unroll
-    for (int j = 0; j < MAXLH; ++j) st[j][0] = st[j][1] = st[j][2] = st[j][3] = 0.f;
-    // the recurrence itself is only in registers; the loads of segment r - 2 are issued right after the arithmetic of segment r
-    // (two register sets used alternately), so that a thread has up to two segments' worth of loads in flight
+    for (int j = 0; j < LH; ++j) st[j] = make_float2(0.f, 0.f);
     struct Loads {
-        float4 f;
-        float4 dF[MAXLH];
+        float2 f, dF[LH];
         float d;
     };
     auto fetch = [&](Loads& L, int r) {
-        L.f = (r >= 0 && r < p.NS - 1) ? __ldg(reinterpret_cast<const float4*>(F + (long)r * KV)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        L.d = (r >= 0 && r < p.NS - 1) ? __ldg(D + r) : 0.f;
+        const bool in = r >= 0 && r < p.NS - 1;
+        L.f = ldg2_if(F + (long)r * KV, in);
+        L.d = in ? __ldg(D + r) : 0.f;
 #pragma unroll
-        for (int j = 0; j < MAXLH; ++j)
-            L.dF[j] = (r >= 0 && j < p.LH && ((r >> j) & 1)) ? __ldg(reinterpret_cast<const float4*>(dF + ((long)r * p.LH + j) * KV))
-                                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < LH; ++j) L.dF[j] = ldg2_if(dF + ((long)r * LH + j) * KV, r >= 0 && ((r >> j) & 1));
     };
     auto process = [&](const Loads& L, int r) {
-        float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 f = L.f;
+        float2 out = make_float2(0.f, 0.f);
         const float d = (r < p.NS - 1) ? __expf(L.d) : 0.f;
+        float y[LH];
 #pragma unroll
-        for (int j = 0; j < MAXLH; ++j) {
-            if (j < p.LH) {
-                const bool bit = (r >> j) & 1;
-                if (!bit) {
-                    out.x += st[j][0]; out.y += st[j][1]; out.z += st[j][2]; out.w += st[j][3];
-                    if (r < p.NS - 1) {
-                        // <F_r, adjoint of level j after segment r>
-                        float y = f.x * st[j][0] + f.y * st[j][1] + f.z * st[j][2] + f.w * st[j][3];
-#pragma unroll
-                        for (int dd = 16; dd > 0; dd >>= 1) y += __shfl_xor_sync(0xffffffffu, y, dd);
-                        if (lane == 0) atomicAdd(Yseg + (long)r * p.LH + j, y);
-                    }
-                }
-                const int period = 2 << j;
-                if ((r % period) == 0) {
-                    st[j][0] = st[j][1] = st[j][2] = st[j][3] = 0.f;
-                } else {
-                    st[j][0] *= d; st[j][1] *= d; st[j][2] *= d; st[j][3] *= d;
-                }
-                if (bit) {
-                    st[j][0] += L.dF[j].x; st[j][1] += L.dF[j].y; st[j][2] += L.dF[j].z; st[j][3] += L.dF[j].w;
-                }
+        for (int j = 0; j < LH; ++j) {
+            const bool bit = (r >> j) & 1;
+            // <F_r, adjoint of level j after segment r>; zero where the level has no contributor here
+            y[j] = bit ? 0.f : L.f.x * st[j].x + L.f.y * st[j].y;
+            if (!bit) {
+                out.x += st[j].x;
+                out.y += st[j].y;
             }
+            const float m = (r & ((2 << j) - 1)) == 0 ? 0.f : d;
+            st[j].x = st[j].x * m + L.dF[j].x;
+            st[j].y = st[j].y * m + L.dF[j].y;
         }
-        if (r < p.NS - 1) *reinterpret_cast<float4*>(dH + (long)r * KV) = out;
+        if (r < p.NS - 1) {
+#pragma unroll
+            for (int j = 0; j < LH; ++j)
+#pragma unroll
+                for (int dd = 16; dd > 0; dd >>= 1) y[j] += __shfl_xor_sync(0xffffffffu, y[j], dd);
+            // lane j adds the total of level j
+            float mine = 0.f;
+#pragma unroll
+            for (int j = 0; j < LH; ++j) mine = lane == j ? y[j] : mine;
+            if (lane < LH && !((r >> lane) & 1)) atomicAdd(Yseg + (long)r * LH + lane, mine);
+            *reinterpret_cast<float2*>(dH + (long)r * KV) = out;
+        }
     };
     Loads A, B;
     fetch(A, p.NS - 1);
@@ -944,6 +949,15 @@ __global__ void __launch_bounds__(256) m2_seg_dscan_kernel(const Mamba2Params p,
             process(B, r - 1);
             fetch(B, r - 3);
         }
+    }
+}
+
+template <int LH>
+static void launch_dscan(const Mamba2Params& p, int KV, cudaStream_t stream) {
+    if constexpr (LH > 0) {
+        if (p.LH != LH) return launch_dscan<LH - 1>(p, KV, stream);
+        m2_seg_dscan_kernel<LH><<<dim3((KV / 2 + 127) / 128, p.B * p.H), 128, 0, stream>>>(p, KV);
+        LLATTN_LAUNCHED();
     }
 }
 
@@ -968,8 +982,7 @@ __global__ void __launch_bounds__(256) m2_bwd_init_kernel(const float* __restric
     }
 }
 
-// dg for one (batch, head) per CTA.
-//   dg[r] = sum_{t >= r, t in chunk(r)} w[t]  +  X[chunk(r)]
+// dg[r] = sum_{t >= r, t in chunk(r)} w[t]  +  X[chunk(r)]
 // w[t] = q_t.dq_t - k_t.dk_t is the gradient w.r.t. the in-chunk cumulative sum G_t (the
 // reference's dg before its reverse in-chunk cumsum, chunkwise.py:793-874, 1596); X[c] is the
 // gradient that reaches the end of chunk c from every (target, source) pair that straddles it
@@ -978,130 +991,116 @@ __global__ void __launch_bounds__(256) m2_bwd_init_kernel(const float* __restric
 // Y over the block's contributor chunks up to c (bit l of c clear), or the sum of the reader
 // totals Z over the reader chunks after c (bit set).  Sums never extend beyond one block pair, so
 // rounding differences between the two sides do not accumulate along the sequence.
+//
+// The table X is built by one CTA per (batch, head) and level, whose running sums are warp scans; then a thread per (chunk, head) walks
+// the chunk's tokens, heads on neighbouring lanes.  (One kernel in which every slice of 64 chunks built the whole table, by chains of up
+// to 2^l additions, took 162 us at T = 65536, 32 heads.)
+
+// running sums over 32 chunks or segments, one a lane, inside half-blocks of `half` of them (a power of two)
+__device__ __forceinline__ float half_suffix(float v, int half, int lane) {       // exclusive, from the end
+    float s = v;
+    const int n = half < 32 ? half : 32;
+    for (int d = 1; d < n; d <<= 1) {
+        const float t = __shfl_down_sync(0xffffffffu, s, d);
+        if ((lane & (n - 1)) + d < n) s += t;
+    }
+    const float e = __shfl_down_sync(0xffffffffu, s, 1);
+    return (lane & (n - 1)) == n - 1 ? 0.f : e;
+}
+__device__ __forceinline__ float half_prefix(float v, int half, int lane) {       // inclusive, from the start
+    const int n = half < 32 ? half : 32;
+    for (int d = 1; d < n; d <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, v, d);
+        if ((lane & (n - 1)) >= d) v += t;
+    }
+    return v;
+}
+
 template <int MLOW>
-__global__ void __launch_bounds__(256) m2_dg_kernel(const Mamba2Params p, float* __restrict__ dg) {
-    extern __shared__ float sx[];
+__global__ void __launch_bounds__(256) m2_dg_table_kernel(const Mamba2Params p, int nlev) {
     constexpr int SEG = 1 << MLOW;
-    float* X = sx;                 // [NT]  (combined-high prefix inside a segment)
-    float* XS = sx + p.NT;         // [NS]  (sum over high levels of the prefix over earlier segments)
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int h = blockIdx.x % p.H, b = blockIdx.x / p.H;
-    const long bh = (long)b * p.H + h;
-    // blockIdx.y selects a slice of 64 chunks for the token pass; every CTA of a (batch, head)
-    // rebuilds the small per-chunk table X (a few thousand scalar operations)
-    const int c_begin = blockIdx.y * 64, c_end = min(p.NT, c_begin + 64);
+    const long bh = blockIdx.x;
+    const int lv = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float* Zc = p.Zc + bh * p.NT * p.LZ;
     const float* Yc = p.Yc + bh * p.NT * (MLOW + 1);
-    const float* Yseg = p.Yseg + bh * p.NS * p.LH;
-    // stage the per-chunk scalar tables in shared memory: the sweeps below are serial chains
-    float* sZ = sx + p.NT + p.NS;                       // [NT][LZ]
-    float* sY = sZ + p.NT * p.LZ;                       // [NT][MLOW+1]
-    float* sYs = sY + p.NT * (MLOW + 1);                // [NS][LH]
-    for (int i = tid; i < p.NT + p.NS; i += 256) sx[i] = 0.f;
-    // eight loads per thread are in flight before the first of them is stored
-    for (int i0 = 0; i0 < p.NT * p.LZ; i0 += 8 * 256) {
-        float tmp[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * 256 + tid, c = i / p.LZ, lvz = i - c * p.LZ;
-            tmp[u] = (i < p.NT * p.LZ && ((c >> lvz) & 1)) ? __ldg(Zc + i) : 0.f;          // only reader entries were written
+    float* X = p.Xt + bh * p.NT;
+    if (lv == nlev) {
+        // contributor totals of all high levels together: running sum inside each segment
+        for (int c0 = warp * 32; c0 < p.NT; c0 += 256) {
+            const int c = c0 + lane;
+            const float v = c < p.NT ? Yc[(long)c * (MLOW + 1) + MLOW] : 0.f;
+            const float x = half_prefix(v, SEG, lane);
+            if (c < p.NT) atomicAdd(&X[c], x);
         }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * 256 + tid;
-            if (i < p.NT * p.LZ) sZ[i] = tmp[u];
-        }
+        return;
     }
-    for (int i0 = 0; i0 < p.NT * (MLOW + 1); i0 += 4 * 256) {
-        float tmp[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * 256 + tid;
-            tmp[u] = (i < p.NT * (MLOW + 1)) ? __ldg(Yc + i) : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * 256 + tid;
-            if (i < p.NT * (MLOW + 1)) sY[i] = tmp[u];
-        }
-    }
-    for (int i = tid; i < p.NS * p.LH; i += 256) sYs[i] = __ldg(Yseg + i);
-    __syncthreads();
-    int nlev = 0;
-    while ((1 << nlev) < p.NT) ++nlev;          // inter-chunk levels in use
-    // every level writes its own row XL[lv][c] (no shared-memory atomics); rows are summed per chunk below
-    float* XL = sYs + p.NS * (p.LH > 0 ? p.LH : 1);     // [nlev][NT]
-    // One level per warp and round.  Within a block pair of 2^(lv+1) chunks the contributor sweep runs forwards over the first
-    // half (inclusive running sum of Y) and the reader sweep backwards over the second half (running sum of Z, exclusive): the
-    // half-blocks are independent, so each lane takes one (block, sweep) with the same branch-free loop and the longest chain is
-    // 2^lv steps instead of two passes over all chunks.
-    for (int lv = warp; lv < nlev; lv += 8) {
-        const int hl = 1 << lv, period = 2 << lv;
-        float* xl = XL + lv * p.NT;
-        for (int c = lane; c < p.NT; c += 32) xl[c] = 0.f;
-        __syncwarp();
-        const int nblk = (p.NT + period - 1) / period;
-        for (int t = lane; t < 2 * nblk; t += 32) {
-            const int base = (t >> 1) * period;
-            const bool rev = t & 1;
-            const bool active = rev || lv < MLOW;
-            const float* src = rev ? sZ + lv : sY + lv;
-            const int stride = rev ? p.LZ : (MLOW + 1);
-            const int c0 = rev ? base + period - 1 : base, dir = rev ? -1 : 1;
-            float run = 0.f;
-            for (int k = 0; k < hl; ++k) {
-                const int c = c0 + dir * k;
-                if (active && c < p.NT) {
-                    const float v = src[c * stride];
-                    xl[c] = rev ? run : run + v;
-                    run += v;
-                }
+    const int half = 1 << lv;
+    // readers: after c, to the end of its half-block
+    if (half <= 32) {
+        for (int c0 = warp * 32; c0 < p.NT; c0 += 256) {
+            const int c = c0 + lane;
+            const bool reader = c < p.NT && ((c >> lv) & 1);
+            const float x = half_suffix(reader ? Zc[(long)c * p.LZ + lv] : 0.f, half, lane);
+            float add = reader ? x : 0.f;
+            if (lv < MLOW) {
+                // contributors: up to and with c
+                const bool contributes = c < p.NT && !((c >> lv) & 1);
+                const float y = half_prefix(contributes ? Yc[(long)c * (MLOW + 1) + lv] : 0.f, half, lane);
+                if (contributes) add = y;
             }
+            if (c < p.NT) atomicAdd(&X[c], add);
         }
-        if (lv >= MLOW && lane == 31) {
-            // contributor totals of the high levels live per segment
-            const int j = lv - MLOW, pj = 2 << j;
-            float run = 0.f;
-            for (int r = 0; r < p.NS; ++r) {
-                if ((r & (pj - 1)) == 0) run = 0.f;
-                if (!((r >> j) & 1)) {
-                    atomicAdd(&XS[r], run);
-                    if (r < p.NS - 1) run += sYs[r * p.LH + j];
-                }
+    } else {
+        const int nhalf = (p.NT + half - 1) / half;                    // half-blocks; the odd ones read
+        for (int hb = 1 + 2 * warp; hb < nhalf; hb += 16) {
+            float carry = 0.f;
+            for (int c0 = (hb + 1) * half - 32; c0 >= hb * half; c0 -= 32) {
+                const int c = c0 + lane;
+                const float v = c < p.NT ? Zc[(long)c * p.LZ + lv] : 0.f;
+                const float x = half_suffix(v, 32, lane);
+                if (c < p.NT) atomicAdd(&X[c], carry + x);
+                carry += __shfl_sync(0xffffffffu, x + v, 0);
             }
         }
     }
-    if (warp == (nlev & 7)) {
-        // combined high levels: running sum inside each segment, one segment per lane (on the warp with the fewest levels)
-        for (int c0 = lane * SEG; c0 < p.NT; c0 += 32 * SEG) {
-            float run = 0.f;
-            for (int c = c0; c < c0 + SEG && c < p.NT; ++c) {
-                run += sY[c * (MLOW + 1) + MLOW];
-                X[c] = run;
+    if (lv >= MLOW) {
+        // contributors of a high level, per segment: the segments before this one in its half-block
+        const int j = lv - MLOW, hs = 1 << j;
+        const float* Ys = p.Yseg + bh * p.NS * p.LH;
+        for (int hb = 2 * warp; hb * hs < p.NS; hb += 16) {
+            float carry = 0.f;
+            for (int r0 = hb * hs; r0 < (hb + 1) * hs; r0 += 32) {
+                const int r = r0 + lane;
+                const bool in = lane < hs && r < p.NS - 1;
+                const float v = in ? Ys[(long)r * p.LH + j] : 0.f;
+                const float incl = half_prefix(v, 32, lane);
+                const float before = __shfl_up_sync(0xffffffffu, incl, 1);
+                const float excl = carry + (lane == 0 ? 0.f : before);
+                carry += __shfl_sync(0xffffffffu, incl, 31);
+                if (lane < hs && r < p.NS)
+                    for (int c = r * SEG; c < (r + 1) * SEG && c < p.NT; ++c) atomicAdd(&X[c], excl);
             }
         }
     }
-    __syncthreads();
-    // a warp's (up to eight) chunks: all loads first
-    float w0[8], w1[8];
+}
+
+__global__ void __launch_bounds__(128) m2_dg_kernel(const Mamba2Params p, float* __restrict__ dg) {
+    const long i = (long)blockIdx.x * 128 + threadIdx.x;               // (batch, chunk, head)
+    if (i >= (long)p.B * p.NT * p.H) return;
+    const int h = (int)(i % p.H);
+    const long bc = i / p.H;
+    const int c = (int)(bc % p.NT), b = (int)(bc / p.NT);
+    const long base = bc * CH * p.H + h;
+    float run = p.Xt[((long)b * p.H + h) * p.NT + c];
+    for (int t = CH; t > 0; t -= 16) {
+        float w[16];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int c = c_begin + warp + u * 8;
-        const long base = ((long)b * p.T + (long)c * CH) * p.H + h;
-        w0[u] = (c < c_end) ? __ldg(p.wq + base + (long)(63 - 2 * lane) * p.H) : 0.f;
-        w1[u] = (c < c_end) ? __ldg(p.wq + base + (long)(62 - 2 * lane) * p.H) : 0.f;
-    }
+        for (int u = 0; u < 16; ++u) w[u] = __ldg(p.wq + base + (long)(t - 1 - u) * p.H);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int c = c_begin + warp + u * 8;
-        if (c >= c_end) break;
-        const long base = ((long)b * p.T + (long)c * CH) * p.H + h;
-        float x0 = w0[u], x1 = w1[u];
-        warp_cumsum64(x0, x1, lane);
-        float add = X[c] + XS[c / SEG];
-        for (int lv = 0; lv < nlev; ++lv) add += XL[lv * p.NT + c];
-        dg[base + (long)(63 - 2 * lane) * p.H] = x0 + add;
-        dg[base + (long)(62 - 2 * lane) * p.H] = x1 + add;
+        for (int u = 0; u < 16; ++u) {
+            run += w[u];
+            dg[base + (long)(t - 1 - u) * p.H] = run;
+        }
     }
 }
 
@@ -1154,11 +1153,7 @@ static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStre
                 kern<<<grid, 256, SegDSmem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
             }
         }
-        {
-            dim3 grid((KV / 4 + 255) / 256, p.B * p.H);
-            if (p.LH <= 5) { m2_seg_dscan_kernel<5><<<grid, 256, 0, stream>>>(p, KV); LLATTN_LAUNCHED(); }
-            else { m2_seg_dscan_kernel<MAX_LH_B><<<grid, 256, 0, stream>>>(p, KV); LLATTN_LAUNCHED(); }
-        }
+        launch_dscan<M2_MAX_LH>(p, KV, stream);
     }
     if (use_tc) return mamba2_bwd2_tc_launch(p, stream);
     auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;
@@ -1218,13 +1213,10 @@ int mamba2_bwd_init(const float* gc, float* g, long BT, int H, void* acc, size_t
 }
 
 int mamba2_dg(const Mamba2Params& p, float* dg, cudaStream_t stream) {
-    dim3 grid(p.B * p.H, (p.NT + 63) / 64);
-    const size_t smem = (size_t)(p.NT + p.NS + p.NT * p.LZ + p.NT * (M2_MLOW + 1) + p.NS * (p.LH > 0 ? p.LH : 1) + (size_t)p.LZ * p.NT) * sizeof(float);
-    if (smem > 48 * 1024) {
-        cudaError_t e = allow_smem(m2_dg_kernel<M2_MLOW>, smem);
-        if (e != cudaSuccess) return (int)e;
-    }
-    m2_dg_kernel<M2_MLOW><<<grid, 256, smem, stream>>>(p, dg); LLATTN_LAUNCHED();
+    int nlev = 0;
+    while ((1 << nlev) < p.NT) ++nlev;          // inter-chunk levels in use
+    m2_dg_table_kernel<M2_MLOW><<<dim3(p.B * p.H, nlev + 1), 256, 0, stream>>>(p, nlev); LLATTN_LAUNCHED();
+    m2_dg_kernel<<<(unsigned)(((long)p.B * p.NT * p.H + 127) / 128), 128, 0, stream>>>(p, dg); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

@@ -205,7 +205,7 @@ static unsigned prep_grid(llattn::PrepArgs& a, long rows, int H, int P, int L, i
     a.lam8 = H * L % 8 == 0;
     a.lam_blocks = (H * L / (a.lam8 ? 8 : 1) + threads - 1) / threads;
     a.run = 64;
-    while (a.run > (backward ? 8 : 4) && (long)a.row_blocks * ((a.tokens + a.run - 1) / a.run) * threads < 148 * 6 * 256) a.run /= 2;
+    while (a.run > (backward ? 8 : 4) && (long)a.row_blocks * ((a.tokens + a.run - 1) / a.run) * threads < 148 * 8 * 256) a.run /= 2;
     // forward: eight tokens a thread
     const int groups = H * L / (a.lam8 ? 8 : 1), per = groups < threads ? threads / groups : 1;
     a.lam_runs = backward ? llattn::lambda_runs(a.tokens, a.lam_blocks) : (a.tokens + 8 * per - 1) / (8 * per);
