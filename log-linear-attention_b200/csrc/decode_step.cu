@@ -75,6 +75,7 @@ __device__ __forceinline__ float layer_lambda(const M2StepArgs& a, long bh, int 
 // is a handful of dependent memory round trips (8 columns, or every live level in one group, were slower: 10.2 / 9.9 us).
 template <int COLS, int RPT, int NG, int CTAS>
 __global__ void __launch_bounds__(ST_THREADS, CTAS) m2_layer_step_kernel(const __grid_constant__ M2StepArgs a) {
+    chain_wait();
     constexpr int C4 = COLS / 4;                    // lanes per row, four columns each
     constexpr int R = ST_THREADS / C4;              // rows per pass
     extern __shared__ float sh[];                   // q[K] | k[K]
@@ -240,6 +241,7 @@ struct GdnStepArgs {
 // store and the output; more live levels take another round.
 template <int THREADS, int RPT, int NG, int CTAS>
 __global__ void __launch_bounds__(THREADS, CTAS) gdn_layer_step_kernel(const __grid_constant__ GdnStepArgs a) {
+    chain_wait();
     constexpr int COLS = 16, C4 = 4, R = THREADS / C4, NW = THREADS / 32;
     __shared__ float sQ[256], sK[256];
     __shared__ float sLam[ST_MAXL];
@@ -463,9 +465,9 @@ int llattn_mamba2_layer_step(float* states, const void* q, const void* k, const 
     cudaStream_t st = (cudaStream_t)stream;
     // whole rows per CTA once that gives two CTAs for every SM
     if (V % 64 == 0 && (long)B * H * (V / 64) >= 296)
-        llattn::m2_layer_step_kernel<64, 2, 4, 2><<<B * H * (V / 64), llattn::ST_THREADS, sm, st>>>(a);
+        llattn::launch_chained(llattn::m2_layer_step_kernel<64, 2, 4, 2>, B * H * (V / 64), llattn::ST_THREADS, sm, st, a);
     else
-        llattn::m2_layer_step_kernel<16, 2, 6, 2><<<B * H * (V / 16), llattn::ST_THREADS, sm, st>>>(a);
+        llattn::launch_chained(llattn::m2_layer_step_kernel<16, 2, 6, 2>, B * H * (V / 16), llattn::ST_THREADS, sm, st, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -487,10 +489,10 @@ int llattn_gdn_layer_step(float* states, const void* q, const void* k, const voi
     // K = 128: with two CTAs for every SM and more, CTAs of half the size (four of them on an SM) overlap one's reduction with
     // another's loads better: 13.2 against 15.2 us at B = 4, 54.6 against 60.3 us at B = 16 (H = 16, V = 128, eight live levels);
     // below, the larger ones have fewer rows per thread: 6.2 against 8.3 us at B = 1
-    if (K <= 64) llattn::gdn_layer_step_kernel<256, 1, 8, 2><<<grid, 256, 0, st>>>(a);
-    else if (K <= 128 && grid >= 296) llattn::gdn_layer_step_kernel<128, 4, 4, 4><<<grid, 128, 0, st>>>(a);
-    else if (K <= 128) llattn::gdn_layer_step_kernel<256, 2, 4, 2><<<grid, 256, 0, st>>>(a);
-    else llattn::gdn_layer_step_kernel<512, 2, 4, 1><<<grid, 512, 0, st>>>(a);
+    if (K <= 64) llattn::launch_chained(llattn::gdn_layer_step_kernel<256, 1, 8, 2>, grid, 256, 0, st, a);
+    else if (K <= 128 && grid >= 296) llattn::launch_chained(llattn::gdn_layer_step_kernel<128, 4, 4, 4>, grid, 128, 0, st, a);
+    else if (K <= 128) llattn::launch_chained(llattn::gdn_layer_step_kernel<256, 2, 4, 2>, grid, 256, 0, st, a);
+    else llattn::launch_chained(llattn::gdn_layer_step_kernel<512, 2, 4, 1>, grid, 512, 0, st, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

@@ -69,6 +69,7 @@ struct ScanBwdSmem {
 
 template <int KD>
 __global__ void __launch_bounds__(256, 1) gdn_scan_bwd_kernel(const GdnParams p) {
+    chain_wait();
     using SM = ScanBwdSmem<KD>;
     constexpr int LDK = SM::LDK, LDS = SM::LDS;
     static_assert(KD == 128, "one 16-row state tile per warp");
@@ -275,6 +276,7 @@ struct LevSmem {
 
 template <int KD, int VD>
 __global__ void __launch_bounds__(256, 1) gdn_bwd_levels_kernel(const GdnParams p) {
+    chain_wait();
     using SM = LevSmem<KD, VD>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, LDH = SM::LDH;
     constexpr int NVH = VD / 64;
@@ -485,7 +487,7 @@ int gdn_bwd_scan_dispatch(const GdnParams& p, cudaStream_t stream) {
     const size_t sm = ScanBwdSmem<128>::total;
     cudaError_t e;
     if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * (p.V / GDN_VS), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * (p.V / GDN_VS), 256, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
@@ -495,7 +497,7 @@ static int launch_levels(const GdnParams& p, cudaStream_t stream) {
     const size_t sm = LevSmem<KD, VD>::total;
     cudaError_t e;
     if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-    kern<<<p.B * p.NT * p.H, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.NT * p.H, 256, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

@@ -44,6 +44,7 @@ struct ChunkBwdSmem {
 // the chunk total of d_kd.kd (inside d_gl); otherwise a row pass over the K-wide gradients derives them here.
 template <int KD, int VD, bool FUSED>
 __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p) {
+    chain_wait();
     using SM = ChunkBwdSmem<KD, VD>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, LDP = SM::LDP;
     constexpr int NPK = KD / 32, NPV = VD / 32;       // 16-column pairs per warp for 64 x K and 64 x V results
@@ -630,7 +631,7 @@ static int launch_chunk(const GdnParams& p, cudaStream_t stream) {
     const size_t sm = ChunkBwdSmem<KD, VD>::total;
     cudaError_t e;
     if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-    kern<<<p.B * p.NT * p.H, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.NT * p.H, 256, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

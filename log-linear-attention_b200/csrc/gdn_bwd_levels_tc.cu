@@ -70,6 +70,7 @@ __device__ __forceinline__ LevStep lev_step(int s, int c, int per_half, bool tra
 }
 
 __global__ void __launch_bounds__(glt::NTHREADS, 1) gdn_bwd_levels_tc_kernel(const __grid_constant__ GdnParams p) {
+    chain_wait();
     using SM = LevTcSmem;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -621,7 +622,7 @@ int gdn_bwd_levels_tc_dispatch(const GdnParams& p0, cudaStream_t stream) {
     const int grid = nitems < sms ? nitems : sms;
     auto kern = gdn_bwd_levels_tc_kernel;
     if ((e = allow_smem(kern, LevTcSmem::total)) != cudaSuccess) return (int)e;
-    kern<<<grid, glt::NTHREADS, LevTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, grid, glt::NTHREADS, LevTcSmem::total, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

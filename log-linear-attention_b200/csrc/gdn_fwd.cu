@@ -53,6 +53,7 @@ struct PrepSmem {
 // being solved for, and the intra-chunk output is skipped.
 template <int KD, int VD, bool FROM_SAVED>
 __global__ void __launch_bounds__(256, 1) gdn_chunk_prep_kernel(const GdnParams p) {
+    chain_wait();
     using SM = PrepSmem<KD, VD>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, LDP = SM::LDP, LDA = SM::LDA;
     constexpr int NPK = KD / 32, NPV = VD / 32;
@@ -406,6 +407,7 @@ struct ScanSmem {
 // keeps the workspace for the backward); OUT = false skips the output (recomputation only).
 template <int KD, bool SAVE, bool OUT>
 __global__ void __launch_bounds__(256, 1) gdn_scan_kernel(const GdnParams p) {
+    chain_wait();
     using SM = ScanSmem<KD>;
     constexpr int LDK = SM::LDK, LDS = SM::LDS;
     constexpr int MT = KD / 128;               // state rows per warp = 16 * MT (8 warps over KD rows)
@@ -668,14 +670,14 @@ static int launch_gdn_fwd(const GdnParams& p, cudaStream_t stream) {
         auto kern = gdn_chunk_prep_kernel<KD, VD, BWD>;
         const size_t sm = PrepSmem<KD, VD>::total;
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-        kern<<<p.B * p.NT * p.H, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+        llattn::launch_chained(kern, p.B * p.NT * p.H, 256, sm, stream, p); LLATTN_LAUNCHED();
     }
     if (KD == 128 && g_use_tensor_core_path.load()) return gdn_scan_tc_dispatch(p, BWD ? 2 : (KEEP ? 1 : 0), stream);
     {
         auto kern = gdn_scan_kernel<KD, BWD || KEEP, !BWD>;
         const size_t sm = ScanSmem<KD>::total;
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-        kern<<<p.B * p.H * (p.V / GDN_VS), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+        llattn::launch_chained(kern, p.B * p.H * (p.V / GDN_VS), 256, sm, stream, p); LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();
 }

@@ -41,6 +41,7 @@ static_assert(PrepTcSmem::total <= 232448, "shared memory of one CTA");
 
 template <int VD>
 __global__ void __launch_bounds__(gpt::NTHREADS, 1) gdn_chunk_prep_tc_kernel(const __grid_constant__ GdnParams p) {
+    chain_wait();
     using SM = PrepTcSmem;
     constexpr int LDA = gpt::LDA;
     constexpr uint32_t V_BYTES = CH * VD * 2;
@@ -629,7 +630,7 @@ static int launch_prep_tc(GdnParams& p, cudaStream_t stream) {
     const int grid = nitems < sms ? nitems : sms;
     auto kern = gdn_chunk_prep_tc_kernel<VD>;
     if ((e = allow_smem(kern, PrepTcSmem::total)) != cudaSuccess) return (int)e;
-    kern<<<grid, gpt::NTHREADS, PrepTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, grid, gpt::NTHREADS, PrepTcSmem::total, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

@@ -82,6 +82,7 @@ struct ScanTcSmem {
 // the workspace for the backward; V a multiple of 64); OUT = false skips the output (recomputation only).
 template <bool SAVE, bool OUT>
 __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __grid_constant__ GdnParams p) {
+    chain_wait();
     using SM = ScanTcSmem;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -457,6 +458,7 @@ struct ScanBwdTcSmem {
 };
 
 __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_bwd_tc_kernel(const __grid_constant__ GdnParams p) {
+    chain_wait();
     using SM = ScanBwdTcSmem;
     constexpr int TCOLS = 256;                 // one 32-column slot per level
     extern __shared__ unsigned char smem_raw[];
@@ -703,7 +705,7 @@ static int launch_scan_tc(GdnParams& p, cudaStream_t stream) {
     auto kern = gdn_scan_tc_kernel<SAVE, OUT>;
     cudaError_t e;
     if ((e = allow_smem(kern, ScanTcSmem::total)) != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * (p.V / gtc::VS), gtc::NTHREADS, ScanTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * (p.V / gtc::VS), gtc::NTHREADS, ScanTcSmem::total, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
@@ -724,7 +726,7 @@ int gdn_scan_bwd_tc_dispatch(const GdnParams& p0, cudaStream_t stream) {
     auto kern = gdn_scan_bwd_tc_kernel;
     cudaError_t e;
     if ((e = allow_smem(kern, ScanBwdTcSmem::total)) != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * (p.V / gtc::VS), gtc::NTHREADS, ScanBwdTcSmem::total, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * (p.V / gtc::VS), gtc::NTHREADS, ScanBwdTcSmem::total, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

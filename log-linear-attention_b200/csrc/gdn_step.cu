@@ -20,6 +20,7 @@ template <int MAXL, int RPT>   // RPT = K / 32 rows per thread
 __global__ void __launch_bounds__(256) gdn_step_kernel(float* __restrict__ states, const bf16* __restrict__ q, const bf16* __restrict__ k,
                                                        const bf16* __restrict__ v, const bf16* __restrict__ beta, const float* __restrict__ g,
                                                        const bf16* __restrict__ lam, bf16* __restrict__ o, int H, int K, int V, int L, int carry) {
+    chain_wait();
     __shared__ float sQ[256], sK[256];
     __shared__ float sRed[8][GS_VC][MAXL];
     __shared__ float sO[8][GS_VC];
@@ -127,7 +128,7 @@ extern "C" int llattn_gdn_step(float* states, const void* q, const void* k, cons
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned grid = (unsigned)(B * H * (V / llattn::GS_VC));
 #define LLATTN_GDN_STEP(MAXL, RPT)                                                                                          \
-    llattn::gdn_step_kernel<MAXL, RPT><<<grid, 256, 0, st>>>(states, (const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, \
+    llattn::launch_chained(llattn::gdn_step_kernel<MAXL, RPT>, grid, 256, 0, st, states, (const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, \
                                                              (const bf*)lambda, (bf*)o, H, K, V, L, carry_level)
     const int rpt = K / 32;
     if (L <= 16) {

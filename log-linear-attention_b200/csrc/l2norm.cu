@@ -16,6 +16,7 @@ namespace llattn {
 template <int LPR>
 __global__ void __launch_bounds__(256) l2norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                                          long rows, int D, float scale, float eps) {
+    chain_wait();
     const int lane = threadIdx.x % LPR;
     const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
     const bool active = row < rows && lane * 8 < D;
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(256) l2norm_fwd_kernel(const __nv_bfloat16* __
 template <int LPR>
 __global__ void __launch_bounds__(256) l2norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ dy,
                                                          __nv_bfloat16* __restrict__ dx, long rows, int D, float scale, float eps) {
+    chain_wait();
     const int lane = threadIdx.x % LPR;
     const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
     const bool active = row < rows && lane * 8 < D;
@@ -104,6 +106,7 @@ struct GdnGradOut {
 };
 
 __global__ void __launch_bounds__(256) gdn_grad_out_kernel(const __grid_constant__ GdnGradOut a) {
+    chain_wait();
     const int lane = threadIdx.x & 15;
     const long row = (long)blockIdx.x * 16 + (threadIdx.x >> 4);
     const bool have = row < a.rows, act = have && lane * 8 < a.K;
@@ -181,7 +184,7 @@ int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const flo
     using bf = __nv_bfloat16;
     llattn::GdnGradOut a{(const bf*)q, (const bf*)k, dq, dk, dbeta, dlambda, dg, (bf*)gq, (bf*)gk, (bf*)gbeta, (bf*)glambda, gg, rep, rows, K, K_in, L, scale,
                          lambda_mul};
-    llattn::gdn_grad_out_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, (cudaStream_t)stream>>>(a);
+    llattn::launch_chained(llattn::gdn_grad_out_kernel, (unsigned)((rows + 15) / 16), 256, 0, (cudaStream_t)stream, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -200,9 +203,9 @@ int llattn_l2norm_fwd(const void* x, void* y, long rows, int D, float scale, voi
     __nv_bfloat16* yo = (__nv_bfloat16*)y;
     const int lpr = D <= 64 ? 8 : (D <= 128 ? 16 : 32);
     const long blocks = (rows * lpr + 255) / 256;
-    if (lpr == 8) { llattn::l2norm_fwd_kernel<8><<<(unsigned)blocks, 256, 0, st>>>(xi, yo, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
-    else if (lpr == 16) { llattn::l2norm_fwd_kernel<16><<<(unsigned)blocks, 256, 0, st>>>(xi, yo, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
-    else { llattn::l2norm_fwd_kernel<32><<<(unsigned)blocks, 256, 0, st>>>(xi, yo, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
+    if (lpr == 8) { llattn::launch_chained(llattn::l2norm_fwd_kernel<8>, (unsigned)blocks, 256, 0, st, xi, yo, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
+    else if (lpr == 16) { llattn::launch_chained(llattn::l2norm_fwd_kernel<16>, (unsigned)blocks, 256, 0, st, xi, yo, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
+    else { llattn::launch_chained(llattn::l2norm_fwd_kernel<32>, (unsigned)blocks, 256, 0, st, xi, yo, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
     return (int)cudaGetLastError();
 }
 
@@ -215,9 +218,9 @@ int llattn_l2norm_bwd(const void* x, const float* dy, void* dx, long rows, int D
     __nv_bfloat16* o = (__nv_bfloat16*)dx;
     const int lpr = D <= 64 ? 8 : (D <= 128 ? 16 : 32);
     const long blocks = (rows * lpr + 255) / 256;
-    if (lpr == 8) { llattn::l2norm_bwd_kernel<8><<<(unsigned)blocks, 256, 0, st>>>(xi, dy, o, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
-    else if (lpr == 16) { llattn::l2norm_bwd_kernel<16><<<(unsigned)blocks, 256, 0, st>>>(xi, dy, o, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
-    else { llattn::l2norm_bwd_kernel<32><<<(unsigned)blocks, 256, 0, st>>>(xi, dy, o, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
+    if (lpr == 8) { llattn::launch_chained(llattn::l2norm_bwd_kernel<8>, (unsigned)blocks, 256, 0, st, xi, dy, o, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
+    else if (lpr == 16) { llattn::launch_chained(llattn::l2norm_bwd_kernel<16>, (unsigned)blocks, 256, 0, st, xi, dy, o, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
+    else { llattn::launch_chained(llattn::l2norm_bwd_kernel<32>, (unsigned)blocks, 256, 0, st, xi, dy, o, rows, D, scale, 1e-6f); LLATTN_LAUNCHED(); }
     return (int)cudaGetLastError();
 }
 

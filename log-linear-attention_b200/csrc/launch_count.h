@@ -3,6 +3,7 @@
 #pragma once
 #include <atomic>
 
+#include "chained_launch.h"
 #include "launch_cache.h"
 
 namespace llattn {

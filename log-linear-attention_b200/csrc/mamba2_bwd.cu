@@ -79,6 +79,7 @@ struct Bwd1Smem {
 
 template <int KD, int VD, int MLOW>
 __global__ void __launch_bounds__(256, 1) m2_bwd_fwdorder_kernel(const Mamba2Params p) {
+    chain_wait();
     using SM = Bwd1Smem<KD, VD, MLOW>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, LDP = SM::LDP;
     constexpr int SEG = 1 << MLOW, MT = KD / 64, NPS = VD / 32, NPK = KD / 32;
@@ -377,6 +378,7 @@ struct Bwd2Smem {
 
 template <int KD, int VD, int MLOW>
 __global__ void __launch_bounds__(256, 1) m2_bwd_revorder_kernel(const Mamba2Params p) {
+    chain_wait();
     using SM = Bwd2Smem<KD, VD, MLOW>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, LDP = SM::LDP;
     constexpr int SEG = 1 << MLOW, MT = KD / 64, NPS = VD / 32, NPK = KD / 32;
@@ -651,6 +653,7 @@ struct HiBwdSmem {
 
 template <int KD, int VD, int MLOW>
 __global__ void __launch_bounds__(256, 1) m2_hi_bwd_q_kernel(const Mamba2Params p) {
+    chain_wait();
     using SM = HiBwdSmem<KD, VD>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, SEG = 1 << MLOW, NPK = KD / 32;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -782,6 +785,7 @@ struct SegDSmem {
 
 template <int KD, int VD, int MLOW>
 __global__ void __launch_bounds__(256, 1) m2_seg_dstate_kernel(const Mamba2Params p) {
+    chain_wait();
     using SM = SegDSmem<KD, VD, MLOW>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, SEG = SM::SEG, MT = KD / 64, NPS = VD / 32;
     const int j = blockIdx.y;
@@ -886,6 +890,7 @@ __device__ __forceinline__ float2 ldg2_if(const float* ptr, bool p) {
 
 template <int LH>
 __global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p, int KV) {
+    chain_wait();
     const long bh = blockIdx.y;
     const int e2 = (blockIdx.x * 128 + threadIdx.x) * 2;
     if (e2 >= KV) return;                       // whole warps: KV is a multiple of 64
@@ -956,7 +961,7 @@ template <int LH>
 static void launch_dscan(const Mamba2Params& p, int KV, cudaStream_t stream) {
     if constexpr (LH > 0) {
         if (p.LH != LH) return launch_dscan<LH - 1>(p, KV, stream);
-        m2_seg_dscan_kernel<LH><<<dim3((KV / 2 + 127) / 128, p.B * p.H), 128, 0, stream>>>(p, KV);
+        llattn::launch_chained(m2_seg_dscan_kernel<LH>, dim3((KV / 2 + 127) / 128, p.B * p.H), 128, 0, stream, p, KV);
         LLATTN_LAUNCHED();
     }
 }
@@ -969,6 +974,7 @@ static void launch_dscan(const Mamba2Params& p, int KV, cudaStream_t stream) {
 __global__ void __launch_bounds__(256) m2_bwd_init_kernel(const float* __restrict__ gc, float* __restrict__ g, unsigned n, unsigned H,
                                                           float4* __restrict__ acc, long acc4, float4* __restrict__ dl, long dl4,
                                                           float* __restrict__ dl_tail, int ntail) {
+    chain_wait();
     const long i0 = (long)blockIdx.x * 256 + threadIdx.x, step = (long)gridDim.x * 256;
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     for (long i = i0; i < acc4; i += step) acc[i] = z;
@@ -1018,6 +1024,7 @@ __device__ __forceinline__ float half_prefix(float v, int half, int lane) {     
 
 template <int MLOW>
 __global__ void __launch_bounds__(256) m2_dg_table_kernel(const Mamba2Params p, int nlev) {
+    chain_wait();
     constexpr int SEG = 1 << MLOW;
     const long bh = blockIdx.x;
     const int lv = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1085,6 +1092,7 @@ __global__ void __launch_bounds__(256) m2_dg_table_kernel(const Mamba2Params p, 
 }
 
 __global__ void __launch_bounds__(128) m2_dg_kernel(const Mamba2Params p, float* __restrict__ dg) {
+    chain_wait();
     const long i = (long)blockIdx.x * 128 + threadIdx.x;               // (batch, chunk, head)
     if (i >= (long)p.B * p.NT * p.H) return;
     const int h = (int)(i % p.H);
@@ -1105,6 +1113,7 @@ __global__ void __launch_bounds__(128) m2_dg_kernel(const Mamba2Params p, float*
 }
 
 __global__ void m2_cast_bf16_kernel(const float* __restrict__ src, bf16* __restrict__ dst, long n) {
+    chain_wait();
     const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i + 3 < n) {
         float4 x = *reinterpret_cast<const float4*>(src + i);
@@ -1126,7 +1135,7 @@ static int launch_fwdorder(const Mamba2Params& p, bool use_tc, cudaStream_t stre
     cudaError_t e;
     auto kern = m2_bwd_fwdorder_kernel<KD, VD, MLOW>;
     if ((e = allow_smem(kern, Bwd1Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * p.NS, 256, Bwd1Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * p.NS, 256, Bwd1Smem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
@@ -1144,13 +1153,13 @@ static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStre
             {
                 auto kern = m2_hi_bwd_q_kernel<KD, VD, MLOW>;
                 if ((e = allow_smem(kern, HiBwdSmem<KD, VD>::total)) != cudaSuccess) return (int)e;
-                kern<<<p.B * p.H * (p.NT - SEG), 256, HiBwdSmem<KD, VD>::total, stream>>>(p); LLATTN_LAUNCHED();
+                llattn::launch_chained(kern, p.B * p.H * (p.NT - SEG), 256, HiBwdSmem<KD, VD>::total, stream, p); LLATTN_LAUNCHED();
             }
             {
                 auto kern = m2_seg_dstate_kernel<KD, VD, MLOW>;
                 if ((e = allow_smem(kern, SegDSmem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
                 dim3 grid(p.B * p.H * (p.NS - 1), p.LH);
-                kern<<<grid, 256, SegDSmem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
+                llattn::launch_chained(kern, grid, 256, SegDSmem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
             }
         }
         launch_dscan<M2_MAX_LH>(p, KV, stream);
@@ -1158,7 +1167,7 @@ static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStre
     if (use_tc) return mamba2_bwd2_tc_launch(p, stream);
     auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;
     if ((e = allow_smem(kern, Bwd2Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * p.NS, 256, Bwd2Smem<KD, VD, MLOW>::total, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * p.NS, 256, Bwd2Smem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
@@ -1206,7 +1215,7 @@ int mamba2_bwd_init(const float* gc, float* g, long BT, int H, void* acc, size_t
     if (acc4 > most) most = acc4;
     if (dl4 > most) most = dl4;
     const long blocks = (most + 255) / 256;
-    m2_bwd_init_kernel<<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream>>>(
+    llattn::launch_chained(m2_bwd_init_kernel, (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, 
         gc, g, (unsigned)(BT * H), (unsigned)H, (float4*)acc, acc4, (float4*)dl, dl4, dl + dl4 * 4, (int)tail);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
@@ -1215,14 +1224,14 @@ int mamba2_bwd_init(const float* gc, float* g, long BT, int H, void* acc, size_t
 int mamba2_dg(const Mamba2Params& p, float* dg, cudaStream_t stream) {
     int nlev = 0;
     while ((1 << nlev) < p.NT) ++nlev;          // inter-chunk levels in use
-    m2_dg_table_kernel<M2_MLOW><<<dim3(p.B * p.H, nlev + 1), 256, 0, stream>>>(p, nlev); LLATTN_LAUNCHED();
-    m2_dg_kernel<<<(unsigned)(((long)p.B * p.NT * p.H + 127) / 128), 128, 0, stream>>>(p, dg); LLATTN_LAUNCHED();
+    llattn::launch_chained(m2_dg_table_kernel<M2_MLOW>, dim3(p.B * p.H, nlev + 1), 256, 0, stream, p, nlev); LLATTN_LAUNCHED();
+    llattn::launch_chained(m2_dg_kernel, (unsigned)(((long)p.B * p.NT * p.H + 127) / 128), 128, 0, stream, p, dg); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
 void cast_f32_to_bf16(const float* src, void* dst, long n, cudaStream_t stream) {
     const long thr = (n + 3) / 4;
-    m2_cast_bf16_kernel<<<(unsigned)((thr + 255) / 256), 256, 0, stream>>>(src, reinterpret_cast<bf16*>(dst), n); LLATTN_LAUNCHED();
+    llattn::launch_chained(m2_cast_bf16_kernel, (unsigned)((thr + 255) / 256), 256, 0, stream, src, reinterpret_cast<bf16*>(dst), n); LLATTN_LAUNCHED();
 }
 
 }  // namespace llattn

@@ -47,6 +47,7 @@ __device__ __forceinline__ uint32_t box_offset(int row, int col) {
 
 template <int MLOW>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(const __grid_constant__ Mamba2Params p) {
+    chain_wait();
     using SM = Bwd1TcSmem<MLOW>;
     constexpr int MP = SM::MP;
     constexpr int SEGP = 1 << MP;
@@ -752,6 +753,7 @@ struct Bwd2TcSmem {
 
 template <int MLOW>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(const __grid_constant__ Mamba2Params p) {
+    chain_wait();
     using SM = Bwd2TcSmem<MLOW>;
     constexpr int MP = SM::MP;
     constexpr int SEGP = 1 << MP;
@@ -1314,7 +1316,7 @@ int mamba2_bwd2_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     const size_t sm = Bwd2TcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * p.NS, tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * p.NS, tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
@@ -1336,7 +1338,7 @@ int mamba2_bwd1_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
     if ((e = sm_count(&sms, dev)) != cudaSuccess) return (int)e;
     const int nitems = p.B * p.H * p.NS;
-    kern<<<nitems < sms ? nitems : sms, tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();      // persistent: one CTA per SM
+    llattn::launch_chained(kern, nitems < sms ? nitems : sms, tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();      // persistent: one CTA per SM
     return (int)cudaGetLastError();
 }
 

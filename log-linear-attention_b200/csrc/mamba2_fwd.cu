@@ -43,6 +43,7 @@ struct FwdSmem {
 
 template <int KD, int VD, int MLOW>
 __global__ void __launch_bounds__(256, 1) m2_chunk_fwd_kernel(const Mamba2Params p) {
+    chain_wait();
     using SM = FwdSmem<KD, VD, MLOW>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, LDP = SM::LDP;
     constexpr int SEG = 1 << MLOW;
@@ -290,6 +291,7 @@ struct SegSmem {
 
 template <int KD, int VD, int MLOW>
 __global__ void __launch_bounds__(256, 1) m2_seg_state_kernel(const Mamba2Params p) {
+    chain_wait();
     using SM = SegSmem<KD, VD, MLOW>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, SEG = SM::SEG;
     constexpr int MT = KD / 64, NPS = VD / 32;
@@ -386,6 +388,7 @@ __global__ void __launch_bounds__(256, 1) m2_seg_state_kernel(const Mamba2Params
 constexpr int MAX_LH = 10;
 
 __global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p, int KV) {
+    chain_wait();
     const long bh = blockIdx.y;
     const int e4 = (blockIdx.x * 256 + threadIdx.x) * 4;
     if (e4 >= KV) return;
@@ -459,6 +462,7 @@ struct HiSmem {
 
 template <int KD, int VD, int MLOW>
 __global__ void __launch_bounds__(256, 1) m2_hi_out_kernel(const Mamba2Params p) {
+    chain_wait();
     using SM = HiSmem<KD, VD>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, SEG = 1 << MLOW, NPS = VD / 32;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -582,11 +586,11 @@ static int launch_states(Mamba2Params p, cudaStream_t stream) {
         auto kern = m2_seg_state_kernel<KD, VD, MLOW>;
         size_t sm = SegSmem<KD, VD, MLOW>::total;
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-        kern<<<p.B * p.H * (p.NS - 1), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), 256, sm, stream, p); LLATTN_LAUNCHED();
     }
     const int KV = KD * VD;
     dim3 grid((KV / 4 + 255) / 256, p.B * p.H);
-    m2_seg_scan_kernel<<<grid, 256, 0, stream>>>(p, KV); LLATTN_LAUNCHED();
+    llattn::launch_chained(m2_seg_scan_kernel, grid, 256, 0, stream, p, KV); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
@@ -605,7 +609,7 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
             auto kern = m2_hi_out_kernel<KD, VD, MLOW>;
             size_t sm = HiSmem<KD, VD>::total;
             if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-            kern<<<p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+            llattn::launch_chained(kern, p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream, p); LLATTN_LAUNCHED();
         }
     }
     if (use_tc) {
@@ -615,7 +619,7 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
         auto kern = m2_chunk_fwd_kernel<KD, VD, MLOW>;
         size_t sm = FwdSmem<KD, VD, MLOW>::total;
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-        kern<<<p.B * p.H * p.NS, 256, sm, stream>>>(p); LLATTN_LAUNCHED();
+        llattn::launch_chained(kern, p.B * p.H * p.NS, 256, sm, stream, p); LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();
 }

@@ -32,6 +32,7 @@ struct FwdTcSmem {
 
 template <int MLOW>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const __grid_constant__ Mamba2Params p) {
+    chain_wait();
     using SM = FwdTcSmem<MLOW>;
     constexpr int MP = SM::MP;
     constexpr int SEGP = 1 << MP;                    // pairs per segment
@@ -490,7 +491,7 @@ int mamba2_fwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     const size_t sm = FwdTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * p.NS, tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * p.NS, tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

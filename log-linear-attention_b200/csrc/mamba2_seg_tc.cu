@@ -69,6 +69,7 @@ struct HiBwdTcSmem {
 
 template <int MLOW>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __grid_constant__ Mamba2Params p) {
+    chain_wait();
     using SM = HiBwdTcSmem<MLOW>;
     constexpr int SEG = SM::SEG, NDLH = tcs::MAXLH + 1;
     // tensor memory: dF slots 0..4 (64 columns each), dq (128 columns), T (64 columns).  The level reads
@@ -403,6 +404,7 @@ struct HiOutTcSmem {
 
 template <int MLOW, int MAXL>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __grid_constant__ Mamba2Params p) {
+    chain_wait();
     using SM = HiOutTcSmem<MLOW, MAXL>;
     static_assert(MAXL * 64 <= tc::TM_COLS, "one 64-column tensor-memory slot per level");
     constexpr int SEG = SM::SEG;
@@ -553,6 +555,7 @@ struct SegStateTcSmem {
 
 template <int MLOW>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_seg_state_tc_kernel(const __grid_constant__ Mamba2Params p) {
+    chain_wait();
     using SM = SegStateTcSmem<MLOW>;
     constexpr int SEG = SM::SEG, SEGP = SEG / 2;
     extern __shared__ unsigned char smem_raw[];
@@ -691,7 +694,7 @@ int mamba2_seg_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     const size_t sm = SegStateTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
-    kern<<<p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
@@ -707,13 +710,13 @@ int mamba2_hi_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
         const size_t sm = HiOutTcSmem<M2_MLOW, 5>::total;
         cudaError_t e = allow_smem(kern, sm);
         if (e != cudaSuccess) return (int)e;
-        kern<<<p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
+        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     } else {
         auto kern = m2_hi_out_tc_kernel<M2_MLOW, 8>;
         const size_t sm = HiOutTcSmem<M2_MLOW, 8>::total;
         cudaError_t e = allow_smem(kern, sm);
         if (e != cudaSuccess) return (int)e;
-        kern<<<p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream>>>(p); LLATTN_LAUNCHED();
+        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();
 }
@@ -733,7 +736,7 @@ int mamba2_hi_bwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     // one launch per window of five segment levels (a single one up to T = 16384); dq, the q.dq totals and
     // the per-level outputs of different windows add up or are disjoint
     for (p.lev_lo = 0; p.lev_lo < p.LH; p.lev_lo += tcs::MAXLH) {
-        kern<<<p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream>>>(p);
+        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p);
         LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();

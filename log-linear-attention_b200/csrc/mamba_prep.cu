@@ -38,6 +38,7 @@ struct PrepArgs {
 // with the next token in flight, 212 us with two and a thread per lambda column).
 template <int LPR>
 __global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_constant__ PrepArgs a) {
+    chain_wait();
     constexpr int U = 2;
     const int lam_grid = a.lam_blocks * a.lam_runs;
     if ((int)blockIdx.x < lam_grid) {
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_consta
 // d dt_bias, dD (H) and dL (H,L): one global atomic per thread and entry at the end of the run.
 template <int LPR>
 __global__ void __launch_bounds__(256, 4) m2_prep_bwd_kernel(const __grid_constant__ PrepArgs a) {
+    chain_wait();
     const int lam_grid = a.lam_blocks * a.lam_runs;
     if ((int)blockIdx.x < lam_grid) {
         const int per = (a.tokens + a.lam_runs - 1) / a.lam_runs, t0 = blockIdx.x / a.lam_blocks * per, t1 = min(a.tokens, t0 + per);
@@ -153,6 +155,7 @@ __global__ void __launch_bounds__(256, 4) m2_prep_bwd_kernel(const __grid_consta
 template <int LPR, bool F32OUT>
 __global__ void __launch_bounds__(256) m2_residual_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ x,
                                                           const float* __restrict__ D, void* __restrict__ y, long rows, int H, int P) {
+    chain_wait();
     const int lane = threadIdx.x % LPR;
     const long row = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
     if (row >= rows || lane * 8 >= P) return;
@@ -226,10 +229,10 @@ int llattn_mamba2_layer_prep_fwd(const void* x, const void* dt_raw, const void* 
     a.v = (bf*)v; a.lam = (bf*)lambda; a.g = g;
     int threads;
     const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, false, threads);
-    if (a.lpr == 4) llattn::m2_prep_fwd_kernel<4><<<grid, threads, 0, st>>>(a);
-    else if (a.lpr == 8) llattn::m2_prep_fwd_kernel<8><<<grid, threads, 0, st>>>(a);
-    else if (a.lpr == 16) llattn::m2_prep_fwd_kernel<16><<<grid, threads, 0, st>>>(a);
-    else llattn::m2_prep_fwd_kernel<32><<<grid, threads, 0, st>>>(a);
+    if (a.lpr == 4) llattn::launch_chained(llattn::m2_prep_fwd_kernel<4>, grid, threads, 0, st, a);
+    else if (a.lpr == 8) llattn::launch_chained(llattn::m2_prep_fwd_kernel<8>, grid, threads, 0, st, a);
+    else if (a.lpr == 16) llattn::launch_chained(llattn::m2_prep_fwd_kernel<16>, grid, threads, 0, st, a);
+    else llattn::launch_chained(llattn::m2_prep_fwd_kernel<32>, grid, threads, 0, st, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -257,10 +260,10 @@ int llattn_mamba2_layer_prep_bwd(const void* x, const void* dt_raw, const void* 
     a.dx = (bf*)dx; a.ddt = (bf*)ddt; a.ddl = (bf*)ddl; a.dA = dA; a.dbias = dt_bias ? dbias : nullptr; a.dLp = dLp; a.dD = dD;
     int threads;
     const unsigned grid = prep_grid(a, rows, H, P, L, lambda_mode, true, threads);
-    if (a.lpr == 4) llattn::m2_prep_bwd_kernel<4><<<grid, threads, 0, st>>>(a);
-    else if (a.lpr == 8) llattn::m2_prep_bwd_kernel<8><<<grid, threads, 0, st>>>(a);
-    else if (a.lpr == 16) llattn::m2_prep_bwd_kernel<16><<<grid, threads, 0, st>>>(a);
-    else llattn::m2_prep_bwd_kernel<32><<<grid, threads, 0, st>>>(a);
+    if (a.lpr == 4) llattn::launch_chained(llattn::m2_prep_bwd_kernel<4>, grid, threads, 0, st, a);
+    else if (a.lpr == 8) llattn::launch_chained(llattn::m2_prep_bwd_kernel<8>, grid, threads, 0, st, a);
+    else if (a.lpr == 16) llattn::launch_chained(llattn::m2_prep_bwd_kernel<16>, grid, threads, 0, st, a);
+    else llattn::launch_chained(llattn::m2_prep_bwd_kernel<32>, grid, threads, 0, st, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -283,8 +286,8 @@ int llattn_mamba2_residual(const void* o, const void* x, const float* D, void* y
     const unsigned blocks = (unsigned)((rows * lpr + 255) / 256);
 #define RES(LPRV)                                                                                                          \
     do {                                                                                                                   \
-        if (y_is_f32) llattn::m2_residual_kernel<LPRV, true><<<blocks, 256, 0, st>>>((const bf*)o, (const bf*)x, D, y, rows, H, P);   \
-        else llattn::m2_residual_kernel<LPRV, false><<<blocks, 256, 0, st>>>((const bf*)o, (const bf*)x, D, y, rows, H, P);           \
+        if (y_is_f32) llattn::launch_chained(llattn::m2_residual_kernel<LPRV, true>, blocks, 256, 0, st, (const bf*)o, (const bf*)x, D, y, rows, H, P);   \
+        else llattn::launch_chained(llattn::m2_residual_kernel<LPRV, false>, blocks, 256, 0, st, (const bf*)o, (const bf*)x, D, y, rows, H, P);           \
     } while (0)
     if (lpr == 4) RES(4);
     else if (lpr == 8) RES(8);

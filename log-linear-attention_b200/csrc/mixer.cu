@@ -44,6 +44,7 @@ struct MixerArgs {
 // ---- forward: a thread walks `run` tokens of four neighbouring channels, eight tokens at a time, with the last three inputs in
 // registers.  The sixteen threads of a head share softplus(dt): each evaluates the one of a token in sixteen.
 __global__ void __launch_bounds__(128, 6) mixer_prep_kernel(const __grid_constant__ MixerArgs a) {
+    chain_wait();
     constexpr int N = 4, U = 8;
     const bool vec = (a.W & 3) == 0;
     const int lam_grid = a.lam_blocks * a.B * a.lam_runs;
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(128, 6) mixer_prep_kernel(const __grid_constan
 // evaluated by the next run too.  Sums over tokens (taps, bias, A, dt_bias) stay in registers until the end of the run, and the
 // sixteen threads of a head share what depends on the token alone: each has one token of a block of sixteen.
 __global__ void __launch_bounds__(128, 4) mixer_prep_bwd_kernel(const __grid_constant__ MixerArgs a) {
+    chain_wait();
     constexpr int N = 4, U = 4;
     const bool vec = (a.W & 3) == 0;
     const int lam_grid = a.lam_blocks * a.B * a.lam_runs;
@@ -317,6 +319,7 @@ __device__ __forceinline__ float block_sum(float v, float (&s)[2][16], int turn)
 // ---- out = RMSNorm((o + D x) silu(z)) w, one CTA a token, NV groups of eight columns a thread
 template <int NV>
 __global__ void __launch_bounds__(512) mixer_norm_kernel(const __grid_constant__ NormArgs a) {
+    chain_wait();
     __shared__ float sred[2][16];
     const int tid = threadIdx.x;
     const bool vec = (a.W & 7) == 0;
@@ -354,6 +357,7 @@ __global__ void __launch_bounds__(512) mixer_norm_kernel(const __grid_constant__
 // ---- its backward: persistent CTAs walk the tokens, so that the sums over tokens (w, D) stay in registers
 template <int NV, int THREADS>
 __global__ void __launch_bounds__(THREADS, NV == 1 ? 768 / THREADS : 1) mixer_norm_bwd_kernel(const __grid_constant__ NormArgs a) {
+    chain_wait();
     __shared__ float sred[2][16];
     const int tid = threadIdx.x, lane = tid & 31;
     int turn = 0;
@@ -469,7 +473,7 @@ int llattn_mixer_prep_fwd(const void* zx, const void* conv_w, int conv_w_f32, co
     a.run = mixer_run(B, T, ch / 128 + 1, 16, 64);
     mixer_lambda_blocks(a, false);
     const unsigned grid = (unsigned)(a.conv_blocks * B * ((T + a.run - 1) / a.run) + a.lam_blocks * B * a.lam_runs);
-    llattn::mixer_prep_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
+    llattn::launch_chained(llattn::mixer_prep_kernel, grid, 128, 0, (cudaStream_t)stream, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -494,7 +498,7 @@ int llattn_mixer_prep_bwd(const void* zx, const void* conv_w, int conv_w_f32, co
     a.run = mixer_run(B, T, ch / 128 + 1, 16, 128);
     mixer_lambda_blocks(a, true);
     const unsigned grid = (unsigned)(a.conv_blocks * B * ((T + a.run - 1) / a.run) + a.lam_blocks * B * a.lam_runs);
-    llattn::mixer_prep_bwd_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
+    llattn::launch_chained(llattn::mixer_prep_bwd_kernel, grid, 128, 0, (cudaStream_t)stream, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -516,8 +520,8 @@ int llattn_mixer_norm_fwd(const void* o, const void* x, const void* D, int d_f32
     a.o = (const bf*)o; a.x = (const bf*)x; a.zx = (const bf*)zx; a.D = D; a.d_f32 = d_f32; a.w = w; a.w_f32 = w_f32;
     a.out = (bf*)out; a.rstd = rstd; a.rows = (int)rows; a.dim = H * llattn::MX_P; a.W = zx_width; a.eps = eps;
     cudaStream_t st = (cudaStream_t)stream;
-    if (a.dim <= 4096) llattn::mixer_norm_kernel<1><<<(unsigned)rows, norm_threads(a.dim), 0, st>>>(a);
-    else llattn::mixer_norm_kernel<2><<<(unsigned)rows, 512, 0, st>>>(a);
+    if (a.dim <= 4096) llattn::launch_chained(llattn::mixer_norm_kernel<1>, (unsigned)rows, norm_threads(a.dim), 0, st, a);
+    else llattn::launch_chained(llattn::mixer_norm_kernel<2>, (unsigned)rows, 512, 0, st, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -536,7 +540,7 @@ int llattn_mixer_norm_bwd(const void* o, const void* x, const void* D, int d_f32
     // as many CTAs as are resident (85 registers a thread; 128 for heads beyond 4096 columns)
     auto launch = [&](auto kern, int threads, int per_sm) {
         const long most = 148l * per_sm;
-        kern<<<(unsigned)(rows < most ? rows : most), threads, 0, st>>>(a);
+        llattn::launch_chained(kern, (unsigned)(rows < most ? rows : most), threads, 0, st, a);
     };
     if (a.dim <= 1024) launch(llattn::mixer_norm_bwd_kernel<1, 128>, 128, 6);
     else if (a.dim <= 2048) launch(llattn::mixer_norm_bwd_kernel<1, 256>, 256, 3);

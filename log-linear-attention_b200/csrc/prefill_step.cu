@@ -23,6 +23,7 @@ template <int KD, int VD>
 __global__ void __launch_bounds__(256, 1) mamba2_final_state_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v,
                                                                     const float* __restrict__ g, float* __restrict__ states,
                                                                     int B, int T, int H, int G, int L) {
+    chain_wait();
     constexpr int LDK = KD + PAD, LDV = VD + PAD;
     constexpr int MT = KD / 128;                         // 16-row tiles of the K x V result per warp (8 warps)
     static_assert(KD % 128 == 0 || KD == 64, "K rows are split over the warps");
@@ -144,6 +145,7 @@ template <int KD>
 __global__ void __launch_bounds__(256) mamba2_prompt_state_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v, const float* __restrict__ g,
                                                                   float* __restrict__ states, const float* __restrict__ seg_F,
                                                                   const float* __restrict__ seg_D, int T, int Tp, int H, int G, int L) {
+    chain_wait();
     using SM = PromptStateSmem<KD>;
     constexpr int VD = 64, LDK = SM::LDK, LDV = SM::LDV, KV = KD * VD, SEG = 512;
     constexpr int MT = KD / 64, NPW = VD / 32;           // a warp: 16 MT rows x 32 columns (4 x 2 warps)
@@ -289,6 +291,7 @@ template <int MAXL>
 __global__ void __launch_bounds__(256) mamba2_step_kernel(float* __restrict__ states, const bf16* __restrict__ q, const bf16* __restrict__ k,
                                                           const bf16* __restrict__ v, const float* __restrict__ g, const bf16* __restrict__ lam,
                                                           bf16* __restrict__ o, int H, int G, int K, int V, int L, int carry) {
+    chain_wait();
     extern __shared__ float sh[];                        // q[K] | k[K] | partial outputs [256]
     float* sQ = sh;
     float* sKk = sh + K;
@@ -363,8 +366,9 @@ int llattn_mamba2_final_state(const void* k, const void* v, const float* g, floa
     using bf = __nv_bfloat16;
     dim3 grid(B * H, L);
     cudaStream_t st = (cudaStream_t)stream;
-    if (K == 128) llattn::mamba2_final_state_kernel<128, 64><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, B, T, H, G, L);
-    else llattn::mamba2_final_state_kernel<64, 64><<<grid, 256, 0, st>>>((const bf*)k, (const bf*)v, g, states, B, T, H, G, L);
+    if (K == 128) llattn::launch_chained(llattn::mamba2_final_state_kernel<128, 64>, grid, 256, 0, st, (const bf*)k, (const bf*)v, g, states, B,
+            T, H, G, L);
+    else llattn::launch_chained(llattn::mamba2_final_state_kernel<64, 64>, grid, 256, 0, st, (const bf*)k, (const bf*)v, g, states, B, T, H, G, L);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -385,7 +389,7 @@ int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, fl
     cudaStream_t st = (cudaStream_t)stream;
     auto launch = [&](auto kern, size_t sm) -> cudaError_t {
         const cudaError_t e = llattn::allow_smem(kern, sm);
-        if (e == cudaSuccess) kern<<<grid, 256, sm, st>>>((const bf*)k, (const bf*)v, g, states, seg_F, seg_D, T, Tp, H, G, L);
+        if (e == cudaSuccess) llattn::launch_chained(kern, grid, 256, sm, st, (const bf*)k, (const bf*)v, g, states, seg_F, seg_D, T, Tp, H, G, L);
         return e;
     };
     const cudaError_t e = K == 128 ? launch(llattn::mamba2_prompt_state_kernel<128>, llattn::PromptStateSmem<128>::total)
@@ -405,9 +409,11 @@ int llattn_mamba2_step(float* states, const void* q, const void* k, const void* 
     cudaStream_t st = (cudaStream_t)stream;
     const size_t sm = (size_t)(2 * K + 256) * sizeof(float);
     if (L <= 16)
-        llattn::mamba2_step_kernel<16><<<B * H, 256, sm, st>>>(states, (const bf*)q, (const bf*)k, (const bf*)v, g, (const bf*)lambda, (bf*)o, H, G, K, V, L, carry_level);
+        llattn::launch_chained(llattn::mamba2_step_kernel<16>, B * H, 256, sm, st, states, (const bf*)q, (const bf*)k, (const bf*)v, g,
+                (const bf*)lambda, (bf*)o, H, G, K, V, L, carry_level);
     else
-        llattn::mamba2_step_kernel<32><<<B * H, 256, sm, st>>>(states, (const bf*)q, (const bf*)k, (const bf*)v, g, (const bf*)lambda, (bf*)o, H, G, K, V, L, carry_level);
+        llattn::launch_chained(llattn::mamba2_step_kernel<32>, B * H, 256, sm, st, states, (const bf*)q, (const bf*)k, (const bf*)v, g,
+                (const bf*)lambda, (bf*)o, H, G, K, V, L, carry_level);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(256) m2_prompt_prep_kernel(const bf16* __restr
                                                              const uint4* __restrict__ q, const uint4* __restrict__ k, bf16* __restrict__ v,
                                                              float* __restrict__ g, bf16* __restrict__ lam, uint4* __restrict__ qp, uint4* __restrict__ kp,
                                                              int B, int T, int Tp, int H, int P, int L, int Lo, int mode, int row_blocks, int qk16) {
+    chain_wait();
     if ((int)blockIdx.x >= row_blocks) {
         // qk16: 16-byte words of a token of q (and of k)
         const unsigned e = (blockIdx.x - row_blocks) * 256u + threadIdx.x;
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(256) m2_prompt_prep_kernel(const bf16* __restr
 template <bool F32OUT>
 __global__ void __launch_bounds__(256) m2_prompt_residual_kernel(const bf16* __restrict__ o, const bf16* __restrict__ x, const void* __restrict__ D,
                                                                  void* __restrict__ y, int B, int T, int Tp, int H, int P) {
+    chain_wait();
     const unsigned p8 = P / 8;
     const unsigned e = blockIdx.x * 256u + threadIdx.x;
     const unsigned row = e / p8, c = (e % p8) * 8;
@@ -119,6 +121,7 @@ struct PadList {
 };
 
 __global__ void __launch_bounds__(256) pad_tokens_kernel(const __grid_constant__ PadList l) {
+    chain_wait();
     int i = 0;
     while (i + 1 < l.n && blockIdx.x >= l.first_block[i + 1]) ++i;
     const unsigned per = l.dst_bytes[i] / l.unit[i], real = l.src_bytes[i] / l.unit[i];
@@ -150,6 +153,7 @@ struct GdnPrepArgs {
 };
 
 __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_constant__ GdnPrepArgs a) {
+    chain_wait();
     const int lane = threadIdx.x & 15;
     const unsigned row = blockIdx.x * 16u + (threadIdx.x >> 4);
     const unsigned heads = a.H * a.rep, rows = (unsigned)a.B * a.Tp * heads;
@@ -224,6 +228,7 @@ constexpr int TAIL_KD = 128;
 __global__ void __launch_bounds__(256) gdn_tail_states_kernel(const bf16* __restrict__ kn, const bf16* __restrict__ v, const bf16* __restrict__ beta,
                                                               const float* __restrict__ g, float* __restrict__ states, int T, int Tp, int H,
                                                               int K, int Vs, int rep, int L) {
+    chain_wait();
     constexpr int KR = TAIL_KD / 32;
     __shared__ __align__(16) bf16 sK[CH * TAIL_KD];
     __shared__ float sV[CH][33];
@@ -326,7 +331,7 @@ int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_
     const int row_blocks = (int)((rows * lpr + 255) / 256);
     const unsigned grid = row_blocks + (unsigned)((copies + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
-#define LLATTN_PP(N) llattn::m2_prompt_prep_kernel<N><<<grid, 256, 0, st>>>((const bf*)x, (const bf*)dt_raw, dt_bias, bias_is_f32, A, (const bf*)dl, Lp, lp_is_f32, (const uint4*)q, (const uint4*)k, (bf*)v, g, (bf*)lambda, (uint4*)q_pad, (uint4*)k_pad, B, T, Tp, H, P, L, L_out, lambda_mode, row_blocks, qk16)
+#define LLATTN_PP(N) llattn::launch_chained(llattn::m2_prompt_prep_kernel<N>, grid, 256, 0, st, (const bf*)x, (const bf*)dt_raw, dt_bias, bias_is_f32, A, (const bf*)dl, Lp, lp_is_f32, (const uint4*)q, (const uint4*)k, (bf*)v, g, (bf*)lambda, (uint4*)q_pad, (uint4*)k_pad, B, T, Tp, H, P, L, L_out, lambda_mode, row_blocks, qk16)
     if (lpr == 8) LLATTN_PP(8);
     else if (lpr == 16) LLATTN_PP(16);
     else LLATTN_PP(32);
@@ -341,8 +346,8 @@ int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, v
     using bf = __nv_bfloat16;
     const unsigned grid = (unsigned)(((long)B * T * H * (P / 8) + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
-    if (y_is_f32) llattn::m2_prompt_residual_kernel<true><<<grid, 256, 0, st>>>((const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
-    else llattn::m2_prompt_residual_kernel<false><<<grid, 256, 0, st>>>((const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
+    if (y_is_f32) llattn::launch_chained(llattn::m2_prompt_residual_kernel<true>, grid, 256, 0, st, (const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
+    else llattn::launch_chained(llattn::m2_prompt_residual_kernel<false>, grid, 256, 0, st, (const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -365,7 +370,7 @@ int llattn_pad_tokens(int n, const void* const* src, void* const* dst, const int
     }
     if (blocks > 0x7ffffffful) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     l.first_block[n] = (unsigned)blocks;
-    llattn::pad_tokens_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(l);
+    llattn::launch_chained(llattn::pad_tokens_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, l);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -383,7 +388,7 @@ int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const vo
     llattn::GdnPrepArgs a{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, (const bf*)lambda, (bf*)qn, (bf*)kn, (bf*)v_pad,
                           (bf*)beta_pad, g_pad, (bf*)lambda_pad, B, T, Tp, H, G, K, K_out, V, rep, L, L_out, scale, lambda_mul};
     const unsigned grid = (unsigned)(((long)B * Tp * H * rep + 15) / 16);
-    llattn::gdn_prompt_prep_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
+    llattn::launch_chained(llattn::gdn_prompt_prep_kernel, grid, 256, 0, (cudaStream_t)stream, a);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
@@ -396,7 +401,8 @@ int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, co
     if (!kn || !v || !beta || !g || !states) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
     dim3 grid(B * H, L, V / 32);
-    llattn::gdn_tail_states_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const bf*)kn, (const bf*)v, (const bf*)beta, g, states, T, Tp, H, K, V, rep, L);
+    llattn::launch_chained(llattn::gdn_tail_states_kernel, grid, 256, 0, (cudaStream_t)stream, (const bf*)kn, (const bf*)v, (const bf*)beta, g,
+            states, T, Tp, H, K, V, rep, L);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
