@@ -52,7 +52,7 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
     p.LH = ceil_log2i(p.NS);
     p.o_has_high = p.NS > 1;
     p.LZ = llattn::M2_MLOW + p.LH;
-    const size_t KV = (size_t)p.K * p.V, BH = (size_t)p.B * p.H;
+    const size_t KV = llattn::M2_KV, BH = (size_t)p.B * p.H;
     Carver c(ws);
     p.err = c.take<int>(64);      // status word first (256 bytes)
     if (backward) {
@@ -70,7 +70,7 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
         p.seg_F = c.take<float>(BH * p.NS * KV);
         p.seg_D = c.take<float>(BH * p.NS);
         p.seg_H0 = c.take<__nv_bfloat16>(BH * p.NS * p.LH * KV);
-        p.o_hi = c.take<__nv_bfloat16>((size_t)p.B * p.T * p.H * p.V);
+        p.o_hi = c.take<__nv_bfloat16>(BH * ((p.NT + 1) / 2) * 128 * p.V);      // whole pairs of chunks
     }
     if (backward && p.NS > 1) {
         p.seg_dF = c.take<float>(BH * p.NS * p.LH * KV);
@@ -205,10 +205,10 @@ int llattn_mamba2_bwd(const void* q, const void* k, const void* v, const float* 
                                    nullptr, 0, B, T, H, G, K, V, L, stream);
 }
 
-int llattn_mamba2_bwd_saved(const void* q, const void* k, const void* v, const float* g_cum, const void* lambda,
-                            const void* d_o, void* dq, void* dk, void* dv, float* dg, float* dlambda,
-                            void* workspace, size_t workspace_bytes, const void* fwd_workspace, size_t fwd_workspace_bytes,
-                            int B, int T, int H, int G, int K, int V, int L, void* stream) {
+static int mamba2_bwd_impl(const void* q, const void* k, const void* v, const float* g_cum, const void* lambda,
+                           const void* d_o, void* dq, void* dk, void* dv, float* dg, float* dlambda,
+                           void* workspace, size_t workspace_bytes, const void* fwd_workspace, size_t fwd_workspace_bytes,
+                           int B, int T, int H, int G, int K, int V, int L, int chunk_rounding, void* stream) {
     int rc = check_shape(B, T, H, G, K, V, L);
     if (rc != 0) return rc;
     if (!q || !k || !v || !g_cum || !lambda || !d_o || !dq || !dk || !dv || !dg || !dlambda) return LLATTN_ERR_NULL;
@@ -228,6 +228,7 @@ int llattn_mamba2_bwd_saved(const void* q, const void* k, const void* v, const f
         p.reuse_states = 1;
     }
     cudaStream_t st = (cudaStream_t)stream;
+    p.chunk_rounding = chunk_rounding;
     p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
     p.l = (const __nv_bfloat16*)lambda; p.d_o = (const __nv_bfloat16*)d_o;
     p.dv = (__nv_bfloat16*)dv; p.dl = dlambda;
@@ -246,6 +247,22 @@ int llattn_mamba2_bwd_saved(const void* q, const void* k, const void* v, const f
         llattn::cast_f32_to_bf16(p.dk_acc, dk, (long)nqk, st);
     }
     return (int)cudaGetLastError();
+}
+
+int llattn_mamba2_bwd_saved(const void* q, const void* k, const void* v, const float* g_cum, const void* lambda,
+                            const void* d_o, void* dq, void* dk, void* dv, float* dg, float* dlambda,
+                            void* workspace, size_t workspace_bytes, const void* fwd_workspace, size_t fwd_workspace_bytes,
+                            int B, int T, int H, int G, int K, int V, int L, void* stream) {
+    return mamba2_bwd_impl(q, k, v, g_cum, lambda, d_o, dq, dk, dv, dg, dlambda, workspace, workspace_bytes, fwd_workspace, fwd_workspace_bytes,
+                           B, T, H, G, K, V, L, 0, stream);
+}
+
+int llattn_mamba2_bwd_layer(const void* q, const void* k, const void* v, const float* g_cum, const void* lambda,
+                            const void* d_o, void* dq, void* dk, void* dv, float* dg, float* dlambda,
+                            void* workspace, size_t workspace_bytes, const void* fwd_workspace, size_t fwd_workspace_bytes,
+                            int B, int T, int H, int G, int K, int V, int L, void* stream) {
+    return mamba2_bwd_impl(q, k, v, g_cum, lambda, d_o, dq, dk, dv, dg, dlambda, workspace, workspace_bytes, fwd_workspace, fwd_workspace_bytes,
+                           B, T, H, G, K, V, L, 1, stream);
 }
 
 // ---------------------------------------------------------------- Gated DeltaNet

@@ -23,7 +23,7 @@ using torch::autograd::Variable;
 using torch::autograd::variable_list;
 
 #define LLATTN_FUNCS(F)                                                                                                             \
-    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved)        \
+    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
     F(llattn_mamba2_layer_prep_fwd) F(llattn_mamba2_layer_prep_bwd) F(llattn_mamba2_layer_step) F(llattn_gdn_layer_step)            \
     F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mixer_prep_fwd)            \
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
@@ -132,7 +132,7 @@ struct ScanGrads {
     Tensor dq, dk, dv, dg, dl;       // dl fp32
 };
 ScanGrads mamba2_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g_cum, const Tensor& l, const Tensor& d_o, const Tensor& fws,
-                     void* stream, bool status) {
+                     void* stream, bool status, bool layer) {
     const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
     ScanGrads r;
     const Tensor qk = empty({2, B, T, G, K}, at::kBFloat16, q);      // side by side: one conversion pass writes both
@@ -143,9 +143,9 @@ ScanGrads mamba2_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     r.dl = empty(l.sizes(), at::kFloat, l);
     const size_t n = lib.llattn_mamba2_bwd_workspace_bytes(B, T, H, G, K, V, L);
     const Tensor ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
-    check(lib.llattn_mamba2_bwd_saved(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g_cum), l.data_ptr(), d_o.data_ptr(), r.dq.data_ptr(),
-                                      r.dk.data_ptr(), r.dv.data_ptr(), fptr(r.dg), fptr(r.dl), ws.data_ptr(), ws.numel(), ptr(fws),
-                                      fws.defined() ? fws.numel() : 0, B, T, H, G, K, V, L, stream),
+    const auto bwd = layer ? lib.llattn_mamba2_bwd_layer : lib.llattn_mamba2_bwd_saved;
+    check(bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g_cum), l.data_ptr(), d_o.data_ptr(), r.dq.data_ptr(), r.dk.data_ptr(), r.dv.data_ptr(),
+              fptr(r.dg), fptr(r.dl), ws.data_ptr(), ws.numel(), ptr(fws), fws.defined() ? fws.numel() : 0, B, T, H, G, K, V, L, stream),
           "llattn_mamba2_bwd_saved");
     if (status) check_status(ws, stream, "llattn_mamba2_bwd_saved");
     return r;
@@ -154,13 +154,14 @@ ScanGrads mamba2_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
 // ---- hattention_kernel, Mamba-2 structure
 struct Mamba2Kernel : torch::autograd::Function<Mamba2Kernel> {
     static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool keep,
-                          bool status) {
+                          bool status, bool layer) {
         On on(q);
         const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
         Scan s = mamba2_fwd(q_, k_, v_, g_, l_, on.stream, status);
         if (ctx) {
             ctx->save_for_backward({q_, k_, v_, s.g_cum, l_, keep ? s.ws : Tensor()});
             ctx->saved_data["status"] = status;
+            ctx->saved_data["layer"] = layer;
         }
         return s.o;
     }
@@ -168,12 +169,12 @@ struct Mamba2Kernel : torch::autograd::Function<Mamba2Kernel> {
         const auto s = ctx->get_saved_variables();
         On on(s[0]);
         ScanGrads r = mamba2_bwd(s[0], s[1], s[2], s[3], s[4], d[0].to(at::kBFloat16).contiguous(), s[5], on.stream,
-                                 ctx->saved_data["status"].toBool());
-        return {r.dq, r.dk, r.dv, r.dg, r.dl.to(at::kBFloat16), Tensor(), Tensor()};
+                                 ctx->saved_data["status"].toBool(), ctx->saved_data["layer"].toBool());
+        return {r.dq, r.dk, r.dv, r.dg, r.dl.to(at::kBFloat16), Tensor(), Tensor(), Tensor()};
     }
 };
 
-py::object hattention_mamba2(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool keep, bool status) {
+py::object hattention_mamba2(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool keep, bool status, bool layer) {
     if (!bf16(q) || !bf16(k) || !bf16(v) || !is(g, at::kFloat) || !bf16(l) || k.dim() != 4 || v.dim() != 4 || l.dim() != 4 || q.sizes() != k.sizes() ||
         !same_device({q, k, v, g, l}))
         return py::none();
@@ -182,7 +183,8 @@ py::object hattention_mamba2(const Tensor& q, const Tensor& k, const Tensor& v, 
         !mamba2_shape(T, H, k.size(2), k.size(3), v.size(3), L))
         return py::none();
     py::gil_scoped_release nogil;
-    Tensor o = wants_grad({q, k, v, g, l}) ? Mamba2Kernel::apply(q, k, v, g, l, keep, status) : Mamba2Kernel::forward(nullptr, q, k, v, g, l, false, status);
+    Tensor o = wants_grad({q, k, v, g, l}) ? Mamba2Kernel::apply(q, k, v, g, l, keep, status, layer)
+                                             : Mamba2Kernel::forward(nullptr, q, k, v, g, l, false, status, layer);
     py::gil_scoped_acquire gil;
     return py::cast(o);
 }
@@ -221,7 +223,7 @@ struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
         On on(x);
         const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), L = dl.size(3);
         const Tensor dy = d[0].to(at::kBFloat16).contiguous();
-        ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool());
+        ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool(), true);
         const Tensor dx = at::empty_like(x), ddt = at::empty_like(dt), ddl = at::empty_like(dl);
         const Tensor acc = at::zeros({3 * H + H * L}, at::TensorOptions().dtype(at::kFloat).device(x.device()));
         float* a = fptr(acc);
@@ -273,8 +275,7 @@ py::object mamba2_prompt(const Tensor& x, const Tensor& dt, const Tensor& A, con
     const Tensor D = of(D_), bias = of(bias_);
     if (!layer_operands(x, dt, A, Bm, Cm, dl, Lp, D, bias) || wants_grad({x, dt, A, Bm, Cm, dl, Lp, D, bias})) return py::none();
     const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), G = Bm.size(2), N = Bm.size(3), L = dl.size(3);
-    // an even number of chunks, which the tensor-core kernels take
-    const int Tp = T <= 64 ? 64 : (T + 127) / 128 * 128, Lo = T < 64 ? std::max(L, 7) : L;
+    const int Tp = (T + 63) / 64 * 64, Lo = T < 64 ? std::max(L, 7) : L;
     if (T < 1 || L < 1 + bit_length(T - 1) || !mamba2_shape(Tp, H, G, N, P, Lo)) return py::none();
     Tensor y, states;
     {
@@ -357,7 +358,7 @@ struct Mixer : torch::autograd::Function<Mixer> {
         check(lib.llattn_mixer_norm_bwd(o.data_ptr(), x.data_ptr(), ptr(D), f32(D), z.data_ptr(), W, nw.data_ptr(), f32(nw), dn.data_ptr(), fptr(rstd),
                                         dy.data_ptr(), dzx.data_ptr(), a + at_n, a + at_D, (long)B * T, H, on.stream),
               "llattn_mixer_norm_bwd");
-        ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool());
+        ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool(), true);
         check(lib.llattn_mixer_prep_bwd(z.data_ptr(), cw.data_ptr(), f32(cw), ptr(cb), f32(cb), ptr(bias), f32(bias), fptr(A), Lp.data_ptr(), f32(Lp), ptr(D),
                                         f32(D), r.dv.data_ptr(), dy.data_ptr(), r.dq.data_ptr(), r.dk.data_ptr(), fptr(r.dg), fptr(r.dl), dzx.data_ptr(), a,
                                         a + at_b, a + at_A, a + at_dt, a + at_L, B, T, H, G, N, L, (int)ctx->saved_data["mode"].toInt(), on.stream),

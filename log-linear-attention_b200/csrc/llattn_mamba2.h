@@ -11,6 +11,7 @@
 namespace llattn {
 
 constexpr int M2_MLOW = 3;   // a segment is 2^M2_MLOW chunks (512 tokens)
+constexpr int M2_KV = 128 * 64;   // elements between two segment states (K = 64 uses the first half of them, or has zeros behind them)
 constexpr int M2_MAX_LH = 10;   // segment levels held by the per-level scans over segments (T <= 512 * 2^10)
 
 struct Mamba2Params {
@@ -51,9 +52,11 @@ struct Mamba2Params {
     int NT, NS, LH;
     int o_has_high;
     int lev_lo;                  // first segment level handled by one launch of the tensor-core high-level backward
+    int chunk_rounding;          // backward: a sequence of an odd number of chunks, or with K = 64, takes the chunk-by-chunk kernels
     int reuse_states;            // backward: seg_D / seg_H0 come from the forward call, do not recompute them
 };
 
+bool mamba2_uses_tc(const Mamba2Params& p);
 int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream);
 int mamba2_bwd_dispatch(Mamba2Params p, cudaStream_t stream);
 // segment summaries and the per-level scan over segments only (needs NS > 1)

@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(256, 1) m2_bwd_revorder_kernel(const Mamba2Par
 #pragma unroll
     for (int lv = 0; lv <= MLOW; ++lv) zero_acc(RM[lv]);
     if (p.NS > 1 && r < p.NS - 1) {
-        const float* dH = p.seg_dHf + (((long)b * p.H + h) * p.NS + r) * KD * VD;
+        const float* dH = p.seg_dHf + (((long)b * p.H + h) * p.NS + r) * M2_KV;
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -674,11 +674,10 @@ __global__ void __launch_bounds__(256, 1) m2_hi_bwd_q_kernel(const Mamba2Params 
     const int wr = warp & 3, wc = warp >> 2;
     const int row0 = wr * 16, colk = wc * (KD / 2);
     const int lr = lane >> 2;
-    const long KV = (long)KD * VD;
-    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * KV;
+    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * M2_KV;
 
     auto issue_state = [&](int j, int slot) {
-        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * KV, VD, tid);
+        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * M2_KV, VD, tid);
         cp_async_commit();
     };
     load_tile_async<CH, KD, 256>(sQ, p.q + (((long)b * p.T + t0) * p.G + grp) * KD, (long)p.G * KD, tid);
@@ -858,7 +857,7 @@ __global__ void __launch_bounds__(256, 1) m2_seg_dstate_kernel(const Mamba2Param
         warp_gemm<MT, NPS, true, true>(acc, sQs, LDK, wr * 16 * MT, sDO + st * CH * LDV, LDV, wc * (VD / 2), CH, lane);
         __syncthreads();
     }
-    float* dF = p.seg_dF + ((((long)b * p.H + h) * p.NS + r) * p.LH + j) * KD * VD;
+    float* dF = p.seg_dF + ((((long)b * p.H + h) * p.NS + r) * p.LH + j) * M2_KV;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -894,10 +893,10 @@ __global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p,
     const long bh = blockIdx.y;
     const int e2 = (blockIdx.x * 128 + threadIdx.x) * 2;
     if (e2 >= KV) return;                       // whole warps: KV is a multiple of 64
-    const float* dF = p.seg_dF + bh * p.NS * LH * KV + e2;
-    const float* F = p.seg_F + bh * p.NS * KV + e2;
+    const float* dF = p.seg_dF + bh * p.NS * LH * M2_KV + e2;
+    const float* F = p.seg_F + bh * p.NS * M2_KV + e2;
     const float* D = p.seg_D + bh * p.NS;
-    float* dH = p.seg_dHf + bh * p.NS * KV + e2;
+    float* dH = p.seg_dHf + bh * p.NS * M2_KV + e2;
     float* Yseg = p.Yseg + bh * p.NS * LH;
     const int lane = threadIdx.x & 31;
     float2 st[LH];
@@ -909,10 +908,10 @@ __global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p,
     };
     auto fetch = [&](Loads& L, int r) {
         const bool in = r >= 0 && r < p.NS - 1;
-        L.f = ldg2_if(F + (long)r * KV, in);
+        L.f = ldg2_if(F + (long)r * M2_KV, in);
         L.d = in ? __ldg(D + r) : 0.f;
 #pragma unroll
-        for (int j = 0; j < LH; ++j) L.dF[j] = ldg2_if(dF + ((long)r * LH + j) * KV, r >= 0 && ((r >> j) & 1));
+        for (int j = 0; j < LH; ++j) L.dF[j] = ldg2_if(dF + ((long)r * LH + j) * M2_KV, r >= 0 && ((r >> j) & 1));
     };
     auto process = [&](const Loads& L, int r) {
         float2 out = make_float2(0.f, 0.f);
@@ -941,7 +940,7 @@ __global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p,
 #pragma unroll
             for (int j = 0; j < LH; ++j) mine = lane == j ? y[j] : mine;
             if (lane < LH && !((r >> lane) & 1)) atomicAdd(Yseg + (long)r * LH + lane, mine);
-            *reinterpret_cast<float2*>(dH + (long)r * KV) = out;
+            *reinterpret_cast<float2*>(dH + (long)r * M2_KV) = out;
         }
     };
     Loads A, B;
@@ -1143,10 +1142,8 @@ template <int KD, int VD, int MLOW>
 static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStream_t stream) {
     cudaError_t e;
     constexpr int SEG = 1 << MLOW;
-    const int KV = KD * VD;
     if (p.NS > 1) {
-        const bool hi_tc = (KD == 128 && VD == 64 && (p.NT % 2) == 0 && p.L <= 20 && p.LH <= 10 && g_use_tensor_core_path.load());
-        if (hi_tc) {
+        if (use_tc) {
             const int rc = mamba2_hi_bwd_tc_launch(p, stream);
             if (rc != 0) return rc;
         } else {
@@ -1162,7 +1159,7 @@ static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStre
                 llattn::launch_chained(kern, grid, 256, SegDSmem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
             }
         }
-        launch_dscan<M2_MAX_LH>(p, KV, stream);
+        launch_dscan<M2_MAX_LH>(p, use_tc ? M2_KV : KD * VD, stream);
     }
     if (use_tc) return mamba2_bwd2_tc_launch(p, stream);
     auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;
@@ -1178,7 +1175,7 @@ static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
         // forward high-level states: recomputed unless the caller kept the forward call's workspace
         if ((rc = mamba2_fwd_states_dispatch(p, stream)) != 0) return rc;
     }
-    const bool use_tc = (KD == 128 && VD == 64 && (p.NT % 2) == 0 && p.L <= 20 && g_use_tensor_core_path.load());
+    const bool use_tc = mamba2_uses_tc(p) && !(p.chunk_rounding && (KD != 128 || (p.NT % 2) != 0));
     // The forward-order pass and the chain high levels -> reverse-order pass only meet in the accumulators they add to.  A pass has one CTA
     // per (batch, head, segment) and one fits on an SM: below three waves of them the two run side by side (two of 64 CTAs each then
     // take the time of one), beyond that each fills the chip by itself.

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
         r = (item / p.H) % p.NS;
         b = item / (p.H * p.NS);
         grp = h / (p.H / p.G);
-        npairs = min(SEGP, p.NT / 2 - r * SEGP);
+        npairs = min(SEGP, (p.NT + 1) / 2 - r * SEGP);
     };
     decode(blockIdx.x);
     const int L = p.L;
@@ -132,21 +132,21 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
                 bool ok = true;
                 for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
                     decode(item);
-                    const int brow = b * p.T + r * SEGP * tc::PT;
+                    const int brow = r * SEGP * tc::PT;
                     for (int pl = 0; pl < npairs; ++pl, ++gs) {
                         const int row0 = brow + pl * tc::PT;
                         if (gs >= 1 && !umma::mbar_wait(empty_vd, (gs - 1) & 1, abort_flag)) { ok = false; break; }
                         tma::expect_tx(full_vd, 2 * tc::V_BYTES);
-                        tma::load_panel(sV, &p.tm_v, 0, h, row0, full_vd);
-                        tma::load_panel(sDO, &p.tm_do, 0, h, row0, full_vd);
+                        tma::load_seq_panel(sV, &p.tm_v, 0, h, row0, b, full_vd);
+                        tma::load_seq_panel(sDO, &p.tm_do, 0, h, row0, b, full_vd);
                         if (gs >= 1 && !umma::mbar_wait(empty_qk, (gs - 1) & 1, abort_flag)) { ok = false; break; }
                         tma::expect_tx(full_qk, tc::Q_BYTES);
-                        tma::load_panel(sQ, &p.tm_q, 0, grp, row0, full_qk);
-                        tma::load_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, full_qk);
+                        tma::load_seq_panel(sQ, &p.tm_q, 0, grp, row0, b, full_qk);
+                        tma::load_seq_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, full_qk);
                         if (gs >= 1 && !umma::mbar_wait(empty_k, (gs - 1) & 1, abort_flag)) { ok = false; break; }
                         tma::expect_tx(full_k, tc::Q_BYTES);
-                        tma::load_panel(sK, &p.tm_k, 0, grp, row0, full_k);
-                        tma::load_panel(sK + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, full_k);
+                        tma::load_seq_panel(sK, &p.tm_k, 0, grp, row0, b, full_k);
+                        tma::load_seq_panel(sK + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, b, full_k);
                     }
                 }
             }
@@ -162,25 +162,25 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
                 for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
                   decode(item);
                   for (int pl = 0; pl < npairs; ++pl, ++gs) {
-                    const int grow = b * p.T + (r * SEGP + pl) * tc::PT;
+                    const int grow = (r * SEGP + pl) * tc::PT;
                     // dk first: its staging area is the q / k tile space, which the next pair's loads wait for
                     // (in two halves: columns 0..63 are staged in the q tile as soon as the dk product is complete, columns
                     // 64..127 in the k tile once the whole batch is, so that half of the reduce-add is over by then)
                     if (!umma::mbar_wait(dk_ready, gs & 1, abort_flag)) { ok = false; break; }
 #pragma unroll
-                    for (int bx = 0; bx < 2; ++bx) tma::reduce_add_box(&p.tm_dk, bx * 32, grp, grow, sStage2 + bx * 16384);
+                    for (int bx = 0; bx < 2; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage2 + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();             // the q tile's space has been read: the next q may be loaded
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(empty_qk)) : "memory");
                     if (!umma::mbar_wait(dk_ready1, gs & 1, abort_flag)) { ok = false; break; }
 #pragma unroll
-                    for (int bx = 2; bx < 4; ++bx) tma::reduce_add_box(&p.tm_dk, bx * 32, grp, grow, sStage2 + bx * 16384);
+                    for (int bx = 2; bx < 4; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage2 + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(empty_k)) : "memory");
                     if (!umma::mbar_wait(dq_ready, gs & 1, abort_flag)) { ok = false; break; }
 #pragma unroll
-                    for (int bx = 0; bx < 4; ++bx) tma::reduce_add_box(&p.tm_dq, bx * 32, grp, grow, sStage + bx * 16384);
+                    for (int bx = 0; bx < 4; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, grp, grow, b, sStage + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(stage_free)) : "memory");
@@ -275,18 +275,20 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
         const int rr = e / NC, cc = e - rr * NC;
         lam_rc[i] = (rr < tc::PT) ? (uint32_t)((rr << 8) | cc) : 0xffffffffu;
     }
-    // (tok0: first token of the pair counted over the whole batch, b * T + t0; hh: its head)
-    auto fetch_small = [&](long tok0, int hh) {
+    // (tok0: first token of the pair counted over the whole batch, b * T + t0; hh: its head;
+    //  left: tokens of the sequence from tok0 on; rows behind them take zeros)
+    auto fetch_small = [&](long tok0, int hh, int left) {
         const unsigned short* lp = reinterpret_cast<const unsigned short*>(p.l) + (tok0 * p.H + hh) * L;
 #pragma unroll
         for (int i = 0; i < LAMR; ++i)
-            if (lam_rc[i] != 0xffffffffu) lam_r[i] = lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)];
+            if (lam_rc[i] != 0xffffffffu)
+                lam_r[i] = (int)(lam_rc[i] >> 8) < left ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
     };
     // raw g of a pair: one warp (the one that builds the decay tables), four consecutive tokens per lane
-    auto fetch_g = [&](long tok0, int hh) {
+    auto fetch_g = [&](long tok0, int hh, int left) {
         const float* gp = p.g + (tok0 + 4 * lane) * p.H + hh;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) g_n[i] = gp[(long)i * p.H];
+        for (int i = 0; i < 4; ++i) g_n[i] = 4 * lane < left ? gp[(long)i * p.H] : 0.f;
     };
     // Decay tables of a pair from the g values in g_n, by one full warp: G (pair-wide inclusive cumulative sum),
     // Cf = exp(G[end of 32-block] - G[j]), Vf = exp(G[127] - G[j]).  Built ahead of the pair that reads them, so that
@@ -326,10 +328,11 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
     };
     {
         const long tok0 = (long)b * p.T + (long)r * SEGP * tc::PT;       // first pair of the CTA's first item
-        fetch_small(tok0, h);
+        const int left = p.T - r * SEGP * tc::PT;
+        fetch_small(tok0, h, left);
         store_lam();
         if (warp == TABLE_WARP) {
-            fetch_g(tok0, h);
+            fetch_g(tok0, h, left);
             decay_tables(sGp);
         }
     }
@@ -358,14 +361,16 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
         const int nitem = item + gridDim.x;
         const bool have_next = (pl + 1 < npairs) || (nitem < nitems);
         long ntok = (long)b * p.T + t0 + tc::PT;
-        int nh = h;
+        int nh = h, nleft = p.T - (int)t0 - tc::PT;
         if (pl + 1 >= npairs && nitem < nitems) {
             nh = nitem % p.H;
-            ntok = (long)(nitem / (p.H * p.NS)) * p.T + (long)((nitem / p.H) % p.NS) * SEGP * tc::PT;
+            nleft = ((nitem / p.H) % p.NS) * SEGP * tc::PT;
+            ntok = (long)(nitem / (p.H * p.NS)) * p.T + nleft;
+            nleft = p.T - nleft;
         }
         if (have_next) {
-            fetch_small(ntok, nh);
-            if (warp == TABLE_WARP) fetch_g(ntok, nh);
+            fetch_small(ntok, nh, nleft);
+            if (warp == TABLE_WARP) fetch_g(ntok, nh, nleft);
         }
         STAMP();   // 1 small fetches issued
         int nread = 0;
@@ -612,7 +617,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
 #pragma unroll
             for (int e = tid; e < tc::PT * NLAM; e += 256) {
                 const int rr = e / NLAM, i = e - rr * NLAM;
-                if (i < L) gdl[(long)rr * p.H * L + i] = sDL[rr * tcb::NDL + i] + sDL[(128 + rr) * tcb::NDL + i];
+                if (i < L && t0 + rr < p.T) gdl[(long)rr * p.H * L + i] = sDL[rr * tcb::NDL + i] + sDL[(128 + rr) * tcb::NDL + i];
             }
         }
         float wq_row = 0.f;                          // valid for ch == 1 threads: q_i . dq_i  (column half 0 stages its dk half meanwhile)
@@ -638,12 +643,13 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
             const int cpart = tid / (NLAM - 7), i = 7 + tid % (NLAM - 7);
             const float z = sWk[256 + (cpart * 2) * 16 + i] + sWk[256 + (cpart * 2 + 1) * 16 + i];
             const long cidx = ((long)b * p.H + h) * p.NT + (r * SEGP + pl) * 2 + cpart;
+            const bool in_seq = (r * SEGP + pl) * 2 + cpart < p.NT;
             if (i == 7) {
                 if (cpart == 1) {
-                    p.Zc[cidx * p.LZ + 0] = z;                         // chunk level 0: reader is the second chunk
+                    if (in_seq) p.Zc[cidx * p.LZ + 0] = z;             // chunk level 0: reader is the second chunk
                     p.Yc[(cidx - 1) * (MLOW + 1) + 0] = z;             // ... and its contributor total, same block pair
                 }
-            } else if ((pl >> (i - 8)) & 1) {
+            } else if (in_seq && ((pl >> (i - 8)) & 1)) {
                 p.Zc[cidx * p.LZ + (i - 7)] = z;                       // pair level i-8 = chunk level i-7
             }
         }
@@ -674,7 +680,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
         if (tid == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(dq_ready)) : "memory");
         if (ch == 1) {
             const float w = wq_row - ((sWk[row] + sWk[128 + row]) + (sWk[256 + row] + sWk[384 + row]));
-            red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, w);
+            if (t0 + row < p.T) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, w);
         }
         STAMP();   // 11 reduces issued
         // ---- pair summary and the Fenwick carry over pair levels
@@ -793,7 +799,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
     const int b = blockIdx.x / (p.H * p.NS);
     const int grp = h / (p.H / p.G);
     const int L = p.L;
-    const int npairs = min(SEGP, p.NT / 2 - r * SEGP);
+    const int npairs = min(SEGP, (p.NT + 1) / 2 - r * SEGP);
 
     if (tid == 0) {
 #pragma unroll
@@ -813,7 +819,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
         RegisterSplit<56, 224>::release();
         if (warp == tc::MMA_WARP + 1) {
             if (lane == 0) {
-                const int brow = b * p.T + r * SEGP * tc::PT;
+                const int brow = r * SEGP * tc::PT;
                 for (int it = 0; it < npairs; ++it) {
                     const int row0 = brow + (npairs - 1 - it) * tc::PT;
                     // k is free once the element-wise threads have taken its row sums (its products belong to the early part of
@@ -821,14 +827,14 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
                     // pair's results
                     if (it >= 1 && !umma::mbar_wait(empty_k, (it - 1) & 1, abort_flag)) break;
                     tma::expect_tx(full_qk, 2 * tc::Q_BYTES);
-                    tma::load_panel(sK, &p.tm_k, 0, grp, row0, full_qk);
-                    tma::load_panel(sK + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, full_qk);
+                    tma::load_seq_panel(sK, &p.tm_k, 0, grp, row0, b, full_qk);
+                    tma::load_seq_panel(sK + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, b, full_qk);
                     if (it >= 1 && !umma::mbar_wait(empty_qvd, (it - 1) & 1, abort_flag)) break;
-                    tma::load_panel(sQ, &p.tm_q, 0, grp, row0, full_qk);
-                    tma::load_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, full_qk);
+                    tma::load_seq_panel(sQ, &p.tm_q, 0, grp, row0, b, full_qk);
+                    tma::load_seq_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, full_qk);
                     tma::expect_tx(full_vd, 2 * tc::V_BYTES);
-                    tma::load_panel(sV, &p.tm_v, 0, h, row0, full_vd);
-                    tma::load_panel(sDO, &p.tm_do, 0, h, row0, full_vd);
+                    tma::load_seq_panel(sV, &p.tm_v, 0, h, row0, b, full_vd);
+                    tma::load_seq_panel(sDO, &p.tm_do, 0, h, row0, b, full_vd);
                 }
             }
             return;
@@ -838,10 +844,10 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
             //      element-wise thread stalls on a bulk-group wait
             if (lane == 0) {
                 for (int it = 0; it < npairs; ++it) {
-                    const int grow = b * p.T + (r * SEGP + (npairs - 1 - it)) * tc::PT;
+                    const int grow = (r * SEGP + (npairs - 1 - it)) * tc::PT;
                     if (!umma::mbar_wait(dk_ready, it & 1, abort_flag)) break;
 #pragma unroll
-                    for (int bx = 0; bx < 4; ++bx) tma::reduce_add_box(&p.tm_dk, bx * 32, grp, grow, sStage + bx * 16384);
+                    for (int bx = 0; bx < 4; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(stage_free)) : "memory");
@@ -928,14 +934,15 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
         const unsigned short* lp = reinterpret_cast<const unsigned short*>(p.l) + (((long)b * p.T + t0) * p.H + h) * L;
 #pragma unroll
         for (int i = 0; i < LAMR; ++i)
-            if (lam_rc[i] != 0xffffffffu) lam_r[i] = lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)];
+            if (lam_rc[i] != 0xffffffffu)
+                lam_r[i] = t0 + (lam_rc[i] >> 8) < p.T ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
     };
     // raw g of a pair: one warp (the one that builds the decay tables), four consecutive tokens per lane
     auto fetch_g = [&](int pl) {
         const long t0 = (long)(r * SEGP + pl) * tc::PT;
         const float* gp = p.g + ((long)b * p.T + t0 + 4 * lane) * p.H + h;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) g_n[i] = gp[(long)i * p.H];
+        for (int i = 0; i < 4; ++i) g_n[i] = t0 + 4 * lane < p.T ? gp[(long)i * p.H] : 0.f;
     };
     // Decay tables of a pair from the g values in g_n, by one full warp: G (pair-wide inclusive cumulative sum),
     // Cf = exp(G[end of 32-block] - G[j]), Vf = exp(G[127] - G[j]).  Built ahead of the pair that reads them, so that
@@ -1276,11 +1283,11 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
 #pragma unroll
             for (int i = tid; i < tc::PT * 8; i += 256) {
                 const int rr = i >> 3, c = (i & 7) * 8;
-                *reinterpret_cast<uint4*>(gdv + (long)rr * p.H * tc::VD + c) =
-                    *reinterpret_cast<const uint4*>(sVs + umma::tile_offset(rr, c, tc::PT));
+                if (t0 + rr < p.T)
+                    *reinterpret_cast<uint4*>(gdv + (long)rr * p.H * tc::VD + c) = *reinterpret_cast<const uint4*>(sVs + umma::tile_offset(rr, c, tc::PT));
             }
         }
-        if (ch == 0) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, -(sMisc[row] + sMisc[128 + row]));
+        if (ch == 0 && t0 + row < p.T) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, -(sMisc[row] + sMisc[128 + row]));
         if (tid < 2 * (MP + 1)) {
             // Y of chunk (2*pair + cpart): pair level lv -> chunk level lv + 1 ; index MP -> combined high levels (slot MLOW)
             const int lv = tid >> 1, cpart = tid & 1;
@@ -1288,7 +1295,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
 #pragma unroll
             for (int w = 0; w < 8; ++w) y += sMisc[256 + w * 8 + lv * 2 + cpart];
             const long cidx = ((long)b * p.H + h) * p.NT + (r * SEGP + pl) * 2 + cpart;
-            p.Yc[cidx * (MLOW + 1) + (lv == MP ? MLOW : lv + 1)] = y;
+            if ((r * SEGP + pl) * 2 + cpart < p.NT) p.Yc[cidx * (MLOW + 1) + (lv == MP ? MLOW : lv + 1)] = y;
         }
         STAMPR();   // 10 dv out
         if (it + 1 < npairs) store_lam();
@@ -1306,12 +1313,11 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
 int mamba2_bwd2_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
-    const long BT = (long)p.B * p.T;
-    if ((rc = tma::make_panel_map(&p.tm_q, p.q, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_k, p.k, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_v, p.v, BT, p.H, p.V, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_do, p.d_o, BT, p.H, p.V, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_f32_box_map(&p.tm_dk, p.dk_acc, BT, p.G, p.K, tc::PT)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_dk, p.dk_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
     auto kern = m2_bwd_revorder_tc_kernel<M2_MLOW>;
     const size_t sm = Bwd2TcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
@@ -1323,13 +1329,12 @@ int mamba2_bwd2_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
 int mamba2_bwd1_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
-    const long BT = (long)p.B * p.T;
-    if ((rc = tma::make_panel_map(&p.tm_q, p.q, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_k, p.k, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_v, p.v, BT, p.H, p.V, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_do, p.d_o, BT, p.H, p.V, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_f32_box_map(&p.tm_dq, p.dq_acc, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_f32_box_map(&p.tm_dk, p.dk_acc, BT, p.G, p.K, tc::PT)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_dk, p.dk_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
     auto kern = m2_bwd_fwdorder_tc_kernel<M2_MLOW>;
     const size_t sm = Bwd1TcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);

@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(256, 1) m2_seg_state_kernel(const Mamba2Params
         warp_gemm<MT, NPS, true, true>(acc, sK + st * CH * LDK, LDK, wr * 16 * MT, sVs, LDV, wc * (VD / 2), CH, lane);
         __syncthreads();
     }
-    float* F = p.seg_F + (((long)b * p.H + h) * p.NS + r) * KD * VD;
+    float* F = p.seg_F + (((long)b * p.H + h) * p.NS + r) * M2_KV;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -392,9 +392,9 @@ __global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p, 
     const long bh = blockIdx.y;
     const int e4 = (blockIdx.x * 256 + threadIdx.x) * 4;
     if (e4 >= KV) return;
-    const float* F = p.seg_F + bh * p.NS * KV + e4;
+    const float* F = p.seg_F + bh * p.NS * M2_KV + e4;
     const float* D = p.seg_D + bh * p.NS;
-    bf16* H0 = p.seg_H0 + bh * p.NS * p.LH * KV + e4;
+    bf16* H0 = p.seg_H0 + bh * p.NS * p.LH * M2_KV + e4;
     float st[MAX_LH][4];
 #pragma unroll
     for (int j = 0; j < MAX_LH; ++j) st[j][0] = st[j][1] = st[j][2] = st[j][3] = 0.f;
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p, 
           fb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
           db[u] = 0.f;
           if (r < p.NS - 1) {
-              fb[u] = __ldg(reinterpret_cast<const float4*>(F + (long)r * KV));
+              fb[u] = __ldg(reinterpret_cast<const float4*>(F + (long)r * M2_KV));
               db[u] = __ldg(D + r);
           }
       }
@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p, 
                     uint2 pk;
                     pk.x = pack_bf16(st[j][0], st[j][1]);
                     pk.y = pack_bf16(st[j][2], st[j][3]);
-                    *reinterpret_cast<uint2*>(H0 + ((long)r * p.LH + j) * KV) = pk;
+                    *reinterpret_cast<uint2*>(H0 + ((long)r * p.LH + j) * M2_KV) = pk;
                 }
                 const int period = 2 << j;
                 if ((r % period) == period - 1) {
@@ -481,11 +481,10 @@ __global__ void __launch_bounds__(256, 1) m2_hi_out_kernel(const Mamba2Params p)
     const int wr = warp & 3, wc = warp >> 2;
     const int row0 = wr * 16, col0 = wc * (VD / 2);
     const int lr = lane >> 2, lc2 = (lane & 3) * 2;
-    const long KV = (long)KD * VD;
-    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * KV;
+    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * M2_KV;
 
     auto issue_state = [&](int j, int slot) {
-        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * KV, VD, tid);
+        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * M2_KV, VD, tid);
         cp_async_commit();
     };
     load_tile_async<CH, KD, 256>(sQ, p.q + (((long)b * p.T + t0) * p.G + grp) * KD, (long)p.G * KD, tid);
@@ -550,7 +549,7 @@ __global__ void __launch_bounds__(256, 1) m2_hi_out_kernel(const Mamba2Params p)
     }
     if (p.o_has_high == 2) {
         // column-chunk-major scratch read by the tcgen05 chunk kernel: [bh][pair][8-col chunk][128 rows][8]
-        bf16* gh = p.o_hi + (((long)b * p.H + h) * (p.NT / 2) + (c >> 1)) * (8 * 128 * 8);
+        bf16* gh = p.o_hi + (((long)b * p.H + h) * ((p.NT + 1) / 2) + (c >> 1)) * (8 * 128 * 8);
 #pragma unroll
         for (int nt = 0; nt < 2 * NPS; ++nt)
 #pragma unroll
@@ -576,10 +575,20 @@ __global__ void __launch_bounds__(256, 1) m2_hi_out_kernel(const Mamba2Params p)
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
+std::atomic<int> g_use_tensor_core_path{1};
+
+// The tensor-core kernels take 64 or 128 state rows (K = 64 fills half of their tiles; the tensor maps supply zeros for the other half) and
+// any number of chunks (the second chunk of a last pair may lie beyond the sequence: zeros again, and nothing is written there).  They
+// hold 20 lambda levels.  Forward + backward of T = 57792 (903 chunks), 32 heads, took 10.8 ms on the warp-level kernels, which
+// sequences of an odd number of chunks and K = 64 went to before, and takes 3.8 ms here; T = 16384, 32 heads, K = 64: 1.98 -> 0.98 ms; a single
+// chunk, forward: 61 -> 18 us of which most is the host's.  More levels than 20 do not fit the tables in shared memory.
+bool mamba2_uses_tc(const Mamba2Params& p) { return p.V == 64 && p.L <= 20 && g_use_tensor_core_path.load(); }
+
 template <int KD, int VD, int MLOW>
 static int launch_states(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
-    if (KD == 128 && VD == 64 && g_use_tensor_core_path.load()) {
+    const bool use_tc = mamba2_uses_tc(p) || (KD == 128 && g_use_tensor_core_path.load());
+    if (use_tc) {
         int rc = mamba2_seg_state_tc_launch(p, stream);
         if (rc != 0) return rc;
     } else {
@@ -588,7 +597,7 @@ static int launch_states(Mamba2Params p, cudaStream_t stream) {
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
         llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), 256, sm, stream, p); LLATTN_LAUNCHED();
     }
-    const int KV = KD * VD;
+    const int KV = use_tc ? M2_KV : KD * VD;
     dim3 grid((KV / 4 + 255) / 256, p.B * p.H);
     llattn::launch_chained(m2_seg_scan_kernel, grid, 256, 0, stream, p, KV); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
@@ -597,7 +606,7 @@ static int launch_states(Mamba2Params p, cudaStream_t stream) {
 template <int KD, int VD, int MLOW>
 static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
-    const bool use_tc = (KD == 128 && VD == 64 && (p.NT % 2) == 0 && p.L <= 20 && g_use_tensor_core_path.load());
+    const bool use_tc = mamba2_uses_tc(p);
     if (p.NS > 1) {
         p.o_has_high = use_tc ? 2 : 1;      // 2: partial output goes to the column-chunk-major scratch
         int rc = launch_states<KD, VD, MLOW>(p, stream);
@@ -612,19 +621,13 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
             llattn::launch_chained(kern, p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream, p); LLATTN_LAUNCHED();
         }
     }
-    if (use_tc) {
-        return mamba2_fwd_tc_launch(p, stream);
-    }
-    {
-        auto kern = m2_chunk_fwd_kernel<KD, VD, MLOW>;
-        size_t sm = FwdSmem<KD, VD, MLOW>::total;
-        if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-        llattn::launch_chained(kern, p.B * p.H * p.NS, 256, sm, stream, p); LLATTN_LAUNCHED();
-    }
+    if (use_tc) return mamba2_fwd_tc_launch(p, stream);
+    auto kern = m2_chunk_fwd_kernel<KD, VD, MLOW>;
+    size_t sm = FwdSmem<KD, VD, MLOW>::total;
+    if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
+    llattn::launch_chained(kern, p.B * p.H * p.NS, 256, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
-
-std::atomic<int> g_use_tensor_core_path{1};
 
 int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream) {
     if (p.K == 128 && p.V == 64) return launch_fwd<128, 64, M2_MLOW>(p, stream);

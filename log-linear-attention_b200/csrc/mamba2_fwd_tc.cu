@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
     const int b = blockIdx.x / (p.H * p.NS);
     const int grp = h / (p.H / p.G);
     const int L = p.L;
-    const int npairs = min(SEGP, p.NT / 2 - r * SEGP);
+    const int npairs = min(SEGP, (p.NT + 1) / 2 - r * SEGP);
     const bool hi_init = (p.o_has_high != 0) && (r != 0);
 
     if (tid == 0) {
@@ -84,18 +84,18 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
         if (warp == tc::MMA_WARP + 1) {
             // ---- TMA producer: one lane streams the tiles of the segment through the stages
             if (lane == 0) {
-                const int brow = b * p.T + r * SEGP * tc::PT;
+                const int brow = r * SEGP * tc::PT;
                 for (int pl = 0; pl < npairs; ++pl) {
                     const int st = pl & 1, row0 = brow + pl * tc::PT;
                     if (pl >= 2 && !umma::mbar_wait(&empty_kv[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
                     tma::expect_tx(&full_kv[st], tc::Q_BYTES + tc::V_BYTES);
-                    tma::load_panel(sK + st * tc::Q_BYTES, &p.tm_k, 0, grp, row0, &full_kv[st]);
-                    tma::load_panel(sK + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, &full_kv[st]);
-                    tma::load_panel(sV + st * tc::V_BYTES, &p.tm_v, 0, h, row0, &full_kv[st]);
+                    tma::load_seq_panel(sK + st * tc::Q_BYTES, &p.tm_k, 0, grp, row0, b, &full_kv[st]);
+                    tma::load_seq_panel(sK + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, b, &full_kv[st]);
+                    tma::load_seq_panel(sV + st * tc::V_BYTES, &p.tm_v, 0, h, row0, b, &full_kv[st]);
                     if (pl >= 1 && !umma::mbar_wait(empty_q, (pl - 1) & 1, abort_flag)) break;
                     tma::expect_tx(full_q, tc::Q_BYTES);
-                    tma::load_panel(sQ, &p.tm_q, 0, grp, row0, full_q);
-                    tma::load_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, full_q);
+                    tma::load_seq_panel(sQ, &p.tm_q, 0, grp, row0, b, full_q);
+                    tma::load_seq_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, full_q);
                 }
             }
             return;
@@ -176,14 +176,15 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
         const unsigned short* lp = reinterpret_cast<const unsigned short*>(p.l) + (((long)b * p.T + t0) * p.H + h) * L;
 #pragma unroll
         for (int i = 0; i < LAMR; ++i)
-            if (lam_rc[i] != 0xffffffffu) lam_r[i] = lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)];
+            if (lam_rc[i] != 0xffffffffu)
+                lam_r[i] = t0 + (lam_rc[i] >> 8) < p.T ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
     };
     // raw g of a pair: one warp (the one that builds the decay tables), four consecutive tokens per lane
     auto fetch_g = [&](int pl) {
         const long t0 = (long)(r * SEGP + pl) * tc::PT;
         const float* gp = p.g + ((long)b * p.T + t0 + 4 * lane) * p.H + h;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) g_n[i] = gp[(long)i * p.H];
+        for (int i = 0; i < 4; ++i) g_n[i] = t0 + 4 * lane < p.T ? gp[(long)i * p.H] : 0.f;
     };
     // Decay tables of pair `pl` from the g values in g_n, by one full warp: G (pair-wide inclusive cumulative sum),
     // Cf = exp(G[end of 32-block] - G[j]), Vf = exp(G[127] - G[j]); also the in-chunk cumulative sum to global memory.
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
             tG[4 * lane + i] = G;
             tG[128 + 4 * lane + i] = fexp(gend - G);
             tG[256 + 4 * lane + i] = fexp(glp - G);
-            gc[(long)i * p.H] = cbase + gq[i];
+            if (t0 + 4 * lane < p.T) gc[(long)i * p.H] = cbase + gq[i];
         }
     };
     constexpr int TABLE_WARP = 4;                    // lane quarter 0 (one 32 x 32 block of the S tile): the warp with slack
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
         uint4 ohi[4];
         if (hi_init) {
             // scratch layout [batch*head][pair][8-column chunk][128 rows][8]: a warp reads 512 contiguous bytes
-            const bf16* gh = p.o_hi + ((((long)b * p.H + h) * (p.NT / 2) + (r * SEGP + pl)) * 8 + ch * 4) * (tc::PT * 8) + row * 8;
+            const bf16* gh = p.o_hi + ((((long)b * p.H + h) * ((p.NT + 1) / 2) + (r * SEGP + pl)) * 8 + ch * 4) * (tc::PT * 8) + row * 8;
 #pragma unroll
             for (int c = 0; c < 4; ++c) ohi[c] = *reinterpret_cast<const uint4*>(gh + c * tc::PT * 8);
         }
@@ -425,8 +426,8 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
             for (int i = tid; i < tc::PT * 8; i += 256) {
                 const int rr = i >> 3, c = (i & 7) * 8;
-                *reinterpret_cast<uint4*>(go + (long)rr * p.H * tc::VD + c) =
-                    *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
+                if (t0 + rr < p.T)
+                    *reinterpret_cast<uint4*>(go + (long)rr * p.H * tc::VD + c) = *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
             }
         }
         STAMP();                                     // 10: output stored
@@ -484,9 +485,9 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 int mamba2_fwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
-    if ((rc = tma::make_panel_map(&p.tm_q, p.q, (long)p.B * p.T, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_k, p.k, (long)p.B * p.T, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_v, p.v, (long)p.B * p.T, p.H, p.V, tc::PT)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     auto kern = m2_chunk_fwd_tc_kernel<M2_MLOW>;
     const size_t sm = FwdTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);

@@ -25,9 +25,15 @@ __device__ __forceinline__ uint32_t box_offset_f32(int row, int col) {
 template <int SEG>
 __device__ __forceinline__ void segment_cumsum(const Mamba2Params& p, int b, int h, int r, int nchunks, float* sGs, float* sTot,
                                                int warp, int lane, int tid) {
-    for (int c = warp; c < nchunks; c += 8) {
+    // (a pair whose second chunk is beyond the sequence: a chunk without decay)
+    const int npad = (nchunks + 1) & ~1;
+    for (int c = warp; c < npad; c += 8) {
         const float* gp = p.g + ((long)b * p.T + (long)(r * SEG + c) * CH) * p.H + h;
-        float x0 = gp[(long)(2 * lane) * p.H], x1 = gp[(long)(2 * lane + 1) * p.H];
+        float x0 = 0.f, x1 = 0.f;
+        if (c < nchunks) {
+            x0 = gp[(long)(2 * lane) * p.H];
+            x1 = gp[(long)(2 * lane + 1) * p.H];
+        }
         warp_cumsum64(x0, x1, lane);
         sGs[c * CH + 2 * lane] = x0;
         sGs[c * CH + 2 * lane + 1] = x1;
@@ -36,7 +42,7 @@ __device__ __forceinline__ void segment_cumsum(const Mamba2Params& p, int b, int
     bar_compute();
     if (tid == 0) {
         float run = 0.f;
-        for (int c = 0; c < nchunks; ++c) {
+        for (int c = 0; c < npad; ++c) {
             const float t = sTot[c];
             sTot[c] = run;
             run += t;
@@ -44,7 +50,7 @@ __device__ __forceinline__ void segment_cumsum(const Mamba2Params& p, int b, int
         sTot[SEG] = run;
     }
     bar_compute();
-    for (int i = tid; i < nchunks * CH; i += 256) sGs[i] += sTot[i / CH];
+    for (int i = tid; i < npad * CH; i += 256) sGs[i] += sTot[i / CH];
     bar_compute();
 }
 
@@ -111,7 +117,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
     const int b = blockIdx.x / (p.H * (p.NS - 1));
     const int grp = h / (p.H / p.G);
     const int nchunks = min(SEG, p.NT - r * SEG);
-    const int npairs = nchunks / 2;
+    const int npairs = (nchunks + 1) / 2;
     // set high levels of this segment inside this launch's window of five levels, in increasing order
     int lev[tcs::MAXLH], nl = 0;
 #pragma unroll
@@ -145,16 +151,16 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
                     const int row0 = ((((b * p.H + h) * p.NS + r) * p.LH) + lev[i]) * tc::KD;
                     tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, row0, full_h);
                 }
-                const int brow = b * p.T + r * SEG * CH;
+                const int brow = r * SEG * CH;
                 for (int pl = 0; pl < npairs; ++pl) {
                     const int row0 = brow + pl * tc::PT;
                     if (pl >= 1 && !umma::mbar_wait(empty_do, (pl - 1) & 1, abort_flag)) break;
                     tma::expect_tx(full_do, tc::V_BYTES);
-                    tma::load_panel(sDO, &p.tm_do, 0, h, row0, full_do);
+                    tma::load_seq_panel(sDO, &p.tm_do, 0, h, row0, b, full_do);
                     if (pl >= 1 && !umma::mbar_wait(empty_q, (pl - 1) & 1, abort_flag)) break;
                     tma::expect_tx(full_q, tc::Q_BYTES);
-                    tma::load_panel(sQ, &p.tm_q, 0, grp, row0, full_q);
-                    tma::load_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, full_q);
+                    tma::load_seq_panel(sQ, &p.tm_q, 0, grp, row0, b, full_q);
+                    tma::load_seq_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, full_q);
                 }
             }
             return;
@@ -242,7 +248,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
         const bf16* lrow = p.l + (((long)b * p.T + t0 + row) * p.H + h) * p.L + INTRA_LEVELS + MLOW;
 #pragma unroll
         for (int i = 0; i < tcs::MAXLH; ++i)
-            if (i < nl) lam_next[i] = lrow[lev[i]];
+            if (i < nl) lam_next[i] = t0 + row < p.T ? lrow[lev[i]] : __float2bfloat16(0.f);
     };
     fetch_lambda(0);
 
@@ -319,14 +325,14 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
             float wsum = 0.f;
             for (int i = ch; i < nl; i += 2) {
                 const float dlv = sDL[row * NDLH + i] + sDL[(128 + row) * NDLH + i];
-                gdl[lev[i]] = dlv;
+                if (t0 + row < p.T) gdl[lev[i]] = dlv;
                 float z = lamv[i] * dlv;
                 wsum += z;
 #pragma unroll
                 for (int d = 16; d > 0; d >>= 1) z += __shfl_xor_sync(0xffffffffu, z, d);
                 if (lane == 0) sTot[SEG + 1 + rb * tcs::MAXLH + i] = z;        // per 32-row block
             }
-            if (ch < nl) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, wsum);
+            if (ch < nl && t0 + row < p.T) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, wsum);
         }
         umma::mbar_wait(barB, pl & 1, abort_flag);
         umma::fence_after_sync();
@@ -349,10 +355,10 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
         umma::fence_before_sync();
         bar_compute();
         if (tid == 0) {
-            const int grow = b * p.T + (int)t0;
+            const int grow = (int)t0;
 #pragma unroll
             for (int bx = 0; bx < 4; ++bx) {
-                tma::reduce_add_box(&p.tm_dq, bx * 32, grp, grow, sStage + bx * 16384);
+                if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, grp, grow, b, sStage + bx * 16384);
                 tma::commit_group();                 // one group per box: the next pair waits for them one by one
             }
         }
@@ -360,7 +366,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
             const int i = tid >> 1, cpart = tid & 1;
             const float z = sTot[SEG + 1 + (cpart * 2) * tcs::MAXLH + i] + sTot[SEG + 1 + (cpart * 2 + 1) * tcs::MAXLH + i];
             const long cidx = ((long)b * p.H + h) * p.NT + r * SEG + pl * 2 + cpart;
-            p.Zc[cidx * p.LZ + MLOW + lev[i]] = z;
+            if (pl * 2 + cpart < nchunks) p.Zc[cidx * p.LZ + MLOW + lev[i]] = z;
         }
         umma::fence_before_sync();
         bar_work();                                  // end of the pair
@@ -428,7 +434,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __g
     const int b = blockIdx.x / (p.H * (p.NS - 1));
     const int grp = h / (p.H / p.G);
     const int nchunks = min(SEG, p.NT - r * SEG);
-    const int npairs = nchunks / 2;
+    const int npairs = (nchunks + 1) / 2;
     int lev[MAXL], nl = 0;
 #pragma unroll
     for (int j = 0; j < MAXL; ++j)
@@ -452,13 +458,13 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __g
                     const int row0 = ((((b * p.H + h) * p.NS + r) * p.LH) + lev[i]) * tc::KD;
                     tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, row0, full_h);
                 }
-                const int brow = b * p.T + r * SEG * CH;
+                const int brow = r * SEG * CH;
                 for (int pl = 0; pl < npairs; ++pl) {
                     const int st = pl & 1, row0 = brow + pl * tc::PT;
                     if (pl >= 2 && !umma::mbar_wait(&empty_q[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
                     tma::expect_tx(&full_q[st], tc::Q_BYTES);
-                    tma::load_panel(sQ + st * tc::Q_BYTES, &p.tm_q, 0, grp, row0, &full_q[st]);
-                    tma::load_panel(sQ + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, &full_q[st]);
+                    tma::load_seq_panel(sQ + st * tc::Q_BYTES, &p.tm_q, 0, grp, row0, b, &full_q[st]);
+                    tma::load_seq_panel(sQ + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, &full_q[st]);
                 }
             }
             return;
@@ -512,7 +518,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __g
         const bf16* lrow = p.l + (((long)b * p.T + t0 + row) * p.H + h) * p.L + INTRA_LEVELS + MLOW;
         float lamv[MAXL];
 #pragma unroll
-        for (int i = 0; i < MAXL; ++i) lamv[i] = (i < nl) ? __bfloat162float(lrow[lev[i]]) * sc : 0.f;
+        for (int i = 0; i < MAXL; ++i) lamv[i] = (i < nl && t0 + row < p.T) ? __bfloat162float(lrow[lev[i]]) * sc : 0.f;
         umma::fence_before_sync();
         bar_work();
         umma::mbar_wait(barA, pl & 1, abort_flag);
@@ -527,7 +533,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __g
             for (int e = 0; e < 32; ++e) o[e] += lamv[i] * t[e];
         }
         // column-chunk-major scratch [bh][pair][8-col chunk][128 rows][8]
-        bf16* gh = p.o_hi + ((((long)b * p.H + h) * (p.NT / 2) + (r * (SEG / 2) + pl)) * 8 + ch * 4) * (tc::PT * 8) + row * 8;
+        bf16* gh = p.o_hi + ((((long)b * p.H + h) * ((p.NT + 1) / 2) + (r * (SEG / 2) + pl)) * 8 + ch * 4) * (tc::PT * 8) + row * 8;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
             *reinterpret_cast<uint4*>(gh + c * tc::PT * 8) =
@@ -592,14 +598,14 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_seg_state_tc_kernel(const 
         RegisterSplit<56, 224>::release();
         if (warp == tc::MMA_WARP + 1) {
             if (lane == 0) {
-                const int brow = b * p.T + r * SEG * CH;
+                const int brow = r * SEG * CH;
                 for (int pl = 0; pl < SEGP; ++pl) {
                     const int st = pl & 1, row0 = brow + pl * tc::PT;
                     if (pl >= 2 && !umma::mbar_wait(&empty_kv[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
                     tma::expect_tx(&full_kv[st], tc::Q_BYTES + tc::V_BYTES);
-                    tma::load_panel(sK + st * tc::Q_BYTES, &p.tm_k, 0, grp, row0, &full_kv[st]);
-                    tma::load_panel(sK + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, &full_kv[st]);
-                    tma::load_panel(sV + st * tc::V_BYTES, &p.tm_v, 0, h, row0, &full_kv[st]);
+                    tma::load_seq_panel(sK + st * tc::Q_BYTES, &p.tm_k, 0, grp, row0, b, &full_kv[st]);
+                    tma::load_seq_panel(sK + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, b, &full_kv[st]);
+                    tma::load_seq_panel(sV + st * tc::V_BYTES, &p.tm_v, 0, h, row0, b, &full_kv[st]);
                 }
             }
             return;
@@ -687,9 +693,8 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_seg_state_tc_kernel(const 
 int mamba2_seg_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
-    const long BT = (long)p.B * p.T;
-    if ((rc = tma::make_panel_map(&p.tm_k, p.k, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_v, p.v, BT, p.H, p.V, tc::PT)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     auto kern = m2_seg_state_tc_kernel<M2_MLOW>;
     const size_t sm = SegStateTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
@@ -701,9 +706,8 @@ int mamba2_seg_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
 int mamba2_hi_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
-    const long BT = (long)p.B * p.T;
-    if ((rc = tma::make_panel_map(&p.tm_q, p.q, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * p.K, 1, p.V, tc::KD)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * tc::KD, 1, p.V, tc::KD)) != 0) return rc;
     // up to five segment levels (T <= 16384) with the smaller shared-memory footprint, else up to eight
     if (p.LH <= 5) {
         auto kern = m2_hi_out_tc_kernel<M2_MLOW, 5>;
@@ -724,11 +728,10 @@ int mamba2_hi_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
 int mamba2_hi_bwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
-    const long BT = (long)p.B * p.T;
-    if ((rc = tma::make_panel_map(&p.tm_q, p.q, BT, p.G, p.K, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_do, p.d_o, BT, p.H, p.V, tc::PT)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * p.K, 1, p.V, tc::KD)) != 0) return rc;
-    if ((rc = tma::make_f32_box_map(&p.tm_dq, p.dq_acc, BT, p.G, p.K, tc::PT)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * tc::KD, 1, p.V, tc::KD)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
     auto kern = m2_hi_bwd_tc_kernel<M2_MLOW>;
     const size_t sm = HiBwdTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);

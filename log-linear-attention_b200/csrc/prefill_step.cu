@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(256) mamba2_prompt_state_kernel(const bf16* __
     if (seg_F != nullptr && s1 - s0 >= SEG) {
         // behind the bucket: whole segments up to the one of the last token, then that segment's tokens up to the last one
         const int r0 = s0 / SEG, r1 = s1 / SEG, rl = m / SEG, NS = (Tp + SEG - 1) / SEG;
-        const float *D = seg_D + bh * NS, *F = seg_F + bh * NS * KV;
+        const float *D = seg_D + bh * NS, *F = seg_F + bh * NS * M2_KV;
         float part = 0.f;
         for (int r = r1 + tid; r < rl; r += 256) part += D[r];
         for (int t = rl * SEG + tid; t <= m; t += 256) part += gb[(long)t * H];
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) mamba2_prompt_state_kernel(const bf16* __
             const float w = fexp(after);
 #pragma unroll
             for (int i = 0; i < KV / 1024; ++i) {
-                const float4 f = *reinterpret_cast<const float4*>(F + (long)r * KV + i * 1024 + tid * 4);
+                const float4 f = *reinterpret_cast<const float4*>(F + (long)r * M2_KV + i * 1024 + tid * 4);
                 acc[i].x += w * f.x; acc[i].y += w * f.y; acc[i].z += w * f.z; acc[i].w += w * f.w;
             }
             after += D[r];

@@ -58,6 +58,33 @@ inline int make_f32_box_map(CUtensorMap* out, const void* base, long BT, int NH,
     return r == CUDA_SUCCESS ? 0 : ERR_TENSOR_MAP;
 }
 
+// The same tensors with the batch as a dimension of its own, (B, T, NH, C): a box that reaches beyond the T tokens of a sequence, or beyond
+// C columns, reads zeros there and writes nothing, so that a sequence may end inside a box and a 64-column tensor fills half a tile.
+// elem_bytes 2: bf16, box of 64 columns; 4: fp32, box of 32 columns; 128-byte swizzled either way.
+inline int make_seq_map(CUtensorMap* out, const void* base, long B, long T, int NH, int C, int box_rows, int elem_bytes) {
+    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static EncodeFn fn = nullptr;
+    if (!fn) {
+        void* ptr = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres);
+        if (e != cudaSuccess || qres != cudaDriverEntryPointSuccess || !ptr) return ERR_TENSOR_MAP;
+        fn = reinterpret_cast<EncodeFn>(ptr);
+    }
+    const bool f32 = elem_bytes == 4;
+    const cuuint64_t row = (cuuint64_t)C * elem_bytes;
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)NH, (cuuint64_t)T, (cuuint64_t)B};
+    const cuuint64_t strides[3] = {row, row * NH, row * NH * T};
+    const cuuint32_t box[4] = {f32 ? 32u : 64u, 1, (cuuint32_t)box_rows, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box,
+                    estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                    f32 ? CU_TENSOR_MAP_L2_PROMOTION_NONE : CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : ERR_TENSOR_MAP;
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ void expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(bytes) : "memory");
@@ -70,11 +97,18 @@ __device__ __forceinline__ void load_panel(void* smem_dst, const CUtensorMap* ma
           "r"((uint32_t)__cvta_generic_to_shared(bar))
         : "memory");
 }
-// global[box] += shared[box] (fp32) for one 128 x 32 box; col0 * 4 bytes must be a multiple of 16
-__device__ __forceinline__ void reduce_add_box(const CUtensorMap* map, int col0, int head, int row0, const void* smem_src) {
+// For maps of make_seq_map, rows [tok0, tok0 + box_rows) of sequence `batch`: load_panel, and global[box] += shared[box] (fp32)
+__device__ __forceinline__ void load_seq_panel(void* smem_dst, const CUtensorMap* map, int col0, int head, int tok0, int batch, uint64_t* bar) {
     asm volatile(
-        "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];\n"
-        ::"l"(map), "r"(col0), "r"(head), "r"(row0), "r"((uint32_t)__cvta_generic_to_shared(smem_src))
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n"
+        ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(map), "r"(col0), "r"(head), "r"(tok0), "r"(batch),
+          "r"((uint32_t)__cvta_generic_to_shared(bar))
+        : "memory");
+}
+__device__ __forceinline__ void reduce_add_seq_box(const CUtensorMap* map, int col0, int head, int tok0, int batch, const void* smem_src) {
+    asm volatile(
+        "cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n"
+        ::"l"(map), "r"(col0), "r"(head), "r"(tok0), "r"(batch), "r"((uint32_t)__cvta_generic_to_shared(smem_src))
         : "memory");
 }
 // global[box] = shared[box] for one box of a map; col0 * element size must be a multiple of 16 bytes and no coordinate negative

@@ -119,11 +119,6 @@ def final_states(k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, L: int) -> t
     return st
 
 
-def prompt_length(T: int) -> int:
-    """Length that a prompt's tensors are padded to: an even number of chunks (what the tensor-core kernels take)."""
-    return CHUNK if T <= CHUNK else -(-T // (2 * CHUNK)) * 2 * CHUNK
-
-
 def pad_tokens(tensors, widths, B: int, T: int, Tp: int):
     """Contiguous (B,T,...) tensors copied to (B,Tp,...), zeros behind the T tokens, in one launch; `widths`: values of a
     token in each copy (at least as many as in the tensor; the rest are zero)."""
@@ -162,7 +157,7 @@ def prompt_forward(q, k, v, g, l, level_base: int, htype: HType, chunk_size: int
         q, k, v = (x.to(torch.bfloat16) for x in (q, k, v))
     elif not (q.dtype == k.dtype == v.dtype == torch.bfloat16):
         raise NotImplementedError(f"q / k / v must be bfloat16 (got {q.dtype}, {k.dtype}, {v.dtype})")
-    Tp, Lo = prompt_length(T), max(L, get_num_levels(CHUNK, 2) if T < CHUNK else 0)
+    Tp, Lo = -(-T // CHUNK) * CHUNK, max(L, get_num_levels(CHUNK, 2) if T < CHUNK else 0)
     with torch.cuda.device(q.device):
         q_, k_, v_, l_ = (_as(x, torch.bfloat16) for x in (q, k, v, l))
         g_ = _as(g, torch.float32)

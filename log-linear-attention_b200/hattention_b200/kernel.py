@@ -111,13 +111,19 @@ def hattention_kernel(
     use_qk_l2norm_in_kernel: bool = False,
 ) -> torch.Tensor:
     """o = log-linear attention(q, k, v, g, l[, b]) with gradients; see kernel.py:338-374."""
+    return kernel_call(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chunk_sizes, chunkwise, use_qk_l2norm_in_kernel)
+
+
+def kernel_call(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chunk_sizes=None, chunkwise=True,
+                use_qk_l2norm_in_kernel=False, in_layer=False):
+    """hattention_kernel; `in_layer`: the gradients go on into the sums over tokens of a Mamba-2 layer (llattn_mamba2_bwd_layer)."""
     if chunk_sizes is None:
         chunk_sizes = (64, 64)
     if chunkwise and not head_first and level_base == 2 and htype == HType.WEAK and tuple(chunk_sizes) == (64, 64):
         # bf16 operands of the supported shapes: the native nodes; everything else, errors included, below
         o = None
         if hstruct == HStruct.MAMBA2 and b is None and scale is None and not use_qk_l2norm_in_kernel:
-            o = _lib.host().hattention_mamba2(q, k, v, g, l, KEEP_FORWARD_STATES, _lib.CHECK_STATUS)
+            o = _lib.host().hattention_mamba2(q, k, v, g, l, KEEP_FORWARD_STATES, _lib.CHECK_STATUS, in_layer)
         elif hstruct == HStruct.GDELTA and b is not None and scale is not None and use_qk_l2norm_in_kernel:
             o = gdn_native(q, k, v, b, g, l, scale, 0.0)
         if o is not None:

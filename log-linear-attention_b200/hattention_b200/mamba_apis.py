@@ -7,7 +7,7 @@ import torch
 
 from . import _lib, kernel
 from .base import HStruct, HType
-from .kernel import hattention_kernel, hattention_prefill, hattention_step
+from .kernel import hattention_prefill, hattention_step
 from .recurrent import HState
 
 try:
@@ -168,8 +168,8 @@ def hmamba_chunk_scan_combined(
     x = (x * dt[..., None]).to(x.dtype)      # an fp32 dt must not promote the kernel's v operand (bf16 only)
     g = A[None, None, :] * dt
     lam = compute_lambda(L[None, None], dl, lambda_mode)
-    y = hattention_kernel(q=C, k=B, v=x, b=None, g=g, l=lam, scale=None, head_first=False,
-                          level_base=lambda_level_base, htype=lambda_htype, hstruct=lambda_hstruct)
+    y = kernel.kernel_call(q=C, k=B, v=x, b=None, g=g, l=lam, scale=None, head_first=False,
+                           level_base=lambda_level_base, htype=lambda_htype, hstruct=lambda_hstruct, in_layer=True)
     if D is not None:
         y = y + D_residual
     return y, None
