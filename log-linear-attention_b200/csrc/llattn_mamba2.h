@@ -57,6 +57,9 @@ struct Mamba2Params {
 };
 
 bool mamba2_uses_tc(const Mamba2Params& p);
+// Whether every pair of chunks and all 128 state rows of the tensor-core tiles hold data.  Their kernels come without the tests for it then:
+// with them the kernel of the high levels' gradients takes 1069 instead of 958 us at B = 1, T = 65536, 32 heads, the reverse-order one 911 instead of 878.
+inline bool mamba2_whole_pairs(const Mamba2Params& p) { return p.NT % 2 == 0 && p.K == 128; }
 int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream);
 int mamba2_bwd_dispatch(Mamba2Params p, cudaStream_t stream);
 // segment summaries and the per-level scan over segments only (needs NS > 1)

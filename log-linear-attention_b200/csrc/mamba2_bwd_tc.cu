@@ -45,7 +45,7 @@ __device__ __forceinline__ uint32_t box_offset(int row, int col) {
     return (uint32_t)(row * 128 + (((col >> 2) ^ (row & 7)) << 4) + (col & 3) * 4);
 }
 
-template <int MLOW>
+template <int MLOW, bool WHOLE>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = Bwd1TcSmem<MLOW>;
@@ -168,19 +168,19 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
                     // 64..127 in the k tile once the whole batch is, so that half of the reduce-add is over by then)
                     if (!umma::mbar_wait(dk_ready, gs & 1, abort_flag)) { ok = false; break; }
 #pragma unroll
-                    for (int bx = 0; bx < 2; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage2 + bx * 16384);
+                    for (int bx = 0; bx < 2; ++bx) if (WHOLE || bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage2 + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();             // the q tile's space has been read: the next q may be loaded
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(empty_qk)) : "memory");
                     if (!umma::mbar_wait(dk_ready1, gs & 1, abort_flag)) { ok = false; break; }
 #pragma unroll
-                    for (int bx = 2; bx < 4; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage2 + bx * 16384);
+                    for (int bx = 2; bx < 4; ++bx) if (WHOLE || bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage2 + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(empty_k)) : "memory");
                     if (!umma::mbar_wait(dq_ready, gs & 1, abort_flag)) { ok = false; break; }
 #pragma unroll
-                    for (int bx = 0; bx < 4; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, grp, grow, b, sStage + bx * 16384);
+                    for (int bx = 0; bx < 4; ++bx) if (WHOLE || bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, grp, grow, b, sStage + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(stage_free)) : "memory");
@@ -282,13 +282,13 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
 #pragma unroll
         for (int i = 0; i < LAMR; ++i)
             if (lam_rc[i] != 0xffffffffu)
-                lam_r[i] = (int)(lam_rc[i] >> 8) < left ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
+                lam_r[i] = (WHOLE || (int)(lam_rc[i] >> 8) < left) ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
     };
     // raw g of a pair: one warp (the one that builds the decay tables), four consecutive tokens per lane
     auto fetch_g = [&](long tok0, int hh, int left) {
         const float* gp = p.g + (tok0 + 4 * lane) * p.H + hh;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) g_n[i] = 4 * lane < left ? gp[(long)i * p.H] : 0.f;
+        for (int i = 0; i < 4; ++i) g_n[i] = (WHOLE || 4 * lane < left) ? gp[(long)i * p.H] : 0.f;
     };
     // Decay tables of a pair from the g values in g_n, by one full warp: G (pair-wide inclusive cumulative sum),
     // Cf = exp(G[end of 32-block] - G[j]), Vf = exp(G[127] - G[j]).  Built ahead of the pair that reads them, so that
@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
 #pragma unroll
             for (int e = tid; e < tc::PT * NLAM; e += 256) {
                 const int rr = e / NLAM, i = e - rr * NLAM;
-                if (i < L && t0 + rr < p.T) gdl[(long)rr * p.H * L + i] = sDL[rr * tcb::NDL + i] + sDL[(128 + rr) * tcb::NDL + i];
+                if (i < L && (WHOLE || t0 + rr < p.T)) gdl[(long)rr * p.H * L + i] = sDL[rr * tcb::NDL + i] + sDL[(128 + rr) * tcb::NDL + i];
             }
         }
         float wq_row = 0.f;                          // valid for ch == 1 threads: q_i . dq_i  (column half 0 stages its dk half meanwhile)
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
             const int cpart = tid / (NLAM - 7), i = 7 + tid % (NLAM - 7);
             const float z = sWk[256 + (cpart * 2) * 16 + i] + sWk[256 + (cpart * 2 + 1) * 16 + i];
             const long cidx = ((long)b * p.H + h) * p.NT + (r * SEGP + pl) * 2 + cpart;
-            const bool in_seq = (r * SEGP + pl) * 2 + cpart < p.NT;
+            const bool in_seq = WHOLE || (r * SEGP + pl) * 2 + cpart < p.NT;
             if (i == 7) {
                 if (cpart == 1) {
                     if (in_seq) p.Zc[cidx * p.LZ + 0] = z;             // chunk level 0: reader is the second chunk
@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_fwdorder_tc_kernel(con
         if (tid == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(dq_ready)) : "memory");
         if (ch == 1) {
             const float w = wq_row - ((sWk[row] + sWk[128 + row]) + (sWk[256 + row] + sWk[384 + row]));
-            if (t0 + row < p.T) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, w);
+            if (WHOLE || t0 + row < p.T) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, w);
         }
         STAMP();   // 11 reduces issued
         // ---- pair summary and the Fenwick carry over pair levels
@@ -757,7 +757,7 @@ struct Bwd2TcSmem {
     static constexpr uint32_t total = bar_off + 128 + 1024;
 };
 
-template <int MLOW>
+template <int MLOW, bool WHOLE>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = Bwd2TcSmem<MLOW>;
@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
                     const int grow = (r * SEGP + (npairs - 1 - it)) * tc::PT;
                     if (!umma::mbar_wait(dk_ready, it & 1, abort_flag)) break;
 #pragma unroll
-                    for (int bx = 0; bx < 4; ++bx) if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage + bx * 16384);
+                    for (int bx = 0; bx < 4; ++bx) if (WHOLE || bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, grp, grow, b, sStage + bx * 16384);
                     tma::commit_group();
                     tma::wait_group_read0();
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(stage_free)) : "memory");
@@ -935,14 +935,14 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
 #pragma unroll
         for (int i = 0; i < LAMR; ++i)
             if (lam_rc[i] != 0xffffffffu)
-                lam_r[i] = t0 + (lam_rc[i] >> 8) < p.T ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
+                lam_r[i] = (WHOLE || t0 + (lam_rc[i] >> 8) < p.T) ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
     };
     // raw g of a pair: one warp (the one that builds the decay tables), four consecutive tokens per lane
     auto fetch_g = [&](int pl) {
         const long t0 = (long)(r * SEGP + pl) * tc::PT;
         const float* gp = p.g + ((long)b * p.T + t0 + 4 * lane) * p.H + h;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) g_n[i] = t0 + 4 * lane < p.T ? gp[(long)i * p.H] : 0.f;
+        for (int i = 0; i < 4; ++i) g_n[i] = (WHOLE || t0 + 4 * lane < p.T) ? gp[(long)i * p.H] : 0.f;
     };
     // Decay tables of a pair from the g values in g_n, by one full warp: G (pair-wide inclusive cumulative sum),
     // Cf = exp(G[end of 32-block] - G[j]), Vf = exp(G[127] - G[j]).  Built ahead of the pair that reads them, so that
@@ -1283,11 +1283,11 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
 #pragma unroll
             for (int i = tid; i < tc::PT * 8; i += 256) {
                 const int rr = i >> 3, c = (i & 7) * 8;
-                if (t0 + rr < p.T)
+                if (WHOLE || t0 + rr < p.T)
                     *reinterpret_cast<uint4*>(gdv + (long)rr * p.H * tc::VD + c) = *reinterpret_cast<const uint4*>(sVs + umma::tile_offset(rr, c, tc::PT));
             }
         }
-        if (ch == 0 && t0 + row < p.T) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, -(sMisc[row] + sMisc[128 + row]));
+        if (ch == 0 && (WHOLE || t0 + row < p.T)) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, -(sMisc[row] + sMisc[128 + row]));
         if (tid < 2 * (MP + 1)) {
             // Y of chunk (2*pair + cpart): pair level lv -> chunk level lv + 1 ; index MP -> combined high levels (slot MLOW)
             const int lv = tid >> 1, cpart = tid & 1;
@@ -1295,7 +1295,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
 #pragma unroll
             for (int w = 0; w < 8; ++w) y += sMisc[256 + w * 8 + lv * 2 + cpart];
             const long cidx = ((long)b * p.H + h) * p.NT + (r * SEGP + pl) * 2 + cpart;
-            if ((r * SEGP + pl) * 2 + cpart < p.NT) p.Yc[cidx * (MLOW + 1) + (lv == MP ? MLOW : lv + 1)] = y;
+            if (WHOLE || (r * SEGP + pl) * 2 + cpart < p.NT) p.Yc[cidx * (MLOW + 1) + (lv == MP ? MLOW : lv + 1)] = y;
         }
         STAMPR();   // 10 dv out
         if (it + 1 < npairs) store_lam();
@@ -1318,7 +1318,7 @@ int mamba2_bwd2_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_dk, p.dk_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
-    auto kern = m2_bwd_revorder_tc_kernel<M2_MLOW>;
+    auto kern = mamba2_whole_pairs(p) ? m2_bwd_revorder_tc_kernel<M2_MLOW, true> : m2_bwd_revorder_tc_kernel<M2_MLOW, false>;
     const size_t sm = Bwd2TcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
@@ -1335,7 +1335,7 @@ int mamba2_bwd1_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_dk, p.dk_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
-    auto kern = m2_bwd_fwdorder_tc_kernel<M2_MLOW>;
+    auto kern = mamba2_whole_pairs(p) ? m2_bwd_fwdorder_tc_kernel<M2_MLOW, true> : m2_bwd_fwdorder_tc_kernel<M2_MLOW, false>;
     const size_t sm = Bwd1TcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;

@@ -30,7 +30,7 @@ struct FwdTcSmem {
     static constexpr uint32_t total = bar_off + 128 + 1024;             // + slack for 1024-byte alignment
 };
 
-template <int MLOW>
+template <int MLOW, bool WHOLE>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = FwdTcSmem<MLOW>;
@@ -177,14 +177,14 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
         for (int i = 0; i < LAMR; ++i)
             if (lam_rc[i] != 0xffffffffu)
-                lam_r[i] = t0 + (lam_rc[i] >> 8) < p.T ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
+                lam_r[i] = (WHOLE || t0 + (lam_rc[i] >> 8) < p.T) ? lp[(long)(lam_rc[i] >> 8) * p.H * L + (lam_rc[i] & 255)] : (unsigned short)0;
     };
     // raw g of a pair: one warp (the one that builds the decay tables), four consecutive tokens per lane
     auto fetch_g = [&](int pl) {
         const long t0 = (long)(r * SEGP + pl) * tc::PT;
         const float* gp = p.g + ((long)b * p.T + t0 + 4 * lane) * p.H + h;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) g_n[i] = t0 + 4 * lane < p.T ? gp[(long)i * p.H] : 0.f;
+        for (int i = 0; i < 4; ++i) g_n[i] = (WHOLE || t0 + 4 * lane < p.T) ? gp[(long)i * p.H] : 0.f;
     };
     // Decay tables of pair `pl` from the g values in g_n, by one full warp: G (pair-wide inclusive cumulative sum),
     // Cf = exp(G[end of 32-block] - G[j]), Vf = exp(G[127] - G[j]); also the in-chunk cumulative sum to global memory.
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
             tG[4 * lane + i] = G;
             tG[128 + 4 * lane + i] = fexp(gend - G);
             tG[256 + 4 * lane + i] = fexp(glp - G);
-            if (t0 + 4 * lane < p.T) gc[(long)i * p.H] = cbase + gq[i];
+            if (WHOLE || t0 + 4 * lane < p.T) gc[(long)i * p.H] = cbase + gq[i];
         }
     };
     constexpr int TABLE_WARP = 4;                    // lane quarter 0 (one 32 x 32 block of the S tile): the warp with slack
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
             for (int i = tid; i < tc::PT * 8; i += 256) {
                 const int rr = i >> 3, c = (i & 7) * 8;
-                if (t0 + rr < p.T)
+                if (WHOLE || t0 + rr < p.T)
                     *reinterpret_cast<uint4*>(go + (long)rr * p.H * tc::VD + c) = *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
             }
         }
@@ -488,7 +488,7 @@ int mamba2_fwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
-    auto kern = m2_chunk_fwd_tc_kernel<M2_MLOW>;
+    auto kern = mamba2_whole_pairs(p) ? m2_chunk_fwd_tc_kernel<M2_MLOW, true> : m2_chunk_fwd_tc_kernel<M2_MLOW, false>;
     const size_t sm = FwdTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;

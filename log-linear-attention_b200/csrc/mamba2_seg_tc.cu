@@ -73,7 +73,7 @@ struct HiBwdTcSmem {
     static constexpr uint32_t total = sink_off + 256 * 4 + 1024;
 };
 
-template <int MLOW>
+template <int MLOW, bool WHOLE>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = HiBwdTcSmem<MLOW>;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
         const bf16* lrow = p.l + (((long)b * p.T + t0 + row) * p.H + h) * p.L + INTRA_LEVELS + MLOW;
 #pragma unroll
         for (int i = 0; i < tcs::MAXLH; ++i)
-            if (i < nl) lam_next[i] = t0 + row < p.T ? lrow[lev[i]] : __float2bfloat16(0.f);
+            if (i < nl) lam_next[i] = (WHOLE || t0 + row < p.T) ? lrow[lev[i]] : __float2bfloat16(0.f);
     };
     fetch_lambda(0);
 
@@ -325,14 +325,14 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
             float wsum = 0.f;
             for (int i = ch; i < nl; i += 2) {
                 const float dlv = sDL[row * NDLH + i] + sDL[(128 + row) * NDLH + i];
-                if (t0 + row < p.T) gdl[lev[i]] = dlv;
+                if (WHOLE || t0 + row < p.T) gdl[lev[i]] = dlv;
                 float z = lamv[i] * dlv;
                 wsum += z;
 #pragma unroll
                 for (int d = 16; d > 0; d >>= 1) z += __shfl_xor_sync(0xffffffffu, z, d);
                 if (lane == 0) sTot[SEG + 1 + rb * tcs::MAXLH + i] = z;        // per 32-row block
             }
-            if (ch < nl && t0 + row < p.T) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, wsum);
+            if (ch < nl && (WHOLE || t0 + row < p.T)) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, wsum);
         }
         umma::mbar_wait(barB, pl & 1, abort_flag);
         umma::fence_after_sync();
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
             const int grow = (int)t0;
 #pragma unroll
             for (int bx = 0; bx < 4; ++bx) {
-                if (bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, grp, grow, b, sStage + bx * 16384);
+                if (WHOLE || bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, grp, grow, b, sStage + bx * 16384);
                 tma::commit_group();                 // one group per box: the next pair waits for them one by one
             }
         }
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
             const int i = tid >> 1, cpart = tid & 1;
             const float z = sTot[SEG + 1 + (cpart * 2) * tcs::MAXLH + i] + sTot[SEG + 1 + (cpart * 2 + 1) * tcs::MAXLH + i];
             const long cidx = ((long)b * p.H + h) * p.NT + r * SEG + pl * 2 + cpart;
-            if (pl * 2 + cpart < nchunks) p.Zc[cidx * p.LZ + MLOW + lev[i]] = z;
+            if (WHOLE || pl * 2 + cpart < nchunks) p.Zc[cidx * p.LZ + MLOW + lev[i]] = z;
         }
         umma::fence_before_sync();
         bar_work();                                  // end of the pair
@@ -408,7 +408,7 @@ struct HiOutTcSmem {
     static constexpr uint32_t total = bar_off + 128 + 1024;
 };
 
-template <int MLOW, int MAXL>
+template <int MLOW, int MAXL, bool WHOLE>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = HiOutTcSmem<MLOW, MAXL>;
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __g
         const bf16* lrow = p.l + (((long)b * p.T + t0 + row) * p.H + h) * p.L + INTRA_LEVELS + MLOW;
         float lamv[MAXL];
 #pragma unroll
-        for (int i = 0; i < MAXL; ++i) lamv[i] = (i < nl && t0 + row < p.T) ? __bfloat162float(lrow[lev[i]]) * sc : 0.f;
+        for (int i = 0; i < MAXL; ++i) lamv[i] = (i < nl && (WHOLE || t0 + row < p.T)) ? __bfloat162float(lrow[lev[i]]) * sc : 0.f;
         umma::fence_before_sync();
         bar_work();
         umma::mbar_wait(barA, pl & 1, abort_flag);
@@ -710,13 +710,13 @@ int mamba2_hi_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * tc::KD, 1, p.V, tc::KD)) != 0) return rc;
     // up to five segment levels (T <= 16384) with the smaller shared-memory footprint, else up to eight
     if (p.LH <= 5) {
-        auto kern = m2_hi_out_tc_kernel<M2_MLOW, 5>;
+        auto kern = mamba2_whole_pairs(p) ? m2_hi_out_tc_kernel<M2_MLOW, 5, true> : m2_hi_out_tc_kernel<M2_MLOW, 5, false>;
         const size_t sm = HiOutTcSmem<M2_MLOW, 5>::total;
         cudaError_t e = allow_smem(kern, sm);
         if (e != cudaSuccess) return (int)e;
         llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     } else {
-        auto kern = m2_hi_out_tc_kernel<M2_MLOW, 8>;
+        auto kern = mamba2_whole_pairs(p) ? m2_hi_out_tc_kernel<M2_MLOW, 8, true> : m2_hi_out_tc_kernel<M2_MLOW, 8, false>;
         const size_t sm = HiOutTcSmem<M2_MLOW, 8>::total;
         cudaError_t e = allow_smem(kern, sm);
         if (e != cudaSuccess) return (int)e;
@@ -732,7 +732,7 @@ int mamba2_hi_bwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * tc::KD, 1, p.V, tc::KD)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
-    auto kern = m2_hi_bwd_tc_kernel<M2_MLOW>;
+    auto kern = mamba2_whole_pairs(p) ? m2_hi_bwd_tc_kernel<M2_MLOW, true> : m2_hi_bwd_tc_kernel<M2_MLOW, false>;
     const size_t sm = HiBwdTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
