@@ -13,65 +13,52 @@
 // Aw and Au come from the forward; d(M^-1) = -M^-T dM^-1 M^-T turns their gradients into dA.
 #include "llattn_common.cuh"
 #include "llattn_gdn.h"
-#include "tc_common.cuh"
 
 namespace llattn {
 
+// Shared memory: three 64-row tiles of K or V columns and five 64 x 64 tiles, each used for several operands in turn, so that two
+// CTAs fit on an SM (109,600 bytes with V = 128).  k stays in the first; the others hold
+//     S1: q -> v -> w -> dw          S2: d_o -> d_u -> -(d_qd exp(G)) -> q
+//     Aw    QK -> dKK    Au -> dQK    Ta: P -> dAu -> dAu Au^T -> Aw * beta_j -> dAw    Tb: dX -> dAw Aw^T
+// What bounds it: a chunk is a chain of barrier-separated small products whose latency one CTA of 8 warps does not fill: with fifteen tiles
+// of its own and one CTA per SM it took 1121 us at B = 4, T = 8192, 16 heads, V = 128, and takes 1000 us with two.  The load / store
+// pipe is at 68 % then (ldmatrix of the operands 40 %), DRAM at 32 %.  (16 warps per chunk: 1180, the smaller warp tiles read more operands.)
 template <int KD, int VD>
 struct ChunkBwdSmem {
     static constexpr int LDK = KD + PAD, LDV = VD + PAD, LDP = CH + PAD;
-    static constexpr size_t q_off = 0;                                   // bf16 [64][LDK]
-    static constexpr size_t k_off = q_off + 1ull * CH * LDK * 2;
-    static constexpr size_t w_off = k_off + 1ull * CH * LDK * 2;          // w
-    static constexpr size_t dqd_off = w_off + 1ull * CH * LDK * 2;        // -(d_qd exp(G))
-    static constexpr size_t dw_off = dqd_off + 1ull * CH * LDK * 2;       // dw
-    static constexpr size_t v_off = dw_off + 1ull * CH * LDK * 2;         // bf16 [64][LDV]
-    static constexpr size_t do_off = v_off + 1ull * CH * LDV * 2;
-    static constexpr size_t du_off = do_off + 1ull * CH * LDV * 2;
-    static constexpr size_t qk_off = du_off + 1ull * CH * LDV * 2;        // bf16 [64][LDP] tril(q k^T), later dKK
-    static constexpr size_t aw_off = qk_off + 1ull * CH * LDP * 2;
-    static constexpr size_t au_off = aw_off + 1ull * CH * LDP * 2;
-    static constexpr size_t kk_off = au_off + 1ull * CH * LDP * 2;        // k k^T
-    static constexpr size_t ta_off = kk_off + 1ull * CH * LDP * 2;        // Aw*beta_j, P, dAw, dAu
-    static constexpr size_t tb_off = ta_off + 1ull * CH * LDP * 2;        // dX, dAw Aw^T, dAu Au^T
-    static constexpr size_t dqk_off = tb_off + 1ull * CH * LDP * 2;       // dQK
-    static constexpr size_t f_off = dqk_off + 1ull * CH * LDP * 2;        // floats
-    // floats: G[64] beta[64] eG[64] eGk[64] dG[64] dB[64] lam[64][8] dL[64][8] misc[8] part[22][64]
-    static constexpr size_t total = f_off + (6 * CH + 2 * CH * 8 + 8 + 22 * CH) * 4;
+    static constexpr size_t BIG = 1ull * CH * LDK * 2, SMALL = 1ull * CH * LDP * 2;
+    static_assert(VD <= KD, "a tile of V columns fits the place of one of K columns");
+    static constexpr size_t k_off = 0, s1_off = BIG, s2_off = 2 * BIG;
+    static constexpr size_t aw_off = 3 * BIG, qk_off = aw_off + SMALL, au_off = qk_off + SMALL, ta_off = au_off + SMALL, tb_off = ta_off + SMALL;
+    static constexpr size_t f_off = tb_off + SMALL;
+    // floats: G[64] beta[64] eG[64] eGk[64] dG[64] lam[64][8] dL[64][8] misc[8] part[22][64]
+    static constexpr size_t total = f_off + (5 * CH + 2 * CH * 8 + 8 + 22 * CH) * 4;
 };
 
 // FUSED: the level-gradient kernel has already written -(d_qd exp(G)) in bf16, the per-token sums d_qd.qd + d_wd.wd - d_kd.kd and
 // the chunk total of d_kd.kd (inside d_gl); otherwise a row pass over the K-wide gradients derives them here.
 template <int KD, int VD, bool FUSED>
-__global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p) {
+__global__ void __launch_bounds__(256, 2) gdn_bwd_chunk_kernel(const GdnParams p) {
     chain_wait();
     using SM = ChunkBwdSmem<KD, VD>;
     constexpr int LDK = SM::LDK, LDV = SM::LDV, LDP = SM::LDP;
     constexpr int NPK = KD / 32, NPV = VD / 32;       // 16-column pairs per warp for 64 x K and 64 x V results
     static_assert(KD == 128, "row passes assume one float4 per lane per row");
     extern __shared__ __align__(16) unsigned char smem[];
-    bf16* sQ = reinterpret_cast<bf16*>(smem + SM::q_off);
     bf16* sK = reinterpret_cast<bf16*>(smem + SM::k_off);
-    bf16* sW = reinterpret_cast<bf16*>(smem + SM::w_off);
-    bf16* sDqd = reinterpret_cast<bf16*>(smem + SM::dqd_off);
-    bf16* sDW = reinterpret_cast<bf16*>(smem + SM::dw_off);
-    bf16* sV = reinterpret_cast<bf16*>(smem + SM::v_off);
-    bf16* sDo = reinterpret_cast<bf16*>(smem + SM::do_off);
-    bf16* sDU = reinterpret_cast<bf16*>(smem + SM::du_off);
-    bf16* sQK = reinterpret_cast<bf16*>(smem + SM::qk_off);
+    bf16* s1 = reinterpret_cast<bf16*>(smem + SM::s1_off);
+    bf16* s2 = reinterpret_cast<bf16*>(smem + SM::s2_off);
     bf16* sAw = reinterpret_cast<bf16*>(smem + SM::aw_off);
+    bf16* sQK = reinterpret_cast<bf16*>(smem + SM::qk_off);
     bf16* sAu = reinterpret_cast<bf16*>(smem + SM::au_off);
-    bf16* sKK = reinterpret_cast<bf16*>(smem + SM::kk_off);
     bf16* sTa = reinterpret_cast<bf16*>(smem + SM::ta_off);
     bf16* sTb = reinterpret_cast<bf16*>(smem + SM::tb_off);
-    bf16* sDQK = reinterpret_cast<bf16*>(smem + SM::dqk_off);
     float* sG = reinterpret_cast<float*>(smem + SM::f_off);
     float* sBe = sG + CH;
     float* sEG = sBe + CH;
     float* sEGk = sEG + CH;
     float* sDG = sEGk + CH;
-    float* sDB = sDG + CH;
-    float* sLam = sDB + CH;           // [64][8]   (the dB slot itself is unused: beta gradients are summed from the partial slots)
+    float* sLam = sDG + CH;           // [64][8]
     float* sDL = sLam + CH * 8;       // [64][8]
     float* sMisc = sDL + CH * 8;      // [0] = sum d_kd . kd
     // partial sums of the decay (G) and beta gradients, one slot per producing warp group so that no stage needs shared-memory
@@ -88,17 +75,13 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rbw = warp & 3;               // row block of the warp
-#ifdef LLATTN_STAMPS
-    int nstamp = 0;
-    const int stamp_slot = (blockIdx.x == 3000 && (tid & 31) == 0 && (warp == 0 || warp == 7 || warp == 2)) ? (warp == 0 ? 0 : (warp == 7 ? 1 : 2)) : -1;
-#endif
-    STAMP();
     const int h = blockIdx.x % p.H;
     const int c = (blockIdx.x / p.H) % p.NT;
     const int b = blockIdx.x / (p.H * p.NT);
     const long rowbase = ((long)b * p.T + (long)c * CH) * p.H + h;
     const int r0 = (warp & 3) * 16, cw = warp >> 2;
     const int lr = lane >> 2, lc2 = (lane & 3) * 2;
+    const int c0k = cw * (KD / 2), c0v = cw * (VD / 2);
 
     // the small loads go first: their latency passes while the tile copies are being issued
     float gv = 0.f;
@@ -114,23 +97,29 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
     }
     float grow = 0.f;
     if (FUSED && tid < CH) grow = __ldg(p.d_grow + rowbase + (long)tid * p.H);
-    // two groups: the first products (k k^T, q k^T, Aw * beta_j) wait for q, k, Aw only
-    load_tile_async<CH, KD, 256>(sQ, p.q + rowbase * KD, (long)p.H * KD, tid);
+    // two groups: the first products (k k^T, q k^T) wait for q, k, Aw only
+    load_tile_async<CH, KD, 256>(s1, p.q + rowbase * KD, (long)p.H * KD, tid);
     load_tile_async<CH, KD, 256>(sK, p.k + rowbase * KD, (long)p.H * KD, tid);
     load_tile_async<CH, CH, 256>(sAw, p.Aw + rowbase * CH, (long)p.H * CH, tid);
     cp_async_commit();
-    load_tile_async<CH, VD, 256>(sV, p.v + rowbase * VD, (long)p.H * VD, tid);
-    load_tile_async<CH, VD, 256>(sDo, p.d_o + rowbase * VD, (long)p.H * VD, tid);
-    load_tile_async<CH, VD, 256>(sDU, p.d_u + rowbase * VD, (long)p.H * VD, tid);
+    load_tile_async<CH, VD, 256>(s2, p.d_o + rowbase * VD, (long)p.H * VD, tid);
     load_tile_async<CH, CH, 256>(sAu, p.Au + rowbase * CH, (long)p.H * CH, tid);
-    if (FUSED) load_tile_async<CH, KD, 256>(sDqd, p.dqd_neg + rowbase * KD, (long)p.H * KD, tid);
     cp_async_commit();
-    if (FUSED) {
-        // the fp32 level gradients are read as accumulator fragments in later stages: bring their 3 x 64 rows x 512 bytes into L2 now
-        const long off = (rowbase + (long)(tid >> 2) * p.H) * KD + (tid & 3) * 32;
-        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.d_wd + off));
-        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.d_kd + off));
-        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.d_qd + off));
+    // what later stages read goes into L2 now: v, d_u and the bf16 d_qd term (tiles that take the place of earlier ones), and the fp32 level
+    // gradients (read as accumulator fragments, 3 x 64 rows x 512 bytes)
+    {
+        const long row = rowbase + (long)(tid >> 2) * p.H;
+        if ((tid & 3) < VD / 64) {
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.v + row * VD + (tid & 3) * 64));
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.d_u + row * VD + (tid & 3) * 64));
+        }
+        if (FUSED) {
+            if ((tid & 3) < 2) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.dqd_neg + row * KD + (tid & 3) * 64));
+            const long off = row * KD + (tid & 3) * 32;
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.d_wd + off));
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.d_kd + off));
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.d_qd + off));
+        }
     }
     if (tid < CH) {
         sG[tid] = gv;
@@ -144,110 +133,47 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
     }
     if (tid == 0) sMisc[0] = 0.f;
     __syncthreads();
-    STAMP();
     if (tid < CH) {
         sEG[tid] = fexp(sG[tid]);
         sEGk[tid] = fexp(sG[CH - 1] - sG[tid]);
     }
-    __syncthreads();
-    STAMP();
-
-    // ---- row pass over the K-wide gradients: -(d_qd exp(G)) as a bf16 operand; the decay terms
-    //      dG_i += d_qd.qd + d_wd.wd - d_kd.kd and the chunk total of d_kd.kd
-    if (!FUSED) {
-        float kdsum = 0.f;
-        // four rows per batch: every load of a batch is issued before the first use, so a batch pays the load latency once
-#pragma unroll
-        for (int bt = 0; bt < CH / 32; ++bt) {
-            float4 a[4], bw[4], ck[4];
-            uint2 xq[4], xw[4], xk[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = (bt * 4 + u) * 8 + warp;
-                const long off = (rowbase + (long)i * p.H) * KD + lane * 4;
-                a[u] = __ldg(reinterpret_cast<const float4*>(p.d_qd + off));
-                bw[u] = __ldg(reinterpret_cast<const float4*>(p.d_wd + off));
-                ck[u] = __ldg(reinterpret_cast<const float4*>(p.d_kd + off));
-                xq[u] = __ldg(reinterpret_cast<const uint2*>(p.qd + off));
-                xw[u] = __ldg(reinterpret_cast<const uint2*>(p.wd + off));
-                xk[u] = __ldg(reinterpret_cast<const uint2*>(p.kd + off));
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = (bt * 4 + u) * 8 + warp;
-                const __nv_bfloat162 q0 = *reinterpret_cast<const __nv_bfloat162*>(&xq[u].x), q1 = *reinterpret_cast<const __nv_bfloat162*>(&xq[u].y);
-                const __nv_bfloat162 w0 = *reinterpret_cast<const __nv_bfloat162*>(&xw[u].x), w1 = *reinterpret_cast<const __nv_bfloat162*>(&xw[u].y);
-                const __nv_bfloat162 k0 = *reinterpret_cast<const __nv_bfloat162*>(&xk[u].x), k1 = *reinterpret_cast<const __nv_bfloat162*>(&xk[u].y);
-                float dq_ = a[u].x * __bfloat162float(q0.x) + a[u].y * __bfloat162float(q0.y) + a[u].z * __bfloat162float(q1.x) + a[u].w * __bfloat162float(q1.y);
-                float dw_ = bw[u].x * __bfloat162float(w0.x) + bw[u].y * __bfloat162float(w0.y) + bw[u].z * __bfloat162float(w1.x) + bw[u].w * __bfloat162float(w1.y);
-                float dk_ = ck[u].x * __bfloat162float(k0.x) + ck[u].y * __bfloat162float(k0.y) + ck[u].z * __bfloat162float(k1.x) + ck[u].w * __bfloat162float(k1.y);
-                float r = dq_ + dw_ - dk_;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) {
-                    r += __shfl_xor_sync(0xffffffffu, r, d);
-                    dk_ += __shfl_xor_sync(0xffffffffu, dk_, d);
-                }
-                if (lane == 0) sDG[i] += r;          // one warp per row: no other writer at this point
-                kdsum += dk_;
-                const float eg = -sEG[i];
-                uint2 o;
-                o.x = pack_bf16(a[u].x * eg, a[u].y * eg);
-                o.y = pack_bf16(a[u].z * eg, a[u].w * eg);
-                *reinterpret_cast<uint2*>(sDqd + i * LDK + lane * 4) = o;
-            }
-        }
-        if (lane == 0) atomicAdd(&sMisc[0], kdsum);
-    }
     cp_async_wait<1>();
     __syncthreads();
-    STAMP();
 
-    // ---- KK = k k^T, QK = tril(q k^T), Aw * beta_j
+    // ---- KK = k k^T (kept in registers: its reader has the same fragment), QK = tril(q k^T)
+    uint32_t kk[4][2];
     {
-        float accK[1][4][4], accQ[1][4][4];
-        zero_acc(accK);
-        zero_acc(accQ);
-        warp_gemm<1, 2, false, false>(accK, sK, LDK, r0, sK, LDK, cw * 32, KD, lane);
-        warp_gemm<1, 2, false, false>(accQ, sQ, LDK, r0, sK, LDK, cw * 32, KD, lane);
+        float acc[1][4][4];
+        zero_acc(acc);
+        warp_gemm<1, 2, false, false>(acc, sK, LDK, r0, sK, LDK, cw * 32, KD, lane);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) kk[nt][hh] = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
+        zero_acc(acc);
+        warp_gemm<1, 2, false, false>(acc, s1, LDK, r0, sK, LDK, cw * 32, KD, lane);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 const int i = r0 + lr + hh * 8, j = cw * 32 + nt * 8 + lc2;
-                *reinterpret_cast<uint32_t*>(sKK + i * LDP + j) = pack_bf16(accK[0][nt][hh * 2], accK[0][nt][hh * 2 + 1]);
                 *reinterpret_cast<uint32_t*>(sQK + i * LDP + j) =
-                    pack_bf16(j <= i ? accQ[0][nt][hh * 2] : 0.f, j + 1 <= i ? accQ[0][nt][hh * 2 + 1] : 0.f);
+                    pack_bf16(j <= i ? acc[0][nt][hh * 2] : 0.f, j + 1 <= i ? acc[0][nt][hh * 2 + 1] : 0.f);
             }
-        for (int e = tid; e < CH * CH / 2; e += 256) {
-            const int i = e / (CH / 2), j = (e % (CH / 2)) * 2;
-            const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(sAw + i * LDP + j);
-            *reinterpret_cast<uint32_t*>(sTa + i * LDP + j) = pack_bf16(__bfloat162float(x.x) * sBe[j], __bfloat162float(x.y) * sBe[j + 1]);
-        }
     }
-    cp_async_wait<0>();                        // v, do, d_u, Au (and the bf16 d_qd term) have landed
-    __syncthreads();
-    STAMP();
+    __syncthreads();                           // QK complete, q consumed
+    load_tile_async<CH, VD, 256>(s1, p.v + rowbase * VD, (long)p.H * VD, tid);
+    cp_async_commit();
 
-    // ---- w = (Aw * beta_j) k ;  X = QK Aw ;  dP = do v^T
-    float accX[1][4][4], accP[1][4][4];
+    // ---- X = QK Aw ;  dP = do v^T ;  P and dX
     {
-        float acc[1][2 * NPK][4];
-        zero_acc(acc);
-        warp_gemm<1, NPK, false, true>(acc, sTa, LDP, r0, sK, LDK, cw * (KD / 2), CH, lane);
-#pragma unroll
-        for (int nt = 0; nt < 2 * NPK; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-                *reinterpret_cast<uint32_t*>(sW + (r0 + lr + hh * 8) * LDK + cw * (KD / 2) + nt * 8 + lc2) =
-                    pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
+        float accX[1][4][4], accP[1][4][4];
         zero_acc(accX);
         zero_acc(accP);
         warp_gemm<1, 2, false, true>(accX, sQK, LDP, r0, sAw, LDP, cw * 32, CH, lane);
-        warp_gemm<1, 2, false, false>(accP, sDo, LDV, r0, sV, LDV, cw * 32, VD, lane);
-    }
-    __syncthreads();                           // Aw * beta_j has been consumed: its tile becomes P
-    STAMP();
-    {
+        cp_async_wait<0>();                    // v, do, Au have landed
+        __syncthreads();
+        warp_gemm<1, 2, false, false>(accP, s2, LDV, r0, s1, LDV, cw * 32, VD, lane);
         float rs[2] = {0.f, 0.f};
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
@@ -328,27 +254,31 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
             if ((lane & 3) == 0) pRowG_P[cw * CH + r0 + lr + hh * 8] = rs[hh];
         }
     }
-    __syncthreads();
-    STAMP();
+    __syncthreads();                           // P and dX complete
 
-    // ---- dv = P^T do + beta * (Au^T d_u) ;  dbeta_i += (Au^T d_u)_i . v_i
+    float dqk[1][4][4];
     {
+        // ---- dv = P^T do + beta * (Au^T d_u) ;  dbeta_i += (Au^T d_u)_i . v_i ;  while d_u arrives: the first term of dQK, dX Aw^T
         float acc[1][2 * NPV][4], acc2[1][2 * NPV][4];
         zero_acc(acc);
+        warp_gemm<1, NPV, true, true>(acc, sTa, LDP, r0, s2, LDV, c0v, CH, lane);
+        __syncthreads();                       // do and P consumed
+        load_tile_async<CH, VD, 256>(s2, p.d_u + rowbase * VD, (long)p.H * VD, tid);
+        cp_async_commit();
+        zero_acc(dqk);
+        warp_gemm<1, 2, false, false>(dqk, sTb, LDP, r0, sAw, LDP, cw * 32, CH, lane);
+        cp_async_wait<0>();
+        __syncthreads();
         zero_acc(acc2);
-        const int c0 = cw * (VD / 2);
-        warp_gemm<1, NPV, true, true>(acc, sTa, LDP, r0, sDo, LDV, c0, CH, lane);
-        STAMP();
-        warp_gemm<1, NPV, true, true>(acc2, sAu, LDP, r0, sDU, LDV, c0, CH, lane);
-        STAMP();
+        warp_gemm<1, NPV, true, true>(acc2, sAu, LDP, r0, s2, LDV, c0v, CH, lane);
         float rb[2] = {0.f, 0.f};
 #pragma unroll
         for (int nt = 0; nt < 2 * NPV; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + lr + hh * 8, j = c0 + nt * 8 + lc2;
+                const int i = r0 + lr + hh * 8, j = c0v + nt * 8 + lc2;
                 const float bi = sBe[i];
-                const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(sV + i * LDV + j);
+                const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(s1 + i * LDV + j);
                 rb[hh] += acc2[0][nt][hh * 2] * __bfloat162float(x.x) + acc2[0][nt][hh * 2 + 1] * __bfloat162float(x.y);
                 const float d0 = acc[0][nt][hh * 2] + bi * acc2[0][nt][hh * 2], d1 = acc[0][nt][hh * 2 + 1] + bi * acc2[0][nt][hh * 2 + 1];
                 if (p.dv_bf16) *reinterpret_cast<uint32_t*>(p.dv_bf16 + (rowbase + (long)i * p.H) * VD + j) = pack_bf16(d0, d1);
@@ -361,121 +291,11 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
             if ((lane & 3) == 0) pRowB_V[cw * CH + r0 + lr + hh * 8] = rb[hh];
         }
     }
-    STAMP();
-    // ---- dQK = tril(dX Aw^T - (d_qd exp(G)) w^T)
+    // ---- dAu = (d_u v^T) * beta_j
     {
         float acc[1][4][4];
         zero_acc(acc);
-        warp_gemm<1, 2, false, false>(acc, sTb, LDP, r0, sAw, LDP, cw * 32, CH, lane);
-        warp_gemm<1, 2, false, false>(acc, sDqd, LDK, r0, sW, LDK, cw * 32, KD, lane);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + lr + hh * 8, j = cw * 32 + nt * 8 + lc2;
-                *reinterpret_cast<uint32_t*>(sDQK + i * LDP + j) =
-                    pack_bf16(j <= i ? acc[0][nt][hh * 2] : 0.f, j + 1 <= i ? acc[0][nt][hh * 2 + 1] : 0.f);
-            }
-    }
-    STAMP();
-    // ---- dw = d_wd exp(G) - QK^T (d_qd exp(G))
-    {
-        float acc[1][2 * NPK][4];
-        zero_acc(acc);
-        const int c0 = cw * (KD / 2);
-        // the fp32 gradient fragment is requested before the product so that its latency overlaps the MMAs
-        float2 pre[2 * NPK][2];
-#pragma unroll
-        for (int nt = 0; nt < 2 * NPK; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-                pre[nt][hh] = *reinterpret_cast<const float2*>(p.d_wd + (rowbase + (long)(r0 + lr + hh * 8) * p.H) * KD + c0 + nt * 8 + lc2);
-        warp_gemm<1, NPK, true, true>(acc, sQK, LDP, r0, sDqd, LDK, c0, CH, lane);
-#pragma unroll
-        for (int nt = 0; nt < 2 * NPK; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + lr + hh * 8, j = c0 + nt * 8 + lc2;
-                const float2 d = pre[nt][hh];
-                const float eg = sEG[i];
-                *reinterpret_cast<uint32_t*>(sDW + i * LDK + j) = pack_bf16(acc[0][nt][hh * 2] + d.x * eg, acc[0][nt][hh * 2 + 1] + d.y * eg);
-            }
-    }
-    __syncthreads();                           // dw and dQK complete; P has been consumed
-    STAMP();
-    // ---- dAw = QK^T dX + (dw k^T) * beta_j   -> tile
-    {
-        float acc[1][4][4], acc2[1][4][4];
-        zero_acc(acc);
-        zero_acc(acc2);
-        warp_gemm<1, 2, true, true>(acc, sQK, LDP, r0, sTb, LDP, cw * 32, CH, lane);
-        warp_gemm<1, 2, false, false>(acc2, sDW, LDK, r0, sK, LDK, cw * 32, KD, lane);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + lr + hh * 8, j = cw * 32 + nt * 8 + lc2;
-                *reinterpret_cast<uint32_t*>(sTa + i * LDP + j) =
-                    pack_bf16(acc[0][nt][hh * 2] + acc2[0][nt][hh * 2] * sBe[j], acc[0][nt][hh * 2 + 1] + acc2[0][nt][hh * 2 + 1] * sBe[j + 1]);
-            }
-    }
-    __syncthreads();                           // dAw complete; dX and QK have been consumed
-    STAMP();
-    // ---- dAw Aw^T -> tile
-    {
-        float acc[1][4][4];
-        zero_acc(acc);
-        warp_gemm<1, 2, false, false>(acc, sTa, LDP, r0, sAw, LDP, cw * 32, CH, lane);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-                *reinterpret_cast<uint32_t*>(sTb + (r0 + lr + hh * 8) * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
-    }
-    __syncthreads();
-    STAMP();
-    // ---- dA (from Aw) = -Aw^T (dAw Aw^T) ;  d(beta k) = Aw^T dw starts the dk accumulator
-    float dA1[1][4][4];
-    float dk_acc[1][2 * NPK][4];
-    {
-        zero_acc(dA1);
-        warp_gemm<1, 2, true, true>(dA1, sAw, LDP, r0, sTb, LDP, cw * 32, CH, lane);
-        zero_acc(dk_acc);
-        const int c0 = cw * (KD / 2);
-        float2 pre[2 * NPK][2];
-#pragma unroll
-        for (int nt = 0; nt < 2 * NPK; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-                pre[nt][hh] = *reinterpret_cast<const float2*>(p.d_kd + (rowbase + (long)(r0 + lr + hh * 8) * p.H) * KD + c0 + nt * 8 + lc2);
-        warp_gemm<1, NPK, true, true>(dk_acc, sAw, LDP, r0, sDW, LDK, c0, CH, lane);
-        float rb[2] = {0.f, 0.f};
-#pragma unroll
-        for (int nt = 0; nt < 2 * NPK; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + lr + hh * 8, j = c0 + nt * 8 + lc2;
-                const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(sK + i * LDK + j);
-                rb[hh] += dk_acc[0][nt][hh * 2] * __bfloat162float(x.x) + dk_acc[0][nt][hh * 2 + 1] * __bfloat162float(x.y);
-                const float bi = sBe[i];
-                const float2 d = pre[nt][hh];
-                const float ek = sEGk[i];
-                dk_acc[0][nt][hh * 2] = dk_acc[0][nt][hh * 2] * bi + d.x * ek;
-                dk_acc[0][nt][hh * 2 + 1] = dk_acc[0][nt][hh * 2 + 1] * bi + d.y * ek;
-            }
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 1);
-            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 2);
-            if ((lane & 3) == 0) pRowB_K[cw * CH + r0 + lr + hh * 8] = rb[hh];
-        }
-    }
-    STAMP();
-    // ---- dAu = (d_u v^T) * beta_j -> tile (the dAw tile has been consumed before the last barrier)
-    {
-        float acc[1][4][4];
-        zero_acc(acc);
-        warp_gemm<1, 2, false, false>(acc, sDU, LDV, r0, sV, LDV, cw * 32, VD, lane);
+        warp_gemm<1, 2, false, false>(acc, s2, LDV, r0, s1, LDV, cw * 32, VD, lane);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -484,26 +304,30 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
                 *reinterpret_cast<uint32_t*>(sTa + (r0 + lr + hh * 8) * LDP + j) = pack_bf16(acc[0][nt][hh * 2] * sBe[j], acc[0][nt][hh * 2 + 1] * sBe[j + 1]);
             }
     }
-    __syncthreads();                           // dAu complete; (dAw Aw^T) consumed
-    STAMP();
+    __syncthreads();                           // dAu complete; v and d_u consumed
+    if (FUSED) {
+        load_tile_async<CH, KD, 256>(s2, p.dqd_neg + rowbase * KD, (long)p.H * KD, tid);
+        cp_async_commit();
+    }
+    // ---- dAu Au^T takes the place of dAu
     {
         float acc[1][4][4];
         zero_acc(acc);
         warp_gemm<1, 2, false, false>(acc, sTa, LDP, r0, sAu, LDP, cw * 32, CH, lane);
+        __syncthreads();
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh)
-                *reinterpret_cast<uint32_t*>(sTb + (r0 + lr + hh * 8) * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
+                *reinterpret_cast<uint32_t*>(sTa + (r0 + lr + hh * 8) * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
     }
     __syncthreads();
-    STAMP();
-    // ---- dAg = -Au^T (dAu Au^T);  dA = dA1 + dAg * Gamma;  decay and beta terms;  dKK = beta_i dA
+    // ---- dAg = -Au^T (dAu Au^T), times Gamma, and its decay terms
+    float dag[1][4][4];
     {
-        float dAg[1][4][4];
-        zero_acc(dAg);
-        warp_gemm<1, 2, true, true>(dAg, sAu, LDP, r0, sTb, LDP, cw * 32, CH, lane);
-        float rs[2] = {0.f, 0.f}, rb[2] = {0.f, 0.f};
+        zero_acc(dag);
+        warp_gemm<1, 2, true, true>(dag, sAu, LDP, r0, sTa, LDP, cw * 32, CH, lane);
+        float rs[2] = {0.f, 0.f};
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
             float cs[2] = {0.f, 0.f};
@@ -513,25 +337,19 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
             for (int hh = 0; hh < 2; ++hh) {
                 const int i = r0 + lr + hh * 8;
                 const float gi = sG[i], bi = sBe[i];
-                float dkk[2] = {0.f, 0.f};
-                const float2 kkv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sKK + i * LDP + cw * 32 + nt * 8 + lc2));
+                const float2 kkv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&kk[nt][hh]));
                 if (cw * 4 + nt <= (r0 >> 3) + hh)       // 8 x 8 blocks above the diagonal hold no causal pair (the same for the whole warp)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int j = cw * 32 + nt * 8 + lc2 + e;
                     if (j < i) {
-                        const float gam = fexp(gi - gjA[e]);
-                        const float kk = e ? kkv.y : kkv.x;
-                        const float dag = -dAg[0][nt][hh * 2 + e];
-                        const float s = dag * bi * kk * gam;
+                        const float d = -dag[0][nt][hh * 2 + e] * fexp(gi - gjA[e]);
+                        const float s = d * bi * (e ? kkv.y : kkv.x);
                         rs[hh] += s;
                         cs[e] += s;
-                        const float da = -dA1[0][nt][hh * 2 + e] + dag * gam;
-                        rb[hh] += da * kk;
-                        dkk[e] = bi * da;
+                        dag[0][nt][hh * 2 + e] = d;
                     }
                 }
-                *reinterpret_cast<uint32_t*>(sQK + i * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(dkk[0], dkk[1]);
             }
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
@@ -544,53 +362,224 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
         for (int hh = 0; hh < 2; ++hh) {
             rs[hh] += __shfl_xor_sync(0xffffffffu, rs[hh], 1);
             rs[hh] += __shfl_xor_sync(0xffffffffu, rs[hh], 2);
-            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 1);
-            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 2);
-            if ((lane & 3) == 0) {
-                pRowG_A[cw * CH + r0 + lr + hh * 8] = rs[hh];
-                pRowB_A[cw * CH + r0 + lr + hh * 8] = rb[hh];
-            }
+            if ((lane & 3) == 0) pRowG_A[cw * CH + r0 + lr + hh * 8] = rs[hh];
         }
     }
-    __syncthreads();                           // dKK complete (in the QK tile)
-    STAMP();
-    // ---- dq = d_qd exp(G) + dQK k ;  dk += dQK^T q + (dKK + dKK^T) k
+    __syncthreads();                           // Au and its products consumed
+    // row pass over the K-wide gradients: -(d_qd exp(G)) as a bf16 operand; the decay terms
+    //      dG_i += d_qd.qd + d_wd.wd - d_kd.kd and the chunk total of d_kd.kd
+    if (!FUSED) {
+        float kdsum = 0.f;
+        // four rows per batch: every load of a batch is issued before the first use, so a batch pays the load latency once
+#pragma unroll
+        for (int bt = 0; bt < CH / 32; ++bt) {
+            float4 a[4], bw[4], ck[4];
+            uint2 xq[4], xw[4], xk[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = (bt * 4 + u) * 8 + warp;
+                const long off = (rowbase + (long)i * p.H) * KD + lane * 4;
+                a[u] = __ldg(reinterpret_cast<const float4*>(p.d_qd + off));
+                bw[u] = __ldg(reinterpret_cast<const float4*>(p.d_wd + off));
+                ck[u] = __ldg(reinterpret_cast<const float4*>(p.d_kd + off));
+                xq[u] = __ldg(reinterpret_cast<const uint2*>(p.qd + off));
+                xw[u] = __ldg(reinterpret_cast<const uint2*>(p.wd + off));
+                xk[u] = __ldg(reinterpret_cast<const uint2*>(p.kd + off));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = (bt * 4 + u) * 8 + warp;
+                const __nv_bfloat162 q0 = *reinterpret_cast<const __nv_bfloat162*>(&xq[u].x), q1 = *reinterpret_cast<const __nv_bfloat162*>(&xq[u].y);
+                const __nv_bfloat162 w0 = *reinterpret_cast<const __nv_bfloat162*>(&xw[u].x), w1 = *reinterpret_cast<const __nv_bfloat162*>(&xw[u].y);
+                const __nv_bfloat162 k0 = *reinterpret_cast<const __nv_bfloat162*>(&xk[u].x), k1 = *reinterpret_cast<const __nv_bfloat162*>(&xk[u].y);
+                float dq_ = a[u].x * __bfloat162float(q0.x) + a[u].y * __bfloat162float(q0.y) + a[u].z * __bfloat162float(q1.x) + a[u].w * __bfloat162float(q1.y);
+                float dw_ = bw[u].x * __bfloat162float(w0.x) + bw[u].y * __bfloat162float(w0.y) + bw[u].z * __bfloat162float(w1.x) + bw[u].w * __bfloat162float(w1.y);
+                float dk_ = ck[u].x * __bfloat162float(k0.x) + ck[u].y * __bfloat162float(k0.y) + ck[u].z * __bfloat162float(k1.x) + ck[u].w * __bfloat162float(k1.y);
+                float r = dq_ + dw_ - dk_;
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) {
+                    r += __shfl_xor_sync(0xffffffffu, r, d);
+                    dk_ += __shfl_xor_sync(0xffffffffu, dk_, d);
+                }
+                if (lane == 0) sDG[i] += r;          // one warp per row: no other writer at this point
+                kdsum += dk_;
+                const float eg = -sEG[i];
+                uint2 o;
+                o.x = pack_bf16(a[u].x * eg, a[u].y * eg);
+                o.y = pack_bf16(a[u].z * eg, a[u].w * eg);
+                *reinterpret_cast<uint2*>(s2 + i * LDK + lane * 4) = o;
+            }
+        }
+        if (lane == 0) atomicAdd(&sMisc[0], kdsum);
+    }
+    // ---- w = (Aw * beta_j) k
+    for (int e = tid; e < CH * CH / 2; e += 256) {
+        const int i = e / (CH / 2), j = (e % (CH / 2)) * 2;
+        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(sAw + i * LDP + j);
+        *reinterpret_cast<uint32_t*>(sTa + i * LDP + j) = pack_bf16(__bfloat162float(x.x) * sBe[j], __bfloat162float(x.y) * sBe[j + 1]);
+    }
+    __syncthreads();
     {
-        const int c0 = cw * (KD / 2);
         float acc[1][2 * NPK][4];
         zero_acc(acc);
+        warp_gemm<1, NPK, false, true>(acc, sTa, LDP, r0, sK, LDK, c0k, CH, lane);
+#pragma unroll
+        for (int nt = 0; nt < 2 * NPK; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh)
+                *reinterpret_cast<uint32_t*>(s1 + (r0 + lr + hh * 8) * LDK + c0k + nt * 8 + lc2) = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
+    }
+    cp_async_wait<0>();                        // the bf16 d_qd term has landed
+    __syncthreads();
+    // ---- dQK = tril(dX Aw^T - (d_qd exp(G)) w^T), in the place of Au
+    warp_gemm<1, 2, false, false>(dqk, s2, LDK, r0, s1, LDK, cw * 32, KD, lane);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int i = r0 + lr + hh * 8, j = cw * 32 + nt * 8 + lc2;
+            *reinterpret_cast<uint32_t*>(sAu + i * LDP + j) =
+                pack_bf16(j <= i ? dqk[0][nt][hh * 2] : 0.f, j + 1 <= i ? dqk[0][nt][hh * 2 + 1] : 0.f);
+        }
+    // ---- dw = d_wd exp(G) - QK^T (d_qd exp(G)), in the place of w
+    {
+        float acc[1][2 * NPK][4];
+        zero_acc(acc);
+        warp_gemm<1, NPK, true, true>(acc, sQK, LDP, r0, s2, LDK, c0k, CH, lane);
+        __syncthreads();                       // w and d_qd consumed
+        load_tile_async<CH, KD, 256>(s2, p.q + rowbase * KD, (long)p.H * KD, tid);
+        cp_async_commit();
+#pragma unroll
+        for (int nt = 0; nt < 2 * NPK; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int i = r0 + lr + hh * 8, j = c0k + nt * 8 + lc2;
+                const float2 d = *reinterpret_cast<const float2*>(p.d_wd + (rowbase + (long)i * p.H) * KD + j);
+                const float eg = sEG[i];
+                *reinterpret_cast<uint32_t*>(s1 + i * LDK + j) = pack_bf16(acc[0][nt][hh * 2] + d.x * eg, acc[0][nt][hh * 2 + 1] + d.y * eg);
+            }
+    }
+    __syncthreads();                           // dw complete
+    // ---- dAw = QK^T dX + (dw k^T) * beta_j
+    {
+        float acc[1][4][4], acc2[1][4][4];
+        zero_acc(acc);
+        zero_acc(acc2);
+        warp_gemm<1, 2, true, true>(acc, sQK, LDP, r0, sTb, LDP, cw * 32, CH, lane);
+        warp_gemm<1, 2, false, false>(acc2, s1, LDK, r0, sK, LDK, cw * 32, KD, lane);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int i = r0 + lr + hh * 8, j = cw * 32 + nt * 8 + lc2;
+                *reinterpret_cast<uint32_t*>(sTa + i * LDP + j) =
+                    pack_bf16(acc[0][nt][hh * 2] + acc2[0][nt][hh * 2] * sBe[j], acc[0][nt][hh * 2 + 1] + acc2[0][nt][hh * 2 + 1] * sBe[j + 1]);
+            }
+    }
+    __syncthreads();                           // dAw complete; dX and QK have been consumed
+    // ---- dAw Aw^T
+    {
+        float acc[1][4][4];
+        zero_acc(acc);
+        warp_gemm<1, 2, false, false>(acc, sTa, LDP, r0, sAw, LDP, cw * 32, CH, lane);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh)
+                *reinterpret_cast<uint32_t*>(sTb + (r0 + lr + hh * 8) * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
+    }
+    __syncthreads();
+    // ---- dA = dAg * Gamma - Aw^T (dAw Aw^T) ;  its beta term ;  dKK = beta_i dA, in the place of QK
+    {
+        float acc[1][4][4];
+        zero_acc(acc);
+        warp_gemm<1, 2, true, true>(acc, sAw, LDP, r0, sTb, LDP, cw * 32, CH, lane);
+        float rb[2] = {0.f, 0.f};
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int i = r0 + lr + hh * 8;
+                const float bi = sBe[i];
+                const float2 kkv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&kk[nt][hh]));
+                float dkk[2] = {0.f, 0.f};
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    if (cw * 32 + nt * 8 + lc2 + e < i) {
+                        const float da = dag[0][nt][hh * 2 + e] - acc[0][nt][hh * 2 + e];
+                        rb[hh] += da * (e ? kkv.y : kkv.x);
+                        dkk[e] = bi * da;
+                    }
+                *reinterpret_cast<uint32_t*>(sQK + i * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(dkk[0], dkk[1]);
+            }
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 1);
+            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 2);
+            if ((lane & 3) == 0) pRowB_A[cw * CH + r0 + lr + hh * 8] = rb[hh];
+        }
+    }
+    // ---- dk = beta * (Aw^T dw) + d_kd exp(gl - G) + dQK^T q + (dKK + dKK^T) k ;  dbeta_i += (Aw^T dw)_i . k_i
+    {
+        float acc[1][2 * NPK][4];
+        zero_acc(acc);
+        warp_gemm<1, NPK, true, true>(acc, sAw, LDP, r0, s1, LDK, c0k, CH, lane);
+        float rb[2] = {0.f, 0.f};
+#pragma unroll
+        for (int nt = 0; nt < 2 * NPK; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int i = r0 + lr + hh * 8, j = c0k + nt * 8 + lc2;
+                const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(sK + i * LDK + j);
+                rb[hh] += acc[0][nt][hh * 2] * __bfloat162float(x.x) + acc[0][nt][hh * 2 + 1] * __bfloat162float(x.y);
+                const float bi = sBe[i];
+                const float2 d = *reinterpret_cast<const float2*>(p.d_kd + (rowbase + (long)i * p.H) * KD + j);
+                const float ek = sEGk[i];
+                acc[0][nt][hh * 2] = acc[0][nt][hh * 2] * bi + d.x * ek;
+                acc[0][nt][hh * 2 + 1] = acc[0][nt][hh * 2 + 1] * bi + d.y * ek;
+            }
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 1);
+            rb[hh] += __shfl_xor_sync(0xffffffffu, rb[hh], 2);
+            if ((lane & 3) == 0) pRowB_K[cw * CH + r0 + lr + hh * 8] = rb[hh];
+        }
+        cp_async_wait<0>();                    // q is back
+        __syncthreads();                       // dKK complete
+        warp_gemm<1, NPK, true, true>(acc, sAu, LDP, r0, s2, LDK, c0k, CH, lane);
+        warp_gemm<1, NPK, false, true>(acc, sQK, LDP, r0, sK, LDK, c0k, CH, lane);
+        warp_gemm<1, NPK, true, true>(acc, sQK, LDP, r0, sK, LDK, c0k, CH, lane);
+#pragma unroll
+        for (int nt = 0; nt < 2 * NPK; ++nt)
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int i = r0 + lr + hh * 8, j = c0k + nt * 8 + lc2;
+                *reinterpret_cast<float2*>(p.dk + (rowbase + (long)i * p.H) * KD + j) = make_float2(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
+            }
+    }
+    // ---- dq = d_qd exp(G) + dQK k
+    {
+        float acc[1][2 * NPK][4];
+        zero_acc(acc);
+        // the fp32 gradient fragment is requested before the product so that its latency overlaps the MMAs
         float2 pre[2 * NPK][2];
 #pragma unroll
         for (int nt = 0; nt < 2 * NPK; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh)
-                pre[nt][hh] = *reinterpret_cast<const float2*>(p.d_qd + (rowbase + (long)(r0 + lr + hh * 8) * p.H) * KD + c0 + nt * 8 + lc2);
-        warp_gemm<1, NPK, false, true>(acc, sDQK, LDP, r0, sK, LDK, c0, CH, lane);
-        STAMP();
+                pre[nt][hh] = *reinterpret_cast<const float2*>(p.d_qd + (rowbase + (long)(r0 + lr + hh * 8) * p.H) * KD + c0k + nt * 8 + lc2);
+        warp_gemm<1, NPK, false, true>(acc, sAu, LDP, r0, sK, LDK, c0k, CH, lane);
 #pragma unroll
         for (int nt = 0; nt < 2 * NPK; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + lr + hh * 8, j = c0 + nt * 8 + lc2;
-                const long off = (rowbase + (long)i * p.H) * KD + j;
+                const int i = r0 + lr + hh * 8, j = c0k + nt * 8 + lc2;
                 const float2 d = pre[nt][hh];
                 const float eg = sEG[i];
-                *reinterpret_cast<float2*>(p.dq + off) = make_float2(acc[0][nt][hh * 2] + d.x * eg, acc[0][nt][hh * 2 + 1] + d.y * eg);
-            }
-        STAMP();
-        warp_gemm<1, NPK, true, true>(dk_acc, sDQK, LDP, r0, sQ, LDK, c0, CH, lane);
-        warp_gemm<1, NPK, false, true>(dk_acc, sQK, LDP, r0, sK, LDK, c0, CH, lane);
-        warp_gemm<1, NPK, true, true>(dk_acc, sQK, LDP, r0, sK, LDK, c0, CH, lane);
-        STAMP();
-#pragma unroll
-        for (int nt = 0; nt < 2 * NPK; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int i = r0 + lr + hh * 8, j = c0 + nt * 8 + lc2;
-                *reinterpret_cast<float2*>(p.dk + (rowbase + (long)i * p.H) * KD + j) = make_float2(dk_acc[0][nt][hh * 2], dk_acc[0][nt][hh * 2 + 1]);
+                *reinterpret_cast<float2*>(p.dq + (rowbase + (long)i * p.H) * KD + j) =
+                    make_float2(acc[0][nt][hh * 2] + d.x * eg, acc[0][nt][hh * 2 + 1] + d.y * eg);
             }
     }
-    STAMP();
     // ---- dg = reverse cumulative sum of dG (the chunk total also collects the state-decay part and
     //      the total of d_kd . kd) ;  dbeta ;  d lambda of the intra-chunk levels
     if (warp == 0) {
@@ -622,7 +611,6 @@ __global__ void __launch_bounds__(256, 1) gdn_bwd_chunk_kernel(const GdnParams p
         const int i = e >> 3, lv = e & 7;
         if (lv < INTRA_LEVELS) p.dl[(rowbase + (long)i * p.H) * p.L + lv] = sDL[e];
     }
-    STAMP();
 }
 
 template <int KD, int VD, bool FUSED>
@@ -643,9 +631,3 @@ int gdn_bwd_chunk_dispatch(const GdnParams& p, cudaStream_t stream) {
 }
 
 }  // namespace llattn
-
-#ifdef LLATTN_STAMPS
-extern "C" int llattn_debug_read_stamps_gdn_chunk(long long* host_dst) {
-    return (int)cudaMemcpyFromSymbol(host_dst, llattn::g_stamps, sizeof(llattn::g_stamps));
-}
-#endif
