@@ -124,14 +124,14 @@ size_t llattn_mamba2_fwd_workspace_bytes(int B, int T, int H, int G, int K, int 
     return setup(p, nullptr, false);
 }
 
-int llattn_mamba2_fwd(const void* q, const void* k, const void* v, const float* g, const void* lambda,
-                      void* o, float* g_cum, void* workspace, size_t workspace_bytes,
-                      int B, int T, int H, int G, int K, int V, int L, void* stream) {
+static int mamba2_fwd_impl(llattn::Mamba2Params& p, const void* q, const void* k, const void* v, const float* g, const void* lambda,
+                           void* o, float* g_cum, void* workspace, size_t workspace_bytes,
+                           int B, int T, int H, int G, int K, int V, int L, void* stream) {
     int rc = check_shape(B, T, H, G, K, V, L);
     if (rc != 0) return rc;
-    if (!q || !k || !v || !g || !lambda || !o || !g_cum) return LLATTN_ERR_NULL;
-    llattn::Mamba2Params p = {};
+    if (!q || !k || !v || !g || !lambda || (!o && !p.res_D) || !g_cum) return LLATTN_ERR_NULL;
     p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
+    if (p.res_D && !llattn::mamba2_uses_tc(p)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     const size_t need = setup(p, nullptr, false);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) return LLATTN_ERR_WORKSPACE;
     setup(p, workspace, false);
@@ -141,6 +141,24 @@ int llattn_mamba2_fwd(const void* q, const void* k, const void* v, const float* 
     cudaError_t e = cudaMemsetAsync(p.err, 0, sizeof(int), (cudaStream_t)stream);
     if (e != cudaSuccess) return (int)e;
     return llattn::mamba2_fwd_dispatch(p, (cudaStream_t)stream);
+}
+
+int llattn_mamba2_fwd(const void* q, const void* k, const void* v, const float* g, const void* lambda,
+                      void* o, float* g_cum, void* workspace, size_t workspace_bytes,
+                      int B, int T, int H, int G, int K, int V, int L, void* stream) {
+    llattn::Mamba2Params p = {};
+    return mamba2_fwd_impl(p, q, k, v, g, lambda, o, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);
+}
+
+int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, const float* g, const void* lambda,
+                               const void* x, const void* D, void* y, int y_is_f32, int T_y, float* g_cum, void* workspace, size_t workspace_bytes,
+                               int B, int T, int H, int G, int K, int V, int L, void* stream) {
+    if (!x || !D || !y) return LLATTN_ERR_NULL;
+    if (T_y <= 0 || T_y > T) return LLATTN_ERR_BAD_LENGTH;
+    if (((uintptr_t)x | (uintptr_t)y) & 15) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    llattn::Mamba2Params p = {};
+    p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_T = T_y; p.res_f32 = y_is_f32;
+    return mamba2_fwd_impl(p, q, k, v, g, lambda, nullptr, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);
 }
 
 size_t llattn_static_scratch_bytes(void) { return LLATTN_STATIC_SCRATCH_BYTES; }

@@ -23,7 +23,7 @@ using torch::autograd::Variable;
 using torch::autograd::variable_list;
 
 #define LLATTN_FUNCS(F)                                                                                                             \
-    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
+    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_fwd_residual) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
     F(llattn_mamba2_layer_prep_fwd) F(llattn_mamba2_layer_prep_bwd) F(llattn_mamba2_layer_step) F(llattn_gdn_layer_step)            \
     F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mixer_prep_fwd)            \
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
@@ -128,6 +128,29 @@ Scan mamba2_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&
     if (status) check_status(s.ws, stream, "llattn_mamba2_fwd");
     return s;
 }
+// the same with y = o + D x of the first x.size(1) tokens in the place of o
+Scan mamba2_fwd_residual(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, const Tensor& x, const Tensor& D,
+                         void* stream, bool status) {
+    const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3), Ty = x.size(1);
+    Scan s;
+    s.o = empty(x.sizes(), f32(D) ? at::kFloat : at::kBFloat16, x);
+    s.g_cum = at::empty_like(g);
+    const size_t n = lib.llattn_mamba2_fwd_workspace_bytes(B, T, H, G, K, V, L);
+    s.ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
+    const int rc = lib.llattn_mamba2_fwd_residual(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), l.data_ptr(), x.data_ptr(), D.data_ptr(),
+                                                  s.o.data_ptr(), f32(D), Ty, fptr(s.g_cum), s.ws.data_ptr(), s.ws.numel(), B, T, H, G, K, V, L, stream);
+    if (rc == LLATTN_ERR_UNSUPPORTED_SHAPE) {
+        const Tensor y = s.o;
+        s = mamba2_fwd(q, k, v, g, l, stream, status);
+        check(lib.llattn_mamba2_prompt_residual(s.o.data_ptr(), x.data_ptr(), ptr(D), y.data_ptr(), f32(D), B, Ty, T, H, V, stream),
+              "llattn_mamba2_prompt_residual");
+        s.o = y;
+        return s;
+    }
+    check(rc, "llattn_mamba2_fwd_residual");
+    if (status) check_status(s.ws, stream, "llattn_mamba2_fwd_residual");
+    return s;
+}
 struct ScanGrads {
     Tensor dq, dk, dv, dg, dl;       // dl fp32
 };
@@ -201,13 +224,8 @@ struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
         check(lib.llattn_mamba2_layer_prep_fwd(x_.data_ptr(), dt_.data_ptr(), ptr(b_), f32(b_), fptr(A_), dl_.data_ptr(), Lp_.data_ptr(), f32(Lp_),
                                                v.data_ptr(), fptr(g), lam.data_ptr(), (long)B * T * H, H, P, L, (int)mode, on.stream),
               "llattn_mamba2_layer_prep_fwd");
-        Scan s = mamba2_fwd(q, k, v, g, lam, on.stream, status);
-        Tensor y = s.o;
-        if (D_.defined()) {
-            y = empty(x_.sizes(), f32(D_) ? at::kFloat : at::kBFloat16, x);
-            check(lib.llattn_mamba2_prompt_residual(s.o.data_ptr(), x_.data_ptr(), ptr(D_), y.data_ptr(), f32(D_), B, T, T, H, P, on.stream),
-                  "llattn_mamba2_prompt_residual");
-        }
+        const Scan s = D_.defined() ? mamba2_fwd_residual(q, k, v, g, lam, x_, D_, on.stream, status) : mamba2_fwd(q, k, v, g, lam, on.stream, status);
+        const Tensor& y = s.o;
         if (ctx) {
             ctx->save_for_backward({x_, dt_, A_, k, q, dl_, Lp_, D_, b_, v, s.g_cum, lam, keep ? s.ws : Tensor()});
             ctx->saved_data["mode"] = mode;
@@ -298,19 +316,13 @@ py::object mamba2_prompt(const Tensor& x, const Tensor& dt, const Tensor& A, con
             q = qp;
             k = kp;
         }
-        Scan s = mamba2_fwd(q, k, v, g, lam, on.stream, status);
+        const Scan s = D_c.defined() ? mamba2_fwd_residual(q, k, v, g, lam, x_, D_c, on.stream, status) : mamba2_fwd(q, k, v, g, lam, on.stream, status);
         states = empty({B, H, L, N, P}, at::kFloat, x);
         check(lib.llattn_mamba2_prompt_states(k.data_ptr(), v.data_ptr(), fptr(g), fptr(states), s.ws.data_ptr(), s.ws.numel(), B, T, Tp, H, G, N, P, L,
                                               on.stream),
               "llattn_mamba2_prompt_states");
         states = states.permute({0, 1, 3, 4, 2});
-        if (D_c.defined() || (Tp != T && B > 1)) {
-            y = empty({B, T, H, P}, D_c.defined() && f32(D_c) ? at::kFloat : at::kBFloat16, x);
-            check(lib.llattn_mamba2_prompt_residual(s.o.data_ptr(), x_.data_ptr(), ptr(D_c), y.data_ptr(), f32(y), B, T, Tp, H, P, on.stream),
-                  "llattn_mamba2_prompt_residual");
-        } else {
-            y = s.o.narrow(1, 0, T);
-        }
+        y = D_c.defined() ? s.o : s.o.narrow(1, 0, T).contiguous();
     }
     return py::make_tuple(y, states);
 }

@@ -53,6 +53,11 @@ struct Mamba2Params {
     int o_has_high;
     int lev_lo;                  // first segment level handled by one launch of the tensor-core high-level backward
     int chunk_rounding;          // backward: a sequence of an odd number of chunks, or with K = 64, takes the chunk-by-chunk kernels
+    // forward of a layer: y = o + D x takes the place of o (tensor-core kernels; res_D NULL: none)
+    const __nv_bfloat16* res_x;  // (B,res_T,H,V)
+    const void* res_D;           // (H), fp32 like y if res_f32, else bf16
+    void* res_y;                 // (B,res_T,H,V)
+    int res_T, res_f32;          // res_T <= T: a prompt's tokens without its padding
     int reuse_states;            // backward: seg_D / seg_H0 come from the forward call, do not recompute them
 };
 

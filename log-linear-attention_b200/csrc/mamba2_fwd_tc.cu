@@ -30,7 +30,10 @@ struct FwdTcSmem {
     static constexpr uint32_t total = bar_off + 128 + 1024;             // + slack for 1024-byte alignment
 };
 
-template <int MLOW, bool WHOLE>
+// RES: 0 writes o; 1, 2 write y = o + D x of a layer (bf16 / fp32), o rounded to bf16 first as if it were stored.  As a pass of its own that sum
+// reads o and x again and took 45 of 494 us for a layer's forward at B = 8, T = 4096, 24 heads; here x is on its way while the level
+// reads are summed.
+template <int MLOW, bool WHOLE, int RES>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = FwdTcSmem<MLOW>;
@@ -391,6 +394,15 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = 0.f;
         }
+        uint4 xr[RES ? 4 : 1];
+        if (RES) {
+            const bf16* gx = p.res_x + (((long)b * p.res_T + t0) * p.H + h) * tc::VD + (tid & 7) * 8;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int rr = (tid >> 3) + u * 32;
+                xr[u] = t0 + rr < p.res_T ? __ldg(reinterpret_cast<const uint4*>(gx + (long)rr * p.H * tc::VD)) : make_uint4(0, 0, 0, 0);
+            }
+        }
         if (nread > 0) {
             int slot = 0;
 #pragma unroll
@@ -422,9 +434,36 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
                 *reinterpret_cast<uint4*>(sP + umma::tile_offset(row, ch * 32 + c * 8, tc::PT)) = x;
             }
             asm volatile("bar.sync 2, 256;\n" ::: "memory");
+            if (RES) {
+                const float dh = load_param(p.res_D, h, RES == 2);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int rr = (tid >> 3) + u * 32, c = (tid & 7) * 8;
+                    if (t0 + rr >= p.res_T) continue;
+                    const uint4 ov = *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
+                    const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, xw[4] = {xr[u].x, xr[u].y, xr[u].z, xr[u].w};
+                    float y[8];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 of = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ow[e]));
+                        const float2 xf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xw[e]));
+                        y[2 * e] = of.x + xf.x * dh;
+                        y[2 * e + 1] = of.y + xf.y * dh;
+                    }
+                    const long at = (((long)b * p.res_T + t0 + rr) * p.H + h) * tc::VD + c;
+                    if (RES == 2) {
+                        float* w = reinterpret_cast<float*>(p.res_y) + at;
+                        *reinterpret_cast<float4*>(w) = make_float4(y[0], y[1], y[2], y[3]);
+                        *reinterpret_cast<float4*>(w + 4) = make_float4(y[4], y[5], y[6], y[7]);
+                    } else {
+                        *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.res_y) + at) =
+                            make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
+                    }
+                }
+            }
             bf16* go = p.o + (((long)b * p.T + t0) * p.H + h) * tc::VD;
 #pragma unroll
-            for (int i = tid; i < tc::PT * 8; i += 256) {
+            for (int i = RES ? tc::PT * 8 : tid; i < tc::PT * 8; i += 256) {
                 const int rr = i >> 3, c = (i & 7) * 8;
                 if (WHOLE || t0 + rr < p.T)
                     *reinterpret_cast<uint4*>(go + (long)rr * p.H * tc::VD + c) = *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
@@ -482,18 +521,24 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
     bar_work();
 }
 
+template <int RES>
+static int launch_chunk_fwd(const Mamba2Params& p, cudaStream_t stream) {
+    auto kern = mamba2_whole_pairs(p) ? m2_chunk_fwd_tc_kernel<M2_MLOW, true, RES> : m2_chunk_fwd_tc_kernel<M2_MLOW, false, RES>;
+    const size_t sm = FwdTcSmem<M2_MLOW>::total;
+    cudaError_t e = allow_smem(kern, sm);
+    if (e != cudaSuccess) return (int)e;
+    llattn::launch_chained(kern, p.B * p.H * p.NS, tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
 int mamba2_fwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
     if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
-    auto kern = mamba2_whole_pairs(p) ? m2_chunk_fwd_tc_kernel<M2_MLOW, true> : m2_chunk_fwd_tc_kernel<M2_MLOW, false>;
-    const size_t sm = FwdTcSmem<M2_MLOW>::total;
-    cudaError_t e = allow_smem(kern, sm);
-    if (e != cudaSuccess) return (int)e;
-    llattn::launch_chained(kern, p.B * p.H * p.NS, tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
-    return (int)cudaGetLastError();
+    if (!p.res_D) return launch_chunk_fwd<0>(p, stream);
+    return p.res_f32 ? launch_chunk_fwd<2>(p, stream) : launch_chunk_fwd<1>(p, stream);
 }
 
 }  // namespace llattn
