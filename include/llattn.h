@@ -61,7 +61,7 @@ int llattn_mamba2_fwd(const void* q, const void* k, const void* v, const float* 
                       int B, int T, int H, int G, int K, int V, int L, void* stream);
 
 /* llattn_mamba2_fwd whose output leaves as y (B,T_y,H,V) = o + D x, o rounded to bf16 first: the D residual of a Mamba-2 layer, of the first
- * T_y <= T tokens.  x is (B,T_y,H,V) bf16; y and D (H) are fp32 (y_is_f32 != 0) or bf16; x and y are 16-byte aligned.  LLATTN_ERR_UNSUPPORTED_SHAPE
+ * T_y <= T tokens.  x is (B,T_y,H,V) bf16; y and D (H) are fp32 (y_is_f32 != 0) or bf16; x is 16-byte, y 32-byte aligned.  LLATTN_ERR_UNSUPPORTED_SHAPE
  * where the tensor-core kernels do not run (L > 20): there o and the sum are two calls (llattn_mamba2_prompt_residual). */
 int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, const float* g, const void* lambda,
                                const void* x, const void* D, void* y, int y_is_f32, int T_y, float* g_cum, void* workspace, size_t workspace_bytes,

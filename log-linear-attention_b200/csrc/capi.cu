@@ -155,7 +155,7 @@ int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, cons
                                int B, int T, int H, int G, int K, int V, int L, void* stream) {
     if (!x || !D || !y) return LLATTN_ERR_NULL;
     if (T_y <= 0 || T_y > T) return LLATTN_ERR_BAD_LENGTH;
-    if (((uintptr_t)x | (uintptr_t)y) & 15) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (((uintptr_t)x & 15) || ((uintptr_t)y & 31)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     llattn::Mamba2Params p = {};
     p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_T = T_y; p.res_f32 = y_is_f32;
     return mamba2_fwd_impl(p, q, k, v, g, lambda, nullptr, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);

@@ -31,8 +31,8 @@ struct FwdTcSmem {
 };
 
 // RES: 0 writes o; 1, 2 write y = o + D x of a layer (bf16 / fp32), o rounded to bf16 first as if it were stored.  As a pass of its own that sum
-// reads o and x again and took 45 of 494 us for a layer's forward at B = 8, T = 4096, 24 heads; here x is on its way while the level
-// reads are summed.
+// reads o and x again and took 45 of 494 us for a layer's forward at B = 8, T = 4096, 24 heads; here x comes to L2 while the
+// products run and is read while the level reads are summed (466 us).
 template <int MLOW, bool WHOLE, int RES>
 __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
@@ -268,6 +268,9 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
             for (int c = 0; c < 4; ++c) ohi[c] = *reinterpret_cast<const uint4*>(gh + c * tc::PT * 8);
         }
+        // x rows of the pair into L2 (held in registers from here on they cost the products below more than they save)
+        if (RES && ch == 0 && t0 + row < p.res_T)
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.res_x + (((long)b * p.res_T + t0 + row) * p.H + h) * tc::VD));
         STAMP();                                     // 1: small fetches issued
         umma::mbar_wait(&full_kv[st], (pl >> 1) & 1, abort_flag);      // the v tile (read below with generic loads)
         STAMP();                                     // 2: tiles landed
@@ -452,9 +455,10 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
                     }
                     const long at = (((long)b * p.res_T + t0 + rr) * p.H + h) * tc::VD + c;
                     if (RES == 2) {
-                        float* w = reinterpret_cast<float*>(p.res_y) + at;
-                        *reinterpret_cast<float4*>(w) = make_float4(y[0], y[1], y[2], y[3]);
-                        *reinterpret_cast<float4*>(w + 4) = make_float4(y[4], y[5], y[6], y[7]);
+                        uint32_t w[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(y[e]);
+                        st_global_32B(reinterpret_cast<float*>(p.res_y) + at, w);
                     } else {
                         *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.res_y) + at) =
                             make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
