@@ -346,6 +346,13 @@ int llattn_gdn_bwd_kept_bf16dv(const void* q, const void* k, const void* v, cons
                                size_t fwd_workspace_bytes, void* workspace, size_t workspace_bytes,
                                int B, int T, int H, int K, int V, int L, void* stream);
 
+/* llattn_gdn_bwd_kept_bf16dv that also takes the backward of the l2 normalisation (below): q = l2norm(raw_q) * scale, k = l2norm(raw_k), and gq,
+ * gk (B,T,H,K) bf16 are the gradients of raw_q, raw_k.  K = 128. */
+int llattn_gdn_bwd_kept_normed(const void* q, const void* k, const void* raw_q, const void* raw_k, float scale, const void* v, const void* beta,
+                               const float* g_cum, const void* lambda, const void* Aw, const void* Au, const void* d_o, void* gq, void* gk,
+                               void* dv_bf16, float* dbeta, float* dg, float* dlambda, const void* fwd_workspace, size_t fwd_workspace_bytes,
+                               void* workspace, size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream);
+
 /* Row-wise L2 normalisation of q / k and its backward, as applied around the Gated DeltaNet drivers
  * when use_qk_l2norm_in_kernel is set.  Replace fla.modules.l2norm.l2norm_fwd / l2norm_bwd with the
  * scale folded in (hattention/kernel.py:20-29: l2norm_and_scale_fwd / l2norm_and_scale_bwd).
@@ -359,7 +366,7 @@ int llattn_l2norm_bwd(const void* x, const float* dy, void* dx, long rows, int D
  * most 128: padded keys) at raw q, k (q with `scale`), gbeta (rows) and glambda (rows,L) bf16; lambda_mul != 0: glambda is
  * rounded, multiplied and rounded again, as the reference's lambda / scale differentiates (gated_delta_rule_apis.py:65-70).  The fp32
  * inputs have `rep` rows for each row of the results, which are summed (parts of a wide value head); gg (rows) takes the sums of dg where
- * dg is given. */
+ * dg is given.  Without q (NULL) dbeta and dlambda only. */
 int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const float* dk, const float* dbeta, const float* dlambda,
                         const float* dg, void* gq, void* gk, void* gbeta, void* glambda, float* gg, long rows, int rep, int K, int K_in, int L,
                         float scale, float lambda_mul, void* stream);

@@ -462,16 +462,29 @@ size_t llattn_gdn_bwd_workspace_bytes(int B, int T, int H, int K, int V, int L) 
     return gdn_bwd_setup(p, nullptr);
 }
 
+struct GdnNormOut {
+    const void *raw_q, *raw_k;
+    void *gq, *gk;
+    float scale;
+};
+
 static int gdn_bwd_impl(const void* q, const void* k, const void* v, const void* beta, const float* g_cum, const void* lambda,
                         const void* Aw, const void* Au, const void* d_o, float* dq, float* dk, float* dv, float* dbeta, float* dg,
                         float* dlambda, const void* fwd_workspace, size_t fwd_workspace_bytes, void* workspace,
-                        size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream, void* dv_bf16 = nullptr) {
+                        size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream, void* dv_bf16 = nullptr,
+                        const GdnNormOut* norm = nullptr) {
     int rc = gdn_check(B, T, H, K, V, L);
     if (rc != 0) return rc;
-    if (!q || !k || !v || !beta || !g_cum || !lambda || !Aw || !Au || !d_o || !dq || !dk || (!dv && !dv_bf16) || !dbeta || !dg || !dlambda)
+    if (!q || !k || !v || !beta || !g_cum || !lambda || !Aw || !Au || !d_o || (!norm && (!dq || !dk)) || (!dv && !dv_bf16) || !dbeta || !dg || !dlambda)
         return LLATTN_ERR_NULL;
     llattn::GdnParams p = {};
     p.B = B; p.T = T; p.H = H; p.K = K; p.V = V; p.L = L;
+    if (norm) {
+        // the kernel that takes the normalisation's backward along is the one behind the tensor-core level gradients
+        if (!llattn::gdn_bwd_levels_writes_row_terms(p)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+        p.raw_q = (const __nv_bfloat16*)norm->raw_q; p.raw_k = (const __nv_bfloat16*)norm->raw_k;
+        p.gq = (__nv_bfloat16*)norm->gq; p.gk = (__nv_bfloat16*)norm->gk; p.q_scale = norm->scale;
+    }
     const bool kept = fwd_workspace != nullptr;
     if (kept) {
         // chunk matrices and level states as llattn_gdn_fwd_keep left them
@@ -517,6 +530,16 @@ int llattn_gdn_bwd_kept_bf16dv(const void* q, const void* k, const void* v, cons
     if (!fwd_workspace || !dv_bf16) return LLATTN_ERR_NULL;
     return gdn_bwd_impl(q, k, v, beta, g_cum, lambda, Aw, Au, d_o, dq, dk, nullptr, dbeta, dg, dlambda, fwd_workspace,
                         fwd_workspace_bytes, workspace, workspace_bytes, B, T, H, K, V, L, stream, dv_bf16);
+}
+
+int llattn_gdn_bwd_kept_normed(const void* q, const void* k, const void* raw_q, const void* raw_k, float scale, const void* v, const void* beta,
+                               const float* g_cum, const void* lambda, const void* Aw, const void* Au, const void* d_o, void* gq, void* gk,
+                               void* dv_bf16, float* dbeta, float* dg, float* dlambda, const void* fwd_workspace, size_t fwd_workspace_bytes,
+                               void* workspace, size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream) {
+    if (!fwd_workspace || !dv_bf16 || !raw_q || !raw_k || !gq || !gk) return LLATTN_ERR_NULL;
+    const GdnNormOut norm{raw_q, raw_k, gq, gk, scale};
+    return gdn_bwd_impl(q, k, v, beta, g_cum, lambda, Aw, Au, d_o, nullptr, nullptr, nullptr, dbeta, dg, dlambda, fwd_workspace,
+                        fwd_workspace_bytes, workspace, workspace_bytes, B, T, H, K, V, L, stream, dv_bf16, &norm);
 }
 
 size_t llattn_gdn_bwd_kept_workspace_bytes(int B, int T, int H, int K, int V, int L) {

@@ -29,7 +29,7 @@ using torch::autograd::variable_list;
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
     F(llattn_gdn_fwd_workspace_bytes) F(llattn_gdn_fwd_keep_workspace_bytes) F(llattn_gdn_fwd) F(llattn_gdn_fwd_keep)                \
     F(llattn_gdn_prefill_parts) F(llattn_gdn_prompt_states) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
-    F(llattn_gdn_bwd_kept_workspace_bytes) F(llattn_gdn_bwd_kept_bf16dv) F(llattn_gdn_grad_out) F(llattn_workspace_status)
+    F(llattn_gdn_bwd_kept_workspace_bytes) F(llattn_gdn_bwd_kept_bf16dv) F(llattn_gdn_bwd_kept_normed) F(llattn_gdn_grad_out) F(llattn_workspace_status)
 
 struct Library {
 #define LLATTN_MEMBER(name) decltype(&::name) name = nullptr;
@@ -521,32 +521,49 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
                   "llattn_gdn_prompt_prep");
         }
         const Tensor d_o = d[0].to(at::kBFloat16).contiguous();
-        // fp32 gradients of what the parts of a head share: dq | dk | dbeta | dlambda in one buffer, and dg, which is handed on as it is
-        // where a head has one part
+        // fp32 gradients of what the parts of a head share; dg is handed on as it is where a head has one part
         const int64_t rows = (int64_t)B * T * a.H, prows = rows * a.rep;
-        const Tensor out = empty({prows * (2 * GDN_K + 1 + a.L)}, at::kFloat, q), dgp = empty({B, T, H}, at::kFloat, q);
-        float *dq = fptr(out), *dk = dq + prows * GDN_K, *db = dk + prows * GDN_K, *dl = db + prows;
+        const Tensor gqk = empty({2, B, T, a.H, a.K}, at::kBFloat16, q), gq = gqk.select(0, 0), gk = gqk.select(0, 1);
+        const Tensor dgp = empty({B, T, H}, at::kFloat, q), dlb = empty({prows * (a.L + 1)}, at::kFloat, q);
+        float *dl = fptr(dlb), *db = dl + prows * a.L;
         const size_t bytes = (kept ? lib.llattn_gdn_bwd_kept_workspace_bytes : lib.llattn_gdn_bwd_workspace_bytes)(B, T, H, GDN_K, V, a.L);
         const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
         Tensor dv = empty(v.sizes(), kept ? at::kBFloat16 : at::kFloat, q);
-        if (kept) {
+        // heads of one part and full width: the kernels take the backward of the normalisation along
+        bool normed = kept && a.rep == 1 && a.K == GDN_K;
+        if (normed) {
             const Tensor& fws = s[10];
-            check(lib.llattn_gdn_bwd_kept_bf16dv(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(),
-                                                 Au.data_ptr(), d_o.data_ptr(), dq, dk, dv.data_ptr(), db, fptr(dgp), dl, fws.data_ptr(), fws.numel(),
-                                                 ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
-                  "llattn_gdn_bwd_kept_bf16dv");
-        } else {
-            check(lib.llattn_gdn_bwd(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(), Au.data_ptr(),
-                                     d_o.data_ptr(), dq, dk, fptr(dv), db, fptr(dgp), dl, ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
-                  "llattn_gdn_bwd");
-            dv = dv.to(at::kBFloat16);
+            const int rc = lib.llattn_gdn_bwd_kept_normed(qn.data_ptr(), kn.data_ptr(), q.data_ptr(), k.data_ptr(), (float)scale, v.data_ptr(), b.data_ptr(),
+                                                          fptr(g_cum), l.data_ptr(), Aw.data_ptr(), Au.data_ptr(), d_o.data_ptr(), gq.data_ptr(),
+                                                          gk.data_ptr(), dv.data_ptr(), db, fptr(dgp), dl, fws.data_ptr(), fws.numel(), ws.data_ptr(),
+                                                          bytes, B, T, H, GDN_K, V, a.L, on.stream);
+            normed = rc != LLATTN_ERR_UNSUPPORTED_SHAPE;
+            if (normed) check(rc, "llattn_gdn_bwd_kept_normed");
+        }
+        Tensor dqk;
+        float *dq = nullptr, *dk = nullptr;
+        if (!normed) {
+            dqk = empty({2 * prows * GDN_K}, at::kFloat, q);
+            dq = fptr(dqk);
+            dk = dq + prows * GDN_K;
+            if (kept) {
+                const Tensor& fws = s[10];
+                check(lib.llattn_gdn_bwd_kept_bf16dv(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(),
+                                                     Au.data_ptr(), d_o.data_ptr(), dq, dk, dv.data_ptr(), db, fptr(dgp), dl, fws.data_ptr(), fws.numel(),
+                                                     ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
+                      "llattn_gdn_bwd_kept_bf16dv");
+            } else {
+                check(lib.llattn_gdn_bwd(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g_cum), l.data_ptr(), Aw.data_ptr(), Au.data_ptr(),
+                                         d_o.data_ptr(), dq, dk, fptr(dv), db, fptr(dgp), dl, ws.data_ptr(), bytes, B, T, H, GDN_K, V, a.L, on.stream),
+                      "llattn_gdn_bwd");
+                dv = dv.to(at::kBFloat16);
+            }
         }
         if (status) check_status(ws, on.stream, "llattn_gdn_bwd");
-        const Tensor gqk = empty({2, B, T, a.H, a.K}, at::kBFloat16, q), gq = gqk.select(0, 0), gk = gqk.select(0, 1);
         const Tensor gb = empty({B, T, a.H}, at::kBFloat16, q), gl = empty({B, T, a.H, a.L}, at::kBFloat16, q);
         const Tensor gg = a.rep > 1 ? empty({B, T, a.H}, at::kFloat, q) : dgp;
-        check(lib.llattn_gdn_grad_out(q.data_ptr(), k.data_ptr(), dq, dk, db, dl, a.rep > 1 ? fptr(dgp) : nullptr, gq.data_ptr(), gk.data_ptr(), gb.data_ptr(),
-                                      gl.data_ptr(), fptr(gg), rows, a.rep, a.K, GDN_K, a.L, (float)scale, (float)lam_mul, on.stream),
+        check(lib.llattn_gdn_grad_out(normed ? nullptr : q.data_ptr(), k.data_ptr(), dq, dk, db, dl, a.rep > 1 ? fptr(dgp) : nullptr, gq.data_ptr(),
+                                      gk.data_ptr(), gb.data_ptr(), gl.data_ptr(), fptr(gg), rows, a.rep, a.K, GDN_K, a.L, (float)scale, (float)lam_mul, on.stream),
               "llattn_gdn_grad_out");
         return {gq, gk, dv, gb, gg, gl, Tensor(), Tensor(), Tensor(), Tensor()};
     }

@@ -53,6 +53,10 @@ struct GdnParams {
     float* d_wd;                 // (B,T,H,K)
     float* d_kd;                 // (B,T,H,K)
     float* d_gl;                 // (B,NT,H)  gradient w.r.t. the chunk's total log decay, scan part
+    // with raw_q not null the gradients of the rows before their l2 normalisation leave in the place of dq, dk (K = 128)
+    const __nv_bfloat16 *raw_q, *raw_k;      // (B,T,H,K)
+    __nv_bfloat16 *gq, *gk;                  // (B,T,H,K)
+    float q_scale;                           // q = normalised raw_q times this
     float* dq;                   // (B,T,H,K) fp32 results
     float* dk;
     float* dv;                   // (B,T,H,V)
