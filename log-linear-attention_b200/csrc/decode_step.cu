@@ -16,7 +16,7 @@
 // Measured on a B200, eight live levels of L = 15 (the bytes are those levels read and written once):
 //   Mamba-2, K = 128, V = 64: B = 1, H = 48 7.5 us; B = 4, H = 32 13.7 us; B = 64, H = 32 188 us = 5.7 TB/s (the level-innermost
 //   kernel behind the layer's torch operators: 110 us and 1200 us for a call at B = 1 and B = 64)
-//   delta rule, K = V = 128: B = 1, H = 16 6.2 us; B = 16, H = 16 54.6 us = 4.9 TB/s (414 us for a call before)
+//   delta rule, K = V = 128: B = 1, H = 16 6.2 us; B = 16, H = 16 48.4 us = 5.5 TB/s (414 us for a call before)
 #include "llattn_common.cuh"
 #include "../../include/llattn.h"
 
@@ -236,13 +236,13 @@ struct GdnStepArgs {
     float lam_mul;          // lambda is rounded to bf16 after this factor; 0: taken as it is
 };
 
-// A CTA owns 16 value columns of one (batch, head).  The slice of NG levels is in registers between the two passes over it:
+// A CTA owns COLS value columns of one (batch, head).  The slice of NG levels is in registers between the two passes over it:
 // k^T S_l of every level first (warp shuffles, then one exchange through shared memory for all of them), then the update, the
 // store and the output; more live levels take another round.
-template <int THREADS, int RPT, int NG, int CTAS>
+template <int THREADS, int RPT, int NG, int CTAS, int COLS = 16>
 __global__ void __launch_bounds__(THREADS, CTAS) gdn_layer_step_kernel(const __grid_constant__ GdnStepArgs a) {
     chain_wait();
-    constexpr int COLS = 16, C4 = 4, R = THREADS / C4, NW = THREADS / 32;
+    constexpr int C4 = COLS / 4, R = THREADS / C4, NW = THREADS / 32;
     __shared__ float sQ[256], sK[256];
     __shared__ float sLam[ST_MAXL];
     __shared__ float4 sRed[NW][NG + 1][C4];
@@ -486,10 +486,12 @@ int llattn_gdn_layer_step(float* states, const void* q, const void* k, const voi
                           H, G, K, V, L, live, carry_level, l2norm, scale, lambda_mul};
     const unsigned grid = (unsigned)(B * H * (V / 16));
     cudaStream_t st = (cudaStream_t)stream;
-    // K = 128: with two CTAs for every SM and more, CTAs of half the size (four of them on an SM) overlap one's reduction with
-    // another's loads better: 13.2 against 15.2 us at B = 4, 54.6 against 60.3 us at B = 16 (H = 16, V = 128, eight live levels);
-    // below, the larger ones have fewer rows per thread: 6.2 against 8.3 us at B = 1
+    // K = 128: with two CTAs for every SM and more, each thread takes four rows, so that more CTAs share an SM and one's reduction overlaps
+    // another's loads: 13.2 against 15.2 us at B = 4, 54.6 against 60.3 us at B = 16 (H = 16, V = 128, eight live levels); below, two rows
+    // each: 6.2 against 8.3 us at B = 1.  Where V allows, the CTA is 32 columns wide (whole 128-byte lines) and takes three levels a round:
+    // 48.4 against 51.1 us at B = 16, 91.1 against 95.9 at B = 32, 20.8 against 23.5 at B = 8 (four levels a round 51.7, two 51.6)
     if (K <= 64) llattn::launch_chained(llattn::gdn_layer_step_kernel<256, 1, 8, 2>, grid, 256, 0, st, a);
+    else if (K <= 128 && grid >= 296 && V % 32 == 0) llattn::launch_chained(llattn::gdn_layer_step_kernel<256, 4, 3, 2, 32>, grid / 2, 256, 0, st, a);
     else if (K <= 128 && grid >= 296) llattn::launch_chained(llattn::gdn_layer_step_kernel<128, 4, 4, 4>, grid, 128, 0, st, a);
     else if (K <= 128) llattn::launch_chained(llattn::gdn_layer_step_kernel<256, 2, 4, 2>, grid, 256, 0, st, a);
     else llattn::launch_chained(llattn::gdn_layer_step_kernel<512, 2, 4, 1>, grid, 512, 0, st, a);

@@ -67,7 +67,7 @@ def _pair_of_states(hstruct, B, H, K, V, L, position):
 
 # few heads / many heads, one live level, all of them, levels that merge far up
 @pytest.mark.parametrize("B,H,G,K,V,L,position", [(1, 2, 1, 128, 64, 15, 1), (1, 6, 2, 64, 64, 13, 4090), (5, 64, 1, 128, 64, 20, 21845),
-                                                  (1, 2, 1, 96, 16, 9, 128), (2, 3, 3, 256, 128, 12, 1000)])
+                                                  (1, 2, 1, 96, 16, 9, 128), (2, 3, 3, 256, 128, 12, 1000), (20, 15, 1, 128, 16, 13, 2047)])
 @pytest.mark.parametrize("struct", ["MAMBA2", "GDELTA"])
 def test_level_major_steps(B, H, G, K, V, L, position, struct):
     from hattention_b200.base import HStruct, HType
