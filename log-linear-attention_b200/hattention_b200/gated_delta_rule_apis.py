@@ -12,6 +12,20 @@ from .kernel import gdn_native, hattention_kernel, hattention_step, prefill
 SCALE_LAMBDA = True
 
 
+def _decode(q, k, v, g, l, beta, scale, s):
+    """One token through the native call, or None for what it does not take."""
+    if q.dtype != torch.bfloat16 or s.base != 2 or s.htype != HType.WEAK or s.hstruct != HStruct.GDELTA:
+        return None
+    T, heads, K = q.shape[1:] if q.dim() == 4 else (0, 0, 0)
+    if T != 1:
+        return None
+    if T < heads:
+        warnings.warn(f"seq_len ({T}) < num_heads ({heads}): inputs may be in head-first format", stacklevel=2)
+    if scale is None:
+        scale = K ** -0.5
+    return _lib.host().gdn_step(s.states, s.counts, q, k, v, beta, g, l, scale, 1.0 / scale if SCALE_LAMBDA else 0.0)
+
+
 @torch.compiler.disable
 def chunk_h_gated_delta_rule(
     q: torch.Tensor,
@@ -32,6 +46,13 @@ def chunk_h_gated_delta_rule(
     in the kernel is mandatory, scale defaults to K^-1/2 and lambda is divided by it; training call without
     states, prompt call with `output_final_state=True` (-> `hattention_prefill`), and one-token call with an
     `initial_state` (-> `hattention_step`)."""
+    if initial_state is not None and output_final_state is not False and cu_seqlens is None and use_qk_l2norm_in_kernel is True \
+            and not head_first:
+        # a decode step: the native call takes only bf16 operands of a one-token call, which makes the checks below (5 of 14 us of a
+        # step at small batches) its own; it declines before anything is written
+        o = _decode(q, k, v, g, l, beta, scale, initial_state)
+        if o is not None:
+            return o, initial_state
     assert q.dtype == k.dtype == v.dtype
     assert q.dtype != torch.float32, "ChunkGatedDeltaRuleFunction does not support float32. Please use bfloat16."
     assert len(beta.shape) == 3, "beta must be of shape [B, T, H] if head_first=False, or [B, H, T] otherwise."
@@ -54,10 +75,6 @@ def chunk_h_gated_delta_rule(
                 and q.shape[1] == k.shape[1] == v.shape[1] == beta.shape[1] == g.shape[1] == l.shape[1] == 1):
             raise ValueError
         s = initial_state
-        if s.base == 2 and s.htype == HType.WEAK and s.hstruct == HStruct.GDELTA:
-            o = _lib.host().gdn_step(s.states, s.counts, q, k, v, beta, g, l, scale, lambda_mul)
-            if o is not None:
-                return o, s
         q, k, v, beta, g, l = (x.squeeze(1) for x in (q, k, v, beta, g, l))
         if SCALE_LAMBDA:
             l = l / scale
