@@ -222,25 +222,63 @@ __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_const
 // independent of the others: level 0 is the last token alone, level j + 1 (for each set bit j of the last token's position in
 // the chunk) starts from zero at the first of its 2^j tokens, takes their writes and then the transitions of the tokens behind
 // them, and the levels of earlier chunks take the transitions of all.  fp32 throughout, as the decode kernel steps.
-// Level-major states of value heads that are processed as `rep` parts of Vs columns.  One warp holds four value columns of one level (lane: KR = Ko / 32 state rows), so a token is four dot products over the
-// lanes and no barrier; grid (B*H, levels, V / 32).
-constexpr int TAIL_KD = 128;
-__global__ void __launch_bounds__(256) gdn_tail_states_kernel(const bf16* __restrict__ kn, const bf16* __restrict__ v, const bf16* __restrict__ beta,
+// Level-major states of value heads that are processed as `rep` parts of Vs columns.
+//
+// A warp holds sixteen columns of one level: a lane has two of them and 32 of the 128 state rows (four lanes a column pair), as pairs of
+// rows, so that a token is 96 packed fp32 instructions and four shuffles, without a barrier.  What bounds it is that chain of at most 64
+// tokens and the fp32 rate: every live level takes every token of the chunk.  (Four columns a warp with the rows over all 32 lanes
+// was bound by the twenty shuffles of a token: T = 827, 59 tokens, 16 heads of 128 x 128 31 us, now 24; T = 777, 9 tokens, 12.1 and 8.6.)
+// Four warps a CTA; grid (B*H, 64-column blocks, levels).
+constexpr int TAIL_KD = 128, TAIL_COLS = 64;
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 x) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__global__ void __launch_bounds__(128) gdn_tail_states_kernel(const bf16* __restrict__ kn, const bf16* __restrict__ v, const bf16* __restrict__ beta,
                                                               const float* __restrict__ g, float* __restrict__ states, int T, int Tp, int H,
-                                                              int K, int Vs, int rep, int L) {
+                                                              int K, int Vs, int rep, int L, unsigned live) {
     chain_wait();
-    constexpr int KR = TAIL_KD / 32;
     __shared__ __align__(16) bf16 sK[CH * TAIL_KD];
-    __shared__ float sV[CH][33];
+    __shared__ __align__(16) float sV[CH * TAIL_COLS];
     __shared__ float sB[CH], sD[CH];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int lev = blockIdx.y;
+    // the live levels first, from the highest down (the lower ones see fewer tokens), then the dead ones, which are cleared: in the
+    // order of the levels some SMs got three of the long CTAs and others none
+    int lev = -1;
+    {
+        const unsigned nl = __popc(live), all = L < 32 ? (1u << L) - 1u : ~0u;
+        unsigned left = blockIdx.z < nl ? live : all & ~live;
+        const unsigned skip = blockIdx.z < nl ? blockIdx.z : blockIdx.z - nl;
+        for (unsigned i = 0; i <= skip; ++i) {
+            lev = 31 - __clz(left);
+            left &= ~(1u << lev);
+        }
+    }
     const int h = blockIdx.x % H, b = blockIdx.x / H;
     const int m = T - 1, c0 = m & ~(CH - 1), n = m - c0 + 1;
-    const int col = blockIdx.z * 32 + warp * 4;              // first of this warp's columns in the slice of Vs columns
+    const int cols = min(TAIL_COLS, Vs - (int)blockIdx.y * TAIL_COLS);
+    const int cl = warp * 16 + (lane >> 2) * 2, r = lane & 3;        // the lane's columns in the block; its rows: 8-row groups 4 j + r
     const int V = Vs * rep;                                  // H counts parts of value heads, rep of them in one
     const long bh = (long)b * H + h;
-    float* S = states + (bh / rep * L + lev) * (long)K * V + bh % rep * Vs + col;
+    float* S = states + (bh / rep * L + lev) * (long)K * V + bh % rep * Vs + blockIdx.y * TAIL_COLS + cl;
     // tokens [s0, s1) of the chunk write to this level; [s1, n) only advance it
     int s0 = -1, s1 = 0;
     if (lev == 0) {
@@ -254,59 +292,83 @@ __global__ void __launch_bounds__(256) gdn_tail_states_kernel(const bf16* __rest
     } else if (lev - INTRA_LEVELS < 25 && ((m >> (lev - 1)) & 1)) {
         s0 = s1 = 0;
     }
-    float4 s[KR];
+    const bool mine = cl < cols;
+    f32x2 s[2][16];                                          // [column][pair of rows]
 #pragma unroll
-    for (int i = 0; i < KR; ++i) {
-        const int row = lane * KR + i;
-        s[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (s0 >= 0 && lev >= INTRA_LEVELS && row < K) s[i] = *reinterpret_cast<const float4*>(S + (long)row * V);
+    for (int i = 0; i < 16; ++i) {
+        const int row = ((i >> 2) * 4 + r) * 8 + (i & 3) * 2;
+        float2 x[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        if (mine && s0 >= 0 && lev >= INTRA_LEVELS)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (row + e < K) x[e] = *reinterpret_cast<const float2*>(S + (long)(row + e) * V);
+        s[0][i] = pack2(x[0].x, x[1].x);
+        s[1][i] = pack2(x[0].y, x[1].y);
     }
     if (s0 >= 0) {
         const long t0 = (long)b * Tp + c0;
-        for (int e = tid; e < n * (TAIL_KD / 8); e += 256) {
+        for (int e = tid; e < n * (TAIL_KD / 8); e += 128) {
             const int i = e / (TAIL_KD / 8), c8 = (e % (TAIL_KD / 8)) * 8;
             *reinterpret_cast<uint4*>(sK + i * TAIL_KD + c8) = *reinterpret_cast<const uint4*>(kn + ((t0 + i) * H + h) * TAIL_KD + c8);
         }
-        for (int e = tid; e < n * 32; e += 256)
-            sV[e >> 5][e & 31] = __bfloat162float(v[((t0 + (e >> 5)) * H + h) * Vs + blockIdx.z * 32 + (e & 31)]);
-        for (int i = tid; i < n; i += 256) {
+        for (int e = tid; e < n * (TAIL_COLS / 2); e += 128) {
+            const int i = e / (TAIL_COLS / 2), c = (e % (TAIL_COLS / 2)) * 2;
+            float2 x = make_float2(0.f, 0.f);
+            if (c < cols)
+                x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(v + ((t0 + i) * H + h) * Vs + blockIdx.y * TAIL_COLS + c));
+            *reinterpret_cast<float2*>(sV + i * TAIL_COLS + c) = x;
+        }
+        for (int i = tid; i < n; i += 128) {
             sB[i] = __bfloat162float(beta[(t0 + i) * H + h]);
             sD[i] = fexp(g[(t0 + i) * H + h]);
         }
         __syncthreads();
         for (int t = s0; t < n; ++t) {
-            const uint2 raw = *reinterpret_cast<const uint2*>(sK + t * TAIL_KD + lane * KR);
-            const __nv_bfloat162 k01 = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), k23 = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-            const float kr[KR] = {__bfloat162float(k01.x), __bfloat162float(k01.y), __bfloat162float(k23.x), __bfloat162float(k23.y)};
-            float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+            f32x2 k[16];
 #pragma unroll
-            for (int i = 0; i < KR; ++i) {
-                d.x += kr[i] * s[i].x; d.y += kr[i] * s[i].y; d.z += kr[i] * s[i].z; d.w += kr[i] * s[i].w;
+            for (int j = 0; j < 4; ++j) {
+                const uint4 raw = *reinterpret_cast<const uint4*>(sK + t * TAIL_KD + (j * 4 + r) * 8);
+                const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) k[j * 4 + u] = pack2(__uint_as_float(w[u] << 16), __uint_as_float(w[u] & 0xffff0000u));
+            }
+            float d[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                f32x2 a0 = mul2(k[0], s[c][0]), a1 = mul2(k[1], s[c][1]);
+#pragma unroll
+                for (int i = 2; i < 16; i += 2) {
+                    a0 = fma2(k[i], s[c][i], a0);
+                    a1 = fma2(k[i + 1], s[c][i + 1], a1);
+                }
+                const float2 x = unpack2(a0), y = unpack2(a1);
+                d[c] = (x.x + x.y) + (y.x + y.y);
             }
 #pragma unroll
-            for (int w = 16; w > 0; w >>= 1) {
-                d.x += __shfl_xor_sync(0xffffffffu, d.x, w);
-                d.y += __shfl_xor_sync(0xffffffffu, d.y, w);
-                d.z += __shfl_xor_sync(0xffffffffu, d.z, w);
-                d.w += __shfl_xor_sync(0xffffffffu, d.w, w);
+            for (int w = 1; w < 4; w <<= 1) {
+                d[0] += __shfl_xor_sync(0xffffffffu, d[0], w);
+                d[1] += __shfl_xor_sync(0xffffffffu, d[1], w);
             }
             const float dec = sD[t], be = sB[t];
-            float4 w4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (t < s1) w4 = make_float4(sV[t][warp * 4], sV[t][warp * 4 + 1], sV[t][warp * 4 + 2], sV[t][warp * 4 + 3]);
+            float2 w2 = make_float2(0.f, 0.f);
+            if (t < s1) w2 = *reinterpret_cast<const float2*>(sV + t * TAIL_COLS + cl);
+            // s' = dec (s - beta k d) + beta k w
+            const float x0 = be * (w2.x - dec * d[0]), x1 = be * (w2.y - dec * d[1]);
+            const f32x2 dec2 = pack2(dec, dec), x02 = pack2(x0, x0), x12 = pack2(x1, x1);
 #pragma unroll
-            for (int i = 0; i < KR; ++i) {
-                const float bk = be * kr[i];
-                s[i].x = dec * (s[i].x - bk * d.x) + bk * w4.x;
-                s[i].y = dec * (s[i].y - bk * d.y) + bk * w4.y;
-                s[i].z = dec * (s[i].z - bk * d.z) + bk * w4.z;
-                s[i].w = dec * (s[i].w - bk * d.w) + bk * w4.w;
+            for (int i = 0; i < 16; ++i) {
+                s[0][i] = fma2(dec2, s[0][i], mul2(k[i], x02));
+                s[1][i] = fma2(dec2, s[1][i], mul2(k[i], x12));
             }
         }
     }
+    if (!mine) return;
 #pragma unroll
-    for (int i = 0; i < KR; ++i) {
-        const int row = lane * KR + i;
-        if (row < K) *reinterpret_cast<float4*>(S + (long)row * V) = s[i];
+    for (int i = 0; i < 16; ++i) {
+        const int row = ((i >> 2) * 4 + r) * 8 + (i & 3) * 2;
+        const float2 x = unpack2(s[0][i]), y = unpack2(s[1][i]);
+        if (row < K) *reinterpret_cast<float2*>(S + (long)row * V) = make_float2(x.x, y.x);
+        if (row + 1 < K) *reinterpret_cast<float2*>(S + (long)(row + 1) * V) = make_float2(x.y, y.y);
     }
 }
 
@@ -400,9 +462,9 @@ int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, co
     if (T > 1 && L < 1 + (32 - __builtin_clz((unsigned)(T - 1) | 1u))) return LLATTN_ERR_TOO_FEW_LEVELS;
     if (!kn || !v || !beta || !g || !states) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
-    dim3 grid(B * H, L, V / 32);
-    llattn::launch_chained(llattn::gdn_tail_states_kernel, grid, 256, 0, (cudaStream_t)stream, (const bf*)kn, (const bf*)v, (const bf*)beta, g,
-            states, T, Tp, H, K, V, rep, L);
+    dim3 grid(B * H, (V + llattn::TAIL_COLS - 1) / llattn::TAIL_COLS, L);
+    llattn::launch_chained(llattn::gdn_tail_states_kernel, grid, 128, 0, (cudaStream_t)stream, (const bf*)kn, (const bf*)v, (const bf*)beta, g,
+            states, T, Tp, H, K, V, rep, L, 1u | (unsigned)(T - 1) << 1);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
