@@ -52,6 +52,9 @@ int llattn_workspace_status(const void* workspace, int* status_host, void* strea
 /* Chunk length the kernels are built for (64, as hattention/kernel.py:355-356 fixes it). */
 int llattn_chunk(void);
 
+/* Zero bytes on the stream (accumulators of the calls below). */
+int llattn_clear(void* dst, size_t bytes, void* stream);
+
 /* Log-linear Mamba-2 forward.  Replaces hattention.chunkwise.chunkwise_fwd
  * (hattention/chunkwise.py:1118-1275) with output_final_state=False: writes o and the in-chunk
  * inclusive cumulative sum of g (the reference returns both). */

@@ -115,6 +115,10 @@ int llattn_workspace_status(const void* workspace, int* status_host, void* strea
     if (e != cudaSuccess) return (int)e;
     return (int)cudaStreamSynchronize((cudaStream_t)stream);
 }
+int llattn_clear(void* dst, size_t bytes, void* stream) {
+    if (!dst) return LLATTN_ERR_NULL;
+    return (int)cudaMemsetAsync(dst, 0, bytes, (cudaStream_t)stream);
+}
 int llattn_chunk(void) { return 64; }
 
 size_t llattn_mamba2_fwd_workspace_bytes(int B, int T, int H, int G, int K, int V, int L) {

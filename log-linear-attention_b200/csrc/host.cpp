@@ -13,6 +13,7 @@
 #include <dlfcn.h>
 #include <torch/extension.h>
 
+#include <ATen/cuda/EmptyTensor.h>
 #include "../../include/llattn.h"
 
 namespace {
@@ -29,7 +30,7 @@ using torch::autograd::variable_list;
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
     F(llattn_gdn_fwd_workspace_bytes) F(llattn_gdn_fwd_keep_workspace_bytes) F(llattn_gdn_fwd) F(llattn_gdn_fwd_keep)                \
     F(llattn_gdn_prefill_parts) F(llattn_gdn_prompt_states) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
-    F(llattn_gdn_bwd_kept_workspace_bytes) F(llattn_gdn_bwd_kept_bf16dv) F(llattn_gdn_bwd_kept_normed) F(llattn_gdn_grad_out) F(llattn_workspace_status)
+    F(llattn_gdn_bwd_kept_workspace_bytes) F(llattn_gdn_bwd_kept_bf16dv) F(llattn_gdn_bwd_kept_normed) F(llattn_gdn_grad_out) F(llattn_workspace_status) F(llattn_clear)
 
 struct Library {
 #define LLATTN_MEMBER(name) decltype(&::name) name = nullptr;
@@ -65,7 +66,13 @@ inline Tensor contiguous(const Tensor& t) { return t.defined() ? t.contiguous() 
 using Maybe = std::optional<Tensor>;     // a tensor that may be absent: autograd functions take no undefined tensors
 inline Tensor of(const Maybe& t) { return t.has_value() ? *t : Tensor(); }
 inline Tensor empty(at::IntArrayRef size, at::ScalarType dt, const Tensor& like) {
-    return at::empty(size, at::TensorOptions().dtype(dt).device(like.device()));
+    return at::detail::empty_cuda(size, dt, like.device(), std::nullopt);        // behind the dispatcher: 1 us less a tensor
+}
+inline Tensor contiguous_like(const Tensor& t) { return empty(t.sizes(), t.scalar_type(), t); }
+inline Tensor zeros(int64_t n, const Tensor& like, void* stream) {
+    const Tensor t = empty({n}, at::kFloat, like);
+    check(lib.llattn_clear(t.data_ptr(), n * sizeof(float), stream), "llattn_clear");
+    return t;
 }
 inline bool wants_grad(std::initializer_list<Tensor> ts) {
     if (!at::GradMode::is_enabled()) return false;
@@ -118,8 +125,8 @@ struct Scan {
 Scan mamba2_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, void* stream, bool status) {
     const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
     Scan s;
-    s.o = at::empty_like(v);
-    s.g_cum = at::empty_like(g);
+    s.o = contiguous_like(v);
+    s.g_cum = contiguous_like(g);
     const size_t n = lib.llattn_mamba2_fwd_workspace_bytes(B, T, H, G, K, V, L);
     s.ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
     check(lib.llattn_mamba2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), l.data_ptr(), s.o.data_ptr(), fptr(s.g_cum), s.ws.data_ptr(),
@@ -134,7 +141,7 @@ Scan mamba2_fwd_residual(const Tensor& q, const Tensor& k, const Tensor& v, cons
     const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3), Ty = x.size(1);
     Scan s;
     s.o = empty(x.sizes(), f32(D) ? at::kFloat : at::kBFloat16, x);
-    s.g_cum = at::empty_like(g);
+    s.g_cum = contiguous_like(g);
     const size_t n = lib.llattn_mamba2_fwd_workspace_bytes(B, T, H, G, K, V, L);
     s.ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
     const int rc = lib.llattn_mamba2_fwd_residual(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), l.data_ptr(), x.data_ptr(), D.data_ptr(),
@@ -161,8 +168,8 @@ ScanGrads mamba2_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     const Tensor qk = empty({2, B, T, G, K}, at::kBFloat16, q);      // side by side: one conversion pass writes both
     r.dq = qk.select(0, 0);
     r.dk = qk.select(0, 1);
-    r.dv = at::empty_like(v);
-    r.dg = at::empty_like(g_cum);
+    r.dv = contiguous_like(v);
+    r.dg = contiguous_like(g_cum);
     r.dl = empty(l.sizes(), at::kFloat, l);
     const size_t n = lib.llattn_mamba2_bwd_workspace_bytes(B, T, H, G, K, V, L);
     const Tensor ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
@@ -220,7 +227,7 @@ struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
         const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), L = dl.size(3);
         const Tensor x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), A_ = A.to(at::kFloat).contiguous(), Lp_ = Lp.contiguous(),
                      D_ = contiguous(of(D)), b_ = contiguous(of(bias)), q = Cm.contiguous(), k = Bm.contiguous();
-        const Tensor v = at::empty_like(x_), g = empty({B, T, H}, at::kFloat, x), lam = at::empty_like(dl_);
+        const Tensor v = contiguous_like(x_), g = empty({B, T, H}, at::kFloat, x), lam = contiguous_like(dl_);
         check(lib.llattn_mamba2_layer_prep_fwd(x_.data_ptr(), dt_.data_ptr(), ptr(b_), f32(b_), fptr(A_), dl_.data_ptr(), Lp_.data_ptr(), f32(Lp_),
                                                v.data_ptr(), fptr(g), lam.data_ptr(), (long)B * T * H, H, P, L, (int)mode, on.stream),
               "llattn_mamba2_layer_prep_fwd");
@@ -242,8 +249,8 @@ struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
         const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), L = dl.size(3);
         const Tensor dy = d[0].to(at::kBFloat16).contiguous();
         ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool(), true);
-        const Tensor dx = at::empty_like(x), ddt = at::empty_like(dt), ddl = at::empty_like(dl);
-        const Tensor acc = at::zeros({3 * H + H * L}, at::TensorOptions().dtype(at::kFloat).device(x.device()));
+        const Tensor dx = contiguous_like(x), ddt = contiguous_like(dt), ddl = contiguous_like(dl);
+        const Tensor acc = zeros(3 * H + (int64_t)H * L, x, on.stream);
         float* a = fptr(acc);
         check(lib.llattn_mamba2_layer_prep_bwd(x.data_ptr(), dt.data_ptr(), ptr(bias), f32(bias), fptr(A), dl.data_ptr(), Lp.data_ptr(), f32(Lp), ptr(D),
                                                f32(D), r.dv.data_ptr(), fptr(r.dg), fptr(r.dl), dy.data_ptr(), dx.data_ptr(), ddt.data_ptr(), ddl.data_ptr(),
@@ -306,7 +313,7 @@ py::object mamba2_prompt(const Tensor& x, const Tensor& dt, const Tensor& A, con
         const Tensor v = empty({B, Tp, H, P}, at::kBFloat16, x), g = empty({B, Tp, H}, at::kFloat, x), lam = empty({B, Tp, H, Lo}, at::kBFloat16, x);
         if (Tp != T) {
             qp = empty({B, Tp, G, N}, at::kBFloat16, x);
-            kp = at::empty_like(qp);
+            kp = contiguous_like(qp);
         }
         check(lib.llattn_mamba2_prompt_prep(x_.data_ptr(), dt_.data_ptr(), ptr(b_), f32(b_), fptr(A_), dl_.data_ptr(), Lp_.data_ptr(), f32(Lp_),
                                             q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), ptr(qp), ptr(kp), B, T, Tp, H, G, N, P, L,
@@ -362,10 +369,10 @@ struct Mixer : torch::autograd::Function<Mixer> {
         On on(z);
         const int B = z.size(0), T = z.size(1), W = z.size(2), H = Lp.size(0), L = Lp.size(1), dim = H * 64, G = k.size(2), N = k.size(3);
         const Tensor dn = d[0].to(at::kBFloat16).contiguous();
-        const Tensor dzx = at::empty_like(z), dy = empty(x.sizes(), at::kBFloat16, x);
+        const Tensor dzx = contiguous_like(z), dy = empty(x.sizes(), at::kBFloat16, x);
         // sums over tokens: conv taps and bias, norm weight, A, dt_bias, D, L
         const int64_t ch = dim + 2 * G * N, at_b = ch * 4, at_n = ch * 5, at_A = at_n + dim, at_dt = at_A + H, at_D = at_dt + H, at_L = at_D + H;
-        const Tensor acc = at::zeros({at_L + (int64_t)H * L}, at::TensorOptions().dtype(at::kFloat).device(z.device()));
+        const Tensor acc = zeros(at_L + (int64_t)H * L, z, on.stream);
         float* a = fptr(acc);
         check(lib.llattn_mixer_norm_bwd(o.data_ptr(), x.data_ptr(), ptr(D), f32(D), z.data_ptr(), W, nw.data_ptr(), f32(nw), dn.data_ptr(), fptr(rstd),
                                         dy.data_ptr(), dzx.data_ptr(), a + at_n, a + at_D, (long)B * T, H, on.stream),
@@ -475,9 +482,9 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
         const int B = a.B, H = a.heads(), V = a.width;
         const size_t keep_need = lib.llattn_gdn_fwd_keep_workspace_bytes(B, T, H, GDN_K, V, a.L);
         const bool keep = ctx != nullptr && (int64_t)keep_need <= keep_bytes;
-        const Tensor g_cum = at::empty_like(a.g), A = empty({2, B, T, H, 64}, at::kBFloat16, q), Aw = A.select(0, 0), Au = A.select(0, 1);
+        const Tensor g_cum = contiguous_like(a.g), A = empty({2, B, T, H, 64}, at::kBFloat16, q), Aw = A.select(0, 0), Au = A.select(0, 1);
         const size_t bytes = keep ? keep_need : lib.llattn_gdn_fwd_workspace_bytes(B, T, H, GDN_K, V, a.L);
-        const Tensor ws = empty({(int64_t)bytes}, at::kByte, q), o = at::empty_like(v_);
+        const Tensor ws = empty({(int64_t)bytes}, at::kByte, q), o = contiguous_like(v_);
         check((keep ? lib.llattn_gdn_fwd_keep : lib.llattn_gdn_fwd)(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(),
                                                                    o.data_ptr(), fptr(g_cum), Aw.data_ptr(), Au.data_ptr(), ws.data_ptr(), bytes, B, T, H,
                                                                    GDN_K, V, a.L, on.stream),
@@ -599,7 +606,7 @@ py::object gdn_prompt(const Tensor& q, const Tensor& k, const Tensor& v, const T
                                   on.stream);
         const int B = a.B, H = a.heads(), K = a.K, V = a.width;
         states = empty({B, a.H, L, K, a.V}, at::kFloat, q);
-        const Tensor g_cum = at::empty_like(a.g), A = empty({2, B, Tp, H, 64}, at::kBFloat16, q), out = empty({B, Tp, a.H, a.V}, at::kBFloat16, q);
+        const Tensor g_cum = contiguous_like(a.g), A = empty({2, B, Tp, H, 64}, at::kBFloat16, q), out = empty({B, Tp, a.H, a.V}, at::kBFloat16, q);
         const size_t bytes = lib.llattn_gdn_fwd_workspace_bytes(B, Tp, H, GDN_K, V, Lo);
         const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
         check(lib.llattn_gdn_prefill_parts(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(), out.data_ptr(),
