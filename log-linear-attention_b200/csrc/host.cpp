@@ -342,8 +342,7 @@ struct Mixer : torch::autograd::Function<Mixer> {
         const int B = zx.size(0), T = zx.size(1), W = zx.size(2), H = Lp.size(0), L = Lp.size(1), dim = H * 64, N = (W - 2 * dim - H - H * L) / (2 * G);
         const Tensor z = zx.contiguous(), cw_ = cw.contiguous(), cb_ = contiguous(of(cb)), b_ = contiguous(bias), A_ = A.to(at::kFloat).contiguous(),
                      Lp_ = Lp.contiguous(), D_ = contiguous(D), nw_ = nw.contiguous();
-        const Tensor xv = empty({2, B, T, H, 64}, at::kBFloat16, zx), x = xv.select(0, 0), v = xv.select(0, 1);
-        const Tensor kq = empty({2, B, T, G, N}, at::kBFloat16, zx), k = kq.select(0, 0), q = kq.select(0, 1);
+        const Tensor x = empty({B, T, H, 64}, at::kBFloat16, zx), v = contiguous_like(x), k = empty({B, T, G, N}, at::kBFloat16, zx), q = contiguous_like(k);
         const Tensor g = empty({B, T, H}, at::kFloat, zx), lam = empty({B, T, H, L}, at::kBFloat16, zx);
         check(lib.llattn_mixer_prep_fwd(z.data_ptr(), cw_.data_ptr(), f32(cw_), ptr(cb_), f32(cb_), ptr(b_), f32(b_), fptr(A_), Lp_.data_ptr(), f32(Lp_),
                                         x.data_ptr(), v.data_ptr(), k.data_ptr(), q.data_ptr(), fptr(g), lam.data_ptr(), B, T, H, (int)G, N, L, (int)mode,
@@ -447,9 +446,8 @@ GdnInputs gdn_prepare(const Tensor& q, const Tensor& k, const Tensor& v, const T
     a.split();
     const int B = a.B, H = a.heads(), L = l.size(3);
     const bool pad = Tp != T, own = pad || a.rep > 1, own_l = own || lam_mul != 0.0 || Lo != L;
-    const Tensor qk = empty({2, B, Tp, H, GDN_K}, at::kBFloat16, q);
-    a.qn = qk.select(0, 0);
-    a.kn = qk.select(0, 1);
+    a.qn = empty({B, Tp, H, GDN_K}, at::kBFloat16, q);
+    a.kn = contiguous_like(a.qn);
     a.v = pad ? empty({B, Tp, H, a.width}, at::kBFloat16, q) : v;
     a.b = own ? empty({B, Tp, H}, at::kBFloat16, q) : b;
     a.g = own ? empty({B, Tp, H}, at::kFloat, q) : g;
@@ -482,7 +480,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
         const int B = a.B, H = a.heads(), V = a.width;
         const size_t keep_need = lib.llattn_gdn_fwd_keep_workspace_bytes(B, T, H, GDN_K, V, a.L);
         const bool keep = ctx != nullptr && (int64_t)keep_need <= keep_bytes;
-        const Tensor g_cum = contiguous_like(a.g), A = empty({2, B, T, H, 64}, at::kBFloat16, q), Aw = A.select(0, 0), Au = A.select(0, 1);
+        const Tensor g_cum = contiguous_like(a.g), Aw = empty({B, T, H, 64}, at::kBFloat16, q), Au = contiguous_like(Aw);
         const size_t bytes = keep ? keep_need : lib.llattn_gdn_fwd_workspace_bytes(B, T, H, GDN_K, V, a.L);
         const Tensor ws = empty({(int64_t)bytes}, at::kByte, q), o = contiguous_like(v_);
         check((keep ? lib.llattn_gdn_fwd_keep : lib.llattn_gdn_fwd)(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(),
@@ -520,9 +518,8 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
             qn = s[8];
             kn = s[9];
         } else {
-            const Tensor qk = empty({2, B, T, H, GDN_K}, at::kBFloat16, q);
-            qn = qk.select(0, 0);
-            kn = qk.select(0, 1);
+            qn = empty({B, T, H, GDN_K}, at::kBFloat16, q);
+            kn = contiguous_like(qn);
             check(lib.llattn_gdn_prompt_prep(q.data_ptr(), k.data_ptr(), nullptr, nullptr, nullptr, nullptr, qn.data_ptr(), kn.data_ptr(), nullptr, nullptr,
                                              nullptr, nullptr, B, T, T, a.H, a.H, a.K, GDN_K, a.V, a.rep, a.L, a.L, (float)scale, 0.f, on.stream),
                   "llattn_gdn_prompt_prep");
@@ -530,7 +527,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
         const Tensor d_o = d[0].to(at::kBFloat16).contiguous();
         // fp32 gradients of what the parts of a head share; dg is handed on as it is where a head has one part
         const int64_t rows = (int64_t)B * T * a.H, prows = rows * a.rep;
-        const Tensor gqk = empty({2, B, T, a.H, a.K}, at::kBFloat16, q), gq = gqk.select(0, 0), gk = gqk.select(0, 1);
+        const Tensor gq = empty({B, T, a.H, a.K}, at::kBFloat16, q), gk = contiguous_like(gq);
         const Tensor dgp = empty({B, T, H}, at::kFloat, q), dlb = empty({prows * (a.L + 1)}, at::kFloat, q);
         float *dl = fptr(dlb), *db = dl + prows * a.L;
         const size_t bytes = (kept ? lib.llattn_gdn_bwd_kept_workspace_bytes : lib.llattn_gdn_bwd_workspace_bytes)(B, T, H, GDN_K, V, a.L);
@@ -606,11 +603,11 @@ py::object gdn_prompt(const Tensor& q, const Tensor& k, const Tensor& v, const T
                                   on.stream);
         const int B = a.B, H = a.heads(), K = a.K, V = a.width;
         states = empty({B, a.H, L, K, a.V}, at::kFloat, q);
-        const Tensor g_cum = contiguous_like(a.g), A = empty({2, B, Tp, H, 64}, at::kBFloat16, q), out = empty({B, Tp, a.H, a.V}, at::kBFloat16, q);
+        const Tensor g_cum = contiguous_like(a.g), Aw = empty({B, Tp, H, 64}, at::kBFloat16, q), Au = contiguous_like(Aw), out = empty({B, Tp, a.H, a.V}, at::kBFloat16, q);
         const size_t bytes = lib.llattn_gdn_fwd_workspace_bytes(B, Tp, H, GDN_K, V, Lo);
         const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
         check(lib.llattn_gdn_prefill_parts(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(), out.data_ptr(),
-                                           fptr(g_cum), A.select(0, 0).data_ptr(), A.select(0, 1).data_ptr(), fptr(states), K, a.rep, L, ws.data_ptr(), bytes,
+                                           fptr(g_cum), Aw.data_ptr(), Au.data_ptr(), fptr(states), K, a.rep, L, ws.data_ptr(), bytes,
                                            B, Tp, H, GDN_K, V, Lo, on.stream),
               "llattn_gdn_prefill_parts");
         check(lib.llattn_gdn_prompt_states(a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), fptr(states), B, T, Tp, H, K, V, a.rep, L, on.stream),
