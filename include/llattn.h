@@ -70,6 +70,12 @@ int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, cons
                                const void* x, const void* D, void* y, int y_is_f32, int T_y, float* g_cum, void* workspace, size_t workspace_bytes,
                                int B, int T, int H, int G, int K, int V, int L, void* stream);
 
+/* llattn_mamba2_fwd_residual and llattn_mamba2_prompt_states (of the first T_y tokens, state_levels levels) in one call, the states beside the
+ * output where both leave room.  Without D (NULL) y is o, (B,T,H,V) bf16. */
+int llattn_mamba2_fwd_prompt(const void* q, const void* k, const void* v, const float* g, const void* lambda,
+                             const void* x, const void* D, void* y, int y_is_f32, int T_y, float* states, int state_levels, float* g_cum,
+                             void* workspace, size_t workspace_bytes, int B, int T, int H, int G, int K, int V, int L, void* stream);
+
 /* Forward for callers that cannot hand the library a scratch buffer.  (No counterpart in the
  * reference: its drivers allocate with torch on every call.)
  *

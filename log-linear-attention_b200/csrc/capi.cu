@@ -165,6 +165,20 @@ int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, cons
     return mamba2_fwd_impl(p, q, k, v, g, lambda, nullptr, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);
 }
 
+int llattn_mamba2_fwd_prompt(const void* q, const void* k, const void* v, const float* g, const void* lambda,
+                             const void* x, const void* D, void* y, int y_is_f32, int T_y, float* states, int state_levels, float* g_cum,
+                             void* workspace, size_t workspace_bytes, int B, int T, int H, int G, int K, int V, int L, void* stream) {
+    if (!y || !states || (D && !x)) return LLATTN_ERR_NULL;
+    if (T_y <= 0 || T_y > T) return LLATTN_ERR_BAD_LENGTH;
+    if (D && (((uintptr_t)x & 15) || ((uintptr_t)y & 31))) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    const int rc = llattn::mamba2_prompt_states_check(B, T_y, H, G, K, V, state_levels);
+    if (rc != 0) return rc;
+    llattn::Mamba2Params p = {};
+    if (D) { p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_T = T_y; p.res_f32 = y_is_f32; }
+    p.pr_states = states; p.pr_T = T_y; p.pr_L = state_levels;
+    return mamba2_fwd_impl(p, q, k, v, g, lambda, D ? nullptr : y, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);
+}
+
 size_t llattn_static_scratch_bytes(void) { return LLATTN_STATIC_SCRATCH_BYTES; }
 
 int llattn_static_scratch_status(int* status_host, void* stream) {

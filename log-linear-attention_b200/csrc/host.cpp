@@ -24,7 +24,7 @@ using torch::autograd::Variable;
 using torch::autograd::variable_list;
 
 #define LLATTN_FUNCS(F)                                                                                                             \
-    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_fwd_residual) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
+    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_fwd_residual) F(llattn_mamba2_fwd_prompt) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
     F(llattn_mamba2_layer_prep_fwd) F(llattn_mamba2_layer_prep_bwd) F(llattn_mamba2_layer_step) F(llattn_gdn_layer_step)            \
     F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mixer_prep_fwd)            \
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
@@ -323,13 +323,25 @@ py::object mamba2_prompt(const Tensor& x, const Tensor& dt, const Tensor& A, con
             q = qp;
             k = kp;
         }
-        const Scan s = D_c.defined() ? mamba2_fwd_residual(q, k, v, g, lam, x_, D_c, on.stream, status) : mamba2_fwd(q, k, v, g, lam, on.stream, status);
         states = empty({B, H, L, N, P}, at::kFloat, x);
-        check(lib.llattn_mamba2_prompt_states(k.data_ptr(), v.data_ptr(), fptr(g), fptr(states), s.ws.data_ptr(), s.ws.numel(), B, T, Tp, H, G, N, P, L,
-                                              on.stream),
-              "llattn_mamba2_prompt_states");
+        const Tensor g_cum = contiguous_like(g);
+        const size_t n = std::max<size_t>(lib.llattn_mamba2_fwd_workspace_bytes(B, Tp, H, G, N, P, Lo), 256);
+        const Tensor ws = empty({(int64_t)n}, at::kByte, x);
+        y = D_c.defined() ? empty(x.sizes(), f32(D_c) ? at::kFloat : at::kBFloat16, x) : contiguous_like(v);
+        const int rc = lib.llattn_mamba2_fwd_prompt(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), x_.data_ptr(), ptr(D_c), y.data_ptr(),
+                                                    f32(y), T, fptr(states), L, fptr(g_cum), ws.data_ptr(), n, B, Tp, H, G, N, P, Lo, on.stream);
+        if (rc == LLATTN_ERR_UNSUPPORTED_SHAPE) {
+            const Scan s = D_c.defined() ? mamba2_fwd_residual(q, k, v, g, lam, x_, D_c, on.stream, status) : mamba2_fwd(q, k, v, g, lam, on.stream, status);
+            y = s.o;
+            check(lib.llattn_mamba2_prompt_states(k.data_ptr(), v.data_ptr(), fptr(g), fptr(states), s.ws.data_ptr(), s.ws.numel(), B, T, Tp, H, G, N, P, L,
+                                                  on.stream),
+                  "llattn_mamba2_prompt_states");
+        } else {
+            check(rc, "llattn_mamba2_fwd_prompt");
+            if (status) check_status(ws, on.stream, "llattn_mamba2_fwd_prompt");
+        }
         states = states.permute({0, 1, 3, 4, 2});
-        y = D_c.defined() ? s.o : s.o.narrow(1, 0, T).contiguous();
+        if (!D_c.defined()) y = y.narrow(1, 0, T).contiguous();
     }
     return py::make_tuple(y, states);
 }

@@ -58,6 +58,8 @@ struct Mamba2Params {
     const void* res_D;           // (H), fp32 like y if res_f32, else bf16
     void* res_y;                 // (B,res_T,H,V)
     int res_T, res_f32;          // res_T <= T: a prompt's tokens without its padding
+    float* pr_states;            // forward of a prompt: also the level states after its first pr_T tokens, (B,H,pr_L,K,V)
+    int pr_T, pr_L;
     int reuse_states;            // backward: seg_D / seg_H0 come from the forward call, do not recompute them
 };
 
@@ -78,6 +80,9 @@ int mamba2_seg_state_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_hi_out_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 extern std::atomic<int> g_use_tensor_core_path;   // test hook, see llattn_testing.h
 // segment summaries and decays inside the workspace of a forward call (null when it has one segment only)
+int mamba2_prompt_states_check(int B, int T, int H, int G, int K, int V, int L);
+int mamba2_prompt_states_launch(const __nv_bfloat16* k, const __nv_bfloat16* v, const float* g, float* states, const float* seg_F, const float* seg_D,
+                                int B, int T, int Tp, int H, int G, int K, int L, cudaStream_t stream);
 int mamba2_fwd_workspace_segments(const void* ws, size_t bytes, int B, int T, int H, int G, int K, int V, const float** F, const float** D);
 // clears acc_bytes (a multiple of 16) at acc and ndl floats at dl, and takes the in-chunk cumulative sum of g apart
 int mamba2_bwd_init(const float* gc, float* g, long BT, int H, void* acc, size_t acc_bytes, float* dl, long ndl, cudaStream_t stream);

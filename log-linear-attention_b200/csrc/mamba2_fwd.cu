@@ -18,6 +18,7 @@
 //     and the chunk kernel adds that partial output to its own before the single final store.
 #include "llattn_common.cuh"
 #include "llattn_mamba2.h"
+#include "side_stream.h"
 
 namespace llattn {
 
@@ -607,26 +608,48 @@ template <int KD, int VD, int MLOW>
 static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
     const bool use_tc = mamba2_uses_tc(p);
+    // A prompt's level states need its segment summaries only, the output three more kernels.  While the chunk kernel leaves SMs idle (it
+    // takes one CTA per segment and SM) they are made beside those: B = 1, T = 1000, 48 heads, 96 CTAs: 62 -> 57 us for the call;
+    // T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs.
+    // Within a segment there is too little to run beside for the events to pay.
+    SideStream* side = nullptr;
+    auto states = [&](cudaStream_t on) {
+        return mamba2_prompt_states_launch(p.k, p.v, p.g, p.pr_states, p.seg_F, p.seg_D, p.B, p.pr_T, p.T, p.H, p.G, p.K, p.pr_L, on);
+    };
+    auto output = [&]() -> int {
+        if (p.NS > 1) {
+            if (use_tc && p.LH <= 8) {
+                const int rc = mamba2_hi_out_tc_launch(p, stream);
+                if (rc != 0) return rc;
+            } else {
+                auto kern = m2_hi_out_kernel<KD, VD, MLOW>;
+                size_t sm = HiSmem<KD, VD>::total;
+                if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
+                llattn::launch_chained(kern, p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream, p); LLATTN_LAUNCHED();
+            }
+        }
+        if (use_tc) return mamba2_fwd_tc_launch(p, stream);
+        auto kern = m2_chunk_fwd_kernel<KD, VD, MLOW>;
+        size_t sm = FwdSmem<KD, VD, MLOW>::total;
+        if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
+        llattn::launch_chained(kern, p.B * p.H * p.NS, 256, sm, stream, p); LLATTN_LAUNCHED();
+        return (int)cudaGetLastError();
+    };
+    int rc;
     if (p.NS > 1) {
         p.o_has_high = use_tc ? 2 : 1;      // 2: partial output goes to the column-chunk-major scratch
-        int rc = launch_states<KD, VD, MLOW>(p, stream);
-        if (rc != 0) return rc;
-        if (use_tc && p.LH <= 8) {
-            rc = mamba2_hi_out_tc_launch(p, stream);
-            if (rc != 0) return rc;
-        } else {
-            auto kern = m2_hi_out_kernel<KD, VD, MLOW>;
-            size_t sm = HiSmem<KD, VD>::total;
-            if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-            llattn::launch_chained(kern, p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream, p); LLATTN_LAUNCHED();
-        }
+        if ((rc = launch_states<KD, VD, MLOW>(p, stream)) != 0) return rc;
+        if (p.pr_states && (long)p.B * p.H * p.NS * 4 < 148 * 3) side = SideStream::get(stream);
     }
-    if (use_tc) return mamba2_fwd_tc_launch(p, stream);
-    auto kern = m2_chunk_fwd_kernel<KD, VD, MLOW>;
-    size_t sm = FwdSmem<KD, VD, MLOW>::total;
-    if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-    llattn::launch_chained(kern, p.B * p.H * p.NS, 256, sm, stream, p); LLATTN_LAUNCHED();
-    return (int)cudaGetLastError();
+    if (side) {
+        if ((e = side->fork(stream)) != cudaSuccess) return (int)e;
+        const int rs = states(side->stream());
+        rc = output();
+        if ((e = side->join(stream)) != cudaSuccess) return (int)e;
+        return rc != 0 ? rc : rs;
+    }
+    if ((rc = output()) != 0 || !p.pr_states) return rc;
+    return states(stream);
 }
 
 int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream) {

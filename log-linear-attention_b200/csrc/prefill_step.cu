@@ -347,20 +347,35 @@ __global__ void __launch_bounds__(256) mamba2_step_kernel(float* __restrict__ st
     }
 }
 
-}  // namespace llattn
+int mamba2_prompt_states_launch(const bf16* k, const bf16* v, const float* g, float* states, const float* seg_F, const float* seg_D,
+                                int B, int T, int Tp, int H, int G, int K, int L, cudaStream_t stream) {
+    dim3 grid(B * H, L);
+    auto launch = [&](auto kern, size_t sm) -> cudaError_t {
+        const cudaError_t e = allow_smem(kern, sm);
+        if (e == cudaSuccess) launch_chained(kern, grid, 256, sm, stream, k, v, g, states, seg_F, seg_D, T, Tp, H, G, L);
+        return e;
+    };
+    const cudaError_t e = K == 128 ? launch(mamba2_prompt_state_kernel<128>, PromptStateSmem<128>::total)
+                                   : launch(mamba2_prompt_state_kernel<64>, PromptStateSmem<64>::total);
+    if (e != cudaSuccess) return (int)e;
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
 
-extern "C" {
-
-static int final_state_check(int B, int T, int H, int G, int K, int V, int L) {
+int mamba2_prompt_states_check(int B, int T, int H, int G, int K, int V, int L) {
     if (B <= 0 || T <= 0 || H <= 0 || G <= 0 || H % G != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!((K == 64 || K == 128) && V == 64) || L <= 0 || L > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (L < 1 + (32 - __builtin_clz((unsigned)(T - 1) | 1u)) && T > 1) return LLATTN_ERR_TOO_FEW_LEVELS;
     return 0;
 }
 
+}  // namespace llattn
+
+extern "C" {
+
 int llattn_mamba2_final_state(const void* k, const void* v, const float* g, float* states,
                               int B, int T, int H, int G, int K, int V, int L, void* stream) {
-    const int rc = final_state_check(B, T, H, G, K, V, L);
+    const int rc = llattn::mamba2_prompt_states_check(B, T, H, G, K, V, L);
     if (rc != 0) return rc;
     if (!k || !v || !g || !states) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
@@ -375,7 +390,7 @@ int llattn_mamba2_final_state(const void* k, const void* v, const float* g, floa
 
 int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, float* states, const void* fwd_workspace,
                                 size_t fwd_workspace_bytes, int B, int T, int Tp, int H, int G, int K, int V, int L, void* stream) {
-    const int rc = final_state_check(B, T, H, G, K, V, L);
+    const int rc = llattn::mamba2_prompt_states_check(B, T, H, G, K, V, L);
     if (rc != 0) return rc;
     if (Tp < T || Tp % 64 != 0) return LLATTN_ERR_BAD_LENGTH;
     if (!k || !v || !g || !states) return LLATTN_ERR_NULL;
@@ -385,18 +400,7 @@ int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, fl
         if (e != 0) return e;
     }
     using bf = __nv_bfloat16;
-    dim3 grid(B * H, L);
-    cudaStream_t st = (cudaStream_t)stream;
-    auto launch = [&](auto kern, size_t sm) -> cudaError_t {
-        const cudaError_t e = llattn::allow_smem(kern, sm);
-        if (e == cudaSuccess) llattn::launch_chained(kern, grid, 256, sm, st, (const bf*)k, (const bf*)v, g, states, seg_F, seg_D, T, Tp, H, G, L);
-        return e;
-    };
-    const cudaError_t e = K == 128 ? launch(llattn::mamba2_prompt_state_kernel<128>, llattn::PromptStateSmem<128>::total)
-                                   : launch(llattn::mamba2_prompt_state_kernel<64>, llattn::PromptStateSmem<64>::total);
-    if (e != cudaSuccess) return (int)e;
-    LLATTN_LAUNCHED();
-    return (int)cudaGetLastError();
+    return llattn::mamba2_prompt_states_launch((const bf*)k, (const bf*)v, g, states, seg_F, seg_D, B, T, Tp, H, G, K, L, (cudaStream_t)stream);
 }
 
 int llattn_mamba2_step(float* states, const void* q, const void* k, const void* v, const float* g, const void* lambda, void* o,
