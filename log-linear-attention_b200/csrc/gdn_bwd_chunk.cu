@@ -18,10 +18,10 @@ namespace llattn {
 
 // Shared memory: three 64-row tiles of K or V columns and five 64 x 64 tiles, each used for several operands in turn, so that two
 // CTAs fit on an SM (109,600 bytes with V = 128).  k stays in the first; the others hold
-//     S1: q -> v -> w -> dw          S2: d_o -> d_u -> -(d_qd exp(G)) -> q
-//     Aw    QK -> dKK    Au -> dQK    Ta: P -> dAu -> dAu Au^T -> Aw * beta_j -> dAw    Tb: dX -> dAw Aw^T
+//     S1: q -> v -> dAu Au^T -> w -> dw          S2: d_o -> d_u -> -(d_qd exp(G)) -> q
+//     Aw    QK -> dKK    Au -> dQK    Ta: P -> dAu -> Aw * beta_j -> dAw    Tb: dX -> dAw Aw^T
 // What bounds it: a chunk is a chain of barrier-separated small products whose latency one CTA of 8 warps does not fill: with fifteen tiles
-// of its own and one CTA per SM it took 1121 us at B = 4, T = 8192, 16 heads, V = 128, and takes 1000 us with two.  The load / store
+// of its own and one CTA per SM it took 1121 us at B = 4, T = 8192, 16 heads, V = 128, and takes 985 us with two.  The load / store
 // pipe is at 68 % then (ldmatrix of the operands 40 %), DRAM at 32 %.  (16 warps per chunk: 1180, the smaller warp tiles read more operands.)
 template <int KD, int VD>
 struct ChunkBwdSmem {
@@ -39,7 +39,7 @@ struct ChunkBwdSmem {
 // the chunk total of d_kd.kd (inside d_gl); otherwise a row pass over the K-wide gradients derives them here.
 // NORM: the backward of the l2 normalisation of q and k, (g - y (y . g)) rstd with y = f rstd, is taken on the accumulator fragments (the two
 // halves of a row's sums meet in shared memory) and bf16 rows leave.  As a pass of its own it read the fp32 dq, dk that this kernel wrote:
-// 1000 + 189 us at B = 4, T = 8192, 16 heads against 1040 with both (and 16 for what is left of that pass, dbeta and dlambda).
+// 985 + 189 us at B = 4, T = 8192, 16 heads against 1026 with both (and 16 for what is left of that pass, dbeta and dlambda).
 template <int KD, int VD, bool FUSED, bool NORM>
 __global__ void __launch_bounds__(256, 2) gdn_bwd_chunk_kernel(const GdnParams p) {
     chain_wait();
@@ -348,24 +348,29 @@ __global__ void __launch_bounds__(256, 2) gdn_bwd_chunk_kernel(const GdnParams p
         load_tile_async<CH, KD, 256>(s2, p.dqd_neg + rowbase * KD, (long)p.H * KD, tid);
         cp_async_commit();
     }
-    // ---- dAu Au^T takes the place of dAu
+    // ---- dAu Au^T, in the place of v
     {
         float acc[1][4][4];
         zero_acc(acc);
         warp_gemm<1, 2, false, false>(acc, sTa, LDP, r0, sAu, LDP, cw * 32, CH, lane);
-        __syncthreads();
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh)
-                *reinterpret_cast<uint32_t*>(sTa + (r0 + lr + hh * 8) * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
+                *reinterpret_cast<uint32_t*>(s1 + (r0 + lr + hh * 8) * LDP + cw * 32 + nt * 8 + lc2) = pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
     }
     __syncthreads();
+    // ---- Aw * beta_j, in the place of dAu
+    for (int e = tid; e < CH * CH / 2; e += 256) {
+        const int i = e / (CH / 2), j = (e % (CH / 2)) * 2;
+        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(sAw + i * LDP + j);
+        *reinterpret_cast<uint32_t*>(sTa + i * LDP + j) = pack_bf16(__bfloat162float(x.x) * sBe[j], __bfloat162float(x.y) * sBe[j + 1]);
+    }
     // ---- dAg = -Au^T (dAu Au^T), times Gamma, and its decay terms
     float dag[1][4][4];
     {
         zero_acc(dag);
-        warp_gemm<1, 2, true, true>(dag, sAu, LDP, r0, sTa, LDP, cw * 32, CH, lane);
+        warp_gemm<1, 2, true, true>(dag, sAu, LDP, r0, s1, LDP, cw * 32, CH, lane);
         float rs[2] = {0.f, 0.f};
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
@@ -404,7 +409,7 @@ __global__ void __launch_bounds__(256, 2) gdn_bwd_chunk_kernel(const GdnParams p
             if ((lane & 3) == 0) pRowG_A[cw * CH + r0 + lr + hh * 8] = rs[hh];
         }
     }
-    __syncthreads();                           // Au and its products consumed
+    __syncthreads();                           // Au and its products consumed, Aw * beta_j complete
     // row pass over the K-wide gradients: -(d_qd exp(G)) as a bf16 operand; the decay terms
     //      dG_i += d_qd.qd + d_wd.wd - d_kd.kd and the chunk total of d_kd.kd
     if (!FUSED) {
@@ -452,12 +457,6 @@ __global__ void __launch_bounds__(256, 2) gdn_bwd_chunk_kernel(const GdnParams p
         if (lane == 0) atomicAdd(&sMisc[0], kdsum);
     }
     // ---- w = (Aw * beta_j) k
-    for (int e = tid; e < CH * CH / 2; e += 256) {
-        const int i = e / (CH / 2), j = (e % (CH / 2)) * 2;
-        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(sAw + i * LDP + j);
-        *reinterpret_cast<uint32_t*>(sTa + i * LDP + j) = pack_bf16(__bfloat162float(x.x) * sBe[j], __bfloat162float(x.y) * sBe[j + 1]);
-    }
-    __syncthreads();
     {
         float acc[1][2 * NPK][4];
         zero_acc(acc);
