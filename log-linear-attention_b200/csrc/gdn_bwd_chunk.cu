@@ -21,7 +21,8 @@ namespace llattn {
 //     S1: q -> v -> dAu Au^T -> w -> dw          S2: d_o -> d_u -> -(d_qd exp(G)) -> q
 //     Aw    QK -> dKK    Au -> dQK    Ta: P -> dAu -> Aw * beta_j -> dAw    Tb: dX -> dAw Aw^T
 // What bounds it: a chunk is a chain of barrier-separated small products whose latency one CTA of 8 warps does not fill: with fifteen tiles
-// of its own and one CTA per SM it took 1121 us at B = 4, T = 8192, 16 heads, V = 128, and takes 985 us with two.  The load / store
+// of its own and one CTA per SM it took 1121 us at B = 4, T = 8192, 16 heads, V = 128, and took 1000 us with two; with NORM
+// (below) 1041, and 1027 once two barriers had gone.  The load / store
 // pipe is at 68 % then (ldmatrix of the operands 40 %), DRAM at 32 %.  (16 warps per chunk: 1180, the smaller warp tiles read more operands.)
 template <int KD, int VD>
 struct ChunkBwdSmem {
@@ -39,7 +40,7 @@ struct ChunkBwdSmem {
 // the chunk total of d_kd.kd (inside d_gl); otherwise a row pass over the K-wide gradients derives them here.
 // NORM: the backward of the l2 normalisation of q and k, (g - y (y . g)) rstd with y = f rstd, is taken on the accumulator fragments (the two
 // halves of a row's sums meet in shared memory) and bf16 rows leave.  As a pass of its own it read the fp32 dq, dk that this kernel wrote:
-// 985 + 189 us at B = 4, T = 8192, 16 heads against 1026 with both (and 16 for what is left of that pass, dbeta and dlambda).
+// 1000 + 189 us at B = 4, T = 8192, 16 heads against 1041 with both (and 16 for what is left of that pass, dbeta and dlambda).
 template <int KD, int VD, bool FUSED, bool NORM>
 __global__ void __launch_bounds__(256, 2) gdn_bwd_chunk_kernel(const GdnParams p) {
     chain_wait();
