@@ -1138,19 +1138,27 @@ static int launch_fwdorder(const Mamba2Params& p, bool use_tc, cudaStream_t stre
     return (int)cudaGetLastError();
 }
 
+// dq, d lambda and the reader totals of the high levels (warp-level kernels; the tensor-core one makes the reader summaries as well)
 template <int KD, int VD, int MLOW>
-static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStream_t stream) {
+static int launch_high_q(const Mamba2Params& p, cudaStream_t stream) {
     cudaError_t e;
-    constexpr int SEG = 1 << MLOW;
+    auto kern = m2_hi_bwd_q_kernel<KD, VD, MLOW>;
+    if ((e = allow_smem(kern, HiBwdSmem<KD, VD>::total)) != cudaSuccess) return (int)e;
+    llattn::launch_chained(kern, p.B * p.H * (p.NT - (1 << MLOW)), 256, HiBwdSmem<KD, VD>::total, stream, p); LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
+template <int KD, int VD, int MLOW>
+static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStream_t stream, bool with_q) {
+    cudaError_t e;
     if (p.NS > 1) {
         if (use_tc) {
             const int rc = mamba2_hi_bwd_tc_launch(p, stream);
             if (rc != 0) return rc;
         } else {
-            {
-                auto kern = m2_hi_bwd_q_kernel<KD, VD, MLOW>;
-                if ((e = allow_smem(kern, HiBwdSmem<KD, VD>::total)) != cudaSuccess) return (int)e;
-                llattn::launch_chained(kern, p.B * p.H * (p.NT - SEG), 256, HiBwdSmem<KD, VD>::total, stream, p); LLATTN_LAUNCHED();
+            if (with_q) {
+                const int rc = launch_high_q<KD, VD, MLOW>(p, stream);
+                if (rc != 0) return rc;
             }
             {
                 auto kern = m2_seg_dstate_kernel<KD, VD, MLOW>;
@@ -1184,12 +1192,15 @@ static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
             cudaError_t e;
             if ((e = side->fork(stream)) != cudaSuccess) return (int)e;
             rc = launch_fwdorder<KD, VD, MLOW>(p, use_tc, side->stream());
-            const int rc2 = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream);
+            // (the warp-level kernel of the high levels' dq is not part of that chain: a layer's step at B = 2, T = 1984, 8 heads, K = 128
+            //  224 -> 200 us, 24 heads with K = 64 341 -> 322, B = 2, T = 4032, 4 heads 178 -> 168)
+            if (rc == 0 && p.NS > 1 && !use_tc) rc = launch_high_q<KD, VD, MLOW>(p, side->stream());
+            const int rc2 = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream, false);
             if ((e = side->join(stream)) != cudaSuccess) return (int)e;
             return rc != 0 ? rc : rc2;
         }
     }
-    if ((rc = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream)) != 0) return rc;
+    if ((rc = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream, true)) != 0) return rc;
     return launch_fwdorder<KD, VD, MLOW>(p, use_tc, stream);
 }
 
