@@ -65,15 +65,16 @@ int llattn_mamba2_fwd(const void* q, const void* k, const void* v, const float* 
 
 /* llattn_mamba2_fwd whose output leaves as y (B,T_y,H,V) = o + D x, o rounded to bf16 first: the D residual of a Mamba-2 layer, of the first
  * T_y <= T tokens.  x is (B,T_y,H,V) bf16; y and D (H) are fp32 (y_is_f32 != 0) or bf16; x is 16-byte, y 32-byte aligned.  LLATTN_ERR_UNSUPPORTED_SHAPE
- * where the tensor-core kernels do not run (L > 20): there o and the sum are two calls (llattn_mamba2_prompt_residual). */
+ * where the tensor-core kernels do not run (L > 20): there o and the sum are two calls (llattn_mamba2_residual). */
 int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, const float* g, const void* lambda,
                                const void* x, const void* D, void* y, int y_is_f32, int T_y, float* g_cum, void* workspace, size_t workspace_bytes,
                                int B, int T, int H, int G, int K, int V, int L, void* stream);
 
-/* llattn_mamba2_fwd_residual and llattn_mamba2_prompt_states (of the first T_y tokens, state_levels levels) in one call, the states beside the
- * output where both leave room.  Without D (NULL) y is o, (B,T,H,V) bf16. */
+/* A prompt of T whole-chunk tokens and a tail of `tail` < 64 (split q .. lambda, plain x and y, see the prompts below) in one call: the
+ * forward with y = o + D x (D x rounded to bf16 first where they are bf16), llattn_mamba2_prompt_states and llattn_mamba2_prompt_tail for
+ * state_levels levels, the states beside the output where both leave room.  Without D (NULL) y is o, bf16.  tail_part: as there. */
 int llattn_mamba2_fwd_prompt(const void* q, const void* k, const void* v, const float* g, const void* lambda,
-                             const void* x, const void* D, void* y, int y_is_f32, int T_y, float* states, int state_levels, float* g_cum,
+                             const void* x, const void* D, void* y, int y_is_f32, int tail, float* tail_part, float* states, int state_levels, float* g_cum,
                              void* workspace, size_t workspace_bytes, int B, int T, int H, int G, int K, int V, int L, void* stream);
 
 /* Forward for callers that cannot hand the library a scratch buffer.  (No counterpart in the
@@ -229,15 +230,31 @@ int llattn_gdn_layer_step(float* states, const void* q, const void* k, const voi
                           const void* lambda, void* o, int B, int H, int G, int K, int V, int L, unsigned live, int carry_level,
                           int l2norm, float scale, float lambda_mul, int device, void* stream);
 
-/* Prompts: the chunkwise kernels run on tensors of Tp >= T tokens whose last Tp - T tokens are zero (they leave the states as
- * they are), so that no token of a ragged prompt is stepped.  Together these replace hattention_prefill (hattention/kernel.py:
- * 469-560) and the torch operators of the layer around it (hattention/mamba_apis.py:346-399).
- *   pad_tokens: n <= 8 tensors (B,T,...) of src_bytes[i] per token copied to (B,Tp,...) of dst_bytes[i] >= src_bytes[i]
- *   mamba2_prompt_prep: llattn_mamba2_prep_fwd writing v, g, lambda (L_out >= L columns) Tp tokens long, and, where q_pad and
- *     k_pad are given, q and k; dt_bias (may be NULL) and Lp are fp32 or bf16 by their flags
- *   mamba2_prompt_residual: y (B,T,H,P) = o (B,Tp,H,P) + D x; y and D are fp32 (y_is_f32 != 0) or bf16; D may be NULL
- *   mamba2_prompt_states: the level states after T tokens, level-major, every level written; k, v, g are Tp tokens long.  With the
- *     workspace of the forward call on them (may be NULL) the levels that hold whole 512-token segments are sums of its summaries.
+/* Prompts of T + tail tokens, T % 64 == 0, tail < 64: the whole chunks through the chunkwise kernels, the tail behind them in kernels
+ * that keep in fp32 what a decode step keeps in fp32.  Together these replace hattention_prefill (hattention/kernel.py:469-560) and
+ * the torch operators of the layer around it (hattention/mamba_apis.py:346-399).  "Split" tensors hold the B x T tokens of whole
+ * chunks first and the B x tail others behind them (the plain (B,T+tail,...) for B = 1 or without a tail).
+ *   mamba2_prompt_prep: split v, g, lambda of plain x, dt, dl, and, where q_split and k_split are given, split copies of q and k; rounded
+ *     as torch's operators on bf16 tensors round; dt_bias (may be NULL) and Lp are fp32 or bf16 by their flags
+ *   mamba2_prompt_residual: y = o + D x of the whole chunks; o (B,T,H,P), plain x, y; y and D are fp32 (y_is_f32 != 0) or bf16
+ *   mamba2_prompt_states: the level states after T tokens, level-major; k, v, g of the whole chunks.  With the workspace of the forward
+ *     call on them (may be NULL) the levels that hold whole 512-token segments are sums of its summaries.  With a tail: as the first
+ *     token of it finds them once the cascade has run, and without the levels 0 .. 6.
+ *   mamba2_prompt_tail: outputs of the tail (y plain, with D its residual) and the level states after it, from those; split q .. lambda;
+ *     tail_part: B tail H V floats of scratch (16-byte aligned; may be NULL for T = 0) */
+int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
+                              const void* Lp, int lp_is_f32, const void* q, const void* k, void* v, float* g, void* lambda, void* q_split,
+                              void* k_split, int B, int T, int tail, int H, int G, int K, int P, int L, int lambda_mode, void* stream);
+int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, void* y, int y_is_f32, int B, int T, int tail, int H, int P,
+                                  void* stream);
+int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, float* states, const void* fwd_workspace,
+                                size_t fwd_workspace_bytes, int B, int T, int tail, int H, int G, int K, int V, int L, void* stream);
+int llattn_mamba2_prompt_tail(const void* q, const void* k, const void* v, const float* g, const void* lambda, const void* x, const void* D,
+                              int y_is_f32, void* y, float* states, int state_levels, float* tail_part, int B, int T, int tail, int H, int G, int K,
+                              int V, int L, void* stream);
+
+/* Delta-rule prompts run the chunkwise kernels on tensors of Tp >= T tokens whose last Tp - T tokens are zero (they leave the states as
+ * they are).
  *   gdn_prompt_prep: a value head of V columns as `rep` heads of V / rep columns that share everything else ((B,T,H,V) is (B,T,H rep,V / rep)
  *     in memory).  One row per part: l2norm of q (scaled) and k, K_out >= K columns wide (at most 128), and, each where its pointer is given,
  *     v, beta and g, lambda (times lambda_mul unless 0, L_out columns), all Tp tokens long.  q, k have G groups of H / G heads.
@@ -245,16 +262,6 @@ int llattn_gdn_layer_step(float* states, const void* q, const void* k, const voi
  *     (B,H / rep,state_levels,state_rows,rep V); other levels are left alone
  *   gdn_prompt_states: advances those levels by the tokens of the last chunk and writes the levels inside it, so that every level is as of
  *     token T - 1; kn (B,Tp,H,128), v (B,Tp,H,V), states (B,H / rep,L,K,rep V); T is in the last 64 tokens of Tp */
-int llattn_pad_tokens(int n, const void* const* src, void* const* dst, const int* src_bytes, const int* dst_bytes, int B, int T, int Tp,
-                      void* stream);
-int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl,
-                              const void* Lp, int lp_is_f32, const void* q, const void* k, void* v, float* g, void* lambda, void* q_pad,
-                              void* k_pad, int B, int T, int Tp, int H, int G, int K, int P, int L, int L_out, int lambda_mode,
-                              void* stream);
-int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, void* y, int y_is_f32, int B, int T, int Tp, int H, int P,
-                                  void* stream);
-int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, float* states, const void* fwd_workspace,
-                                size_t fwd_workspace_bytes, int B, int T, int Tp, int H, int G, int K, int V, int L, void* stream);
 int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                            void* qn, void* kn, void* v_pad, void* beta_pad, float* g_pad, void* lambda_pad,
                            int B, int T, int Tp, int H, int G, int K, int K_out, int V, int rep, int L, int L_out, float scale,

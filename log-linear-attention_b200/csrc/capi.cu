@@ -136,6 +136,7 @@ static int mamba2_fwd_impl(llattn::Mamba2Params& p, const void* q, const void* k
     if (!q || !k || !v || !g || !lambda || (!o && !p.res_D) || !g_cum) return LLATTN_ERR_NULL;
     p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
     if (p.res_D && !llattn::mamba2_uses_tc(p)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (p.oT == 0) p.oT = T;
     const size_t need = setup(p, nullptr, false);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) return LLATTN_ERR_WORKSPACE;
     setup(p, workspace, false);
@@ -161,21 +162,25 @@ int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, cons
     if (T_y <= 0 || T_y > T) return LLATTN_ERR_BAD_LENGTH;
     if (((uintptr_t)x & 15) || ((uintptr_t)y & 31)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     llattn::Mamba2Params p = {};
-    p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_T = T_y; p.res_f32 = y_is_f32;
+    p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_T = p.res_n = T_y; p.res_f32 = y_is_f32;
     return mamba2_fwd_impl(p, q, k, v, g, lambda, nullptr, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);
 }
 
 int llattn_mamba2_fwd_prompt(const void* q, const void* k, const void* v, const float* g, const void* lambda,
-                             const void* x, const void* D, void* y, int y_is_f32, int T_y, float* states, int state_levels, float* g_cum,
+                             const void* x, const void* D, void* y, int y_is_f32, int tail, float* tail_part, float* states, int state_levels, float* g_cum,
                              void* workspace, size_t workspace_bytes, int B, int T, int H, int G, int K, int V, int L, void* stream) {
-    if (!y || !states || (D && !x)) return LLATTN_ERR_NULL;
-    if (T_y <= 0 || T_y > T) return LLATTN_ERR_BAD_LENGTH;
+    if (!y || !states || (D && !x) || (tail > 0 && !tail_part)) return LLATTN_ERR_NULL;
+    if (T <= 0 || tail < 0 || tail >= llattn_chunk()) return LLATTN_ERR_BAD_LENGTH;
     if (D && (((uintptr_t)x & 15) || ((uintptr_t)y & 31))) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    const int rc = llattn::mamba2_prompt_states_check(B, T_y, H, G, K, V, state_levels);
+    const int rc = llattn::mamba2_prompt_states_check(B, T + tail, H, G, K, V, state_levels);
     if (rc != 0) return rc;
     llattn::Mamba2Params p = {};
-    if (D) { p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_T = T_y; p.res_f32 = y_is_f32; }
-    p.pr_states = states; p.pr_T = T_y; p.pr_L = state_levels;
+    if (D) {
+        p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_f32 = y_is_f32;
+        p.res_T = T + tail; p.res_n = T; p.res_round = 1;
+    }
+    p.oT = T + tail;
+    p.pr_states = states; p.pr_part = tail_part; p.pr_n = tail; p.pr_L = state_levels;
     return mamba2_fwd_impl(p, q, k, v, g, lambda, D ? nullptr : y, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);
 }
 
@@ -220,6 +225,7 @@ int llattn_mamba2_fwd_static(const void* q, const void* k, const void* v, const 
     setup(p, g_static_scratch_addr[dev], false);
     p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
     p.g = g; p.l = (const __nv_bfloat16*)lambda;
+    p.oT = T;
     p.o = (__nv_bfloat16*)o; p.g_cum = g_cum;
     e = cudaMemsetAsync(p.err, 0, sizeof(int), (cudaStream_t)stream);
     if (e != cudaSuccess) return (int)e;

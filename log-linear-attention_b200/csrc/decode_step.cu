@@ -17,17 +17,13 @@
 //   Mamba-2, K = 128, V = 64: B = 1, H = 48 7.5 us; B = 4, H = 32 13.7 us; B = 64, H = 32 188 us = 5.7 TB/s (the level-innermost
 //   kernel behind the layer's torch operators: 110 us and 1200 us for a call at B = 1 and B = 64)
 //   delta rule, K = V = 128: B = 1, H = 16 6.2 us; B = 16, H = 16 48.4 us = 5.5 TB/s (414 us for a call before)
-#include "llattn_common.cuh"
+#include "rowwise.cuh"
 #include "../../include/llattn.h"
 
 namespace llattn {
 
 constexpr int ST_THREADS = 256;
 constexpr int ST_MAXL = 32;
-
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
-// torch's softplus: identity above 20
-__device__ __forceinline__ float softplus_torch(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
 // 16 bytes if p, else zeros, without a branch: a branch around every load of a group keeps the compiler from having them all in
 // flight (the delta-rule step took 177 us instead of 103 at B = 16, H = 16, K = V = 128)
@@ -64,10 +60,7 @@ struct M2StepArgs {
 __device__ __forceinline__ float layer_lambda(const M2StepArgs& a, long bh, int h, int l) {
     const float d = __bfloat162float(a.dl[bh * a.L + l]);
     if (a.Lp == nullptr) return d;
-    const float lp = bf16_round(load_param(a.Lp, h * a.L + l, a.lp_f32));
-    if (a.lambda_mode == 0) return bf16_round(softplus_torch(bf16_round(lp * d)));
-    if (a.lambda_mode == 1) return bf16_round(expf(bf16_round(-bf16_round(expf(lp)) * bf16_round(softplus_torch(d)))));
-    return bf16_round(lp * d);
+    return lambda_torch(a.lambda_mode, load_param(a.Lp, h * a.L + l, a.lp_f32), d);
 }
 
 // A CTA owns COLS value columns of one (batch, head).  COLS = 64 (whole rows of a 64-wide head, 256 contiguous bytes) for
@@ -124,13 +117,13 @@ __global__ void __launch_bounds__(ST_THREADS, CTAS) m2_layer_step_kernel(const _
             float t = __bfloat162float(a.dt[bh]);
             if (a.bias != nullptr) t += load_param(a.bias, h, a.bias_f32);
             const bool half = a.bias == nullptr || !a.bias_f32;      // dt stays bf16 between torch's operators
-            if (half) t = bf16_round(t);
+            if (half) t = round_bf16(t);
             if (a.softplus) {
                 t = softplus_torch(t);
-                if (half) t = bf16_round(t);
+                if (half) t = round_bf16(t);
             }
             g = a.A[h] * t;
-            xv = bf16_round(xv * t);
+            xv = round_bf16(xv * t);
         } else {
             g = a.g[bh];
         }
@@ -209,11 +202,11 @@ __global__ void __launch_bounds__(ST_THREADS, CTAS) m2_layer_step_kernel(const _
 #pragma unroll
         for (int w = 0; w < 8; ++w) o += reinterpret_cast<const float*>(sO[w])[tid];
         const long at = bh * a.V + cb * COLS + tid;
-        o = bf16_round(o);
+        o = round_bf16(o);
         if (a.D != nullptr) {
             const float xd = __bfloat162float(a.x[at]) * load_param(a.D, h, a.d_f32);
             if (a.d_f32) reinterpret_cast<float*>(a.y)[at] = o + xd;
-            else reinterpret_cast<bf16*>(a.y)[at] = __float2bfloat16(o + bf16_round(xd));
+            else reinterpret_cast<bf16*>(a.y)[at] = __float2bfloat16(o + round_bf16(xd));
         } else {
             reinterpret_cast<bf16*>(a.y)[at] = __float2bfloat16(o);
         }
@@ -296,14 +289,14 @@ __global__ void __launch_bounds__(THREADS, CTAS) gdn_layer_step_kernel(const __g
             if (lane + 32 * i < a.K) {
                 float y = f[i];
                 if (a.l2norm) {
-                    y = bf16_round(y * rstd);
-                    if (warp == 0) y = bf16_round(y * a.scale);
+                    y = round_bf16(y * rstd);
+                    if (warp == 0) y = round_bf16(y * a.scale);
                 }
                 dst[lane + 32 * i] = y;
             }
     } else if (warp == 2 && lane < a.L) {
         const float l = __bfloat162float(a.lam[bh * a.L + lane]);
-        sLam[lane] = a.lam_mul != 0.f ? bf16_round(l * a.lam_mul) : l;
+        sLam[lane] = a.lam_mul != 0.f ? round_bf16(l * a.lam_mul) : l;
     }
     const float dec = fexp(a.g[bh]);
     const float be = __bfloat162float(a.beta[bh]);

@@ -26,7 +26,7 @@ using torch::autograd::variable_list;
 #define LLATTN_FUNCS(F)                                                                                                             \
     F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_fwd_residual) F(llattn_mamba2_fwd_prompt) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
     F(llattn_mamba2_layer_prep_fwd) F(llattn_mamba2_layer_prep_bwd) F(llattn_mamba2_layer_step) F(llattn_gdn_layer_step)            \
-    F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mixer_prep_fwd)            \
+    F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mamba2_prompt_tail) F(llattn_mamba2_residual) F(llattn_mixer_prep_fwd)            \
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
     F(llattn_gdn_fwd_workspace_bytes) F(llattn_gdn_fwd_keep_workspace_bytes) F(llattn_gdn_fwd) F(llattn_gdn_fwd_keep)                \
     F(llattn_gdn_prefill_parts) F(llattn_gdn_prompt_states) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
@@ -135,22 +135,22 @@ Scan mamba2_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor&
     if (status) check_status(s.ws, stream, "llattn_mamba2_fwd");
     return s;
 }
-// the same with y = o + D x of the first x.size(1) tokens in the place of o
+// the same with y = o + D x in the place of o
 Scan mamba2_fwd_residual(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, const Tensor& x, const Tensor& D,
                          void* stream, bool status) {
-    const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3), Ty = x.size(1);
+    const int B = k.size(0), T = k.size(1), G = k.size(2), K = k.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
     Scan s;
     s.o = empty(x.sizes(), f32(D) ? at::kFloat : at::kBFloat16, x);
     s.g_cum = contiguous_like(g);
     const size_t n = lib.llattn_mamba2_fwd_workspace_bytes(B, T, H, G, K, V, L);
     s.ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
     const int rc = lib.llattn_mamba2_fwd_residual(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), l.data_ptr(), x.data_ptr(), D.data_ptr(),
-                                                  s.o.data_ptr(), f32(D), Ty, fptr(s.g_cum), s.ws.data_ptr(), s.ws.numel(), B, T, H, G, K, V, L, stream);
+                                                  s.o.data_ptr(), f32(D), T, fptr(s.g_cum), s.ws.data_ptr(), s.ws.numel(), B, T, H, G, K, V, L, stream);
     if (rc == LLATTN_ERR_UNSUPPORTED_SHAPE) {
-        const Tensor y = s.o;
+        const Tensor y = s.o, D32 = D.to(at::kFloat);
         s = mamba2_fwd(q, k, v, g, l, stream, status);
-        check(lib.llattn_mamba2_prompt_residual(s.o.data_ptr(), x.data_ptr(), ptr(D), y.data_ptr(), f32(D), B, Ty, T, H, V, stream),
-              "llattn_mamba2_prompt_residual");
+        check(lib.llattn_mamba2_residual(s.o.data_ptr(), x.data_ptr(), fptr(D32), y.data_ptr(), f32(D), (long)B * T * H, H, V, stream),
+              "llattn_mamba2_residual");
         s.o = y;
         return s;
     }
@@ -294,56 +294,108 @@ py::object mamba2_layer(const Tensor& x, const Tensor& dt, const Tensor& A, cons
     return py::cast(y);
 }
 
-// ---- a prompt of any length: outputs and level states (level-major).  (y, states) or None
+// ---- a prompt of any length: outputs and level states (level-major), after its T0 whole-chunk tokens and the n < 64 behind them
+struct Prompt {
+    int B, T0, n, H, G, N, P, L;
+    Prompt(int B, int T, int H, int G, int N, int P, int L) : B(B), T0(T / 64 * 64), n(T % 64), H(H), G(G), N(N), P(P), L(L) {}
+    int T() const { return T0 + n; }
+    bool takes() const { return T() > 0 && L >= 1 + bit_length(T() - 1) && (T0 == 0 || mamba2_shape(T0, H, G, N, P, L)); }
+    // several sequences with tails: the tensors hold the whole chunks of all of them first, then the tails
+    bool split() const { return B > 1 && n > 0 && T0 > 0; }
+    Tensor parts(const Tensor& t) const {
+        if (!split()) return t;
+        return at::cat({t.narrow(1, 0, T0).reshape({-1}), t.narrow(1, T0, n).reshape({-1})});
+    }
+    // tensors of B T() tokens, split; x as it is and D, or neither.  (y, states (B,H,L,N,P))
+    std::pair<Tensor, Tensor> run(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& lam, const Tensor& x, const Tensor& D,
+                                  void* stream, bool status) const {
+        const bool y32 = f32(D);
+        const Tensor y = empty({B, T(), H, P}, y32 ? at::kFloat : at::kBFloat16, v), states = empty({B, H, L, N, P}, at::kFloat, v);
+        const Tensor part = n > 0 && T0 > 0 ? empty({B, n, H, P}, at::kFloat, v) : Tensor();
+        int rc = 0;
+        if (T0 > 0) {
+            const Tensor g_cum = empty({B, T0, H}, at::kFloat, v);
+            const size_t bytes = std::max<size_t>(lib.llattn_mamba2_fwd_workspace_bytes(B, T0, H, G, N, P, L), 256);
+            const Tensor ws = empty({(int64_t)bytes}, at::kByte, v);
+            rc = lib.llattn_mamba2_fwd_prompt(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), ptr(x), ptr(D), y.data_ptr(), y32, n,
+                                              fptr(part), fptr(states), L, fptr(g_cum), ws.data_ptr(), bytes, B, T0, H, G, N, P, L, stream);
+            if (rc == 0 && status) check_status(ws, stream, "llattn_mamba2_fwd_prompt");
+            if (rc != LLATTN_ERR_UNSUPPORTED_SHAPE || !D.defined()) {
+                check(rc, "llattn_mamba2_fwd_prompt");
+                return {y, states};
+            }
+            const Tensor o = empty({B, T0, H, P}, at::kBFloat16, v);
+            check(lib.llattn_mamba2_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), o.data_ptr(), fptr(g_cum), ws.data_ptr(), bytes, B,
+                                        T0, H, G, N, P, L, stream),
+                  "llattn_mamba2_fwd");
+            if (status) check_status(ws, stream, "llattn_mamba2_fwd");
+            check(lib.llattn_mamba2_prompt_residual(o.data_ptr(), x.data_ptr(), ptr(D), y.data_ptr(), y32, B, T0, n, H, P, stream),
+                  "llattn_mamba2_prompt_residual");
+            check(lib.llattn_mamba2_prompt_states(k.data_ptr(), v.data_ptr(), fptr(g), fptr(states), ws.data_ptr(), bytes, B, T0, n, H, G, N, P, L, stream),
+                  "llattn_mamba2_prompt_states");
+        }
+        if (n > 0)
+            check(lib.llattn_mamba2_prompt_tail(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), ptr(x), ptr(D), y32, y.data_ptr(),
+                                                fptr(states), L, fptr(part), B, T0, n, H, G, N, P, L, stream),
+                  "llattn_mamba2_prompt_tail");
+        return {y, states};
+    }
+};
+
 py::object mamba2_prompt(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm, const Tensor& dl, const Tensor& Lp,
                          const Maybe& D_, const Maybe& bias_, int64_t mode, bool status) {
     const Tensor D = of(D_), bias = of(bias_);
     if (!layer_operands(x, dt, A, Bm, Cm, dl, Lp, D, bias) || wants_grad({x, dt, A, Bm, Cm, dl, Lp, D, bias})) return py::none();
-    const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), G = Bm.size(2), N = Bm.size(3), L = dl.size(3);
-    const int Tp = (T + 63) / 64 * 64, Lo = T < 64 ? std::max(L, 7) : L;
-    if (T < 1 || L < 1 + bit_length(T - 1) || !mamba2_shape(Tp, H, G, N, P, Lo)) return py::none();
-    Tensor y, states;
+    const Prompt p(x.size(0), x.size(1), x.size(2), Bm.size(2), Bm.size(3), x.size(3), dl.size(3));
+    if (!p.takes()) return py::none();
+    std::pair<Tensor, Tensor> r;
     {
         py::gil_scoped_release nogil;
         at::NoGradGuard no_grad;
         On on(x);
         const Tensor x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), A_ = A.to(at::kFloat).contiguous(), Lp_ = Lp.contiguous(),
                      D_c = contiguous(D), b_ = contiguous(bias);
-        Tensor q = Cm.contiguous(), k = Bm.contiguous(), qp, kp;
-        const Tensor v = empty({B, Tp, H, P}, at::kBFloat16, x), g = empty({B, Tp, H}, at::kFloat, x), lam = empty({B, Tp, H, Lo}, at::kBFloat16, x);
-        if (Tp != T) {
-            qp = empty({B, Tp, G, N}, at::kBFloat16, x);
-            kp = contiguous_like(qp);
+        Tensor q = Cm.contiguous(), k = Bm.contiguous(), qs, ks;
+        const Tensor v = contiguous_like(x_), g = empty(dt_.sizes(), at::kFloat, x), lam = contiguous_like(dl_);
+        if (p.split()) {
+            qs = contiguous_like(q);
+            ks = contiguous_like(q);
         }
         check(lib.llattn_mamba2_prompt_prep(x_.data_ptr(), dt_.data_ptr(), ptr(b_), f32(b_), fptr(A_), dl_.data_ptr(), Lp_.data_ptr(), f32(Lp_),
-                                            q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), ptr(qp), ptr(kp), B, T, Tp, H, G, N, P, L,
-                                            Lo, (int)mode, on.stream),
+                                            q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), ptr(qs), ptr(ks), p.B, p.T0, p.n, p.H, p.G,
+                                            p.N, p.P, p.L, (int)mode, on.stream),
               "llattn_mamba2_prompt_prep");
-        if (Tp != T) {
-            q = qp;
-            k = kp;
+        if (p.split()) {
+            q = qs;
+            k = ks;
         }
-        states = empty({B, H, L, N, P}, at::kFloat, x);
-        const Tensor g_cum = contiguous_like(g);
-        const size_t n = std::max<size_t>(lib.llattn_mamba2_fwd_workspace_bytes(B, Tp, H, G, N, P, Lo), 256);
-        const Tensor ws = empty({(int64_t)n}, at::kByte, x);
-        y = D_c.defined() ? empty(x.sizes(), f32(D_c) ? at::kFloat : at::kBFloat16, x) : contiguous_like(v);
-        const int rc = lib.llattn_mamba2_fwd_prompt(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g), lam.data_ptr(), x_.data_ptr(), ptr(D_c), y.data_ptr(),
-                                                    f32(y), T, fptr(states), L, fptr(g_cum), ws.data_ptr(), n, B, Tp, H, G, N, P, Lo, on.stream);
-        if (rc == LLATTN_ERR_UNSUPPORTED_SHAPE) {
-            const Scan s = D_c.defined() ? mamba2_fwd_residual(q, k, v, g, lam, x_, D_c, on.stream, status) : mamba2_fwd(q, k, v, g, lam, on.stream, status);
-            y = s.o;
-            check(lib.llattn_mamba2_prompt_states(k.data_ptr(), v.data_ptr(), fptr(g), fptr(states), s.ws.data_ptr(), s.ws.numel(), B, T, Tp, H, G, N, P, L,
-                                                  on.stream),
-                  "llattn_mamba2_prompt_states");
-        } else {
-            check(rc, "llattn_mamba2_fwd_prompt");
-            if (status) check_status(ws, on.stream, "llattn_mamba2_fwd_prompt");
-        }
-        states = states.permute({0, 1, 3, 4, 2});
-        if (!D_c.defined()) y = y.narrow(1, 0, T).contiguous();
+        r = p.run(q, k, v, g, lam, D_c.defined() ? x_ : Tensor(), D_c, on.stream, status);
+        r.second = r.second.permute({0, 1, 3, 4, 2});
     }
-    return py::make_tuple(y, states);
+    return py::make_tuple(r.first, r.second);
+}
+
+// hattention_prefill, Mamba-2 structure, on the scan's own operands: (o, level-major states) or None
+py::object mamba2_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool status) {
+    if (!bf16(q) || !bf16(k) || !bf16(v) || !is(g, at::kFloat) || !bf16(l) || k.dim() != 4 || v.dim() != 4 || l.dim() != 4 || q.sizes() != k.sizes() ||
+        !same_device({q, k, v, g, l}))
+        return py::none();
+    const int64_t B = k.size(0), T = k.size(1), G = k.size(2), N = k.size(3), H = v.size(2), P = v.size(3), L = l.size(3);
+    if (B < 1 || v.size(0) != B || v.size(1) != T || g.sizes() != at::IntArrayRef({B, T, H}) || l.sizes() != at::IntArrayRef({B, T, H, L}) || G < 1 ||
+        H % G != 0 || (N != 64 && N != 128) || P != 64 || L > 32 || T > 600000 || B * T * H >= (int64_t(1) << 28))
+        return py::none();
+    const Prompt p(B, T, H, G, N, P, L);
+    if (!p.takes()) return py::none();
+    std::pair<Tensor, Tensor> r;
+    {
+        py::gil_scoped_release nogil;
+        at::NoGradGuard no_grad;
+        On on(q);
+        r = p.run(p.parts(q.contiguous()), p.parts(k.contiguous()), p.parts(v.contiguous()), p.parts(g.contiguous()), p.parts(l.contiguous()), Tensor(), Tensor(),
+                  on.stream, status);
+        r.second = r.second.permute({0, 1, 3, 4, 2});
+    }
+    return py::make_tuple(r.first, r.second);
 }
 
 // ---- the mixer between its projections
@@ -718,6 +770,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("hattention_mamba2", &hattention_mamba2);
     m.def("mamba2_layer", &mamba2_layer);
     m.def("mamba2_prompt", &mamba2_prompt);
+    m.def("mamba2_prefill", &mamba2_prefill);
     m.def("mamba2_mixer", &mamba2_mixer);
     m.def("mamba2_step", &mamba2_step);
     m.def("hattention_gdn", &hattention_gdn);

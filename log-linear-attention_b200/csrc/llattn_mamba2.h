@@ -57,9 +57,13 @@ struct Mamba2Params {
     const __nv_bfloat16* res_x;  // (B,res_T,H,V)
     const void* res_D;           // (H), fp32 like y if res_f32, else bf16
     void* res_y;                 // (B,res_T,H,V)
-    int res_T, res_f32;          // res_T <= T: a prompt's tokens without its padding
-    float* pr_states;            // forward of a prompt: also the level states after its first pr_T tokens, (B,H,pr_L,K,V)
-    int pr_T, pr_L;
+    int res_T, res_f32;          // res_T: tokens of a sequence of x and y
+    int res_n;                   // the first res_n <= T of them are written
+    int res_round;               // bf16 y: D x is rounded to bf16 before the sum, as two operators would
+    int oT;                      // tokens of a sequence of o (T, or those of the prompt whose whole chunks these are)
+    float* pr_states;            // forward of the whole chunks of a prompt of T + pr_n tokens: also its level states, (B,H,pr_L,K,V)
+    float* pr_part;              // (B,pr_n,H,V) scratch of the tail
+    int pr_n, pr_L;
     int reuse_states;            // backward: seg_D / seg_H0 come from the forward call, do not recompute them
 };
 
@@ -82,7 +86,19 @@ extern std::atomic<int> g_use_tensor_core_path;   // test hook, see llattn_testi
 // segment summaries and decays inside the workspace of a forward call (null when it has one segment only)
 int mamba2_prompt_states_check(int B, int T, int H, int G, int K, int V, int L);
 int mamba2_prompt_states_launch(const __nv_bfloat16* k, const __nv_bfloat16* v, const float* g, float* states, const float* seg_F, const float* seg_D,
-                                int B, int T, int Tp, int H, int G, int K, int L, cudaStream_t stream);
+                                int B, int T0, int n, int H, int G, int K, int L, cudaStream_t stream);
+// the tokens of a prompt behind its last whole chunk; bases of the tensors of all B (T0 + n) tokens
+struct Mamba2Tail {
+    const __nv_bfloat16 *q, *k, *v, *lam, *x;
+    const float* g;
+    const void* D;               // (H) or null
+    void* y;                     // (B,T0+n,H,64)
+    float* states;               // (B,H,L,K,64)
+    float* part;                 // (B,n,H,64) what the tokens among themselves add to the outputs
+    int T0, n, H, G, L, lam_L, d_f32;
+};
+int mamba2_tail_intra_launch(const Mamba2Tail& a, int B, int K, cudaStream_t stream);       // before or beside the whole chunks
+int mamba2_tail_levels_launch(const Mamba2Tail& a, int B, int K, cudaStream_t stream);      // behind the states after them
 int mamba2_fwd_workspace_segments(const void* ws, size_t bytes, int B, int T, int H, int G, int K, int V, const float** F, const float** D);
 // clears acc_bytes (a multiple of 16) at acc and ndl floats at dl, and takes the in-chunk cumulative sum of g apart
 int mamba2_bwd_init(const float* gc, float* g, long BT, int H, void* acc, size_t acc_bytes, float* dl, long ndl, cudaStream_t stream);

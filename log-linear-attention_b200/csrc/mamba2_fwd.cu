@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256, 1) m2_chunk_fwd_kernel(const Mamba2Params
         {
             float acc[1][2 * NPS][4];
             const int col0 = wc * (VD / 2);
-            bf16* go = p.o + (((long)b * p.T + t0) * p.H + h) * VD;
+            bf16* go = p.o + (((long)b * p.oT + t0) * p.H + h) * VD;
             if (hi_init) {
 #pragma unroll
                 for (int nt = 0; nt < 2 * NPS; ++nt)
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(256, 1) m2_hi_out_kernel(const Mamba2Params p)
             }
         return;
     }
-    bf16* go = p.o + (((long)b * p.T + t0) * p.H + h) * VD;
+    bf16* go = p.o + (((long)b * p.oT + t0) * p.H + h) * VD;
 #pragma unroll
     for (int nt = 0; nt < 2 * NPS; ++nt)
 #pragma unroll
@@ -608,13 +608,17 @@ template <int KD, int VD, int MLOW>
 static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
     const bool use_tc = mamba2_uses_tc(p);
-    // A prompt's level states need its segment summaries only, the output three more kernels.  While the chunk kernel leaves SMs idle (it
-    // takes one CTA per segment and SM) they are made beside those: B = 1, T = 1000, 48 heads, 96 CTAs: 62 -> 57 us for the call;
-    // T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs.
-    // Within a segment there is too little to run beside for the events to pay.
+    // A prompt's level states and its tail need the segment summaries only (part of the tail not even those), the output three more kernels.
+    // The states are made beside those while the chunk kernel leaves SMs idle (it takes one CTA per segment and SM): B = 1, T = 1000, 48 heads,
+    // 96 CTAs: 62 -> 57 us for the call without a tail's kernels; T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs; within a segment
+    // there is too little to run beside for the events to pay.  With a tail always: its kernels are chains of latency (T = 1500 87.6 -> 74.5 us,
+    // T = 3000 139 -> 119, T = 500 44.5 -> 42, four sequences of T = 700, 32 heads 123 -> 102).
     SideStream* side = nullptr;
-    auto states = [&](cudaStream_t on) {
-        return mamba2_prompt_states_launch(p.k, p.v, p.g, p.pr_states, p.seg_F, p.seg_D, p.B, p.pr_T, p.T, p.H, p.G, p.K, p.pr_L, on);
+    const Mamba2Tail tail{p.q, p.k, p.v, p.l, p.res_x, p.g, p.res_D, p.res_D ? p.res_y : p.o, p.pr_states, p.pr_part, p.T, p.pr_n, p.H, p.G, p.pr_L, p.L,
+                          p.res_f32};
+    auto states = [&](cudaStream_t on) -> int {
+        const int rc = mamba2_prompt_states_launch(p.k, p.v, p.g, p.pr_states, p.seg_F, p.seg_D, p.B, p.T, p.pr_n, p.H, p.G, p.K, p.pr_L, on);
+        return rc != 0 || p.pr_n == 0 ? rc : mamba2_tail_levels_launch(tail, p.B, p.K, on);
     };
     auto output = [&]() -> int {
         if (p.NS > 1) {
@@ -636,17 +640,25 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
         return (int)cudaGetLastError();
     };
     int rc;
-    if (p.NS > 1) {
+    if (p.pr_states && (p.pr_n > 0 || (p.NS > 1 && (long)p.B * p.H * p.NS * 4 < 148 * 3))) side = SideStream::get(stream);
+    if (p.pr_n > 0) {
+        if (side && (e = side->fork(stream)) != cudaSuccess) return (int)e;
+        rc = mamba2_tail_intra_launch(tail, p.B, p.K, side ? side->stream() : stream);
+        if (rc != 0 && !side) return rc;
+    } else {
+        rc = 0;
+    }
+    if (rc == 0 && p.NS > 1) {
         p.o_has_high = use_tc ? 2 : 1;      // 2: partial output goes to the column-chunk-major scratch
-        if ((rc = launch_states<KD, VD, MLOW>(p, stream)) != 0) return rc;
-        if (p.pr_states && (long)p.B * p.H * p.NS * 4 < 148 * 3) side = SideStream::get(stream);
+        rc = launch_states<KD, VD, MLOW>(p, stream);
+        if (rc != 0 && !side) return rc;
     }
     if (side) {
-        if ((e = side->fork(stream)) != cudaSuccess) return (int)e;
-        const int rs = states(side->stream());
-        rc = output();
-        if ((e = side->join(stream)) != cudaSuccess) return (int)e;
-        return rc != 0 ? rc : rs;
+        if (rc == 0 && p.NS > 1) rc = (int)side->fork(stream);       // for the summaries
+        if (rc == 0) rc = output();                                  // first: it is the longer chain
+        if (rc == 0) rc = states(side->stream());
+        const int rj = (int)side->join(stream);
+        return rc != 0 ? rc : rj;
     }
     if ((rc = output()) != 0 || !p.pr_states) return rc;
     return states(stream);

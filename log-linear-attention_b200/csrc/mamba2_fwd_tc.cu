@@ -11,6 +11,7 @@
 //     the masks / decays / lambda weights are applied on the way from tensor memory to the bf16
 //     P tile; level-state masters stay in registers in the tensor-memory readout layout (one
 //     state row per thread), their bf16 copies are written once as MN-major operands.
+#include "rowwise.cuh"
 #include "tc_common.cuh"
 
 namespace llattn {
@@ -30,7 +31,8 @@ struct FwdTcSmem {
     static constexpr uint32_t total = bar_off + 128 + 1024;             // + slack for 1024-byte alignment
 };
 
-// RES: 0 writes o; 1, 2 write y = o + D x of a layer (bf16 / fp32), o rounded to bf16 first as if it were stored.  As a pass of its own that sum
+// RES: 0 writes o; 1, 2 write y = o + D x of a layer (bf16 / fp32), o rounded to bf16 first as if it were stored; 3 is 1 with D x rounded to
+// bf16 too (prompts, whose sum is two operators' with a bf16 D).  As a pass of its own that sum
 // reads o and x again and took 45 of 494 us for a layer's forward at B = 8, T = 4096, 24 heads; here x comes to L2 while the
 // products run and is read while the level reads are summed (466 us).
 template <int MLOW, bool WHOLE, int RES>
@@ -269,7 +271,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
             for (int c = 0; c < 4; ++c) ohi[c] = *reinterpret_cast<const uint4*>(gh + c * tc::PT * 8);
         }
         // x rows of the pair into L2 (held in registers from here on they cost the products below more than they save)
-        if (RES && ch == 0 && t0 + row < p.res_T)
+        if (RES && ch == 0 && t0 + row < p.res_n)
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.res_x + (((long)b * p.res_T + t0 + row) * p.H + h) * tc::VD));
         STAMP();                                     // 1: small fetches issued
         umma::mbar_wait(&full_kv[st], (pl >> 1) & 1, abort_flag);      // the v tile (read below with generic loads)
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int rr = (tid >> 3) + u * 32;
-                xr[u] = t0 + rr < p.res_T ? __ldg(reinterpret_cast<const uint4*>(gx + (long)rr * p.H * tc::VD)) : make_uint4(0, 0, 0, 0);
+                xr[u] = t0 + rr < p.res_n ? __ldg(reinterpret_cast<const uint4*>(gx + (long)rr * p.H * tc::VD)) : make_uint4(0, 0, 0, 0);
             }
         }
         if (nread > 0) {
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int rr = (tid >> 3) + u * 32, c = (tid & 7) * 8;
-                    if (t0 + rr >= p.res_T) continue;
+                    if (t0 + rr >= p.res_n) continue;
                     const uint4 ov = *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
                     const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, xw[4] = {xr[u].x, xr[u].y, xr[u].z, xr[u].w};
                     float y[8];
@@ -450,8 +452,8 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
                     for (int e = 0; e < 4; ++e) {
                         const float2 of = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ow[e]));
                         const float2 xf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xw[e]));
-                        y[2 * e] = of.x + xf.x * dh;
-                        y[2 * e + 1] = of.y + xf.y * dh;
+                        y[2 * e] = of.x + (RES == 3 ? round_bf16(xf.x * dh) : xf.x * dh);
+                        y[2 * e + 1] = of.y + (RES == 3 ? round_bf16(xf.y * dh) : xf.y * dh);
                     }
                     const long at = (((long)b * p.res_T + t0 + rr) * p.H + h) * tc::VD + c;
                     if (RES == 2) {
@@ -465,7 +467,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
                     }
                 }
             }
-            bf16* go = p.o + (((long)b * p.T + t0) * p.H + h) * tc::VD;
+            bf16* go = p.o + (((long)b * p.oT + t0) * p.H + h) * tc::VD;
 #pragma unroll
             for (int i = RES ? tc::PT * 8 : tid; i < tc::PT * 8; i += 256) {
                 const int rr = i >> 3, c = (i & 7) * 8;
@@ -542,7 +544,8 @@ int mamba2_fwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     if (!p.res_D) return launch_chunk_fwd<0>(p, stream);
-    return p.res_f32 ? launch_chunk_fwd<2>(p, stream) : launch_chunk_fwd<1>(p, stream);
+    if (p.res_f32) return launch_chunk_fwd<2>(p, stream);
+    return p.res_round ? launch_chunk_fwd<3>(p, stream) : launch_chunk_fwd<1>(p, stream);
 }
 
 }  // namespace llattn

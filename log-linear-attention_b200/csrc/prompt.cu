@@ -4,98 +4,90 @@
 // chunks, steps the remaining tokens one by one and rebuilds the levels inside the last chunk (postprocess_prefill_hstate_,
 // :378-466), and the torch operators around it (hattention/mamba_apis.py:346-399, gated_delta_rule_apis.py:65-92).
 //
-// Here the tensors that the chunkwise kernels read are written Tp >= T tokens long by the pass that prepares them anyway.  A
-// token of zeros (k, v, beta zero, log decay zero) leaves every level state as it is and its output rows are not used, so the
-// chunkwise kernels cover the whole prompt and no token is stepped: a 1000-token prompt of 48 heads is eight launches instead
-// of forty decode steps behind the chunkwise launches.
-#include "llattn_common.cuh"
+// Here the whole chunks of a prompt go through the chunkwise kernels and the n < 64 tokens behind them (its tail) through one kernel that
+// keeps in fp32 what a decode step keeps in fp32, for all of them at once.  The tensors that the passes read hold the B T0 tokens of whole
+// chunks first and the B n tails behind them, so that each part is a plain tensor of its own; for one sequence, or without a tail,
+// that is how they are stored anyway.
+#include "rowwise.cuh"
 #include "../../include/llattn.h"
 
 namespace llattn {
 
-__device__ __forceinline__ float softplus_p(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
+// place of token (b, t) in those tensors
+__device__ __forceinline__ long split_token(unsigned b, unsigned t, int B, int T0, int n) {
+    return t < (unsigned)T0 ? (long)b * T0 + t : (long)B * T0 + (long)b * n + (t - T0);
+}
 
-// ---- log-linear Mamba-2: the preparation of mamba_prep.cu with the padding of v, g, lambda, q and k in the same launch.
-// LPR lanes per (b, t, h) row of the padded tensors; the blocks behind those of the rows copy q and k (16 bytes a thread).
+// ---- log-linear Mamba-2: what torch's operators make of x, dt, A, dl and L before the scan of a prompt: dt + bias rounded to bf16 unless the
+// bias is fp32, softplus and A dt in fp32, lambda rounded at every operator.  LPR lanes per (b, t, h) row; the blocks behind those of the rows
+// copy q and k (16 bytes a thread) where several sequences have tails.
 template <int LPR>
 __global__ void __launch_bounds__(256) m2_prompt_prep_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dt_raw, const void* __restrict__ dt_bias, int bias_f32,
                                                              const float* __restrict__ A, const bf16* __restrict__ dl, const void* __restrict__ Lp, int lp_f32,
                                                              const uint4* __restrict__ q, const uint4* __restrict__ k, bf16* __restrict__ v,
-                                                             float* __restrict__ g, bf16* __restrict__ lam, uint4* __restrict__ qp, uint4* __restrict__ kp,
-                                                             int B, int T, int Tp, int H, int P, int L, int Lo, int mode, int row_blocks, int qk16) {
+                                                             float* __restrict__ g, bf16* __restrict__ lam, uint4* __restrict__ qs, uint4* __restrict__ ks,
+                                                             int B, int T0, int n, int H, int P, int L, int mode, int row_blocks, int qk16) {
     chain_wait();
+    const unsigned T = T0 + n;
     if ((int)blockIdx.x >= row_blocks) {
         // qk16: 16-byte words of a token of q (and of k)
         const unsigned e = (blockIdx.x - row_blocks) * 256u + threadIdx.x;
-        const unsigned n = (unsigned)B * Tp * qk16;
-        if (e >= 2u * n) return;
-        const bool is_k = e >= n;
-        const unsigned i = is_k ? e - n : e;
-        const unsigned c = i % qk16, tok = i / qk16, t = tok % Tp, b = tok / Tp;
-        uint4 w = make_uint4(0, 0, 0, 0);
-        if (t < (unsigned)T) w = (is_k ? k : q)[((long)b * T + t) * qk16 + c];
-        (is_k ? kp : qp)[i] = w;
+        const unsigned all = (unsigned)B * T * qk16;
+        if (e >= 2u * all) return;
+        const bool is_k = e >= all;
+        const unsigned i = is_k ? e - all : e;
+        const unsigned c = i % qk16, tok = i / qk16;
+        (is_k ? ks : qs)[split_token(tok / T, tok % T, B, T0, n) * qk16 + c] = (is_k ? k : q)[i];
         return;
     }
     const int lane = threadIdx.x % LPR;
     const unsigned row = (blockIdx.x * 256u + threadIdx.x) / LPR;
-    if (row >= (unsigned)B * Tp * H) return;
+    if (row >= (unsigned)B * T * H) return;
     const int h = row % H;
-    const unsigned tok = row / H, t = tok % Tp, b = tok / Tp;
-    const bool in = t < (unsigned)T;
-    const long src = in ? ((long)b * T + t) * H + h : 0;
-    float dt = 0.f;
-    if (in) {
-        dt = __bfloat162float(dt_raw[src]);
-        if (dt_bias) dt += load_param(dt_bias, h, bias_f32);
-        dt = softplus_p(dt);
+    const unsigned tok = row / H;
+    const long dst = split_token(tok / T, tok % T, B, T0, n) * H + h;
+    float dt = __bfloat162float(dt_raw[row]);
+    if (dt_bias) {
+        dt += load_param(dt_bias, h, bias_f32);
+        if (!bias_f32) dt = round_bf16(dt);
     }
-    if (lane == 0) g[row] = in ? A[h] * dt : 0.f;
+    dt = softplus_torch(dt);
+    if (lane == 0) g[dst] = A[h] * dt;
     if (lane * 8 < P) {
-        uint4 out = make_uint4(0, 0, 0, 0);
-        if (in) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(x + src * P + lane * 8);
-            const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&raw);
-            uint32_t* o = reinterpret_cast<uint32_t*>(&out);
+        uint4 out;
+        const uint4 raw = *reinterpret_cast<const uint4*>(x + (long)row * P + lane * 8);
+        const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&raw);
+        uint32_t* o = reinterpret_cast<uint32_t*>(&out);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = pack_bf16(__bfloat162float(hx[i].x) * dt, __bfloat162float(hx[i].y) * dt);
-        }
-        *reinterpret_cast<uint4*>(v + (long)row * P + lane * 8) = out;
+        for (int i = 0; i < 4; ++i) o[i] = pack_bf16(__bfloat162float(hx[i].x) * dt, __bfloat162float(hx[i].y) * dt);
+        *reinterpret_cast<uint4*>(v + dst * P + lane * 8) = out;
     }
-    for (int j = lane; j < Lo; j += LPR) {
-        float r = 0.f;
-        if (in && j < L) {
-            const float lp = load_param(Lp, h * L + j, lp_f32), d = __bfloat162float(dl[src * L + j]);
-            if (mode == 0) r = softplus_p(lp * d);
-            else if (mode == 1) r = __expf(-__expf(lp) * softplus_p(d));
-            else r = lp * d;
-        }
-        lam[(long)row * Lo + j] = __float2bfloat16(r);
-    }
+    for (int j = lane; j < L; j += LPR)
+        lam[dst * L + j] = __float2bfloat16(lambda_torch(mode, load_param(Lp, h * L + j, lp_f32), __bfloat162float(dl[(long)row * L + j])));
 }
 
-// y = o + D x for the T tokens of x; o is Tp tokens long; y has the dtype of D (bf16 without D).  P / 8 threads a row.
+// y = o + D x for the whole chunks: T0 tokens of each sequence of o, the first T0 of the T0 + n of those of x and y; y has the dtype of D, and
+// a bf16 D x is rounded before the sum, as two operators would.  P / 8 threads a row.
 template <bool F32OUT>
 __global__ void __launch_bounds__(256) m2_prompt_residual_kernel(const bf16* __restrict__ o, const bf16* __restrict__ x, const void* __restrict__ D,
-                                                                 void* __restrict__ y, int B, int T, int Tp, int H, int P) {
+                                                                 void* __restrict__ y, int B, int T0, int n, int H, int P) {
     chain_wait();
     const unsigned p8 = P / 8;
     const unsigned e = blockIdx.x * 256u + threadIdx.x;
     const unsigned row = e / p8, c = (e % p8) * 8;
-    if (row >= (unsigned)B * T * H) return;
-    const unsigned h = row % H, tok = row / H, t = tok % T, b = tok / T;
-    const long at = (long)row * P + c;
-    const uint4 ro = *reinterpret_cast<const uint4*>(o + (((long)b * Tp + t) * H + h) * P + c);
-    uint4 rx = make_uint4(0, 0, 0, 0);
-    if (D) rx = *reinterpret_cast<const uint4*>(x + at);
-    const float d = D ? load_param(D, h, F32OUT) : 0.f;
+    if (row >= (unsigned)B * T0 * H) return;
+    const unsigned h = row % H, tok = row / H, t = tok % T0, b = tok / T0;
+    const long at = (((long)b * (T0 + n) + t) * H + h) * P + c;
+    const uint4 ro = *reinterpret_cast<const uint4*>(o + (long)row * P + c), rx = *reinterpret_cast<const uint4*>(x + at);
+    const float d = load_param(D, h, F32OUT);
     const __nv_bfloat162* ho = reinterpret_cast<const __nv_bfloat162*>(&ro);
     const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&rx);
     float r[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        r[2 * i] = __bfloat162float(ho[i].x) + __bfloat162float(hx[i].x) * d;
-        r[2 * i + 1] = __bfloat162float(ho[i].y) + __bfloat162float(hx[i].y) * d;
+        const float x0 = __bfloat162float(hx[i].x) * d, x1 = __bfloat162float(hx[i].y) * d;
+        r[2 * i] = __bfloat162float(ho[i].x) + (F32OUT ? x0 : round_bf16(x0));
+        r[2 * i + 1] = __bfloat162float(ho[i].y) + (F32OUT ? x1 : round_bf16(x1));
     }
     if (F32OUT) {
         float* w = reinterpret_cast<float*>(y) + at;
@@ -108,31 +100,6 @@ __global__ void __launch_bounds__(256) m2_prompt_residual_kernel(const bf16* __r
         for (int i = 0; i < 4; ++i) w[i] = pack_bf16(r[2 * i], r[2 * i + 1]);
         *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(y) + at) = out;
     }
-}
-
-// ---- token-padded copies of up to eight (B, T, ...) tensors in one launch
-struct PadList {
-    const void* src[8];
-    void* dst[8];
-    int src_bytes[8], dst_bytes[8];     // bytes of a token (the rest of a longer destination row is zero)
-    int unit[8];                        // copy unit: 16, 4 or 2 bytes
-    unsigned first_block[9];
-    int n, B, T, Tp;
-};
-
-__global__ void __launch_bounds__(256) pad_tokens_kernel(const __grid_constant__ PadList l) {
-    chain_wait();
-    int i = 0;
-    while (i + 1 < l.n && blockIdx.x >= l.first_block[i + 1]) ++i;
-    const unsigned per = l.dst_bytes[i] / l.unit[i], real = l.src_bytes[i] / l.unit[i];
-    const unsigned long e = (unsigned long)(blockIdx.x - l.first_block[i]) * 256u + threadIdx.x;
-    if (e >= (unsigned long)l.B * l.Tp * per) return;
-    const unsigned c = (unsigned)(e % per), tok = (unsigned)(e / per), t = tok % l.Tp, b = tok / l.Tp;
-    const bool in = t < (unsigned)l.T && c < real;
-    const unsigned long s = ((unsigned long)b * l.T + t) * real + c;
-    if (l.unit[i] == 16) reinterpret_cast<uint4*>(l.dst[i])[e] = in ? reinterpret_cast<const uint4*>(l.src[i])[s] : make_uint4(0, 0, 0, 0);
-    else if (l.unit[i] == 4) reinterpret_cast<uint32_t*>(l.dst[i])[e] = in ? reinterpret_cast<const uint32_t*>(l.src[i])[s] : 0u;
-    else reinterpret_cast<unsigned short*>(l.dst[i])[e] = in ? reinterpret_cast<const unsigned short*>(l.src[i])[s] : (unsigned short)0;
 }
 
 // ---- Gated DeltaNet: q, k normalised (q scaled), widened to Ko columns and expanded to one per head, lambda scaled, and every
@@ -377,23 +344,23 @@ __global__ void __launch_bounds__(128) gdn_tail_states_kernel(const bf16* __rest
 extern "C" {
 
 int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_bias, int bias_is_f32, const float* A, const void* dl, const void* Lp,
-                              int lp_is_f32, const void* q, const void* k, void* v, float* g, void* lambda, void* q_pad, void* k_pad,
-                              int B, int T, int Tp, int H, int G, int K, int P, int L, int L_out, int lambda_mode, void* stream) {
-    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || G <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+                              int lp_is_f32, const void* q, const void* k, void* v, float* g, void* lambda, void* q_split, void* k_split,
+                              int B, int T, int tail, int H, int G, int K, int P, int L, int lambda_mode, void* stream) {
+    if (B <= 0 || T < 0 || tail < 0 || T + tail <= 0 || H <= 0 || G <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (P <= 0 || P > 256 || P % 8 != 0 || (G * K) % 8 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (L <= 0 || L > 64 || L_out < L || L_out > 64 || lambda_mode < 0 || lambda_mode > 2) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (L <= 0 || L > 64 || lambda_mode < 0 || lambda_mode > 2) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!x || !dt_raw || !A || !dl || !Lp || !v || !g || !lambda) return LLATTN_ERR_NULL;
-    if ((q_pad != nullptr) != (k_pad != nullptr) || (q_pad && (!q || !k))) return LLATTN_ERR_NULL;
+    if ((q_split != nullptr) != (k_split != nullptr) || (q_split && (!q || !k))) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
-    const long rows = (long)B * Tp * H;
+    const long rows = (long)B * (T + tail) * H;
     const int lpr = P <= 64 ? 8 : (P <= 128 ? 16 : 32);
     const int qk16 = G * K / 8;
-    const long copies = q_pad ? 2l * B * Tp * qk16 : 0;
+    const long copies = q_split ? 2l * B * (T + tail) * qk16 : 0;
     if (rows * lpr > 0x7fffff00l || copies > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     const int row_blocks = (int)((rows * lpr + 255) / 256);
     const unsigned grid = row_blocks + (unsigned)((copies + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
-#define LLATTN_PP(N) llattn::launch_chained(llattn::m2_prompt_prep_kernel<N>, grid, 256, 0, st, (const bf*)x, (const bf*)dt_raw, dt_bias, bias_is_f32, A, (const bf*)dl, Lp, lp_is_f32, (const uint4*)q, (const uint4*)k, (bf*)v, g, (bf*)lambda, (uint4*)q_pad, (uint4*)k_pad, B, T, Tp, H, P, L, L_out, lambda_mode, row_blocks, qk16)
+#define LLATTN_PP(N) llattn::launch_chained(llattn::m2_prompt_prep_kernel<N>, grid, 256, 0, st, (const bf*)x, (const bf*)dt_raw, dt_bias, bias_is_f32, A, (const bf*)dl, Lp, lp_is_f32, (const uint4*)q, (const uint4*)k, (bf*)v, g, (bf*)lambda, (uint4*)q_split, (uint4*)k_split, B, T, tail, H, P, L, lambda_mode, row_blocks, qk16)
     if (lpr == 8) LLATTN_PP(8);
     else if (lpr == 16) LLATTN_PP(16);
     else LLATTN_PP(32);
@@ -402,37 +369,14 @@ int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_
     return (int)cudaGetLastError();
 }
 
-int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, void* y, int y_is_f32, int B, int T, int Tp, int H, int P, void* stream) {
-    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || P <= 0 || P % 8 != 0 || (long)B * T * H * P > 0x7fffff00l * 8) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (!o || !y || (D && !x)) return LLATTN_ERR_NULL;
+int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, void* y, int y_is_f32, int B, int T, int tail, int H, int P, void* stream) {
+    if (B <= 0 || T <= 0 || tail < 0 || H <= 0 || P <= 0 || P % 8 != 0 || (long)B * T * H * P > 0x7fffff00l * 8) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!o || !y || !D || !x) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
     const unsigned grid = (unsigned)(((long)B * T * H * (P / 8) + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
-    if (y_is_f32) llattn::launch_chained(llattn::m2_prompt_residual_kernel<true>, grid, 256, 0, st, (const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
-    else llattn::launch_chained(llattn::m2_prompt_residual_kernel<false>, grid, 256, 0, st, (const bf*)o, (const bf*)x, D, y, B, T, Tp, H, P);
-    LLATTN_LAUNCHED();
-    return (int)cudaGetLastError();
-}
-
-int llattn_pad_tokens(int n, const void* const* src, void* const* dst, const int* src_bytes, const int* dst_bytes, int B, int T, int Tp,
-                      void* stream) {
-    if (n <= 0 || n > 8 || B <= 0 || T <= 0 || Tp < T || (long)B * Tp > 0x7fffffffl) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    llattn::PadList l = {};
-    l.n = n; l.B = B; l.T = T; l.Tp = Tp;
-    unsigned long blocks = 0;
-    for (int i = 0; i < n; ++i) {
-        if (!src[i] || !dst[i]) return LLATTN_ERR_NULL;
-        if (src_bytes[i] <= 0 || dst_bytes[i] < src_bytes[i]) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-        const size_t all = (size_t)src[i] | (size_t)dst[i] | (size_t)src_bytes[i] | (size_t)dst_bytes[i];
-        l.unit[i] = (all & 15) == 0 ? 16 : ((all & 3) == 0 ? 4 : 2);
-        if (all & 1) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-        l.src[i] = src[i]; l.dst[i] = dst[i]; l.src_bytes[i] = src_bytes[i]; l.dst_bytes[i] = dst_bytes[i];
-        l.first_block[i] = (unsigned)blocks;
-        blocks += ((unsigned long)B * Tp * (dst_bytes[i] / l.unit[i]) + 255) / 256;
-    }
-    if (blocks > 0x7ffffffful) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    l.first_block[n] = (unsigned)blocks;
-    llattn::launch_chained(llattn::pad_tokens_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, l);
+    if (y_is_f32) llattn::launch_chained(llattn::m2_prompt_residual_kernel<true>, grid, 256, 0, st, (const bf*)o, (const bf*)x, D, y, B, T, tail, H, P);
+    else llattn::launch_chained(llattn::m2_prompt_residual_kernel<false>, grid, 256, 0, st, (const bf*)o, (const bf*)x, D, y, B, T, tail, H, P);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

@@ -10,6 +10,16 @@ __device__ __forceinline__ float softplus_row(float x) { return x > 20.f ? x : l
 __device__ __forceinline__ float sigmoid_row(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
+// What torch's operators on bf16 tensors give, each result rounded to bf16: the inference calls (prompts, decode steps) keep these rounding
+// points of the operator sequence around the recurrence.
+__device__ __forceinline__ float softplus_torch(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+__device__ __forceinline__ float lambda_torch(int mode, float lp, float d) {
+    lp = round_bf16(lp);
+    if (mode == 0) return round_bf16(softplus_torch(round_bf16(lp * d)));
+    if (mode == 1) return round_bf16(expf(round_bf16(-round_bf16(expf(lp)) * round_bf16(softplus_torch(d)))));
+    return round_bf16(lp * d);
+}
+
 // N consecutive bf16 values as packed words; `vec`: the address is a multiple of the words' size
 template <int N>
 struct Packed {

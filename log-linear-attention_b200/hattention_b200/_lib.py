@@ -73,8 +73,6 @@ def lib():
     for name, args in {
         "llattn_mamba2_layer_step": [_P] * 8 + [_I, _P, _I, _P, _I] + [_P] * 2 + [_I] * 6 + [_U] + [_I] * 4 + [_P],
         "llattn_gdn_layer_step": [_P] * 8 + [_I] * 6 + [_U, _I, _I, _F, _F, _I, _P],
-        "llattn_pad_tokens": [_I] + [_P] * 4 + [_I] * 3 + [_P],
-        "llattn_mamba2_prompt_states": [_P] * 5 + [ctypes.c_size_t] + [_I] * 8 + [_P],
     }.items():
         fn = getattr(L, name)
         fn.restype, fn.argtypes = _I, args

@@ -4,14 +4,12 @@ reference's `hattention/chunkwise.py` (`chunkwise_fwd` :1118-1129, `chunkwise_bw
 The work is done by libllattn.so; these functions validate arguments the way the reference
 does, allocate outputs and scratch with torch, and launch on the current CUDA stream.
 """
-import ctypes
 from typing import Optional, Tuple
 
 import torch
 
 from . import _lib
 from .base import HType, ceil_log, get_num_levels
-from .recurrent import level_major_states
 
 CHUNK = 64
 
@@ -119,55 +117,22 @@ def final_states(k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, L: int) -> t
     return st
 
 
-def pad_tokens(tensors, widths, B: int, T: int, Tp: int):
-    """Contiguous (B,T,...) tensors copied to (B,Tp,...), zeros behind the T tokens, in one launch; `widths`: values of a
-    token in each copy (at least as many as in the tensor; the rest are zero)."""
-    n = len(tensors)
-    out = [torch.empty(B, Tp, w, dtype=x.dtype, device=x.device) for x, w in zip(tensors, widths)]
-    ptrs, ints = ctypes.c_void_p * n, ctypes.c_int * n
-    rc = _lib.lib().llattn_pad_tokens(
-        n, ptrs(*(x.data_ptr() for x in tensors)), ptrs(*(x.data_ptr() for x in out)),
-        ints(*(x.numel() // (B * T) * x.element_size() for x in tensors)), ints(*(w * x.element_size() for x, w in zip(out, widths))),
-        B, T, Tp, _stream())
-    _lib.check(rc, "llattn_pad_tokens")
-    return out
-
-
-def prompt_forward_padded(q, k, v, g, l, T: int, L: int, level_base: int, htype: HType, chunk_size: int):
-    """Outputs (B,Tp,H,V) and the level states after the first T of Tp tokens (the others are zero), level-major, for the L levels
-    that the caller asked for (the columns of `l` beyond them are zero)."""
-    B, Tp, H, G, K, V, Lp = _check(q, k, v, g, l, False, level_base, htype, chunk_size)
-    if 1 + (T - 1).bit_length() > L:
-        raise ValueError("more tokens than the levels can hold")
-    kept = []
-    o, _, _ = chunkwise_fwd(q, k, v, g, l, False, level_base, htype, chunk_size, False, keep_workspace=kept)
-    states = level_major_states((B, H, K, V, L), q.device)
-    rc = _lib.lib().llattn_mamba2_prompt_states(k.data_ptr(), v.data_ptr(), g.data_ptr(), states.data_ptr(), kept[0].data_ptr(),
-                                                kept[0].numel(), B, T, Tp, H, G, K, V, L, _stream())
-    _lib.check(rc, "llattn_mamba2_prompt_states")
-    return o, states
-
-
 def prompt_forward(q, k, v, g, l, level_base: int, htype: HType, chunk_size: int):
-    """Outputs (B,T,H,V) and level states (B,H,K,V,L) after a prompt of any length."""
-    B, T, G, K = k.shape
-    H, V = v.shape[2:]
-    L = l.shape[-1]
-    if T < CHUNK:
-        q, k, v = (x.to(torch.bfloat16) for x in (q, k, v))
-    elif not (q.dtype == k.dtype == v.dtype == torch.bfloat16):
-        raise NotImplementedError(f"q / k / v must be bfloat16 (got {q.dtype}, {k.dtype}, {v.dtype})")
-    Tp, Lo = -(-T // CHUNK) * CHUNK, max(L, get_num_levels(CHUNK, 2) if T < CHUNK else 0)
-    with torch.cuda.device(q.device):
-        q_, k_, v_, l_ = (_as(x, torch.bfloat16) for x in (q, k, v, l))
-        g_ = _as(g, torch.float32)
-        if Tp != T:
-            q_, k_, v_, g_, l_ = pad_tokens((q_, k_, v_, g_, l_), (G * K, G * K, H * V, H, H * L), B, T, Tp)
-            q_, k_, v_, l_ = q_.view(B, Tp, G, K), k_.view(B, Tp, G, K), v_.view(B, Tp, H, V), l_.view(B, Tp, H, L)
-        if Lo != L:
-            l_ = torch.nn.functional.pad(l_, (0, Lo - L))
-        o, states = prompt_forward_padded(q_, k_, v_, g_, l_, T, L, level_base, htype, chunk_size)
-    return (o if Tp == T else o[:, :T].contiguous()), states
+    """Outputs (B,T,H,V) and level states (B,H,K,V,L), level-major, after a prompt of any length: the whole chunks through the chunkwise
+    kernels, the tokens behind them (fp32 states and products, as decode steps have) in one kernel."""
+    T = k.shape[1]
+    T0 = T - T % CHUNK
+    if T0:
+        _check(q[:, :T0], k[:, :T0], v[:, :T0], g[:, :T0], l[:, :T0], False, level_base, htype, chunk_size)
+    elif level_base != 2 or htype != HType.WEAK:
+        raise NotImplementedError
+    if 1 + (T - 1).bit_length() > l.shape[-1]:
+        raise ValueError("more tokens than the levels can hold")
+    bf = torch.bfloat16
+    r = _lib.host().mamba2_prefill(q.to(bf), k.to(bf), v.to(bf), g.to(torch.float32), l.to(bf), _lib.CHECK_STATUS)
+    if r is None:
+        raise ValueError("unsupported prompt (K 64 or 128, V 64, at most 32 levels, consistent shapes on one CUDA device)")
+    return r
 
 
 def chunkwise_bwd(

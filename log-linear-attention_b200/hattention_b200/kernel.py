@@ -244,9 +244,9 @@ def gdn_layer_step(hstate: HState, q, k, v, b, g, l, scale: Optional[float] = No
 def hattention_prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct,
                        chunk_size: Optional[int] = None, use_qk_l2norm_in_kernel: bool = False):
     """Outputs for a prompt and the level states to continue from, signature of the reference's
-    `hattention_prefill` (kernel.py:469-560).  The whole prompt goes through the chunkwise kernels, on tensors padded
-    with zero tokens where its length is not a number of chunks; the level states come from one more kernel.  Shapes
-    that the chunkwise kernels do not take and that are shorter than a chunk are stepped token by token."""
+    `hattention_prefill` (kernel.py:469-560).  The whole chunks of the prompt go through the chunkwise kernels; the
+    tokens behind them keep the fp32 states and products of decode steps, in kernels that take all of them at once.
+    Shapes that those kernels do not take and that are shorter than a chunk are stepped token by token."""
     return prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chunk_size, use_qk_l2norm_in_kernel)
 
 
@@ -266,7 +266,7 @@ def prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chu
             raise ValueError
         if use_qk_l2norm_in_kernel or scale is not None:
             raise NotImplementedError
-        chunkwise = T >= chunk_size or (K in (64, 128) and V == 64)
+        chunkwise = T >= chunk_size or (chunk_size == 64 and K in (64, 128) and V == 64)
     else:
         if b is None:
             raise ValueError
