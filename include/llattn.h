@@ -253,24 +253,22 @@ int llattn_mamba2_prompt_tail(const void* q, const void* k, const void* v, const
                               int y_is_f32, void* y, float* states, int state_levels, float* tail_part, int B, int T, int tail, int H, int G, int K,
                               int V, int L, void* stream);
 
-/* Delta-rule prompts run the chunkwise kernels on tensors of Tp >= T tokens whose last Tp - T tokens are zero (they leave the states as
- * they are).
- *   gdn_prompt_prep: a value head of V columns as `rep` heads of V / rep columns that share everything else ((B,T,H,V) is (B,T,H rep,V / rep)
- *     in memory).  One row per part: l2norm of q (scaled) and k, K_out >= K columns wide (at most 128), and, each where its pointer is given,
- *     v, beta and g, lambda (times lambda_mul unless 0, L_out columns), all Tp tokens long.  q, k have G groups of H / G heads.
- *   gdn_prefill_parts: llattn_gdn_prefill on H = heads x rep parts, the inter-chunk levels written into level-major states
- *     (B,H / rep,state_levels,state_rows,rep V); other levels are left alone
- *   gdn_prompt_states: advances those levels by the tokens of the last chunk and writes the levels inside it, so that every level is as of
- *     token T - 1; kn (B,Tp,H,128), v (B,Tp,H,V), states (B,H / rep,L,K,rep V); T is in the last 64 tokens of Tp */
+/*   gdn_prompt_prep: a value head of V columns as `rep` heads of V / rep columns that share everything else ((B,T,H,V) is (B,T,H rep,V / rep)
+ *     in memory).  Split, one row per part: l2norm of q (scaled) and k, K_out >= K columns wide (at most 128), and, each where its pointer is
+ *     given, v, beta and g, lambda (times lambda_mul unless 0).  q, k have G groups of H / G heads.
+ *   gdn_prompt: outputs and level states of a prompt from those: heads counts parts, V (64 or 128) the columns of one.  o_chunks
+ *     (B,T,heads,V) receives the whole chunks' outputs (g_cum, Aw, Au of them as in llattn_gdn_fwd; none of these is used for T = 0), o
+ *     (B,T+tail,heads,V) those of the tail (o_chunks may be o for B = 1 or without a tail); states level-major (B,heads / rep,state_levels,
+ *     state_rows,rep V), every level written; scratch (16-byte aligned) for a tail only. */
 int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
-                           void* qn, void* kn, void* v_pad, void* beta_pad, float* g_pad, void* lambda_pad,
-                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int rep, int L, int L_out, float scale,
-                           float lambda_mul, void* stream);
-int llattn_gdn_prefill_parts(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
-                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int rep, int state_levels,
-                             void* workspace, size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream);
-int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, const float* g, float* states, int B, int T, int Tp, int H,
-                             int K, int V, int rep, int L, void* stream);
+                           void* qn, void* kn, void* v_split, void* beta_split, float* g_split, void* lambda_split,
+                           int B, int T, int tail, int H, int G, int K, int K_out, int V, int rep, int L, float scale, float lambda_mul,
+                           void* stream);
+size_t llattn_gdn_prompt_scratch_bytes(int B, int T, int tail, int heads, int rep, int V);
+int llattn_gdn_prompt(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda, void* o_chunks, void* o,
+                      float* g_cum, void* Aw, void* Au, float* states, int state_rows, int rep, int state_levels, void* scratch,
+                      size_t scratch_bytes, void* workspace, size_t workspace_bytes, int B, int T, int tail, int heads, int K, int V, int L,
+                      void* stream);
 
 /* Log-linear Gated DeltaNet forward.  Replaces hattention.chunkwise_hgdn.chunkwise_fwd
  * (hattention/chunkwise_hgdn.py:566-788) with output_final_state=False.  q and k are per head,

@@ -359,23 +359,61 @@ size_t llattn_gdn_fwd_keep_workspace_bytes(int B, int T, int H, int K, int V, in
 static int gdn_fwd_impl(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                         void* o, float* g_cum, void* Aw, void* Au, void* workspace, size_t workspace_bytes,
                         int B, int T, int H, int K, int V, int L, void* stream, bool keep,
-                        const llattn::GdnStateOut& final_states = llattn::GdnStateOut{});
+                        const llattn::GdnStateOut& final_states = llattn::GdnStateOut{}, llattn::GdnTail* tail = nullptr);
 
-int llattn_gdn_prefill_parts(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
-                             void* o, float* g_cum, void* Aw, void* Au, float* states, int state_rows, int rep, int state_levels,
-                             void* workspace, size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream) {
-    if (!states) return LLATTN_ERR_NULL;
-    if (state_rows <= 0 || state_rows > K || rep <= 0 || H % rep != 0 || state_levels > L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    llattn::GdnStateOut out;
-    out.p = states;
-    out.rows = state_rows;
-    out.rep = rep;
-    out.part = V;
-    out.col = 1;
-    out.row = (long)rep * V;
-    out.level = (long)state_rows * out.row;
-    out.bh = out.level * state_levels;
-    return gdn_fwd_impl(q, k, v, beta, g, lambda, o, g_cum, Aw, Au, workspace, workspace_bytes, B, T, H, K, V, L, stream, false, out);
+static int gdn_prompt_check(int B, int T, int tail, int heads, int rep, int K, int V, int state_levels) {
+    if (B <= 0 || heads <= 0 || rep <= 0 || heads % rep != 0 || K <= 0 || K > 128 || (V != 64 && V != 128)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (T < 0 || T % 64 != 0 || tail < 0 || tail >= 64 || T + tail <= 0) return LLATTN_ERR_BAD_LENGTH;
+    if (state_levels > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    const int m = T + tail - 1;
+    if (state_levels < 1 + (m > 0 ? 32 - __builtin_clz((unsigned)m) : 0)) return LLATTN_ERR_TOO_FEW_LEVELS;
+    return 0;
+}
+
+size_t llattn_gdn_prompt_scratch_bytes(int B, int T, int tail, int heads, int rep, int V) {
+    if (B <= 0 || T < 0 || tail <= 0 || heads <= 0 || rep <= 0 || V <= 0) return 0;
+    return sizeof(float) * llattn::gdn_tail_scratch_floats(B, T, tail, heads / rep, V * rep);
+}
+
+int llattn_gdn_prompt(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda, void* o_chunks, void* o,
+                      float* g_cum, void* Aw, void* Au, float* states, int state_rows, int rep, int state_levels, void* scratch, size_t scratch_bytes,
+                      void* workspace, size_t workspace_bytes, int B, int T, int tail, int heads, int K, int V, int L, void* stream) {
+    int rc = gdn_prompt_check(B, T, tail, heads, rep, state_rows, V, state_levels);
+    if (rc != 0) return rc;
+    if (K != 128 || L != state_levels) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!q || !k || !v || !beta || !g || !lambda || !o || !states) return LLATTN_ERR_NULL;
+    const int H = heads / rep;
+    cudaStream_t st = (cudaStream_t)stream;
+    using bf = __nv_bfloat16;
+    llattn::GdnTail t = {};
+    if (tail > 0) {
+        if (!scratch || ((uintptr_t)scratch & 15) || scratch_bytes < sizeof(float) * llattn::gdn_tail_scratch_floats(B, T, tail, H, V * rep))
+            return LLATTN_ERR_WORKSPACE;
+        if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)states) & 15 || (uintptr_t)o & 7) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+        t.q = (const bf*)q; t.k = (const bf*)k; t.v = (const bf*)v; t.beta = (const bf*)beta; t.lam = (const bf*)lambda; t.g = g;
+        t.o = (bf*)o; t.states = states;
+        t.B = B; t.T0 = T; t.n = tail; t.H = H; t.rep = rep; t.K = state_rows; t.V = V * rep; t.L = state_levels;
+        llattn::gdn_tail_scratch(t, (float*)scratch);
+    }
+    if (T > 0) {
+        llattn::GdnStateOut out;
+        out.p = states;
+        out.rows = state_rows;
+        out.rep = rep;
+        out.part = V;
+        out.col = 1;
+        out.row = (long)rep * V;
+        out.level = (long)state_rows * out.row;
+        out.bh = out.level * state_levels;
+        rc = gdn_fwd_impl(q, k, v, beta, g, lambda, o_chunks, g_cum, Aw, Au, workspace, workspace_bytes, B, T, heads, K, V, L, stream, false, out,
+                          tail > 0 ? &t : nullptr);
+        const int rj = llattn::gdn_tail_join(t, st);
+        if (rc != 0 || rj != 0) return rc != 0 ? rc : rj;
+        if (tail == 0)
+            return llattn::gdn_prompt_states_launch((const bf*)k, (const bf*)v, (const bf*)beta, g, states, B, T, heads, state_rows, V, rep, state_levels, st);
+        return llattn::gdn_tail_apply_launch(t, st);
+    }
+    return llattn::gdn_tail_prep_launch(t, st);
 }
 
 int llattn_gdn_prefill(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
@@ -410,7 +448,7 @@ int llattn_gdn_fwd_keep(const void* q, const void* k, const void* v, const void*
 
 static int gdn_fwd_impl(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
                         void* o, float* g_cum, void* Aw, void* Au, void* workspace, size_t workspace_bytes,
-                        int B, int T, int H, int K, int V, int L, void* stream, bool keep, const llattn::GdnStateOut& final_states) {
+                        int B, int T, int H, int K, int V, int L, void* stream, bool keep, const llattn::GdnStateOut& final_states, llattn::GdnTail* tail) {
     int rc = gdn_check(B, T, H, K, V, L);
     if (rc != 0) return rc;
     if (!q || !k || !v || !beta || !g || !lambda || !o || !g_cum || !Aw || !Au) return LLATTN_ERR_NULL;
@@ -424,6 +462,7 @@ static int gdn_fwd_impl(const void* q, const void* k, const void* v, const void*
     p.beta = (const __nv_bfloat16*)beta; p.g = g; p.l = (const __nv_bfloat16*)lambda;
     p.o = (__nv_bfloat16*)o; p.g_cum = g_cum; p.Aw = (__nv_bfloat16*)Aw; p.Au = (__nv_bfloat16*)Au;
     p.final_states = final_states;
+    p.tail = tail;
     cudaError_t e0 = cudaMemsetAsync(p.err, 0, sizeof(int), (cudaStream_t)stream);
     if (e0 != cudaSuccess) return (int)e0;
     return keep ? llattn::gdn_fwd_keep_dispatch(p, (cudaStream_t)stream) : llattn::gdn_fwd_dispatch(p, (cudaStream_t)stream);

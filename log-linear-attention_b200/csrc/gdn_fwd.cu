@@ -672,6 +672,10 @@ static int launch_gdn_fwd(const GdnParams& p, cudaStream_t stream) {
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
         llattn::launch_chained(kern, p.B * p.NT * p.H, 256, sm, stream, p); LLATTN_LAUNCHED();
     }
+    if (!BWD && p.tail) {
+        const int rc = gdn_tail_prep_launch(*p.tail, stream);
+        if (rc != 0) return rc;
+    }
     if (KD == 128 && g_use_tensor_core_path.load()) return gdn_scan_tc_dispatch(p, BWD ? 2 : (KEEP ? 1 : 0), stream);
     {
         auto kern = gdn_scan_kernel<KD, BWD || KEEP, !BWD>;

@@ -29,7 +29,7 @@ using torch::autograd::variable_list;
     F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mamba2_prompt_tail) F(llattn_mamba2_residual) F(llattn_mixer_prep_fwd)            \
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
     F(llattn_gdn_fwd_workspace_bytes) F(llattn_gdn_fwd_keep_workspace_bytes) F(llattn_gdn_fwd) F(llattn_gdn_fwd_keep)                \
-    F(llattn_gdn_prefill_parts) F(llattn_gdn_prompt_states) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
+    F(llattn_gdn_prompt) F(llattn_gdn_prompt_scratch_bytes) F(llattn_gdn_bwd_workspace_bytes) F(llattn_gdn_bwd)                      \
     F(llattn_gdn_bwd_kept_workspace_bytes) F(llattn_gdn_bwd_kept_bf16dv) F(llattn_gdn_bwd_kept_normed) F(llattn_gdn_grad_out) F(llattn_workspace_status) F(llattn_clear)
 
 struct Library {
@@ -496,30 +496,30 @@ struct GdnInputs {
     }
 };
 
-// l2norm of q and k, lambda times its factor, the parts of wide heads and (T < Tp) padding; what none of these changes is used as it is
-GdnInputs gdn_prepare(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, int T, int Tp, int Lo, double scale,
+// l2norm of q and k, lambda times its factor, the parts of wide heads, split into T0 tokens of whole chunks and n others where several sequences
+// have both; what none of these changes is used as it is
+GdnInputs gdn_prepare(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, int T0, int n, double scale,
                       double lam_mul, void* stream) {
     GdnInputs a;
     a.B = q.size(0);
-    a.T = Tp;
+    a.T = T0 + n;
     a.G = q.size(2);
     a.K = q.size(3);
     a.H = v.size(2);
     a.V = v.size(3);
-    a.L = Lo;
+    a.L = l.size(3);
     a.split();
-    const int B = a.B, H = a.heads(), L = l.size(3);
-    const bool pad = Tp != T, own = pad || a.rep > 1, own_l = own || lam_mul != 0.0 || Lo != L;
-    a.qn = empty({B, Tp, H, GDN_K}, at::kBFloat16, q);
+    const int B = a.B, H = a.heads(), T = a.T, L = a.L;
+    const bool split = B > 1 && T0 > 0 && n > 0, own = split || a.rep > 1, own_l = own || lam_mul != 0.0;
+    a.qn = empty({B, T, H, GDN_K}, at::kBFloat16, q);
     a.kn = contiguous_like(a.qn);
-    a.v = pad ? empty({B, Tp, H, a.width}, at::kBFloat16, q) : v;
-    a.b = own ? empty({B, Tp, H}, at::kBFloat16, q) : b;
-    a.g = own ? empty({B, Tp, H}, at::kFloat, q) : g;
-    a.l = own_l ? empty({B, Tp, H, Lo}, at::kBFloat16, q) : l;
+    a.v = split ? empty({B, T, H, a.width}, at::kBFloat16, q) : v;
+    a.b = own ? empty({B, T, H}, at::kBFloat16, q) : b;
+    a.g = own ? empty({B, T, H}, at::kFloat, q) : g;
+    a.l = own_l ? empty({B, T, H, L}, at::kBFloat16, q) : l;
     check(lib.llattn_gdn_prompt_prep(q.data_ptr(), k.data_ptr(), v.data_ptr(), b.data_ptr(), fptr(g), l.data_ptr(), a.qn.data_ptr(), a.kn.data_ptr(),
-                                     pad ? a.v.data_ptr() : nullptr, own ? a.b.data_ptr() : nullptr, own ? fptr(a.g) : nullptr,
-                                     own_l ? a.l.data_ptr() : nullptr, B, T, Tp, a.H, a.G, a.K, GDN_K, a.V, a.rep, L, Lo, (float)scale, (float)lam_mul,
-                                     stream),
+                                     split ? a.v.data_ptr() : nullptr, own ? a.b.data_ptr() : nullptr, own ? fptr(a.g) : nullptr,
+                                     own_l ? a.l.data_ptr() : nullptr, B, T0, n, a.H, a.G, a.K, GDN_K, a.V, a.rep, L, (float)scale, (float)lam_mul, stream),
           "llattn_gdn_prompt_prep");
     return a;
 }
@@ -540,7 +540,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
         On on(q);
         const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), b_ = b.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
         const int T = q.size(1);
-        GdnInputs a = gdn_prepare(q_, k_, v_, b_, g_, l_, T, T, l.size(3), scale, lam_mul, on.stream);
+        GdnInputs a = gdn_prepare(q_, k_, v_, b_, g_, l_, T, 0, scale, lam_mul, on.stream);
         const int B = a.B, H = a.heads(), V = a.width;
         const size_t keep_need = lib.llattn_gdn_fwd_keep_workspace_bytes(B, T, H, GDN_K, V, a.L);
         const bool keep = ctx != nullptr && (int64_t)keep_need <= keep_bytes;
@@ -585,7 +585,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
             qn = empty({B, T, H, GDN_K}, at::kBFloat16, q);
             kn = contiguous_like(qn);
             check(lib.llattn_gdn_prompt_prep(q.data_ptr(), k.data_ptr(), nullptr, nullptr, nullptr, nullptr, qn.data_ptr(), kn.data_ptr(), nullptr, nullptr,
-                                             nullptr, nullptr, B, T, T, a.H, a.H, a.K, GDN_K, a.V, a.rep, a.L, a.L, (float)scale, 0.f, on.stream),
+                                             nullptr, nullptr, B, T, 0, a.H, a.H, a.K, GDN_K, a.V, a.rep, a.L, (float)scale, 0.f, on.stream),
                   "llattn_gdn_prompt_prep");
         }
         const Tensor d_o = d[0].to(at::kBFloat16).contiguous();
@@ -656,28 +656,38 @@ py::object hattention_gdn(const Tensor& q, const Tensor& k, const Tensor& v, con
 py::object gdn_prompt(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, double scale, double lam_mul,
                       bool status) {
     if (!gdn_operands(q, k, v, b, g, l)) return py::none();
-    const int T = q.size(1), L = l.size(3), Tp = (T + 63) / 64 * 64, Lo = T < 64 ? std::max(L, 7) : L;
-    if (Tp > 16384 || L < 1 + bit_length(T - 1) || Lo < 7 + ceil_log2(Tp / 64)) return py::none();
+    const int T = q.size(1), L = l.size(3), T0 = T / 64 * 64, n = T % 64;
+    if (T0 > 16384 || L < 1 + bit_length(T - 1)) return py::none();
     Tensor o, states;
     {
         py::gil_scoped_release nogil;
         at::NoGradGuard no_grad;
         On on(q);
-        GdnInputs a = gdn_prepare(q.contiguous(), k.contiguous(), v.contiguous(), b.contiguous(), g.contiguous(), l.contiguous(), T, Tp, Lo, scale, lam_mul,
+        GdnInputs a = gdn_prepare(q.contiguous(), k.contiguous(), v.contiguous(), b.contiguous(), g.contiguous(), l.contiguous(), T0, n, scale, lam_mul,
                                   on.stream);
         const int B = a.B, H = a.heads(), K = a.K, V = a.width;
         states = empty({B, a.H, L, K, a.V}, at::kFloat, q);
-        const Tensor g_cum = contiguous_like(a.g), Aw = empty({B, Tp, H, 64}, at::kBFloat16, q), Au = contiguous_like(Aw), out = empty({B, Tp, a.H, a.V}, at::kBFloat16, q);
-        const size_t bytes = lib.llattn_gdn_fwd_workspace_bytes(B, Tp, H, GDN_K, V, Lo);
-        const Tensor ws = empty({(int64_t)bytes}, at::kByte, q);
-        check(lib.llattn_gdn_prefill_parts(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(), out.data_ptr(),
-                                           fptr(g_cum), Aw.data_ptr(), Au.data_ptr(), fptr(states), K, a.rep, L, ws.data_ptr(), bytes,
-                                           B, Tp, H, GDN_K, V, Lo, on.stream),
-              "llattn_gdn_prefill_parts");
-        check(lib.llattn_gdn_prompt_states(a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), fptr(states), B, T, Tp, H, K, V, a.rep, L, on.stream),
-              "llattn_gdn_prompt_states");
-        if (status) check_status(ws, on.stream, "llattn_gdn_prefill_parts");
-        o = Tp == T ? out : out.narrow(1, 0, T).contiguous();
+        o = empty({B, T, a.H, a.V}, at::kBFloat16, q);
+        Tensor chunks = o, g_cum, Aw, Au, ws, scratch;
+        size_t bytes = 0, more = 0;
+        if (T0 > 0) {
+            if (n > 0 && B > 1) chunks = empty({B, T0, a.H, a.V}, at::kBFloat16, q);
+            g_cum = empty({B, T0, H}, at::kFloat, q);
+            Aw = empty({B, T0, H, 64}, at::kBFloat16, q);
+            Au = contiguous_like(Aw);
+            bytes = lib.llattn_gdn_fwd_workspace_bytes(B, T0, H, GDN_K, V, L);
+            ws = empty({(int64_t)bytes}, at::kByte, q);
+        }
+        if (n > 0) {
+            more = lib.llattn_gdn_prompt_scratch_bytes(B, T0, n, H, a.rep, V);
+            scratch = empty({(int64_t)more}, at::kByte, q);
+        }
+        check(lib.llattn_gdn_prompt(a.qn.data_ptr(), a.kn.data_ptr(), a.v.data_ptr(), a.b.data_ptr(), fptr(a.g), a.l.data_ptr(), chunks.data_ptr(),
+                                    o.data_ptr(), fptr(g_cum), ptr(Aw), ptr(Au), fptr(states), K, a.rep, L, ptr(scratch), more, ptr(ws), bytes, B, T0, n, H,
+                                    GDN_K, V, L, on.stream),
+              "llattn_gdn_prompt");
+        if (status && T0 > 0) check_status(ws, on.stream, "llattn_gdn_prompt");
+        if (chunks.data_ptr() != o.data_ptr()) o.narrow(1, 0, T0).copy_(chunks);
         states = states.permute({0, 1, 3, 4, 2});
     }
     return py::make_tuple(o, states);

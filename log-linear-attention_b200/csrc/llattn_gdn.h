@@ -20,6 +20,21 @@ struct GdnStateOut {
     int rows = 0, rep = 1;
 };
 
+class SideStream;
+
+// The tokens of a prompt behind its last whole chunk (gdn_tail.cu).  H counts whole heads of V columns, rep parts each; the tensors hold the B T0 tokens of
+// whole chunks first and the B n others behind them, rows of H rep parts (v and o: of H heads, the same memory).
+struct GdnTail {
+    const __nv_bfloat16 *q, *k;  // normalised (q scaled), 128 columns
+    const __nv_bfloat16 *v, *beta, *lam;
+    const float* g;
+    __nv_bfloat16* o;            // (B,T0+n,H,V)
+    float* states;               // (B,H,L,K,V): in, the levels of whole chunks before the last of them; out, all levels after the last token
+    float *scratch, *writes, *part;
+    int B, T0, n, H, rep, K, V, L;
+    SideStream* side = nullptr;  // host: where the preparation runs
+};
+
 struct GdnParams {
     // inputs (q, k already L2-normalised / scaled by the caller, one q/k per head)
     const __nv_bfloat16* q;      // (B,T,H,K)
@@ -32,6 +47,7 @@ struct GdnParams {
     __nv_bfloat16* o;            // (B,T,H,V)
     float* g_cum;                // (B,T,H)
     GdnStateOut final_states;    // optional, fp32: level states as of the start of the last chunk
+    GdnTail* tail = nullptr;     // host: a prompt's tail, prepared beside the scan
     __nv_bfloat16* Aw;           // (B,T,H,64)  (I + A)^-1 rows, saved for the backward
     __nv_bfloat16* Au;           // (B,T,H,64)  (I + A*Gamma)^-1 rows
     // scratch written by the chunk preparation, read by the scan
@@ -71,6 +87,13 @@ struct GdnParams {
     alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_qd, tm_wd, tm_kd, tm_wk, tm_u, tm_do, tm_hs, tm_dhs, tm_dqd, tm_dwd, tm_dkd;
 };
 
+size_t gdn_tail_scratch_floats(int B, int T0, int n, int H, int V);
+void gdn_tail_scratch(GdnTail& a, float* base);                           // sets the three scratch pointers
+int gdn_tail_prep_launch(GdnTail& a, cudaStream_t stream);                // on a side stream where there is one: join before the apply
+int gdn_tail_join(const GdnTail& a, cudaStream_t stream);
+int gdn_tail_apply_launch(const GdnTail& a, cudaStream_t stream);
+int gdn_prompt_states_launch(const __nv_bfloat16* kn, const __nv_bfloat16* v, const __nv_bfloat16* beta, const float* g, float* states, int B, int T, int H,
+                             int K, int V, int rep, int L, cudaStream_t stream);
 bool gdn_bwd_levels_writes_row_terms(const GdnParams& p);
 int gdn_fwd_dispatch(const GdnParams& p, cudaStream_t stream);
 int gdn_fwd_keep_dispatch(const GdnParams& p, cudaStream_t stream);

@@ -8,8 +8,8 @@
 // keeps in fp32 what a decode step keeps in fp32, for all of them at once.  The tensors that the passes read hold the B T0 tokens of whole
 // chunks first and the B n tails behind them, so that each part is a plain tensor of its own; for one sequence, or without a tail,
 // that is how they are stored anyway.
+#include "llattn_gdn.h"
 #include "rowwise.cuh"
-#include "../../include/llattn.h"
 
 namespace llattn {
 
@@ -102,20 +102,20 @@ __global__ void __launch_bounds__(256) m2_prompt_residual_kernel(const bf16* __r
     }
 }
 
-// ---- Gated DeltaNet: q, k normalised (q scaled), widened to Ko columns and expanded to one per head, lambda scaled, and every
-// tensor padded to Tp tokens, in one launch.  16 lanes per (b, t, h) row.
+// ---- Gated DeltaNet: q, k normalised (q scaled), widened to Ko columns and expanded to one per head, lambda scaled, split into whole chunks and
+// tails, in one launch.  16 lanes per (b, t, h) row.
 struct GdnPrepArgs {
     const bf16 *q, *k;       // (B,T,G,K)
     const bf16 *v;           // (B,T,H,V)
     const bf16* beta;        // (B,T,H)
     const float* g;          // (B,T,H)
     const bf16* l;           // (B,T,H,L)
-    // results, one row per part of a head: a value head of V columns is `rep` heads of V / rep columns that share q, k, beta, g, lambda
-    bf16 *qn, *kn;           // (B,Tp,H rep,Ko)
-    bf16 *vp, *bp;           // (B,Tp,H rep,V / rep), (B,Tp,H rep)
-    float* gp;               // (B,Tp,H rep)
-    bf16* lp;                // (B,Tp,H rep,Lo)
-    int B, T, Tp, H, G, K, Ko, V, rep, L, Lo;
+    // results, split, one row per part of a head: a value head of V columns is `rep` heads of V / rep columns that share q, k, beta, g, lambda
+    bf16 *qn, *kn;           // (B,T,H rep,Ko)
+    bf16 *vp, *bp;           // (B,T,H rep,V / rep), (B,T,H rep)
+    float* gp;               // (B,T,H rep)
+    bf16* lp;                // (B,T,H rep,Lo)
+    int B, T0, n, H, G, K, Ko, V, rep, L;
     float scale, lam_mul;    // lam_mul = 0: lambda as it is
 };
 
@@ -123,18 +123,18 @@ __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_const
     chain_wait();
     const int lane = threadIdx.x & 15;
     const unsigned row = blockIdx.x * 16u + (threadIdx.x >> 4);
-    const unsigned heads = a.H * a.rep, rows = (unsigned)a.B * a.Tp * heads;
+    const unsigned heads = a.H * a.rep, T = a.T0 + a.n, rows = (unsigned)a.B * T * heads;
     const bool have = row < rows;
-    const unsigned hp = row % heads, h = hp / a.rep, part = hp % a.rep, tok = row / heads, t = tok % a.Tp, b = tok / a.Tp;
-    const bool in = have && t < (unsigned)a.T;
-    const long tr = in ? (long)b * a.T + t : 0;
+    const unsigned hp = row % heads, h = hp / a.rep, part = hp % a.rep, tok = row / heads;
+    const long dst = split_token(tok / T, tok % T, a.B, a.T0, a.n) * heads + hp;
+    const long tr = have ? tok : 0;
     const long src = tr * a.H + h, qsrc = tr * a.G + h / (a.H / a.G);
     uint4 raw[2];
     float rstd[2];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
         raw[w] = make_uint4(0, 0, 0, 0);
-        if (in && lane * 8 < a.K) raw[w] = *reinterpret_cast<const uint4*>((w ? a.k : a.q) + qsrc * a.K + lane * 8);
+        if (have && lane * 8 < a.K) raw[w] = *reinterpret_cast<const uint4*>((w ? a.k : a.q) + qsrc * a.K + lane * 8);
         const __nv_bfloat162* f = reinterpret_cast<const __nv_bfloat162*>(&raw[w]);
         float ss = 0.f;
 #pragma unroll
@@ -158,34 +158,29 @@ __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_const
                 o[i] = __floats2bfloat162_rn(__bfloat162float(f[i].x) * rstd[w], __bfloat162float(f[i].y) * rstd[w]);
                 if (w == 0) o[i] = __floats2bfloat162_rn(__bfloat162float(o[i].x) * a.scale, __bfloat162float(o[i].y) * a.scale);
             }
-            *reinterpret_cast<uint4*>((w ? a.kn : a.qn) + (long)row * a.Ko + lane * 8) = out;
+            *reinterpret_cast<uint4*>((w ? a.kn : a.qn) + dst * a.Ko + lane * 8) = out;
         }
     }
     if (a.vp) {
         const int width = a.V / a.rep;
         for (int c = lane * 8; c < width; c += 128) {
-            uint4 w = make_uint4(0, 0, 0, 0);
-            if (in) w = *reinterpret_cast<const uint4*>(a.v + src * a.V + part * width + c);
-            *reinterpret_cast<uint4*>(a.vp + (long)row * width + c) = w;
+            *reinterpret_cast<uint4*>(a.vp + dst * width + c) = *reinterpret_cast<const uint4*>(a.v + src * a.V + part * width + c);
         }
     }
     if (a.lp)
-        for (int j = lane; j < a.Lo; j += 16) {
-            float x = 0.f;
-            if (in && j < a.L) {
-                x = __bfloat162float(a.l[src * a.L + j]);
-                if (a.lam_mul != 0.f) x *= a.lam_mul;
-            }
-            a.lp[(long)row * a.Lo + j] = __float2bfloat16(x);
+        for (int j = lane; j < a.L; j += 16) {
+            float x = __bfloat162float(a.l[src * a.L + j]);
+            if (a.lam_mul != 0.f) x *= a.lam_mul;
+            a.lp[dst * a.L + j] = __float2bfloat16(x);
         }
     if (lane == 0 && a.gp) {
-        a.gp[row] = in ? a.g[src] : 0.f;
-        a.bp[row] = in ? a.beta[src] : __float2bfloat16(0.f);
+        a.gp[dst] = a.g[src];
+        a.bp[dst] = a.beta[src];
     }
 }
 
-// ---- Gated DeltaNet: the level states after the last token of a prompt.  The scan over chunks leaves the inter-chunk levels as
-// they stand before the last chunk; the tokens of that chunk advance them, and build the levels inside it.  Every level is
+// ---- Gated DeltaNet: the level states after the last token of a prompt without a tail (gdn_tail.cu has the others).  The scan over chunks leaves the
+// inter-chunk levels as they stand before the last chunk; the tokens of that chunk advance them, and build the levels inside it.  Every level is
 // independent of the others: level 0 is the last token alone, level j + 1 (for each set bit j of the last token's position in
 // the chunk) starts from zero at the first of its 2^j tokens, takes their writes and then the transitions of the tokens behind
 // them, and the levels of earlier chunks take the transitions of all.  fp32 throughout, as the decode kernel steps.
@@ -197,31 +192,10 @@ __global__ void __launch_bounds__(256) gdn_prompt_prep_kernel(const __grid_const
 // was bound by the twenty shuffles of a token: T = 827, 59 tokens, 16 heads of 128 x 128 31 us, now 24; T = 777, 9 tokens, 12.1 and 8.6.)
 // Four warps a CTA; grid (B*H, 64-column blocks, levels).
 constexpr int TAIL_KD = 128, TAIL_COLS = 64;
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 x) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 
 __global__ void __launch_bounds__(128) gdn_tail_states_kernel(const bf16* __restrict__ kn, const bf16* __restrict__ v, const bf16* __restrict__ beta,
-                                                              const float* __restrict__ g, float* __restrict__ states, int T, int Tp, int H,
-                                                              int K, int Vs, int rep, int L, unsigned live) {
+                                                              const float* __restrict__ g, float* __restrict__ states, int T, int H, int K, int Vs,
+                                                              int rep, int L, unsigned live) {
     chain_wait();
     __shared__ __align__(16) bf16 sK[CH * TAIL_KD];
     __shared__ __align__(16) float sV[CH * TAIL_COLS];
@@ -273,7 +247,7 @@ __global__ void __launch_bounds__(128) gdn_tail_states_kernel(const bf16* __rest
         s[1][i] = pack2(x[0].y, x[1].y);
     }
     if (s0 >= 0) {
-        const long t0 = (long)b * Tp + c0;
+        const long t0 = (long)b * T + c0;
         for (int e = tid; e < n * (TAIL_KD / 8); e += 128) {
             const int i = e / (TAIL_KD / 8), c8 = (e % (TAIL_KD / 8)) * 8;
             *reinterpret_cast<uint4*>(sK + i * TAIL_KD + c8) = *reinterpret_cast<const uint4*>(kn + ((t0 + i) * H + h) * TAIL_KD + c8);
@@ -339,6 +313,14 @@ __global__ void __launch_bounds__(128) gdn_tail_states_kernel(const bf16* __rest
     }
 }
 
+int gdn_prompt_states_launch(const bf16* kn, const bf16* v, const bf16* beta, const float* g, float* states, int B, int T, int H, int K, int V, int rep,
+                             int L, cudaStream_t stream) {
+    dim3 grid(B * H, (V + TAIL_COLS - 1) / TAIL_COLS, L);
+    launch_chained(gdn_tail_states_kernel, grid, 128, 0, stream, kn, v, beta, g, states, T, H, K, V, rep, L, 1u | (unsigned)(T - 1) << 1);
+    LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
+}
+
 }  // namespace llattn
 
 extern "C" {
@@ -382,33 +364,18 @@ int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, v
 }
 
 int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const void* beta, const float* g, const void* lambda,
-                           void* qn, void* kn, void* v_pad, void* beta_pad, float* g_pad, void* lambda_pad,
-                           int B, int T, int Tp, int H, int G, int K, int K_out, int V, int rep, int L, int L_out, float scale,
-                           float lambda_mul, void* stream) {
-    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || G <= 0 || H % G != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+                           void* qn, void* kn, void* v_split, void* beta_split, float* g_split, void* lambda_split,
+                           int B, int T, int tail, int H, int G, int K, int K_out, int V, int rep, int L, float scale, float lambda_mul, void* stream) {
+    if (B <= 0 || T < 0 || tail < 0 || T + tail <= 0 || H <= 0 || G <= 0 || H % G != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (K <= 0 || K % 8 != 0 || K_out < K || K_out > 128 || K_out % 8 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (V <= 0 || rep <= 0 || V % (8 * rep) != 0 || L <= 0 || L_out < L) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if ((long)B * Tp * H * rep > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (!q || !k || !qn || !kn || (v_pad && !v) || (lambda_pad && !lambda) || (g_pad && (!g || !beta || !beta_pad))) return LLATTN_ERR_NULL;
+    if (V <= 0 || rep <= 0 || V % (8 * rep) != 0 || L <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if ((long)B * (T + tail) * H * rep > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (!q || !k || !qn || !kn || (v_split && !v) || (lambda_split && !lambda) || (g_split && (!g || !beta || !beta_split))) return LLATTN_ERR_NULL;
     using bf = __nv_bfloat16;
-    llattn::GdnPrepArgs a{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, (const bf*)lambda, (bf*)qn, (bf*)kn, (bf*)v_pad,
-                          (bf*)beta_pad, g_pad, (bf*)lambda_pad, B, T, Tp, H, G, K, K_out, V, rep, L, L_out, scale, lambda_mul};
-    const unsigned grid = (unsigned)(((long)B * Tp * H * rep + 15) / 16);
+    llattn::GdnPrepArgs a{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, (const bf*)lambda, (bf*)qn, (bf*)kn, (bf*)v_split,
+                          (bf*)beta_split, g_split, (bf*)lambda_split, B, T, tail, H, G, K, K_out, V, rep, L, scale, lambda_mul};
+    const unsigned grid = (unsigned)(((long)B * (T + tail) * H * rep + 15) / 16);
     llattn::launch_chained(llattn::gdn_prompt_prep_kernel, grid, 256, 0, (cudaStream_t)stream, a);
-    LLATTN_LAUNCHED();
-    return (int)cudaGetLastError();
-}
-
-int llattn_gdn_prompt_states(const void* kn, const void* v, const void* beta, const float* g, float* states, int B, int T, int Tp, int H,
-                             int K, int V, int rep, int L, void* stream) {
-    if (B <= 0 || T <= 0 || Tp < T || H <= 0 || rep <= 0 || H % rep != 0 || K <= 0 || K > llattn::TAIL_KD) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (V <= 0 || V % 32 != 0 || L <= 0 || L > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (T > 1 && L < 1 + (32 - __builtin_clz((unsigned)(T - 1) | 1u))) return LLATTN_ERR_TOO_FEW_LEVELS;
-    if (!kn || !v || !beta || !g || !states) return LLATTN_ERR_NULL;
-    using bf = __nv_bfloat16;
-    dim3 grid(B * H, (V + llattn::TAIL_COLS - 1) / llattn::TAIL_COLS, L);
-    llattn::launch_chained(llattn::gdn_tail_states_kernel, grid, 128, 0, (cudaStream_t)stream, (const bf*)kn, (const bf*)v, (const bf*)beta, g,
-            states, T, Tp, H, K, V, rep, L, 1u | (unsigned)(T - 1) << 1);
     LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }

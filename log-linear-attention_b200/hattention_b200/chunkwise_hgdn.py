@@ -227,17 +227,19 @@ def chunkwise_bwd(q, k, v, b, g, l, Aw, Au, do, head_first, level_base, htype, c
 
 def prompt_forward(q, k, v, b, g, l, scale, head_first, level_base: int, htype: HType, chunk_size: int, lambda_mul: float = 0.0):
     """Outputs (B,T,H,V) and level states (B,H,K,V,L), level-major, after a prompt of any length: q, k raw (normalised here, q also
-    scaled), l multiplied by lambda_mul unless that is 0.  The tensors are padded with zero tokens to whole chunks by the pass that
-    normalises q and k; the scan over chunks leaves the inter-chunk levels, and one kernel advances them by the last chunk's tokens
-    and builds the levels inside it."""
+    scaled), l multiplied by lambda_mul unless that is 0.  The whole chunks go through the chunkwise kernels; the states are carried over the
+    last of them and over the tokens behind it in fp32, as decode steps do, and those tokens' outputs come from these states."""
+    if head_first or level_base != 2 or htype != HType.WEAK or chunk_size != CHUNK:
+        raise NotImplementedError
     bf = torch.bfloat16
     r = _lib.host().gdn_prompt(q.to(bf), k.to(bf), v.to(bf), b.to(bf), g.to(torch.float32), l.to(bf), scale, lambda_mul, _lib.CHECK_STATUS)
     if r is None:
-        T = q.shape[1]
-        _check(q[:, :T // CHUNK * CHUNK], k[:, :T // CHUNK * CHUNK], v, b[:, :T // CHUNK * CHUNK], g[:, :T // CHUNK * CHUNK],
-               l[:, :T // CHUNK * CHUNK], head_first, level_base, htype, chunk_size)
+        T = q.shape[1] // CHUNK * CHUNK
+        if T:
+            _check(q[:, :T], k[:, :T], v, b[:, :T], g[:, :T], l[:, :T], head_first, level_base, htype, chunk_size)
         _v_slices(v.shape[-1])
-        raise ValueError("unsupported GDN prompt (K at most 128 and a multiple of 8, V a multiple of 64, T <= 16384, enough lambda levels)")
+        raise ValueError("unsupported GDN prompt (K at most 128 and a multiple of 8, V a multiple of 64, at most 16384 tokens of whole "
+                         "chunks, enough lambda levels)")
     return r
 
 

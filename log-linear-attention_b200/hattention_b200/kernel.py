@@ -272,7 +272,7 @@ def prefill(q, k, v, b, g, l, scale, head_first, level_base, htype, hstruct, chu
             raise ValueError
         if not use_qk_l2norm_in_kernel or scale is None:
             raise NotImplementedError
-        chunkwise = T >= chunk_size or (K <= 128 and V % 64 == 0 and V <= 384)
+        chunkwise = T >= chunk_size or (chunk_size == 64 and K <= 128 and V % 64 == 0 and V <= 384)
     ragged = T % chunk_size != 0
     if (ragged or hstruct == HStruct.GDELTA) and not (q.dtype == k.dtype == v.dtype == l.dtype):
         raise TypeError

@@ -75,3 +75,45 @@ def test_layer_prompt_rounds_like_the_torch_operators(B, T, mode, params):
     # the same operands but for the last bit of the exponentials' fp32 values: a value in a few hundred falls on the other side of a rounding
     assert rel(y, yt) < 5e-4
     assert rel(s.states, st.states) < 5e-4
+
+
+# tails of one token, of 63; no whole chunk, one, an odd number, a power of two; narrow keys, parts of wide values, several sequences
+@pytest.mark.parametrize("B,T,H,Dk,Dv", [(1, 1, 2, 128, 128), (2, 63, 2, 64, 64), (1, 65, 2, 128, 128), (3, 90, 2, 128, 64), (1, 255, 2, 128, 192),
+                                         (1, 330, 2, 96, 256), (2, 521, 2, 128, 128), (1, 800, 2, 128, 64), (1, 1050, 1, 128, 384)])
+def test_gdn_tail_keeps_fp32(B, T, H, Dk, Dv):
+    from hattention_b200.gated_delta_rule_apis import chunk_h_gated_delta_rule
+    L, T0 = 13, T // 64 * 64
+    q, k, v, b, g, l = orc.make_gdn_inputs(B, T, H, Dk, Dv, L, seed=T)
+    q, k, v, b, l = (x.bfloat16().float() for x in (q, k, v, b, l))
+    scale = Dk ** -0.5
+    d = lambda x: x.bfloat16().to(DEV)
+    o, hs = chunk_h_gated_delta_rule(d(q), d(k), d(v), g.float().to(DEV), d(l), d(b), output_final_state=True, use_qk_l2norm_in_kernel=True)
+    # the recurrence on the rounded operands that a step takes
+    from hattention_b200.chunkwise_hgdn import l2norm_fwd
+    qn, kn = l2norm_fwd(d(q), scale).double().cpu(), l2norm_fwd(d(k)).double().cpu()
+    want, st = orc.recurrent(qn, kn, v.double(), g.double(), (d(l) / scale).double().cpu(), b=b.double())
+    assert o.is_contiguous() and hs.counts == list(st.counts)
+    states = torch.stack(st.states, dim=-1)
+    if T0 < T:
+        # one rounding to bf16 (the chunkwise kernels are at 3.4e-3 here), and the levels below a chunk in fp32
+        assert rel(o[:, T0:], want[:, T0:]) < 2.5e-3
+        assert rel(hs.states[..., :7], states[..., :7]) < 2e-6
+        if T0:
+            # the lowest level above them holds the last whole chunk, in fp32; what the others have from the scan is decayed by then
+            N = T0 // 64
+            low = 7 + (N & -N).bit_length() - 1
+            if N % 2:
+                assert rel(hs.states[..., low], states[..., low]) < 2e-6
+            assert rel(hs.states[..., 7:], states[..., 7:]) < 2e-3
+
+
+def test_gdn_tail_after_a_decay_to_nothing():
+    """A log decay of -inf among the tokens behind the last whole chunk empties every level and leaves no NaN."""
+    from hattention_b200.gated_delta_rule_apis import chunk_h_gated_delta_rule
+    q, k, v, b, g, l = orc.make_gdn_inputs(1, 70, 2, 128, 64, 9, seed=0)
+    d = lambda x: x.bfloat16().to(DEV)
+    g = g.float().to(DEV)
+    g[:, 67] = float("-inf")
+    o, hs = chunk_h_gated_delta_rule(d(q), d(k), d(v), g, d(l), d(b), output_final_state=True, use_qk_l2norm_in_kernel=True)
+    assert torch.isfinite(o).all() and torch.isfinite(hs.states).all()
+    assert (hs.states[..., 7:] == 0).all()
