@@ -36,6 +36,7 @@ extern "C" {
 #define LLATTN_ERR_NULL (-6)                /* a required pointer is NULL                    */
 #define LLATTN_ERR_STATIC_SCRATCH (-7)      /* problem needs more than LLATTN_STATIC_SCRATCH_BYTES */
 #define LLATTN_ERR_TENSOR_MAP (-8)          /* the driver refused a TMA tensor map for these pointers */
+#define LLATTN_ERR_ALIGNMENT (-9)           /* a pointer that the kernels access in 16-byte words */
 
 /* Size of the built-in scratch array used by llattn_mamba2_fwd_static (16 MiB). */
 #define LLATTN_STATIC_SCRATCH_BYTES (16u << 20)

@@ -1,6 +1,7 @@
 // extern "C" entry points of libllattn.so: argument checks, workspace carving, launches.
 #include <stdint.h>
 
+#include "launch_cache.h"
 #include "llattn_gdn.h"
 #include "llattn_mamba2.h"
 #include "llattn_testing.h"
@@ -134,6 +135,8 @@ static int mamba2_fwd_impl(llattn::Mamba2Params& p, const void* q, const void* k
     int rc = check_shape(B, T, H, G, K, V, L);
     if (rc != 0) return rc;
     if (!q || !k || !v || !g || !lambda || (!o && !p.res_D) || !g_cum) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {q, k, v})) return LLATTN_ERR_ALIGNMENT;
+    p.o = (__nv_bfloat16*)o;
     p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
     if (p.res_D && !llattn::mamba2_uses_tc(p)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (p.oT == 0) p.oT = T;
@@ -160,7 +163,7 @@ int llattn_mamba2_fwd_residual(const void* q, const void* k, const void* v, cons
                                int B, int T, int H, int G, int K, int V, int L, void* stream) {
     if (!x || !D || !y) return LLATTN_ERR_NULL;
     if (T_y <= 0 || T_y > T) return LLATTN_ERR_BAD_LENGTH;
-    if (((uintptr_t)x & 15) || ((uintptr_t)y & 31)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (llattn::misaligned(16, {x}) || llattn::misaligned(32, {y})) return LLATTN_ERR_ALIGNMENT;
     llattn::Mamba2Params p = {};
     p.res_x = (const __nv_bfloat16*)x; p.res_D = D; p.res_y = y; p.res_T = p.res_n = T_y; p.res_f32 = y_is_f32;
     return mamba2_fwd_impl(p, q, k, v, g, lambda, nullptr, g_cum, workspace, workspace_bytes, B, T, H, G, K, V, L, stream);
@@ -171,7 +174,7 @@ int llattn_mamba2_fwd_prompt(const void* q, const void* k, const void* v, const 
                              void* workspace, size_t workspace_bytes, int B, int T, int H, int G, int K, int V, int L, void* stream) {
     if (!y || !states || (D && !x) || (tail > 0 && !tail_part)) return LLATTN_ERR_NULL;
     if (T <= 0 || tail < 0 || tail >= llattn_chunk()) return LLATTN_ERR_BAD_LENGTH;
-    if (D && (((uintptr_t)x & 15) || ((uintptr_t)y & 31))) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (llattn::misaligned(16, {x, y, states, tail_part}) || (D && llattn::misaligned(32, {y}))) return LLATTN_ERR_ALIGNMENT;
     const int rc = llattn::mamba2_prompt_states_check(B, T + tail, H, G, K, V, state_levels);
     if (rc != 0) return rc;
     llattn::Mamba2Params p = {};
@@ -204,6 +207,7 @@ int llattn_mamba2_fwd_static(const void* q, const void* k, const void* v, const 
     int rc = check_shape(B, T, H, G, K, V, L);
     if (rc != 0) return rc;
     if (!q || !k || !v || !g || !lambda || !o || !g_cum) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {q, k, v})) return LLATTN_ERR_ALIGNMENT;
     llattn::Mamba2Params p = {};
     p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
     const size_t need = setup(p, nullptr, false);
@@ -254,6 +258,7 @@ static int mamba2_bwd_impl(const void* q, const void* k, const void* v, const fl
     int rc = check_shape(B, T, H, G, K, V, L);
     if (rc != 0) return rc;
     if (!q || !k || !v || !g_cum || !lambda || !d_o || !dq || !dk || !dv || !dg || !dlambda) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {q, k, v, d_o}) || llattn::misaligned(8, {dq, dk})) return LLATTN_ERR_ALIGNMENT;
     llattn::Mamba2Params p = {};
     p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
     const size_t need = setup(p, nullptr, true);
@@ -389,7 +394,7 @@ int llattn_gdn_prompt(const void* q, const void* k, const void* v, const void* b
     if (tail > 0) {
         if (!scratch || ((uintptr_t)scratch & 15) || scratch_bytes < sizeof(float) * llattn::gdn_tail_scratch_floats(B, T, tail, H, V * rep))
             return LLATTN_ERR_WORKSPACE;
-        if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)states) & 15 || (uintptr_t)o & 7) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+        if (llattn::misaligned(16, {q, k, v, states}) || llattn::misaligned(8, {o})) return LLATTN_ERR_ALIGNMENT;
         t.q = (const bf*)q; t.k = (const bf*)k; t.v = (const bf*)v; t.beta = (const bf*)beta; t.lam = (const bf*)lambda; t.g = g;
         t.o = (bf*)o; t.states = states;
         t.B = B; t.T0 = T; t.n = tail; t.H = H; t.rep = rep; t.K = state_rows; t.V = V * rep; t.L = state_levels;
@@ -600,6 +605,7 @@ int llattn_gdn_bwd_kept_normed(const void* q, const void* k, const void* raw_q, 
                                void* dv_bf16, float* dbeta, float* dg, float* dlambda, const void* fwd_workspace, size_t fwd_workspace_bytes,
                                void* workspace, size_t workspace_bytes, int B, int T, int H, int K, int V, int L, void* stream) {
     if (!fwd_workspace || !dv_bf16 || !raw_q || !raw_k || !gq || !gk) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {raw_q, raw_k, gq, gk})) return LLATTN_ERR_ALIGNMENT;
     const GdnNormOut norm{raw_q, raw_k, gq, gk, scale};
     return gdn_bwd_impl(q, k, v, beta, g_cum, lambda, Aw, Au, d_o, nullptr, nullptr, nullptr, dbeta, dg, dlambda, fwd_workspace,
                         fwd_workspace_bytes, workspace, workspace_bytes, B, T, H, K, V, L, stream, dv_bf16, &norm);

@@ -449,6 +449,7 @@ int llattn_mamba2_layer_step(float* states, const void* q, const void* k, const 
     if (lambda_mode < 0 || lambda_mode > 2) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (carry_level < 0 || carry_level >= L || (L < 32 && (live >> L) != 0)) return LLATTN_ERR_TOO_FEW_LEVELS;
     if (!states || !q || !k || !x || !dl || !y || (!dt && !g) || (dt && !A)) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {states})) return LLATTN_ERR_ALIGNMENT;
     OnDevice on(device);
     if (on.err != cudaSuccess) return (int)on.err;
     using bf = __nv_bfloat16;
@@ -472,6 +473,7 @@ int llattn_gdn_layer_step(float* states, const void* q, const void* k, const voi
     if (K <= 0 || K > 256 || V <= 0 || V % 16 != 0 || L <= 0 || L > 32) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (carry_level < 0 || carry_level >= L || (L < 32 && (live >> L) != 0)) return LLATTN_ERR_TOO_FEW_LEVELS;
     if (!states || !q || !k || !v || !beta || !g || !lambda || !o) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {states}) || llattn::misaligned(8, {v})) return LLATTN_ERR_ALIGNMENT;
     OnDevice on(device);
     if (on.err != cudaSuccess) return (int)on.err;
     using bf = __nv_bfloat16;

@@ -62,7 +62,19 @@ inline bool f32(const Tensor& t) { return t.defined() && t.scalar_type() == at::
 inline bool param(const Tensor& t) { return !t.defined() || (t.is_cuda() && (t.scalar_type() == at::kFloat || t.scalar_type() == at::kBFloat16)); }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
-inline Tensor contiguous(const Tensor& t) { return t.defined() ? t.contiguous() : t; }
+// contiguous, and where the kernels' 16-byte accesses can start: a contiguous view into a larger tensor may start anywhere
+inline bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+inline Tensor contiguous(const Tensor& t) {
+    if (!t.defined()) return t;
+    const Tensor c = t.contiguous();
+    return aligned(c) ? c : c.clone();
+}
+// what a node saved; hooks may hand back any tensor of the same values
+inline variable_list saved(AutogradContext* ctx) {
+    variable_list s = ctx->get_saved_variables();
+    for (Tensor& t : s) t = contiguous(t);
+    return s;
+}
 using Maybe = std::optional<Tensor>;     // a tensor that may be absent: autograd functions take no undefined tensors
 inline Tensor of(const Maybe& t) { return t.has_value() ? *t : Tensor(); }
 inline Tensor empty(at::IntArrayRef size, at::ScalarType dt, const Tensor& like) {
@@ -186,7 +198,7 @@ struct Mamba2Kernel : torch::autograd::Function<Mamba2Kernel> {
     static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool keep,
                           bool status, bool layer) {
         On on(q);
-        const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
+        const Tensor q_ = contiguous(q), k_ = contiguous(k), v_ = contiguous(v), g_ = contiguous(g), l_ = contiguous(l);
         Scan s = mamba2_fwd(q_, k_, v_, g_, l_, on.stream, status);
         if (ctx) {
             ctx->save_for_backward({q_, k_, v_, s.g_cum, l_, keep ? s.ws : Tensor()});
@@ -196,9 +208,9 @@ struct Mamba2Kernel : torch::autograd::Function<Mamba2Kernel> {
         return s.o;
     }
     static variable_list backward(AutogradContext* ctx, variable_list d) {
-        const auto s = ctx->get_saved_variables();
+        const auto s = saved(ctx);
         On on(s[0]);
-        ScanGrads r = mamba2_bwd(s[0], s[1], s[2], s[3], s[4], d[0].to(at::kBFloat16).contiguous(), s[5], on.stream,
+        ScanGrads r = mamba2_bwd(s[0], s[1], s[2], s[3], s[4], contiguous(d[0].to(at::kBFloat16)), s[5], on.stream,
                                  ctx->saved_data["status"].toBool(), ctx->saved_data["layer"].toBool());
         return {r.dq, r.dk, r.dv, r.dg, r.dl.to(at::kBFloat16), Tensor(), Tensor(), Tensor()};
     }
@@ -225,8 +237,8 @@ struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
                           const Tensor& Lp, const Maybe& D, const Maybe& bias, int64_t mode, bool keep, bool status) {
         On on(x);
         const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), L = dl.size(3);
-        const Tensor x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), A_ = A.to(at::kFloat).contiguous(), Lp_ = Lp.contiguous(),
-                     D_ = contiguous(of(D)), b_ = contiguous(of(bias)), q = Cm.contiguous(), k = Bm.contiguous();
+        const Tensor x_ = contiguous(x), dt_ = contiguous(dt), dl_ = contiguous(dl), A_ = contiguous(A.to(at::kFloat)), Lp_ = contiguous(Lp),
+                     D_ = contiguous(of(D)), b_ = contiguous(of(bias)), q = contiguous(Cm), k = contiguous(Bm);
         const Tensor v = contiguous_like(x_), g = empty({B, T, H}, at::kFloat, x), lam = contiguous_like(dl_);
         check(lib.llattn_mamba2_layer_prep_fwd(x_.data_ptr(), dt_.data_ptr(), ptr(b_), f32(b_), fptr(A_), dl_.data_ptr(), Lp_.data_ptr(), f32(Lp_),
                                                v.data_ptr(), fptr(g), lam.data_ptr(), (long)B * T * H, H, P, L, (int)mode, on.stream),
@@ -242,12 +254,12 @@ struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
         return y;
     }
     static variable_list backward(AutogradContext* ctx, variable_list d) {
-        const auto s = ctx->get_saved_variables();
+        const auto s = saved(ctx);
         const Tensor &x = s[0], &dt = s[1], &A = s[2], &k = s[3], &q = s[4], &dl = s[5], &Lp = s[6], &D = s[7], &bias = s[8], &v = s[9], &g_cum = s[10],
                      &lam = s[11], &ws = s[12];
         On on(x);
         const int B = x.size(0), T = x.size(1), H = x.size(2), P = x.size(3), L = dl.size(3);
-        const Tensor dy = d[0].to(at::kBFloat16).contiguous();
+        const Tensor dy = contiguous(d[0].to(at::kBFloat16));
         ScanGrads r = mamba2_bwd(q, k, v, g_cum, lam, dy, ws, on.stream, ctx->saved_data["status"].toBool(), true);
         const Tensor dx = contiguous_like(x), ddt = contiguous_like(dt), ddl = contiguous_like(dl);
         const Tensor acc = zeros(3 * H + (int64_t)H * L, x, on.stream);
@@ -353,9 +365,9 @@ py::object mamba2_prompt(const Tensor& x, const Tensor& dt, const Tensor& A, con
         py::gil_scoped_release nogil;
         at::NoGradGuard no_grad;
         On on(x);
-        const Tensor x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), A_ = A.to(at::kFloat).contiguous(), Lp_ = Lp.contiguous(),
+        const Tensor x_ = contiguous(x), dt_ = contiguous(dt), dl_ = contiguous(dl), A_ = contiguous(A.to(at::kFloat)), Lp_ = contiguous(Lp),
                      D_c = contiguous(D), b_ = contiguous(bias);
-        Tensor q = Cm.contiguous(), k = Bm.contiguous(), qs, ks;
+        Tensor q = contiguous(Cm), k = contiguous(Bm), qs, ks;
         const Tensor v = contiguous_like(x_), g = empty(dt_.sizes(), at::kFloat, x), lam = contiguous_like(dl_);
         if (p.split()) {
             qs = contiguous_like(q);
@@ -391,7 +403,7 @@ py::object mamba2_prefill(const Tensor& q, const Tensor& k, const Tensor& v, con
         py::gil_scoped_release nogil;
         at::NoGradGuard no_grad;
         On on(q);
-        r = p.run(p.parts(q.contiguous()), p.parts(k.contiguous()), p.parts(v.contiguous()), p.parts(g.contiguous()), p.parts(l.contiguous()), Tensor(), Tensor(),
+        r = p.run(p.parts(contiguous(q)), p.parts(contiguous(k)), p.parts(contiguous(v)), p.parts(contiguous(g)), p.parts(contiguous(l)), Tensor(), Tensor(),
                   on.stream, status);
         r.second = r.second.permute({0, 1, 3, 4, 2});
     }
@@ -404,8 +416,8 @@ struct Mixer : torch::autograd::Function<Mixer> {
                           const Tensor& D, const Tensor& nw, double eps, int64_t G, int64_t mode, bool keep, bool status) {
         On on(zx);
         const int B = zx.size(0), T = zx.size(1), W = zx.size(2), H = Lp.size(0), L = Lp.size(1), dim = H * 64, N = (W - 2 * dim - H - H * L) / (2 * G);
-        const Tensor z = zx.contiguous(), cw_ = cw.contiguous(), cb_ = contiguous(of(cb)), b_ = contiguous(bias), A_ = A.to(at::kFloat).contiguous(),
-                     Lp_ = Lp.contiguous(), D_ = contiguous(D), nw_ = nw.contiguous();
+        const Tensor z = contiguous(zx), cw_ = contiguous(cw), cb_ = contiguous(of(cb)), b_ = contiguous(bias), A_ = contiguous(A.to(at::kFloat)),
+                     Lp_ = contiguous(Lp), D_ = contiguous(D), nw_ = contiguous(nw);
         const Tensor x = empty({B, T, H, 64}, at::kBFloat16, zx), v = contiguous_like(x), k = empty({B, T, G, N}, at::kBFloat16, zx), q = contiguous_like(k);
         const Tensor g = empty({B, T, H}, at::kFloat, zx), lam = empty({B, T, H, L}, at::kBFloat16, zx);
         check(lib.llattn_mixer_prep_fwd(z.data_ptr(), cw_.data_ptr(), f32(cw_), ptr(cb_), f32(cb_), ptr(b_), f32(b_), fptr(A_), Lp_.data_ptr(), f32(Lp_),
@@ -426,12 +438,12 @@ struct Mixer : torch::autograd::Function<Mixer> {
         return out;
     }
     static variable_list backward(AutogradContext* ctx, variable_list d) {
-        const auto s = ctx->get_saved_variables();
+        const auto s = saved(ctx);
         const Tensor &z = s[0], &cw = s[1], &cb = s[2], &bias = s[3], &A = s[4], &Lp = s[5], &D = s[6], &nw = s[7], &x = s[8], &v = s[9], &k = s[10],
                      &q = s[11], &g_cum = s[12], &lam = s[13], &o = s[14], &rstd = s[15], &ws = s[16];
         On on(z);
         const int B = z.size(0), T = z.size(1), W = z.size(2), H = Lp.size(0), L = Lp.size(1), dim = H * 64, G = k.size(2), N = k.size(3);
-        const Tensor dn = d[0].to(at::kBFloat16).contiguous();
+        const Tensor dn = contiguous(d[0].to(at::kBFloat16));
         const Tensor dzx = contiguous_like(z), dy = empty(x.sizes(), at::kBFloat16, x);
         // sums over tokens: conv taps and bias, norm weight, A, dt_bias, D, L
         const int64_t ch = dim + 2 * G * N, at_b = ch * 4, at_n = ch * 5, at_A = at_n + dim, at_dt = at_A + H, at_D = at_dt + H, at_L = at_D + H;
@@ -538,7 +550,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
     static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l,
                           double scale, double lam_mul, int64_t keep_bytes, bool status) {
         On on(q);
-        const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), b_ = b.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
+        const Tensor q_ = contiguous(q), k_ = contiguous(k), v_ = contiguous(v), b_ = contiguous(b), g_ = contiguous(g), l_ = contiguous(l);
         const int T = q.size(1);
         GdnInputs a = gdn_prepare(q_, k_, v_, b_, g_, l_, T, 0, scale, lam_mul, on.stream);
         const int B = a.B, H = a.heads(), V = a.width;
@@ -563,7 +575,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
         return o;
     }
     static variable_list backward(AutogradContext* ctx, variable_list d) {
-        const auto s = ctx->get_saved_variables();
+        const auto s = saved(ctx);
         On on(s[0]);
         const Tensor &q = s[0], &k = s[1], &v = s[2], &b = s[3], &g_cum = s[4], &l = s[5], &Aw = s[6], &Au = s[7];
         const bool kept = s.size() > 8, status = ctx->saved_data["status"].toBool();
@@ -588,7 +600,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
                                              nullptr, nullptr, B, T, 0, a.H, a.H, a.K, GDN_K, a.V, a.rep, a.L, (float)scale, 0.f, on.stream),
                   "llattn_gdn_prompt_prep");
         }
-        const Tensor d_o = d[0].to(at::kBFloat16).contiguous();
+        const Tensor d_o = contiguous(d[0].to(at::kBFloat16));
         // fp32 gradients of what the parts of a head share; dg is handed on as it is where a head has one part
         const int64_t rows = (int64_t)B * T * a.H, prows = rows * a.rep;
         const Tensor gq = empty({B, T, a.H, a.K}, at::kBFloat16, q), gk = contiguous_like(gq);
@@ -663,7 +675,7 @@ py::object gdn_prompt(const Tensor& q, const Tensor& k, const Tensor& v, const T
         py::gil_scoped_release nogil;
         at::NoGradGuard no_grad;
         On on(q);
-        GdnInputs a = gdn_prepare(q.contiguous(), k.contiguous(), v.contiguous(), b.contiguous(), g.contiguous(), l.contiguous(), T0, n, scale, lam_mul,
+        GdnInputs a = gdn_prepare(contiguous(q), contiguous(k), contiguous(v), contiguous(b), contiguous(g), contiguous(l), T0, n, scale, lam_mul,
                                   on.stream);
         const int B = a.B, H = a.heads(), K = a.K, V = a.width;
         states = empty({B, a.H, L, K, a.V}, at::kFloat, q);
@@ -722,7 +734,7 @@ Cascade cascade(const py::list& counts, int64_t L) {
     return c;
 }
 bool level_major(const Tensor& s) {
-    if (!is(s, at::kFloat) || s.dim() != 5) return false;
+    if (!is(s, at::kFloat) || s.dim() != 5 || !aligned(s)) return false;
     const int64_t H = s.size(1), K = s.size(2), V = s.size(3), L = s.size(4);
     const auto st = s.strides();
     return V % 16 == 0 && st[0] == H * L * K * V && st[1] == L * K * V && st[2] == V && st[3] == 1 && st[4] == K * V;
@@ -741,8 +753,8 @@ py::object mamba2_step(const Tensor& states, const py::list& counts, const Tenso
         Bm.size(0) != B || Cm.sizes() != Bm.sizes() || dl.sizes() != at::IntArrayRef({B, H, L}) || Lp.sizes() != at::IntArrayRef({H, L}) ||
         (D.defined() && D.sizes() != at::IntArrayRef({H})) || (bias.defined() && bias.sizes() != at::IntArrayRef({H})) || V > 256 || K > 1024)
         return py::none();
-    const Tensor q = Cm.contiguous(), k = Bm.contiguous(), x_ = x.contiguous(), dt_ = dt.contiguous(), dl_ = dl.contiguous(), Lp_ = Lp.contiguous(),
-                 A_ = A.to(at::kFloat).contiguous(), D_c = contiguous(D), b_ = contiguous(bias);
+    const Tensor q = contiguous(Cm), k = contiguous(Bm), x_ = contiguous(x), dt_ = contiguous(dt), dl_ = contiguous(dl), Lp_ = contiguous(Lp),
+                 A_ = contiguous(A.to(at::kFloat)), D_c = contiguous(D), b_ = contiguous(bias);
     const Tensor y = empty({B, H, V}, f32(D_c) ? at::kFloat : at::kBFloat16, x);
     const Cascade c = cascade(counts, L);
     const int dev = x.device().index();
@@ -763,7 +775,7 @@ py::object gdn_step(const Tensor& states, const py::list& counts, const Tensor& 
     if (q.size(1) != 1 || v.size(0) != B || v.size(1) != 1 || b.sizes() != at::IntArrayRef({B, 1, H}) || g.sizes() != b.sizes() ||
         l.sizes() != at::IntArrayRef({B, 1, H, L}) || states.sizes() != at::IntArrayRef({B, H, K, V, L}) || G <= 0 || H % G != 0 || K > 256)
         return py::none();
-    const Tensor q_ = q.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(), b_ = b.contiguous(), g_ = g.contiguous(), l_ = l.contiguous();
+    const Tensor q_ = contiguous(q), k_ = contiguous(k), v_ = contiguous(v), b_ = contiguous(b), g_ = contiguous(g), l_ = contiguous(l);
     const Tensor o = empty({B, 1, H, V}, at::kBFloat16, q);
     const Cascade c = cascade(counts, L);
     const int dev = q.device().index();

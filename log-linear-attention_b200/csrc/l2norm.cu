@@ -209,6 +209,7 @@ int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const flo
                         float scale, float lambda_mul, void* stream) {
     if (rows <= 0 || rep <= 0 || K <= 0 || K % 8 != 0 || K_in < K || K_in % 8 != 0 || K_in > 128 || L <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if ((q && (!k || !dq || !dk || !gq || !gk)) || !dbeta || !dlambda || !gbeta || !glambda || (dg && !gg)) return LLATTN_ERR_NULL;
+    if (q && llattn::misaligned(16, {q, k, dq, dk, gq, gk})) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     llattn::GdnGradOut a{(const bf*)q, (const bf*)k, dq, dk, dbeta, dlambda, dg, (bf*)gq, (bf*)gk, (bf*)gbeta, (bf*)glambda, gg, rep, rows, K, K_in, L, scale,
                          lambda_mul};
@@ -226,6 +227,7 @@ int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const flo
 static int l2norm_check(const void* a, const void* b, long rows, int D) {
     if (rows <= 0 || D <= 0 || D > 256 || D % 8 != 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!a || !b) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {a, b})) return LLATTN_ERR_ALIGNMENT;
     return 0;
 }
 
@@ -247,6 +249,7 @@ int llattn_l2norm_bwd(const void* x, const float* dy, void* dx, long rows, int D
     int rc = l2norm_check(x, dx, rows, D);
     if (rc != 0) return rc;
     if (!dy) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {dy})) return LLATTN_ERR_ALIGNMENT;
     cudaStream_t st = (cudaStream_t)stream;
     const __nv_bfloat16* xi = (const __nv_bfloat16*)x;
     __nv_bfloat16* o = (__nv_bfloat16*)dx;

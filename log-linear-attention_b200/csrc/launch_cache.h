@@ -5,8 +5,16 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <initializer_list>
 
 namespace llattn {
+
+// Whether one of the pointers (a null one is not) does not start on a multiple of `bytes`: vector loads and stores there would fault.
+inline bool misaligned(size_t bytes, std::initializer_list<const void*> ptrs) {
+    for (const void* p : ptrs)
+        if (reinterpret_cast<uintptr_t>(p) % bytes != 0) return true;
+    return false;
+}
 
 // The kernel may use `bytes` of dynamic shared memory on the current device.
 inline cudaError_t allow_smem_of(const void* fn, size_t bytes) {

@@ -28,7 +28,7 @@ struct PrepArgs {
     int tokens, run;                           // B T, and how many of them a thread walks
     int lpr;                                   // lanes of a head, 8 columns each
     int row_blocks, lam_blocks;                // blocks of the x part and of the lambda part per run; the latter come first
-    int lam8, lam_runs;                        // the lambda columns come in eights; runs of that part
+    int lam8, lam_runs;                        // the lambda columns come in eights, at 16-byte boundaries; runs of that part
 };
 
 // Both passes: a group of LPR lanes owns one head and walks `run` tokens, eight columns a lane.  What depends on the (token, head)
@@ -205,7 +205,7 @@ static unsigned prep_grid(llattn::PrepArgs& a, long rows, int H, int P, int L, i
     const int want = (H * a.lpr + 31) / 32 * 32;
     threads = want < 64 ? 64 : want > 256 ? 256 : want;
     a.row_blocks = (H * a.lpr + threads - 1) / threads;
-    a.lam8 = H * L % 8 == 0;
+    a.lam8 = H * L % 8 == 0 && !llattn::misaligned(16, {a.dl, a.lam, a.dlam, a.ddl});
     a.lam_blocks = (H * L / (a.lam8 ? 8 : 1) + threads - 1) / threads;
     a.run = 64;
     while (a.run > (backward ? 8 : 4) && (long)a.row_blocks * ((a.tokens + a.run - 1) / a.run) * threads < 148 * 8 * 256) a.run /= 2;
@@ -221,6 +221,7 @@ int llattn_mamba2_layer_prep_fwd(const void* x, const void* dt_raw, const void* 
     int rc = prep_check(rows, H, P, L, lambda_mode);
     if (rc != 0) return rc;
     if (!x || !dt_raw || !A || !dl || !Lp || !v || !g || !lambda) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {x, v})) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     cudaStream_t st = (cudaStream_t)stream;
     llattn::PrepArgs a = {};
@@ -251,6 +252,7 @@ int llattn_mamba2_layer_prep_bwd(const void* x, const void* dt_raw, const void* 
     if (!x || !dt_raw || !A || !dl || !Lp || !dv || !dg || !dlambda || !dx || !ddt || !ddl || !dA || !dLp) return LLATTN_ERR_NULL;
     if (D && (!dy || !dD)) return LLATTN_ERR_NULL;
     if (dt_bias && !dbias) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {x, dv, dx}) || (D && llattn::misaligned(16, {dy}))) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     cudaStream_t st = (cudaStream_t)stream;
     llattn::PrepArgs a = {};
@@ -280,6 +282,7 @@ int llattn_mamba2_residual(const void* o, const void* x, const float* D, void* y
     int rc = prep_check(rows, H, P, 1, 0);
     if (rc != 0) return rc;
     if (!o || !x || !D || !y) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {o, x, y})) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     cudaStream_t st = (cudaStream_t)stream;
     const int lpr = llattn::lanes_per_row(P);

@@ -462,6 +462,7 @@ int llattn_mixer_prep_fwd(const void* zx, const void* conv_w, int conv_w_f32, co
     const int rc = mixer_check(B, T, H, G, N, L, lambda_mode);
     if (rc != 0) return rc;
     if (!zx || !conv_w || !A || !Lp || !x || !v || !k || !q || !g || !lambda) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {zx, x, v, k, q, lambda})) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     llattn::MixerArgs a = {};
     a.zx = (const bf*)zx; a.conv_w = conv_w; a.conv_w_f32 = conv_w_f32; a.conv_b = conv_b; a.conv_b_f32 = conv_b_f32;
@@ -486,6 +487,7 @@ int llattn_mixer_prep_bwd(const void* zx, const void* conv_w, int conv_w_f32, co
     if (rc != 0) return rc;
     if (!zx || !conv_w || !A || !Lp || !dv || !dq || !dk || !dg || !dlambda || !dzx || !dconv_w || !dA || !dLp) return LLATTN_ERR_NULL;
     if ((conv_b && !dconv_b) || (dt_bias && !dbias) || (D && !dy)) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {zx, dv, dq, dk, dlambda, dzx, dconv_w, dconv_b}) || (D && llattn::misaligned(16, {dy}))) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     llattn::MixerArgs a = {};
     a.zx = (const bf*)zx; a.conv_w = conv_w; a.conv_w_f32 = conv_w_f32; a.conv_b = conv_b; a.conv_b_f32 = conv_b_f32;
@@ -515,6 +517,7 @@ int llattn_mixer_norm_fwd(const void* o, const void* x, const void* D, int d_f32
     const int rc = norm_check(rows, H);
     if (rc != 0) return rc;
     if (!o || !zx || !w || !out || !rstd || (D && !x)) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {o, zx, out}) || (D && llattn::misaligned(16, {x}))) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     llattn::NormArgs a = {};
     a.o = (const bf*)o; a.x = (const bf*)x; a.zx = (const bf*)zx; a.D = D; a.d_f32 = d_f32; a.w = w; a.w_f32 = w_f32;
@@ -531,6 +534,7 @@ int llattn_mixer_norm_bwd(const void* o, const void* x, const void* D, int d_f32
     const int rc = norm_check(rows, H);
     if (rc != 0) return rc;
     if (!o || !zx || !w || !dn || !rstd || !dy || !dzx || !dw || (D && (!x || !dD))) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {o, zx, dn, dy, dzx, dw}) || (D && llattn::misaligned(16, {x}))) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     llattn::NormArgs a = {};
     a.o = (const bf*)o; a.x = (const bf*)x; a.zx = (const bf*)zx; a.D = D; a.d_f32 = d_f32; a.w = w; a.w_f32 = w_f32;

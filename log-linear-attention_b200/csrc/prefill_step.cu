@@ -763,6 +763,7 @@ int llattn_mamba2_prompt_states(const void* k, const void* v, const float* g, fl
     const int rc = llattn::mamba2_prompt_states_check(B, T + tail, H, G, K, V, L);
     if (rc != 0) return rc;
     if (!k || !v || !g || !states) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {k, v, states})) return LLATTN_ERR_ALIGNMENT;
     const float *seg_F = nullptr, *seg_D = nullptr;
     if (fwd_workspace != nullptr) {
         const int e = llattn::mamba2_fwd_workspace_segments(fwd_workspace, fwd_workspace_bytes, B, T, H, G, K, V, &seg_F, &seg_D);
@@ -780,7 +781,7 @@ int llattn_mamba2_prompt_tail(const void* q, const void* k, const void* v, const
     if (rc != 0) return rc;
     if (L < state_levels) return LLATTN_ERR_TOO_FEW_LEVELS;
     if (!q || !k || !v || !g || !lambda || !y || !states || (D && !x) || (T > 0 && !tail_part)) return LLATTN_ERR_NULL;
-    if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)states | (uintptr_t)tail_part) & 15) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    if (llattn::misaligned(16, {q, k, v, states, tail_part})) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     const llattn::Mamba2Tail a{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)lambda, (const bf*)x, g, D, y, states, tail_part, T, tail, H, G,
                                state_levels, L, y_is_f32};

@@ -333,6 +333,7 @@ int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_
     if (L <= 0 || L > 64 || lambda_mode < 0 || lambda_mode > 2) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!x || !dt_raw || !A || !dl || !Lp || !v || !g || !lambda) return LLATTN_ERR_NULL;
     if ((q_split != nullptr) != (k_split != nullptr) || (q_split && (!q || !k))) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {x, v, q_split, k_split}) || (q_split && llattn::misaligned(16, {q, k}))) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     const long rows = (long)B * (T + tail) * H;
     const int lpr = P <= 64 ? 8 : (P <= 128 ? 16 : 32);
@@ -354,6 +355,7 @@ int llattn_mamba2_prompt_prep(const void* x, const void* dt_raw, const void* dt_
 int llattn_mamba2_prompt_residual(const void* o, const void* x, const void* D, void* y, int y_is_f32, int B, int T, int tail, int H, int P, void* stream) {
     if (B <= 0 || T <= 0 || tail < 0 || H <= 0 || P <= 0 || P % 8 != 0 || (long)B * T * H * P > 0x7fffff00l * 8) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!o || !y || !D || !x) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {o, x, y})) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     const unsigned grid = (unsigned)(((long)B * T * H * (P / 8) + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
@@ -371,6 +373,7 @@ int llattn_gdn_prompt_prep(const void* q, const void* k, const void* v, const vo
     if (V <= 0 || rep <= 0 || V % (8 * rep) != 0 || L <= 0) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if ((long)B * (T + tail) * H * rep > 0x7fffff00l) return LLATTN_ERR_UNSUPPORTED_SHAPE;
     if (!q || !k || !qn || !kn || (v_split && !v) || (lambda_split && !lambda) || (g_split && (!g || !beta || !beta_split))) return LLATTN_ERR_NULL;
+    if (llattn::misaligned(16, {q, k, qn, kn, v_split}) || (v_split && llattn::misaligned(16, {v}))) return LLATTN_ERR_ALIGNMENT;
     using bf = __nv_bfloat16;
     llattn::GdnPrepArgs a{(const bf*)q, (const bf*)k, (const bf*)v, (const bf*)beta, g, (const bf*)lambda, (bf*)qn, (bf*)kn, (bf*)v_split,
                           (bf*)beta_split, g_split, (bf*)lambda_split, B, T, tail, H, G, K, K_out, V, rep, L, scale, lambda_mul};

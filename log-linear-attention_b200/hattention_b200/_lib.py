@@ -16,6 +16,7 @@ ERRORS = {
     -6: "null pointer",
     -7: "problem needs more scratch than the built-in static array holds",
     -8: "the driver refused a TMA tensor map for these pointers",
+    -9: "a pointer does not start on the 16-byte boundary that the kernels' accesses need",
 }
 
 _SHAPE = [ctypes.c_int] * 7
@@ -110,6 +111,12 @@ def lib():
     L.llattn_selftest_umma.argtypes = [_P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P, _P]
     _lib = L
     return L
+
+
+def aligned(x):
+    """A tensor contiguous and from a 16-byte boundary on, where the kernels' vector accesses can start."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
 
 
 _host = None

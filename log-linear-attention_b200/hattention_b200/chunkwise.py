@@ -51,7 +51,7 @@ def _check(q, k, v, g, l, head_first, level_base, htype, chunk_size):
 
 
 def _as(x, dtype):
-    return x.to(dtype).contiguous()
+    return _lib.aligned(x.to(dtype))
 
 
 def _stream():

@@ -21,7 +21,7 @@ def l2norm_fwd(x: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     reference's `* scale`, hattention/kernel.py:20-23), one CUDA pass."""
     if not x.is_cuda:
         raise RuntimeError("l2norm_fwd needs a CUDA tensor (there is no CPU path)")
-    xb = x.to(torch.bfloat16).contiguous()
+    xb = _lib.aligned(x.to(torch.bfloat16))
     y = torch.empty_like(xb)
     D = xb.shape[-1]
     with torch.cuda.device(x.device):
@@ -35,8 +35,8 @@ def l2norm_bwd(x: torch.Tensor, dy: torch.Tensor, scale: float = 1.0) -> torch.T
     """Gradient w.r.t. x of l2norm_fwd(x, scale) given dy (hattention/kernel.py:26-29), bf16."""
     if not x.is_cuda:
         raise RuntimeError("l2norm_bwd needs CUDA tensors (there is no CPU path)")
-    xb = x.to(torch.bfloat16).contiguous()
-    g = dy.to(torch.float32).contiguous()
+    xb = _lib.aligned(x.to(torch.bfloat16))
+    g = _lib.aligned(dy.to(torch.float32))
     dx = torch.empty_like(xb)
     D = xb.shape[-1]
     with torch.cuda.device(x.device):
@@ -137,7 +137,7 @@ def chunkwise_fwd(
         if G != H:   # one q/k per head, as the reference expands them (chunkwise_hgdn.py:613-620)
             q = q.repeat_interleave(H // G, dim=2)
             k = k.repeat_interleave(H // G, dim=2)
-        q_, k_, v_, b_, l_ = (x.to(torch.bfloat16).contiguous() for x in (q, k, v, b, l))
+        q_, k_, v_, b_, l_ = (_lib.aligned(x.to(torch.bfloat16)) for x in (q, k, v, b, l))
         g_ = g.to(torch.float32).contiguous()
         o = torch.empty_like(v_)
         g_cum = torch.empty_like(g_)
@@ -198,7 +198,7 @@ def chunkwise_bwd(q, k, v, b, g, l, Aw, Au, do, head_first, level_base, htype, c
         return dq[..., :K].contiguous(), dk[..., :K].contiguous(), dv, db, dg, dl
     lib = _lib.lib()
     with torch.cuda.device(q.device):
-        q_, k_, v_, b_, l_, do_, Aw_, Au_ = (x.to(torch.bfloat16).contiguous() for x in (q, k, v, b, l, do, Aw, Au))
+        q_, k_, v_, b_, l_, do_, Aw_, Au_ = (_lib.aligned(x.to(torch.bfloat16)) for x in (q, k, v, b, l, do, Aw, Au))
         gc_ = g.to(torch.float32).contiguous()
         f32 = dict(dtype=torch.float32, device=q.device)
         dq, dk = torch.empty(B, T, H, K, **f32), torch.empty(B, T, H, K, **f32)

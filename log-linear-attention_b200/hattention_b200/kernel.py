@@ -165,7 +165,7 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
     if not v.is_cuda:
         raise RuntimeError("the decode kernels need CUDA tensors (there is no CPU path)")
     if is_level_major(hstate.states):
-        q_, k_, v_, l_ = (x.to(torch.bfloat16).contiguous() for x in (q, k, v, l))
+        q_, k_, v_, l_ = (_lib.aligned(x.to(torch.bfloat16)) for x in (q, k, v, l))
         g_ = g.contiguous()
         if hstruct == HStruct.MAMBA2:
             o = mamba2_layer_step(hstate, q_, k_, v_, None, g_, l_)
@@ -173,6 +173,8 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
             o = gdn_layer_step(hstate, q_, k_, v_, b.to(torch.bfloat16).contiguous(), g_, l_, scale if use_qk_l2norm_in_kernel else None)
         return o.to(v.dtype), hstate
     lib = _lib.lib()
+    if not hstate.states.is_contiguous():
+        hstate.states = hstate.states.contiguous()           # these kernels take the level innermost
     if hstruct == HStruct.GDELTA:
         if use_qk_l2norm_in_kernel:
             from .chunkwise_hgdn import l2norm_fwd

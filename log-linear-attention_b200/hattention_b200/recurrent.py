@@ -7,9 +7,10 @@ from .base import HStruct, HType
 
 
 def is_level_major(states: torch.Tensor) -> bool:
-    """Whether a (B,H,K,V,L) tensor is stored (B,H,L,K,V): one contiguous K x V block per level of a head."""
+    """Whether a (B,H,K,V,L) tensor is stored (B,H,L,K,V): one contiguous K x V block per level of a head, at the 16-byte boundary that
+    the kernels for that layout need."""
     B, H, K, V, L = states.shape
-    return states.stride() == (H * L * K * V, L * K * V, V, 1, K * V)
+    return states.stride() == (H * L * K * V, L * K * V, V, 1, K * V) and (not states.is_cuda or states.data_ptr() % 16 == 0)
 
 
 def level_major_states(shape, device, dtype=torch.float32, zero=False) -> torch.Tensor:

@@ -182,3 +182,42 @@ def test_decode_state_counts_follow_the_cascade():
         ref.set_counts_after(T)
         assert hs.counts == ref.counts, T
         assert sum(hs.counts) == T
+
+
+def test_misaligned_pointers_are_refused(lib):
+    """Pointers between the boundaries of the vector accesses come back as an error code before anything touches a device."""
+    P, I, F, Z = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_size_t
+    ok, odd, null = P(4096), P(4098), P(0)
+
+    def call(name, *args):
+        fn = getattr(lib, name)
+        old = fn.argtypes
+        fn.argtypes = None
+        try:
+            return fn(*args)
+        finally:
+            fn.argtypes = old
+
+    step = [I(x) for x in (1, 2, 1, 128, 64, 9)]
+    assert call("llattn_mamba2_layer_step", odd, ok, ok, ok, null, ok, ok, null, I(0), null, I(0), null, I(0), null, ok, *step, ctypes.c_uint(1), I(0), I(2), I(0),
+                I(0), null) == -9
+    assert call("llattn_gdn_layer_step", ok, ok, ok, odd, ok, ok, ok, ok, *step, ctypes.c_uint(1), I(0), I(1), F(1), F(0), I(0), null) == -9
+    rows = [ctypes.c_long(64), I(2), I(64), I(9), I(0), null]
+    assert call("llattn_mamba2_layer_prep_fwd", odd, ok, ok, I(0), ok, ok, ok, I(0), ok, ok, ok, *rows) == -9
+    assert call("llattn_mamba2_layer_prep_bwd", ok, ok, ok, I(0), ok, ok, ok, I(0), null, I(0), ok, ok, ok, null, odd, ok, ok, ok, ok, ok, null, *rows) == -9
+    mixer = [I(x) for x in (1, 64, 2, 1, 128, 9, 0)] + [null]
+    assert call("llattn_mixer_prep_fwd", odd, ok, I(0), ok, I(0), ok, I(0), ok, ok, I(0), *[ok] * 6, *mixer) == -9
+    assert call("llattn_mixer_prep_bwd", ok, ok, I(0), ok, I(0), ok, I(0), ok, ok, I(0), null, I(0), ok, null, ok, ok, ok, ok, odd, *[ok] * 5, *mixer) == -9
+    norm = [ctypes.c_long(64), I(2)]
+    assert call("llattn_mixer_norm_fwd", ok, ok, null, I(0), odd, I(400), ok, I(0), ok, ok, *norm, F(1e-6), null) == -9
+    assert call("llattn_mixer_norm_bwd", ok, ok, null, I(0), ok, I(400), ok, I(0), odd, ok, ok, ok, ok, null, *norm, null) == -9
+    assert call("llattn_mamba2_prompt_prep", odd, ok, null, I(0), ok, ok, ok, I(0), ok, ok, ok, ok, ok, null, null, *[I(x) for x in (1, 64, 3, 2, 1, 128, 64, 9, 0)],
+                null) == -9
+    assert call("llattn_mamba2_prompt_tail", odd, ok, ok, ok, ok, null, null, I(0), ok, ok, I(9), ok, *[I(x) for x in (1, 64, 3, 2, 1, 128, 64, 9)], null) == -9
+    assert call("llattn_gdn_prompt_prep", ok, odd, ok, ok, ok, ok, ok, ok, null, null, null, null, *[I(x) for x in (1, 64, 3, 2, 2, 128, 128, 128, 1, 9)], F(1), F(0),
+                null) == -9
+    assert call("llattn_gdn_grad_out", odd, ok, ok, ok, ok, ok, null, ok, ok, ok, ok, null, ctypes.c_long(64), *[I(x) for x in (1, 128, 128, 9)], F(1), F(0), null) == -9
+    assert call("llattn_l2norm_fwd", odd, ok, ctypes.c_long(64), I(128), F(1), null) == -9
+    shape = [I(x) for x in (1, 64, 2, 1, 128, 64, 9)]
+    assert call("llattn_mamba2_fwd", odd, ok, ok, ok, ok, ok, ok, ok, Z(1 << 30), *shape, null) == -9
+    assert call("llattn_mamba2_bwd_saved", ok, ok, ok, ok, ok, odd, *[ok] * 6, Z(1 << 30), null, Z(0), *shape, null) == -9
