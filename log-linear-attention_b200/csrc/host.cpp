@@ -72,7 +72,8 @@ inline Tensor contiguous(const Tensor& t) {
 // what a node saved; hooks may hand back any tensor of the same values
 inline variable_list saved(AutogradContext* ctx) {
     variable_list s = ctx->get_saved_variables();
-    for (Tensor& t : s) t = contiguous(t);
+    for (Tensor& t : s)
+        if (t.defined() && !(t.is_contiguous() && aligned(t))) t = contiguous(t);
     return s;
 }
 using Maybe = std::optional<Tensor>;     // a tensor that may be absent: autograd functions take no undefined tensors
@@ -92,6 +93,12 @@ inline bool wants_grad(std::initializer_list<Tensor> ts) {
         if (t.defined() && t.requires_grad()) return true;
     return false;
 }
+// A forward-mode derivative on an operand: the nodes have none to hand on, so such calls go the general way, whose autograd function says so.
+inline bool has_tangent(std::initializer_list<Tensor> ts) {
+    for (const Tensor& t : ts)
+        if (t.defined() && t._fw_grad(0).defined()) return true;
+    return false;
+}
 inline bool same_device(std::initializer_list<Tensor> ts) {
     const Tensor* first = nullptr;
     for (const Tensor& t : ts) {
@@ -101,6 +108,7 @@ inline bool same_device(std::initializer_list<Tensor> ts) {
     }
     return true;
 }
+inline bool native_set(std::initializer_list<Tensor> ts) { return same_device(ts) && !has_tangent(ts); }
 inline int ceil_log2(int64_t x) {
     int l = 0;
     while ((int64_t(1) << l) < x) ++l;
@@ -218,7 +226,7 @@ struct Mamba2Kernel : torch::autograd::Function<Mamba2Kernel> {
 
 py::object hattention_mamba2(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& l, bool keep, bool status, bool layer) {
     if (!bf16(q) || !bf16(k) || !bf16(v) || !is(g, at::kFloat) || !bf16(l) || k.dim() != 4 || v.dim() != 4 || l.dim() != 4 || q.sizes() != k.sizes() ||
-        !same_device({q, k, v, g, l}))
+        !native_set({q, k, v, g, l}))
         return py::none();
     const int64_t B = k.size(0), T = k.size(1), H = v.size(2), L = l.size(3);
     if (v.size(0) != B || v.size(1) != T || g.sizes() != at::IntArrayRef({B, T, H}) || l.sizes() != at::IntArrayRef({B, T, H, L}) ||
@@ -285,7 +293,7 @@ struct Mamba2Layer : torch::autograd::Function<Mamba2Layer> {
 bool layer_operands(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& Bm, const Tensor& Cm, const Tensor& dl, const Tensor& Lp,
                     const Tensor& D, const Tensor& bias) {
     if (!bf16(x) || !bf16(dt) || !bf16(Bm) || !bf16(Cm) || !bf16(dl) || !A.is_cuda() || !A.is_floating_point() || !param(Lp) || !param(D) || !param(bias) ||
-        x.dim() != 4 || Bm.dim() != 4 || dl.dim() != 4 || Lp.dim() != 2 || Cm.sizes() != Bm.sizes() || !same_device({x, dt, A, Bm, Cm, dl, Lp, D, bias}))
+        x.dim() != 4 || Bm.dim() != 4 || dl.dim() != 4 || Lp.dim() != 2 || Cm.sizes() != Bm.sizes() || !native_set({x, dt, A, Bm, Cm, dl, Lp, D, bias}))
         return false;
     const int64_t B = x.size(0), T = x.size(1), H = x.size(2), L = dl.size(3);
     return dt.sizes() == at::IntArrayRef({B, T, H}) && A.sizes() == at::IntArrayRef({H}) && Bm.size(0) == B && Bm.size(1) == T &&
@@ -477,7 +485,7 @@ py::object mamba2_mixer(const Tensor& zx, const Tensor& cw, const Maybe& cb_, co
                         const Tensor& D, const Tensor& nw, double eps, int64_t G, int64_t mode, bool keep, bool status) {
     const Tensor cb = of(cb_);
     if (!bf16(zx) || !param(cw) || !param(cb) || !param(bias) || !param(Lp) || !param(D) || !param(nw) || !A.is_cuda() || !A.is_floating_point() ||
-        zx.dim() != 3 || Lp.dim() != 2 || !same_device({zx, cw, cb, bias, A, Lp, D, nw}))
+        zx.dim() != 3 || Lp.dim() != 2 || !native_set({zx, cw, cb, bias, A, Lp, D, nw}))
         return py::none();
     const int64_t T = zx.size(1), H = Lp.size(0), L = Lp.size(1), dim = H * 64, rest = zx.size(2) - 2 * dim - H - H * L;
     if (G <= 0 || rest <= 0 || rest % (2 * G) != 0) return py::none();
@@ -652,7 +660,7 @@ struct GdnKernel : torch::autograd::Function<GdnKernel> {
 // hattention_kernel, delta-rule structure: l2norm of q (scaled) and k, lambda times lam_mul unless that is 0
 py::object hattention_gdn(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g, const Tensor& l, double scale, double lam_mul,
                           int64_t keep_bytes, bool status) {
-    if (!gdn_operands(q, k, v, b, g, l)) return py::none();
+    if (!gdn_operands(q, k, v, b, g, l) || has_tangent({q, k, v, b, g, l})) return py::none();
     const int64_t T = q.size(1);
     if (T % 64 != 0 || T > 16384 || l.size(3) < 7 + ceil_log2(T / 64)) return py::none();
     const bool grad = wants_grad({q, k, v, b, g, l});
@@ -746,7 +754,7 @@ py::object mamba2_step(const Tensor& states, const py::list& counts, const Tenso
     const Tensor D = of(D_), bias = of(bias_);
     if (!bf16(x) || !bf16(dt) || !bf16(Bm) || !bf16(Cm) || !bf16(dl) || !A.is_cuda() || !A.is_floating_point() || !param(Lp) || !param(D) || !param(bias) ||
         x.dim() != 3 || Bm.dim() != 3 || dl.dim() != 3 || !level_major(states) || wants_grad({x, dt, A, Bm, Cm, dl, Lp, D, bias}) ||
-        !same_device({states, x, dt, A, Bm, Cm, dl, Lp, D, bias}))
+        !native_set({states, x, dt, A, Bm, Cm, dl, Lp, D, bias}))
         return py::none();
     const int64_t B = x.size(0), H = x.size(1), V = x.size(2), G = Bm.size(1), K = Bm.size(2), L = dl.size(2);
     if (states.sizes() != at::IntArrayRef({B, H, K, V, L}) || dt.sizes() != at::IntArrayRef({B, H}) || A.sizes() != at::IntArrayRef({H}) || G <= 0 || H % G != 0 ||
@@ -769,7 +777,7 @@ py::object mamba2_step(const Tensor& states, const py::list& counts, const Tenso
 py::object gdn_step(const Tensor& states, const py::list& counts, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& g,
                     const Tensor& l, double scale, double lam_mul) {
     if (!bf16(q) || !bf16(k) || !bf16(v) || !bf16(b) || !is(g, at::kFloat) || !bf16(l) || q.dim() != 4 || v.dim() != 4 || l.dim() != 4 ||
-        q.sizes() != k.sizes() || !level_major(states) || !same_device({states, q, k, v, b, g, l}))
+        q.sizes() != k.sizes() || !level_major(states) || !native_set({states, q, k, v, b, g, l}))
         return py::none();
     const int64_t B = q.size(0), G = q.size(2), K = q.size(3), H = v.size(2), V = v.size(3), L = l.size(3);
     if (q.size(1) != 1 || v.size(0) != B || v.size(1) != 1 || b.sizes() != at::IntArrayRef({B, 1, H}) || g.sizes() != b.sizes() ||
