@@ -53,7 +53,7 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
     p.LH = ceil_log2i(p.NS);
     p.o_has_high = p.NS > 1;
     p.LZ = llattn::M2_MLOW + p.LH;
-    const size_t KV = llattn::M2_KV, BH = (size_t)p.B * p.H;
+    const size_t KV = (size_t)p.K * p.V, BH = (size_t)p.B * p.H;
     Carver c(ws);
     p.err = c.take<int>(64);      // status word first (256 bytes)
     if (backward) {
@@ -71,7 +71,8 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
         p.seg_F = c.take<float>(BH * p.NS * KV);
         p.seg_D = c.take<float>(BH * p.NS);
         p.seg_H0 = c.take<__nv_bfloat16>(BH * p.NS * p.LH * KV);
-        p.o_hi = c.take<__nv_bfloat16>(BH * ((p.NT + 1) / 2) * 128 * p.V);      // whole pairs of chunks
+        // whole pairs of chunks for the tensor-core kernels
+        p.o_hi = c.take<__nv_bfloat16>(BH * (p.warp_level ? p.NT : (p.NT + 1) / 2 * 2) * 64 * p.V);
     }
     if (backward && p.NS > 1) {
         p.seg_dF = c.take<float>(BH * p.NS * p.LH * KV);
@@ -210,7 +211,11 @@ int llattn_mamba2_fwd_static(const void* q, const void* k, const void* v, const 
     if (llattn::misaligned(16, {q, k, v})) return LLATTN_ERR_ALIGNMENT;
     llattn::Mamba2Params p = {};
     p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
-    const size_t need = setup(p, nullptr, false);
+    size_t need = setup(p, nullptr, false);
+    if (need > (size_t)LLATTN_STATIC_SCRATCH_BYTES) {
+        p.warp_level = 1;                        // an odd number of chunks may still fit
+        need = setup(p, nullptr, false);
+    }
     if (need > (size_t)LLATTN_STATIC_SCRATCH_BYTES) return LLATTN_ERR_STATIC_SCRATCH;
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);

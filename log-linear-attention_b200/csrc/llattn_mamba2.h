@@ -11,7 +11,6 @@
 namespace llattn {
 
 constexpr int M2_MLOW = 3;   // a segment is 2^M2_MLOW chunks (512 tokens)
-constexpr int M2_KV = 128 * 64;   // elements between two segment states (K = 64 uses the first half of them, or has zeros behind them)
 constexpr int M2_MAX_LH = 10;   // segment levels held by the per-level scans over segments (T <= 512 * 2^10)
 
 struct Mamba2Params {
@@ -60,6 +59,7 @@ struct Mamba2Params {
     int res_T, res_f32;          // res_T: tokens of a sequence of x and y
     int res_n;                   // the first res_n <= T of them are written
     int res_round;               // bf16 y: D x is rounded to bf16 before the sum, as two operators would
+    int warp_level;              // forward: keep to the warp-level chunk kernels, whose partial outputs take no whole pairs of chunks
     int oT;                      // tokens of a sequence of o (T, or those of the prompt whose whole chunks these are)
     float* pr_states;            // forward of the whole chunks of a prompt of T + pr_n tokens: also its level states, (B,H,pr_L,K,V)
     float* pr_part;              // (B,pr_n,H,V) scratch of the tail

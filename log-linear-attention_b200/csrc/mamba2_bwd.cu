@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(256, 1) m2_bwd_revorder_kernel(const Mamba2Par
 #pragma unroll
     for (int lv = 0; lv <= MLOW; ++lv) zero_acc(RM[lv]);
     if (p.NS > 1 && r < p.NS - 1) {
-        const float* dH = p.seg_dHf + (((long)b * p.H + h) * p.NS + r) * M2_KV;
+        const float* dH = p.seg_dHf + (((long)b * p.H + h) * p.NS + r) * KD * VD;
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -674,10 +674,10 @@ __global__ void __launch_bounds__(256, 1) m2_hi_bwd_q_kernel(const Mamba2Params 
     const int wr = warp & 3, wc = warp >> 2;
     const int row0 = wr * 16, colk = wc * (KD / 2);
     const int lr = lane >> 2;
-    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * M2_KV;
+    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * KD * VD;
 
     auto issue_state = [&](int j, int slot) {
-        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * M2_KV, VD, tid);
+        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * KD * VD, VD, tid);
         cp_async_commit();
     };
     load_tile_async<CH, KD, 256>(sQ, p.q + (((long)b * p.T + t0) * p.G + grp) * KD, (long)p.G * KD, tid);
@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(256, 1) m2_seg_dstate_kernel(const Mamba2Param
         warp_gemm<MT, NPS, true, true>(acc, sQs, LDK, wr * 16 * MT, sDO + st * CH * LDV, LDV, wc * (VD / 2), CH, lane);
         __syncthreads();
     }
-    float* dF = p.seg_dF + ((((long)b * p.H + h) * p.NS + r) * p.LH + j) * M2_KV;
+    float* dF = p.seg_dF + ((((long)b * p.H + h) * p.NS + r) * p.LH + j) * KD * VD;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -887,16 +887,16 @@ __device__ __forceinline__ float2 ldg2_if(const float* ptr, bool p) {
     return r;
 }
 
-template <int LH>
-__global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p, int KV) {
+template <int LH, int KV>
+__global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p) {
     chain_wait();
     const long bh = blockIdx.y;
     const int e2 = (blockIdx.x * 128 + threadIdx.x) * 2;
     if (e2 >= KV) return;                       // whole warps: KV is a multiple of 64
-    const float* dF = p.seg_dF + bh * p.NS * LH * M2_KV + e2;
-    const float* F = p.seg_F + bh * p.NS * M2_KV + e2;
+    const float* dF = p.seg_dF + bh * p.NS * LH * KV + e2;
+    const float* F = p.seg_F + bh * p.NS * KV + e2;
     const float* D = p.seg_D + bh * p.NS;
-    float* dH = p.seg_dHf + bh * p.NS * M2_KV + e2;
+    float* dH = p.seg_dHf + bh * p.NS * KV + e2;
     float* Yseg = p.Yseg + bh * p.NS * LH;
     const int lane = threadIdx.x & 31;
     float2 st[LH];
@@ -908,10 +908,10 @@ __global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p,
     };
     auto fetch = [&](Loads& L, int r) {
         const bool in = r >= 0 && r < p.NS - 1;
-        L.f = ldg2_if(F + (long)r * M2_KV, in);
+        L.f = ldg2_if(F + (long)r * KV, in);
         L.d = in ? __ldg(D + r) : 0.f;
 #pragma unroll
-        for (int j = 0; j < LH; ++j) L.dF[j] = ldg2_if(dF + ((long)r * LH + j) * M2_KV, r >= 0 && ((r >> j) & 1));
+        for (int j = 0; j < LH; ++j) L.dF[j] = ldg2_if(dF + ((long)r * LH + j) * KV, r >= 0 && ((r >> j) & 1));
     };
     auto process = [&](const Loads& L, int r) {
         float2 out = make_float2(0.f, 0.f);
@@ -940,7 +940,7 @@ __global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p,
 #pragma unroll
             for (int j = 0; j < LH; ++j) mine = lane == j ? y[j] : mine;
             if (lane < LH && !((r >> lane) & 1)) atomicAdd(Yseg + (long)r * LH + lane, mine);
-            *reinterpret_cast<float2*>(dH + (long)r * M2_KV) = out;
+            *reinterpret_cast<float2*>(dH + (long)r * KV) = out;
         }
     };
     Loads A, B;
@@ -956,11 +956,11 @@ __global__ void __launch_bounds__(128) m2_seg_dscan_kernel(const Mamba2Params p,
     }
 }
 
-template <int LH>
-static void launch_dscan(const Mamba2Params& p, int KV, cudaStream_t stream) {
+template <int LH, int KV>
+static void launch_dscan(const Mamba2Params& p, cudaStream_t stream) {
     if constexpr (LH > 0) {
-        if (p.LH != LH) return launch_dscan<LH - 1>(p, KV, stream);
-        llattn::launch_chained(m2_seg_dscan_kernel<LH>, dim3((KV / 2 + 127) / 128, p.B * p.H), 128, 0, stream, p, KV);
+        if (p.LH != LH) return launch_dscan<LH - 1, KV>(p, stream);
+        llattn::launch_chained(m2_seg_dscan_kernel<LH, KV>, dim3((KV / 2 + 127) / 128, p.B * p.H), 128, 0, stream, p);
         LLATTN_LAUNCHED();
     }
 }
@@ -1167,7 +1167,7 @@ static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStre
                 llattn::launch_chained(kern, grid, 256, SegDSmem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
             }
         }
-        launch_dscan<M2_MAX_LH>(p, use_tc ? M2_KV : KD * VD, stream);
+        launch_dscan<M2_MAX_LH, KD * VD>(p, stream);
     }
     if (use_tc) return mamba2_bwd2_tc_launch(p, stream);
     auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;

@@ -994,8 +994,8 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_bwd_revorder_tc_kernel(con
     for (int lv = 0; lv <= MP; ++lv)
 #pragma unroll
         for (int e = 0; e < 32; ++e) RM[lv][e] = 0.f;
-    if (p.NS > 1 && r < p.NS - 1) {
-        const float* dH = p.seg_dHf + (((long)b * p.H + h) * p.NS + r) * tc::KD * tc::VD + row * tc::VD + ch * 32;
+    if (p.NS > 1 && r < p.NS - 1 && (WHOLE || row < p.K)) {
+        const float* dH = p.seg_dHf + (((long)b * p.H + h) * p.NS + r) * (WHOLE ? tc::KD : p.K) * tc::VD + row * tc::VD + ch * 32;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const float4 x = *reinterpret_cast<const float4*>(dH + c * 4);

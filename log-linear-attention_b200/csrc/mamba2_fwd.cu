@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(256, 1) m2_seg_state_kernel(const Mamba2Params
         warp_gemm<MT, NPS, true, true>(acc, sK + st * CH * LDK, LDK, wr * 16 * MT, sVs, LDV, wc * (VD / 2), CH, lane);
         __syncthreads();
     }
-    float* F = p.seg_F + (((long)b * p.H + h) * p.NS + r) * M2_KV;
+    float* F = p.seg_F + (((long)b * p.H + h) * p.NS + r) * KD * VD;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -388,14 +388,15 @@ __global__ void __launch_bounds__(256, 1) m2_seg_state_kernel(const Mamba2Params
 // ------------------------------------------------------------------------------------------
 constexpr int MAX_LH = 10;
 
-__global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p, int KV) {
+template <int KV>
+__global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p) {
     chain_wait();
     const long bh = blockIdx.y;
     const int e4 = (blockIdx.x * 256 + threadIdx.x) * 4;
     if (e4 >= KV) return;
-    const float* F = p.seg_F + bh * p.NS * M2_KV + e4;
+    const float* F = p.seg_F + bh * p.NS * KV + e4;
     const float* D = p.seg_D + bh * p.NS;
-    bf16* H0 = p.seg_H0 + bh * p.NS * p.LH * M2_KV + e4;
+    bf16* H0 = p.seg_H0 + bh * p.NS * p.LH * KV + e4;
     float st[MAX_LH][4];
 #pragma unroll
     for (int j = 0; j < MAX_LH; ++j) st[j][0] = st[j][1] = st[j][2] = st[j][3] = 0.f;
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p, 
           fb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
           db[u] = 0.f;
           if (r < p.NS - 1) {
-              fb[u] = __ldg(reinterpret_cast<const float4*>(F + (long)r * M2_KV));
+              fb[u] = __ldg(reinterpret_cast<const float4*>(F + (long)r * KV));
               db[u] = __ldg(D + r);
           }
       }
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(256) m2_seg_scan_kernel(const Mamba2Params p, 
                     uint2 pk;
                     pk.x = pack_bf16(st[j][0], st[j][1]);
                     pk.y = pack_bf16(st[j][2], st[j][3]);
-                    *reinterpret_cast<uint2*>(H0 + ((long)r * p.LH + j) * M2_KV) = pk;
+                    *reinterpret_cast<uint2*>(H0 + ((long)r * p.LH + j) * KV) = pk;
                 }
                 const int period = 2 << j;
                 if ((r % period) == period - 1) {
@@ -482,10 +483,10 @@ __global__ void __launch_bounds__(256, 1) m2_hi_out_kernel(const Mamba2Params p)
     const int wr = warp & 3, wc = warp >> 2;
     const int row0 = wr * 16, col0 = wc * (VD / 2);
     const int lr = lane >> 2, lc2 = (lane & 3) * 2;
-    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * M2_KV;
+    const bf16* H0 = p.seg_H0 + (((long)b * p.H + h) * p.NS + r) * p.LH * KD * VD;
 
     auto issue_state = [&](int j, int slot) {
-        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * M2_KV, VD, tid);
+        load_tile_async<KD, VD, 256>(sH + slot * KD * LDV, H0 + (long)j * KD * VD, VD, tid);
         cp_async_commit();
     };
     load_tile_async<CH, KD, 256>(sQ, p.q + (((long)b * p.T + t0) * p.G + grp) * KD, (long)p.G * KD, tid);
@@ -584,7 +585,7 @@ std::atomic<int> g_use_tensor_core_path{1};
 // sequences of an odd number of chunks and K = 64 went to before, and takes 3.8 ms here; T = 16384, 32 heads, K = 64: 1.98 -> 0.98 ms; a single
 // chunk, forward: 61 -> 18 us of which most is the host's.  More levels than 20 do not fit the tables in shared memory.
 // o and dv leave them in 16-byte stores (the warp-level kernels write pairs of values).
-bool mamba2_uses_tc(const Mamba2Params& p) { return p.V == 64 && p.L <= 20 && !misaligned(16, {p.o, p.dv}) && g_use_tensor_core_path.load(); }
+bool mamba2_uses_tc(const Mamba2Params& p) { return p.V == 64 && p.L <= 20 && !p.warp_level && !misaligned(16, {p.o, p.dv}) && g_use_tensor_core_path.load(); }
 
 template <int KD, int VD, int MLOW>
 static int launch_states(Mamba2Params p, cudaStream_t stream) {
@@ -599,9 +600,9 @@ static int launch_states(Mamba2Params p, cudaStream_t stream) {
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
         llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), 256, sm, stream, p); LLATTN_LAUNCHED();
     }
-    const int KV = use_tc ? M2_KV : KD * VD;
+    constexpr int KV = KD * VD;
     dim3 grid((KV / 4 + 255) / 256, p.B * p.H);
-    llattn::launch_chained(m2_seg_scan_kernel, grid, 256, 0, stream, p, KV); LLATTN_LAUNCHED();
+    llattn::launch_chained(m2_seg_scan_kernel<KV>, grid, 256, 0, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
     const int L = p.L;
     const int npairs = min(SEGP, (p.NT + 1) / 2 - r * SEGP);
     const bool hi_init = (p.o_has_high != 0) && (r != 0);
+    const int res_n = RES == 1 ? p.res_T : p.res_n;  // (a layer's y has the tokens of x)
 
     if (tid == 0) {
 #pragma unroll
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
             for (int c = 0; c < 4; ++c) ohi[c] = *reinterpret_cast<const uint4*>(gh + c * tc::PT * 8);
         }
         // x rows of the pair into L2 (held in registers from here on they cost the products below more than they save)
-        if (RES && ch == 0 && t0 + row < p.res_n)
+        if (RES && ch == 0 && t0 + row < res_n)
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.res_x + (((long)b * p.res_T + t0 + row) * p.H + h) * tc::VD));
         STAMP();                                     // 1: small fetches issued
         umma::mbar_wait(&full_kv[st], (pl >> 1) & 1, abort_flag);      // the v tile (read below with generic loads)
@@ -405,7 +406,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int rr = (tid >> 3) + u * 32;
-                xr[u] = t0 + rr < p.res_n ? __ldg(reinterpret_cast<const uint4*>(gx + (long)rr * p.H * tc::VD)) : make_uint4(0, 0, 0, 0);
+                xr[u] = t0 + rr < res_n ? __ldg(reinterpret_cast<const uint4*>(gx + (long)rr * p.H * tc::VD)) : make_uint4(0, 0, 0, 0);
             }
         }
         if (nread > 0) {
@@ -444,7 +445,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_chunk_fwd_tc_kernel(const 
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int rr = (tid >> 3) + u * 32, c = (tid & 7) * 8;
-                    if (t0 + rr >= p.res_n) continue;
+                    if (t0 + rr >= res_n) continue;
                     const uint4 ov = *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
                     const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, xw[4] = {xr[u].x, xr[u].y, xr[u].z, xr[u].w};
                     float y[8];

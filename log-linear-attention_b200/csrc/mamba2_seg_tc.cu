@@ -145,11 +145,12 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
         RegisterSplit<120, 192>::release();
         if (warp == tc::MMA_WARP + 1) {
             if (lane == 0) {
-                // level states of the segment: rows of the (B*H*NS*LH*K, V) matrix
+                // level states of the segment, K x V matrices (rows beyond K: zeros)
                 tma::expect_tx(full_h, nl * tc::H_BYTES);
                 for (int i = 0; i < nl; ++i) {
-                    const int row0 = ((((b * p.H + h) * p.NS + r) * p.LH) + lev[i]) * tc::KD;
-                    tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, row0, full_h);
+                    const int at = (((b * p.H + h) * p.NS + r) * p.LH) + lev[i];
+                    if (WHOLE) tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, at * tc::KD, full_h);
+                    else tma::load_seq_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, 0, at, full_h);
                 }
                 const int brow = r * SEG * CH;
                 for (int pl = 0; pl < npairs; ++pl) {
@@ -378,7 +379,8 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
     for (int i = 0; i < nl; ++i) {
         float t[32];
         umma::tmem_ld32(umma::tmem_addr(tbase + TM_DF + i * 64, warp, ch * 32), t);
-        float* dF = p.seg_dF + ((((long)b * p.H + h) * p.NS + r) * p.LH + lev[i]) * tc::KD * tc::VD + row * tc::VD + ch * 32;
+        float* dF = p.seg_dF + ((((long)b * p.H + h) * p.NS + r) * p.LH + lev[i]) * (WHOLE ? tc::KD : p.K) * tc::VD + row * tc::VD + ch * 32;
+        if (WHOLE || row < p.K)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             uint32_t w[8];
@@ -455,8 +457,9 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __g
             if (lane == 0) {
                 tma::expect_tx(full_h, nl * tc::H_BYTES);
                 for (int i = 0; i < nl; ++i) {
-                    const int row0 = ((((b * p.H + h) * p.NS + r) * p.LH) + lev[i]) * tc::KD;
-                    tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, row0, full_h);
+                    const int at = (((b * p.H + h) * p.NS + r) * p.LH) + lev[i];
+                    if (WHOLE) tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, at * tc::KD, full_h);
+                    else tma::load_seq_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, 0, at, full_h);
                 }
                 const int brow = r * SEG * CH;
                 for (int pl = 0; pl < npairs; ++pl) {
@@ -676,7 +679,8 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_seg_state_tc_kernel(const 
     {
         float t[32];
         umma::tmem_ld32(umma::tmem_addr(tbase, warp, ch * 32), t);
-        float* F = p.seg_F + (((long)b * p.H + h) * p.NS + r) * tc::KD * tc::VD + row * tc::VD + ch * 32;
+        float* F = p.seg_F + (((long)b * p.H + h) * p.NS + r) * p.K * tc::VD + row * tc::VD + ch * 32;
+        if (row < p.K)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             uint32_t w[8];
@@ -688,6 +692,13 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_seg_state_tc_kernel(const 
     if (tid == 0) p.seg_D[((long)b * p.H + h) * p.NS + r] = gend;
     umma::fence_before_sync();
     bar_work();
+}
+
+// level states as one matrix of their rows where they fill the 128 rows of a tile, else each as a sequence of its own, with zeros behind it
+static int make_states_map(Mamba2Params& p) {
+    const long n = (long)p.B * p.H * p.NS * p.LH;
+    return mamba2_whole_pairs(p) ? tma::make_panel_map(&p.tm_h0, p.seg_H0, n * tc::KD, 1, p.V, tc::KD)
+                                 : tma::make_seq_map(&p.tm_h0, p.seg_H0, n, p.K, 1, p.V, tc::KD, 2);
 }
 
 int mamba2_seg_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
@@ -707,7 +718,7 @@ int mamba2_hi_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
     if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * tc::KD, 1, p.V, tc::KD)) != 0) return rc;
+    if ((rc = make_states_map(p)) != 0) return rc;
     // up to five segment levels (T <= 16384) with the smaller shared-memory footprint, else up to eight
     if (p.LH <= 5) {
         auto kern = mamba2_whole_pairs(p) ? m2_hi_out_tc_kernel<M2_MLOW, 5, true> : m2_hi_out_tc_kernel<M2_MLOW, 5, false>;
@@ -730,7 +741,7 @@ int mamba2_hi_bwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     int rc;
     if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
-    if ((rc = tma::make_panel_map(&p.tm_h0, p.seg_H0, (long)p.B * p.H * p.NS * p.LH * tc::KD, 1, p.V, tc::KD)) != 0) return rc;
+    if ((rc = make_states_map(p)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
     auto kern = mamba2_whole_pairs(p) ? m2_hi_bwd_tc_kernel<M2_MLOW, true> : m2_hi_bwd_tc_kernel<M2_MLOW, false>;
     const size_t sm = HiBwdTcSmem<M2_MLOW>::total;

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) mamba2_prompt_state_kernel(const bf16* __
     auto add_segments = [&](bool have) {
         // behind the bucket: whole segments up to the one of the last token, then that segment's tokens up to the last one
         const int r0 = s0 / SEG, r1 = min(s1 / SEG, rl);
-        const float *D = seg_D + bh * NS, *F = seg_F + bh * NS * M2_KV;
+        const float *D = seg_D + bh * NS, *F = seg_F + bh * NS * KV;
         float part = 0.f;
         for (int r = r1 + tid; r < rl; r += 256) part += D[r];
         for (int t = rl * SEG + tid; t <= m; t += 256) part += gb[(long)t * H];
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) mamba2_prompt_state_kernel(const bf16* __
             const float w = fexp(after);
 #pragma unroll
             for (int i = 0; i < KV / 1024; ++i) {
-                const float4 f = *reinterpret_cast<const float4*>(F + (long)r * M2_KV + i * 1024 + tid * 4);
+                const float4 f = *reinterpret_cast<const float4*>(F + (long)r * KV + i * 1024 + tid * 4);
                 acc[i].x += w * f.x; acc[i].y += w * f.y; acc[i].z += w * f.z; acc[i].w += w * f.w;
             }
             after += D[r];

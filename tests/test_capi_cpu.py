@@ -221,3 +221,23 @@ def test_misaligned_pointers_are_refused(lib):
     shape = [I(x) for x in (1, 64, 2, 1, 128, 64, 9)]
     assert call("llattn_mamba2_fwd", odd, ok, ok, ok, ok, ok, ok, ok, Z(1 << 30), *shape, null) == -9
     assert call("llattn_mamba2_bwd_saved", ok, ok, ok, ok, ok, odd, *[ok] * 6, Z(1 << 30), null, Z(0), *shape, null) == -9
+
+
+def test_static_scratch_serves_narrow_states_and_odd_chunk_counts(lib):
+    """The state part of the scratch goes with the state width: 0.8 MiB per (batch, head) at T = 4096, K = 64, so 19 of them fit; and 97 of 9 chunks at
+    K = 128 do without the half pair of partial outputs.  Beyond that the call is refused before a device is touched."""
+    need = lambda K, T, bh: lib.llattn_mamba2_fwd_workspace_bytes(1, T, bh, 1, K, 64, 13)
+    # states: NS summaries in fp32 and NS LH level states in bf16; partial outputs: bf16 rows
+    per = lambda K, T: (lambda NS, LH: NS * K * 64 * 4 + NS * LH * K * 64 * 2 + NS * 4)(-(-T // 512), max(0, (-(-T // 512) - 1).bit_length())) + T * 128
+    for K in (64, 128):
+        assert abs(need(K, 4096, 8) - 8 * per(K, 4096)) < 2048
+    assert need(64, 4096, 19) <= lib.llattn_static_scratch_bytes() < need(64, 4096, 20)
+    null, dummy = ctypes.c_void_p(0), ctypes.c_void_p(4096)
+    static = lambda K, T, bh: lib.llattn_mamba2_fwd_static(*([null] + [dummy] * 6), 1, T, bh, 1, K, 64, 13, null)
+    import torch
+    if torch.cuda.is_available():
+        return                                        # a call that is not refused would launch
+    run = lambda K, T, bh: lib.llattn_mamba2_fwd_static(*([dummy] * 7), 1, T, bh, 1, K, 64, 13, null)
+    assert static(64, 4096, 19) == -6
+    assert run(64, 4096, 20) == -7 and run(128, 576, 98) == -7
+    assert run(64, 4096, 19) > 0 and run(128, 576, 97) > 0      # no device here: a CUDA error code, not a refusal
