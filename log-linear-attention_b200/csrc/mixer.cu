@@ -251,9 +251,9 @@ __global__ void __launch_bounds__(128, 4) mixer_prep_bwd_kernel(const __grid_con
                 dp[2][i] = dpt[i];
             }
         }
-        if (is_x && ((t - t0) & 15) == 16 - U) {
-            // the block of sixteen tokens is complete: one token a thread
-            const int tt = t - (16 - U) + lane16;
+        if (is_x && (((t - t0) & 15) == 16 - U || t + U >= t1 + MX_W - 1)) {
+            // the block of sixteen tokens, or what the run has of it, is complete: one token a thread
+            const int tt = t - ((t - t0) & 15) + lane16;
             if (tt < t1) {
                 const float dgv = a.dg[(row0 + tt) * a.H + h];
                 const float draw = (dot16 + Ah * dgv) * (raw16 > 20.f ? 1.f : sigmoid_row(raw16));
