@@ -42,5 +42,6 @@ def test_mixer_matches_torch_operators(B, T, H, G, N, L, mode, params, bias):
     assert y1.dtype == y0.dtype and rel(y1, y0) < 1e-2
     for k in g0:
         assert g1[k].shape == g0[k].shape and g1[k].dtype == g0[k].dtype, k
-        # per-head gradients are sums over B T tokens of signed terms that nearly cancel in the short cases
-        assert rel(g1[k], g0[k]) < (0.25 if k in ("A", "Lp", "D", "dtb") else 1.5e-2), (k, rel(g1[k], g0[k]))
+        # the gradients of A and dt_bias are sums over B T tokens of signed terms that nearly cancel in the short cases: what the scan rounds differently
+        # is a tenth of them there (test_pass_gradients_gpu.py compares these sums alone, with fp64)
+        assert rel(g1[k], g0[k]) < (0.25 if k in ("A", "dtb") else 3e-2 if k in ("Lp", "D") else 1.5e-2), (k, rel(g1[k], g0[k]))
