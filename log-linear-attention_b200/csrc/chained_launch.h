@@ -1,6 +1,6 @@
 // Chained launches (programmatic dependent launch): a kernel of a call is set up while the last CTAs of the kernel before it in the stream
-// finish.  Every kernel of the library is launched this way and begins with chain_wait(): it waits until everything before it in the
-// stream is complete and visible, so nothing but the moment of the launch changes.  A short call is a dozen kernels of 3 to 20 us, with a
+// finish.  Every kernel of a call is launched this way (the self-tests' are not) and begins with chain_wait(): it waits until everything before
+// it in the stream is complete and visible, so nothing but the moment of the launch changes.  A short call is a dozen kernels of 3 to 20 us, with a
 // microsecond or more between each two when they are launched plainly (B = 2, T = 1984, 8 heads: 229 -> 200 us a step).
 //
 // No kernel lets its successor start earlier (griddepcontrol.launch_dependents): waiting CTAs take shared memory and registers from the

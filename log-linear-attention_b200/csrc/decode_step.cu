@@ -457,7 +457,8 @@ int llattn_mamba2_layer_step(float* states, const void* q, const void* k, const 
                          H, G, K, V, L, live, carry_level, lambda_mode, dt_softplus, lp_is_f32, d_is_f32, bias_is_f32};
     const size_t sm = (size_t)2 * K * sizeof(float);
     cudaStream_t st = (cudaStream_t)stream;
-    // whole rows per CTA once that gives two CTAs for every SM
+    // whole rows per CTA once that gives two CTAs for every SM (K = 128, V = 64, whole rows / 16 columns: 192 heads 24.9 / 25.5 us, 240 28.4 / 32.4, 288 33.1 /
+    // 35.9, 384 49.3 / 48.6: the line is on the safe side)
     if (V % 64 == 0 && (long)B * H * (V / 64) >= 296)
         llattn::launch_chained(llattn::m2_layer_step_kernel<64, 2, 4, 2>, B * H * (V / 64), llattn::ST_THREADS, sm, st, a);
     else

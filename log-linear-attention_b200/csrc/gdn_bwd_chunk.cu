@@ -17,7 +17,7 @@
 namespace llattn {
 
 // Shared memory: three 64-row tiles of K or V columns and five 64 x 64 tiles, each used for several operands in turn, so that two
-// CTAs fit on an SM (109,600 bytes with V = 128).  k stays in the first; the others hold
+// CTAs fit on an SM (109,344 bytes with V = 128).  k stays in the first; the others hold
 //     S1: q -> v -> dAu Au^T -> w -> dw          S2: d_o -> d_u -> -(d_qd exp(G)) -> q
 //     Aw    QK -> dKK    Au -> dQK    Ta: P -> dAu -> Aw * beta_j -> dAw    Tb: dX -> dAw Aw^T
 // What bounds it: a chunk is a chain of barrier-separated small products whose latency one CTA of 8 warps does not fill: with fifteen tiles

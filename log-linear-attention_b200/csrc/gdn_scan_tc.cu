@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
         if (OUT && c == NT - 1 && p.final_states.p != nullptr) {
             // prefill hand-off: the level states every token of the last chunk starts from.  Level 7 + lv holds the block
             // of 2^lv chunks for each set bit lv of c (the binary-indexed tree as it stands before this chunk); the
-            // caller steps the last chunk's tokens through the decode kernel, which fills levels 0..6.
+            // kernels of a prompt (prompt.cu, gdn_tail.cu), or decode steps, carry them over the last chunk and fill levels 0..6.
             const GdnStateOut& fs = p.final_states;
             const long bh = (long)b * p.H + h;
             float* dst = fs.p + bh / fs.rep * fs.bh + bh % fs.rep * fs.part + row * fs.row + INTRA_LEVELS * fs.level;

@@ -558,7 +558,8 @@ int gdn_tail_apply_launch(const GdnTail& a, cudaStream_t stream) {
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = sm_count(&sms, dev)) != cudaSuccess) return (int)e;
     const int slots = tail_slots(a.T0);
-    // one CTA fits on an SM: 32 columns each while they all run at once, which halves the chain of one
+    // one CTA fits on an SM: 32 columns each while they all run at once, which halves the chain of one.  The call with 32 / 64: T = 777 at 8, 16, 24 heads
+    // (64, 128, 192 CTAs of 32) 70.4 / 74.2, 85.0 / 91.8, 113.7 / 108.5 us; T = 1000 at 8 and 16 heads (128, 256) 78.5 / 84.5, 110.4 / 106.2
     e = (long)a.B * a.H * (a.V / 32) * slots <= sms ? launch_apply<32>(a, slots, stream) : launch_apply<64>(a, slots, stream);
     if (e != cudaSuccess) return (int)e;
     const long all = (long)a.B * a.n * a.H * a.V;

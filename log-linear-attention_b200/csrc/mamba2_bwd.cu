@@ -1183,10 +1183,15 @@ static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
         // forward high-level states: recomputed unless the caller kept the forward call's workspace
         if ((rc = mamba2_fwd_states_dispatch(p, stream)) != 0) return rc;
     }
+    // chunk_rounding keeps the digits that a layer's gradients had where only the warp-level kernels took these shapes.  It is not the more accurate
+    // choice: the error of sum_t dg dt against fp64, in its absolute terms (mean of 4 heads and seeds, warp-level / tensor cores): T = 192 1.0e-3 / 1.0e-3,
+    // T = 1088 1.5e-3 / 5.8e-4, T = 2112 7.3e-4 / 6.0e-4; K = 64, T = 576 2.2e-3 / 1.2e-3, T = 1088 7.9e-4 / 4.5e-4; even counts, which have no such
+    // choice: T = 256 2.3e-3 / 1.6e-3, T = 2048 1.1e-3 / 7.8e-4.  Nor the faster one: see mamba2_uses_tc.
     const bool use_tc = mamba2_uses_tc(p) && !(p.chunk_rounding && (KD != 128 || (p.NT % 2) != 0));
     // The forward-order pass and the chain high levels -> reverse-order pass only meet in the accumulators they add to.  A pass has one CTA
-    // per (batch, head, segment) and one fits on an SM: below three waves of them the two run side by side (two of 64 CTAs each then
-    // take the time of one), beyond that each fills the chip by itself.
+    // per (batch, head, segment) and one fits on an SM: below three waves of them the two run side by side, beyond that each fills the chip by itself.
+    // A layer's step side by side and in turn, by CTAs of a pass: 64 195 / 178 us (there the events cost the host more), 128 190 / 206, 256 315 / 340,
+    // 320 404 / 440, 384 450 / 479; 512 572 / 608 and 768 845 / 872, where it would still gain 3 to 6 %.
     if ((long)p.B * p.H * p.NS < 3 * 148) {
         if (SideStream* side = SideStream::get(stream)) {
             cudaError_t e;

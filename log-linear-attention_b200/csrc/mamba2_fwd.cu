@@ -612,8 +612,9 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     const bool use_tc = mamba2_uses_tc(p);
     // A prompt's level states and its tail need the segment summaries only (part of the tail not even those), the output three more kernels.
     // The states are made beside those while the chunk kernel leaves SMs idle (it takes one CTA per segment and SM): B = 1, T = 1000, 48 heads,
-    // 96 CTAs: 62 -> 57 us for the call without a tail's kernels; T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs; within a segment
-    // there is too little to run beside for the events to pay.  With a tail always: its kernels are chains of latency (T = 1500 87.6 -> 74.5 us,
+    // 96 CTAs: 62 -> 57 us for the call without a tail's kernels; T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs (T = 1024 at 32, 48,
+    // 64 heads, beside / behind: 55.0 / 58.8, 61.7 / 65.5, 69.4 / 70.3; T = 1536 at 32, 48: 59.5 / 62.1, 72.2 / 71.0); within a segment there is too
+    // little to run beside for the events to pay.  With a tail always: its kernels are chains of latency (T = 1500 87.6 -> 74.5 us,
     // T = 3000 139 -> 119, T = 500 44.5 -> 42, four sequences of T = 700, 32 heads 123 -> 102).
     SideStream* side = nullptr;
     const Mamba2Tail tail{p.q, p.k, p.v, p.l, p.res_x, p.g, p.res_D, p.res_D ? p.res_y : p.o, p.pr_states, p.pr_part, p.T, p.pr_n, p.H, p.G, p.pr_L, p.L,

@@ -1,5 +1,5 @@
 // Log-linear Mamba-2 chunk kernel on the 5th-generation tensor cores (tcgen05.mma, accumulators in
-// tensor memory), K = 128, V = 64.  Same mathematics and same segment organisation as
+// tensor memory), K = 64 or 128, V = 64.  Same mathematics and same segment organisation as
 // m2_chunk_fwd_kernel (mamba2_fwd.cu); the differences are the tile shapes:
 //   * the CTA walks its segment in PAIRS of chunks (128 tokens) so that every product has M = 128:
 //       S  = q k^T              128 x 128 x 128   (the 128 x 128 masked tile covers levels 0..7, i.e.

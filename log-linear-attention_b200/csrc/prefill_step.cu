@@ -10,6 +10,8 @@
 // level):   S_l = sum_{s in bucket l} exp(sum_{r = s+1 .. m} g_r) k_s v_s^T .
 //   mamba2_final_state_kernel : one CTA per (batch, head, level) sums its bucket with warp-level MMA
 //       (decay folded into v), 64 tokens at a time from the end of the bucket backwards.
+//   mamba2_prompt_state_kernel : the same states level-major, with the segment summaries of the forward call
+//   mamba2_tail_intra_kernel, mamba2_tail_levels_kernel : the tokens of a prompt behind its last whole chunk
 //   mamba2_step_kernel : one CTA per (batch, head); the host passes the carry level j of the cascade
 //       (levels 0..j are summed into level j); then every level is decayed by exp(g), level 0 becomes
 //       k v^T, and o = q . sum_l lambda_l S_l.  HBM-bound: reads and writes L*K*V floats per head.

@@ -6,7 +6,8 @@
 namespace llattn {
 
 __device__ __forceinline__ float softplus_row(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
-// 2 ulp; a correctly rounded division would be a third of the instructions of the passes that use it
+// within the 2 ulp of __fdividef and, for negative x, the 2 + 1.2 |x| ulp of __expf(-x): far below the rounding to bf16 behind it.  A correctly
+// rounded division would be a third of the instructions of the passes that use it
 __device__ __forceinline__ float sigmoid_row(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
 

@@ -48,8 +48,8 @@ def chunk_h_gated_delta_rule(
     `initial_state` (-> `hattention_step`)."""
     if initial_state is not None and output_final_state is not False and cu_seqlens is None and use_qk_l2norm_in_kernel is True \
             and not head_first:
-        # a decode step: the native call takes only bf16 operands of a one-token call, which makes the checks below (5 of 14 us of a
-        # step at small batches) its own; it declines before anything is written
+        # a decode step: the native call takes only bf16 operands of a one-token call, which makes the checks below (1.4 of 14.7 us
+        # of a step at small batches) its own; it declines before anything is written
         o = _decode(q, k, v, g, l, beta, scale, initial_state)
         if o is not None:
             return o, initial_state

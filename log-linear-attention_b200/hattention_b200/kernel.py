@@ -168,7 +168,7 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
         q_, k_, v_, l_ = (_lib.aligned(x.to(torch.bfloat16)) for x in (q, k, v, l))
         g_ = g.contiguous()
         if hstruct == HStruct.MAMBA2:
-            o = mamba2_layer_step(hstate, q_, k_, v_, None, g_, l_)
+            o = mamba2_layer_step(hstate, q_, k_, v_, g_, l_)
         else:
             o = gdn_layer_step(hstate, q_, k_, v_, b.to(torch.bfloat16).contiguous(), g_, l_, scale if use_qk_l2norm_in_kernel else None)
         return o.to(v.dtype), hstate
@@ -200,44 +200,40 @@ def hattention_step(hstate: HState, q, k, v, b, g, l, scale, level_base, htype, 
     return o.to(v.dtype), hstate
 
 
-def mamba2_layer_step(hstate: HState, q, k, x, dt, g, dl, Lp=None, A=None, D=None, dt_bias=None, lambda_mode: int = 2,
-                      dt_softplus: bool = False) -> torch.Tensor:
-    """One launch of `llattn_mamba2_layer_step` on a level-major state: contiguous bf16 q, k, x, dt, dl; fp32 g, A; fp32 or bf16
-    Lp, D, dt_bias.  Without dt, x is v and g the log decay; without Lp, dl is lambda."""
-    B, G, K = k.shape
-    _, H, V = x.shape
-    L = dl.shape[-1]
-    dev = x.device.index
-    f32 = torch.float32
-    y = torch.empty(B, H, V, dtype=f32 if D is not None and D.dtype == f32 else torch.bfloat16, device=x.device)
+def _step_levels(hstate: HState):
+    """Runs the cascade on the counts and counts the new token: the levels that held tokens, as bits, and the one that receives the merged ones."""
     live = hstate.live_levels()
     carry = hstate.cascade_counts()
     hstate.counts[0] += 1
-    rc = _lib.lib().llattn_mamba2_layer_step(
-        hstate.states.data_ptr(), q.data_ptr(), k.data_ptr(), x.data_ptr(), None if dt is None else dt.data_ptr(),
-        None if g is None else g.data_ptr(), dl.data_ptr(), None if Lp is None else Lp.data_ptr(), Lp is not None and Lp.dtype == f32,
-        None if D is None else D.data_ptr(), D is not None and D.dtype == f32, None if dt_bias is None else dt_bias.data_ptr(),
-        dt_bias is not None and dt_bias.dtype == f32, None if A is None else A.data_ptr(), y.data_ptr(), B, H, G, K, V, L, live, carry,
-        lambda_mode, dt_softplus, dev, torch._C._cuda_getCurrentRawStream(dev))
-    if rc != 0:
-        _lib.check(rc, "llattn_mamba2_layer_step")
-    return y
+    return live, carry
 
 
-def gdn_layer_step(hstate: HState, q, k, v, b, g, l, scale: Optional[float] = None, lambda_mul: float = 0.0) -> torch.Tensor:
-    """One launch of `llattn_gdn_layer_step` on a level-major state: contiguous bf16 q, k, v, b, l; fp32 g.  With a scale q and k
-    are normalised (and q scaled) first; lambda_mul != 0 multiplies lambda."""
+def mamba2_layer_step(hstate: HState, q, k, v, g, l) -> torch.Tensor:
+    """One launch of `llattn_mamba2_layer_step` on a level-major state, with v, the log decay and lambda given: contiguous bf16 q, k, v, l; fp32 g."""
     B, G, K = k.shape
     _, H, V = v.shape
     dev = v.device.index
     o = torch.empty(B, H, V, dtype=torch.bfloat16, device=v.device)
-    live = hstate.live_levels()
-    carry = hstate.cascade_counts()
-    hstate.counts[0] += 1
+    live, carry = _step_levels(hstate)
+    rc = _lib.lib().llattn_mamba2_layer_step(
+        hstate.states.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), None, g.data_ptr(), l.data_ptr(), None, 0, None, 0, None, 0, None,
+        o.data_ptr(), B, H, G, K, V, l.shape[-1], live, carry, 2, 0, dev, torch._C._cuda_getCurrentRawStream(dev))
+    if rc != 0:
+        _lib.check(rc, "llattn_mamba2_layer_step")
+    return o
+
+
+def gdn_layer_step(hstate: HState, q, k, v, b, g, l, scale: Optional[float] = None) -> torch.Tensor:
+    """One launch of `llattn_gdn_layer_step` on a level-major state: contiguous bf16 q, k, v, b, l; fp32 g.  With a scale q and k
+    are normalised (and q scaled) first."""
+    B, G, K = k.shape
+    _, H, V = v.shape
+    dev = v.device.index
+    o = torch.empty(B, H, V, dtype=torch.bfloat16, device=v.device)
+    live, carry = _step_levels(hstate)
     rc = _lib.lib().llattn_gdn_layer_step(
         hstate.states.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), b.data_ptr(), g.data_ptr(), l.data_ptr(), o.data_ptr(),
-        B, H, G, K, V, l.shape[-1], live, carry, scale is not None, scale or 1.0, lambda_mul, dev,
-        torch._C._cuda_getCurrentRawStream(dev))
+        B, H, G, K, V, l.shape[-1], live, carry, scale is not None, scale or 1.0, 0.0, dev, torch._C._cuda_getCurrentRawStream(dev))
     if rc != 0:
         _lib.check(rc, "llattn_gdn_layer_step")
     return o

@@ -300,8 +300,9 @@ def hmamba_split_conv1d_scan_combined(
 ) -> torch.Tensor:
     """Signature, checks and data flow of the reference's function of this name (mamba_apis.py:116-262):
     split -> depthwise causal conv + SiLU on (x, B, C) -> hmamba_chunk_scan_combined -> gated RMSNorm ->
-    output projection.  The convolution, the norm and the projection are torch ops here (the reference
-    calls causal_conv1d / mamba_ssm kernels for the first two); the scan is this package's CUDA path."""
+    output projection.  bf16 rows with heads of 64 and four taps take the package's own passes for everything between
+    the two projections (csrc/mixer.cu; the reference calls causal_conv1d / mamba_ssm kernels for the convolution and
+    the norm); other operands take torch operators around the scan.  The output projection is torch's."""
     if initial_states is not None or seq_idx is not None:
         raise NotImplementedError
     if tuple(dt_limit) != (0.0, float("inf")):
