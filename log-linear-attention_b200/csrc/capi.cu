@@ -71,8 +71,9 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
         p.seg_F = c.take<float>(BH * p.NS * KV);
         p.seg_D = c.take<float>(BH * p.NS);
         p.seg_H0 = c.take<__nv_bfloat16>(BH * p.NS * p.LH * KV);
-        // whole pairs of chunks for the tensor-core kernels
-        p.o_hi = c.take<__nv_bfloat16>(BH * (p.warp_level ? p.NT : (p.NT + 1) / 2 * 2) * 64 * p.V);
+        // a level state for every pair of chunks (K = 64 leaves half of it unused: hosts have sized this part by the value rows)
+        __nv_bfloat16* lo = c.take<__nv_bfloat16>(BH * (p.warp_level ? p.NT : (p.NT + 1) / 2 * 2) * 64 * p.V);
+        p.lo_H = p.warp_level ? nullptr : lo;
     }
     if (backward && p.NS > 1) {
         p.seg_dF = c.take<float>(BH * p.NS * p.LH * KV);

@@ -15,8 +15,9 @@ constexpr int M2_MAX_LH = 10;   // segment levels held by the per-level scans ov
 
 struct Mamba2Params {
     // tensor maps (64-column panels, 128 rows) for the tcgen05 kernels; valid only when those run
-    alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_do;
+    alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_x, tm_y;
     alignas(64) CUtensorMap tm_h0;             // level states of the segments as a (B*H*NS*LH*K, V) matrix
+    alignas(64) CUtensorMap tm_lo;             // level states inside the segments as a (B*H*ceil(NT/2)*K, V) matrix
     alignas(64) CUtensorMap tm_dq, tm_dk;      // fp32 (B*T, G, K) accumulators, 32-column boxes (reduce-add)
     // inputs
     const __nv_bfloat16* q;      // (B,T,G,K)
@@ -37,7 +38,8 @@ struct Mamba2Params {
     float* seg_F;                // (B,H,NS,K,V)
     float* seg_D;                // (B,H,NS)
     __nv_bfloat16* seg_H0;       // (B,H,NS,LH,K,V)
-    __nv_bfloat16* o_hi;         // (B*H, NT/2, 8, 128, 8) high-level partial output, column-chunk major (tcgen05 chunk kernel)
+    __nv_bfloat16* lo_H;         // (B,H,ceil(NT/2),K,V) level states inside the segments, in the place of the first pair of chunks that reads them (null:
+                                 // not made); the place of a segment's first pair, which reads none, holds the decays over its pairs, fp32
     float* seg_dF;               // (B,H,NS,LH,K,V) reader summaries (backward)
     float* seg_dHf;              // (B,H,NS,K,V) gradient w.r.t. the segment summaries (backward)
     // per-chunk scalars from which the decay gradient across chunk boundaries is assembled
@@ -49,7 +51,8 @@ struct Mamba2Params {
     int* err;                    // device status word: set to 1 when a bounded wait on the tensor core gave up
     int B, T, H, G, K, V, L;
     int NT, NS, LH;
-    int o_has_high;
+    int o_has_high;              // warp-level chunk kernel: o holds the partial output of the high levels
+    int hc;                      // heads per CTA of the output kernel
     int lev_lo;                  // first segment level handled by one launch of the tensor-core high-level backward
     int chunk_rounding;          // backward: a sequence of an odd number of chunks, or with K = 64, takes the chunk-by-chunk kernels
     // forward of a layer: y = o + D x takes the place of o (tensor-core kernels; res_D NULL: none)
@@ -75,13 +78,13 @@ int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream);
 int mamba2_bwd_dispatch(Mamba2Params p, cudaStream_t stream);
 // segment summaries and the per-level scan over segments only (needs NS > 1)
 int mamba2_fwd_states_dispatch(Mamba2Params p, cudaStream_t stream);
-// tcgen05 version of the chunk kernel (K = 128, V = 64, even number of chunks)
-int mamba2_fwd_tc_launch(const Mamba2Params& p, cudaStream_t stream);
+// outputs on tcgen05 (K = 64 or 128, V = 64): sequences of one segment, and any other
+int mamba2_fwd_one_segment_tc_launch(const Mamba2Params& p, cudaStream_t stream);
+int mamba2_out_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_bwd1_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_bwd2_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_hi_bwd_tc_launch(const Mamba2Params& p, cudaStream_t stream);
-int mamba2_seg_state_tc_launch(const Mamba2Params& p, cudaStream_t stream);
-int mamba2_hi_out_tc_launch(const Mamba2Params& p, cudaStream_t stream);
+int mamba2_state_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 extern std::atomic<int> g_use_tensor_core_path;   // test hook, see llattn_testing.h
 // segment summaries and decays inside the workspace of a forward call (null when it has one segment only)
 int mamba2_prompt_states_check(int B, int T, int H, int G, int K, int V, int L);

@@ -549,20 +549,6 @@ __global__ void __launch_bounds__(256, 1) m2_hi_out_kernel(const Mamba2Params p)
         rem &= rem - 1;
         slot ^= 1;
     }
-    if (p.o_has_high == 2) {
-        // column-chunk-major scratch read by the tcgen05 chunk kernel: [bh][pair][8-col chunk][128 rows][8]
-        bf16* gh = p.o_hi + (((long)b * p.H + h) * ((p.NT + 1) / 2) + (c >> 1)) * (8 * 128 * 8);
-#pragma unroll
-        for (int nt = 0; nt < 2 * NPS; ++nt)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int i = (c & 1) * CH + row0 + lr + hh * 8;
-                const int cc = col0 + nt * 8;
-                *reinterpret_cast<uint32_t*>(gh + ((long)(cc >> 3) * 128 + i) * 8 + lc2) =
-                    pack_bf16(acc[0][nt][hh * 2], acc[0][nt][hh * 2 + 1]);
-            }
-        return;
-    }
     bf16* go = p.o + (((long)b * p.oT + t0) * p.H + h) * VD;
 #pragma unroll
     for (int nt = 0; nt < 2 * NPS; ++nt)
@@ -590,9 +576,8 @@ bool mamba2_uses_tc(const Mamba2Params& p) { return p.V == 64 && p.L <= 20 && !p
 template <int KD, int VD, int MLOW>
 static int launch_states(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
-    const bool use_tc = mamba2_uses_tc(p) || (KD == 128 && g_use_tensor_core_path.load());
-    if (use_tc) {
-        int rc = mamba2_seg_state_tc_launch(p, stream);
+    if (p.lo_H || (KD == 128 && g_use_tensor_core_path.load())) {
+        const int rc = mamba2_state_tc_launch(p, stream);
         if (rc != 0) return rc;
     } else {
         auto kern = m2_seg_state_kernel<KD, VD, MLOW>;
@@ -610,6 +595,7 @@ template <int KD, int VD, int MLOW>
 static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
     const bool use_tc = mamba2_uses_tc(p);
+    if (!use_tc) p.lo_H = nullptr;
     // A prompt's level states and its tail need the segment summaries only (part of the tail not even those), the output three more kernels.
     // The states are made beside those while the chunk kernel leaves SMs idle (it takes one CTA per segment and SM): B = 1, T = 1000, 48 heads,
     // 96 CTAs: 62 -> 57 us for the call without a tail's kernels; T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs (T = 1024 at 32, 48,
@@ -624,18 +610,14 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
         return rc != 0 || p.pr_n == 0 ? rc : mamba2_tail_levels_launch(tail, p.B, p.K, on);
     };
     auto output = [&]() -> int {
+        // two to four pairs of chunks without scratch for their level states: in order, on chip
+        if (use_tc) return p.NS == 1 && p.NT > 2 ? mamba2_fwd_one_segment_tc_launch(p, stream) : mamba2_out_tc_launch(p, stream);
         if (p.NS > 1) {
-            if (use_tc && p.LH <= 8) {
-                const int rc = mamba2_hi_out_tc_launch(p, stream);
-                if (rc != 0) return rc;
-            } else {
-                auto kern = m2_hi_out_kernel<KD, VD, MLOW>;
-                size_t sm = HiSmem<KD, VD>::total;
-                if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
-                llattn::launch_chained(kern, p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream, p); LLATTN_LAUNCHED();
-            }
+            auto kern = m2_hi_out_kernel<KD, VD, MLOW>;
+            size_t sm = HiSmem<KD, VD>::total;
+            if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
+            llattn::launch_chained(kern, p.B * p.H * (p.NT - (1 << MLOW)), 256, sm, stream, p); LLATTN_LAUNCHED();
         }
-        if (use_tc) return mamba2_fwd_tc_launch(p, stream);
         auto kern = m2_chunk_fwd_kernel<KD, VD, MLOW>;
         size_t sm = FwdSmem<KD, VD, MLOW>::total;
         if ((e = allow_smem(kern, sm)) != cudaSuccess) return (int)e;
@@ -652,7 +634,6 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
         rc = 0;
     }
     if (rc == 0 && p.NS > 1) {
-        p.o_has_high = use_tc ? 2 : 1;      // 2: partial output goes to the column-chunk-major scratch
         rc = launch_states<KD, VD, MLOW>(p, stream);
         if (rc != 0 && !side) return rc;
     }
@@ -674,6 +655,7 @@ int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream) {
 }
 
 int mamba2_fwd_states_dispatch(Mamba2Params p, cudaStream_t stream) {
+    p.lo_H = nullptr;
     if (p.K == 128 && p.V == 64) return launch_states<128, 64, M2_MLOW>(p, stream);
     if (p.K == 64 && p.V == 64) return launch_states<64, 64, M2_MLOW>(p, stream);
     return LLATTN_ERR_UNSUPPORTED_SHAPE;

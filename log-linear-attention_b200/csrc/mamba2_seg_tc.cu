@@ -1,10 +1,9 @@
 // Segment-level ("high" Fenwick levels) kernels of the log-linear Mamba-2 path on tcgen05 / TMA
 // (K = 128, V = 64, segments of 2^MLOW chunks = 2^(MLOW-1) pairs of 128 tokens).  Same mathematics
-// as m2_seg_state_kernel / m2_hi_out_kernel (mamba2_fwd.cu) and m2_seg_dstate_kernel /
+// as m2_seg_state_kernel (mamba2_fwd.cu) and m2_seg_dstate_kernel /
 // m2_hi_bwd_q_kernel (mamba2_bwd.cu); one CTA per (batch, head, segment) handles every high level
 // of its segment, so q / do / k / v tiles and the level states are loaded once per segment.
-//   seg_state  : F_r      = sum_pairs k^T (v * exp(G_end - G))                      (fp32 K x V)
-//   hi_out     : o_hi     = sum_{j set in r} lambda_j exp(G) * (q H0[r][j])         (bf16, column-chunk-major scratch)
+//   state      : F_r      = sum_pairs k^T (v * exp(G_end - G))                      (fp32 K x V), and the level states inside the segment
 //   seg_dstate : dF[r][j] = sum_pairs q^T (do * lambda_j exp(G))                     (fp32 K x V per set level)
 //   hi_bwd_q   : dlambda_j = exp(G) (do . (q H0_j)) ; dq += (do * lambda_j exp(G)) H0_j^T   (TMA reduce-add)
 // G is the cumulative log decay from the start of the segment (inclusive).
@@ -398,300 +397,195 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __g
 }
 
 // ------------------------------------------------------------------------------------------
-// forward: partial output of the high levels, o_hi = sum_j lambda_j exp(G) (q H0[r][j])
+// forward: level states inside a segment and the segment's summary.  One CTA per (batch, head, segment) walks its pairs of 128 tokens:
+//   KV_p = k^T (v exp(G_end of the pair - G))                  tensor core, one 64-column slot per pair
+//   F    = KV_0; then KV_p + exp(glp_p) F                      fp32 in registers
+// What later pairs of the segment read leaves as bf16 K x V tiles, in the place of the first pair that reads it: F after pair 0 (read by pair 1), F after
+// pair 1 (pairs 2 and 3), KV_2 (pair 3); the first pair's place takes the decays glp; F after the last pair is the segment's summary, with its total decay, for the scan over segments.
+// The last segment of a sequence has no summary and its last pair no reader.
+// Two CTAs per SM: the products are short, a CTA mostly waits for its tiles.
 // ------------------------------------------------------------------------------------------
-template <int MLOW, int MAXL>
-struct HiOutTcSmem {
-    static constexpr int SEG = 1 << MLOW;
-    static constexpr uint32_t q_off = 0;                                   // [2] 32 KB
-    static constexpr uint32_t h_off = q_off + 2 * tc::Q_BYTES;
-    static constexpr uint32_t gs_off = h_off + MAXL * tc::H_BYTES;
-    static constexpr uint32_t bar_off = gs_off + (SEG * 64 + SEG + 32) * 4;
-    static constexpr uint32_t total = bar_off + 128 + 1024;
-};
-
-template <int MLOW, int MAXL, bool WHOLE>
-__global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_out_tc_kernel(const __grid_constant__ Mamba2Params p) {
-    chain_wait();
-    using SM = HiOutTcSmem<MLOW, MAXL>;
-    static_assert(MAXL * 64 <= tc::TM_COLS, "one 64-column tensor-memory slot per level");
-    constexpr int SEG = SM::SEG;
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    unsigned char* sQ = smem + SM::q_off;
-    unsigned char* sH = smem + SM::h_off;
-    float* sGs = reinterpret_cast<float*>(smem + SM::gs_off);
-    float* sTot = sGs + SEG * 64;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
-    uint64_t* barA = bars + 0;       // level reads of a pair complete
-    uint64_t* full_q = bars + 1;     // [2]
-    uint64_t* full_h = bars + 3;
-    uint64_t* empty_q = bars + 4;    // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 64);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 72);
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int h = blockIdx.x % p.H;
-    const int r = 1 + (blockIdx.x / p.H) % (p.NS - 1);
-    const int b = blockIdx.x / (p.H * (p.NS - 1));
-    const int grp = h / (p.H / p.G);
-    const int nchunks = min(SEG, p.NT - r * SEG);
-    const int npairs = (nchunks + 1) / 2;
-    int lev[MAXL], nl = 0;
-#pragma unroll
-    for (int j = 0; j < MAXL; ++j)
-        if (j < p.LH && ((r >> j) & 1)) lev[nl++] = j;
-
-    if (tid == 0) {
-#pragma unroll
-        for (int i = 0; i < 6; ++i) umma::mbar_init(&bars[i], 1);
-        umma::fence_mbar_init();
-        *abort_flag = *p.err;
-    }
-    __syncthreads();
-    if (*abort_flag) return;
-
-    if (warp >= tc::MMA_WARP) {
-        RegisterSplit<56, 224>::release();
-        if (warp == tc::MMA_WARP + 1) {
-            if (lane == 0) {
-                tma::expect_tx(full_h, nl * tc::H_BYTES);
-                for (int i = 0; i < nl; ++i) {
-                    const int at = (((b * p.H + h) * p.NS + r) * p.LH) + lev[i];
-                    if (WHOLE) tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, at * tc::KD, full_h);
-                    else tma::load_seq_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, 0, at, full_h);
-                }
-                const int brow = r * SEG * CH;
-                for (int pl = 0; pl < npairs; ++pl) {
-                    const int st = pl & 1, row0 = brow + pl * tc::PT;
-                    if (pl >= 2 && !umma::mbar_wait(&empty_q[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
-                    tma::expect_tx(&full_q[st], tc::Q_BYTES);
-                    tma::load_seq_panel(sQ + st * tc::Q_BYTES, &p.tm_q, 0, grp, row0, b, &full_q[st]);
-                    tma::load_seq_panel(sQ + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, &full_q[st]);
-                }
-            }
-            return;
-        }
-        if (warp > tc::MMA_WARP) return;
-        umma::tmem_alloc(tmem_slot, tc::TM_COLS);
-        umma::fence_before_sync();
-        bar_work();
-        umma::fence_after_sync();
-        const uint32_t tbase = *tmem_slot;
-        if (lane == 0) umma::mbar_wait(full_h, 0, abort_flag);
-        for (int pl = 0; pl < npairs; ++pl) {
-            const int st = pl & 1;
-            bar_work();                              // the slots of the previous pair have been read
-            umma::fence_after_sync();
-            if (lane == 0) {
-                umma::mbar_wait(&full_q[st], (pl >> 1) & 1, abort_flag);
-                // adjacent level states / adjacent result slots: chains of up to four levels (N = 256)
-                for (int i0 = 0; i0 < nl; i0 += 4) {
-                    const int n = (nl - i0) < 4 ? (nl - i0) : 4;
-                    umma::gemm_km<tc::PT, tc::KD, tc::KD>(tbase + i0 * 64, umma::smem_addr(sQ + st * tc::Q_BYTES),
-                                                          umma::smem_addr(sH + i0 * tc::H_BYTES),
-                                                          umma::idesc_bf16(128, 64 * n, false, true), false);
-                }
-                umma::commit(barA);
-                umma::commit(&empty_q[st]);
-            }
-            __syncwarp();
-            if (*abort_flag) break;
-        }
-        umma::fence_before_sync();
-        bar_work();
-        if (*abort_flag && lane == 0) atomicExch(p.err, 1);
-        umma::tmem_dealloc(tbase, tc::TM_COLS);
-        return;
-    }
-
-    RegisterSplit<56, 224>::acquire();
-    const int rb = warp & 3;
-    const int row = rb * 32 + lane;
-    const int ch = warp >> 2;
-    segment_cumsum<SEG>(p, b, h, r, nchunks, sGs, sTot, warp, lane, tid);
-    umma::fence_before_sync();
-    bar_work();
-    umma::fence_after_sync();
-    const uint32_t tbase = *tmem_slot;
-
-    for (int pl = 0; pl < npairs; ++pl) {
-        const long t0 = (long)(r * SEG) * CH + (long)pl * tc::PT;
-        const float sc = fexp(sGs[pl * tc::PT + row]);
-        const bf16* lrow = p.l + (((long)b * p.T + t0 + row) * p.H + h) * p.L + INTRA_LEVELS + MLOW;
-        float lamv[MAXL];
-#pragma unroll
-        for (int i = 0; i < MAXL; ++i) lamv[i] = (i < nl && (WHOLE || t0 + row < p.T)) ? __bfloat162float(lrow[lev[i]]) * sc : 0.f;
-        umma::fence_before_sync();
-        bar_work();
-        umma::mbar_wait(barA, pl & 1, abort_flag);
-        umma::fence_after_sync();
-        float o[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] = 0.f;
-        for (int i = 0; i < nl; ++i) {
-            float t[32];
-            umma::tmem_ld32(umma::tmem_addr(tbase + i * 64, warp, ch * 32), t);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] += lamv[i] * t[e];
-        }
-        // column-chunk-major scratch [bh][pair][8-col chunk][128 rows][8]
-        bf16* gh = p.o_hi + ((((long)b * p.H + h) * ((p.NT + 1) / 2) + (r * (SEG / 2) + pl)) * 8 + ch * 4) * (tc::PT * 8) + row * 8;
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(gh + c * tc::PT * 8) =
-                make_uint4(pack_bf16(o[c * 8], o[c * 8 + 1]), pack_bf16(o[c * 8 + 2], o[c * 8 + 3]),
-                           pack_bf16(o[c * 8 + 4], o[c * 8 + 5]), pack_bf16(o[c * 8 + 6], o[c * 8 + 7]));
-        if (*abort_flag) break;
-    }
-    umma::fence_before_sync();
-    bar_work();
+namespace tcst {
+constexpr int NTHREADS = 320, TMA_WARP = 9, TM_COLS = 256;
 }
-
-// ------------------------------------------------------------------------------------------
-// forward: segment summaries F_r = sum_j k_j^T v_j exp(G_end - G_j), D_r = G_end
-// ------------------------------------------------------------------------------------------
 template <int MLOW>
-struct SegStateTcSmem {
+struct StateTcSmem {
     static constexpr int SEG = 1 << MLOW;
     static constexpr uint32_t k_off = 0;                                   // [2] 32 KB
-    static constexpr uint32_t v_off = k_off + 2 * tc::Q_BYTES;             // [2] 16 KB
-    static constexpr uint32_t vs_off = v_off + 2 * tc::V_BYTES;            // [2] 16 KB
-    static constexpr uint32_t gs_off = vs_off + 2 * tc::V_BYTES;
-    static constexpr uint32_t bar_off = gs_off + (SEG * 64 + SEG + 32) * 4;
-    static constexpr uint32_t total = bar_off + 128 + 1024;
+    static constexpr uint32_t v_off = k_off + 2 * tc::Q_BYTES;             // [2] 16 KB, scaled in place
+    static constexpr uint32_t gs_off = v_off + 2 * tc::V_BYTES;            // float [SEG * 64]: exp(G_end of the pair - G)
+    static constexpr uint32_t tot_off = gs_off + SEG * 64 * 4;             // float [SEG]: chunk totals
+    static constexpr uint32_t bar_off = tot_off + SEG * 4;
+    static constexpr uint32_t total = bar_off + 160 + 1024;
 };
 
 template <int MLOW>
-__global__ void __launch_bounds__(tc::NTHREADS, 1) m2_seg_state_tc_kernel(const __grid_constant__ Mamba2Params p) {
+__global__ void __launch_bounds__(tcst::NTHREADS, 2) m2_state_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
-    using SM = SegStateTcSmem<MLOW>;
+    using SM = StateTcSmem<MLOW>;
     constexpr int SEG = SM::SEG, SEGP = SEG / 2;
+    static_assert(SEGP * 64 <= tcst::TM_COLS && SEG == 8, "a slot per pair, a chunk per warp");
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    unsigned char* smem = umma::align_1024(smem_raw);
     unsigned char* sK = smem + SM::k_off;
     unsigned char* sV = smem + SM::v_off;
-    unsigned char* sVs = smem + SM::vs_off;
-    float* sGs = reinterpret_cast<float*>(smem + SM::gs_off);
-    float* sTot = sGs + SEG * 64;
+    float* sE = reinterpret_cast<float*>(smem + SM::gs_off);
+    float* sTot = reinterpret_cast<float*>(smem + SM::tot_off);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
-    uint64_t* barF = bars + 0;
-    uint64_t* full_kv = bars + 1;    // [2]
-    uint64_t* empty_kv = bars + 3;   // [2] tensor core is done with the k / v / Vs stage
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 64);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 72);
+    uint64_t* full_kv = bars + 0;    // [2]
+    uint64_t* empty_kv = bars + 2;   // [2] tensor core is done with the k / v stage
+    uint64_t* scaled = bars + 4;     // [2] v is scaled (one arrival per element-wise warp)
+    uint64_t* barKV = bars + 6;      // [SEGP] the pair's product is complete
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 128);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 136);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NP = (p.NT + 1) / 2, nseg = p.lo_H ? p.NS : p.NS - 1;
     const int h = blockIdx.x % p.H;
-    const int r = (blockIdx.x / p.H) % (p.NS - 1);          // the last segment has no reader
-    const int b = blockIdx.x / (p.H * (p.NS - 1));
+    const int r = (blockIdx.x / p.H) % nseg;
+    const int b = blockIdx.x / (p.H * nseg);
     const int grp = h / (p.H / p.G);
+    const long bh = (long)b * p.H + h;
+    const bool last = r == p.NS - 1;
+    const int np = last ? NP - r * SEGP - 1 : SEGP;          // pairs that this CTA sums
+    if (np == 0) return;                                     // (uniform)
 
-    if (tid == 0) {
-#pragma unroll
-        for (int i = 0; i < 5; ++i) umma::mbar_init(&bars[i], 1);
+    if (tid == tcst::TMA_WARP * 32) {
+        for (int i = 0; i < 6 + SEGP; ++i) umma::mbar_init(&bars[i], i == 4 || i == 5 ? 8 : 1);
         umma::fence_mbar_init();
         *abort_flag = *p.err;
     }
     __syncthreads();
     if (*abort_flag) return;
-    constexpr uint32_t ID_MM64 = umma::idesc_bf16(128, 64, true, true);
-
-    if (warp >= tc::MMA_WARP) {
-        RegisterSplit<56, 224>::release();
-        if (warp == tc::MMA_WARP + 1) {
-            if (lane == 0) {
-                const int brow = r * SEG * CH;
-                for (int pl = 0; pl < SEGP; ++pl) {
-                    const int st = pl & 1, row0 = brow + pl * tc::PT;
-                    if (pl >= 2 && !umma::mbar_wait(&empty_kv[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
-                    tma::expect_tx(&full_kv[st], tc::Q_BYTES + tc::V_BYTES);
-                    tma::load_seq_panel(sK + st * tc::Q_BYTES, &p.tm_k, 0, grp, row0, b, &full_kv[st]);
-                    tma::load_seq_panel(sK + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, b, &full_kv[st]);
-                    tma::load_seq_panel(sV + st * tc::V_BYTES, &p.tm_v, 0, h, row0, b, &full_kv[st]);
-                }
-            }
-            return;
+    if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tcst::TM_COLS);
+    if (warp < 8) {
+        // one chunk per warp: cumulative decay of the pair, then exp(G_end - G)
+        float x0 = 0.f, x1 = 0.f;
+        if (warp < 2 * np) {
+            const float* gp = p.g + ((long)b * p.T + (long)(r * SEG + warp) * CH) * p.H + h;
+            x0 = gp[(long)(2 * lane) * p.H];
+            x1 = gp[(long)(2 * lane + 1) * p.H];
         }
-        if (warp > tc::MMA_WARP) return;
-        umma::tmem_alloc(tmem_slot, 64);
-        umma::fence_before_sync();
-        bar_work();
-        umma::fence_after_sync();
-        const uint32_t tbase = *tmem_slot;
-        for (int pl = 0; pl < SEGP; ++pl) {
-            const int st = pl & 1;
-            bar_work();                              // Vs of this pair is written
-            umma::fence_after_sync();
-            if (lane == 0) {
-                umma::gemm_mm<tc::PT, tc::PT, tc::PT>(tbase, umma::smem_addr(sK + st * tc::Q_BYTES),
-                                                      umma::smem_addr(sVs + st * tc::V_BYTES), ID_MM64, pl > 0);
-                umma::commit(&empty_kv[st]);
-                if (pl == SEGP - 1) umma::commit(barF);
-            }
-            __syncwarp();
-            if (*abort_flag) break;
-        }
-        umma::fence_before_sync();
-        bar_work();
-        if (*abort_flag && lane == 0) atomicExch(p.err, 1);
-        umma::tmem_dealloc(tbase, 64);
-        return;
+        warp_cumsum64(x0, x1, lane);
+        const float tot = __shfl_sync(0xffffffffu, x1, 31);
+        if (lane == 0) sTot[warp] = tot;
+        asm volatile("bar.sync 2, 256;\n" ::: "memory");
+        const float behind = tot + ((warp & 1) ? 0.f : sTot[warp + 1]);     // from the chunk's start to the pair's end
+        sE[warp * CH + 2 * lane] = fexp(behind - x0);
+        sE[warp * CH + 2 * lane + 1] = fexp(behind - x1);
     }
-
-    RegisterSplit<56, 224>::acquire();
-    const int rb = warp & 3;
-    const int row = rb * 32 + lane;
-    const int ch = warp >> 2;
-    segment_cumsum<SEG>(p, b, h, r, SEG, sGs, sTot, warp, lane, tid);
-    const float gend = sTot[SEG];
     umma::fence_before_sync();
-    bar_work();
+    __syncthreads();
     umma::fence_after_sync();
     const uint32_t tbase = *tmem_slot;
 
-    for (int pl = 0; pl < SEGP; ++pl) {
-        const int st = pl & 1;
-        umma::mbar_wait(&full_kv[st], (pl >> 1) & 1, abort_flag);
-        if (pl >= 2) umma::mbar_wait(&empty_kv[st], ((pl - 2) >> 1) & 1, abort_flag);     // Vs stage is free
-#pragma unroll
-        for (int i = tid; i < tc::PT * (tc::VD / 8); i += 256) {
-            const int j = i / (tc::VD / 8), c = (i % (tc::VD / 8)) * 8;
-            const float sc = fexp(gend - sGs[pl * tc::PT + j]);
-            const uint32_t off = umma::tile_offset(j, c, tc::PT);
-            uint4 x = *reinterpret_cast<const uint4*>(sV + st * tc::V_BYTES + off);
-            uint32_t* xw = reinterpret_cast<uint32_t*>(&x);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                __nv_bfloat162 v2 = *reinterpret_cast<__nv_bfloat162*>(&xw[e]);
-                xw[e] = pack_bf16(__bfloat162float(v2.x) * sc, __bfloat162float(v2.y) * sc);
+    if (warp == tcst::TMA_WARP) {
+        if (lane == 0) {
+            const int brow = r * SEG * CH;
+            int pl = 0;
+            for (; pl < np; ++pl) {
+                const int st = pl & 1, row0 = brow + pl * tc::PT;
+                if (pl >= 2 && !umma::mbar_wait(&empty_kv[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
+                tma::expect_tx(&full_kv[st], tc::Q_BYTES + tc::V_BYTES);
+                tma::load_seq_panel(sK + st * tc::Q_BYTES, &p.tm_k, 0, grp, row0, b, &full_kv[st]);
+                tma::load_seq_panel(sK + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_k, 64, grp, row0, b, &full_kv[st]);
+                tma::load_seq_panel(sV + st * tc::V_BYTES, &p.tm_v, 0, h, row0, b, &full_kv[st]);
             }
-            *reinterpret_cast<uint4*>(sVs + st * tc::V_BYTES + off) = x;
+            // gave up: nothing may still be on its way into shared memory when the CTA ends
+            if (pl < np)
+                for (int i = pl - 2; i < pl; ++i) umma::mbar_wait(&full_kv[i & 1], (i >> 1) & 1, 1u << 16);
         }
-        umma::fence_async_smem();
-        umma::fence_before_sync();
-        bar_work();
-        umma::fence_after_sync();
-        if (*abort_flag) break;
-    }
-    umma::mbar_wait(barF, 0, abort_flag);
-    umma::fence_after_sync();
-    {
-        float t[32];
-        umma::tmem_ld32(umma::tmem_addr(tbase, warp, ch * 32), t);
-        float* F = p.seg_F + (((long)b * p.H + h) * p.NS + r) * p.K * tc::VD + row * tc::VD + ch * 32;
-        if (row < p.K)
+        __syncwarp();
+    } else if (warp == tc::MMA_WARP) {
+        if (lane == 0) {
+            constexpr uint32_t ID_MM64 = umma::idesc_bf16(128, 64, true, true);
+            int pl = 0;
+            for (; pl < np; ++pl) {
+                const int st = pl & 1;
+                if (!umma::mbar_wait(&scaled[st], (pl >> 1) & 1, abort_flag)) break;
+                umma::fence_after_sync();
+                umma::gemm_mm<tc::PT, tc::PT, tc::PT>(tbase + pl * 64, umma::smem_addr(sK + st * tc::Q_BYTES), umma::smem_addr(sV + st * tc::V_BYTES),
+                                                      ID_MM64, false);
+                umma::commit(&empty_kv[st]);
+                umma::commit(&barKV[pl]);
+            }
+            if (pl < np && pl > 0) umma::mbar_wait(&barKV[pl - 1], 0, 1u << 16);     // gave up: no product may still read shared memory
+        }
+        __syncwarp();
+    } else {
+        const int rb = warp & 3, row = rb * 32 + lane, ch = warp >> 2;
+        auto scale_v = [&](int pl) {
+            const int st = pl & 1;
+            umma::mbar_wait(&full_kv[st], (pl >> 1) & 1, abort_flag);
+            unsigned char* cV = sV + st * tc::V_BYTES;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            uint32_t w[8];
+            for (int i = tid; i < tc::PT * (tc::VD / 8); i += 256) {
+                const int j = i / (tc::VD / 8), c = (i % (tc::VD / 8)) * 8;
+                const float sc = sE[pl * tc::PT + j];
+                const uint32_t off = umma::tile_offset(j, c, tc::PT);
+                uint4 x = *reinterpret_cast<const uint4*>(cV + off);
+                uint32_t* xw = reinterpret_cast<uint32_t*>(&x);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(t[c * 8 + e]);
-            st_global_32B(F + c * 8, w);
+                for (int e = 0; e < 4; ++e) {
+                    __nv_bfloat162 v2 = *reinterpret_cast<__nv_bfloat162*>(&xw[e]);
+                    xw[e] = pack_bf16(__bfloat162float(v2.x) * sc, __bfloat162float(v2.y) * sc);
+                }
+                *reinterpret_cast<uint4*>(cV + off) = x;
+            }
+            umma::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(&scaled[st])) : "memory");
+        };
+        float f[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) f[e] = 0.f;
+        float gend = 0.f;
+        scale_v(0);
+        for (int pl = 0; pl < np; ++pl) {
+            if (pl + 1 < np) scale_v(pl + 1);
+            umma::mbar_wait(&barKV[pl], 0, abort_flag);
+            umma::fence_after_sync();
+            float kv[32];
+            umma::tmem_ld32(umma::tmem_addr(tbase + pl * 64, warp, ch * 32), kv);
+            const float glp = sTot[2 * pl] + sTot[2 * pl + 1], dec = fexp(glp);
+            gend += glp;
+            if (tid == 0 && p.lo_H) reinterpret_cast<float*>(p.lo_H + (bh * NP + r * SEGP) * p.K * tc::VD)[pl] = glp;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) f[e] = kv[e] + dec * f[e];
+            if (p.lo_H && pl + 1 < SEGP && row < p.K) {
+                bf16* dst = p.lo_H + ((bh * NP + r * SEGP + pl + 1) * p.K + row) * tc::VD + ch * 32;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const int i = c * 16 + 2 * e;
+                        w[e] = pl == 2 ? pack_bf16(kv[i], kv[i + 1]) : pack_bf16(f[i], f[i + 1]);
+                    }
+                    st_global_32B(dst + c * 16, w);
+                }
+            }
+        }
+        if (!last) {
+            float* F = p.seg_F + (bh * p.NS + r) * p.K * tc::VD + row * tc::VD + ch * 32;
+            if (row < p.K)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                uint32_t w[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(f[c * 8 + e]);
+                st_global_32B(F + c * 8, w);
+            }
+            if (tid == 0) p.seg_D[bh * p.NS + r] = gend;
         }
     }
-    if (tid == 0) p.seg_D[((long)b * p.H + h) * p.NS + r] = gend;
     umma::fence_before_sync();
-    bar_work();
+    __syncthreads();
+    umma::fence_after_sync();
+    if (warp == tc::MMA_WARP) {
+        if (*abort_flag && lane == 0) atomicExch(p.err, 1);
+        umma::tmem_dealloc(tbase, tcst::TM_COLS);
+    }
 }
 
 // level states as one matrix of their rows where they fill the 128 rows of a tile, else each as a sequence of its own, with zeros behind it
@@ -701,38 +595,16 @@ static int make_states_map(Mamba2Params& p) {
                                  : tma::make_seq_map(&p.tm_h0, p.seg_H0, n, p.K, 1, p.V, tc::KD, 2);
 }
 
-int mamba2_seg_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
+int mamba2_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
     if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
-    auto kern = m2_seg_state_tc_kernel<M2_MLOW>;
-    const size_t sm = SegStateTcSmem<M2_MLOW>::total;
+    auto kern = m2_state_tc_kernel<M2_MLOW>;
+    const size_t sm = StateTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
-    llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
-    return (int)cudaGetLastError();
-}
-
-int mamba2_hi_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
-    Mamba2Params p = p_in;
-    int rc;
-    if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
-    if ((rc = make_states_map(p)) != 0) return rc;
-    // up to five segment levels (T <= 16384) with the smaller shared-memory footprint, else up to eight
-    if (p.LH <= 5) {
-        auto kern = mamba2_whole_pairs(p) ? m2_hi_out_tc_kernel<M2_MLOW, 5, true> : m2_hi_out_tc_kernel<M2_MLOW, 5, false>;
-        const size_t sm = HiOutTcSmem<M2_MLOW, 5>::total;
-        cudaError_t e = allow_smem(kern, sm);
-        if (e != cudaSuccess) return (int)e;
-        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
-    } else {
-        auto kern = mamba2_whole_pairs(p) ? m2_hi_out_tc_kernel<M2_MLOW, 8, true> : m2_hi_out_tc_kernel<M2_MLOW, 8, false>;
-        const size_t sm = HiOutTcSmem<M2_MLOW, 8>::total;
-        cudaError_t e = allow_smem(kern, sm);
-        if (e != cudaSuccess) return (int)e;
-        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
-    }
+    llattn::launch_chained(kern, p.B * p.H * (p.lo_H ? p.NS : p.NS - 1), tcst::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 

@@ -61,7 +61,8 @@ inline int make_f32_box_map(CUtensorMap* out, const void* base, long BT, int NH,
 // The same tensors with the batch as a dimension of its own, (B, T, NH, C): a box that reaches beyond the T tokens of a sequence, or beyond
 // C columns, reads zeros there and writes nothing, so that a sequence may end inside a box and a 64-column tensor fills half a tile.
 // elem_bytes 2: bf16, box of 64 columns; 4: fp32, box of 32 columns; 128-byte swizzled either way.
-inline int make_seq_map(CUtensorMap* out, const void* base, long B, long T, int NH, int C, int box_rows, int elem_bytes) {
+// T_store > 0: the sequences are T_store >= T tokens apart.
+inline int make_seq_map(CUtensorMap* out, const void* base, long B, long T, int NH, int C, int box_rows, int elem_bytes, long T_store = 0) {
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -76,7 +77,7 @@ inline int make_seq_map(CUtensorMap* out, const void* base, long B, long T, int 
     const bool f32 = elem_bytes == 4;
     const cuuint64_t row = (cuuint64_t)C * elem_bytes;
     const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)NH, (cuuint64_t)T, (cuuint64_t)B};
-    const cuuint64_t strides[3] = {row, row * NH, row * NH * T};
+    const cuuint64_t strides[3] = {row, row * NH, row * NH * (T_store > 0 ? T_store : T)};
     const cuuint32_t box[4] = {f32 ? 32u : 64u, 1, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box,
@@ -108,6 +109,12 @@ __device__ __forceinline__ void load_seq_panel(void* smem_dst, const CUtensorMap
 __device__ __forceinline__ void reduce_add_seq_box(const CUtensorMap* map, int col0, int head, int tok0, int batch, const void* smem_src) {
     asm volatile(
         "cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n"
+        ::"l"(map), "r"(col0), "r"(head), "r"(tok0), "r"(batch), "r"((uint32_t)__cvta_generic_to_shared(smem_src))
+        : "memory");
+}
+__device__ __forceinline__ void store_seq_box(const CUtensorMap* map, int col0, int head, int tok0, int batch, const void* smem_src) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n"
         ::"l"(map), "r"(col0), "r"(head), "r"(tok0), "r"(batch), "r"((uint32_t)__cvta_generic_to_shared(smem_src))
         : "memory");
 }

@@ -142,6 +142,57 @@ __device__ __forceinline__ void gemm_mm(uint32_t d_tmem, uint32_t a_saddr, int a
     }
 }
 
+// ---- issue by a whole warp that stays converged, the instruction predicated on one elected lane (`lead`): the operands stay in uniform registers.  With
+// the loop inside a branch of one lane an instruction costs 45 cycles to issue whatever its shape; here N = 64 with A in tensor memory runs at 32 cycles,
+// the tensor core's own rate (A in shared memory: 48, the operand fetch).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void mma_ss_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_desc_lo, uint32_t b_desc_lo, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}\n"
+        ::"r"(d_tmem), "r"(a_desc_lo), "r"(b_desc_lo), "r"(idesc), "r"((uint32_t)accumulate), "r"(DESC_HI), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void mma_ts_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 db, {%2, %5};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}\n"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(idesc), "r"((uint32_t)accumulate), "r"(DESC_HI), "r"(lead)
+        : "memory");
+}
+template <int A_ROWS, int B_ROWS, int KRED>
+__device__ __forceinline__ void gemm_kk_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_saddr, uint32_t b_saddr, uint32_t idesc, bool accumulate) {
+    const uint32_t da = desc_lo_kmajor(a_saddr), db = desc_lo_kmajor(b_saddr);
+#pragma unroll
+    for (int kk = 0; kk < KRED; kk += 16) {
+        const uint32_t ka = (kk >> 6) * A_ROWS * ROW_BYTES + (kk & 63) * 2;
+        const uint32_t kb = (kk >> 6) * B_ROWS * ROW_BYTES + (kk & 63) * 2;
+        mma_ss_lead(lead, d_tmem, da + (ka >> 4), db + (kb >> 4), idesc, accumulate || kk > 0);
+    }
+}
+// A in tensor memory (bf16 pairs along the reduction index, a 32-bit column each), B stored [KRED rows][N cols] (MN-major)
+template <int B_ROWS, int KRED>
+__device__ __forceinline__ void gemm_tm_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_saddr, uint32_t idesc, bool accumulate) {
+    const uint32_t db = desc_lo_mnmajor(b_saddr, B_ROWS * ROW_BYTES);
+#pragma unroll
+    for (int kk = 0; kk < KRED; kk += 16)
+        mma_ts_lead(lead, d_tmem, a_tmem + kk / 2, db + ((kk * ROW_BYTES) >> 4), idesc, accumulate || kk > 0);
+}
+template <int A_ROWS, int B_ROWS, int KRED>
+__device__ __forceinline__ void gemm_km_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_saddr, uint32_t b_saddr, uint32_t idesc, bool accumulate) {
+    const uint32_t da = desc_lo_kmajor(a_saddr), db = desc_lo_mnmajor(b_saddr, B_ROWS * ROW_BYTES);
+#pragma unroll
+    for (int kk = 0; kk < KRED; kk += 16) {
+        const uint32_t ka = (kk >> 6) * A_ROWS * ROW_BYTES + (kk & 63) * 2;
+        mma_ss_lead(lead, d_tmem, da + (ka >> 4), db + ((kk * ROW_BYTES) >> 4), idesc, accumulate || kk > 0);
+    }
+}
+
 // ---- completion tracking
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count));
@@ -150,6 +201,12 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 // arrive on `bar` when every tcgen05.mma issued so far by this thread has completed
 __device__ __forceinline__ void commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void commit_lead(uint32_t lead, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n"
+        ::"r"(smem_addr(bar)), "r"(lead)
+        : "memory");
 }
 // bounded wait; returns false if the phase did not complete within the spin limit, or at once if
 // another thread of the CTA has already given up (*abort != 0); sets *abort on giving up
@@ -339,6 +396,18 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
           "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
           "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
         : "memory");
+}
+// the same for packed words
+__device__ __forceinline__ void tmem_st16u(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+          "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st8u(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
