@@ -57,7 +57,7 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
     Carver c(ws);
     p.err = c.take<int>(64);      // status word first (256 bytes)
     if (backward) {
-        // what a call clears: from the status word up to Zc
+        // what a call clears: from the status word up to g
         p.dq_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
         p.dk_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
         p.wq = c.take<float>((size_t)p.B * p.T * p.H);
@@ -74,6 +74,11 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
         // a level state for every pair of chunks (K = 64 leaves half of it unused: hosts have sized this part by the value rows)
         __nv_bfloat16* lo = c.take<__nv_bfloat16>(BH * (p.warp_level ? p.NT : (p.NT + 1) / 2 * 2) * 64 * p.V);
         p.lo_H = p.warp_level ? nullptr : lo;
+    }
+    if (backward && p.NT > 2) {
+        const size_t NP = (p.NT + 1) / 2;
+        if (p.NS == 1) p.lo_H = c.take<__nv_bfloat16>(BH * NP * KV);
+        p.lo_A = c.take<__nv_bfloat16>(BH * NP * KV);
     }
     if (backward && p.NS > 1) {
         p.seg_dF = c.take<float>(BH * p.NS * p.LH * KV);
@@ -278,16 +283,19 @@ static int mamba2_bwd_impl(const void* q, const void* k, const void* v, const fl
         if (fwd_workspace_bytes < fneed || ((uintptr_t)fwd_workspace & 255)) return LLATTN_ERR_WORKSPACE;
         setup(pf, const_cast<void*>(fwd_workspace), false);
         p.seg_F = pf.seg_F; p.seg_D = pf.seg_D; p.seg_H0 = pf.seg_H0;
-        p.reuse_states = 1;
+        if (p.NS > 1) p.lo_H = pf.lo_H;
+        p.reuse_states = p.NS > 1;           // (one segment: the forward call kept none)
     }
     cudaStream_t st = (cudaStream_t)stream;
     p.chunk_rounding = chunk_rounding;
+    p.cum_in = g_cum;
     p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
     p.l = (const __nv_bfloat16*)lambda; p.d_o = (const __nv_bfloat16*)d_o;
     p.dv = (__nv_bfloat16*)dv; p.dl = dlambda;
     const size_t nqk = (size_t)B * T * G * K, nbth = (size_t)B * T * H;
-    if ((rc = llattn::mamba2_bwd_init(g_cum, const_cast<float*>(p.g), (long)B * T, H, p.err, (size_t)((unsigned char*)p.Zc - (unsigned char*)p.err),
-                                      dlambda, (long)(nbth * L), st)) != 0)
+    // (the tensor-core kernels write d lambda of every level)
+    if ((rc = llattn::mamba2_bwd_init(g_cum, const_cast<float*>(p.g), (long)B * T, H, p.err, (size_t)((unsigned char*)p.g - (unsigned char*)p.err),
+                                      dlambda, llattn::mamba2_bwd_uses_tc(p) ? 0 : (long)(nbth * L), st)) != 0)
         return rc;
     rc = llattn::mamba2_bwd_dispatch(p, st);
     if (rc != 0) return rc;

@@ -145,6 +145,17 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     return r;
 }
 
+// two packed bf16 values, exactly; two values rounded to bf16
+__device__ __forceinline__ f32x2 bf16x2_f32x2(uint32_t w) { return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ uint32_t pack_bf16(f32x2 x) {
+    const float2 y = unpack2(x);
+    return pack_bf16(y.x, y.y);
+}
+__device__ __forceinline__ float sum2(f32x2 x) {
+    const float2 y = unpack2(x);
+    return y.x + y.y;
+}
+
 // a per-head parameter that the caller keeps in fp32 or bf16
 __device__ __forceinline__ float load_param(const void* p, int i, bool f32) {
     return f32 ? reinterpret_cast<const float*>(p)[i] : __bfloat162float(reinterpret_cast<const bf16*>(p)[i]);

@@ -18,12 +18,15 @@ struct Mamba2Params {
     alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_do, tm_x, tm_y;
     alignas(64) CUtensorMap tm_h0;             // level states of the segments as a (B*H*NS*LH*K, V) matrix
     alignas(64) CUtensorMap tm_lo;             // level states inside the segments as a (B*H*ceil(NT/2)*K, V) matrix
+    alignas(64) CUtensorMap tm_lo_a, tm_dh, tm_df;   // gradients of the pairs' and of the segments' summaries, what the readers of a segment send back
+    alignas(64) CUtensorMap tm_dv;
     alignas(64) CUtensorMap tm_dq, tm_dk;      // fp32 (B*T, G, K) accumulators, 32-column boxes (reduce-add)
     // inputs
     const __nv_bfloat16* q;      // (B,T,G,K)
     const __nv_bfloat16* k;      // (B,T,G,K)
     const __nv_bfloat16* v;      // (B,T,H,V)
     const float* g;              // (B,T,H) raw log decay
+    const float* cum_in;         // (B,T,H) backward: the forward call's g_cum, for level states that are made again (null: from g)
     const __nv_bfloat16* l;      // (B,T,H,L)
     const __nv_bfloat16* d_o;    // (B,T,H,V) upstream gradient (backward only)
     // outputs
@@ -42,6 +45,7 @@ struct Mamba2Params {
                                  // not made); the place of a segment's first pair, which reads none, holds the decays over its pairs, fp32
     float* seg_dF;               // (B,H,NS,LH,K,V) reader summaries (backward)
     float* seg_dHf;              // (B,H,NS,K,V) gradient w.r.t. the segment summaries (backward)
+    __nv_bfloat16* lo_A;         // (B,H,ceil(NT/2),K,V) gradient of every pair's summary (backward)
     // per-chunk scalars from which the decay gradient across chunk boundaries is assembled
     float* Zc;                   // (B,H,NT,LZ)      reader side: sum_t lambda * dlambda per level
     float* Yc;                   // (B,H,NT,MLOW+1)  contributor side: <KV_c, adjoint state> per low level, + combined high
@@ -71,8 +75,8 @@ struct Mamba2Params {
 };
 
 bool mamba2_uses_tc(const Mamba2Params& p);
-// Whether every pair of chunks and all 128 state rows of the tensor-core tiles hold data.  Their kernels come without the tests for it then:
-// with them the kernel of the high levels' gradients takes 1069 instead of 958 us at B = 1, T = 65536, 32 heads, the reverse-order one 911 instead of 878.
+bool mamba2_bwd_uses_tc(const Mamba2Params& p);
+// Whether every pair of chunks and all 128 state rows of the tensor-core tiles hold data: the kernel of one segment comes without the tests for it then.
 inline bool mamba2_whole_pairs(const Mamba2Params& p) { return p.NT % 2 == 0 && p.K == 128; }
 int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream);
 int mamba2_bwd_dispatch(Mamba2Params p, cudaStream_t stream);
@@ -81,9 +85,11 @@ int mamba2_fwd_states_dispatch(Mamba2Params p, cudaStream_t stream);
 // outputs on tcgen05 (K = 64 or 128, V = 64): sequences of one segment, and any other
 int mamba2_fwd_one_segment_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_out_tc_launch(const Mamba2Params& p, cudaStream_t stream);
-int mamba2_bwd1_tc_launch(const Mamba2Params& p, cudaStream_t stream);
-int mamba2_bwd2_tc_launch(const Mamba2Params& p, cudaStream_t stream);
-int mamba2_hi_bwd_tc_launch(const Mamba2Params& p, cudaStream_t stream);
+int mamba2_heads_per_cta(const Mamba2Params& p, int sms);
+// gradients on tcgen05: what the readers of the high levels send back; behind the scan over segments the gradient of every pair's summary; dq, dk, dv, d lambda
+int mamba2_readers_tc_launch(const Mamba2Params& p, cudaStream_t stream);
+int mamba2_adjoint_tc_launch(const Mamba2Params& p, cudaStream_t stream);
+int mamba2_gradients_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_state_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 extern std::atomic<int> g_use_tensor_core_path;   // test hook, see llattn_testing.h
 // segment summaries and decays inside the workspace of a forward call (null when it has one segment only)

@@ -1129,8 +1129,7 @@ __global__ void m2_cast_bf16_kernel(const float* __restrict__ src, bf16* __restr
 // host side
 // ------------------------------------------------------------------------------------------
 template <int KD, int VD, int MLOW>
-static int launch_fwdorder(const Mamba2Params& p, bool use_tc, cudaStream_t stream) {
-    if (use_tc) return mamba2_bwd1_tc_launch(p, stream);
+static int launch_fwdorder(const Mamba2Params& p, cudaStream_t stream) {
     cudaError_t e;
     auto kern = m2_bwd_fwdorder_kernel<KD, VD, MLOW>;
     if ((e = allow_smem(kern, Bwd1Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
@@ -1138,7 +1137,7 @@ static int launch_fwdorder(const Mamba2Params& p, bool use_tc, cudaStream_t stre
     return (int)cudaGetLastError();
 }
 
-// dq, d lambda and the reader totals of the high levels (warp-level kernels; the tensor-core one makes the reader summaries as well)
+// dq, d lambda and the reader totals of the high levels
 template <int KD, int VD, int MLOW>
 static int launch_high_q(const Mamba2Params& p, cudaStream_t stream) {
     cudaError_t e;
@@ -1149,64 +1148,67 @@ static int launch_high_q(const Mamba2Params& p, cudaStream_t stream) {
 }
 
 template <int KD, int VD, int MLOW>
-static int launch_high_and_revorder(const Mamba2Params& p, bool use_tc, cudaStream_t stream, bool with_q) {
+static int launch_high_and_revorder(const Mamba2Params& p, cudaStream_t stream, bool with_q) {
     cudaError_t e;
     if (p.NS > 1) {
-        if (use_tc) {
-            const int rc = mamba2_hi_bwd_tc_launch(p, stream);
+        if (with_q) {
+            const int rc = launch_high_q<KD, VD, MLOW>(p, stream);
             if (rc != 0) return rc;
-        } else {
-            if (with_q) {
-                const int rc = launch_high_q<KD, VD, MLOW>(p, stream);
-                if (rc != 0) return rc;
-            }
-            {
-                auto kern = m2_seg_dstate_kernel<KD, VD, MLOW>;
-                if ((e = allow_smem(kern, SegDSmem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
-                dim3 grid(p.B * p.H * (p.NS - 1), p.LH);
-                llattn::launch_chained(kern, grid, 256, SegDSmem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
-            }
         }
+        auto kern = m2_seg_dstate_kernel<KD, VD, MLOW>;
+        if ((e = allow_smem(kern, SegDSmem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
+        dim3 grid(p.B * p.H * (p.NS - 1), p.LH);
+        llattn::launch_chained(kern, grid, 256, SegDSmem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
         launch_dscan<M2_MAX_LH, KD * VD>(p, stream);
     }
-    if (use_tc) return mamba2_bwd2_tc_launch(p, stream);
     auto kern = m2_bwd_revorder_kernel<KD, VD, MLOW>;
     if ((e = allow_smem(kern, Bwd2Smem<KD, VD, MLOW>::total)) != cudaSuccess) return (int)e;
     llattn::launch_chained(kern, p.B * p.H * p.NS, 256, Bwd2Smem<KD, VD, MLOW>::total, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
-template <int KD, int VD, int MLOW>
-static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
-    int rc;
-    if (p.NS > 1 && !p.reuse_states) {
-        // forward high-level states: recomputed unless the caller kept the forward call's workspace
-        if ((rc = mamba2_fwd_states_dispatch(p, stream)) != 0) return rc;
-    }
+bool mamba2_bwd_uses_tc(const Mamba2Params& p) {
     // chunk_rounding keeps the digits that a layer's gradients had where only the warp-level kernels took these shapes.  It is not the more accurate
     // choice: the error of sum_t dg dt against fp64, in its absolute terms (mean of 4 heads and seeds, warp-level / tensor cores): T = 192 1.0e-3 / 1.0e-3,
     // T = 1088 1.5e-3 / 5.8e-4, T = 2112 7.3e-4 / 6.0e-4; K = 64, T = 576 2.2e-3 / 1.2e-3, T = 1088 7.9e-4 / 4.5e-4; even counts, which have no such
     // choice: T = 256 2.3e-3 / 1.6e-3, T = 2048 1.1e-3 / 7.8e-4.  Nor the faster one: see mamba2_uses_tc.
-    const bool use_tc = mamba2_uses_tc(p) && !(p.chunk_rounding && (KD != 128 || (p.NT % 2) != 0));
+    return mamba2_uses_tc(p) && !(p.chunk_rounding && (p.K != 128 || (p.NT % 2) != 0));
+}
+
+template <int KD, int VD, int MLOW>
+static int launch_bwd(Mamba2Params p, cudaStream_t stream) {
+    int rc;
+    const bool use_tc = mamba2_bwd_uses_tc(p);
+    if (use_tc ? p.NT > 2 && !p.reuse_states : p.NS > 1 && !p.reuse_states) {
+        // forward level states: recomputed unless the caller kept the forward call's workspace
+        if (!use_tc) p.lo_H = nullptr;
+        if ((rc = mamba2_fwd_states_dispatch(p, stream)) != 0) return rc;
+    }
+    if (use_tc) {
+        if (p.NS > 1) {
+            if ((rc = mamba2_readers_tc_launch(p, stream)) != 0) return rc;
+            launch_dscan<M2_MAX_LH, KD * VD>(p, stream);
+        }
+        if (p.NT > 2 && (rc = mamba2_adjoint_tc_launch(p, stream)) != 0) return rc;
+        return mamba2_gradients_tc_launch(p, stream);
+    }
     // The forward-order pass and the chain high levels -> reverse-order pass only meet in the accumulators they add to.  A pass has one CTA
-    // per (batch, head, segment) and one fits on an SM: below three waves of them the two run side by side, beyond that each fills the chip by itself.
-    // A layer's step side by side and in turn, by CTAs of a pass: 64 195 / 178 us (there the events cost the host more), 128 190 / 206, 256 315 / 340,
-    // 320 404 / 440, 384 450 / 479; 512 572 / 608 and 768 845 / 872, where it would still gain 3 to 6 %.
+    // per (batch, head, segment): below three waves of them the two run side by side, beyond that each fills the chip by itself.
     if ((long)p.B * p.H * p.NS < 3 * 148) {
         if (SideStream* side = SideStream::get(stream)) {
             cudaError_t e;
             if ((e = side->fork(stream)) != cudaSuccess) return (int)e;
-            rc = launch_fwdorder<KD, VD, MLOW>(p, use_tc, side->stream());
-            // (the warp-level kernel of the high levels' dq is not part of that chain: a layer's step at B = 2, T = 1984, 8 heads, K = 128
+            rc = launch_fwdorder<KD, VD, MLOW>(p, side->stream());
+            // (the kernel of the high levels' dq is not part of that chain: a layer's step at B = 2, T = 1984, 8 heads, K = 128
             //  224 -> 200 us, 24 heads with K = 64 341 -> 322, B = 2, T = 4032, 4 heads 178 -> 168)
-            if (rc == 0 && p.NS > 1 && !use_tc) rc = launch_high_q<KD, VD, MLOW>(p, side->stream());
-            const int rc2 = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream, false);
+            if (rc == 0 && p.NS > 1) rc = launch_high_q<KD, VD, MLOW>(p, side->stream());
+            const int rc2 = launch_high_and_revorder<KD, VD, MLOW>(p, stream, false);
             if ((e = side->join(stream)) != cudaSuccess) return (int)e;
             return rc != 0 ? rc : rc2;
         }
     }
-    if ((rc = launch_high_and_revorder<KD, VD, MLOW>(p, use_tc, stream, true)) != 0) return rc;
-    return launch_fwdorder<KD, VD, MLOW>(p, use_tc, stream);
+    if ((rc = launch_high_and_revorder<KD, VD, MLOW>(p, stream, true)) != 0) return rc;
+    return launch_fwdorder<KD, VD, MLOW>(p, stream);
 }
 
 int mamba2_bwd_dispatch(Mamba2Params p, cudaStream_t stream) {

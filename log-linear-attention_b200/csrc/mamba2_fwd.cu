@@ -578,7 +578,7 @@ static int launch_states(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
     if (p.lo_H || (KD == 128 && g_use_tensor_core_path.load())) {
         const int rc = mamba2_state_tc_launch(p, stream);
-        if (rc != 0) return rc;
+        if (rc != 0 || p.NS == 1) return rc;
     } else {
         auto kern = m2_seg_state_kernel<KD, VD, MLOW>;
         size_t sm = SegSmem<KD, VD, MLOW>::total;
@@ -595,7 +595,7 @@ template <int KD, int VD, int MLOW>
 static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
     const bool use_tc = mamba2_uses_tc(p);
-    if (!use_tc) p.lo_H = nullptr;
+    if (!g_use_tensor_core_path.load()) p.lo_H = nullptr;      // (a backward call may want them where this one does not)
     // A prompt's level states and its tail need the segment summaries only (part of the tail not even those), the output three more kernels.
     // The states are made beside those while the chunk kernel leaves SMs idle (it takes one CTA per segment and SM): B = 1, T = 1000, 48 heads,
     // 96 CTAs: 62 -> 57 us for the call without a tail's kernels; T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs (T = 1024 at 32, 48,
@@ -655,7 +655,6 @@ int mamba2_fwd_dispatch(Mamba2Params p, cudaStream_t stream) {
 }
 
 int mamba2_fwd_states_dispatch(Mamba2Params p, cudaStream_t stream) {
-    p.lo_H = nullptr;
     if (p.K == 128 && p.V == 64) return launch_states<128, 64, M2_MLOW>(p, stream);
     if (p.K == 64 && p.V == 64) return launch_states<64, 64, M2_MLOW>(p, stream);
     return LLATTN_ERR_UNSUPPORTED_SHAPE;

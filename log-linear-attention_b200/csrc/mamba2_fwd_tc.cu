@@ -997,7 +997,7 @@ int mamba2_fwd_one_segment_tc_launch(const Mamba2Params& p_in, cudaStream_t stre
 
 // Heads per CTA: the fewest rounds of CTAs over the SMs, a CTA counted as its heads and two more (q, k, S, tables).  Many heads share S and the loads of
 // q and k; few fill the chip when a call is small.
-static int heads_per_cta(const Mamba2Params& p, int sms) {
+int mamba2_heads_per_cta(const Mamba2Params& p, int sms) {
     int reads = 1;                                   // levels that a pair reads at most
     while ((p.NT + 1) / 2 > 1 << reads) ++reads;
     const int per_grp = p.H / p.G, most = min(min(min(tco::HC_MAX, tco::LAM_MAX / p.L), tco::COEF_MAX / reads), per_grp);
@@ -1049,7 +1049,7 @@ int mamba2_out_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = sm_count(&sms, dev);
     if (e != cudaSuccess) return (int)e;
-    p.hc = heads_per_cta(p, sms);
+    p.hc = mamba2_heads_per_cta(p, sms);
     return p.K == 128 ? launch_out_for<128>(p, stream) : launch_out_for<64>(p, stream);
 }
 

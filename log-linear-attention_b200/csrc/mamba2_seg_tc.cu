@@ -1,399 +1,534 @@
-// Segment-level ("high" Fenwick levels) kernels of the log-linear Mamba-2 path on tcgen05 / TMA
-// (K = 128, V = 64, segments of 2^MLOW chunks = 2^(MLOW-1) pairs of 128 tokens).  Same mathematics
-// as m2_seg_state_kernel (mamba2_fwd.cu) and m2_seg_dstate_kernel /
-// m2_hi_bwd_q_kernel (mamba2_bwd.cu); one CTA per (batch, head, segment) handles every high level
-// of its segment, so q / do / k / v tiles and the level states are loaded once per segment.
-//   state      : F_r      = sum_pairs k^T (v * exp(G_end - G))                      (fp32 K x V), and the level states inside the segment
-//   seg_dstate : dF[r][j] = sum_pairs q^T (do * lambda_j exp(G))                     (fp32 K x V per set level)
-//   hi_bwd_q   : dlambda_j = exp(G) (do . (q H0_j)) ; dq += (do * lambda_j exp(G)) H0_j^T   (TMA reduce-add)
-// G is the cumulative log decay from the start of the segment (inclusive).
+// Level states of the log-linear Mamba-2 path and their gradients on tcgen05 / TMA (K = 64 or 128, V = 64, segments of 2^MLOW chunks = 2^(MLOW-1) pairs of
+// 128 tokens): one CTA per (batch, head, segment) makes the states inside its segment and the segment's summary (forward), or what the readers in its
+// segment send back to the states they read (backward).  Same mathematics as m2_seg_state_kernel (mamba2_fwd.cu) and m2_seg_dstate_kernel (mamba2_bwd.cu),
+// which make the part of the segments' summaries.
 #include "tc_common.cuh"
 
 namespace llattn {
 
-namespace tcs {
-constexpr int MAXLH = 5;            // high levels handled by these kernels (T <= 64 * 2^(MLOW+5))
-}
-
-__device__ __forceinline__ uint32_t box_offset_f32(int row, int col) {
-    return (uint32_t)(row * 128 + (((col >> 2) ^ (row & 7)) << 4) + (col & 3) * 4);
-}
-
-// cumulative log decay of a whole segment (SEG chunks) from its start, inclusive, into sGs[SEG*64];
-// all 256 compute threads call it; returns after a bar_compute
-template <int SEG>
-__device__ __forceinline__ void segment_cumsum(const Mamba2Params& p, int b, int h, int r, int nchunks, float* sGs, float* sTot,
-                                               int warp, int lane, int tid) {
-    // (a pair whose second chunk is beyond the sequence: a chunk without decay)
-    const int npad = (nchunks + 1) & ~1;
-    for (int c = warp; c < npad; c += 8) {
-        const float* gp = p.g + ((long)b * p.T + (long)(r * SEG + c) * CH) * p.H + h;
-        float x0 = 0.f, x1 = 0.f;
-        if (c < nchunks) {
-            x0 = gp[(long)(2 * lane) * p.H];
-            x1 = gp[(long)(2 * lane + 1) * p.H];
-        }
-        warp_cumsum64(x0, x1, lane);
-        sGs[c * CH + 2 * lane] = x0;
-        sGs[c * CH + 2 * lane + 1] = x1;
-        if (lane == 31) sTot[c] = x1;
+// cumulative decay from each pair's start, inclusive, of the chunks [0, 8) of segment r, a chunk per warp (zeros behind the sequence): sG[512]; sTot[8] the chunks'
+__device__ __forceinline__ void segment_pair_sums(const Mamba2Params& p, int b, int h, int r, float* sG, float* sTot, int warp, int lane) {
+    const int c = r * 8 + warp;
+    float x0 = 0.f, x1 = 0.f;
+    if (c < p.NT) {
+        const float* gp = p.g + ((long)b * p.T + (long)c * CH) * p.H + h;
+        x0 = gp[(long)(2 * lane) * p.H];
+        x1 = gp[(long)(2 * lane + 1) * p.H];
     }
+    warp_cumsum64(x0, x1, lane);
+    const float tot = __shfl_sync(0xffffffffu, x1, 31);
+    if (lane == 0) sTot[warp] = tot;
     bar_compute();
-    if (tid == 0) {
-        float run = 0.f;
-        for (int c = 0; c < npad; ++c) {
-            const float t = sTot[c];
-            sTot[c] = run;
-            run += t;
-        }
-        sTot[SEG] = run;
+    const float before = (warp & 1) ? sTot[warp - 1] : 0.f;
+    sG[warp * CH + 2 * lane] = x0 + before;
+    sG[warp * CH + 2 * lane + 1] = x1 + before;
+}
+__device__ __forceinline__ void arrive_on(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(bar)) : "memory");
+}
+// a half row of do (32 columns), times rs, into the same place of a tile
+__device__ __forceinline__ void scaled_half_row(unsigned char* dst, const uint4 (&dox)[4], float rs, int row, int ch) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const uint32_t xw[4] = {dox[c].x, dox[c].y, dox[c].z, dox[c].w};
+        uint32_t out[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) out[e] = pack_bf16(__uint_as_float(xw[e] << 16) * rs, __uint_as_float(xw[e] & 0xffff0000u) * rs);
+        *reinterpret_cast<uint4*>(dst + umma::tile_offset(row, ch * 32 + c * 8, tc::PT)) = make_uint4(out[0], out[1], out[2], out[3]);
     }
-    bar_compute();
-    for (int i = tid; i < npad * CH; i += 256) sGs[i] += sTot[i / CH];
-    bar_compute();
 }
 
 // ------------------------------------------------------------------------------------------
-// backward: reader summaries dF[r][j] and, in the same pass over the segment, dq / dlambda of the
-// high levels.  Per pair: T_j = q H0_j (one 64-column slot, level after level), dlambda_j and
-// the scaled copy do * (lambda_j exp(G)); then dq (+)= that copy times H0_j^T and dF_j += q^T times it.
+// backward: what the readers of the high level states send back, dF[r][j] = sum over the pairs of segment r of q^T (do lambda_j exp(G)), G from the segment's
+// start, for every set bit j of r: fp32 K x V summaries for the scan over segments.  One CTA per (batch, head, segment); a job is a level of a pair: a
+// scaled copy of do in a ring of stages times q^T, accumulated in the level's tensor-memory slot.
 // ------------------------------------------------------------------------------------------
+namespace tcr {
+constexpr int MAXLH = 5;                 // high levels of one launch
+constexpr int NST = 6, NTHREADS = 320, TMA_WARP = 9;
+}
 template <int MLOW>
-struct HiBwdTcSmem {
+struct ReadersTcSmem {
     static constexpr int SEG = 1 << MLOW;
-    static constexpr uint32_t q_off = 0;                                   // 32 KB
-    static constexpr uint32_t do_off = q_off + tc::Q_BYTES;                // 16 KB
-    static constexpr uint32_t h_off = do_off + tc::V_BYTES;                // MAXLH x 16 KB states
-    static constexpr uint32_t dos_off = h_off + tcs::MAXLH * tc::H_BYTES;  // MAXLH x 16 KB scaled do ; first 64 KB double as fp32 staging
-    static constexpr uint32_t gs_off = dos_off + tcs::MAXLH * tc::V_BYTES; // float [SEG*64] + [SEG+1]
-    static constexpr uint32_t misc_off = gs_off + (SEG * 64 + SEG + 32) * 4;  // float [2][128][MAXLH+1] dlambda halves
-    static constexpr uint32_t bar_off = misc_off + 2 * 128 * (tcs::MAXLH + 1) * 4;
-    static constexpr uint32_t sink_off = bar_off + 128;                    // uint32 [256], written only (tile release)
-    static constexpr uint32_t total = sink_off + 256 * 4 + 1024;
+    static constexpr uint32_t q_off = 0;                                   // [2] 32 KB
+    static constexpr uint32_t do_off = q_off + 2 * tc::Q_BYTES;            // [2] 16 KB
+    static constexpr uint32_t st_off = do_off + 2 * tc::V_BYTES;           // [NST] 16 KB
+    static constexpr uint32_t gs_off = st_off + tcr::NST * tc::V_BYTES;    // float [SEG * 64], [SEG]
+    static constexpr uint32_t lam_off = gs_off + (SEG * 64 + SEG) * 4;     // bf16 [MAXLH][SEG * 64]
+    static constexpr uint32_t bar_off = lam_off + tcr::MAXLH * SEG * 64 * 2;
+    static constexpr uint32_t total = bar_off + 256 + 1024;
 };
 
-template <int MLOW, bool WHOLE>
-__global__ void __launch_bounds__(tc::NTHREADS, 1) m2_hi_bwd_tc_kernel(const __grid_constant__ Mamba2Params p) {
+template <int MLOW>
+__global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
-    using SM = HiBwdTcSmem<MLOW>;
-    constexpr int SEG = SM::SEG, NDLH = tcs::MAXLH + 1;
-    // tensor memory: dF slots 0..4 (64 columns each), dq (128 columns), T (64 columns).  The level reads
-    // T_j use three adjacent 64-column slots: the two halves of dq (only written after every T of the pair
-    // has been consumed) and T.
-    constexpr int TM_DF = 0, TM_DQ = 320;      // the third T slot is the 64 columns after dq (448..511)
+    using SM = ReadersTcSmem<MLOW>;
+    constexpr int SEG = SM::SEG, SEGP = SEG / 2;
+    static_assert(SEG == 8, "a chunk per warp");
     extern __shared__ unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    unsigned char* smem = umma::align_1024(smem_raw);
     unsigned char* sQ = smem + SM::q_off;
     unsigned char* sDO = smem + SM::do_off;
-    unsigned char* sH = smem + SM::h_off;
-    unsigned char* sDOs = smem + SM::dos_off;
-    unsigned char* sStage = smem + SM::dos_off;
+    unsigned char* sSt = smem + SM::st_off;
     float* sGs = reinterpret_cast<float*>(smem + SM::gs_off);
     float* sTot = sGs + SEG * 64;
-    float* sDL = reinterpret_cast<float*>(smem + SM::misc_off);
+    bf16* sLam = reinterpret_cast<bf16*>(smem + SM::lam_off);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
-    uint64_t* barT = bars + 0;       // [2] first / second chain of level reads complete ([2] unused)
-    uint64_t* barB = bars + 3;       // second batch of a pair complete
-    uint64_t* full_q = bars + 4;     // q tile of a pair
-    uint64_t* full_do = bars + 5;    // do tile of a pair
-    uint64_t* full_h = bars + 6;     // the level states of the segment
-    uint64_t* empty_q = bars + 7;    // second batch done: q may be overwritten
-    uint64_t* empty_do = bars + 8;   // every compute thread holds its do row in registers (256 arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 96);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 104);
-    uint32_t* sink = reinterpret_cast<uint32_t*>(smem + SM::sink_off);
+    uint64_t* full = bars + 0;       // [2] q and do of a pair
+    uint64_t* empty = bars + 2;      // [2] (the products of a pair wait for every thread's copies of its do)
+    uint64_t* done = bars + 4;
+    uint64_t* st_full = bars + 5;    // [NST] 8: a scaled copy is written
+    uint64_t* st_empty = bars + 5 + tcr::NST;
+    constexpr int NBARS = 5 + 2 * tcr::NST;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 200);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 208);
+    static_assert(NBARS * 8 <= 200, "barriers");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#ifdef LLATTN_STAMPS
-    // one CTA's life: entry, before / after the segment's cumulative decay, top of each pair, end of the pairs, reader summaries
-    // written, reduce-adds complete, exit (thread 0)
-    int nstamp = 0;
-    const int stamp_slot = (blockIdx.x == 700 && tid == 0) ? 0 : -1;
-#endif
-    STAMP();
+    const int NP = (p.NT + 1) / 2;
     const int h = blockIdx.x % p.H;
     const int r = 1 + (blockIdx.x / p.H) % (p.NS - 1);
     const int b = blockIdx.x / (p.H * (p.NS - 1));
     const int grp = h / (p.H / p.G);
-    const int nchunks = min(SEG, p.NT - r * SEG);
-    const int npairs = (nchunks + 1) / 2;
-    // set high levels of this segment inside this launch's window of five levels, in increasing order
-    int lev[tcs::MAXLH], nl = 0;
-#pragma unroll
-    for (int jj = 0; jj < tcs::MAXLH; ++jj) {
-        const int j = p.lev_lo + jj;
-        if (j < p.LH && ((r >> j) & 1)) lev[nl++] = j;
-    }
-    if (nl == 0) return;             // nothing to read in this window (uniform for the CTA)
+    const long bh = (long)b * p.H + h;
+    const int npairs = min(SEGP, NP - r * SEGP);
+    // set high levels of this segment inside this launch's window of five levels
+    const int himask = (r >> p.lev_lo) & ((1 << tcr::MAXLH) - 1), nl = __popc(himask);
+    if (nl == 0) return;                     // (uniform)
 
-    if (tid == 0) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) umma::mbar_init(&bars[i], 1);
-        umma::mbar_init(empty_do, 256);
+    if (tid == tcr::TMA_WARP * 32) {
+        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], i >= 5 && i < 5 + tcr::NST ? 8 : 1);
         umma::fence_mbar_init();
         *abort_flag = *p.err;
     }
     __syncthreads();
     if (*abort_flag) return;
-
-    constexpr uint32_t ID_KK128 = umma::idesc_bf16(128, 128, false, false);
-    constexpr uint32_t ID_MM64 = umma::idesc_bf16(128, 64, true, true);
-    auto t_slot = [&](int i) -> uint32_t { return (uint32_t)(TM_DQ + (i % 3) * 64); };   // three adjacent 64-column slots
-
-    if (warp >= tc::MMA_WARP) {
-        RegisterSplit<120, 192>::release();
-        if (warp == tc::MMA_WARP + 1) {
-            if (lane == 0) {
-                // level states of the segment, K x V matrices (rows beyond K: zeros)
-                tma::expect_tx(full_h, nl * tc::H_BYTES);
-                for (int i = 0; i < nl; ++i) {
-                    const int at = (((b * p.H + h) * p.NS + r) * p.LH) + lev[i];
-                    if (WHOLE) tma::load_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, at * tc::KD, full_h);
-                    else tma::load_seq_panel(sH + i * tc::H_BYTES, &p.tm_h0, 0, 0, 0, at, full_h);
-                }
-                const int brow = r * SEG * CH;
-                for (int pl = 0; pl < npairs; ++pl) {
-                    const int row0 = brow + pl * tc::PT;
-                    if (pl >= 1 && !umma::mbar_wait(empty_do, (pl - 1) & 1, abort_flag)) break;
-                    tma::expect_tx(full_do, tc::V_BYTES);
-                    tma::load_seq_panel(sDO, &p.tm_do, 0, h, row0, b, full_do);
-                    if (pl >= 1 && !umma::mbar_wait(empty_q, (pl - 1) & 1, abort_flag)) break;
-                    tma::expect_tx(full_q, tc::Q_BYTES);
-                    tma::load_seq_panel(sQ, &p.tm_q, 0, grp, row0, b, full_q);
-                    tma::load_seq_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, full_q);
-                }
-            }
-            return;
+    if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tc::TM_COLS);
+    if (warp < 8) {
+        // lambda of the levels read
+        const int base = INTRA_LEVELS + MLOW + p.lev_lo;
+        for (int e = tid; e < SEG * 64 * tcr::MAXLH; e += 256) {
+            const int i = e / tcr::MAXLH, j = e - i * tcr::MAXLH, t = r * SEG * 64 + i;
+            if ((himask >> j) & 1) sLam[j * SEG * 64 + i] = t < p.T ? p.l[(((long)b * p.T + t) * p.H + h) * p.L + base + j] : __float2bfloat16(0.f);
         }
-        if (warp > tc::MMA_WARP) return;
-        umma::tmem_alloc(tmem_slot, tc::TM_COLS);
-        umma::fence_before_sync();
-        bar_work();
-        umma::fence_after_sync();
-        const uint32_t tbase = *tmem_slot;
-        const uint32_t aQ = umma::smem_addr(sQ), aH = umma::smem_addr(sH), aDOs = umma::smem_addr(sDOs);
-        if (lane == 0) umma::mbar_wait(full_h, 0, abort_flag);
-        for (int pl = 0; pl < npairs; ++pl) {
-            if (lane == 0) umma::mbar_wait(full_q, pl & 1, abort_flag);
-            __syncwarp();
-            umma::fence_after_sync();
-            // The issue of a tcgen05.mma costs about as much for N = 64 as for N = 256, so the level reads of up
-            // to three levels are ONE chain of eight instructions: the level states are adjacent 64-column
-            // panels of an MN-major B operand and their results adjacent tensor-memory slots.
-            {
-                const int n0 = nl < 3 ? nl : 3;
-                if (lane == 0) {
-                    umma::gemm_km<tc::PT, tc::KD, tc::KD>(tbase + TM_DQ, aQ, aH, umma::idesc_bf16(128, 64 * n0, false, true), false);
-                    umma::commit(&barT[0]);
-                }
-                __syncwarp();
-                if (nl > 3) {
-                    bar_work();                      // the three slots have been read by the compute warps
-                    umma::fence_after_sync();
-                    if (lane == 0) {
-                        umma::gemm_km<tc::PT, tc::KD, tc::KD>(tbase + TM_DQ, aQ, aH + 3 * tc::H_BYTES,
-                                                              umma::idesc_bf16(128, 64 * (nl - 3), false, true), false);
-                        umma::commit(&barT[1]);
-                    }
-                    __syncwarp();
-                }
-            }
-            umma::fence_before_sync();
-            bar_work();                              // scaled copies of do are written, every T consumed
-            umma::fence_after_sync();
-            if (lane == 0) {
-                // reader summaries of up to four levels per chain (N = 256), then dq over all levels
-                const int n0 = nl < 4 ? nl : 4;
-                umma::gemm_mm<tc::PT, tc::PT, tc::PT>(tbase + TM_DF, aQ, aDOs, umma::idesc_bf16(128, 64 * n0, true, true), pl > 0);
-                if (nl > 4)
-                    umma::gemm_mm<tc::PT, tc::PT, tc::PT>(tbase + TM_DF + 4 * 64, aQ, aDOs + 4 * tc::V_BYTES, ID_MM64, pl > 0);
-                for (int i = 0; i < nl; ++i)
-                    umma::gemm_kk<tc::PT, tc::KD, tc::VD>(tbase + TM_DQ, aDOs + i * tc::V_BYTES, aH + i * tc::H_BYTES, ID_KK128, i > 0);
-                umma::commit(barB);
-                // q is free as soon as the batch is done: let the producer refill it while dq is read out
-                umma::mbar_wait(barB, pl & 1, abort_flag);
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(empty_q)) : "memory");
-            }
-            __syncwarp();
-            umma::fence_before_sync();
-            bar_work();                              // end of the pair: dq has left tensor memory
-            umma::fence_after_sync();
-            if (*abort_flag) break;
-        }
-        if (*abort_flag && lane == 0) atomicExch(p.err, 1);
-        umma::fence_before_sync();
-        bar_work();
-        umma::tmem_dealloc(tbase, tc::TM_COLS);
-        return;
+        segment_pair_sums(p, b, h, r, sGs, sTot, warp, lane);
     }
-
-    // ================= warps 0..7 =================
-    RegisterSplit<120, 192>::acquire();
-    const int rb = warp & 3;
-    const int row = rb * 32 + lane;
-    const int ch = warp >> 2;
-    STAMP();
-    segment_cumsum<SEG>(p, b, h, r, nchunks, sGs, sTot, warp, lane, tid);
-    STAMP();
     umma::fence_before_sync();
-    bar_work();
+    __syncthreads();
     umma::fence_after_sync();
     const uint32_t tbase = *tmem_slot;
-    uint32_t phT[2] = {0, 0};
 
-    // this row's lambda of the levels read: requested one pair ahead, so that the loads' latency is not part of a pair
-    bf16 lam_next[tcs::MAXLH];
-    auto fetch_lambda = [&](int pl) {
-        const long t0 = (long)(r * SEG) * CH + (long)pl * tc::PT;
-        const bf16* lrow = p.l + (((long)b * p.T + t0 + row) * p.H + h) * p.L + INTRA_LEVELS + MLOW;
-#pragma unroll
-        for (int i = 0; i < tcs::MAXLH; ++i)
-            if (i < nl) lam_next[i] = (WHOLE || t0 + row < p.T) ? lrow[lev[i]] : __float2bfloat16(0.f);
-    };
-    fetch_lambda(0);
-
-    for (int pl = 0; pl < npairs; ++pl) {
-        STAMP();
-        const long t0 = (long)(r * SEG) * CH + (long)pl * tc::PT;
-        const float sc = fexp(sGs[pl * tc::PT + row]);          // exp(G_i) from the segment start
-        float lamv[tcs::MAXLH];
-#pragma unroll
-        for (int i = 0; i < tcs::MAXLH; ++i) lamv[i] = (i < nl) ? __bfloat162float(lam_next[i]) : 0.f;
-        if (pl + 1 < npairs) fetch_lambda(pl + 1);
-        umma::mbar_wait(full_do, pl & 1, abort_flag);
-        uint4 dox[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) dox[c] = *reinterpret_cast<const uint4*>(sDO + umma::tile_offset(row, ch * 32 + c * 8, tc::PT));
-        {
-            // every thread holds its do row in registers: hand the tile back to the producer (the release must
-            // follow the loads, see release_tile_after_loads)
-            const uint32_t x = dox[0].x ^ dox[0].y ^ dox[0].z ^ dox[0].w ^ dox[1].x ^ dox[1].y ^ dox[1].z ^ dox[1].w ^
-                               dox[2].x ^ dox[2].y ^ dox[2].z ^ dox[2].w ^ dox[3].x ^ dox[3].y ^ dox[3].z ^ dox[3].w;
-            release_tile_after_loads(empty_do, sink + tid, x);
+    if (warp == tcr::TMA_WARP) {
+        if (lane == 0) {
+            int pl = 0;
+            for (; pl < npairs; ++pl) {
+                const int st = pl & 1, row0 = (r * SEGP + pl) * tc::PT;
+                if (pl >= 2 && !umma::mbar_wait(&empty[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
+                tma::expect_tx(&full[st], tc::Q_BYTES + tc::V_BYTES);
+                tma::load_seq_panel(sDO + st * tc::V_BYTES, &p.tm_do, 0, h, row0, b, &full[st]);
+                tma::load_seq_panel(sQ + st * tc::Q_BYTES, &p.tm_q, 0, grp, row0, b, &full[st]);
+                tma::load_seq_panel(sQ + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, &full[st]);
+            }
+            // every load is waited for by the MMA warp, unless a wait gave up: nothing may still be on its way into shared memory when the CTA ends
+            for (int i = max(0, pl - 2); i < pl; ++i) umma::mbar_wait(&full[i & 1], (i >> 1) & 1, 1u << 16);
         }
-        float* myDL = sDL + (ch * 128 + row) * NDLH;
-        for (int i = 0; i < nl; ++i) {
-            if (i == 0 || i == 3) {                  // one completion per chain of level reads
-                umma::mbar_wait(&barT[i / 3], phT[i / 3], abort_flag);
-                phT[i / 3] ^= 1;
+        __syncwarp();
+    } else if (warp == tc::MMA_WARP) {
+        // (the whole warp, see umma::elect_one)
+        constexpr uint32_t ID_MM64 = umma::idesc_bf16(128, 64, true, true);
+        const uint32_t lead = umma::elect_one();
+        auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, umma::mbar_wait(bar, parity, abort_flag)); };
+        int st = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int pl = 0; pl < npairs && ok; ++pl) {
+            if (!(ok = wait(&full[pl & 1], (pl >> 1) & 1))) break;
+            const uint32_t aQ = umma::smem_addr(sQ + (pl & 1) * tc::Q_BYTES);
+            for (int i = 0; i < nl; ++i) {
+                if (!(ok = wait(&st_full[st], ph))) break;
                 umma::fence_after_sync();
-            }
-            float t[32];
-            umma::tmem_ld32(umma::tmem_addr(tbase + t_slot(i), warp, ch * 32), t);
-            if (i == 2 && nl > 3) {
-                umma::fence_before_sync();
-                bar_work();                          // the three slots may be reused
-            }
-            if (i < 4) {
-                // The staging area of the previous pair's dq tile is the memory of the first four scaled copies: box i of
-                // the reduce-add (its own bulk group) must have been read before copy i is written.  Waiting box by box
-                // lets the first copy start after a quarter of the read.
-                if (tid == 0) {
-                    if (i == 0) tma::wait_group_read<3>();
-                    else if (i == 1) tma::wait_group_read<2>();
-                    else if (i == 2) tma::wait_group_read<1>();
-                    else tma::wait_group_read<0>();
+                umma::gemm_mm_lead<tc::PT, tc::PT, tc::PT>(lead, tbase + i * 64, aQ, umma::smem_addr(sSt + st * tc::V_BYTES), ID_MM64, pl > 0);
+                umma::commit_lead(lead, &st_empty[st]);
+                if (++st == tcr::NST) {
+                    st = 0;
+                    ph ^= 1;
                 }
+            }
+            umma::commit_lead(lead, &empty[pl & 1]);
+        }
+        umma::commit_lead(lead, done);
+        if (!ok) umma::mbar_wait(done, 0, 1u << 16);     // gave up: no product may still read shared memory when the CTA ends
+        __syncwarp();
+    } else {
+        const int rb = warp & 3, row = rb * 32 + lane, ch = warp >> 2;
+        int st = 0;
+        uint32_t ph = 1;
+        float before = 0.f;                          // decay of the segment's pairs before this one
+        for (int pl = 0; pl < npairs; ++pl) {
+            const float ehi = fexp(sGs[pl * tc::PT + row] + before);
+            before += sGs[pl * tc::PT + tc::PT - 1];
+            umma::mbar_wait(&full[pl & 1], (pl >> 1) & 1, abort_flag);
+            uint4 dox[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                dox[c] = *reinterpret_cast<const uint4*>(sDO + (pl & 1) * tc::V_BYTES + umma::tile_offset(row, ch * 32 + c * 8, tc::PT));
+            int bits = himask;
+            for (int i = 0; i < nl; ++i) {
+                const int j = __ffs(bits) - 1;
+                bits &= bits - 1;
+                const float rs = __bfloat162float(sLam[j * SEG * 64 + pl * tc::PT + row]) * ehi;
+                umma::mbar_wait(&st_empty[st], ph, abort_flag);
+                scaled_half_row(sSt + st * tc::V_BYTES, dox, rs, row, ch);
+                umma::fence_async_smem();
+                __syncwarp();
+                if (lane == 0) arrive_on(&st_full[st]);
+                if (++st == tcr::NST) {
+                    st = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+        umma::mbar_wait(done, 0, abort_flag);
+        umma::fence_after_sync();
+        // the summaries leave in boxes of 32 columns by way of the ring, two levels at a time
+        int bits = himask;
+        for (int i = 0; i < nl; ++i) {
+            const int j = p.lev_lo + __ffs(bits) - 1;
+            bits &= bits - 1;
+            float t[32];
+            umma::tmem_ld32(umma::tmem_addr(tbase + i * 64, warp, ch * 32), t);
+            unsigned char* box = sSt + ((i & 1) * 2 + ch) * tc::V_BYTES;
+            if (i >= 2) {
+                if (tid == 0) tma::wait_group_read1();
                 bar_compute();
             }
-            const float rs = lamv[i] * sc;
-            float dot = 0.f;
-            unsigned char* dst = sDOs + i * tc::V_BYTES;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const uint32_t* xw = reinterpret_cast<const uint32_t*>(&dox[c]);
-                uint32_t outw[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    __nv_bfloat162 v2 = *reinterpret_cast<const __nv_bfloat162*>(&xw[e]);
-                    const float a0 = __bfloat162float(v2.x), a1 = __bfloat162float(v2.y);
-                    dot += a0 * t[c * 8 + e * 2] + a1 * t[c * 8 + e * 2 + 1];
-                    outw[e] = pack_bf16(a0 * rs, a1 * rs);
-                }
-                *reinterpret_cast<uint4*>(dst + umma::tile_offset(row, ch * 32 + c * 8, tc::PT)) = make_uint4(outw[0], outw[1], outw[2], outw[3]);
-            }
-            myDL[i] = sc * dot;
-        }
-        umma::fence_async_smem();
-        umma::fence_before_sync();
-        bar_work();                                  // scaled copies written; second batch may start
-        umma::fence_after_sync();
-        // ---- dlambda out, reader totals Z per chunk, q.dq contribution
-        {
-            // the two warps of a lane quarter take alternate levels
-            float* gdl = p.dl + (((long)b * p.T + t0 + row) * p.H + h) * p.L + INTRA_LEVELS + MLOW;
-            float wsum = 0.f;
-            for (int i = ch; i < nl; i += 2) {
-                const float dlv = sDL[row * NDLH + i] + sDL[(128 + row) * NDLH + i];
-                if (WHOLE || t0 + row < p.T) gdl[lev[i]] = dlv;
-                float z = lamv[i] * dlv;
-                wsum += z;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) z += __shfl_xor_sync(0xffffffffu, z, d);
-                if (lane == 0) sTot[SEG + 1 + rb * tcs::MAXLH + i] = z;        // per 32-row block
-            }
-            if (ch < nl && (WHOLE || t0 + row < p.T)) red_add_f32(p.wq + ((long)b * p.T + t0 + row) * p.H + h, wsum);
-        }
-        umma::mbar_wait(barB, pl & 1, abort_flag);
-        umma::fence_after_sync();
-        if (nl < 4) {
-            // boxes nl..3 of the previous pair's reduce-add were not waited for above
-            if (tid == 0) tma::wait_group_read<0>();
-            bar_compute();
-        }
-        // ---- dq tile -> fp32 staging (the scaled copies are no longer needed) -> TMA reduce-add
-#pragma unroll
-        for (int hb = 0; hb < 2; ++hb) {
-            float t[32];
-            umma::tmem_ld32(umma::tmem_addr(tbase + TM_DQ, warp, ch * 64 + hb * 32), t);
-            unsigned char* box = sStage + (ch * 2 + hb) * 16384;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
-                *reinterpret_cast<float4*>(box + box_offset_f32(row, c * 4)) = make_float4(t[c * 4], t[c * 4 + 1], t[c * 4 + 2], t[c * 4 + 3]);
-        }
-        umma::fence_async_smem();
-        umma::fence_before_sync();
-        bar_compute();
-        if (tid == 0) {
-            const int grow = (int)t0;
-#pragma unroll
-            for (int bx = 0; bx < 4; ++bx) {
-                if (WHOLE || bx * 32 < p.K) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, grp, grow, b, sStage + bx * 16384);
-                tma::commit_group();                 // one group per box: the next pair waits for them one by one
+                *reinterpret_cast<float4*>(box + row * 128 + ((c ^ (row & 7)) << 4)) = make_float4(t[c * 4], t[c * 4 + 1], t[c * 4 + 2], t[c * 4 + 3]);
+            umma::fence_async_smem();
+            bar_compute();
+            if (tid == 0) {
+                const int at = (int)(((bh * p.NS + r) * p.LH + j) * p.K);
+                if (!*abort_flag)
+                    for (int bx = 0; bx < 2; ++bx) tma::store_box(&p.tm_df, bx * 32, 0, at, sSt + ((i & 1) * 2 + bx) * tc::V_BYTES);
+                tma::commit_group();
             }
         }
-        if (tid < 2 * nl) {
-            const int i = tid >> 1, cpart = tid & 1;
-            const float z = sTot[SEG + 1 + (cpart * 2) * tcs::MAXLH + i] + sTot[SEG + 1 + (cpart * 2 + 1) * tcs::MAXLH + i];
-            const long cidx = ((long)b * p.H + h) * p.NT + r * SEG + pl * 2 + cpart;
-            if (WHOLE || pl * 2 + cpart < nchunks) p.Zc[cidx * p.LZ + MLOW + lev[i]] = z;
-        }
-        umma::fence_before_sync();
-        bar_work();                                  // end of the pair
-        umma::fence_after_sync();
-        if (*abort_flag) break;
+        if (tid == 0) tma::wait_group0();
     }
-    STAMP();
-    // ---- dF[r][j] out
-    for (int i = 0; i < nl; ++i) {
-        float t[32];
-        umma::tmem_ld32(umma::tmem_addr(tbase + TM_DF + i * 64, warp, ch * 32), t);
-        float* dF = p.seg_dF + ((((long)b * p.H + h) * p.NS + r) * p.LH + lev[i]) * (WHOLE ? tc::KD : p.K) * tc::VD + row * tc::VD + ch * 32;
-        if (WHOLE || row < p.K)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            uint32_t w[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(t[c * 8 + e]);
-            st_global_32B(dF + c * 8, w);            // a thread owns its row: 32-byte stores fill whole sectors
-        }
-    }
-    STAMP();
-    if (tid == 0) tma::wait_group0();
-    STAMP();
     umma::fence_before_sync();
-    bar_work();
-    STAMP();
+    __syncthreads();
+    umma::fence_after_sync();
+    if (warp == tc::MMA_WARP) {
+        if (*abort_flag && lane == 0) atomicExch(p.err, 1);
+        umma::tmem_dealloc(tbase, tc::TM_COLS);
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// backward: the gradient of every pair's summary.  One CTA per (batch, head, segment):
+//   R_pl,l = q^T (do lambda_l exp(G))        pairs 1.. of the segment, the pair levels that they read (tensor memory, fp32)
+//   A_pl   = what comes back to pair pl: from later segments, from the pairs of its segment that read a state with it    (one bf16 tile, fp32 until then)
+//   Y      = <k^T (v exp(G_end - G)) of each chunk, A's parts>     contributor totals per level, from the fp32 parts
+// The segment's pairs are walked in order for R, then in reverse for A and Y.
+// ------------------------------------------------------------------------------------------
+namespace tca {
+constexpr int NST = 3, NTHREADS = 320, TMA_WARP = 9;
+constexpr int SLOT_KV = 4;               // slots 0..3: R of (pair 1, level 0), (2, 1), (3, 1), (3, 0); 4..7: two pairs of chunk summaries
+}
+template <int MLOW>
+struct AdjointTcSmem {
+    static constexpr int SEG = 1 << MLOW;
+    static constexpr uint32_t x_off = 0;                                   // [2] 32 KB: q, then k
+    static constexpr uint32_t y_off = x_off + 2 * tc::Q_BYTES;             // [2] 16 KB: do, then v (scaled in place)
+    static constexpr uint32_t st_off = y_off + 2 * tc::V_BYTES;            // [NST] 16 KB: scaled copies of do, then A on its way out
+    static constexpr uint32_t hi_off = st_off + tca::NST * tc::V_BYTES;    // 32 KB: fp32 gradient of the segment's summary, two boxes of 32 columns
+    static constexpr uint32_t gs_off = hi_off + 2 * tc::V_BYTES;           // float [SEG * 64], [SEG]
+    static constexpr uint32_t y_sum_off = gs_off + (SEG * 64 + SEG) * 4;   // float [8][8]
+    static constexpr uint32_t lam_off = y_sum_off + 64 * 4;                // bf16 [2][SEG * 64]
+    static constexpr uint32_t bar_off = lam_off + 2 * SEG * 64 * 2;
+    static constexpr uint32_t total = bar_off + 256 + 1024;
+};
+
+template <int MLOW>
+__global__ void __launch_bounds__(tca::NTHREADS, 1) m2_adjoint_tc_kernel(const __grid_constant__ Mamba2Params p) {
+    chain_wait();
+    using SM = AdjointTcSmem<MLOW>;
+    constexpr int SEG = SM::SEG, SEGP = SEG / 2;
+    static_assert(SEG == 8, "a chunk per warp, four pairs");
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = umma::align_1024(smem_raw);
+    unsigned char* sX = smem + SM::x_off;
+    unsigned char* sY = smem + SM::y_off;
+    unsigned char* sSt = smem + SM::st_off;
+    unsigned char* sHi = smem + SM::hi_off;
+    float* sGs = reinterpret_cast<float*>(smem + SM::gs_off);
+    float* sTot = sGs + SEG * 64;
+    float* sYs = reinterpret_cast<float*>(smem + SM::y_sum_off);
+    bf16* sLam = reinterpret_cast<bf16*>(smem + SM::lam_off);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
+    uint64_t* full = bars + 0;       // [2]
+    uint64_t* empty = bars + 2;      // [2]
+    uint64_t* hi_full = bars + 4;
+    uint64_t* r_full = bars + 5;     // every R is complete
+    uint64_t* scaled = bars + 6;     // [2] 8: v is scaled
+    uint64_t* kv_full = bars + 8;    // [2]
+    uint64_t* st_full = bars + 10;   // [NST] 8
+    uint64_t* st_empty = bars + 10 + tca::NST;
+    constexpr int NBARS = 10 + 2 * tca::NST;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 200);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 208);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NP = (p.NT + 1) / 2;
+    const int h = blockIdx.x % p.H;
+    const int r = (blockIdx.x / p.H) % p.NS;
+    const int b = blockIdx.x / (p.H * p.NS);
+    const int grp = h / (p.H / p.G);
+    const long bh = (long)b * p.H + h;
+    const int npairs = min(SEGP, NP - r * SEGP);
+    const bool later = r < p.NS - 1;                 // later segments read this one's summary
+    const int nr = npairs - 1, nc = later ? SEGP : npairs - 1;      // pairs that read, pairs that are read
+
+    if (tid == tca::TMA_WARP * 32) {
+        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], i == 6 || i == 7 || (i >= 10 && i < 10 + tca::NST) ? 8 : 1);
+        umma::fence_mbar_init();
+        *abort_flag = *p.err;
+    }
+    __syncthreads();
+    if (*abort_flag) return;
+    if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tc::TM_COLS);
+    if (warp < 8) {
+        for (int e = tid; e < SEG * 64 * 2; e += 256) {
+            const int i = e >> 1, j = e & 1, t = r * SEG * 64 + i;
+            sLam[j * SEG * 64 + i] = t < p.T && 8 + j < p.L ? p.l[(((long)b * p.T + t) * p.H + h) * p.L + 8 + j] : __float2bfloat16(0.f);
+        }
+        segment_pair_sums(p, b, h, r, sGs, sTot, warp, lane);
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tbase = *tmem_slot;
+
+    // steps: q, do of the pairs 1..nr, then k, v of the pairs nc - 1..0
+    if (warp == tca::TMA_WARP) {
+        if (lane == 0) {
+            if (later) {
+                tma::expect_tx(hi_full, p.K * tc::VD * 4);
+                for (int bx = 0; bx < 2; ++bx) tma::load_panel(sHi + bx * tc::V_BYTES, &p.tm_dh, bx * 32, 0, (int)((bh * p.NS + r) * p.K), hi_full);
+            }
+            int s = 0;
+            for (; s < nr + nc; ++s) {
+                const int st = s & 1, pl = s < nr ? s + 1 : nc - 1 - (s - nr), row0 = (r * SEGP + pl) * tc::PT;
+                if (s >= 2 && !umma::mbar_wait(&empty[st], ((s - 2) >> 1) & 1, abort_flag)) break;
+                tma::expect_tx(&full[st], tc::Q_BYTES + tc::V_BYTES);
+                tma::load_seq_panel(sY + st * tc::V_BYTES, s < nr ? &p.tm_do : &p.tm_v, 0, h, row0, b, &full[st]);
+                tma::load_seq_panel(sX + st * tc::Q_BYTES, s < nr ? &p.tm_q : &p.tm_k, 0, grp, row0, b, &full[st]);
+                tma::load_seq_panel(sX + st * tc::Q_BYTES + tc::Q_BYTES / 2, s < nr ? &p.tm_q : &p.tm_k, 64, grp, row0, b, &full[st]);
+            }
+            // (see m2_readers_tc_kernel)
+            for (int i = max(0, s - 2); i < s; ++i) umma::mbar_wait(&full[i & 1], (i >> 1) & 1, 1u << 16);
+            if (later) umma::mbar_wait(hi_full, 0, 1u << 16);
+        }
+        __syncwarp();
+    } else if (warp == tc::MMA_WARP) {
+        constexpr uint32_t ID_MM64 = umma::idesc_bf16(128, 64, true, true);
+        const uint32_t lead = umma::elect_one();
+        auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, umma::mbar_wait(bar, parity, abort_flag)); };
+        int st = 0, s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        auto job = [&](uint32_t aQ, int slot) -> bool {
+            if (!wait(&st_full[st], ph)) return false;
+            umma::fence_after_sync();
+            umma::gemm_mm_lead<tc::PT, tc::PT, tc::PT>(lead, tbase + slot * 64, aQ, umma::smem_addr(sSt + st * tc::V_BYTES), ID_MM64, false);
+            umma::commit_lead(lead, &st_empty[st]);
+            if (++st == tca::NST) {
+                st = 0;
+                ph ^= 1;
+            }
+            return true;
+        };
+        for (; s < nr && ok; ++s) {
+            const int pl = s + 1;
+            if (!(ok = wait(&full[s & 1], (s >> 1) & 1))) break;
+            const uint32_t aQ = umma::smem_addr(sX + (s & 1) * tc::Q_BYTES);
+            if (pl & 1) ok = job(aQ, pl == 1 ? 0 : 3);
+            if (ok && pl >= 2) ok = job(aQ, pl - 1);
+            umma::commit_lead(lead, &empty[s & 1]);
+        }
+        umma::commit_lead(lead, r_full);
+        for (; s < nr + nc && ok; ++s) {
+            const int i = s - nr;
+            if (!(ok = wait(&scaled[i & 1], (i >> 1) & 1))) break;
+            umma::fence_after_sync();
+            const uint32_t aK = umma::smem_addr(sX + (s & 1) * tc::Q_BYTES), aV = umma::smem_addr(sY + (s & 1) * tc::V_BYTES);
+            const uint32_t d = tbase + (tca::SLOT_KV + (i & 1) * 2) * 64;
+            umma::gemm_mm_lead<tc::PT, tc::PT, 64>(lead, d, aK, aV, ID_MM64, false);                                           // first chunk of the pair
+            umma::gemm_mm_lead<tc::PT, tc::PT, 64>(lead, d + 64, aK + 64 * umma::ROW_BYTES, aV + 64 * umma::ROW_BYTES, ID_MM64, false);
+            umma::commit_lead(lead, &empty[s & 1]);
+            umma::commit_lead(lead, &kv_full[i & 1]);
+        }
+        if (!ok) umma::mbar_wait(r_full, 0, 1u << 16);   // gave up: no product may still read shared memory when the CTA ends (the later ones are short)
+        __syncwarp();
+    } else {
+        const int rb = warp & 3, row = rb * 32 + lane, ch = warp >> 2;
+        {
+            int st = 0;
+            uint32_t ph = 1;
+            auto copy = [&](const uint4 (&dox)[4], float rs) {
+                umma::mbar_wait(&st_empty[st], ph, abort_flag);
+                scaled_half_row(sSt + st * tc::V_BYTES, dox, rs, row, ch);
+                umma::fence_async_smem();
+                __syncwarp();
+                if (lane == 0) arrive_on(&st_full[st]);
+                if (++st == tca::NST) {
+                    st = 0;
+                    ph ^= 1;
+                }
+            };
+            for (int s = 0; s < nr; ++s) {
+                const int pl = s + 1;
+                const float e = fexp(sGs[pl * tc::PT + row]);
+                umma::mbar_wait(&full[s & 1], (s >> 1) & 1, abort_flag);
+                uint4 dox[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    dox[c] = *reinterpret_cast<const uint4*>(sY + (s & 1) * tc::V_BYTES + umma::tile_offset(row, ch * 32 + c * 8, tc::PT));
+                if (pl & 1) copy(dox, __bfloat162float(sLam[pl * tc::PT + row]) * e);
+                if (pl >= 2) copy(dox, __bfloat162float(sLam[SEG * 64 + pl * tc::PT + row]) * e);
+            }
+        }
+        auto scale_v = [&](int i) {
+            const int s = nr + i, pl = nc - 1 - i;
+            umma::mbar_wait(&full[s & 1], (s >> 1) & 1, abort_flag);
+            unsigned char* cV = sY + (s & 1) * tc::V_BYTES;
+            const float glp = sGs[pl * tc::PT + tc::PT - 1];
+#pragma unroll
+            for (int x = tid; x < tc::PT * (tc::VD / 8); x += 256) {
+                const int j = x / (tc::VD / 8), c = (x % (tc::VD / 8)) * 8;
+                const float sc = fexp(glp - sGs[pl * tc::PT + j]);
+                const uint32_t off = umma::tile_offset(j, c, tc::PT);
+                uint4 y = *reinterpret_cast<const uint4*>(cV + off);
+                uint32_t* yw = reinterpret_cast<uint32_t*>(&y);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) yw[e] = pack_bf16(__uint_as_float(yw[e] << 16) * sc, __uint_as_float(yw[e] & 0xffff0000u) * sc);
+                *reinterpret_cast<uint4*>(cV + off) = y;
+            }
+            umma::fence_async_smem();
+            umma::fence_before_sync();               // (the chunk summaries that these products overwrite have been read)
+            __syncwarp();
+            if (lane == 0) arrive_on(&scaled[i & 1]);
+        };
+        // R0 (level 0, for even pairs), R1 (level 1), the segment's: this thread's 32 columns of state row `row`
+        float R0[32], R1[32], Hi[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) R0[e] = R1[e] = Hi[e] = 0.f;
+        if (nc > 0) scale_v(0);
+        if (later) {
+            umma::mbar_wait(hi_full, 0, abort_flag);
+            if (row < p.K)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const float4 x = *reinterpret_cast<const float4*>(sHi + ch * tc::V_BYTES + row * 128 + ((c ^ (row & 7)) << 4));
+                Hi[c * 4] = x.x; Hi[c * 4 + 1] = x.y; Hi[c * 4 + 2] = x.z; Hi[c * 4 + 3] = x.w;
+            }
+        }
+        umma::mbar_wait(r_full, 0, abort_flag);
+        umma::fence_after_sync();
+        // (what pair 2 or pair 1 finds where the walk starts there, at the end of a sequence)
+        if (nc == 3 || nc == 2) umma::tmem_ld32(umma::tmem_addr(tbase + (nc - 1) * 64, warp, ch * 32), R1);
+        for (int i = 0; i < nc; ++i) {
+            const int pl = nc - 1 - i;
+            if (i + 1 < nc) scale_v(i + 1);
+            const bool l0 = (pl & 1) == 0 && pl + 1 < npairs, l1 = pl < 2 && npairs > 2;
+            if (l0) umma::tmem_ld32(umma::tmem_addr(tbase + (pl == 0 ? 0 : 3) * 64, warp, ch * 32), R0);
+            float ka[32], kb[32];
+            umma::mbar_wait(&kv_full[i & 1], (i >> 1) & 1, abort_flag);
+            umma::fence_after_sync();
+            umma::tmem_ld32(umma::tmem_addr(tbase + (tca::SLOT_KV + (i & 1) * 2) * 64, warp, ch * 32), ka);
+            umma::tmem_ld32(umma::tmem_addr(tbase + (tca::SLOT_KV + (i & 1) * 2 + 1) * 64, warp, ch * 32), kb);
+            uint32_t pk[16];
+            float y[6];
+#pragma unroll
+            for (int u = 0; u < 6; ++u) y[u] = 0.f;
+#pragma unroll
+            for (int e = 0; e < 32; e += 2) {
+                float x0 = Hi[e], x1 = Hi[e + 1];
+                y[4] += ka[e] * x0 + ka[e + 1] * x1;
+                y[5] += kb[e] * x0 + kb[e + 1] * x1;
+                if (l0) {
+                    y[0] += ka[e] * R0[e] + ka[e + 1] * R0[e + 1];
+                    y[1] += kb[e] * R0[e] + kb[e + 1] * R0[e + 1];
+                    x0 += R0[e];
+                    x1 += R0[e + 1];
+                }
+                if (l1) {
+                    y[2] += ka[e] * R1[e] + ka[e + 1] * R1[e + 1];
+                    y[3] += kb[e] * R1[e] + kb[e + 1] * R1[e + 1];
+                    x0 += R1[e];
+                    x1 += R1[e + 1];
+                }
+                pk[e >> 1] = pack_bf16(x0, x1);
+            }
+#pragma unroll
+            for (int u = 0; u < 6; ++u) {
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) y[u] += __shfl_xor_sync(0xffffffffu, y[u], d);
+                if (lane == 0) sYs[warp * 8 + u] = y[u];
+            }
+            unsigned char* out = sSt + (i % tca::NST) * tc::V_BYTES;
+            if (i >= tca::NST) {
+                if (tid == 0) tma::wait_group_read<tca::NST - 1>();
+                bar_compute();
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4*>(out + umma::tile_offset(row, ch * 32 + c * 8, p.K)) = make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
+            umma::fence_async_smem();
+            bar_compute();
+            if (tid == 0) {
+                if (!*abort_flag) tma::store_box(&p.tm_lo_a, 0, 0, (int)((bh * NP + r * SEGP + pl) * p.K), out);
+                tma::commit_group();
+            }
+            if (tid >= 32 && tid < 38) {
+                // contributor totals per chunk: pair levels 0, 1, then the high ones together
+                const int u = tid - 32;
+                float t = 0.f;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) t += sYs[w * 8 + u];
+                const int c = (r * SEGP + pl) * 2 + (u & 1);
+                if (c < p.NT) p.Yc[(bh * p.NT + c) * (MLOW + 1) + 1 + (u >> 1)] = t;
+            }
+            // one pair further back: what the later ones send has decayed over this one, which adds what it reads itself
+            const float dec = fexp(sGs[pl * tc::PT + tc::PT - 1]);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+                Hi[e] *= dec;
+                R1[e] *= dec;
+            }
+            if (pl >= 2) {
+                float t[32];
+                umma::tmem_ld32(umma::tmem_addr(tbase + (pl - 1) * 64, warp, ch * 32), t);
+#pragma unroll
+                for (int e = 0; e < 32; ++e) R1[e] += t[e];
+            }
+            bar_compute();                           // the totals have been read
+        }
+        if (nc < npairs && warp == 0 && lane < 6) {
+            // the sequence's last pair: nobody reads it
+            const int c = (NP - 1) * 2 + (lane & 1);
+            if (c < p.NT) p.Yc[(bh * p.NT + c) * (MLOW + 1) + 1 + (lane >> 1)] = 0.f;
+        }
+        if (tid == 0) tma::wait_group0();
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    if (warp == tc::MMA_WARP) {
+        if (*abort_flag && lane == 0) atomicExch(p.err, 1);
+        umma::tmem_dealloc(tbase, tc::TM_COLS);
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -459,20 +594,34 @@ __global__ void __launch_bounds__(tcst::NTHREADS, 2) m2_state_tc_kernel(const __
     if (*abort_flag) return;
     if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tcst::TM_COLS);
     if (warp < 8) {
-        // one chunk per warp: cumulative decay of the pair, then exp(G_end - G)
-        float x0 = 0.f, x1 = 0.f;
+        // One chunk per warp, four consecutive tokens per lane (both half warps the same): its cumulative decay, summed in the order of the output kernel,
+        // so that the sums of a forward call are the ones that a backward call finds in g_cum; then exp(G_end of the pair - G)
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
         if (warp < 2 * np) {
-            const float* gp = p.g + ((long)b * p.T + (long)(r * SEG + warp) * CH) * p.H + h;
-            x0 = gp[(long)(2 * lane) * p.H];
-            x1 = gp[(long)(2 * lane + 1) * p.H];
+            const float* gp = (p.cum_in ? p.cum_in : p.g) + ((long)b * p.T + (long)(r * SEG + warp) * CH + 4 * (lane & 15)) * p.H + h;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = __ldg(gp + (long)i * p.H);
         }
-        warp_cumsum64(x0, x1, lane);
-        const float tot = __shfl_sync(0xffffffffu, x1, 31);
+        if (!p.cum_in) {
+            x[1] += x[0];
+            x[2] += x[1];
+            x[3] += x[2];
+            float t = x[3];
+#pragma unroll
+            for (int d = 1; d < 16; d <<= 1) {
+                const float u = __shfl_up_sync(0xffffffffu, t, d);
+                if ((lane & 15) >= d) t += u;
+            }
+            const float base = t - x[3];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] += base;
+        }
+        const float tot = __shfl_sync(0xffffffffu, x[3], 15);
         if (lane == 0) sTot[warp] = tot;
-        asm volatile("bar.sync 2, 256;\n" ::: "memory");
+        bar_compute();
         const float behind = tot + ((warp & 1) ? 0.f : sTot[warp + 1]);     // from the chunk's start to the pair's end
-        sE[warp * CH + 2 * lane] = fexp(behind - x0);
-        sE[warp * CH + 2 * lane + 1] = fexp(behind - x1);
+        if (lane < 16)
+            *reinterpret_cast<float4*>(sE + warp * CH + 4 * lane) = make_float4(fexp(behind - x[0]), fexp(behind - x[1]), fexp(behind - x[2]), fexp(behind - x[3]));
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -588,13 +737,6 @@ __global__ void __launch_bounds__(tcst::NTHREADS, 2) m2_state_tc_kernel(const __
     }
 }
 
-// level states as one matrix of their rows where they fill the 128 rows of a tile, else each as a sequence of its own, with zeros behind it
-static int make_states_map(Mamba2Params& p) {
-    const long n = (long)p.B * p.H * p.NS * p.LH;
-    return mamba2_whole_pairs(p) ? tma::make_panel_map(&p.tm_h0, p.seg_H0, n * tc::KD, 1, p.V, tc::KD)
-                                 : tma::make_seq_map(&p.tm_h0, p.seg_H0, n, p.K, 1, p.V, tc::KD, 2);
-}
-
 int mamba2_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
@@ -608,30 +750,39 @@ int mamba2_state_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     return (int)cudaGetLastError();
 }
 
-int mamba2_hi_bwd_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
+int mamba2_readers_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     Mamba2Params p = p_in;
     int rc;
     if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
-    if ((rc = make_states_map(p)) != 0) return rc;
-    if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
-    auto kern = mamba2_whole_pairs(p) ? m2_hi_bwd_tc_kernel<M2_MLOW, true> : m2_hi_bwd_tc_kernel<M2_MLOW, false>;
-    const size_t sm = HiBwdTcSmem<M2_MLOW>::total;
+    if ((rc = tma::make_f32_box_map(&p.tm_df, p.seg_dF, (long)p.B * p.H * p.NS * p.LH * p.K, 1, p.V, p.K)) != 0) return rc;
+    auto kern = m2_readers_tc_kernel<M2_MLOW>;
+    const size_t sm = ReadersTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
-    // one launch per window of five segment levels (a single one up to T = 16384); dq, the q.dq totals and
-    // the per-level outputs of different windows add up or are disjoint
-    for (p.lev_lo = 0; p.lev_lo < p.LH; p.lev_lo += tcs::MAXLH) {
-        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tc::NTHREADS, sm, stream, p);
-        LLATTN_LAUNCHED();
+    // one launch per window of five segment levels (a single one up to T = 16384); their outputs are disjoint
+    for (p.lev_lo = 0; p.lev_lo < p.LH; p.lev_lo += tcr::MAXLH) {
+        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tcr::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     }
     return (int)cudaGetLastError();
 }
 
-}  // namespace llattn
-
-#ifdef LLATTN_STAMPS
-extern "C" int llattn_debug_read_stamps_seg(long long* host_dst) {
-    return (int)cudaMemcpyFromSymbol(host_dst, llattn::g_stamps, sizeof(llattn::g_stamps));
+int mamba2_adjoint_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
+    Mamba2Params p = p_in;
+    const long BH = (long)p.B * p.H;
+    int rc;
+    if ((rc = tma::make_seq_map(&p.tm_q, p.q, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_k, p.k, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
+    if ((rc = tma::make_panel_map(&p.tm_lo_a, p.lo_A, BH * ((p.NT + 1) / 2) * p.K, 1, p.V, p.K)) != 0) return rc;
+    if (p.NS > 1 && (rc = tma::make_f32_box_map(&p.tm_dh, p.seg_dHf, BH * p.NS * p.K, 1, p.V, p.K)) != 0) return rc;
+    auto kern = m2_adjoint_tc_kernel<M2_MLOW>;
+    const size_t sm = AdjointTcSmem<M2_MLOW>::total;
+    cudaError_t e = allow_smem(kern, sm);
+    if (e != cudaSuccess) return (int)e;
+    llattn::launch_chained(kern, p.B * p.H * p.NS, tca::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
+    return (int)cudaGetLastError();
 }
-#endif
+
+}  // namespace llattn

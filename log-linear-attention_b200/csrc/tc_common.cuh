@@ -145,7 +145,7 @@ __device__ __forceinline__ void pair_decay_tables(float* tG, float* cum, int lan
         cf[i] = fexp(gend - G[i]);
         vf[i] = fexp(glp - G[i]);
     }
-    if (cum) *reinterpret_cast<float4*>(cum + 4 * lane) = make_float4(cbase + gq[0], cbase + gq[1], cbase + gq[2], cbase + gq[3]);
+    if (cum) *reinterpret_cast<float4*>(cum + 4 * lane) = make_float4(gq[0] + cbase, gq[1] + cbase, gq[2] + cbase, gq[3] + cbase);
     *reinterpret_cast<float4*>(tG + 4 * lane) = make_float4(G[0], G[1], G[2], G[3]);
     *reinterpret_cast<float4*>(tG + 128 + 4 * lane) = make_float4(cf[0], cf[1], cf[2], cf[3]);
     if (TABLES == 3) *reinterpret_cast<float4*>(tG + 256 + 4 * lane) = make_float4(vf[0], vf[1], vf[2], vf[3]);
@@ -158,7 +158,7 @@ __device__ __forceinline__ void stage_lambda(const Mamba2Params& p, int b, int t
     const bf16* gl = p.l + (((long)b * p.T + t0) * p.H + h0) * L;
     const long ldg = (long)p.H * L;
     constexpr int ROWS = tc::PT / WARPS;
-    static_assert(LD <= 128 && LD % 2 == 0 && (LD / 2) % 2 == 1, "two words a lane; an odd number of words a row");
+    static_assert(LD <= 128 && LD % 2 == 0, "two words a lane");
     if (ncol == L && ((reinterpret_cast<uintptr_t>(gl) | (uintptr_t)(ldg * 2) | (uintptr_t)(n * 2)) & 3) == 0) {
         uint32_t x[ROWS][2];
 #pragma unroll

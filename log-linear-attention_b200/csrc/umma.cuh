@@ -193,6 +193,14 @@ __device__ __forceinline__ void gemm_km_lead(uint32_t lead, uint32_t d_tmem, uin
     }
 }
 
+template <int A_ROWS, int B_ROWS, int KRED>
+__device__ __forceinline__ void gemm_mm_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_saddr, uint32_t b_saddr, uint32_t idesc, bool accumulate) {
+    const uint32_t da = desc_lo_mnmajor(a_saddr, A_ROWS * ROW_BYTES), db = desc_lo_mnmajor(b_saddr, B_ROWS * ROW_BYTES);
+#pragma unroll
+    for (int kk = 0; kk < KRED; kk += 16)
+        mma_ss_lead(lead, d_tmem, da + ((kk * ROW_BYTES) >> 4), db + ((kk * ROW_BYTES) >> 4), idesc, accumulate || kk > 0);
+}
+
 // ---- completion tracking
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count));
