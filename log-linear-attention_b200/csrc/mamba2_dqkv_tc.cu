@@ -6,7 +6,7 @@
 //   m2_dq_tc_kernel    dP = do v^T;  dS = dP decay lambda;  dq += dS k;  per level read: T = q H_l, dq += (do scale_l) H_l^T;  d lambda
 //   m2_dkv_tc_kernel   dP again;  P = S decay lambda, dS;  dv = P^T do + scale (k A);  dk += dS^T q + (v scale) A^T
 // Warps 0..7 turn S and dP into the operand tiles of a head, warps 8..15 do the per-row work of the levels and the outputs, two warps issue the products,
-// one the loads, all ahead of one another as far as their rings allow.  A wait that gives up sets the CTA's abort flag, after which every other wait of
+// one the loads, one the outputs, all ahead of one another as far as their rings allow.  A wait that gives up sets the CTA's abort flag, after which every other wait of
 // the CTA ends at once; the warps that meet at barriers then go through the rest of their loops without waiting.
 //
 // The gradient w.r.t. the cumulative decay needs q_i.dq_i and k_j.dk_j per head, which the sums over heads no longer show: o is linear in lambda, so
@@ -24,7 +24,7 @@ namespace llattn {
 namespace tcg {
 constexpr int HC_MAX = 8;
 constexpr int LAM_LD = 122;                  // row stride of the staged lambda values (as many as the output kernel takes): odd number of 32-bit words
-constexpr int NTHREADS = 640, WORKERS = 512, MMA_WARP = 16, T_WARP = 17, TMA_WARP = 18;   // (20 warps: registers move between warpgroups of four)
+constexpr int NTHREADS = 640, WORKERS = 512, MMA_WARP = 16, T_WARP = 17, TMA_WARP = 18, OUT_WARP = 19;
 constexpr int NST = 3;                       // dq: stages of 16 KB for v and the level states
 // launched with 96 registers a thread, 61440 in all: 256 x 112 + 256 x 104 + 128 x 48
 __device__ __forceinline__ void regs_tiles() { asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n"); }
@@ -78,8 +78,9 @@ __device__ __forceinline__ void stage_gradient(unsigned char* stage, uint32_t ta
 // ------------------------------------------------------------------------------------------
 namespace tcq {
 constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256, TM_T = 384, TM_DOS = 448;     // DOS: two scaled copies of do, bf16, 32 columns each
-constexpr int NDL = 9;                       // per row half: 8 levels inside the pair, sum of bf16(P) dP
-constexpr int NLEV = 13;                     // per row: up to 12 levels read, and a partial row sum
+// sums of a row: d lambda by level (6 and 7: of one half of the row), the other half's of levels 6 and 7, sum of bf16(dS) S by halves, of lambda d lambda over
+// the levels read by sets of warps
+constexpr int C_HALF = 14, C_TILE = 22, C_LEV = 24, NSUM = 27;
 }  // namespace tcq
 
 template <int KD>
@@ -91,11 +92,11 @@ struct DqTcSmem {
     static constexpr uint32_t st_off = do_off + tc::V_BYTES;                        // [NST]
     static constexpr uint32_t g_off = st_off + tcg::NST * tc::V_BYTES;              // float [HC_MAX][2][128]
     static constexpr uint32_t c_off = g_off + tcg::HC_MAX * 256 * 4;                // float [HC_MAX][2]
-    static constexpr uint32_t dl_off = c_off + tcg::HC_MAX * 2 * 4;                 // float [2][128][NDL]
-    static constexpr uint32_t lev_off = dl_off + 2 * 128 * tcq::NDL * 4;            // float [128][NLEV]
-    static constexpr uint32_t lam_off = lev_off + 128 * tcq::NLEV * 4;              // bf16 [128][LAM_LD]
+    static constexpr uint32_t dl_off = c_off + tcg::HC_MAX * 2 * 4;                 // float [2][128][NSUM], of every other head
+    static constexpr uint32_t lam_off = dl_off + 2 * 128 * tcq::NSUM * 4;           // bf16 [128][LAM_LD]
     static constexpr uint32_t bar_off = (lam_off + tc::PT * tcg::LAM_LD * 2 + 15) & ~15u;
     static constexpr uint32_t total = bar_off + 256 + 1024;
+    static_assert(total <= 227 * 1024, "shared memory of an SM");
 };
 
 template <int KD>
@@ -112,15 +113,13 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
     float* sG = reinterpret_cast<float*>(smem + SM::g_off);
     float* sC = reinterpret_cast<float*>(smem + SM::c_off);
     float* sDL = reinterpret_cast<float*>(smem + SM::dl_off);
-    float* sLev = reinterpret_cast<float*>(smem + SM::lev_off);
     bf16* sLam = reinterpret_cast<bf16*>(smem + SM::lam_off);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
     uint64_t* full_qk = bars + 0;
     uint64_t* barS = bars + 1;
     uint64_t* dp_full = bars + 2;
-    uint64_t* ds_full = bars + 3;          // 8: dS and the sums over it are written, dP has been read
+    uint64_t* ds_full = bars + 3;          // 8: dS is written, dP has been read
     uint64_t* ds_empty = bars + 4;
-    uint64_t* dl_empty = bars + 5;         // 8: the sums have been read
     uint64_t* t_empty = bars + 6;          // 4: the warps whose turn the level was
     uint64_t* t_full = bars + 7;           // [2] one per set of warps, each of which sees every other level
     uint64_t* dos_full = bars + 9;         // [2] 4
@@ -129,13 +128,16 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
     uint64_t* do_full = bars + 14;
     uint64_t* do_empty = bars + 15;        // 257: the row threads, and dP
     uint64_t* t_done = bars + 16;
-    uint64_t* st_full = bars + 17;         // [NST]
+    uint64_t* dl_full = bars + 5;          // [2] 16: the sums of a head are written, of its tile and of its levels   (5, 17)
+    uint64_t* dl_full1 = bars + 17;
+    uint64_t* dl_empty = bars + 18;        // [2]
+    uint64_t* st_full = bars + 20;         // [NST]
     uint64_t* st_empty = st_full + tcg::NST;   // [NST] 2: the two issuing warps
-    constexpr int NBARS = 17 + 2 * tcg::NST;
-    static_assert(NBARS * 8 <= 200, "barriers");
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 200);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 208);
-    uint32_t* sink = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 212);     // written only (tile release)
+    constexpr int NBARS = 20 + 2 * tcg::NST;
+    static_assert(NBARS * 8 <= 232, "barriers");
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 232);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 240);
+    uint32_t* sink = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 244);     // written only (tile release)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int L = p.L;
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
     const int nlev = __popc(w.pair);
 
     if (warp == tcg::TMA_WARP && lane == 0) {
-        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], (i == 3 || i == 5) ? 8 : (i == 6 || i == 9 || i == 10) ? 4 : i == 15 ? 257 : i >= NBARS - tcg::NST ? 2 : 1);
+        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], i == 3 ? 8 : (i == 5 || i == 17) ? 16 : (i == 6 || i == 9 || i == 10) ? 4 : i == 15 ? 257 : i >= NBARS - tcg::NST ? 2 : 1);
         umma::fence_mbar_init();
         *abort_flag = *p.err;
     }
@@ -178,6 +180,11 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
         }
         asm volatile("bar.sync 1, 512;\n" ::: "memory");
         if (warp < w.nh) pair_decay_tables<2>(sG + warp * 256, nullptr, lane);
+        if (tid < 2 * tc::PT) {
+            // d lambda of the levels that the pair does not read, for every head
+            for (int i = 8; i < L; ++i)
+                if (!((w.pair >> (i - 8)) & 1)) sDL[tid * tcq::NSUM + i] = 0.f;
+        }
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -232,6 +239,56 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
             }
         }
         __syncwarp();
+      } else if (warp == tcg::OUT_WARP) {
+        // ---- d lambda rows, all levels of them (zeros where the pair reads none); q.dq; totals of level 7
+        const int per = 32 / L, sub = lane / L, i = lane - sub * L, step_s = per * tcq::NSUM;
+        const long step_d = (long)per * p.H * L;
+        const bool halves = i == 6 || i == 7;
+        for (int hh = 0; hh < w.nh; ++hh) {
+            const int h = w.h0 + hh;
+            umma::mbar_wait((hh & 1) ? dl_full1 : dl_full, (hh >> 1) & 1, abort_flag);
+            const float* sums = sDL + (hh & 1) * 128 * tcq::NSUM;
+            float z = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int rr = u * 32 + lane;
+                const float* d = sums + rr * tcq::NSUM;
+                if (w.t0 + rr < p.T)
+                    p.wq[((long)w.b * p.T + w.t0 + rr) * p.H + h] = (d[tcq::C_LEV] + d[tcq::C_LEV + 1]) + (d[tcq::C_TILE] + d[tcq::C_TILE + 1]);
+                if (u >= 2 && L > 7) z += __bfloat162float(sLam[rr * tcg::LAM_LD + hh * L + 7]) * (d[7] + d[7 + tcq::C_HALF]);
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) z += __shfl_xor_sync(0xffffffffu, z, d);
+            if (lane == 0) {
+                // the second chunk reads the first; its contributor total is the same
+                const long c = ((long)w.b * p.H + h) * p.NT + w.pair * 2;
+                if (w.pair * 2 + 1 < p.NT) p.Zc[(c + 1) * p.LZ] = z;
+                p.Yc[c * (M2_MLOW + 1)] = z;
+            }
+            // as many whole rows as fit on the lanes at once: a lane keeps its level, so that a step is two loads, a sum and a store.  (With 32 values of any
+            // rows a step, or several tokens' rows of a wider index, the warp's 1500 instructions a head were the longest chain of the kernel.)
+            const int left = min(tc::PT, p.T - w.t0);
+            const float* src = sums + sub * tcq::NSUM + i;
+            float* dst = p.dl + (((long)w.b * p.T + w.t0 + sub) * p.H + h) * L + i;
+            int n = sub < per ? (left - sub + per - 1) / per : 0;
+            for (; n >= 4; n -= 4) {
+                float v[4], x[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = src[u * step_s];
+                if (halves)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) x[u] = src[u * step_s + tcq::C_HALF];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    *dst = v[u] + x[u];
+                    dst += step_d;
+                }
+                src += 4 * step_s;
+            }
+            for (; n > 0; --n, src += step_s, dst += step_d) *dst = halves ? src[0] + src[tcq::C_HALF] : src[0];
+            __syncwarp();
+            if (lane == 0) arrive(&dl_empty[hh & 1]);
+        }
       } else if (warp == tcg::T_WARP) {
         // (whole warps issue, see umma::elect_one)
         constexpr uint32_t ID_KM64 = umma::idesc_bf16(128, 64, false, true);
@@ -342,8 +399,8 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
             umma::mbar_wait(dp_full, hh & 1, abort_flag);
             if (hh > 0) {
                 umma::mbar_wait(ds_empty, (hh - 1) & 1, abort_flag);
-                umma::mbar_wait(dl_empty, (hh - 1) & 1, abort_flag);
             }
+            if (hh >= 2) umma::mbar_wait(&dl_empty[hh & 1], ((hh >> 1) - 1) & 1, abort_flag);
             umma::fence_after_sync();
             float bins[8];
             f32x2 wq2 = 0;                           // sum_j bf16(dS_ij) S_ij: q_i.dq_i of the tile
@@ -449,24 +506,31 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
                     *reinterpret_cast<uint4*>(sDS + umma::tile_offset(row, j0 + c * 8, tc::PT)) =
                         make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]);
             }
-            float* myDL = sDL + (ch * 128 + row) * tcq::NDL;
+            // (a thread whose columns of the diagonal block lie in the row's own half has levels 0..4 of the row, the other one level 5)
+            float* myDL = sDL + ((hh & 1) * 128 + row) * tcq::NSUM;
+            if (hi) {
+                myDL[5] = bins[5];
+            } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) myDL[i] = bins[i];
-            myDL[8] = sum2(wq2);
+                for (int i = 0; i < 5; ++i) myDL[i] = bins[i];
+            }
+            myDL[6 + ch * tcq::C_HALF] = bins[6];
+            myDL[7 + ch * tcq::C_HALF] = bins[7];
+            myDL[tcq::C_TILE + ch] = sum2(wq2);
             umma::fence_async_smem();
             umma::fence_before_sync();
             __syncwarp();
-            if (lane == 0) arrive(ds_full);
+            if (lane == 0) {
+                arrive(ds_full);
+                arrive((hh & 1) ? dl_full1 : dl_full);
+            }
         }
     } else {
         tcg::regs_rows();
         // ---- levels read: scaled copies of do (tensor memory, A operand of the dq product), d lambda = s_i (do_i . T_i).  A thread has a whole row;
         //      the two sets of four warps take the CTA's levels in turn
         const int rb = warp & 3, row = rb * 32 + lane, set = (warp - 8) >> 2;
-        const int t = w.t0 + row;
-        const bool in = t < p.T;
         int turn = 0;                                // levels so far
-        const int rr0 = (tid - 256) / L, i0 = (tid - 256) % L, drr = 256 / L, di = 256 % L;      // this thread's values of the d lambda rows
         for (int hh = 0; hh < w.nh; ++hh) {
             const int h = w.h0 + hh;
             const float Gi = sG[hh * 256 + row];
@@ -483,6 +547,8 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
                 release_tile_after_loads(do_empty, sink, digest);
             }
             float wsum = 0.f;                        // this set's share of sum_l lambda d lambda
+            float* myLev = sDL + ((hh & 1) * 128 + row) * tcq::NSUM;
+            if (hh >= 2) umma::mbar_wait(&dl_empty[hh & 1], ((hh >> 1) - 1) & 1, abort_flag);
             int bits = w.pair;
             for (int j = 0; j < nlev; ++j, ++turn) {
                 const int lv = __ffs(bits) - 1;
@@ -530,7 +596,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
                 }
                 const float dot = sum2(dot2[0]) + sum2(dot2[1]);
                 const float dlv = sc * dot;
-                sLev[row * tcq::NLEV + lv] = dlv;
+                myLev[8 + lv] = dlv;
                 float z = lm * dlv;
                 wsum += z;
 #pragma unroll
@@ -539,49 +605,12 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
                 const int c = w.pair * 2 + (rb >> 1);
                 if (lane == 0 && c < p.NT) red_add_f32(p.Zc + (((long)w.b * p.H + h) * p.NT + c) * p.LZ + 1 + lv, z);
             }
-            umma::mbar_wait(ds_full, hh & 1, abort_flag);
-            if (set == 1) sLev[row * tcq::NLEV + tcq::NLEV - 1] = wsum;
-            bar_rows();
-            const float* dl0 = sDL + row * tcq::NDL;
-            const float* dl1 = sDL + (128 + row) * tcq::NDL;
-            if (set == 0) {
-                wsum += sLev[row * tcq::NLEV + tcq::NLEV - 1] + (dl0[8] + dl1[8]);
-                if (in) p.wq[((long)w.b * p.T + t) * p.H + h] = wsum;
-            } else if (rb >= 2) {
-                // level 7: the second chunk reads the first; its contributor total is the same
-                float z = L > 7 ? __bfloat162float(sLam[row * tcg::LAM_LD + hh * L + 7]) * (dl0[7] + dl1[7]) : 0.f;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) z += __shfl_xor_sync(0xffffffffu, z, d);
-                const long c = ((long)w.b * p.H + h) * p.NT + w.pair * 2;
-                if (lane == 0) {
-                    if (w.pair * 2 + 1 < p.NT) red_add_f32(p.Zc + (c + 1) * p.LZ, z);
-                    red_add_f32(p.Yc + c * (M2_MLOW + 1), z);
-                }
-            }
-            // d lambda rows, all levels of them
-            {
-                float* gdl = p.dl + (((long)w.b * p.T + w.t0) * p.H + h) * L;
-                const int left = p.T - w.t0;
-                int rr = rr0, i = i0;
-#pragma unroll 4
-                for (int e = tid - 256; e < tc::PT * L; e += 256) {
-                    float v = 0.f;
-                    if (i < 8) v = sDL[rr * tcq::NDL + i] + sDL[(128 + rr) * tcq::NDL + i];
-                    else if ((w.pair >> (i - 8)) & 1) v = sLev[rr * tcq::NLEV + i - 8];
-                    if (rr < left) gdl[(long)rr * p.H * L + i] = v;
-                    rr += drr;
-                    i += di;
-                    if (i >= L) {
-                        i -= L;
-                        ++rr;
-                    }
-                }
-            }
+            myLev[tcq::C_LEV + set] = wsum;
             __syncwarp();
-            if (lane == 0) arrive(dl_empty);
-            bar_rows();                              // the level sums of the next head go to the same place
+            if (lane == 0) arrive((hh & 1) ? dl_full1 : dl_full);
         }
-        // ---- dq of these heads
+        // ---- dq of these heads, in the place of q and k (every level read is behind the barrier, every other product behind `done`)
+        bar_rows();
         umma::mbar_wait(done, 0, abort_flag);
         umma::fence_after_sync();
         stage_gradient<KD>(smem + SM::q_off, tbase + tcq::TM_DQ, warp, row, set, 2);
@@ -621,8 +650,8 @@ struct DkvTcSmem {
     static constexpr uint32_t v_off = do_off + 2 * tc::V_BYTES;
     static constexpr uint32_t a_off = v_off + tc::V_BYTES;
     static constexpr uint32_t g_off = a_off + tc::V_BYTES;                          // float [HC_MAX][2][128]
-    static constexpr uint32_t w_off = g_off + tcg::HC_MAX * 256 * 4;                // float [3][2][128] k.dk halves: of two heads' tiles, of the state
-    static constexpr uint32_t lam_off = w_off + 768 * 4;                            // bf16 [128][LAM_LD]
+    static constexpr uint32_t w_off = g_off + tcg::HC_MAX * 256 * 4;                // float [2][2][2][128] k.dk halves of a head's tile, and with its state, of every other head
+    static constexpr uint32_t lam_off = w_off + 1024 * 4;                           // bf16 [128][LAM_LD]
     static constexpr uint32_t bar_off = (lam_off + tc::PT * tck::LAM_LD * 2 + 15) & ~15u;
     static_assert(lam_off % 16 == 0, "16-byte loads of lambda");
     static constexpr uint32_t total = bar_off + 256 + 1024;
@@ -661,7 +690,8 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
     uint64_t* v_empty = bars + 15;         // 257: the row threads, and dP
     uint64_t* a_full = bars + 16;
     uint64_t* a_read = bars + 17;          // its products are complete
-    constexpr int NBARS = 18;
+    uint64_t* out_full = bars + 18;        // [2] 8: dv and k.dk of a head are written
+    constexpr int NBARS = 20;
     static_assert(NBARS * 8 <= 200, "barriers");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 200);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 208);
@@ -674,7 +704,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
     const bool read = w.pair + 1 < w.NP;
 
     if (warp == tcg::TMA_WARP && lane == 0) {
-        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], (i == 3 || i == 6 || i == 8) ? 8 : i == 15 ? 257 : 1);
+        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], (i == 3 || i == 6 || i == 8 || i >= 18) ? 8 : i == 15 ? 257 : 1);
         umma::fence_mbar_init();
         *abort_flag = *p.err;
     }
@@ -734,6 +764,27 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
                 if (na > 0) umma::mbar_wait(a_full, (na - 1) & 1, limit);
             }
         }
+        __syncwarp();
+      } else if (warp == tcg::OUT_WARP) {
+        for (int hh = 0; hh < w.nh; ++hh) {
+            umma::mbar_wait(&out_full[hh & 1], (hh >> 1) & 1, abort_flag);
+            if (lane == 0) {
+                if (!*abort_flag) tma::store_seq_box(&p.tm_dv, 0, w.h0 + hh, w.t0, w.b, sDO + (hh & 1) * tc::V_BYTES);
+                tma::commit_group();
+            }
+            const float* W = sW + ((hh & 1) * 4 + 2) * 128;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int rr = u * 32 + lane;
+                if (w.t0 + rr < p.T) red_add_f32(p.wq + ((long)w.b * p.T + w.t0 + rr) * p.H + w.h0 + hh, -(W[rr] + W[128 + rr]));
+            }
+            __syncwarp();
+            if (lane == 0) {
+                tma::wait_group_read0();
+                arrive(&do_empty[hh & 1]);
+            }
+        }
+        if (lane == 0) tma::wait_group0();
         __syncwarp();
       } else if (warp == tcg::T_WARP) {
         // states: U = k A, then dk += (v scale) A^T   (whole warps issue, see umma::elect_one)
@@ -893,7 +944,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
                 }
                 store(i0);
             }
-            sW[((hh & 1) * 2 + ch) * 128 + row] = sum2(wk2);
+            sW[((hh & 1) * 4 + ch) * 128 + row] = sum2(wk2);
             umma::fence_async_smem();
             umma::fence_before_sync();
             __syncwarp();
@@ -903,10 +954,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
         tcg::regs_rows();
         // ---- the state contributed to, dv rows.  This thread: row `row`, columns ch*32 .. +31
         const int rb = warp & 3, row = rb * 32 + lane, ch = (warp - 8) >> 2;
-        const int t = w.t0 + row;
-        const bool in = t < p.T;
         for (int hh = 0; hh < w.nh; ++hh) {
-            const int h = w.h0 + hh;
             uint32_t vx[16];
             umma::mbar_wait(v_full, hh & 1, abort_flag);
             {
@@ -965,7 +1013,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
                     vx[e] = pack_bf16(a.x + x[2 * e], a.y + x[2 * e + 1]);
                 }
             }
-            sW[512 + ch * 128 + row] = wk + sW[((hh & 1) * 2 + ch) * 128 + row];     // (the tile's sums are there with dS)
+            sW[((hh & 1) * 4 + 2 + ch) * 128 + row] = wk + sW[((hh & 1) * 4 + ch) * 128 + row];     // (the tile's sums are there with dS)
             umma::fence_before_sync();
             __syncwarp();
             if (lane == 0) arrive(dv_empty);
@@ -976,15 +1024,8 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
                 *reinterpret_cast<uint4*>(sOut + umma::tile_offset(row, ch * 32 + c * 8, tc::PT)) =
                     make_uint4(vx[c * 4], vx[c * 4 + 1], vx[c * 4 + 2], vx[c * 4 + 3]);
             umma::fence_async_smem();
-            bar_rows();
-            if (tid == 256) {
-                if (!*abort_flag) tma::store_seq_box(&p.tm_dv, 0, h, w.t0, w.b, sOut);
-                tma::commit_group();
-                tma::wait_group_read0();
-                arrive(&do_empty[hh & 1]);
-            }
-            if (ch == 1 && in) p.wq[((long)w.b * p.T + t) * p.H + h] -= sW[512 + row] + sW[640 + row];
-            bar_rows();
+            __syncwarp();
+            if (lane == 0) arrive(&out_full[hh & 1]);
         }
         // ---- dk of these heads
         umma::mbar_wait(done, 0, abort_flag);

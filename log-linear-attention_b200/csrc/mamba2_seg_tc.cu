@@ -40,18 +40,20 @@ __device__ __forceinline__ void scaled_half_row(unsigned char* dst, const uint4 
 
 // ------------------------------------------------------------------------------------------
 // backward: what the readers of the high level states send back, dF[r][j] = sum over the pairs of segment r of q^T (do lambda_j exp(G)), G from the segment's
-// start, for every set bit j of r: fp32 K x V summaries for the scan over segments.  One CTA per (batch, head, segment); a job is a level of a pair: a
-// scaled copy of do in a ring of stages times q^T, accumulated in the level's tensor-memory slot.
+// start, for every set bit j of r: fp32 K x V summaries for the scan over segments.  One CTA per (batch, head, segment) and four set levels; a job is a level
+// of a pair: a scaled copy of do in a ring of stages times q^T, accumulated in the level's tensor-memory slot.
+// The kernel is latency throughout (16 % of the issue slots busy with one CTA per SM), so what a CTA holds is cut to let two share an SM: one tile of q, two
+// copies, four slots.
 // ------------------------------------------------------------------------------------------
 namespace tcr {
-constexpr int MAXLH = 5;                 // high levels of one launch
-constexpr int NST = 6, NTHREADS = 320, TMA_WARP = 9;
+constexpr int MAXLH = 4;                 // high levels of a CTA
+constexpr int NST = 2, NTHREADS = 320, TMA_WARP = 9, TM_COLS = 256;
 }
 template <int MLOW>
 struct ReadersTcSmem {
     static constexpr int SEG = 1 << MLOW;
-    static constexpr uint32_t q_off = 0;                                   // [2] 32 KB
-    static constexpr uint32_t do_off = q_off + 2 * tc::Q_BYTES;            // [2] 16 KB
+    static constexpr uint32_t q_off = 0;                                   // 32 KB
+    static constexpr uint32_t do_off = q_off + tc::Q_BYTES;                // [2] 16 KB
     static constexpr uint32_t st_off = do_off + 2 * tc::V_BYTES;           // [NST] 16 KB
     static constexpr uint32_t gs_off = st_off + tcr::NST * tc::V_BYTES;    // float [SEG * 64], [SEG]
     static constexpr uint32_t lam_off = gs_off + (SEG * 64 + SEG) * 4;     // bf16 [MAXLH][SEG * 64]
@@ -60,7 +62,7 @@ struct ReadersTcSmem {
 };
 
 template <int MLOW>
-__global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const __grid_constant__ Mamba2Params p) {
+__global__ void __launch_bounds__(tcr::NTHREADS, 2) m2_readers_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = ReadersTcSmem<MLOW>;
     constexpr int SEG = SM::SEG, SEGP = SEG / 2;
@@ -74,8 +76,9 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
     float* sTot = sGs + SEG * 64;
     bf16* sLam = reinterpret_cast<bf16*>(smem + SM::lam_off);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
-    uint64_t* full = bars + 0;       // [2] q and do of a pair
-    uint64_t* empty = bars + 2;      // [2] (the products of a pair wait for every thread's copies of its do)
+    uint64_t* full = bars + 0;       // [2] do of a pair
+    uint64_t* full_q = bars + 2;
+    uint64_t* empty = bars + 3;      // q and do of a pair (its products wait for every thread's copies of its do)
     uint64_t* done = bars + 4;
     uint64_t* st_full = bars + 5;    // [NST] 8: a scaled copy is written
     uint64_t* st_empty = bars + 5 + tcr::NST;
@@ -88,12 +91,14 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
     const int NP = (p.NT + 1) / 2;
     const int h = blockIdx.x % p.H;
     const int r = 1 + (blockIdx.x / p.H) % (p.NS - 1);
-    const int b = blockIdx.x / (p.H * (p.NS - 1));
+    const int b = (blockIdx.x / (p.H * (p.NS - 1))) % p.B, part = blockIdx.x / (p.H * (p.NS - 1) * p.B);
     const int grp = h / (p.H / p.G);
     const long bh = (long)b * p.H + h;
     const int npairs = min(SEGP, NP - r * SEGP);
-    // set high levels of this segment inside this launch's window of five levels
-    const int himask = (r >> p.lev_lo) & ((1 << tcr::MAXLH) - 1), nl = __popc(himask);
+    // this CTA's four of the segment's set high levels
+    int himask = r;
+    for (int i = 0; i < part * tcr::MAXLH; ++i) himask &= himask - 1;
+    const int nl = min(__popc(himask), tcr::MAXLH);
     if (nl == 0) return;                     // (uniform)
 
     if (tid == tcr::TMA_WARP * 32) {
@@ -103,14 +108,20 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
     }
     __syncthreads();
     if (*abort_flag) return;
-    if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tc::TM_COLS);
+    if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tcr::TM_COLS);
     if (warp < 8) {
         // lambda of the levels read
-        const int base = INTRA_LEVELS + MLOW + p.lev_lo;
-        for (int e = tid; e < SEG * 64 * tcr::MAXLH; e += 256) {
-            const int i = e / tcr::MAXLH, j = e - i * tcr::MAXLH, t = r * SEG * 64 + i;
-            if ((himask >> j) & 1) sLam[j * SEG * 64 + i] = t < p.T ? p.l[(((long)b * p.T + t) * p.H + h) * p.L + base + j] : __float2bfloat16(0.f);
+        unsigned short x[SEG * 64 * tcr::MAXLH / 256];
+        int lev = himask;
+        for (int i = 0; i < (tid & 3) && lev; ++i) lev &= lev - 1;
+        const unsigned short* gl = reinterpret_cast<const unsigned short*>(p.l) + ((long)b * p.T * p.H + h) * p.L + INTRA_LEVELS + MLOW + __ffs(lev) - 1;
+#pragma unroll
+        for (int i = 0; i < SEG * 64 * tcr::MAXLH / 256; ++i) {
+            const int t = r * SEG * 64 + (tid >> 2) + i * 64;
+            x[i] = t < p.T && (tid & 3) < nl ? __ldg(gl + (long)t * p.H * p.L) : (unsigned short)0;
         }
+#pragma unroll
+        for (int i = 0; i < SEG * 64 * tcr::MAXLH / 256; ++i) sLam[(tid & 3) * SEG * 64 + (tid >> 2) + i * 64] = __ushort_as_bfloat16(x[i]);
         segment_pair_sums(p, b, h, r, sGs, sTot, warp, lane);
     }
     umma::fence_before_sync();
@@ -120,17 +131,24 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
 
     if (warp == tcr::TMA_WARP) {
         if (lane == 0) {
-            int pl = 0;
+            int pl = 0, nq = 0;
             for (; pl < npairs; ++pl) {
                 const int st = pl & 1, row0 = (r * SEGP + pl) * tc::PT;
-                if (pl >= 2 && !umma::mbar_wait(&empty[st], ((pl - 2) >> 1) & 1, abort_flag)) break;
-                tma::expect_tx(&full[st], tc::Q_BYTES + tc::V_BYTES);
+                // (its place: free since the q of the pair before was asked for)
+                tma::expect_tx(&full[st], tc::V_BYTES);
                 tma::load_seq_panel(sDO + st * tc::V_BYTES, &p.tm_do, 0, h, row0, b, &full[st]);
-                tma::load_seq_panel(sQ + st * tc::Q_BYTES, &p.tm_q, 0, grp, row0, b, &full[st]);
-                tma::load_seq_panel(sQ + st * tc::Q_BYTES + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, &full[st]);
+                if (pl >= 1 && !umma::mbar_wait(empty, (pl - 1) & 1, abort_flag)) {
+                    ++pl;
+                    break;
+                }
+                tma::expect_tx(full_q, tc::Q_BYTES);
+                tma::load_seq_panel(sQ, &p.tm_q, 0, grp, row0, b, full_q);
+                tma::load_seq_panel(sQ + tc::Q_BYTES / 2, &p.tm_q, 64, grp, row0, b, full_q);
+                nq = pl + 1;
             }
-            // every load is waited for by the MMA warp, unless a wait gave up: nothing may still be on its way into shared memory when the CTA ends
+            // every load is waited for by other warps, unless a wait gave up: nothing may still be on its way into shared memory when the CTA ends
             for (int i = max(0, pl - 2); i < pl; ++i) umma::mbar_wait(&full[i & 1], (i >> 1) & 1, 1u << 16);
+            if (nq > 0) umma::mbar_wait(full_q, (nq - 1) & 1, 1u << 16);
         }
         __syncwarp();
     } else if (warp == tc::MMA_WARP) {
@@ -142,8 +160,8 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
         uint32_t ph = 0;
         bool ok = true;
         for (int pl = 0; pl < npairs && ok; ++pl) {
-            if (!(ok = wait(&full[pl & 1], (pl >> 1) & 1))) break;
-            const uint32_t aQ = umma::smem_addr(sQ + (pl & 1) * tc::Q_BYTES);
+            if (!(ok = wait(full_q, pl & 1))) break;
+            const uint32_t aQ = umma::smem_addr(sQ);
             for (int i = 0; i < nl; ++i) {
                 if (!(ok = wait(&st_full[st], ph))) break;
                 umma::fence_after_sync();
@@ -154,7 +172,7 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
                     ph ^= 1;
                 }
             }
-            umma::commit_lead(lead, &empty[pl & 1]);
+            umma::commit_lead(lead, empty);
         }
         umma::commit_lead(lead, done);
         if (!ok) umma::mbar_wait(done, 0, 1u << 16);     // gave up: no product may still read shared memory when the CTA ends
@@ -172,11 +190,8 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
 #pragma unroll
             for (int c = 0; c < 4; ++c)
                 dox[c] = *reinterpret_cast<const uint4*>(sDO + (pl & 1) * tc::V_BYTES + umma::tile_offset(row, ch * 32 + c * 8, tc::PT));
-            int bits = himask;
             for (int i = 0; i < nl; ++i) {
-                const int j = __ffs(bits) - 1;
-                bits &= bits - 1;
-                const float rs = __bfloat162float(sLam[j * SEG * 64 + pl * tc::PT + row]) * ehi;
+                const float rs = __bfloat162float(sLam[i * SEG * 64 + pl * tc::PT + row]) * ehi;
                 umma::mbar_wait(&st_empty[st], ph, abort_flag);
                 scaled_half_row(sSt + st * tc::V_BYTES, dox, rs, row, ch);
                 umma::fence_async_smem();
@@ -190,14 +205,15 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
         }
         umma::mbar_wait(done, 0, abort_flag);
         umma::fence_after_sync();
-        // the summaries leave in boxes of 32 columns by way of the ring, two levels at a time
+        // the summaries leave in boxes of 32 columns by way of the places of q and do in turn
         int bits = himask;
         for (int i = 0; i < nl; ++i) {
-            const int j = p.lev_lo + __ffs(bits) - 1;
+            const int j = __ffs(bits) - 1;
             bits &= bits - 1;
             float t[32];
             umma::tmem_ld32(umma::tmem_addr(tbase + i * 64, warp, ch * 32), t);
-            unsigned char* box = sSt + ((i & 1) * 2 + ch) * tc::V_BYTES;
+            unsigned char* place = (i & 1) ? sDO : sQ;
+            unsigned char* box = place + ch * tc::V_BYTES;
             if (i >= 2) {
                 if (tid == 0) tma::wait_group_read1();
                 bar_compute();
@@ -210,7 +226,7 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
             if (tid == 0) {
                 const int at = (int)(((bh * p.NS + r) * p.LH + j) * p.K);
                 if (!*abort_flag)
-                    for (int bx = 0; bx < 2; ++bx) tma::store_box(&p.tm_df, bx * 32, 0, at, sSt + ((i & 1) * 2 + bx) * tc::V_BYTES);
+                    for (int bx = 0; bx < 2; ++bx) tma::store_box(&p.tm_df, bx * 32, 0, at, place + bx * tc::V_BYTES);
                 tma::commit_group();
             }
         }
@@ -221,37 +237,38 @@ __global__ void __launch_bounds__(tcr::NTHREADS, 1) m2_readers_tc_kernel(const _
     umma::fence_after_sync();
     if (warp == tc::MMA_WARP) {
         if (*abort_flag && lane == 0) atomicExch(p.err, 1);
-        umma::tmem_dealloc(tbase, tc::TM_COLS);
+        umma::tmem_dealloc(tbase, tcr::TM_COLS);
     }
 }
 
 // ------------------------------------------------------------------------------------------
-// backward: the gradient of every pair's summary.  One CTA per (batch, head, segment):
-//   R_pl,l = q^T (do lambda_l exp(G))        pairs 1.. of the segment, the pair levels that they read (tensor memory, fp32)
-//   A_pl   = what comes back to pair pl: from later segments, from the pairs of its segment that read a state with it    (one bf16 tile, fp32 until then)
-//   Y      = <k^T (v exp(G_end - G)) of each chunk, A's parts>     contributor totals per level, from the fp32 parts
-// The segment's pairs are walked in order for R, then in reverse for A and Y.
+// backward: the gradient of every pair's summary.  One CTA per (batch, head, segment) walks the segment's pairs from the last one on:
+//   R_l  += q^T (do lambda_l exp(G))     what pair pl sends back to the pair levels that it reads (tensor memory, fp32)
+//   A_pl  = what comes back to pair pl: from later segments, from the pairs of its segment that read a state with it    (one bf16 tile, fp32 until then)
+//   Y     = <k^T (v exp(G_end - G)) of each chunk, A's parts>     contributor totals per level, from the fp32 parts
+// Two CTAs per SM, with one tile of each operand and four 64-column slots each, as the steps of a CTA are a chain: R of pair level 1, of pair level 0, the
+// summaries of a pair's two chunks.
 // ------------------------------------------------------------------------------------------
 namespace tca {
-constexpr int NST = 3, NTHREADS = 320, TMA_WARP = 9;
-constexpr int SLOT_KV = 4;               // slots 0..3: R of (pair 1, level 0), (2, 1), (3, 1), (3, 0); 4..7: two pairs of chunk summaries
+constexpr int NTHREADS = 320, TMA_WARP = 9, TM_COLS = 256;
+constexpr int SLOT_R1 = 0, SLOT_R0 = 1, SLOT_KV = 2;
 }
 template <int MLOW>
 struct AdjointTcSmem {
     static constexpr int SEG = 1 << MLOW;
-    static constexpr uint32_t x_off = 0;                                   // [2] 32 KB: q, then k
-    static constexpr uint32_t y_off = x_off + 2 * tc::Q_BYTES;             // [2] 16 KB: do, then v (scaled in place)
-    static constexpr uint32_t st_off = y_off + 2 * tc::V_BYTES;            // [NST] 16 KB: scaled copies of do, then A on its way out
-    static constexpr uint32_t hi_off = st_off + tca::NST * tc::V_BYTES;    // 32 KB: fp32 gradient of the segment's summary, two boxes of 32 columns
+    static constexpr uint32_t x_off = 0;                                   // 32 KB: q or k
+    static constexpr uint32_t y_off = x_off + tc::Q_BYTES;                 // 16 KB: do or v (scaled in place)
+    static constexpr uint32_t d_off = y_off + tc::V_BYTES;                 // 16 KB: a scaled copy of do, or A on its way out
+    static constexpr uint32_t hi_off = d_off + tc::V_BYTES;                // 32 KB: fp32 gradient of the segment's summary, two boxes of 32 columns
     static constexpr uint32_t gs_off = hi_off + 2 * tc::V_BYTES;           // float [SEG * 64], [SEG]
     static constexpr uint32_t y_sum_off = gs_off + (SEG * 64 + SEG) * 4;   // float [8][8]
     static constexpr uint32_t lam_off = y_sum_off + 64 * 4;                // bf16 [2][SEG * 64]
     static constexpr uint32_t bar_off = lam_off + 2 * SEG * 64 * 2;
-    static constexpr uint32_t total = bar_off + 256 + 1024;
+    static constexpr uint32_t total = bar_off + 128 + 1024;
 };
 
 template <int MLOW>
-__global__ void __launch_bounds__(tca::NTHREADS, 1) m2_adjoint_tc_kernel(const __grid_constant__ Mamba2Params p) {
+__global__ void __launch_bounds__(tca::NTHREADS, 2) m2_adjoint_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
     using SM = AdjointTcSmem<MLOW>;
     constexpr int SEG = SM::SEG, SEGP = SEG / 2;
@@ -260,24 +277,24 @@ __global__ void __launch_bounds__(tca::NTHREADS, 1) m2_adjoint_tc_kernel(const _
     unsigned char* smem = umma::align_1024(smem_raw);
     unsigned char* sX = smem + SM::x_off;
     unsigned char* sY = smem + SM::y_off;
-    unsigned char* sSt = smem + SM::st_off;
+    unsigned char* sD = smem + SM::d_off;
     unsigned char* sHi = smem + SM::hi_off;
     float* sGs = reinterpret_cast<float*>(smem + SM::gs_off);
     float* sTot = sGs + SEG * 64;
     float* sYs = reinterpret_cast<float*>(smem + SM::y_sum_off);
     bf16* sLam = reinterpret_cast<bf16*>(smem + SM::lam_off);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
-    uint64_t* full = bars + 0;       // [2]
-    uint64_t* empty = bars + 2;      // [2]
-    uint64_t* hi_full = bars + 4;
-    uint64_t* r_full = bars + 5;     // every R is complete
-    uint64_t* scaled = bars + 6;     // [2] 8: v is scaled
-    uint64_t* kv_full = bars + 8;    // [2]
-    uint64_t* st_full = bars + 10;   // [NST] 8
-    uint64_t* st_empty = bars + 10 + tca::NST;
-    constexpr int NBARS = 10 + 2 * tca::NST;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 200);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 208);
+    uint64_t* full = bars + 0;       // the step's tiles
+    uint64_t* empty = bars + 1;
+    uint64_t* hi_full = bars + 2;
+    uint64_t* r_full = bars + 3;     // a reading step's products are complete
+    uint64_t* scaled = bars + 4;     // 8: v is scaled
+    uint64_t* kv_full = bars + 5;
+    uint64_t* d_full = bars + 6;     // 8: a copy of do is written
+    uint64_t* d_empty = bars + 7;
+    constexpr int NBARS = 8;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 96);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 104);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int NP = (p.NT + 1) / 2;
@@ -288,21 +305,26 @@ __global__ void __launch_bounds__(tca::NTHREADS, 1) m2_adjoint_tc_kernel(const _
     const long bh = (long)b * p.H + h;
     const int npairs = min(SEGP, NP - r * SEGP);
     const bool later = r < p.NS - 1;                 // later segments read this one's summary
-    const int nr = npairs - 1, nc = later ? SEGP : npairs - 1;      // pairs that read, pairs that are read
+    const int nc = later ? SEGP : npairs - 1;        // pairs that are read
 
     if (tid == tca::TMA_WARP * 32) {
-        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], i == 6 || i == 7 || (i >= 10 && i < 10 + tca::NST) ? 8 : 1);
+        for (int i = 0; i < NBARS; ++i) umma::mbar_init(&bars[i], i == 4 || i == 6 ? 8 : 1);
         umma::fence_mbar_init();
         *abort_flag = *p.err;
     }
     __syncthreads();
     if (*abort_flag) return;
-    if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tc::TM_COLS);
+    if (warp == tc::MMA_WARP) umma::tmem_alloc(tmem_slot, tca::TM_COLS);
     if (warp < 8) {
-        for (int e = tid; e < SEG * 64 * 2; e += 256) {
-            const int i = e >> 1, j = e & 1, t = r * SEG * 64 + i;
-            sLam[j * SEG * 64 + i] = t < p.T && 8 + j < p.L ? p.l[(((long)b * p.T + t) * p.H + h) * p.L + 8 + j] : __float2bfloat16(0.f);
+        const unsigned short* gl = reinterpret_cast<const unsigned short*>(p.l) + ((long)b * p.T * p.H + h) * p.L + 8 + (tid & 1);
+        unsigned short x[SEG * 64 * 2 / 256];
+#pragma unroll
+        for (int i = 0; i < SEG * 64 * 2 / 256; ++i) {
+            const int t = r * SEG * 64 + (tid >> 1) + i * 128;
+            x[i] = t < p.T && 8 + (tid & 1) < p.L ? __ldg(gl + (long)t * p.H * p.L) : (unsigned short)0;
         }
+#pragma unroll
+        for (int i = 0; i < SEG * 64 * 2 / 256; ++i) sLam[(tid & 1) * SEG * 64 + (tid >> 1) + i * 128] = __ushort_as_bfloat16(x[i]);
         segment_pair_sums(p, b, h, r, sGs, sTot, warp, lane);
     }
     umma::fence_before_sync();
@@ -310,7 +332,7 @@ __global__ void __launch_bounds__(tca::NTHREADS, 1) m2_adjoint_tc_kernel(const _
     umma::fence_after_sync();
     const uint32_t tbase = *tmem_slot;
 
-    // steps: q, do of the pairs 1..nr, then k, v of the pairs nc - 1..0
+    // steps, for every pair from the last one on: q, do if it reads (any but the segment's first), k, v if it is read
     if (warp == tca::TMA_WARP) {
         if (lane == 0) {
             if (later) {
@@ -318,207 +340,213 @@ __global__ void __launch_bounds__(tca::NTHREADS, 1) m2_adjoint_tc_kernel(const _
                 for (int bx = 0; bx < 2; ++bx) tma::load_panel(sHi + bx * tc::V_BYTES, &p.tm_dh, bx * 32, 0, (int)((bh * p.NS + r) * p.K), hi_full);
             }
             int s = 0;
-            for (; s < nr + nc; ++s) {
-                const int st = s & 1, pl = s < nr ? s + 1 : nc - 1 - (s - nr), row0 = (r * SEGP + pl) * tc::PT;
-                if (s >= 2 && !umma::mbar_wait(&empty[st], ((s - 2) >> 1) & 1, abort_flag)) break;
-                tma::expect_tx(&full[st], tc::Q_BYTES + tc::V_BYTES);
-                tma::load_seq_panel(sY + st * tc::V_BYTES, s < nr ? &p.tm_do : &p.tm_v, 0, h, row0, b, &full[st]);
-                tma::load_seq_panel(sX + st * tc::Q_BYTES, s < nr ? &p.tm_q : &p.tm_k, 0, grp, row0, b, &full[st]);
-                tma::load_seq_panel(sX + st * tc::Q_BYTES + tc::Q_BYTES / 2, s < nr ? &p.tm_q : &p.tm_k, 64, grp, row0, b, &full[st]);
-            }
+            bool ok = true;
+            for (int pl = npairs - 1; pl >= 0 && ok; --pl)
+                for (int own = 0; own < 2; ++own) {
+                    if (own ? pl >= nc : pl == 0) continue;
+                    if (s > 0 && !(ok = umma::mbar_wait(empty, (s - 1) & 1, abort_flag))) break;
+                    const int row0 = (r * SEGP + pl) * tc::PT;
+                    const CUtensorMap* x = own ? &p.tm_k : &p.tm_q;
+                    tma::expect_tx(full, tc::Q_BYTES + tc::V_BYTES);
+                    tma::load_seq_panel(sY, own ? &p.tm_v : &p.tm_do, 0, h, row0, b, full);
+                    tma::load_seq_panel(sX, x, 0, grp, row0, b, full);
+                    tma::load_seq_panel(sX + tc::Q_BYTES / 2, x, 64, grp, row0, b, full);
+                    ++s;
+                }
             // (see m2_readers_tc_kernel)
-            for (int i = max(0, s - 2); i < s; ++i) umma::mbar_wait(&full[i & 1], (i >> 1) & 1, 1u << 16);
+            if (s > 0) umma::mbar_wait(full, (s - 1) & 1, 1u << 16);
             if (later) umma::mbar_wait(hi_full, 0, 1u << 16);
         }
         __syncwarp();
     } else if (warp == tc::MMA_WARP) {
         constexpr uint32_t ID_MM64 = umma::idesc_bf16(128, 64, true, true);
         const uint32_t lead = umma::elect_one();
+        const uint32_t aX = umma::smem_addr(sX), aY = umma::smem_addr(sY), aD = umma::smem_addr(sD);
         auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, umma::mbar_wait(bar, parity, abort_flag)); };
-        int st = 0, s = 0;
-        uint32_t ph = 0;
+        int s = 0, nd = 0, ns = 0, nr = 0;
         bool ok = true;
-        auto job = [&](uint32_t aQ, int slot) -> bool {
-            if (!wait(&st_full[st], ph)) return false;
+        auto job = [&](int slot, bool accumulate) -> bool {
+            if (!wait(d_full, nd & 1)) return false;
+            ++nd;
             umma::fence_after_sync();
-            umma::gemm_mm_lead<tc::PT, tc::PT, tc::PT>(lead, tbase + slot * 64, aQ, umma::smem_addr(sSt + st * tc::V_BYTES), ID_MM64, false);
-            umma::commit_lead(lead, &st_empty[st]);
-            if (++st == tca::NST) {
-                st = 0;
-                ph ^= 1;
-            }
+            umma::gemm_mm_lead<tc::PT, tc::PT, tc::PT>(lead, tbase + slot * 64, aX, aD, ID_MM64, accumulate);
+            umma::commit_lead(lead, d_empty);
             return true;
         };
-        for (; s < nr && ok; ++s) {
-            const int pl = s + 1;
-            if (!(ok = wait(&full[s & 1], (s >> 1) & 1))) break;
-            const uint32_t aQ = umma::smem_addr(sX + (s & 1) * tc::Q_BYTES);
-            if (pl & 1) ok = job(aQ, pl == 1 ? 0 : 3);
-            if (ok && pl >= 2) ok = job(aQ, pl - 1);
-            umma::commit_lead(lead, &empty[s & 1]);
+        for (int pl = npairs - 1; pl >= 0 && ok; --pl) {
+            if (pl > 0) {
+                if (!(ok = wait(full, s & 1))) break;
+                if (pl >= 2) ok = job(tca::SLOT_R1, pl == 2 && npairs == 4);
+                if (ok && (pl & 1)) ok = job(tca::SLOT_R0, false);
+                umma::commit_lead(lead, empty);
+                umma::commit_lead(lead, r_full);
+                ++nr;
+                ++s;
+                if (!ok) break;
+            }
+            if (pl < nc) {
+                if (!(ok = wait(scaled, ns & 1))) break;
+                ++ns;
+                umma::fence_after_sync();
+                umma::gemm_mm_lead<tc::PT, tc::PT, 64>(lead, tbase + tca::SLOT_KV * 64, aX, aY, ID_MM64, false);                   // first chunk of the pair
+                umma::gemm_mm_lead<tc::PT, tc::PT, 64>(lead, tbase + (tca::SLOT_KV + 1) * 64, aX + 64 * umma::ROW_BYTES, aY + 64 * umma::ROW_BYTES, ID_MM64, false);
+                umma::commit_lead(lead, empty);
+                umma::commit_lead(lead, kv_full);
+                ++s;
+            }
         }
-        umma::commit_lead(lead, r_full);
-        for (; s < nr + nc && ok; ++s) {
-            const int i = s - nr;
-            if (!(ok = wait(&scaled[i & 1], (i >> 1) & 1))) break;
-            umma::fence_after_sync();
-            const uint32_t aK = umma::smem_addr(sX + (s & 1) * tc::Q_BYTES), aV = umma::smem_addr(sY + (s & 1) * tc::V_BYTES);
-            const uint32_t d = tbase + (tca::SLOT_KV + (i & 1) * 2) * 64;
-            umma::gemm_mm_lead<tc::PT, tc::PT, 64>(lead, d, aK, aV, ID_MM64, false);                                           // first chunk of the pair
-            umma::gemm_mm_lead<tc::PT, tc::PT, 64>(lead, d + 64, aK + 64 * umma::ROW_BYTES, aV + 64 * umma::ROW_BYTES, ID_MM64, false);
-            umma::commit_lead(lead, &empty[s & 1]);
-            umma::commit_lead(lead, &kv_full[i & 1]);
+        if (!ok) {
+            // gave up: no product may still read shared memory when the CTA ends
+            umma::commit_lead(lead, hi_full);
+            umma::mbar_wait(hi_full, later ? 1 : 0, 1u << 16);
         }
-        if (!ok) umma::mbar_wait(r_full, 0, 1u << 16);   // gave up: no product may still read shared memory when the CTA ends (the later ones are short)
         __syncwarp();
     } else {
         const int rb = warp & 3, row = rb * 32 + lane, ch = warp >> 2;
-        {
-            int st = 0;
-            uint32_t ph = 1;
-            auto copy = [&](const uint4 (&dox)[4], float rs) {
-                umma::mbar_wait(&st_empty[st], ph, abort_flag);
-                scaled_half_row(sSt + st * tc::V_BYTES, dox, rs, row, ch);
-                umma::fence_async_smem();
-                __syncwarp();
-                if (lane == 0) arrive_on(&st_full[st]);
-                if (++st == tca::NST) {
-                    st = 0;
-                    ph ^= 1;
-                }
-            };
-            for (int s = 0; s < nr; ++s) {
-                const int pl = s + 1;
+        const uint32_t tcol = umma::tmem_addr(tbase, warp, ch * 32);
+        int s = 0, nd = 0, nkv = 0, nr = 0, seen = 0;        // steps, copies, summaries, reading steps so far; those whose products are known to be complete
+        bool stored = false;
+        float since = 0.f;                           // decay over the pairs behind this one
+        if (later) umma::mbar_wait(hi_full, 0, abort_flag);
+        for (int pl = npairs - 1; pl >= 0; --pl) {
+            const float glp = sGs[pl * tc::PT + tc::PT - 1];
+            if (pl > 0) {
                 const float e = fexp(sGs[pl * tc::PT + row]);
-                umma::mbar_wait(&full[s & 1], (s >> 1) & 1, abort_flag);
+                umma::mbar_wait(full, s & 1, abort_flag);
+                ++s;
                 uint4 dox[4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    dox[c] = *reinterpret_cast<const uint4*>(sY + (s & 1) * tc::V_BYTES + umma::tile_offset(row, ch * 32 + c * 8, tc::PT));
-                if (pl & 1) copy(dox, __bfloat162float(sLam[pl * tc::PT + row]) * e);
-                if (pl >= 2) copy(dox, __bfloat162float(sLam[SEG * 64 + pl * tc::PT + row]) * e);
-            }
-        }
-        auto scale_v = [&](int i) {
-            const int s = nr + i, pl = nc - 1 - i;
-            umma::mbar_wait(&full[s & 1], (s >> 1) & 1, abort_flag);
-            unsigned char* cV = sY + (s & 1) * tc::V_BYTES;
-            const float glp = sGs[pl * tc::PT + tc::PT - 1];
+                for (int c = 0; c < 4; ++c) dox[c] = *reinterpret_cast<const uint4*>(sY + umma::tile_offset(row, ch * 32 + c * 8, tc::PT));
+                auto copy = [&](float rs) {
+                    if (nd > 0) umma::mbar_wait(d_empty, (nd - 1) & 1, abort_flag);
+                    if (stored) {
+                        if (tid == 0) tma::wait_group_read0();
+                        bar_compute();
+                        stored = false;
+                    }
+                    ++nd;
+                    scaled_half_row(sD, dox, rs, row, ch);
+                    umma::fence_async_smem();
+                    umma::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) arrive_on(d_full);
+                };
+                if (pl >= 2) {
+                    if (pl == 2 && npairs == 4) {
+                        // what pair 3 sent back has decayed over pair 2, which adds to it
+                        for (; seen < nr; ++seen) umma::mbar_wait(r_full, seen & 1, abort_flag);
+                        umma::fence_after_sync();
+                        const float dec = fexp(glp);
 #pragma unroll
-            for (int x = tid; x < tc::PT * (tc::VD / 8); x += 256) {
-                const int j = x / (tc::VD / 8), c = (x % (tc::VD / 8)) * 8;
-                const float sc = fexp(glp - sGs[pl * tc::PT + j]);
-                const uint32_t off = umma::tile_offset(j, c, tc::PT);
-                uint4 y = *reinterpret_cast<const uint4*>(cV + off);
-                uint32_t* yw = reinterpret_cast<uint32_t*>(&y);
+                        for (int c = 0; c < 32; c += 16) {
+                            float t[16];
+                            umma::tmem_ld16(tcol + tca::SLOT_R1 * 64 + c, t);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) yw[e] = pack_bf16(__uint_as_float(yw[e] << 16) * sc, __uint_as_float(yw[e] & 0xffff0000u) * sc);
-                *reinterpret_cast<uint4*>(cV + off) = y;
-            }
-            umma::fence_async_smem();
-            umma::fence_before_sync();               // (the chunk summaries that these products overwrite have been read)
-            __syncwarp();
-            if (lane == 0) arrive_on(&scaled[i & 1]);
-        };
-        // R0 (level 0, for even pairs), R1 (level 1), the segment's: this thread's 32 columns of state row `row`
-        float R0[32], R1[32], Hi[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) R0[e] = R1[e] = Hi[e] = 0.f;
-        if (nc > 0) scale_v(0);
-        if (later) {
-            umma::mbar_wait(hi_full, 0, abort_flag);
-            if (row < p.K)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const float4 x = *reinterpret_cast<const float4*>(sHi + ch * tc::V_BYTES + row * 128 + ((c ^ (row & 7)) << 4));
-                Hi[c * 4] = x.x; Hi[c * 4 + 1] = x.y; Hi[c * 4 + 2] = x.z; Hi[c * 4 + 3] = x.w;
-            }
-        }
-        umma::mbar_wait(r_full, 0, abort_flag);
-        umma::fence_after_sync();
-        // (what pair 2 or pair 1 finds where the walk starts there, at the end of a sequence)
-        if (nc == 3 || nc == 2) umma::tmem_ld32(umma::tmem_addr(tbase + (nc - 1) * 64, warp, ch * 32), R1);
-        for (int i = 0; i < nc; ++i) {
-            const int pl = nc - 1 - i;
-            if (i + 1 < nc) scale_v(i + 1);
-            const bool l0 = (pl & 1) == 0 && pl + 1 < npairs, l1 = pl < 2 && npairs > 2;
-            if (l0) umma::tmem_ld32(umma::tmem_addr(tbase + (pl == 0 ? 0 : 3) * 64, warp, ch * 32), R0);
-            float ka[32], kb[32];
-            umma::mbar_wait(&kv_full[i & 1], (i >> 1) & 1, abort_flag);
-            umma::fence_after_sync();
-            umma::tmem_ld32(umma::tmem_addr(tbase + (tca::SLOT_KV + (i & 1) * 2) * 64, warp, ch * 32), ka);
-            umma::tmem_ld32(umma::tmem_addr(tbase + (tca::SLOT_KV + (i & 1) * 2 + 1) * 64, warp, ch * 32), kb);
-            uint32_t pk[16];
-            float y[6];
-#pragma unroll
-            for (int u = 0; u < 6; ++u) y[u] = 0.f;
-#pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-                float x0 = Hi[e], x1 = Hi[e + 1];
-                y[4] += ka[e] * x0 + ka[e + 1] * x1;
-                y[5] += kb[e] * x0 + kb[e + 1] * x1;
-                if (l0) {
-                    y[0] += ka[e] * R0[e] + ka[e + 1] * R0[e + 1];
-                    y[1] += kb[e] * R0[e] + kb[e + 1] * R0[e + 1];
-                    x0 += R0[e];
-                    x1 += R0[e + 1];
+                            for (int i = 0; i < 16; ++i) t[i] *= dec;
+                            umma::tmem_st16(tcol + tca::SLOT_R1 * 64 + c, t);
+                        }
+                        umma::tmem_wait_st();
+                    }
+                    copy(__bfloat162float(sLam[SEG * 64 + pl * tc::PT + row]) * e);
                 }
-                if (l1) {
-                    y[2] += ka[e] * R1[e] + ka[e + 1] * R1[e + 1];
-                    y[3] += kb[e] * R1[e] + kb[e + 1] * R1[e + 1];
-                    x0 += R1[e];
-                    x1 += R1[e + 1];
+                if (pl & 1) copy(__bfloat162float(sLam[pl * tc::PT + row]) * e);
+                ++nr;
+            }
+            if (pl < nc) {
+                umma::mbar_wait(full, s & 1, abort_flag);
+                ++s;
+#pragma unroll
+                for (int x = tid; x < tc::PT * (tc::VD / 8); x += 256) {
+                    const int j = x / (tc::VD / 8), c = (x % (tc::VD / 8)) * 8;
+                    const float sc = fexp(glp - sGs[pl * tc::PT + j]);
+                    const f32x2 sc2 = pack2(sc, sc);
+                    const uint32_t off = umma::tile_offset(j, c, tc::PT);
+                    uint4 y = *reinterpret_cast<const uint4*>(sY + off);
+                    uint32_t* yw = reinterpret_cast<uint32_t*>(&y);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) yw[e] = pack_bf16(mul2(bf16x2_f32x2(yw[e]), sc2));
+                    *reinterpret_cast<uint4*>(sY + off) = y;
                 }
-                pk[e >> 1] = pack_bf16(x0, x1);
-            }
+                umma::fence_async_smem();
+                umma::fence_before_sync();           // (the summaries that these products overwrite have been read)
+                __syncwarp();
+                if (lane == 0) arrive_on(scaled);
+                const bool l0 = (pl & 1) == 0 && pl + 1 < npairs, l1 = pl < 2 && npairs > 2;
+                // factors of the parts: later segments', pair level 0's, pair level 1's (decayed over pair 1 for pair 0)
+                const float fh = later && row < p.K ? fexp(since) : 0.f, f1 = pl == 0 ? fexp(sGs[2 * tc::PT - 1]) : 1.f;
+                for (; seen < nr; ++seen) umma::mbar_wait(r_full, seen & 1, abort_flag);
+                if (nd > 0) umma::mbar_wait(d_empty, (nd - 1) & 1, abort_flag);
+                if (stored) {
+                    if (tid == 0) tma::wait_group_read0();
+                    bar_compute();
+                }
+                umma::mbar_wait(kv_full, nkv & 1, abort_flag);
+                ++nkv;
+                umma::fence_after_sync();
+                f32x2 y2[6];
 #pragma unroll
-            for (int u = 0; u < 6; ++u) {
+                for (int u = 0; u < 6; ++u) y2[u] = 0;
+                const f32x2 fh2 = pack2(fh, fh), f12 = pack2(f1, f1);
+#pragma unroll 1
+                for (int c = 0; c < 32; c += 8) {
+                    // eight columns at a time: the state parts, then the two chunks' summaries against them
+                    f32x2 hi2[4], r0[4], r1[4], sum[4];
+                    const float4 ha = *reinterpret_cast<const float4*>(sHi + ch * tc::V_BYTES + row * 128 + (((c >> 2) ^ (row & 7)) << 4));
+                    const float4 hb = *reinterpret_cast<const float4*>(sHi + ch * tc::V_BYTES + row * 128 + ((((c >> 2) + 1) ^ (row & 7)) << 4));
+                    float ka[8], kb[8], ta[8], tb[8];
+                    umma::tmem_ld8x4(tcol + tca::SLOT_KV * 64 + c, ka, tcol + (tca::SLOT_KV + 1) * 64 + c, kb, tcol + tca::SLOT_R0 * 64 + c, ta,
+                                     tcol + tca::SLOT_R1 * 64 + c, tb);
+                    hi2[0] = pack2(ha.x, ha.y); hi2[1] = pack2(ha.z, ha.w); hi2[2] = pack2(hb.x, hb.y); hi2[3] = pack2(hb.z, hb.w);
 #pragma unroll
-                for (int d = 16; d > 0; d >>= 1) y[u] += __shfl_xor_sync(0xffffffffu, y[u], d);
-                if (lane == 0) sYs[warp * 8 + u] = y[u];
-            }
-            unsigned char* out = sSt + (i % tca::NST) * tc::V_BYTES;
-            if (i >= tca::NST) {
-                if (tid == 0) tma::wait_group_read<tca::NST - 1>();
+                    for (int e = 0; e < 4; ++e) {
+                        // (what a slot holds before it was ever written, or a row of the summary that does not exist, is no number: selected away)
+                        hi2[e] = fh != 0.f ? mul2(hi2[e], fh2) : 0;
+                        r0[e] = l0 ? pack2(ta[2 * e], ta[2 * e + 1]) : 0;
+                        r1[e] = l1 ? mul2(pack2(tb[2 * e], tb[2 * e + 1]), f12) : 0;
+                        const f32x2 one = pack2(1.f, 1.f);
+                        sum[e] = fma2(r1[e], one, fma2(r0[e], one, hi2[e]));
+                        const f32x2 a2 = pack2(ka[2 * e], ka[2 * e + 1]), b2 = pack2(kb[2 * e], kb[2 * e + 1]);
+                        y2[0] = fma2(a2, r0[e], y2[0]);
+                        y2[1] = fma2(b2, r0[e], y2[1]);
+                        y2[2] = fma2(a2, r1[e], y2[2]);
+                        y2[3] = fma2(b2, r1[e], y2[3]);
+                        y2[4] = fma2(a2, hi2[e], y2[4]);
+                        y2[5] = fma2(b2, hi2[e], y2[5]);
+                    }
+                    *reinterpret_cast<uint4*>(sD + umma::tile_offset(row, ch * 32 + c, tc::PT)) =
+                        make_uint4(pack_bf16(sum[0]), pack_bf16(sum[1]), pack_bf16(sum[2]), pack_bf16(sum[3]));
+                }
+#pragma unroll
+                for (int u = 0; u < 6; ++u) {
+                    float y = sum2(y2[u]);
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) y += __shfl_xor_sync(0xffffffffu, y, d);
+                    if (lane == 0) sYs[warp * 8 + u] = y;
+                }
+                umma::fence_async_smem();
+                umma::fence_before_sync();
                 bar_compute();
-            }
+                if (tid == 0) {
+                    if (!*abort_flag) tma::store_box(&p.tm_lo_a, 0, 0, (int)((bh * NP + r * SEGP + pl) * p.K), sD);
+                    tma::commit_group();
+                }
+                stored = true;
+                if (tid >= 32 && tid < 38) {
+                    // contributor totals per chunk: pair levels 0, 1, then the high ones together
+                    const int u = tid - 32;
+                    float t = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                *reinterpret_cast<uint4*>(out + umma::tile_offset(row, ch * 32 + c * 8, p.K)) = make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
-            umma::fence_async_smem();
-            bar_compute();
-            if (tid == 0) {
-                if (!*abort_flag) tma::store_box(&p.tm_lo_a, 0, 0, (int)((bh * NP + r * SEGP + pl) * p.K), out);
-                tma::commit_group();
+                    for (int w = 0; w < 8; ++w) t += sYs[w * 8 + u];
+                    const int c = (r * SEGP + pl) * 2 + (u & 1);
+                    if (c < p.NT) p.Yc[(bh * p.NT + c) * (MLOW + 1) + 1 + (u >> 1)] = t;
+                }
+                bar_compute();                       // the totals have been read
+            } else if (warp == 0 && lane < 6) {
+                // the sequence's last pair: nobody reads it
+                const int c = (NP - 1) * 2 + (lane & 1);
+                if (c < p.NT) p.Yc[(bh * p.NT + c) * (MLOW + 1) + 1 + (lane >> 1)] = 0.f;
             }
-            if (tid >= 32 && tid < 38) {
-                // contributor totals per chunk: pair levels 0, 1, then the high ones together
-                const int u = tid - 32;
-                float t = 0.f;
-#pragma unroll
-                for (int w = 0; w < 8; ++w) t += sYs[w * 8 + u];
-                const int c = (r * SEGP + pl) * 2 + (u & 1);
-                if (c < p.NT) p.Yc[(bh * p.NT + c) * (MLOW + 1) + 1 + (u >> 1)] = t;
-            }
-            // one pair further back: what the later ones send has decayed over this one, which adds what it reads itself
-            const float dec = fexp(sGs[pl * tc::PT + tc::PT - 1]);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-                Hi[e] *= dec;
-                R1[e] *= dec;
-            }
-            if (pl >= 2) {
-                float t[32];
-                umma::tmem_ld32(umma::tmem_addr(tbase + (pl - 1) * 64, warp, ch * 32), t);
-#pragma unroll
-                for (int e = 0; e < 32; ++e) R1[e] += t[e];
-            }
-            bar_compute();                           // the totals have been read
-        }
-        if (nc < npairs && warp == 0 && lane < 6) {
-            // the sequence's last pair: nobody reads it
-            const int c = (NP - 1) * 2 + (lane & 1);
-            if (c < p.NT) p.Yc[(bh * p.NT + c) * (MLOW + 1) + 1 + (lane >> 1)] = 0.f;
+            since += glp;
         }
         if (tid == 0) tma::wait_group0();
     }
@@ -527,7 +555,7 @@ __global__ void __launch_bounds__(tca::NTHREADS, 1) m2_adjoint_tc_kernel(const _
     umma::fence_after_sync();
     if (warp == tc::MMA_WARP) {
         if (*abort_flag && lane == 0) atomicExch(p.err, 1);
-        umma::tmem_dealloc(tbase, tc::TM_COLS);
+        umma::tmem_dealloc(tbase, tca::TM_COLS);
     }
 }
 
@@ -760,10 +788,8 @@ int mamba2_readers_tc_launch(const Mamba2Params& p_in, cudaStream_t stream) {
     const size_t sm = ReadersTcSmem<M2_MLOW>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
-    // one launch per window of five segment levels (a single one up to T = 16384); their outputs are disjoint
-    for (p.lev_lo = 0; p.lev_lo < p.LH; p.lev_lo += tcr::MAXLH) {
-        llattn::launch_chained(kern, p.B * p.H * (p.NS - 1), tcr::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
-    }
+    // (CTAs for levels that a segment does not have end at once: 1 segment in 32 has five up to T = 16384)
+    llattn::launch_chained(kern, p.B * p.H * (p.NS - 1) * ((p.LH + tcr::MAXLH - 1) / tcr::MAXLH), tcr::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
 }
 
