@@ -438,73 +438,63 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
                     *reinterpret_cast<uint4*>(sDS + umma::tile_offset(row, j0 + c * 8, tc::PT)) =
                         make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]);
             }
-            // diagonal block: levels 0..5, causal mask folded into the exponent.  The level of (row, column) is the position of the highest bit in
-            // which they differ.  With the column's low four bits a compile-time constant, "bit k differs" is one of the thread's own bits or its
-            // complement, so lambda is picked with four selects on predicates; and the d lambda sum of level k is the sum over the sibling block of
-            // size 2^(k-1) of the row's own position, taken from a binary tree of partial sums.  A thread whose sixteen columns lie in the other half
-            // of the 32-block (bit 4 differs) has level 5 throughout.
-            {
-                const int j0 = rb * 32 + ch * 16;
-                uint32_t packed[8];
-                float s[16], dp[16];
-                umma::tmem_ld16x2(umma::tmem_addr(tbase + tcq::TM_S, warp, j0), s, umma::tmem_addr(tbase + tcq::TM_DP, warp, j0), dp);
-                // per half of eight columns: what the levels 0..3 would get if the row's own position lay in this half, and the half's sum
-                float c_own[2], c_sib1[2], c_sib2[2], c_sib4[2], c_sum[2];
+            // diagonal block, eight columns at a time (a run-time loop: short code, see below): levels 0..5, causal mask folded into the exponent.  The level of
+            // (row, column) is the position of the highest bit in which they differ: lambda is picked by selects on the row's own bits, and the d lambda sum of
+            // level k is the sum over the sibling block of size 2^(k-1) of the row's own position, taken from a binary tree of partial sums.  A thread whose
+            // columns lie in the other half of the 32-block (bit 4 differs) has level 5 throughout.
+            // Short code: four or five warps of a scheduler in as many roles do not fit its instruction cache with their loops unrolled (1.4 of 13.7 warps
+            // waited for instructions).
+#pragma unroll 1
+            for (int hf = 0; hf < 2; ++hf) {
+                const int j0 = rb * 32 + ch * 16 + hf * 8;
+                const bool q3 = B3 != (hf != 0);                               // the columns are in the other half of the row's sixteen
+                float s[8], dp[8], es[8];
+                umma::tmem_ld8x2(umma::tmem_addr(tbase + tcq::TM_S, warp, j0), s, umma::tmem_addr(tbase + tcq::TM_DP, warp, j0), dp);
+                const float lm45 = hi ? lam[5] : lam[4];
+                const bool far = hi || q3;
+                uint32_t packed[4];
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    float es[8];
+                for (int e = 0; e < 8; e += 4) {
+                    const float4 gj = *reinterpret_cast<const float4*>(tG + j0 + e);
+                    const float gjv[4] = {gj.x, gj.y, gj.z, gj.w};
 #pragma unroll
-                    for (int e = 0; e < 8; e += 4) {
-                        const float4 gj = *reinterpret_cast<const float4*>(tG + j0 + hf * 8 + e);
-                        const float gjv[4] = {gj.x, gj.y, gj.z, gj.w};
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int ee = hf * 8 + e + u;                     // low four bits of the column
-                        const int jj = ch * 16 + ee;
-                        const float d = (jj <= lane) ? (Gi - gjv[u]) : -INFINITY;
+                    for (int u = 0; u < 4; ++u) {
+                        const int ee = e + u;                                  // low three bits of the column
+                        const float d = (ch * 16 + hf * 8 + ee <= lane) ? (Gi - gjv[u]) : -INFINITY;
                         const float ed = dp[ee] * fexp(d);
-                        es[e + u] = ed * s[ee];
-                        const bool q3 = hf ? !B3 : B3, q2 = ((ee >> 2) & 1) ? !B2 : B2;
-                        const bool q1 = ((ee >> 1) & 1) ? !B1 : B1, q0 = (ee & 1) ? !B0 : B0;
+                        es[ee] = ed * s[ee];
+                        const bool q2 = (ee & 4) ? !B2 : B2, q1 = (ee & 2) ? !B1 : B1, q0 = (ee & 1) ? !B0 : B0;
                         float lm = q0 ? lam[1] : lam[0];
                         lm = q1 ? lam[2] : lm;
                         lm = q2 ? lam[3] : lm;
-                        lm = q3 ? lam[4] : lm;
-                        lm = hi ? lam[5] : lm;
+                        lm = far ? lm45 : lm;
                         dp[ee] = ed * lm;
                     }
 #pragma unroll
                     for (int u = 0; u < 4; u += 2) {
-                        const int ee = hf * 8 + e + u;
-                        const uint32_t ds = pack_bf16(dp[ee], dp[ee + 1]);
-                        wq2 = fma2(bf16x2_f32x2(ds), pack2(s[ee], s[ee + 1]), wq2);
-                        packed[ee >> 1] = ds;
+                        const uint32_t ds = pack_bf16(dp[e + u], dp[e + u + 1]);
+                        wq2 = fma2(bf16x2_f32x2(ds), pack2(s[e + u], s[e + u + 1]), wq2);
+                        packed[(e + u) >> 1] = ds;
                     }
                 }
-                    // walk down the half's tree of partial sums along the row's own bits 2, 1, 0
-                    const float p0 = es[0] + es[1], p1 = es[2] + es[3], p2 = es[4] + es[5], p3 = es[6] + es[7];
-                    const float q0s = p0 + p1, q1s = p2 + p3;
-                    c_sum[hf] = q0s + q1s;
-                    c_sib4[hf] = B2 ? q0s : q1s;
-                    const float e0 = B2 ? p2 : p0, e1 = B2 ? p3 : p1;
-                    c_sib2[hf] = B1 ? e0 : e1;
-                    float f4[4];
+                *reinterpret_cast<uint4*>(sDS + umma::tile_offset(row, j0, tc::PT)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                // walk down the tree of partial sums along the row's own bits 2, 1, 0
+                const float p0 = es[0] + es[1], p1 = es[2] + es[3], p2 = es[4] + es[5], p3 = es[6] + es[7];
+                const float q0s = p0 + p1, q1s = p2 + p3, sum = q0s + q1s;
+                const float e0 = B2 ? p2 : p0, e1 = B2 ? p3 : p1;
+                float f4[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) f4[i] = B2 ? es[4 + i] : es[i];
-                    const float g0 = B1 ? f4[2] : f4[0], g1 = B1 ? f4[3] : f4[1];
-                    c_sib1[hf] = B0 ? g0 : g1;
-                    c_own[hf] = B0 ? g1 : g0;
+                for (int i = 0; i < 4; ++i) f4[i] = B2 ? es[4 + i] : es[i];
+                const float g0 = B1 ? f4[2] : f4[0], g1 = B1 ? f4[3] : f4[1];
+                if (far) {
+                    bins[4] += hi ? 0.f : sum;
+                    bins[5] += hi ? sum : 0.f;
+                } else {
+                    bins[0] = B0 ? g1 : g0;
+                    bins[1] = B0 ? g0 : g1;
+                    bins[2] = B1 ? e0 : e1;
+                    bins[3] = B2 ? q0s : q1s;
                 }
-                bins[0] = hi ? 0.f : (B3 ? c_own[1] : c_own[0]);
-                bins[1] = hi ? 0.f : (B3 ? c_sib1[1] : c_sib1[0]);
-                bins[2] = hi ? 0.f : (B3 ? c_sib2[1] : c_sib2[0]);
-                bins[3] = hi ? 0.f : (B3 ? c_sib4[1] : c_sib4[0]);
-                bins[4] = hi ? 0.f : (B3 ? c_sum[0] : c_sum[1]);
-                bins[5] = hi ? (c_sum[0] + c_sum[1]) : 0.f;
-#pragma unroll
-                for (int c = 0; c < 2; ++c)
-                    *reinterpret_cast<uint4*>(sDS + umma::tile_offset(row, j0 + c * 8, tc::PT)) =
-                        make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]);
             }
             // (a thread whose columns of the diagonal block lie in the row's own half has levels 0..4 of the row, the other one level 5)
             float* myDL = sDL + ((hh & 1) * 128 + row) * tcq::NSUM;
@@ -698,7 +688,6 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
     uint32_t* sink = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 212);     // written only (tile release)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int L = p.L, ncol = min(L, tck::NINTRA);
     const PairWork w(p);
     // whether somebody reads a state that this pair contributes to: any pair but the last one has readers
     const bool read = w.pair + 1 < w.NP;
@@ -724,7 +713,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
     } else {
         HeadsOfTokens<tcg::WORKERS> g;
         g.load(p.g, p, w.b, w.t0, w.h0, w.nh, tid);
-        stage_lambda<tck::LAM_LD, tcg::WORKERS / 32>(p, w.b, w.t0, w.h0, w.nh, ncol, sLam, warp, lane);
+        stage_lambda<tck::LAM_LD, tcg::WORKERS / 32>(p, w.b, w.t0, w.h0, w.nh, tck::NINTRA, sLam, warp, lane);
         g.to_shared<256>(sG, w.nh, tid);
         asm volatile("bar.sync 1, 512;\n" ::: "memory");
         if (warp < w.nh) pair_decay_tables<2>(sG + warp * 256, nullptr, lane);
@@ -892,7 +881,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
                 // lane i of a half warp makes the factor of target i0 + i: exp(G_i - gend), lambda_i
                 const int lev = ((rb ^ ib) == 1) ? 6 : 7, it = i0 + (lane & 15);
                 const float fe = fexp(tG[it] - gend);
-                const float fl = lev < ncol ? __bfloat162float(sLam[it * tck::LAM_LD + hh * ncol + lev]) : 0.f;
+                const float fl = __bfloat162float(sLam[it * tck::LAM_LD + hh * tck::NINTRA + lev]);
                 float s[16], dp[16];
                 umma::tmem_ld16x2(umma::tmem_addr(tbase + tck::TM_S, warp, i0), s, umma::tmem_addr(tbase + tck::TM_DP, warp, i0), dp);
 #pragma unroll
@@ -906,43 +895,40 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
                 }
                 store(i0);
             }
-            {
-                // diagonal block: the level of (target, source) is the position of the highest bit in which they differ; the target's six lambdas are one
-                // load for all lanes, the selects are on the source's own bits
-                const int i0 = rb * 32 + ch * 16;
-                float s[16], dp[16];
-                umma::tmem_ld16x2(umma::tmem_addr(tbase + tck::TM_S, warp, i0), s, umma::tmem_addr(tbase + tck::TM_DP, warp, i0), dp);
+            // diagonal block, eight columns at a time: the level of (target, source) is the position of the highest bit in which they differ; a target's six
+            // lambdas are one load for all lanes, the selects are on the source's own bits
+#pragma unroll 1
+            for (int hf = 0; hf < 2; ++hf) {
+                const int i0 = rb * 32 + ch * 16 + hf * 8;
+                const bool q3 = B3 != (hf != 0);
+                float s[8], dp[8];
+                umma::tmem_ld8x2(umma::tmem_addr(tbase + tck::TM_S, warp, i0), s, umma::tmem_addr(tbase + tck::TM_DP, warp, i0), dp);
+                const bf16* lrow = sLam + i0 * tck::LAM_LD + hh * tck::NINTRA;
 #pragma unroll
-                for (int e = 0; e < 16; e += 2) {
+                for (int e = 0; e < 8; e += 2) {
                     const float2 gi = *reinterpret_cast<const float2*>(tG + i0 + e);
-                    const bool q1 = (e & 2) ? !B1 : B1, q2 = (e & 4) ? !B2 : B2, q3 = (e & 8) ? !B3 : B3;
+                    const bool q1 = (e & 2) ? !B1 : B1, q2 = (e & 4) ? !B2 : B2;
                     float lmv[2], dcv[2];
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
-                        uint32_t lw[4];
-                        if (ncol == tck::NINTRA) {
-                            const uint4 x = *reinterpret_cast<const uint4*>(sLam + (i0 + e + u) * tck::LAM_LD + hh * tck::NINTRA);
-                            lw[0] = x.x; lw[1] = x.y; lw[2] = x.z; lw[3] = x.w;
-                        } else {
-                            const unsigned short* x = reinterpret_cast<const unsigned short*>(sLam + (i0 + e + u) * tck::LAM_LD + hh * ncol);
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) lw[c] = x[2 * c] | (uint32_t)x[2 * c + 1] << 16;
-                        }
+                        const uint4 lw = *reinterpret_cast<const uint4*>(lrow + (e + u) * tck::LAM_LD);
                         const bool q0 = u ? !B0 : B0;
-                        uint32_t lm = q0 ? (lw[0] & 0xffff0000u) : (lw[0] << 16);
-                        lm = q1 ? (lw[1] << 16) : lm;
-                        lm = q2 ? (lw[1] & 0xffff0000u) : lm;
-                        lm = q3 ? (lw[2] << 16) : lm;
-                        lm = hi ? (lw[2] & 0xffff0000u) : lm;
+                        uint32_t lm = q0 ? (lw.x & 0xffff0000u) : (lw.x << 16);
+                        lm = q1 ? (lw.y << 16) : lm;
+                        lm = q2 ? (lw.y & 0xffff0000u) : lm;
+                        lm = q3 ? (lw.z << 16) : lm;
+                        lm = hi ? (lw.z & 0xffff0000u) : lm;
                         lmv[u] = __uint_as_float(lm);
-                        dcv[u] = fexp((ch * 16 + e + u >= lane) ? ((u ? gi.y : gi.x) - Gj) : -INFINITY);
+                        dcv[u] = fexp((ch * 16 + hf * 8 + e + u >= lane) ? ((u ? gi.y : gi.x) - Gj) : -INFINITY);
                     }
                     const f32x2 dec = pack2(dcv[0], dcv[1]), lm2 = pack2(lmv[0], lmv[1]), s2 = pack2(s[e], s[e + 1]);
                     pp[e >> 1] = pack_bf16(mul2(mul2(s2, dec), lm2));
                     pd[e >> 1] = pack_bf16(mul2(mul2(pack2(dp[e], dp[e + 1]), dec), lm2));
                     wk2 = fma2(bf16x2_f32x2(pd[e >> 1]), s2, wk2);
                 }
-                store(i0);
+                const uint32_t off = umma::tile_offset(row, i0, tc::PT);
+                *reinterpret_cast<uint4*>(sP + off) = make_uint4(pp[0], pp[1], pp[2], pp[3]);
+                *reinterpret_cast<uint4*>(sDS + off) = make_uint4(pd[0], pd[1], pd[2], pd[3]);
             }
             sW[((hh & 1) * 4 + ch) * 128 + row] = sum2(wk2);
             umma::fence_async_smem();

@@ -334,35 +334,36 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
             }
             // diagonal block: levels 0..5, causal mask folded into the exponent.  The level of (row, column) is the position of the highest bit in
             // which they differ: per bit, "differs" is the row's own bit or its complement, so lambda is picked by selects on predicates.
-            {
-                float s[32];
-                umma::tmem_ld32(umma::tmem_addr(tbase + tco::TM_S, warp, rb * 32), s);
+            // Eight columns at a time in a run-time loop: four or five warps of a scheduler in as many roles do not fit its instruction cache unrolled.
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                const int j0 = rb * 32 + c * 8;
+                const bool q3 = B3 != ((c & 1) != 0), q4 = B4 != ((c & 2) != 0);
+                const float lm45 = q4 ? lam[5] : lam[4];
+                const bool far = q3 || q4;
+                float s[8];
+                umma::tmem_ld8(umma::tmem_addr(tbase + tco::TM_S, warp, j0), s);
+                uint32_t x[4];
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    uint32_t x[8];
+                for (int e = 0; e < 8; e += 4) {
+                    const float4 gj = *reinterpret_cast<const float4*>(tG + j0 + e);
+                    const float gjv[4] = {gj.x, gj.y, gj.z, gj.w};
+                    const bool q2 = (e & 4) ? !B2 : B2;
+                    float y[4];
 #pragma unroll
-                    for (int e = 0; e < 16; e += 4) {
-                        const float4 gj = *reinterpret_cast<const float4*>(tG + rb * 32 + hf * 16 + e);
-                        const float gjv[4] = {gj.x, gj.y, gj.z, gj.w};
-                        const bool q2 = (e & 4) ? !B2 : B2, q3 = (e & 8) ? !B3 : B3, q4 = hf ? !B4 : B4;
-                        float y[4];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int jj = hf * 16 + e + u;
-                            const bool q1 = (u & 2) ? !B1 : B1, q0 = (u & 1) ? !B0 : B0;
-                            float lm = q0 ? lam[1] : lam[0];
-                            lm = q1 ? lam[2] : lm;
-                            lm = q2 ? lam[3] : lm;
-                            lm = q3 ? lam[4] : lm;
-                            lm = q4 ? lam[5] : lm;
-                            const float d = (jj <= lane) ? (Gi - gjv[u]) : -INFINITY;
-                            y[u] = s[jj] * fexp(d) * lm;
-                        }
-                        x[e / 2] = pack_bf16(y[0], y[1]);
-                        x[e / 2 + 1] = pack_bf16(y[2], y[3]);
+                    for (int u = 0; u < 4; ++u) {
+                        const bool q1 = (u & 2) ? !B1 : B1, q0 = (u & 1) ? !B0 : B0;
+                        float lm = q0 ? lam[1] : lam[0];
+                        lm = q1 ? lam[2] : lm;
+                        lm = q2 ? lam[3] : lm;
+                        lm = far ? lm45 : lm;
+                        const float d = (c * 8 + e + u <= lane) ? (Gi - gjv[u]) : -INFINITY;
+                        y[u] = s[e + u] * fexp(d) * lm;
                     }
-                    umma::tmem_st8u(dst + rb * 16 + hf * 8, x);
+                    x[e / 2] = pack_bf16(y[0], y[1]);
+                    x[e / 2 + 1] = pack_bf16(y[2], y[3]);
                 }
+                umma::tmem_st4u(dst + rb * 16 + c * 4, x);
             }
             umma::tmem_wait_st();
             umma::fence_before_sync();

@@ -150,7 +150,7 @@ __device__ __forceinline__ void pair_decay_tables(float* tG, float* cum, int lan
     *reinterpret_cast<float4*>(tG + 128 + 4 * lane) = make_float4(cf[0], cf[1], cf[2], cf[3]);
     if (TABLES == 3) *reinterpret_cast<float4*>(tG + 256 + 4 * lane) = make_float4(vf[0], vf[1], vf[2], vf[3]);
 }
-// lambda columns [0, ncol) of heads [h0, h0 + nh) for the 128 tokens from t0 on, ncol a head, as rows of LD values (zeros behind the sequence).  A warp takes
+// lambda columns [0, ncol) of heads [h0, h0 + nh) for the 128 tokens from t0 on, ncol a head, as rows of LD values (zeros behind the sequence and the levels).  A warp takes
 // a token at a time, eight or more in flight: with one index over all values (a division each, few loads in flight) this took 12 k cycles a CTA.
 template <int LD, int WARPS>
 __device__ __forceinline__ void stage_lambda(const Mamba2Params& p, int b, int t0, int h0, int nh, int ncol, bf16* sLam, int warp, int lane) {
@@ -177,9 +177,10 @@ __device__ __forceinline__ void stage_lambda(const Mamba2Params& p, int b, int t
         const unsigned short* g16 = reinterpret_cast<const unsigned short*>(gl);
         for (int c0 = 0; c0 < n; c0 += 32) {
             const int cc = c0 + lane, hh = cc / ncol, at = hh * L + cc - hh * ncol;
+            const bool there = cc < n && cc - hh * ncol < L;
             unsigned short x[ROWS];
 #pragma unroll
-            for (int i = 0; i < ROWS; ++i) x[i] = warp + i * WARPS < left && cc < n ? __ldg(g16 + (warp + i * WARPS) * ldg + at) : (unsigned short)0;
+            for (int i = 0; i < ROWS; ++i) x[i] = warp + i * WARPS < left && there ? __ldg(g16 + (warp + i * WARPS) * ldg + at) : (unsigned short)0;
 #pragma unroll
             for (int i = 0; i < ROWS; ++i)
                 if (cc < n) sLam[(warp + i * WARPS) * LD + cc] = __ushort_as_bfloat16(x[i]);
