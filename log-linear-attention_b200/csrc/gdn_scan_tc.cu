@@ -16,7 +16,10 @@
 // and consumed one chunk later.  The bf16 copies are kept transposed ([V column][K]) so that they are K-major B
 // operands whose rows continue from level to level: a range of levels is read by ONE chain with N = 32 x (number
 // of levels) (an instruction costs the same for N = 32 as for N = 128; slots of levels inside the range that are
-// not live receive products of stale copies and are never read).
+// not live receive products of stale copies and are never read).  The issuing warp stays converged and predicates
+// the instructions on an elected lane: the 20 instructions of a chunk are on its chain, and inside a branch of one
+// lane they took twice as long to issue (B = 4, T = 8192, H = 16, forward that keeps its states: 778 -> 747 us; 13 chunks of a prompt,
+// 16 heads: 30.3 -> 29.1; the reverse scan, whose products wait for their operands, is as it was, 725).
 #include "tc_common.cuh"
 #include "llattn_gdn.h"
 
@@ -157,6 +160,7 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
         const uint32_t tbase = *tmem_slot;
         const uint32_t aSt = umma::smem_addr(sSt);
         constexpr uint32_t ID_MK32 = umma::idesc_bf16(128, gtc::VS, true, false);
+        const uint32_t lead = umma::elect_one();
         bool ok = true;
         for (int c = 0; c < NT && ok; ++c) {
             const int st = c & 1;
@@ -170,50 +174,47 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
             int nstamp = 0;
             const int stamp_slot = (blockIdx.x == 5 && c == 37 && lane == 0) ? 2 : -1;
 #endif
-            if (lane == 0) {
-                STAMP();
-                ok = umma::mbar_wait(&full[st], (c >> 1) & 1, abort_flag);
-                if (ok && c > 0) ok = umma::mbar_wait(barS, (c - 1) & 1, abort_flag);
-                STAMP();
-                if (ok && trans) ok = umma::mbar_wait(&barU[st], (c >> 1) & 1, abort_flag);
-                if (ok) {
-                    umma::fence_after_sync();
-                    if (trans) {
-                        // the level that receives this chunk's writes starts from kd^T u (its slot held a dead level); the
-                        // levels below the carry (all live; the element-wise warps add them into that level afterwards) and the
-                        // live levels above it advance in place: master += Wd H_lv
-                        umma::gemm_mk<CH, gtc::VS, CH>(tbase + gtc::TM_M + jc * gtc::VS, aKd, aUT, ID_MK32, false);
-                        if (jc > 0)
-                            umma::gemm_kk<gtc::KD, gtc::ST_ROWS, gtc::KD>(tbase + gtc::TM_M, aWk, aSt, umma::idesc_bf16(128, gtc::VS * jc, false, false), true);
-                        const uint32_t above = live & ~((2u << jc) - 1u);
-                        if (above) {
-                            const int lo = __ffs(above) - 1, hi = 31 - __clz(above);
-                            umma::gemm_kk<gtc::KD, gtc::ST_ROWS, gtc::KD>(tbase + gtc::TM_M + lo * gtc::VS, aWk, aSt + lo * gtc::LV_BYTES,
-                                                                          umma::idesc_bf16(128, gtc::VS * (hi - lo + 1), false, false), true);
-                        }
-                        umma::commit(barT);
+            STAMP();
+            ok = umma::mbar_wait_warp(&full[st], (c >> 1) & 1, abort_flag);
+            if (ok && c > 0) ok = umma::mbar_wait_warp(barS, (c - 1) & 1, abort_flag);
+            STAMP();
+            if (ok && trans) ok = umma::mbar_wait_warp(&barU[st], (c >> 1) & 1, abort_flag);
+            if (ok) {
+                umma::fence_after_sync();
+                if (trans) {
+                    // the level that receives this chunk's writes starts from kd^T u (its slot held a dead level); the
+                    // levels below the carry (all live; the element-wise warps add them into that level afterwards) and the
+                    // live levels above it advance in place: master += Wd H_lv
+                    umma::gemm_mk_lead<CH, gtc::VS, CH>(lead, tbase + gtc::TM_M + jc * gtc::VS, aKd, aUT, ID_MK32, false);
+                    if (jc > 0)
+                        umma::gemm_kk_lead<gtc::KD, gtc::ST_ROWS, gtc::KD>(lead, tbase + gtc::TM_M, aWk, aSt, umma::idesc_bf16(128, gtc::VS * jc, false, false), true);
+                    const uint32_t above = live & ~((2u << jc) - 1u);
+                    if (above) {
+                        const int lo = __ffs(above) - 1, hi = 31 - __clz(above);
+                        umma::gemm_kk_lead<gtc::KD, gtc::ST_ROWS, gtc::KD>(lead, tbase + gtc::TM_M + lo * gtc::VS, aWk, aSt + lo * gtc::LV_BYTES,
+                                                                      umma::idesc_bf16(128, gtc::VS * (hi - lo + 1), false, false), true);
                     }
-                    STAMP();
-                    if (OUT) {
-                        if (c > 0) ok = umma::mbar_wait(barO, (c - 1) & 1, abort_flag);
-                        STAMP();
-                        if (ok && live) {
-                            umma::fence_after_sync();
-                            // readers: qd H_lv in rows 0..63 (rows 64..127 of the M = 128 product are not used), one chain from
-                            // the lowest to the highest live level
-                            const int lo = __ffs(live) - 1, hi = 31 - __clz(live);
-                            umma::gemm_kk<CH, gtc::ST_ROWS, gtc::KD>(tbase + gtc::TM_R + lo * gtc::VS, aQd, aSt + lo * gtc::LV_BYTES,
-                                                                     umma::idesc_bf16(128, gtc::VS * (hi - lo + 1), false, false), false);
-                            umma::commit(barR);
-                        }
-                    }
-                    if (ok) umma::commit(&empty[st]);
-                    STAMP();
+                    umma::commit_lead(lead, barT);
                 }
+                STAMP();
+                if (OUT) {
+                    if (c > 0) ok = umma::mbar_wait_warp(barO, (c - 1) & 1, abort_flag);
+                    STAMP();
+                    if (ok && live) {
+                        umma::fence_after_sync();
+                        // readers: qd H_lv in rows 0..63 (rows 64..127 of the M = 128 product are not used), one chain from
+                        // the lowest to the highest live level
+                        const int lo = __ffs(live) - 1, hi = 31 - __clz(live);
+                        umma::gemm_kk_lead<CH, gtc::ST_ROWS, gtc::KD>(lead, tbase + gtc::TM_R + lo * gtc::VS, aQd, aSt + lo * gtc::LV_BYTES,
+                                                                 umma::idesc_bf16(128, gtc::VS * (hi - lo + 1), false, false), false);
+                        umma::commit_lead(lead, barR);
+                    }
+                }
+                if (ok) umma::commit_lead(lead, &empty[st]);
+                STAMP();
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
-        if (lane == 0 && ok) {
+        if (ok) {
             // every product has completed before tensor memory is released
             const int last = NT - 1;
             umma::mbar_wait(&empty[last & 1], (last >> 1) & 1, abort_flag);
@@ -521,6 +522,7 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_bwd_tc_kernel(const
         umma::fence_after_sync();
         const uint32_t tbase = *tmem_slot;
         const uint32_t aE = umma::smem_addr(sE);
+        const uint32_t lead = umma::elect_one();
         bool ok = true;
         for (int it = 0; it < NT - 1 && ok; ++it) {
             const int c = NT - 1 - it, st = it & 1;
@@ -530,36 +532,33 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_bwd_tc_kernel(const
             const bool trans = (c + 1 < NT);
             const uint32_t written = trans ? ((uint32_t)(c + 1) & lev_mask) : 0u;   // levels that hold a state after this chunk
             const int jc = __ffs(~c) - 1;
-            if (lane == 0) {
-                ok = umma::mbar_wait(&full[st], (it >> 1) & 1, abort_flag);
-                if (ok && it > 0) ok = umma::mbar_wait(barS, (it - 1) & 1, abort_flag);
-                if (ok) ok = umma::mbar_wait(&barD[st], (it >> 1) & 1, abort_flag);
-                if (ok) {
-                    umma::fence_after_sync();
-                    // master += Wd^T E_lv for every level written by this chunk: ONE chain from the carry level (whose
-                    // result is shared by all levels below it) to the highest such level
-                    if (written) {
-                        const int hi = 31 - __clz(written);
-                        umma::gemm_mk<gtc::KD, gtc::ST_ROWS, gtc::KD>(tbase + jc * gtc::VS, aWk, aE + jc * gtc::LV_BYTES,
-                                                                      umma::idesc_bf16(128, gtc::VS * (hi - jc + 1), true, false), true);
-                    }
-                    // qd^T (lambda_lv * do): below the carry into fresh slots (those levels held no state after this chunk),
-                    // above it onto the masters
-                    const uint32_t above = readers & ~((2u << jc) - 1u);
-                    if (jc > 0)
-                        umma::gemm_mk<CH, gtc::ST_ROWS, CH>(tbase, aQd, aDL, umma::idesc_bf16(128, gtc::VS * jc, true, false), false);
-                    if (above) {
-                        const int lo = __ffs(above) - 1, hi = 31 - __clz(above);
-                        umma::gemm_mk<CH, gtc::ST_ROWS, CH>(tbase + lo * gtc::VS, aQd, aDL + lo * gtc::LV_BYTES,
-                                                            umma::idesc_bf16(128, gtc::VS * (hi - lo + 1), true, false), trans);
-                    }
-                    umma::commit(barT);
-                    umma::commit(&empty[st]);
+            ok = umma::mbar_wait_warp(&full[st], (it >> 1) & 1, abort_flag);
+            if (ok && it > 0) ok = umma::mbar_wait_warp(barS, (it - 1) & 1, abort_flag);
+            if (ok) ok = umma::mbar_wait_warp(&barD[st], (it >> 1) & 1, abort_flag);
+            if (ok) {
+                umma::fence_after_sync();
+                // master += Wd^T E_lv for every level written by this chunk: ONE chain from the carry level (whose
+                // result is shared by all levels below it) to the highest such level
+                if (written) {
+                    const int hi = 31 - __clz(written);
+                    umma::gemm_mk_lead<gtc::KD, gtc::ST_ROWS, gtc::KD>(lead, tbase + jc * gtc::VS, aWk, aE + jc * gtc::LV_BYTES,
+                                                                  umma::idesc_bf16(128, gtc::VS * (hi - jc + 1), true, false), true);
                 }
+                // qd^T (lambda_lv * do): below the carry into fresh slots (those levels held no state after this chunk),
+                // above it onto the masters
+                const uint32_t above = readers & ~((2u << jc) - 1u);
+                if (jc > 0)
+                    umma::gemm_mk_lead<CH, gtc::ST_ROWS, CH>(lead, tbase, aQd, aDL, umma::idesc_bf16(128, gtc::VS * jc, true, false), false);
+                if (above) {
+                    const int lo = __ffs(above) - 1, hi = 31 - __clz(above);
+                    umma::gemm_mk_lead<CH, gtc::ST_ROWS, CH>(lead, tbase + lo * gtc::VS, aQd, aDL + lo * gtc::LV_BYTES,
+                                                        umma::idesc_bf16(128, gtc::VS * (hi - lo + 1), true, false), trans);
+                }
+                umma::commit_lead(lead, barT);
+                umma::commit_lead(lead, &empty[st]);
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
-        if (lane == 0 && ok && NT > 1) umma::mbar_wait(&empty[(NT - 2) & 1], ((NT - 2) >> 1) & 1, abort_flag);
+        if (ok && NT > 1) umma::mbar_wait_warp(&empty[(NT - 2) & 1], ((NT - 2) >> 1) & 1, abort_flag);
         __syncwarp();
         if (*abort_flag && lane == 0) atomicExch(p.err, 1);
         umma::fence_before_sync();

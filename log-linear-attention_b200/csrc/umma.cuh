@@ -194,6 +194,16 @@ __device__ __forceinline__ void gemm_km_lead(uint32_t lead, uint32_t d_tmem, uin
 }
 
 template <int A_ROWS, int B_ROWS, int KRED>
+__device__ __forceinline__ void gemm_mk_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_saddr, uint32_t b_saddr, uint32_t idesc, bool accumulate) {
+    const uint32_t da = desc_lo_mnmajor(a_saddr, A_ROWS * ROW_BYTES), db = desc_lo_kmajor(b_saddr);
+#pragma unroll
+    for (int kk = 0; kk < KRED; kk += 16) {
+        const uint32_t kb = (kk >> 6) * B_ROWS * ROW_BYTES + (kk & 63) * 2;
+        mma_ss_lead(lead, d_tmem, da + ((kk * ROW_BYTES) >> 4), db + (kb >> 4), idesc, accumulate || kk > 0);
+    }
+}
+
+template <int A_ROWS, int B_ROWS, int KRED>
 __device__ __forceinline__ void gemm_mm_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_saddr, uint32_t b_saddr, uint32_t idesc, bool accumulate) {
     const uint32_t da = desc_lo_mnmajor(a_saddr, A_ROWS * ROW_BYTES), db = desc_lo_mnmajor(b_saddr, B_ROWS * ROW_BYTES);
 #pragma unroll
@@ -245,6 +255,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
         if (done) return true;
     }
     return false;
+}
+// the same by all lanes of a converged warp: they leave with one answer
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort)) != 0;
 }
 // bounded wait for warps that have nothing else to do until the phase completes: sleeps between polls so that the
 // polling does not compete with the tensor core's operand fetch from shared memory

@@ -1,4 +1,4 @@
-"""The output kernel's CTAs take a pair of chunks and up to eight heads of a q / k group: group sizes that leave a part of a CTA's heads over, one head a
+"""The CTAs of the output and gradient kernels take a pair of chunks and up to eight heads of a q / k group: group sizes that leave a part of a CTA's heads over, one head a
 group, the most lambda levels that it stages, pairs that read no, one and several levels, and what only a layer asks of it."""
 import pytest
 import torch
@@ -21,6 +21,23 @@ def test_heads_and_levels_of_a_cta_match_oracle(B, T, H, N, G, L):
     q, k, v, g, l, do = rounded_inputs(B, T, H, 64, N, G, L, seed=T + 7 * H)
     o, _ = run_cuda(q, k, v, g, l, do)
     assert_close(o, orc.mamba2_chunkwise(q, k, v, g, l), "o")
+
+
+@pytest.mark.parametrize("B,T,H,N,G,L", [
+    (1, 128, 5, 128, 1, 8),        # a single pair: neither states nor readers
+    (2, 256, 3, 64, 1, 9),         # two pairs of one segment, N = 64
+    (1, 512, 9, 128, 1, 20),       # four pairs of one segment, a ninth head on its own, spare lambda levels
+    (1, 640, 9, 128, 1, 11),       # two segments, the last of one pair
+    (2, 1024, 6, 64, 6, 12),       # one head a group
+    (2, 704, 10, 128, 2, 20),      # a last half pair, the most lambda levels
+    (1, 8832, 1, 128, 1, 15),      # eighteen segments: readers of a fifth high level, for which a second CTA is there
+])
+def test_gradients_of_a_cta_match_oracle(B, T, H, N, G, L):
+    q, k, v, g, l, do = rounded_inputs(B, T, H, 64, N, G, L, seed=T + 5 * H)
+    _, grads = run_cuda(q, k, v, g, l, do)
+    _, want = orc.mamba2_grads(q, k, v, g, l, do, fn=orc.mamba2_chunkwise_blocked if T > 4096 else orc.mamba2_chunkwise)
+    for got, ref, key in zip(grads, want, ("dq", "dk", "dv", "dg", "dl")):
+        assert_close(got, ref, key)
 
 
 @pytest.mark.parametrize("params", [torch.float32, torch.bfloat16])
