@@ -18,8 +18,11 @@
 // of levels) (an instruction costs the same for N = 32 as for N = 128; slots of levels inside the range that are
 // not live receive products of stale copies and are never read).  The issuing warp stays converged and predicates
 // the instructions on an elected lane: the 20 instructions of a chunk are on its chain, and inside a branch of one
-// lane they took twice as long to issue (B = 4, T = 8192, H = 16, forward that keeps its states: 778 -> 747 us; 13 chunks of a prompt,
-// 16 heads: 30.3 -> 29.1; the reverse scan, whose products wait for their operands, is as it was, 725).
+// lane they took longer (B = 4, T = 8192, H = 16, forward that keeps its states: 778 -> 747 us).  What need not wait for
+// the copies or delay them is off the chain as well: the products that only add a chunk's writes run while the copies
+// are being written, masters are read and packed before the wait for the reader products, and the tiles kept for the
+// backward leave behind the copies (747 -> 727 us, reverse scan 726 -> 694; six heads of 33 chunks, V = 256: 78 -> 69 and
+// 70 -> 66; 13 chunks of a prompt, 16 heads: 29.1 -> 27.9.  Those stores before the copies: 775 us).
 #include "tc_common.cuh"
 #include "llattn_gdn.h"
 
@@ -176,16 +179,23 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
 #endif
             STAMP();
             ok = umma::mbar_wait_warp(&full[st], (c >> 1) & 1, abort_flag);
-            if (ok && c > 0) ok = umma::mbar_wait_warp(barS, (c - 1) & 1, abort_flag);
             STAMP();
             if (ok && trans) ok = umma::mbar_wait_warp(&barU[st], (c >> 1) & 1, abort_flag);
+            // the level that receives this chunk's writes starts from kd^T u (its slot held a dead level).  Nothing of the last chunk
+            // looks at that slot if c is odd (c - 1 is even: no carry was merged), so that the product runs while the copies are being written
+            const bool early = trans && (c & 1);
+            if (ok && early) {
+                umma::fence_after_sync();
+                umma::gemm_mk_lead<CH, gtc::VS, CH>(lead, tbase + gtc::TM_M + jc * gtc::VS, aKd, aUT, ID_MK32, false);
+            }
+            if (ok && c > 0) ok = umma::mbar_wait_warp(barS, (c - 1) & 1, abort_flag);
+            STAMP();
             if (ok) {
                 umma::fence_after_sync();
                 if (trans) {
-                    // the level that receives this chunk's writes starts from kd^T u (its slot held a dead level); the
-                    // levels below the carry (all live; the element-wise warps add them into that level afterwards) and the
+                    if (!early) umma::gemm_mk_lead<CH, gtc::VS, CH>(lead, tbase + gtc::TM_M + jc * gtc::VS, aKd, aUT, ID_MK32, false);
+                    // the levels below the carry (all live; the element-wise warps add them into that level afterwards) and the
                     // live levels above it advance in place: master += Wd H_lv
-                    umma::gemm_mk_lead<CH, gtc::VS, CH>(lead, tbase + gtc::TM_M + jc * gtc::VS, aKd, aUT, ID_MK32, false);
                     if (jc > 0)
                         umma::gemm_kk_lead<gtc::KD, gtc::ST_ROWS, gtc::KD>(lead, tbase + gtc::TM_M, aWk, aSt, umma::idesc_bf16(128, gtc::VS * jc, false, false), true);
                     const uint32_t above = live & ~((2u << jc) - 1u);
@@ -322,15 +332,9 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
         }
         st_global_32B(p.o + token_row(c) * p.V + col0, w);
     };
-    // bf16 copy of one level's master for the next chunk (and, with SAVE, for the backward)
-    auto publish_level = [&](int lv, const float (&v)[16], int c_next) {
-        uint32_t mine[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) mine[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
-        if (SAVE) {
-            st_global_32B(p.hs + pair_tile(c_next, lv) + (size_t)row * 64 + (vs & 1) * gtc::VS + ch * 16, mine);
-        }
-        ts_state.store(aSt + lv * gtc::LV_BYTES, mine);
+    // with SAVE, one level's master in bf16 for the backward
+    auto keep_level = [&](int lv, const uint32_t (&mine)[8], int c_next) {
+        if (SAVE) st_global_32B(p.hs + pair_tile(c_next, lv) + (size_t)row * 64 + (vs & 1) * gtc::VS + ch * 16, mine);
     };
 
     for (int c = 0; c < NT; ++c) {
@@ -395,34 +399,49 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_tc_kernel(const __g
             umma::tmem_wait_st();
         }
         STAMP();
-        // the reader products of this chunk (issued behind the transition products) still read the bf16 copies:
-        // they must be complete before the copies are replaced
-        if (OUT && live) {
-            const bool ok = umma::mbar_wait(barR, phR, abort_flag);
-            phR ^= 1;
-            if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
-            umma::fence_after_sync();
-        }
-        STAMP();
-        {
-            uint32_t m = (uint32_t)(c + 1) & lev_mask;               // the carry level and the live levels above it
+        // the carry level and the live levels above it, two at a time
+        uint32_t m = (uint32_t)(c + 1) & lev_mask;
+        bool readers_done = !(OUT && live), two = false;
+        int l0 = 0, l1 = 0;
+        uint32_t m0[8], m1[8];
 #pragma unroll 1
-            while (m) {
-                const int l0 = __ffs(m) - 1;
-                m &= m - 1;
-                const bool two = (m != 0);
-                const int l1 = two ? __ffs(m) - 1 : l0;
-                m &= m - 1;
-                float v0[16], v1[16];
-                umma::tmem_ld16x2(tM + l0 * gtc::VS, v0, tM + l1 * gtc::VS, v1);
-                publish_level(l0, v0, c + 1);
-                if (two) publish_level(l1, v1, c + 1);
+        while (m) {
+            l0 = __ffs(m) - 1;
+            m &= m - 1;
+            two = (m != 0);
+            l1 = two ? __ffs(m) - 1 : l0;
+            m &= m - 1;
+            float v0[16], v1[16];
+            umma::tmem_ld16x2(tM + l0 * gtc::VS, v0, tM + l1 * gtc::VS, v1);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                m0[j] = pack_bf16(v0[2 * j], v0[2 * j + 1]);
+                m1[j] = pack_bf16(v1[2 * j], v1[2 * j + 1]);
+            }
+            // the reader products of this chunk (issued behind the transition products) still read the bf16 copies:
+            // they must be complete before the copies are replaced
+            if (!readers_done) {
+                const bool ok = umma::mbar_wait(barR, phR, abort_flag);
+                phR ^= 1;
+                if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
+                umma::fence_after_sync();
+                readers_done = true;
+                STAMP();
+            }
+            ts_state.store(aSt + l0 * gtc::LV_BYTES, m0);
+            if (two) ts_state.store(aSt + l1 * gtc::LV_BYTES, m1);
+            if (m) {
+                keep_level(l0, m0, c + 1);
+                keep_level(l1, m1, c + 1);
             }
         }
+        if (!alive) break;
         STAMP();
         umma::fence_async_smem();
         umma::fence_before_sync();
         mbar_arrive(barS);
+        keep_level(l0, m0, c + 1);               // off the chain
+        if (two) keep_level(l1, m1, c + 1);
         STAMP();
     }
     if (OUT && qrow && alive) {
@@ -533,8 +552,14 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_bwd_tc_kernel(const
             const uint32_t written = trans ? ((uint32_t)(c + 1) & lev_mask) : 0u;   // levels that hold a state after this chunk
             const int jc = __ffs(~c) - 1;
             ok = umma::mbar_wait_warp(&full[st], (it >> 1) & 1, abort_flag);
-            if (ok && it > 0) ok = umma::mbar_wait_warp(barS, (it - 1) & 1, abort_flag);
             if (ok) ok = umma::mbar_wait_warp(&barD[st], (it >> 1) & 1, abort_flag);
+            // qd^T (lambda_lv * do) below the carry goes into fresh slots: those levels held no state after this chunk, and the last
+            // iteration's chunk c + 1 is even, so that it spread no carry over them; it runs while the copies are being written
+            if (ok && jc > 0) {
+                umma::fence_after_sync();
+                umma::gemm_mk_lead<CH, gtc::ST_ROWS, CH>(lead, tbase, aQd, aDL, umma::idesc_bf16(128, gtc::VS * jc, true, false), false);
+            }
+            if (ok && it > 0) ok = umma::mbar_wait_warp(barS, (it - 1) & 1, abort_flag);
             if (ok) {
                 umma::fence_after_sync();
                 // master += Wd^T E_lv for every level written by this chunk: ONE chain from the carry level (whose
@@ -544,11 +569,8 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_bwd_tc_kernel(const
                     umma::gemm_mk_lead<gtc::KD, gtc::ST_ROWS, gtc::KD>(lead, tbase + jc * gtc::VS, aWk, aE + jc * gtc::LV_BYTES,
                                                                   umma::idesc_bf16(128, gtc::VS * (hi - jc + 1), true, false), true);
                 }
-                // qd^T (lambda_lv * do): below the carry into fresh slots (those levels held no state after this chunk),
-                // above it onto the masters
+                // qd^T (lambda_lv * do) above the carry: onto the masters
                 const uint32_t above = readers & ~((2u << jc) - 1u);
-                if (jc > 0)
-                    umma::gemm_mk_lead<CH, gtc::ST_ROWS, CH>(lead, tbase, aQd, aDL, umma::idesc_bf16(128, gtc::VS * jc, true, false), false);
                 if (above) {
                     const int lo = __ffs(above) - 1, hi = 31 - __clz(above);
                     umma::gemm_mk_lead<CH, gtc::ST_ROWS, CH>(lead, tbase + lo * gtc::VS, aQd, aDL + lo * gtc::LV_BYTES,
@@ -660,26 +682,40 @@ __global__ void __launch_bounds__(gtc::NTHREADS, 1) gdn_scan_bwd_tc_kernel(const
             }
             umma::tmem_wait_st();
         }
-        {
-            // adjoints of the states that chunk c reads = of the states written by chunk c - 1: bf16 copies for the next
-            // iteration and, in the [K][32] layout, for the chunk-parallel gradient kernel
-            uint32_t m = (uint32_t)c & lev_mask;
+        // adjoints of the states that chunk c reads = of the states written by chunk c - 1: bf16 copies for the next
+        // iteration, two levels at a time, and, in the [K][32] layout, for the chunk-parallel gradient kernel
+        auto keep_level = [&](int lv, const uint32_t (&mine)[8]) {
+            st_global_32B(p.dhs + pair_tile(c - 1, lv) + (size_t)row * 64 + (vs & 1) * gtc::VS + ch * 16, mine);
+        };
+        bool two = false;
+        int l0 = 0, l1 = 0;
+        uint32_t m0[8], m1[8];
 #pragma unroll 1
-            while (m) {
-                const int lv = __ffs(m) - 1;
-                m &= m - 1;
-                float v[16];
-                umma::tmem_ld16(tM + lv * gtc::VS, v);
-                uint32_t mine[8];
+        for (uint32_t m = (uint32_t)c & lev_mask; m;) {      // (at least one level: c >= 1)
+            l0 = __ffs(m) - 1;
+            m &= m - 1;
+            two = (m != 0);
+            l1 = two ? __ffs(m) - 1 : l0;
+            m &= m - 1;
+            float v0[16], v1[16];
+            umma::tmem_ld16x2(tM + l0 * gtc::VS, v0, tM + l1 * gtc::VS, v1);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) mine[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
-                st_global_32B(p.dhs + pair_tile(c - 1, lv) + (size_t)row * 64 + (vs & 1) * gtc::VS + ch * 16, mine);
-                ts_state.store(aE + lv * gtc::LV_BYTES, mine);
+            for (int j = 0; j < 8; ++j) {
+                m0[j] = pack_bf16(v0[2 * j], v0[2 * j + 1]);
+                m1[j] = pack_bf16(v1[2 * j], v1[2 * j + 1]);
+            }
+            ts_state.store(aE + l0 * gtc::LV_BYTES, m0);
+            if (two) ts_state.store(aE + l1 * gtc::LV_BYTES, m1);
+            if (m) {
+                keep_level(l0, m0);
+                keep_level(l1, m1);
             }
         }
         umma::fence_async_smem();
         umma::fence_before_sync();
         mbar_arrive(barS);
+        keep_level(l0, m0);                                  // the last ones off the chain
+        if (two) keep_level(l1, m1);
     }
     umma::fence_before_sync();
     bar_work();
