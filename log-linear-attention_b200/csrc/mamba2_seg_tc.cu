@@ -412,6 +412,8 @@ __global__ void __launch_bounds__(tca::NTHREADS, 2) m2_adjoint_tc_kernel(const _
             const float glp = sGs[pl * tc::PT + tc::PT - 1];
             if (pl > 0) {
                 const float e = fexp(sGs[pl * tc::PT + row]);
+                // (a pair that nobody reads has not waited for its own products: two completions later their parity would say that they never were)
+                for (; seen < nr; ++seen) umma::mbar_wait(r_full, seen & 1, abort_flag);
                 umma::mbar_wait(full, s & 1, abort_flag);
                 ++s;
                 uint4 dox[4];
@@ -434,7 +436,6 @@ __global__ void __launch_bounds__(tca::NTHREADS, 2) m2_adjoint_tc_kernel(const _
                 if (pl >= 2) {
                     if (pl == 2 && npairs == 4) {
                         // what pair 3 sent back has decayed over pair 2, which adds to it
-                        for (; seen < nr; ++seen) umma::mbar_wait(r_full, seen & 1, abort_flag);
                         umma::fence_after_sync();
                         const float dec = fexp(glp);
 #pragma unroll

@@ -30,6 +30,9 @@ def test_heads_and_levels_of_a_cta_match_oracle(B, T, H, N, G, L):
     (1, 640, 9, 128, 1, 11),       # two segments, the last of one pair
     (2, 1024, 6, 64, 6, 12),       # one head a group
     (2, 704, 10, 128, 2, 20),      # a last half pair, the most lambda levels
+    (1, 384, 3, 128, 1, 10),       # three pairs, the last of which nobody reads
+    (2, 896, 32, 128, 1, 11),      # the same in a second segment, enough of them for either order of completion
+    (1, 1344, 4, 64, 2, 12),       # ... and the last pair a half
     (1, 8832, 1, 128, 1, 15),      # eighteen segments: readers of a fifth high level, for which a second CTA is there
 ])
 def test_gradients_of_a_cta_match_oracle(B, T, H, N, G, L):
