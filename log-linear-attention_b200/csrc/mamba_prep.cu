@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(256, 6) m2_prep_fwd_kernel(const __grid_consta
         const int per = (a.tokens + a.lam_runs - 1) / a.lam_runs, t0 = blockIdx.x / a.lam_blocks * per, t1 = min(a.tokens, t0 + per);
         const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, a.lp_f32, a.H * a.L, a.mode};
         const int block = blockIdx.x % a.lam_blocks;
-        if (a.lam8) lambda_part_fwd<8>(c, a.lam, t0, t1, block, a.lam_blocks);
-        else lambda_part_fwd<1>(c, a.lam, t0, t1, block, a.lam_blocks);
+        if (a.lam8) lambda_part_fwd<8, 1>(c, a.lam, t0, t1, block, a.lam_blocks);
+        else lambda_part_fwd<1, 1>(c, a.lam, t0, t1, block, a.lam_blocks);
         return;
     }
     const int at = blockIdx.x - lam_grid;
@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(256, 4) m2_prep_bwd_kernel(const __grid_consta
         const LambdaCols c{a.dl, (long)a.H * a.L, a.Lp, a.lp_f32, a.H * a.L, a.mode};
         __shared__ float sums[256 * 8];
         const int block = blockIdx.x % a.lam_blocks;
-        if (a.lam8) lambda_part_bwd<8>(c, a.dlam, a.ddl, c.dl_stride, a.dLp, t0, t1, block, a.lam_blocks, sums);
-        else lambda_part_bwd<1>(c, a.dlam, a.ddl, c.dl_stride, a.dLp, t0, t1, block, a.lam_blocks, sums);
+        if (a.lam8) lambda_part_bwd<8, 2>(c, a.dlam, a.ddl, c.dl_stride, a.dLp, t0, t1, block, a.lam_blocks, sums);
+        else lambda_part_bwd<1, 4>(c, a.dlam, a.ddl, c.dl_stride, a.dLp, t0, t1, block, a.lam_blocks, sums);
         return;
     }
     const int at = blockIdx.x - lam_grid;
@@ -211,7 +211,7 @@ static unsigned prep_grid(llattn::PrepArgs& a, long rows, int H, int P, int L, i
     while (a.run > (backward ? 8 : 4) && (long)a.row_blocks * ((a.tokens + a.run - 1) / a.run) * threads < 148 * 8 * 256) a.run /= 2;
     // forward: eight tokens a thread
     const int groups = H * L / (a.lam8 ? 8 : 1), per = groups < threads ? threads / groups : 1;
-    a.lam_runs = backward ? llattn::lambda_runs(a.tokens, a.lam_blocks) : (a.tokens + 8 * per - 1) / (8 * per);
+    a.lam_runs = backward ? llattn::lambda_runs(a.tokens, a.lam_blocks, a.lam8) : (a.tokens + 8 * per - 1) / (8 * per);
     return (unsigned)(a.row_blocks * ((a.tokens + a.run - 1) / a.run) + a.lam_blocks * a.lam_runs);
 }
 

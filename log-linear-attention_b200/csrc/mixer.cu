@@ -55,8 +55,8 @@ __global__ void __launch_bounds__(128, 6) mixer_prep_kernel(const __grid_constan
         const LambdaCols c{rows + a.H, a.W, a.Lp, a.lp_f32, a.H * a.L, a.mode};
         const int block = blockIdx.x % a.lam_blocks;
         bf16* lam = a.lam + (long)b * a.T * a.H * a.L;
-        if (a.lam8) lambda_part_fwd<8>(c, lam, t0, t1, block, a.lam_blocks);
-        else lambda_part_fwd<1>(c, lam, t0, t1, block, a.lam_blocks);
+        if (a.lam8) lambda_part_fwd<8, 2>(c, lam, t0, t1, block, a.lam_blocks);
+        else lambda_part_fwd<1, 2>(c, lam, t0, t1, block, a.lam_blocks);
         return;
     }
     const int nrun = (a.T + a.run - 1) / a.run, at = (blockIdx.x - lam_grid) / a.conv_blocks;
@@ -141,8 +141,8 @@ __global__ void __launch_bounds__(128, 4) mixer_prep_bwd_kernel(const __grid_con
         const LambdaCols c{a.zx + off, a.W, a.Lp, a.lp_f32, a.H * a.L, a.mode};
         const int block = blockIdx.x % a.lam_blocks;
         const float* dlam = a.dlam + row0 * a.H * a.L;
-        if (a.lam8) lambda_part_bwd<8>(c, dlam, a.dzx + off, a.W, a.dLp, t0, t1, block, a.lam_blocks, sums);
-        else lambda_part_bwd<1>(c, dlam, a.dzx + off, a.W, a.dLp, t0, t1, block, a.lam_blocks, sums);
+        if (a.lam8) lambda_part_bwd<8, 2>(c, dlam, a.dzx + off, a.W, a.dLp, t0, t1, block, a.lam_blocks, sums);
+        else lambda_part_bwd<1, 4>(c, dlam, a.dzx + off, a.W, a.dLp, t0, t1, block, a.lam_blocks, sums);
         return;
     }
     const int nrun = (a.T + a.run - 1) / a.run, at = (blockIdx.x - lam_grid) / a.conv_blocks;
@@ -441,10 +441,10 @@ static int mixer_check(int B, int T, int H, int G, int N, int L, int mode) {
     return 0;
 }
 
-// tokens a thread walks: long enough that the halo and the final sums are cheap, short enough to fill the chip
-static int mixer_run(int B, int T, int warps_per_run, int lo, int hi) {
+// tokens a thread walks: long enough that the halo and the final sums are cheap, short enough to give the chip `warps` of them
+static int mixer_run(int B, int T, int warps_per_run, int lo, int hi, long warps) {
     int run = hi;
-    while (run > lo && (long)B * ((T + run - 1) / run) * warps_per_run < 148 * 20) run /= 2;
+    while (run > lo && (long)B * ((T + run - 1) / run) * warps_per_run < warps) run /= 2;
     return run;
 }
 
@@ -453,7 +453,7 @@ static void mixer_lambda_blocks(llattn::MixerArgs& a, bool backward) {
     a.lam_blocks = (a.H * a.L / (a.lam8 ? 8 : 1) + 127) / 128;
     // forward: eight tokens a thread
     const int groups = a.H * a.L / (a.lam8 ? 8 : 1), rows = groups < 128 ? 128 / groups : 1;
-    a.lam_runs = backward ? llattn::lambda_runs(a.T, a.lam_blocks * a.B) : (a.T + 8 * rows - 1) / (8 * rows);
+    a.lam_runs = backward ? llattn::lambda_runs(a.T, a.lam_blocks * a.B, a.lam8) : (a.T + 8 * rows - 1) / (8 * rows);
 }
 
 int llattn_mixer_prep_fwd(const void* zx, const void* conv_w, int conv_w_f32, const void* conv_b, int conv_b_f32, const void* dt_bias,
@@ -471,7 +471,7 @@ int llattn_mixer_prep_fwd(const void* zx, const void* conv_w, int conv_w_f32, co
     a.B = B; a.T = T; a.H = H; a.L = L; a.dim = H * llattn::MX_P; a.gn = G * N; a.W = 2 * a.dim + 2 * a.gn + H + H * L; a.mode = lambda_mode;
     const int ch = a.dim + 2 * a.gn;
     a.conv_blocks = (ch / 4 + 127) / 128;
-    a.run = mixer_run(B, T, ch / 128 + 1, 16, 64);
+    a.run = mixer_run(B, T, ch / 128 + 1, 16, 64, 148 * 20);
     mixer_lambda_blocks(a, false);
     const unsigned grid = (unsigned)(a.conv_blocks * B * ((T + a.run - 1) / a.run) + a.lam_blocks * B * a.lam_runs);
     llattn::launch_chained(llattn::mixer_prep_kernel, grid, 128, 0, (cudaStream_t)stream, a);
@@ -497,7 +497,9 @@ int llattn_mixer_prep_bwd(const void* zx, const void* conv_w, int conv_w_f32, co
     a.B = B; a.T = T; a.H = H; a.L = L; a.dim = H * llattn::MX_P; a.gn = G * N; a.W = 2 * a.dim + 2 * a.gn + H + H * L; a.mode = lambda_mode;
     const int ch = a.dim + 2 * a.gn;
     a.conv_blocks = (ch / 4 + 127) / 128;
-    a.run = mixer_run(B, T, ch / 128 + 1, 16, 128);
+    // short runs end in step with the lambda part: walks of up to 128 tokens for 20 warps an SM took (us, before / now) 149 / 131 at B = 1, T = 8192, 48 heads, 90 / 82 at B = 2,
+    // T = 4096, 24 heads, 261 / 235 at B = 2, T = 8192, 48 heads, 48 / 44 at T = 2048 (with the lambda part's runs halved as well)
+    a.run = mixer_run(B, T, ch / 128 + 1, 16, 32, 148 * 10);
     mixer_lambda_blocks(a, true);
     const unsigned grid = (unsigned)(a.conv_blocks * B * ((T + a.run - 1) / a.run) + a.lam_blocks * B * a.lam_runs);
     llattn::launch_chained(llattn::mixer_prep_bwd_kernel, grid, 128, 0, (cudaStream_t)stream, a);

@@ -107,7 +107,7 @@ __device__ __forceinline__ void red_add_f32x4(float* addr, float a, float b, flo
 
 // The lambda part of a pass: lambda (or the gradients of dl and Lp) of the (head, level) columns of tokens t0 .. t1 - 1 by one CTA.  A
 // thread owns VL neighbouring columns (VL = 8: 16 bytes of dl a load; VL = 1 where the columns do not come in eights) and every
-// (blockDim / columns)-th token.  Row strides are in elements; the pointers are those of the tensors' first token.
+// (blockDim / columns)-th token, UT of them at a time: their loads are issued before the first of their stores.  Row strides are in elements; the pointers are those of the tensors' first token.
 struct LambdaCols {
     const bf16* dl;
     long dl_stride;
@@ -116,21 +116,33 @@ struct LambdaCols {
 };
 
 // Runs of tokens of the lambda part in a backward pass: its sums go to the few addresses of L, so there are only as many runs as fill the chip (at B = 2,
-// T = 16384, 32 heads the backward pass took 214 us with the 2048 runs of its other part, 104 us without its lambda part)
-inline int lambda_runs(int tokens, int blocks) {
-    const int most = blocks >= 296 ? 1 : 296 / blocks, runs = (tokens + 15) / 16;
+// T = 16384, 32 heads the backward pass took 214 us with the 2048 runs of its other part, 104 us without its lambda part).  One CTA per SM: they come
+// first and hold back the other part (that pass with 296 / 148 / 100 / 74 CTAs 128 / 119 / 120 / 124 us, T = 4096 alone 39 / 29 / 25 / 21, B = 4, T = 8192,
+// 16 heads 81 / 79 / 91 / 110); two where a thread has one column (B = 8, T = 2048, 10 heads, L = 15: 75 us, with one 91).
+inline int lambda_runs(int tokens, int blocks, bool eights) {
+    const int ctas = eights ? 148 : 296, most = blocks >= ctas ? 1 : ctas / blocks, runs = (tokens + 15) / 16;
     return runs < most ? runs : most;
 }
 
+// the columns of a token, as they are in memory
 template <int VL>
-__device__ __forceinline__ void load_cols(float (&f)[VL], const bf16* p) {
+struct LambdaRow {
+    Packed<8> w;
+    bf16 one;
+    __device__ __forceinline__ void load(const bf16* p) {
+        if (VL == 8) w.load(p, true);
+        else one = p[0];
+    }
+    __device__ __forceinline__ float operator[](int i) const { return VL == 8 ? w[i] : __bfloat162float(one); }
+};
+template <int VL>
+__device__ __forceinline__ void load_cols(float (&f)[VL], const float* p) {
     if (VL == 8) {
-        Packed<8> r;
-        r.load(p, true);
-#pragma unroll
-        for (int i = 0; i < VL; ++i) f[i] = r[i];
+        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+        f[0] = a.x; f[VL / 8] = a.y; f[VL / 4] = a.z; f[VL * 3 / 8] = a.w;
+        f[VL / 2] = b.x; f[VL * 5 / 8] = b.y; f[VL * 3 / 4] = b.z; f[VL * 7 / 8] = b.w;
     } else {
-        f[0] = __bfloat162float(p[0]);
+        f[0] = p[0];
     }
 }
 template <int VL>
@@ -139,7 +151,7 @@ __device__ __forceinline__ void store_cols(bf16* p, const float (&f)[VL]) {
     else p[0] = __float2bfloat16(f[0]);
 }
 
-template <int VL>
+template <int VL, int UT>
 __device__ __forceinline__ void lambda_part_fwd(const LambdaCols& c, bf16* lam, int t0, int t1, int block, int nblocks) {
     const int groups = c.n / VL;                               // threads of a token
     const int per = min(groups, (int)blockDim.x), rows = blockDim.x / per;
@@ -152,18 +164,23 @@ __device__ __forceinline__ void lambda_part_fwd(const LambdaCols& c, bf16* lam, 
             lp[i] = load_param(c.Lp, e + i, c.lp_f32);
             elp[i] = __expf(lp[i]);
         }
-#pragma unroll 2
-        for (int t = t0 + r; t < t1; t += rows) {
-            float d[VL];
-            load_cols<VL>(d, c.dl + t * c.dl_stride + e);
+        for (int t = t0 + r; t < t1; t += UT * rows) {
+            LambdaRow<VL> in[UT];
 #pragma unroll
-            for (int i = 0; i < VL; ++i) d[i] = lambda_value(c.mode, lp[i], elp[i], d[i]);
-            store_cols<VL>(lam + (long)t * c.n + e, d);
+            for (int u = 0; u < UT; ++u) in[u].load(c.dl + min(t + u * rows, t1 - 1) * c.dl_stride + e);
+#pragma unroll
+            for (int u = 0; u < UT; ++u) {
+                if (t + u * rows >= t1) break;
+                float d[VL];
+#pragma unroll
+                for (int i = 0; i < VL; ++i) d[i] = lambda_value(c.mode, lp[i], elp[i], in[u][i]);
+                store_cols<VL>(lam + (long)(t + u * rows) * c.n + e, d);
+            }
         }
     }
 }
 
-template <int VL>
+template <int VL, int UT>
 __device__ __forceinline__ void lambda_part_bwd(const LambdaCols& c, const float* dlam, bf16* ddl, long ddl_stride, float* dLp, int t0, int t1,
                                                 int block, int nblocks, float* sums) {
     // sums: blockDim * VL floats of shared memory.  The threads that share columns add up there, so that a column costs one global
@@ -182,26 +199,27 @@ __device__ __forceinline__ void lambda_part_bwd(const LambdaCols& c, const float
             elp[i] = __expf(lp[i]);
             sum[i] = 0.f;
         }
-#pragma unroll 2
-        for (int t = act ? t0 + r : t1; t < t1; t += rows) {
-            float d[VL], gl[VL];
-            load_cols<VL>(d, c.dl + t * c.dl_stride + e);
-            const float* g = dlam + (long)t * c.n + e;
-            if (VL == 8) {
-                const float4 a = *reinterpret_cast<const float4*>(g), b = *reinterpret_cast<const float4*>(g + 4);
-                gl[0] = a.x; gl[VL / 8] = a.y; gl[VL / 4] = a.z; gl[VL * 3 / 8] = a.w;
-                gl[VL / 2] = b.x; gl[VL * 5 / 8] = b.y; gl[VL * 3 / 4] = b.z; gl[VL * 7 / 8] = b.w;
-            } else {
-                gl[0] = g[0];
+        for (int t = act ? t0 + r : t1; t < t1; t += UT * rows) {
+            LambdaRow<VL> in[UT];
+            float gl[UT][VL];
+#pragma unroll
+            for (int u = 0; u < UT; ++u) {
+                const long tt = min(t + u * rows, t1 - 1);
+                in[u].load(c.dl + tt * c.dl_stride + e);
+                load_cols<VL>(gl[u], dlam + tt * c.n + e);
             }
 #pragma unroll
-            for (int i = 0; i < VL; ++i) {
-                float gd, gp;
-                lambda_grad(c.mode, lp[i], elp[i], d[i], gl[i], gd, gp);
-                d[i] = gd;
-                sum[i] += gp;
+            for (int u = 0; u < UT; ++u) {
+                if (t + u * rows >= t1) break;
+                float d[VL];
+#pragma unroll
+                for (int i = 0; i < VL; ++i) {
+                    float gp;
+                    lambda_grad(c.mode, lp[i], elp[i], in[u][i], gl[u][i], d[i], gp);
+                    sum[i] += gp;
+                }
+                store_cols<VL>(ddl + (t + u * rows) * ddl_stride + e, d);
             }
-            store_cols<VL>(ddl + t * ddl_stride + e, d);
         }
         if (rows > 1) {
             __syncthreads();
