@@ -596,12 +596,10 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
     cudaError_t e;
     const bool use_tc = mamba2_uses_tc(p);
     if (!g_use_tensor_core_path.load()) p.lo_H = nullptr;      // (a backward call may want them where this one does not)
-    // A prompt's level states and its tail need the segment summaries only (part of the tail not even those), the output three more kernels.
-    // The states are made beside those while the chunk kernel leaves SMs idle (it takes one CTA per segment and SM): B = 1, T = 1000, 48 heads,
-    // 96 CTAs: 62 -> 57 us for the call without a tail's kernels; T = 1500, 144 CTAs: 66.9 -> 67.7, hence three quarters of the SMs (T = 1024 at 32, 48,
-    // 64 heads, beside / behind: 55.0 / 58.8, 61.7 / 65.5, 69.4 / 70.3; T = 1536 at 32, 48: 59.5 / 62.1, 72.2 / 71.0); within a segment there is too
-    // little to run beside for the events to pay.  With a tail always: its kernels are chains of latency (T = 1500 87.6 -> 74.5 us,
-    // T = 3000 139 -> 119, T = 500 44.5 -> 42, four sequences of T = 700, 32 heads 123 -> 102).
+    // A prompt's level states and its tail need the segment summaries only (part of the tail not even those).  With a tail its kernels, which are chains of
+    // latency, always run beside the output's (the call behind / beside, T = 500, 1000, 1500, 3000 at 48 heads: 73 / 56, 79 / 76, 83 / 77, 110 / 102 us; four sequences
+    // of T = 700, 32 heads 104 / 91).  The states alone do once they take longer than the two events: at 1 x 1024 x 32 and 48, 1 x 1536 x 32 (sequences, tokens, heads)
+    // 58 / 59, 60 / 62, 57 / 61; at 1 x 2048 x 48 76 / 76, 4 x 1024 x 32 98 / 93, 1 x 4096 x 48 117 / 115, 2 x 4096 x 48 195 / 190.  Hence 192 segments.
     SideStream* side = nullptr;
     const Mamba2Tail tail{p.q, p.k, p.v, p.l, p.res_x, p.g, p.res_D, p.res_D ? p.res_y : p.o, p.pr_states, p.pr_part, p.T, p.pr_n, p.H, p.G, p.pr_L, p.L,
                           p.res_f32};
@@ -625,7 +623,7 @@ static int launch_fwd(Mamba2Params p, cudaStream_t stream) {
         return (int)cudaGetLastError();
     };
     int rc;
-    if (p.pr_states && (p.pr_n > 0 || (p.NS > 1 && (long)p.B * p.H * p.NS * 4 < 148 * 3))) side = SideStream::get(stream);
+    if (p.pr_states && (p.pr_n > 0 || (p.NS > 1 && (long)p.B * p.H * p.NS >= 192))) side = SideStream::get(stream);
     if (p.pr_n > 0) {
         if (side && (e = side->fork(stream)) != cudaSuccess) return (int)e;
         rc = mamba2_tail_intra_launch(tail, p.B, p.K, side ? side->stream() : stream);
