@@ -72,7 +72,7 @@ def peaks():
 
 def measured_traffic(w):
     """DRAM read + write bytes per launch of the dominant kernel, from the counter file that the ncu recipe in
-    profiles/ writes (captured at batch 1; every CTA handles one (batch, head, segment), so traffic is
+    profiles/ writes (captured at batch 1; a CTA's work lies in one sequence, so traffic is
     proportional to the batch).  None when there is no capture for this shape."""
     path = os.path.join(ROOT, "profiles", "tc_counters_B1.json")
     if not os.path.exists(path):

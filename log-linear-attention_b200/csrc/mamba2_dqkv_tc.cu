@@ -16,6 +16,7 @@
 // What bounds them is the latency of instruction streams: the tile warps' phase between two products (about 2 k cycles a head) and the issue of products.
 // The kernels before walked the segments of one head in order with one pair in flight per SM (15 k cycles a pair, twice) and added 64 KB of fp32 gradients
 // of q or k per pair and head to global memory, three times.
+// B = 2, T = 16384, 32 heads: 323 + 232 us, 871 with the readers' and the adjoints' kernels (140 + 176), where the two walks took 895 and the high levels' kernel 316.
 #include "rowwise.cuh"
 #include "tc_common.cuh"
 

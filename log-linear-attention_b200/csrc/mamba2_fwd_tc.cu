@@ -15,8 +15,10 @@
 // None of them waits for another but through the rings.  A wait that gives up sets the CTA's abort flag, after which every other wait of the CTA ends at
 // once; warps that work in step go through the rest of their loops without waiting.
 //
-// What bounds it is the latency of instruction streams, not a unit (the tensor core is busy a fifth of the time, DRAM a third): one stream of jobs took
+// What bounds it is the latency of instruction streams, not a unit (the tensor core is busy 29 % of the time, DRAM 35 %): one stream of jobs took
 // 1.2 k cycles a job for the waits and the issue of eight instructions, hence two; the row warps' sums overlap the other team's outputs.
+// B = 2, T = 16384, 32 heads: 180 us (half of the issue slots), where a kernel that walked a segment's pairs with one in flight per SM and one for the high levels
+// took 303 + 127; B = 8, T = 4096, 24 heads: the whole forward 465 -> 261 us.
 #include "rowwise.cuh"
 #include "tc_common.cuh"
 
@@ -720,11 +722,6 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
     uint32_t phS = 0, phT = 0, phO = 0, phKV = 0;
 
     for (int pl = 0; pl < npairs; ++pl) {
-#ifdef LLATTN_STAMPS
-        int nstamp = 0;
-        const int stamp_slot = (blockIdx.x == 300 && pl == 2) ? (tid == 0 ? 0 : (tid == 200 ? 1 : (tid == 96 ? 2 : -1))) : -1;
-#endif
-        STAMP();                                     // 0: top of the pair
         const int st = pl & 1;
         const long t0 = (long)pl * tc::PT;
         const float* sGp = sTab + (pl & 1) * 384;    // tables of this pair (written while the previous pair ran)
@@ -734,10 +731,7 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
         // x rows of the pair into L2 (held in registers from here on they cost the products below more than they save)
         if (RES && ch == 0 && t0 + row < res_n)
             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.res_x + (((long)b * p.res_T + t0 + row) * p.H + h) * tc::VD));
-        STAMP();                                     // 1: small fetches issued
         umma::mbar_wait(&full_kv[st], (pl >> 1) & 1, abort_flag);      // the v tile (read below with generic loads)
-        STAMP();                                     // 2: tiles landed
-        STAMP();                                     // 3
         int nread = 0;
 #pragma unroll
         for (int lv = 0; lv < MP; ++lv) nread += (pl >> lv) & 1;
@@ -766,7 +760,6 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
                 *reinterpret_cast<uint4*>(sVs + off) = x;
             }
         }
-        STAMP();                                     // 4: Vs written
         // ---- wait for S (and the level reads); the q tile is then free for the next pair
         umma::mbar_wait(&bars[0], phS, abort_flag);
         phS ^= 1;
@@ -775,8 +768,6 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
             phT ^= 1;
         }
         umma::fence_after_sync();
-        STAMP();                                     // 5: S (and T) complete
-        STAMP();                                     // 6
         // ---- S -> P (bf16, K-major A operand of P v).  This thread: row `row`, and in every 32-column
         //      block jb <= rb the 16 columns [jb*32 + ch*16, +16)
         // blocks above the diagonal: zeros
@@ -832,7 +823,6 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
             }
             *reinterpret_cast<uint2*>(sP + umma::tile_offset(row, j0, tc::PT)) = make_uint2(pack_bf16(s[0], s[1]), pack_bf16(s[2], s[3]));
         }
-        STAMP();                                     // 7: P written
         if (warp == TABLE_WARP && pl + 1 < npairs) {
             decay_tables(pl + 1);
             if (pl + 2 < npairs) fetch_g(pl + 2);
@@ -841,7 +831,6 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
         umma::fence_before_sync();
         bar_work();                                  // barrier 2
         umma::fence_after_sync();
-        STAMP();                                     // 8: after barrier 2
 
         // ---- output row of this thread: columns ch*32 .. +31
         float o[32];
@@ -869,7 +858,6 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
                     ++slot;
                 }
         }
-        STAMP();                                     // 9: level reads accumulated
         {
             umma::mbar_wait(&bars[2], phO, abort_flag);
             phO ^= 1;
@@ -923,10 +911,8 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
                     *reinterpret_cast<uint4*>(go + (long)rr * p.H * tc::VD + c) = *reinterpret_cast<const uint4*>(sP + umma::tile_offset(rr, c, tc::PT));
             }
         }
-        STAMP();                                     // 10: output stored
         // ---- pair summary and the Fenwick carry over pair levels (thread = state row `row`)
         umma::mbar_wait(&bars[3], phKV, abort_flag);
-        STAMP();                                     // 11: pair summary complete
         phKV ^= 1;
         umma::fence_after_sync();
         if (MP > 0 && pl + 1 < npairs) {
@@ -963,12 +949,10 @@ __global__ void __launch_bounds__(tc::NTHREADS, 1) m2_one_segment_tc_kernel(cons
             }
         }
         if (pl + 1 < npairs) store_lam();            // every read of this pair's lambda is done (barrier 2)
-        STAMP();                                     // 12: states merged
         umma::fence_async_smem();
         umma::fence_before_sync();
         bar_work();                                  // barrier 3
         umma::fence_after_sync();
-        STAMP();                                     // 13: after barrier 3
         if (*abort_flag) break;                      // uniform: read after the barrier
     }
     umma::fence_before_sync();

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) mamba2_prompt_state_kernel(const bf16* __
 //
 // Two kernels, because the second sum and the levels that these tokens build need nothing of the whole chunks: mamba2_tail_intra_kernel can run
 // while their segment summaries are made, and the kernel behind the states is short.  As one kernel behind the states it shared the
-// SMs that the output's chunk kernel leaves free and outlasted it: T = 1000, 48 heads, 38 us instead of 11 and 14, 74 us for the call instead of 58.
+// SMs that the output's kernel left free and outlasted it: T = 1000, 48 heads, 38 us instead of 11 and 14, 74 us for the call instead of 58.
 // A CTA owns TL of the 64 columns of one (batch, head); what bounds both is a chain of trips to L2 and of short products.
 // Whole heads (TL = 64) do what the columns share once, sixteen columns a CTA shorten the chain of few heads: the call at 48 heads, T = 1500 74.5 us with 16 and
 // 84.5 with 64, T = 3000 119 and 136; at 128 heads, T = 700 101.7 and 95.5; at 192, T = 100 75.9 and 64.4, T = 400 100 and 90.7.  Hence 96 heads.

@@ -9,7 +9,7 @@
 namespace llattn {
 
 // Optional phase timing for tuning (build with -DLLATTN_STAMPS): three threads of one CTA record
-// clock64() at fixed points of one pair; llattn_debug_read_stamps copies the table to the host.
+// clock64() at fixed points of one pair; a function beside the kernels copies the table to the host.
 #ifdef LLATTN_STAMPS
 static __device__ long long g_stamps[3][32];
 #define STAMP()                                                             \
