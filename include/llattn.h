@@ -134,6 +134,7 @@ int llattn_mamba2_bwd_saved(const void* q, const void* k, const void* v, const f
  * kernels (everything else is as above).  The gradients of A and dt_bias are sums of dg dt over all tokens that cancel to a few per cent
  * of their terms, so their last per cents depend on where intermediate results are rounded, and these calls return the digits that they
  * always did.  Accuracy is not the reason: against fp64 the sums of the tensor-core kernels are as good or better (mamba2_bwd.cu). */
+size_t llattn_mamba2_bwd_layer_workspace_bytes(int B, int T, int H, int G, int K, int V, int L);   /* at most llattn_mamba2_bwd_workspace_bytes */
 int llattn_mamba2_bwd_layer(const void* q, const void* k, const void* v, const float* g_cum, const void* lambda,
                             const void* d_o, void* dq, void* dk, void* dv, float* dg, float* dlambda,
                             void* workspace, size_t workspace_bytes, const void* fwd_workspace, size_t fwd_workspace_bytes,

@@ -71,11 +71,12 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
         p.seg_F = c.take<float>(BH * p.NS * KV);
         p.seg_D = c.take<float>(BH * p.NS);
         p.seg_H0 = c.take<__nv_bfloat16>(BH * p.NS * p.LH * KV);
-        // a level state for every pair of chunks (K = 64 leaves half of it unused: hosts have sized this part by the value rows)
+        // a level state for every pair of chunks (K = 64 leaves half of it unused: hosts have sized this part by the value rows); with more levels than
+        // the tensor-core kernels hold nobody reads them
         __nv_bfloat16* lo = c.take<__nv_bfloat16>(BH * (p.warp_level ? p.NT : (p.NT + 1) / 2 * 2) * 64 * p.V);
-        p.lo_H = p.warp_level ? nullptr : lo;
+        p.lo_H = p.warp_level || p.L > llattn::M2_MAX_L_TC ? nullptr : lo;
     }
-    if (backward && p.NT > 2) {
+    if (backward && p.NT > 2 && llattn::mamba2_bwd_shape_uses_tc(p)) {
         const size_t NP = (p.NT + 1) / 2;
         if (p.NS == 1) p.lo_H = c.take<__nv_bfloat16>(BH * NP * KV);
         p.lo_A = c.take<__nv_bfloat16>(BH * NP * KV);
@@ -254,6 +255,14 @@ size_t llattn_mamba2_bwd_workspace_bytes(int B, int T, int H, int G, int K, int 
     return setup(p, nullptr, true);
 }
 
+size_t llattn_mamba2_bwd_layer_workspace_bytes(int B, int T, int H, int G, int K, int V, int L) {
+    if (check_shape(B, T, H, G, K, V, L) != 0) return 0;
+    llattn::Mamba2Params p = {};
+    p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
+    p.chunk_rounding = 1;
+    return setup(p, nullptr, true);
+}
+
 int llattn_mamba2_bwd(const void* q, const void* k, const void* v, const float* g_cum, const void* lambda,
                       const void* d_o, void* dq, void* dk, void* dv, float* dg, float* dlambda,
                       void* workspace, size_t workspace_bytes,
@@ -272,6 +281,7 @@ static int mamba2_bwd_impl(const void* q, const void* k, const void* v, const fl
     if (llattn::misaligned(16, {q, k, v, d_o}) || llattn::misaligned(8, {dq, dk})) return LLATTN_ERR_ALIGNMENT;
     llattn::Mamba2Params p = {};
     p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
+    p.chunk_rounding = chunk_rounding;
     const size_t need = setup(p, nullptr, true);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255)) return LLATTN_ERR_WORKSPACE;
     setup(p, workspace, true);
@@ -287,7 +297,6 @@ static int mamba2_bwd_impl(const void* q, const void* k, const void* v, const fl
         p.reuse_states = p.NS > 1;           // (one segment: the forward call kept none)
     }
     cudaStream_t st = (cudaStream_t)stream;
-    p.chunk_rounding = chunk_rounding;
     p.cum_in = g_cum;
     p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
     p.l = (const __nv_bfloat16*)lambda; p.d_o = (const __nv_bfloat16*)d_o;

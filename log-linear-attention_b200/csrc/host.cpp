@@ -24,7 +24,7 @@ using torch::autograd::Variable;
 using torch::autograd::variable_list;
 
 #define LLATTN_FUNCS(F)                                                                                                             \
-    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_fwd_residual) F(llattn_mamba2_fwd_prompt) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
+    F(llattn_mamba2_fwd_workspace_bytes) F(llattn_mamba2_fwd) F(llattn_mamba2_fwd_residual) F(llattn_mamba2_fwd_prompt) F(llattn_mamba2_bwd_workspace_bytes) F(llattn_mamba2_bwd_layer_workspace_bytes) F(llattn_mamba2_bwd_saved) F(llattn_mamba2_bwd_layer)        \
     F(llattn_mamba2_layer_prep_fwd) F(llattn_mamba2_layer_prep_bwd) F(llattn_mamba2_layer_step) F(llattn_gdn_layer_step)            \
     F(llattn_mamba2_prompt_prep) F(llattn_mamba2_prompt_residual) F(llattn_mamba2_prompt_states) F(llattn_mamba2_prompt_tail) F(llattn_mamba2_residual) F(llattn_mixer_prep_fwd)            \
     F(llattn_mixer_prep_bwd) F(llattn_mixer_norm_fwd) F(llattn_mixer_norm_bwd) F(llattn_gdn_prompt_prep)                             \
@@ -191,7 +191,7 @@ ScanGrads mamba2_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     r.dv = contiguous_like(v);
     r.dg = contiguous_like(g_cum);
     r.dl = empty(l.sizes(), at::kFloat, l);
-    const size_t n = lib.llattn_mamba2_bwd_workspace_bytes(B, T, H, G, K, V, L);
+    const size_t n = (layer ? lib.llattn_mamba2_bwd_layer_workspace_bytes : lib.llattn_mamba2_bwd_workspace_bytes)(B, T, H, G, K, V, L);
     const Tensor ws = empty({(int64_t)std::max<size_t>(n, 256)}, at::kByte, q);
     const auto bwd = layer ? lib.llattn_mamba2_bwd_layer : lib.llattn_mamba2_bwd_saved;
     check(bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), fptr(g_cum), l.data_ptr(), d_o.data_ptr(), r.dq.data_ptr(), r.dk.data_ptr(), r.dv.data_ptr(),

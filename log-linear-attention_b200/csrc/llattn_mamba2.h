@@ -12,6 +12,7 @@ namespace llattn {
 
 constexpr int M2_MLOW = 3;   // a segment is 2^M2_MLOW chunks (512 tokens)
 constexpr int M2_MAX_LH = 10;   // segment levels held by the per-level scans over segments (T <= 512 * 2^10)
+constexpr int M2_MAX_L_TC = 20;   // lambda levels that the tcgen05 kernels' tables hold; more go to the warp-level kernels
 
 struct Mamba2Params {
     // tensor maps (64-column panels, 128 rows) for the tcgen05 kernels; valid only when those run
@@ -74,6 +75,10 @@ struct Mamba2Params {
 };
 
 bool mamba2_uses_tc(const Mamba2Params& p);
+// by what a call's sizes say alone (the workspace is carved by it)
+inline bool mamba2_bwd_shape_uses_tc(const Mamba2Params& p) {
+    return p.L <= M2_MAX_L_TC && !(p.chunk_rounding && (p.K != 128 || ((p.T / 64) % 2) != 0));
+}
 bool mamba2_bwd_uses_tc(const Mamba2Params& p);
 // Whether every pair of chunks and all 128 state rows of the tensor-core tiles hold data: the kernel of one segment comes without the tests for it then.
 inline bool mamba2_whole_pairs(const Mamba2Params& p) { return p.NT % 2 == 0 && p.K == 128; }

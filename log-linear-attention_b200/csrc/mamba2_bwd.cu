@@ -1172,7 +1172,7 @@ bool mamba2_bwd_uses_tc(const Mamba2Params& p) {
     // choice: the error of sum_t dg dt against fp64, in its absolute terms (mean of 4 heads and seeds, warp-level / tensor cores): T = 192 1.0e-3 / 1.0e-3,
     // T = 1088 1.5e-3 / 5.8e-4, T = 2112 7.3e-4 / 6.0e-4; K = 64, T = 576 2.2e-3 / 1.2e-3, T = 1088 7.9e-4 / 4.5e-4; even counts, which have no such
     // choice: T = 256 2.3e-3 / 1.6e-3, T = 2048 1.1e-3 / 7.8e-4.  Nor the faster one: see mamba2_uses_tc.
-    return mamba2_uses_tc(p) && !(p.chunk_rounding && (p.K != 128 || (p.NT % 2) != 0));
+    return mamba2_uses_tc(p) && mamba2_bwd_shape_uses_tc(p);
 }
 
 template <int KD, int VD, int MLOW>

@@ -571,7 +571,7 @@ std::atomic<int> g_use_tensor_core_path{1};
 // sequences of an odd number of chunks and K = 64 went to before, and takes 3.8 ms here; T = 16384, 32 heads, K = 64: 1.98 -> 0.98 ms; a single
 // chunk, forward: 61 -> 18 us of which most is the host's.  More levels than 20 do not fit the tables in shared memory.
 // o and dv leave them in 16-byte stores (the warp-level kernels write pairs of values).
-bool mamba2_uses_tc(const Mamba2Params& p) { return p.V == 64 && p.L <= 20 && !p.warp_level && !misaligned(16, {p.o, p.dv}) && g_use_tensor_core_path.load(); }
+bool mamba2_uses_tc(const Mamba2Params& p) { return p.V == 64 && p.L <= M2_MAX_L_TC && !p.warp_level && !misaligned(16, {p.o, p.dv}) && g_use_tensor_core_path.load(); }
 
 template <int KD, int VD, int MLOW>
 static int launch_states(Mamba2Params p, cudaStream_t stream) {

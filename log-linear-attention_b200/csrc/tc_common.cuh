@@ -36,7 +36,6 @@ constexpr int TM_S = 0, TM_O = 128, TM_T0 = 192, TM_T1 = 256, TM_KV = 320, TM_CO
 // the CTA is launched with three warpgroups so that registers can be moved from the third to the
 // first two (setmaxnreg); warps 9..11 exit at once
 constexpr int NTHREADS = 384, MMA_WARP = 8;
-constexpr int MAX_L_TC = 20;        // lambda levels supported by this kernel (T up to 64 * 2^13)
 constexpr int LAM_LD = MAX_L + 2;   // row stride of the staged lambda tile: odd number of 32-bit words, no bank conflicts
 }  // namespace tc
 

@@ -39,6 +39,8 @@ def lib():
     L.llattn_mamba2_fwd_workspace_bytes.argtypes = _SHAPE
     L.llattn_mamba2_bwd_workspace_bytes.restype = ctypes.c_size_t
     L.llattn_mamba2_bwd_workspace_bytes.argtypes = _SHAPE
+    L.llattn_mamba2_bwd_layer_workspace_bytes.restype = ctypes.c_size_t
+    L.llattn_mamba2_bwd_layer_workspace_bytes.argtypes = _SHAPE
     L.llattn_mamba2_fwd.restype = ctypes.c_int
     L.llattn_mamba2_fwd.argtypes = [_P] * 7 + [_P, ctypes.c_size_t] + _SHAPE + [_P]
     L.llattn_static_scratch_bytes.restype = ctypes.c_size_t

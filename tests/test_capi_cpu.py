@@ -84,6 +84,19 @@ def test_workspace_sizes(lib):
     assert lib.llattn_mamba2_fwd_workspace_bytes(1, 100, 2, 1, 128, 64, 10) == 0
 
 
+@pytest.mark.parametrize("T,K", [(512, 128), (576, 64), (576, 128), (4096, 64), (4096, 128)])
+def test_backward_workspace_has_tiles_for_the_tensor_core_kernels_only(lib, T, K):
+    """Calls that take the warp-level kernels (more than twenty lambda levels; layers of an odd number of chunks or with K = 64) read neither the level states
+    inside a single segment nor the gradients of the pairs' summaries: their workspace does without those tiles."""
+    B, H = 2, 3
+    need = lambda L: lib.llattn_mamba2_bwd_workspace_bytes(B, T, H, 1, K, 64, L)
+    layer = lambda L: lib.llattn_mamba2_bwd_layer_workspace_bytes(B, T, H, 1, K, 64, L)
+    tiles = (2 if T <= 512 else 1) * B * H * -(-T // 128) * K * 64 * 2
+    assert need(20) - need(21) == tiles
+    assert need(21) == need(32) == layer(21)
+    assert layer(20) == (need(21) if K == 64 or (T // 64) % 2 else need(20))
+
+
 @pytest.mark.parametrize("shape,code", [
     ((1, 100, 2, 1, 128, 64, 10), -2),     # T % 64
     ((1, 1024, 3, 2, 128, 64, 12), -4),    # H % G

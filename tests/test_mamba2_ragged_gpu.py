@@ -53,3 +53,21 @@ def test_layer_backward_keeps_the_rounding_of_the_chunk_kernels(T, N):
         _lib.lib().llattn_testing_use_tensor_core_path(1)
     for a, b in zip(here, want):
         assert (a.double() - b.double()).norm() <= 3e-3 * b.double().norm()
+
+
+@pytest.mark.parametrize("T,L", [(1024, 21), (4160, 24)])
+def test_more_lambda_levels_than_the_tensor_core_kernels_hold(T, L):
+    """More than twenty levels: with N = 64 every kernel is a warp-level one, so that the choice between the two generations changes no digit."""
+    from hattention_b200 import _lib
+    q, k, v, g, l, do = rounded_inputs(1, T, 3, 64, 64, 1, L, seed=T + L)
+    o, grads = run_cuda(q, k, v, g, l, do)
+    try:
+        _lib.lib().llattn_testing_use_tensor_core_path(0)
+        want, _ = run_cuda(q, k, v, g, l, do)
+    finally:
+        _lib.lib().llattn_testing_use_tensor_core_path(1)
+    assert torch.equal(o, want)
+    o_ref, g_ref = orc.mamba2_grads(q, k, v, g, l, do, fn=orc.mamba2_chunkwise_blocked if T > 4096 else orc.mamba2_chunkwise)
+    assert_close(o, o_ref, "o")
+    for got, ref, key in zip(grads, g_ref, ("dq", "dk", "dv", "dg", "dl")):
+        assert_close(got, ref, key)
