@@ -57,14 +57,14 @@ size_t setup(llattn::Mamba2Params& p, void* ws, bool backward) {
     Carver c(ws);
     p.err = c.take<int>(64);      // status word first (256 bytes)
     if (backward) {
-        // what a call clears: from the status word up to g
-        p.dq_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
-        p.dk_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
+        // what a call clears: from the status word up to g (up to the accumulators of q and k where it needs none)
         p.wq = c.take<float>((size_t)p.B * p.T * p.H);
         p.Yseg = c.take<float>(BH * p.NS * (p.LH > 0 ? p.LH : 1));
         p.Xt = c.take<float>(BH * p.NT);
         p.Zc = c.take<float>(BH * p.NT * p.LZ);
         p.Yc = c.take<float>(BH * p.NT * (llattn::M2_MLOW + 1));
+        p.dq_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
+        p.dk_acc = c.take<float>((size_t)p.B * p.T * p.G * p.K);
         p.g = c.take<float>((size_t)p.B * p.T * p.H);
     }
     if (p.NS > 1) {
@@ -116,6 +116,16 @@ extern "C" {
 
 int llattn_version(void) { return 2; }
 void llattn_testing_use_tensor_core_path(int enabled) { llattn::g_use_tensor_core_path.store(enabled ? 1 : 0); }
+int llattn_testing_mamba2_heads_per_cta(int B, int T, int H, int G, int K, int V, int L) {
+    const int rc = check_shape(B, T, H, G, K, V, L);
+    if (rc != 0) return rc;
+    llattn::Mamba2Params p = {};
+    p.B = B; p.T = T; p.H = H; p.G = G; p.K = K; p.V = V; p.L = L;
+    setup(p, nullptr, false);
+    int dev = -1, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || llattn::sm_count(&sms, dev) != cudaSuccess) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    return llattn::mamba2_heads_per_cta(p, sms);
+}
 unsigned long long llattn_kernel_launches(void) { return llattn::g_kernel_launches.load(); }
 
 int llattn_workspace_status(const void* workspace, int* status_host, void* stream) {
@@ -303,12 +313,19 @@ static int mamba2_bwd_impl(const void* q, const void* k, const void* v, const fl
     p.dv = (__nv_bfloat16*)dv; p.dl = dlambda;
     const size_t nqk = (size_t)B * T * G * K, nbth = (size_t)B * T * H;
     // (the tensor-core kernels write d lambda of every level)
-    if ((rc = llattn::mamba2_bwd_init(g_cum, const_cast<float*>(p.g), (long)B * T, H, p.err, (size_t)((unsigned char*)p.g - (unsigned char*)p.err),
-                                      dlambda, llattn::mamba2_bwd_uses_tc(p) ? 0 : (long)(nbth * L), st)) != 0)
+    const bool use_tc = llattn::mamba2_bwd_uses_tc(p);
+    if (use_tc && !llattn::misaligned(16, {dq, dk}) && llattn::mamba2_cta_has_group(p)) {
+        p.dq_out = (__nv_bfloat16*)dq;
+        p.dk_out = (__nv_bfloat16*)dk;
+    }
+    const void* cleared = p.dq_out ? (const void*)p.dq_acc : p.g;
+    if ((rc = llattn::mamba2_bwd_init(g_cum, const_cast<float*>(p.g), (long)B * T, H, p.err, (size_t)((const unsigned char*)cleared - (unsigned char*)p.err),
+                                      dlambda, use_tc ? 0 : (long)(nbth * L), st)) != 0)
         return rc;
     rc = llattn::mamba2_bwd_dispatch(p, st);
     if (rc != 0) return rc;
     if ((rc = llattn::mamba2_dg(p, dg, st)) != 0) return rc;
+    if (p.dq_out) return (int)cudaGetLastError();
     // the accumulators are adjacent (their size is a multiple of 256 bytes); one pass where the results are too
     if ((unsigned char*)dk == (unsigned char*)dq + nqk * 2) {
         llattn::cast_f32_to_bf16(p.dq_acc, dq, (long)(2 * nqk), st);

@@ -21,7 +21,7 @@ struct Mamba2Params {
     alignas(64) CUtensorMap tm_lo;             // level states inside the segments as a (B*H*ceil(NT/2)*K, V) matrix
     alignas(64) CUtensorMap tm_lo_a, tm_dh, tm_df;   // gradients of the pairs' and of the segments' summaries, what the readers of a segment send back
     alignas(64) CUtensorMap tm_dv;
-    alignas(64) CUtensorMap tm_dq, tm_dk;      // fp32 (B*T, G, K) accumulators, 32-column boxes (reduce-add)
+    alignas(64) CUtensorMap tm_dq, tm_dk;      // fp32 (B*T, G, K) accumulators, 32-column boxes (reduce-add); or the bf16 gradients
     // inputs
     const __nv_bfloat16* q;      // (B,T,G,K)
     const __nv_bfloat16* k;      // (B,T,G,K)
@@ -35,6 +35,7 @@ struct Mamba2Params {
     float* g_cum;                // (B,T,H) in-chunk inclusive cumsum of g
     float* dq_acc;               // (B,T,G,K) fp32 accumulators (backward)
     float* dk_acc;               // (B,T,G,K)
+    __nv_bfloat16 *dq_out, *dk_out;   // (B,T,G,K) the gradients themselves, where a CTA has all heads of a group (null: the accumulators)
     __nv_bfloat16* dv;           // (B,T,H,V)
     float* dl;                   // (B,T,H,L)
     float* wq;                   // (B,T,H)  accumulates q.dq - k.dk per token and head (backward)
@@ -90,6 +91,7 @@ int mamba2_fwd_states_dispatch(Mamba2Params p, cudaStream_t stream);
 int mamba2_fwd_one_segment_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_out_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_heads_per_cta(const Mamba2Params& p, int sms);
+bool mamba2_cta_has_group(const Mamba2Params& p);      // one CTA of those kernels has all heads that share q and k
 // gradients on tcgen05: what the readers of the high levels send back; behind the scan over segments the gradient of every pair's summary; dq, dk, dv, d lambda
 int mamba2_readers_tc_launch(const Mamba2Params& p, cudaStream_t stream);
 int mamba2_adjoint_tc_launch(const Mamba2Params& p, cudaStream_t stream);

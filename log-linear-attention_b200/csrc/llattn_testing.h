@@ -12,6 +12,11 @@ extern "C" {
  * is an atomic; calls that are already dispatched keep the kernels they were given. */
 void llattn_testing_use_tensor_core_path(int enabled);
 
+/* Heads of a q / k group that a CTA of the tensor-core output and gradient kernels walks for these sizes on the current
+ * device, so that a test can tell that its sizes reach a CTA's second and third head (and a CTA with what is left over).
+ * Negative: an error code. */
+int llattn_testing_mamba2_heads_per_cta(int B, int T, int H, int G, int K, int V, int L);
+
 /* One CTA waits on an mbarrier that nothing ever completes, with `spin_limit` polls as the bound, and then
  * reports through the same path as the production kernels: *status_dev (device memory) is set to 1 and the
  * kernel returns.  Lets a test see the give-up path without a hung GPU.  spin_limit is clamped to [1, 2^20]. */

@@ -74,6 +74,35 @@ __device__ __forceinline__ void stage_gradient(unsigned char* stage, uint32_t ta
     }
 }
 
+// The same in bf16 (tile layout of the operands), where no other CTA adds to them: the accumulators are neither cleared nor added to nor converted, passes over
+// fp32 gradients that are as large as everything else where every head has its own q and k.  Walking one head a CTA shares nothing, and with the
+// accumulators such calls took longer than on the kernels that walked segments (B = 16, T = 1024, 24 heads and groups: 921, 988 with accumulators, 779 us
+// without; 12 groups of two 775, 683, 576).  The rounding is that of the conversion pass.
+template <int KD>
+__device__ __forceinline__ void stage_gradient_bf16(unsigned char* stage, uint32_t taddr, int warp, int row, int part, int parts) {
+    for (int bx = part; bx < KD / 32; bx += parts) {
+        float t[32];
+        umma::tmem_ld32(umma::tmem_addr(taddr, warp, bx * 32), t);
+#pragma unroll
+        for (int c = 0; c < 32; c += 8)
+            *reinterpret_cast<uint4*>(stage + umma::tile_offset(row, bx * 32 + c, tc::PT)) =
+                make_uint4(pack_bf16(t[c], t[c + 1]), pack_bf16(t[c + 2], t[c + 3]), pack_bf16(t[c + 4], t[c + 5]), pack_bf16(t[c + 6], t[c + 7]));
+    }
+}
+// by one thread: what the two above staged leaves
+template <int KD>
+__device__ __forceinline__ void store_gradient(const CUtensorMap* map, bool whole, int grp, int t0, int b, unsigned char* stage) {
+    if (whole) {
+#pragma unroll
+        for (int c = 0; c < KD; c += 64) tma::store_seq_box(map, c, grp, t0, b, stage + c * tc::PT * 2);
+    } else {
+#pragma unroll
+        for (int bx = 0; bx < KD / 32; ++bx) tma::reduce_add_seq_box(map, bx * 32, grp, t0, b, stage + bx * 16384);
+    }
+    tma::commit_group();
+    tma::wait_group0();
+}
+
 // ------------------------------------------------------------------------------------------
 // dq, d lambda, reader totals
 // ------------------------------------------------------------------------------------------
@@ -604,15 +633,11 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
         bar_rows();
         umma::mbar_wait(done, 0, abort_flag);
         umma::fence_after_sync();
-        stage_gradient<KD>(smem + SM::q_off, tbase + tcq::TM_DQ, warp, row, set, 2);
+        if (p.dq_out) stage_gradient_bf16<KD>(smem + SM::q_off, tbase + tcq::TM_DQ, warp, row, set, 2);
+        else stage_gradient<KD>(smem + SM::q_off, tbase + tcq::TM_DQ, warp, row, set, 2);
         umma::fence_async_smem();
         bar_rows();
-        if (tid == 256 && !*abort_flag) {
-#pragma unroll
-            for (int bx = 0; bx < KD / 32; ++bx) tma::reduce_add_seq_box(&p.tm_dq, bx * 32, w.grp, w.t0, w.b, smem + SM::q_off + bx * 16384);
-            tma::commit_group();
-            tma::wait_group0();
-        }
+        if (tid == 256 && !*abort_flag) store_gradient<KD>(&p.tm_dq, p.dq_out != nullptr, w.grp, w.t0, w.b, smem + SM::q_off);
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -1017,15 +1042,11 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
         // ---- dk of these heads
         umma::mbar_wait(done, 0, abort_flag);
         umma::fence_after_sync();
-        stage_gradient<KD>(smem + SM::q_off, tbase + tck::TM_DK, warp, row, ch, 2);
+        if (p.dk_out) stage_gradient_bf16<KD>(smem + SM::q_off, tbase + tck::TM_DK, warp, row, ch, 2);
+        else stage_gradient<KD>(smem + SM::q_off, tbase + tck::TM_DK, warp, row, ch, 2);
         umma::fence_async_smem();
         bar_rows();
-        if (tid == 256 && !*abort_flag) {
-#pragma unroll
-            for (int bx = 0; bx < KD / 32; ++bx) tma::reduce_add_seq_box(&p.tm_dk, bx * 32, w.grp, w.t0, w.b, smem + SM::q_off + bx * 16384);
-            tma::commit_group();
-            tma::wait_group0();
-        }
+        if (tid == 256 && !*abort_flag) store_gradient<KD>(&p.tm_dk, p.dk_out != nullptr, w.grp, w.t0, w.b, smem + SM::q_off);
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -1047,8 +1068,13 @@ static int gradient_maps(Mamba2Params& p) {
     if ((rc = tma::make_seq_map(&p.tm_v, p.v, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_do, p.d_o, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
     if ((rc = tma::make_seq_map(&p.tm_dv, p.dv, p.B, p.T, p.H, p.V, tc::PT, 2)) != 0) return rc;
-    if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
-    if ((rc = tma::make_seq_map(&p.tm_dk, p.dk_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
+    if (p.dq_out) {
+        if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_out, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+        if ((rc = tma::make_seq_map(&p.tm_dk, p.dk_out, p.B, p.T, p.G, p.K, tc::PT, 2)) != 0) return rc;
+    } else {
+        if ((rc = tma::make_seq_map(&p.tm_dq, p.dq_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
+        if ((rc = tma::make_seq_map(&p.tm_dk, p.dk_acc, p.B, p.T, p.G, p.K, tc::PT, 4)) != 0) return rc;
+    }
     if (NP > 1) {
         if ((rc = tma::make_panel_map(&p.tm_lo, p.lo_H, BH * NP * p.K, 1, p.V, p.K)) != 0) return rc;
         if ((rc = tma::make_panel_map(&p.tm_lo_a, p.lo_A, BH * NP * p.K, 1, p.V, p.K)) != 0) return rc;

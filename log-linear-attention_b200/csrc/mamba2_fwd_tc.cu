@@ -999,6 +999,11 @@ int mamba2_heads_per_cta(const Mamba2Params& p, int sms) {
     return best;
 }
 
+bool mamba2_cta_has_group(const Mamba2Params& p) {
+    int dev = -1, sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && sm_count(&sms, dev) == cudaSuccess && mamba2_heads_per_cta(p, sms) >= p.H / p.G;
+}
+
 template <int KD, int RES>
 static int launch_out(const Mamba2Params& p, cudaStream_t stream) {
     auto kern = m2_out_tc_kernel<KD, RES>;

@@ -101,6 +101,8 @@ def lib():
     L.llattn_selftest_umma_cycles.argtypes = [ctypes.c_int] * 5 + [_P, _P, _P]
     L.llattn_testing_use_tensor_core_path.restype = None        # test-only symbol (csrc/llattn_testing.h)
     L.llattn_testing_use_tensor_core_path.argtypes = [ctypes.c_int]
+    L.llattn_testing_mamba2_heads_per_cta.restype = ctypes.c_int   # test-only symbol
+    L.llattn_testing_mamba2_heads_per_cta.argtypes = _SHAPE
     L.llattn_selftest_wait_timeout.restype = ctypes.c_int       # test-only symbol
     L.llattn_selftest_wait_timeout.argtypes = [ctypes.c_int, _P, _P]
     L.llattn_kernel_launches.restype = ctypes.c_ulonglong

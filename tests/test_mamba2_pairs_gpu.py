@@ -43,6 +43,11 @@ def test_gradients_of_a_cta_match_oracle(B, T, H, N, G, L):
         assert_close(got, ref, key)
 
 
+def heads_per_cta(B, T, H, N, G, L):
+    from hattention_b200 import _lib
+    return _lib.lib().llattn_testing_mamba2_heads_per_cta(B, T, H, G, N, 64, L)
+
+
 @pytest.mark.parametrize("params", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,H", [(576, 9), (1024, 2)])
 def test_residual_of_a_layer(T, H, params):
@@ -63,3 +68,42 @@ def test_residual_of_a_layer(T, H, params):
     # the sum and the product are rounded to fp32 (2^-24 of each, on either side), bf16 results once more
     bound = 2.0 ** -22 * (o.float().abs() + (D.float()[:, None] * x.float()).abs()) + (2.0 ** -8 * want.abs() if params == torch.bfloat16 else 0.)
     assert y.dtype == params and ((y.float() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("B,T,H,N,G,L,heads", [
+    (1, 640, 6, 128, 6, 11, 1),        # one head a group
+    (2, 2112, 4, 64, 4, 13, 1),        # N = 64, a last half pair
+    (1, 64, 3, 128, 3, 8, 1),          # a single chunk
+    (4, 1984, 10, 64, 2, 12, 5),       # five heads a group, all in one CTA
+    (8, 1088, 12, 128, 4, 12, 3),
+])
+def test_gradients_of_whole_groups_leave_as_they_are(B, T, H, N, G, L, heads):
+    """Where a CTA has all heads of a group dq and dk need no accumulators: the digits are those of the accumulators, which serve results that start off a 16-byte boundary."""
+    from hattention_b200 import _lib
+    lib, dev = _lib.lib(), torch.device("cuda:0")
+    assert heads_per_cta(B, T, H, N, G, L) == heads == H // G
+    ins = rounded_inputs(B, T, H, 64, N, G, L, seed=T + H)
+    q, k, v, g, l, do = (x.to(dev) for x in ins)
+    q, k, v, l, do = (x.bfloat16() for x in (q, k, v, l, do))
+    g_cum = torch.cumsum(g.reshape(B, T // 64, 64, H), dim=2).reshape(B, T, H).contiguous()
+    ws = torch.empty(lib.llattn_mamba2_bwd_workspace_bytes(B, T, H, G, N, 64, L), dtype=torch.uint8, device=dev)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def run(offset):
+        n = q.numel()
+        dq, dk = (torch.full((n + 16,), float("nan"), device=dev).bfloat16() for _ in range(2))
+        dv, dg, dl = torch.empty_like(v), torch.empty_like(g), torch.empty(l.shape, device=dev)
+        rc = lib.llattn_mamba2_bwd(*(x.data_ptr() for x in (q, k, v, g_cum, l, do)), dq.data_ptr() + 2 * offset, dk.data_ptr() + 2 * offset,
+                                   *(x.data_ptr() for x in (dv, dg, dl)), ws.data_ptr(), ws.numel(), B, T, H, G, N, 64, L, stream)
+        _lib.check(rc, "llattn_mamba2_bwd")
+        _lib.raise_on_status(ws, stream, "llattn_mamba2_bwd")
+        for x in (dq, dk):
+            assert torch.isnan(x[:offset]).all() and torch.isnan(x[offset + n:]).all()
+        return [x[offset:offset + n].reshape(q.shape) for x in (dq, dk)] + [dv, dg, dl]
+
+    whole, summed = run(0), run(4)
+    _, want = orc.mamba2_grads(*ins, fn=orc.mamba2_chunkwise)
+    for a, b, ref, key in zip(whole, summed, want, ("dq", "dk", "dv", "dg", "dl")):
+        assert_close(a, ref, key)
+        if key != "dg":                                    # (sums of atomic adds)
+            assert torch.equal(a, b), key
