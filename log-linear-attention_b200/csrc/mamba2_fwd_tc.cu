@@ -12,7 +12,7 @@
 //     warp 16 + team       one chain of K / 16 (or 8) tensor-core instructions per job
 //     warps 4 team ..      S -> P of its next head, into tensor memory; a thread has a whole row
 //     warps 8 + 4 team ..  slots -> running sum in registers, output rows
-// None of them waits for another but through the rings.  A wait that gives up sets the CTA's abort flag, after which every other wait of the CTA ends at
+// (warps of two teams; a CTA of one head is one team: warps 0, 4, 8 and 9 on.)  None of them waits for another but through the rings.  A wait that gives up sets the CTA's abort flag, after which every other wait of the CTA ends at
 // once; warps that work in step go through the rest of their loops without waiting.
 //
 // What bounds it is the latency of instruction streams, not a unit (the tensor core is busy 29 % of the time, DRAM 35 %): one stream of jobs took
@@ -27,12 +27,24 @@ namespace llattn {
 namespace tco {
 constexpr int HC_MAX = 8;                 // heads per CTA
 constexpr int LAM_MAX = 120, LAM_LD = 122;   // lambda values of a token staged per CTA; the row stride is an odd number of 32-bit words
-constexpr int INTRA = 8, LAMI_LD = HC_MAX * INTRA + 2;   // of them the levels inside the pair
+constexpr int INTRA = 8;                  // of them the levels inside the pair
 constexpr int COEF_MAX = 56;              // (head, level read) combinations of a CTA
-constexpr int NST = 3, NSLOT = 2;         // per team: stages of 16 KB, tensor-memory slots of 64 columns
-constexpr int NTHREADS = 640, WORKERS = 512, MMA_WARP = 16, TMA_WARP = 18;   // (20 warps: registers move between warpgroups of four)
-constexpr int TM_S = 0, TM_P = 128, TM_SLOT = 256;
-// launched with 96 registers a thread, 61440 in all: 256 x 88 + 256 x 128 + 128 x 48
+constexpr int NSLOT = 2;                  // per team: tensor-memory slots of 64 columns
+// Two teams, one CTA per SM.  A CTA of one head (one head a group, or a call too small to fill the chip with more) has work for one team only: with half of the
+// threads, of tensor memory (P in the place of S) and of shared memory two of them share an SM, which a chain of loads, S, P and two products leaves idle
+// for the most part.  B = 16, T = 1024, 24 heads and groups: 161 -> 92 us (with the kernels that walked segments 131 and 26 for the high levels); calls
+// of fewer CTAs than SMs take what they took.
+template <int TEAMS>
+struct Teams {
+    static constexpr int NST = TEAMS == 2 ? 3 : 2;                            // per team: stages of 16 KB
+    static constexpr int HC = TEAMS == 2 ? HC_MAX : 1;                        // heads
+    static constexpr int LD = TEAMS == 2 ? LAM_LD : 22, LDI = HC * INTRA + 2; // (odd numbers of 32-bit words)
+    static constexpr int COEF = TEAMS == 2 ? COEF_MAX : 12;                   // (a pair reads at most 12 levels)
+    static constexpr int WORKERS = 256 * TEAMS, MMA_WARP = WORKERS / 32, TMA_WARP = MMA_WARP + TEAMS;
+    static constexpr int NTHREADS = TEAMS == 2 ? 640 : 320;                   // (20 warps: registers move between warpgroups of four)
+    static constexpr int TM_S = 0, TM_P = TEAMS == 2 ? 128 : 0, TM_SLOT = 128 * TEAMS, TM_COLS = 256 * TEAMS;
+};
+// two teams: launched with 96 registers a thread, 61440 in all: 256 x 88 + 256 x 128 + 128 x 48
 __device__ __forceinline__ void regs_tiles() { asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n"); }
 __device__ __forceinline__ void regs_rows() { asm volatile("setmaxnreg.inc.sync.aligned.u32 128;\n"); }
 __device__ __forceinline__ void regs_issue() { asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n"); }
@@ -41,32 +53,35 @@ __device__ __forceinline__ void regs_issue() { asm volatile("setmaxnreg.dec.sync
 // the four row warps of a team
 __device__ __forceinline__ void team_barrier(int team) { asm volatile("bar.sync %0, 128;\n" ::"r"(2 + team) : "memory"); }
 
-template <int KD>
+template <int KD, int TEAMS>
 struct OutTcSmem {
-    static constexpr uint32_t st_off = 0;                                           // [2][NST]
-    static constexpr uint32_t q_off = 2 * tco::NST * tc::V_BYTES;
+    using TM = tco::Teams<TEAMS>;
+    static constexpr uint32_t st_off = 0;                                           // [TEAMS][NST]
+    static constexpr uint32_t q_off = TEAMS * TM::NST * tc::V_BYTES;
     static constexpr uint32_t k_off = q_off + tc::PT * KD * 2;                      // k, until S is complete; then per team
-    static constexpr uint32_t x_off = k_off;                                        // [2] rows of x, then of the output
-    static constexpr uint32_t g_off = x_off + 2 * tc::V_BYTES;                      // float [HC_MAX][2][128]: G | Cf
-    static constexpr uint32_t c_off = g_off + tco::HC_MAX * 256 * 4;                // float [HC_MAX][4]: decay since a state was formed (2), D
-    static constexpr uint32_t coef_off = c_off + tco::HC_MAX * 4 * 4;               // float [COEF_MAX][128]: lambda exp(G + c) of the levels read
-    static constexpr uint32_t lami_off = coef_off + tco::COEF_MAX * 128 * 4;        // bf16 [128][LAMI_LD]
-    static constexpr uint32_t lam_off = st_off;                                     // during the preparation: bf16 [128][LAM_LD] ...
-    static constexpr uint32_t cum_off = st_off + 2 * tc::V_BYTES;                   // ... float [HC_MAX][128]
-    static constexpr uint32_t bar_off = (lami_off + tc::PT * tco::LAMI_LD * 2 + 15) & ~15u;
-    static_assert(tc::PT * tco::LAM_LD * 2 <= 2 * tc::V_BYTES, "lambda in the place of two stages");
+    static constexpr uint32_t x_off = k_off;                                        // [TEAMS] rows of x, then of the output
+    static constexpr uint32_t g_off = x_off + 2 * tc::V_BYTES;                      // float [HC][2][128]: G | Cf
+    static constexpr uint32_t c_off = g_off + TM::HC * 256 * 4;                     // float [HC][4]: decay since a state was formed (2), D
+    static constexpr uint32_t coef_off = c_off + TM::HC * 4 * 4;                    // float [COEF][128]: lambda exp(G + c) of the levels read
+    static constexpr uint32_t lami_off = coef_off + TM::COEF * 128 * 4;             // bf16 [128][LDI]
+    static constexpr uint32_t lam_off = st_off;                                     // during the preparation: bf16 [128][LD] ...
+    static constexpr uint32_t cum_off = st_off + 2 * tc::V_BYTES - (TEAMS == 2 ? 0 : 512);      // ... float [HC][128]
+    static constexpr uint32_t bar_off = (lami_off + tc::PT * TM::LDI * 2 + 15) & ~15u;
     static constexpr uint32_t total = bar_off + 320 + 1024;                         // + slack for 1024-byte alignment
+    static_assert(tc::PT * TM::LD * 2 <= cum_off && cum_off + TM::HC * 512 <= q_off, "lambda and the sums in the places of the stages");
+    static_assert(TEAMS == 2 || 2 * (total + 1024) <= 228 * 1024, "two CTAs per SM");
 };
 
 // RES: 0 writes o; 1, 2 write y = o + D x of a layer (bf16 / fp32), o rounded to bf16 first as if it were stored; 3 is 1 with D x rounded to
 // bf16 too (prompts, whose sum is two operators' with a bf16 D).
-template <int KD, int RES>
-__global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __grid_constant__ Mamba2Params p) {
+template <int KD, int RES, int TEAMS>
+__global__ void __launch_bounds__(tco::Teams<TEAMS>::NTHREADS, TEAMS == 2 ? 1 : 2) m2_out_tc_kernel(const __grid_constant__ Mamba2Params p) {
     chain_wait();
-    using SM = OutTcSmem<KD>;
+    using SM = OutTcSmem<KD, TEAMS>;
+    using TM = tco::Teams<TEAMS>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = umma::align_1024(smem_raw);
-    constexpr int NST = tco::NST, NSLOT = tco::NSLOT;
+    constexpr int NST = TM::NST, NSLOT = tco::NSLOT;
     unsigned char* sQ = smem + SM::q_off;
     unsigned char* sK = smem + SM::k_off;
     float* sG = reinterpret_cast<float*>(smem + SM::g_off);
@@ -77,7 +92,7 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::bar_off);
     uint64_t* full_qk = bars + 0;
     uint64_t* barS = bars + 1;
-    constexpr int TEAM_BARS = 5 + 2 * NSLOT + 2 * NST, NBARS = 2 + 2 * TEAM_BARS;
+    constexpr int TEAM_BARS = 5 + 2 * NSLOT + 2 * NST, NBARS = 2 + TEAMS * TEAM_BARS;
     static_assert(NBARS * 8 <= 296, "barriers");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM::bar_off + 296);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SM::bar_off + 304);
@@ -97,7 +112,7 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
     const int t0 = pair * tc::PT;
     const int njobs = __popc(pair) + 1;
 
-    if (warp == tco::TMA_WARP && lane == 0) {
+    if (warp == TM::TMA_WARP && lane == 0) {
         for (int i = 0; i < NBARS; ++i)
             umma::mbar_init(&bars[i], i >= 2 && ((i - 2) % TEAM_BARS == 0 || (i - 2) % TEAM_BARS >= TEAM_BARS - NSLOT) ? 4 : 1);
         umma::fence_mbar_init();
@@ -106,8 +121,8 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
     __syncthreads();
     if (*abort_flag) return;                         // uniform: every thread reads the same shared word
 
-    if (warp >= tco::MMA_WARP) {
-        if (warp == tco::TMA_WARP && lane == 0) {
+    if (warp >= TM::MMA_WARP) {
+        if (warp == TM::TMA_WARP && lane == 0) {
             tma::expect_tx(full_qk, 2 * tc::PT * KD * 2);
 #pragma unroll
             for (int c = 0; c < KD; c += 64) {
@@ -115,16 +130,16 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
                 tma::load_seq_panel(sK + c * tc::PT * 2, &p.tm_k, c, grp, t0, b, full_qk);
             }
         }
-        if (warp == tco::MMA_WARP) umma::tmem_alloc(tmem_slot, tc::TM_COLS);
+        if (warp == TM::MMA_WARP) umma::tmem_alloc(tmem_slot, TM::TM_COLS);
     } else {
         // (loads from global memory together: a latency each, of 1 to 2 k cycles, is what the preparation consists of)
-        HeadsOfTokens<tco::WORKERS> g;
+        HeadsOfTokens<TM::WORKERS> g;
         g.load(p.g, p, b, t0, h0, nh, tid);
         const int pl = pair & 3, hd = tid >> 2;
         float D = pair_decay(p, b, h0, nh, NP, pair, (1 << pl) - 1, tid);
         if (RES && (tid & 3) == 3 && hd < nh) D = load_param(p.res_D, h0 + hd, RES == 2);
-        stage_lambda<tco::LAM_LD, tco::WORKERS / 32>(p, b, t0, h0, nh, L, sLam, warp, lane);
-        g.to_shared<256>(sG, nh, tid);
+        stage_lambda<TM::LD, TM::WORKERS / 32>(p, b, t0, h0, nh, L, sLam, warp, lane);
+        g.template to_shared<256>(sG, nh, tid);
         if (warp == 0) {
             // decay between a state's formation and this pair: of pair level 1, of the high levels; and D
             const float D0 = __shfl_sync(0xffffffffu, D, lane & ~3), D1 = __shfl_sync(0xffffffffu, D, (lane & ~3) + 1);
@@ -135,22 +150,22 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
                 sC[hd * 4 + 2] = D3;
             }
         }
-        asm volatile("bar.sync 1, 512;\n" ::: "memory");
+        asm volatile("bar.sync 1, %0;\n" ::"n"(TM::WORKERS) : "memory");
         // (the in-chunk cumulative sums go to global memory by way of the first stage)
         float* sCum = reinterpret_cast<float*>(smem + SM::cum_off);
         if (warp < nh) pair_decay_tables<2>(sG + warp * 256, sCum + warp * 128, lane);
-        asm volatile("bar.sync 1, 512;\n" ::: "memory");
-        heads_to_global<128, tco::WORKERS>(p.g_cum, p, b, t0, h0, nh, sCum, tid);
-        // what the heads' loops take from lambda: the levels inside the pair, and a factor per level read; two heads at a time
-        for (int hh = tid >> 7; hh < nh; hh += 4) {
+        asm volatile("bar.sync 1, %0;\n" ::"n"(TM::WORKERS) : "memory");
+        heads_to_global<128, TM::WORKERS>(p.g_cum, p, b, t0, h0, nh, sCum, tid);
+        // what the heads' loops take from lambda: the levels inside the pair, and a factor per level read; a head per 128 threads
+        for (int hh = tid >> 7; hh < nh; hh += 2 * TEAMS) {
             const int row = tid & 127;
-            const unsigned short* l = reinterpret_cast<const unsigned short*>(sLam + row * tco::LAM_LD + hh * L);
+            const unsigned short* l = reinterpret_cast<const unsigned short*>(sLam + row * TM::LD + hh * L);
             uint32_t li[tco::INTRA];
 #pragma unroll
             for (int i = 0; i < tco::INTRA; ++i) li[i] = i < L ? l[i] : 0;
 #pragma unroll
             for (int i = 0; i < tco::INTRA; i += 2)
-                *reinterpret_cast<uint32_t*>(sLami + row * tco::LAMI_LD + hh * tco::INTRA + i) = li[i] | li[i + 1] << 16;
+                *reinterpret_cast<uint32_t*>(sLami + row * TM::LDI + hh * tco::INTRA + i) = li[i] | li[i + 1] << 16;
             const float G = sG[hh * 256 + row], c1 = sC[hh * 4], c2 = sC[hh * 4 + 1];
             const float e0 = fexp(G), e1 = fexp(G + c1), e2 = fexp(G + c2);
             float* coef = sCoef + hh * (njobs - 1) * 128 + row;
@@ -169,7 +184,7 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
     umma::fence_after_sync();
     const uint32_t tbase = *tmem_slot;
     // the team's barriers, tensor-memory columns and stages
-    const int team = warp >= tco::MMA_WARP ? (warp & 1) : ((warp >> 2) & 1);
+    const int team = TEAMS == 1 ? 0 : warp >= TM::MMA_WARP ? (warp & 1) : ((warp >> 2) & 1);
     uint64_t* p_full = bars + 2 + team * TEAM_BARS;      // 4: one arrival per warp
     uint64_t* p_empty = p_full + 1;
     uint64_t* x_full = p_full + 2;
@@ -179,18 +194,18 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
     uint64_t* st_empty = st_full + NST;
     uint64_t* slot_full = st_empty + NST;                // [NSLOT]
     uint64_t* slot_empty = slot_full + NSLOT;            // [NSLOT] 4
-    const uint32_t tP = tbase + tco::TM_P + team * 64, tSlot = tbase + tco::TM_SLOT + team * NSLOT * 64;
+    const uint32_t tP = tbase + TM::TM_P + team * 64, tSlot = tbase + TM::TM_SLOT + team * NSLOT * 64;
     unsigned char* sSt = smem + SM::st_off + team * NST * tc::V_BYTES;
     unsigned char* sX = smem + SM::x_off + team * tc::V_BYTES;
 
-    if (warp >= tco::MMA_WARP) {
-      tco::regs_issue();
-      if (warp >= tco::TMA_WARP) {
+    if (warp >= TM::MMA_WARP) {
+      if (TEAMS == 2) tco::regs_issue();
+      if (warp >= TM::TMA_WARP) {
         if (lane == 0) {
             int st = 0, nx = 0;                      // stage, tiles of x requested
             uint32_t ph = 1;                         // parity of the "empty" wait: passes at once on the first round
             bool ok = true;
-            for (int hh = team; hh < nh && ok; hh += 2) {
+            for (int hh = team; hh < nh && ok; hh += TEAMS) {
                 const long bh = (long)b * p.H + h0 + hh;
                 int bits = pair;
                 for (int j = 0; j < njobs; ++j) {
@@ -244,12 +259,12 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
         auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, umma::mbar_wait(bar, parity, abort_flag)); };
         bool ok = wait(full_qk, 0);
         if (team == 0) {
-            umma::gemm_kk_lead<tc::PT, tc::PT, KD>(lead, tbase + tco::TM_S, aQ, umma::smem_addr(sK), ID_S, false);
+            umma::gemm_kk_lead<tc::PT, tc::PT, KD>(lead, tbase + TM::TM_S, aQ, umma::smem_addr(sK), ID_S, false);
             umma::commit_lead(lead, barS);
         }
         int st = 0, slot = 0;
         uint32_t phst = 0, phslot = 1, php = 0;
-        for (int hh = team; hh < nh && ok; hh += 2) {
+        for (int hh = team; hh < nh && ok; hh += TEAMS) {
             for (int j = 0; j < njobs; ++j) {
                 if (!(ok = wait(&st_full[st], phst) && wait(&slot_empty[slot], phslot))) break;
                 const uint32_t d = tSlot + slot * 64, tile = aSt + st * tc::V_BYTES;
@@ -282,40 +297,41 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
         }
         __syncwarp();
       }
-    } else if (warp < 8) {
-        tco::regs_tiles();
+    } else if (warp < 4 * TEAMS) {
+        if (TEAMS == 2) tco::regs_tiles();
         // ---- S -> P of every other head (bf16 pairs, A operand of P v).  This thread: row `row`, the 32-column blocks jb <= rb
         const int rb = warp & 3, row = rb * 32 + lane;
         const bool B0 = lane & 1, B1 = lane & 2, B2 = lane & 4, B3 = lane & 8, B4 = lane & 16;
         const uint32_t dst = umma::tmem_addr(tP, warp, 0);
         umma::mbar_wait(barS, 0, abort_flag);
         umma::fence_after_sync();
-        {
-            // blocks above the diagonal: zeros, which every head leaves as they are
+        auto zeros = [&]() {
             const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll 1
             for (int c = (rb + 1) * 16; c < 64; c += 8) umma::tmem_st8u(dst + c, z);
-        }
-        for (int hh = team; hh < nh; hh += 2) {
+        };
+        // blocks above the diagonal: zeros, which every head leaves as they are
+        if (TEAMS == 2) zeros();
+        for (int hh = team; hh < nh; hh += TEAMS) {
             const float* tG = sG + hh * 256;
             const float* tCf = tG + 128;
             const float Gi = tG[row];
             float lam[8];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const uint32_t w = *reinterpret_cast<const uint32_t*>(sLami + row * tco::LAMI_LD + hh * tco::INTRA + 2 * i);
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(sLami + row * TM::LDI + hh * tco::INTRA + 2 * i);
                 lam[2 * i] = __uint_as_float(w << 16);
                 lam[2 * i + 1] = __uint_as_float(w & 0xffff0000u);
             }
-            if (hh >= 2) {
-                umma::mbar_wait(p_empty, ((hh >> 1) - 1) & 1, abort_flag);
+            if (hh >= TEAMS) {
+                umma::mbar_wait(p_empty, (hh / TEAMS - 1) & 1, abort_flag);
                 umma::fence_after_sync();
             }
             // blocks below the diagonal: one level per block, decay factorised through the block end
 #pragma unroll 1
             for (int jb = 0; jb < rb; ++jb) {
                 float s[32];
-                umma::tmem_ld32(umma::tmem_addr(tbase + tco::TM_S, warp, jb * 32), s);
+                umma::tmem_ld32(umma::tmem_addr(tbase + TM::TM_S, warp, jb * 32), s);
                 const float lm = ((rb ^ jb) == 1) ? lam[6] : lam[7];
                 const float rf = lm * fexp(Gi - tG[jb * 32 + 31]);
                 const f32x2 rf2 = pack2(rf, rf);
@@ -344,7 +360,7 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
                 const float lm45 = q4 ? lam[5] : lam[4];
                 const bool far = q3 || q4;
                 float s[8];
-                umma::tmem_ld8(umma::tmem_addr(tbase + tco::TM_S, warp, j0), s);
+                umma::tmem_ld8(umma::tmem_addr(tbase + TM::TM_S, warp, j0), s);
                 uint32_t x[4];
 #pragma unroll
                 for (int e = 0; e < 8; e += 4) {
@@ -367,18 +383,19 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
                 }
                 umma::tmem_st4u(dst + rb * 16 + c * 4, x);
             }
+            if (TEAMS == 1) zeros();                 // (P grows in the place of S behind the columns that are still to be read)
             umma::tmem_wait_st();
             umma::fence_before_sync();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(p_full)) : "memory");
         }
     } else {
-        tco::regs_rows();
+        if (TEAMS == 2) tco::regs_rows();
         // ---- slots -> output rows of every other head.  This thread: row `row`
         const int rb = warp & 3, row = rb * 32 + lane;
         int slot = 0;
         uint32_t ph = 0;
-        for (int hh = team; hh < nh; hh += 2) {
+        for (int hh = team; hh < nh; hh += TEAMS) {
             const int h = h0 + hh;
             f32x2 o[32];
 #pragma unroll
@@ -388,17 +405,18 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
                 const f32x2 rs2 = pack2(rs, rs);
                 umma::mbar_wait(&slot_full[slot], ph, abort_flag);
                 umma::fence_after_sync();
+                constexpr int CW = TEAMS == 2 ? 32 : 16;         // columns at a time: as many as the registers hold
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    float x[32];
-                    umma::tmem_ld32(umma::tmem_addr(tSlot + slot * 64, warp, hf * 32), x);
-                    if (hf == 1) {
+                for (int c = 0; c < 64; c += CW) {
+                    float x[CW];
+                    umma::tmem_ld(umma::tmem_addr(tSlot + slot * 64, warp, c), x);
+                    if (c == 64 - CW) {
                         umma::fence_before_sync();
                         __syncwarp();
                         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_addr(&slot_empty[slot])) : "memory");
                     }
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) o[hf * 16 + e] = fma2(rs2, pack2(x[2 * e], x[2 * e + 1]), o[hf * 16 + e]);
+                    for (int e = 0; e < CW / 2; ++e) o[c / 2 + e] = fma2(rs2, pack2(x[2 * e], x[2 * e + 1]), o[c / 2 + e]);
                 }
                 if (++slot == NSLOT) {
                     slot = 0;
@@ -409,7 +427,7 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
             // pipe, and with it every wait of the CTA, busy for 1 to 2 k cycles a head.
             const bool issuer = (tid & 127) == 0;
             if (RES) {
-                umma::mbar_wait(x_full, (hh >> 1) & 1, abort_flag);
+                umma::mbar_wait(x_full, (hh / TEAMS) & 1, abort_flag);
                 const float dh = sC[hh * 4 + 2];
                 const f32x2 dh2 = pack2(dh, dh);
 #pragma unroll
@@ -436,7 +454,7 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
                 tma::wait_group_read0();             // the rows of this team's previous head have left
             }
             if (RES == 0) {
-                if (hh < 2) umma::mbar_wait(barS, 0, abort_flag);      // (the place of k)
+                if (hh < TEAMS) umma::mbar_wait(barS, 0, abort_flag);      // (the place of k)
                 team_barrier(team);
             }
             if (RES == 2) {
@@ -484,9 +502,9 @@ __global__ void __launch_bounds__(tco::NTHREADS, 1) m2_out_tc_kernel(const __gri
     umma::fence_before_sync();
     __syncthreads();                                 // everybody is done with tensor memory
     umma::fence_after_sync();
-    if (warp == tco::MMA_WARP) {
+    if (warp == TM::MMA_WARP) {
         if (*abort_flag && lane == 0) atomicExch(p.err, 1);
-        umma::tmem_dealloc(tbase, tc::TM_COLS);
+        umma::tmem_dealloc(tbase, TM::TM_COLS);
     }
 }
 
@@ -1004,15 +1022,19 @@ bool mamba2_cta_has_group(const Mamba2Params& p) {
     return cudaGetDevice(&dev) == cudaSuccess && sm_count(&sms, dev) == cudaSuccess && mamba2_heads_per_cta(p, sms) >= p.H / p.G;
 }
 
-template <int KD, int RES>
-static int launch_out(const Mamba2Params& p, cudaStream_t stream) {
-    auto kern = m2_out_tc_kernel<KD, RES>;
-    const size_t sm = OutTcSmem<KD>::total;
+template <int KD, int RES, int TEAMS>
+static int launch_out_teams(const Mamba2Params& p, cudaStream_t stream) {
+    auto kern = m2_out_tc_kernel<KD, RES, TEAMS>;
+    const size_t sm = OutTcSmem<KD, TEAMS>::total;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return (int)e;
     const int per_grp = p.H / p.G;
-    llattn::launch_chained(kern, p.B * ((p.NT + 1) / 2) * p.G * ((per_grp + p.hc - 1) / p.hc), tco::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
+    llattn::launch_chained(kern, p.B * ((p.NT + 1) / 2) * p.G * ((per_grp + p.hc - 1) / p.hc), tco::Teams<TEAMS>::NTHREADS, sm, stream, p); LLATTN_LAUNCHED();
     return (int)cudaGetLastError();
+}
+template <int KD, int RES>
+static int launch_out(const Mamba2Params& p, cudaStream_t stream) {
+    return p.hc == 1 ? launch_out_teams<KD, RES, 1>(p, stream) : launch_out_teams<KD, RES, 2>(p, stream);
 }
 
 template <int KD>
