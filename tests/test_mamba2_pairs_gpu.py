@@ -1,5 +1,6 @@
-"""The CTAs of the output and gradient kernels take a pair of chunks and up to eight heads of a q / k group: group sizes that leave a part of a CTA's heads over, one head a
-group, the most lambda levels that it stages, pairs that read no, one and several levels, and what only a layer asks of it."""
+"""The CTAs of the output and gradient kernels take a pair of chunks and up to eight heads of a q / k group.  Small calls have a head a CTA: pairs that read no, one and
+several levels, ends of sequences, the most lambda levels.  Calls that fill the chip walk several heads in a CTA, whose rings, sums and places in shared memory are
+written again from the second or third head on: group sizes that leave a part of a CTA's heads over, two groups, narrow states, a last half pair, and what only a layer asks of it."""
 import pytest
 import torch
 
@@ -10,10 +11,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("B,T,H,N,G,L", [
-    (1, 640, 9, 128, 1, 11),       # nine heads a group: a CTA of its own for what is over, two segments, the last of one pair
+    (1, 640, 9, 128, 1, 11),       # two segments, the last of one pair
     (2, 1024, 6, 64, 6, 12),       # one head a group
-    (1, 1088, 13, 64, 1, 12),      # an odd number of chunks, thirteen heads
-    (2, 704, 10, 128, 2, 20),      # the most lambda levels (six heads a CTA at most), a last half pair
+    (1, 1088, 13, 64, 1, 12),      # an odd number of chunks
+    (2, 704, 10, 128, 2, 20),      # the most lambda levels, two groups, a last half pair
     (1, 128, 5, 128, 1, 8),        # a single pair: no states at all
     (1, 4096, 3, 128, 1, 13),      # eight segments: pairs that read up to five levels
 ])
@@ -26,12 +27,12 @@ def test_heads_and_levels_of_a_cta_match_oracle(B, T, H, N, G, L):
 @pytest.mark.parametrize("B,T,H,N,G,L", [
     (1, 128, 5, 128, 1, 8),        # a single pair: neither states nor readers
     (2, 256, 3, 64, 1, 9),         # two pairs of one segment, N = 64
-    (1, 512, 9, 128, 1, 20),       # four pairs of one segment, a ninth head on its own, spare lambda levels
+    (1, 512, 9, 128, 1, 20),       # four pairs of one segment, spare lambda levels
     (1, 640, 9, 128, 1, 11),       # two segments, the last of one pair
     (2, 1024, 6, 64, 6, 12),       # one head a group
     (2, 704, 10, 128, 2, 20),      # a last half pair, the most lambda levels
     (1, 384, 3, 128, 1, 10),       # three pairs, the last of which nobody reads
-    (2, 896, 32, 128, 1, 11),      # the same in a second segment, enough of them for either order of completion
+    (2, 896, 32, 128, 1, 11),      # the same in a second segment, enough of them for either order of completion (four heads a CTA)
     (1, 1344, 4, 64, 2, 12),       # ... and the last pair a half
     (1, 8832, 1, 128, 1, 15),      # eighteen segments: readers of a fifth high level, for which a second CTA is there
 ])
@@ -48,13 +49,31 @@ def heads_per_cta(B, T, H, N, G, L):
     return _lib.lib().llattn_testing_mamba2_heads_per_cta(B, T, H, G, N, 64, L)
 
 
+@pytest.mark.parametrize("B,T,H,N,G,L,heads", [
+    (2, 2112, 13, 128, 1, 20, 4),      # 4 + 4 + 4 + 1 heads, a last half pair, spare lambda levels
+    (4, 1984, 10, 64, 2, 12, 5),       # whole groups of five, N = 64, an odd number of chunks
+    (2, 4096, 9, 128, 1, 13, 5),       # 5 + 4 heads, pairs that read up to five levels
+    (8, 640, 17, 64, 1, 11, 6),        # 6 + 6 + 5 heads, N = 64
+    (8, 384, 26, 128, 2, 10, 5),       # 5 + 5 + 3 heads a group, one segment
+    (16, 128, 48, 128, 1, 20, 6),      # a single pair, as many heads as L = 20 allows
+])
+def test_heads_that_follow_in_a_cta_match_oracle(B, T, H, N, G, L, heads):
+    assert heads_per_cta(B, T, H, N, G, L) == heads
+    q, k, v, g, l, do = rounded_inputs(B, T, H, 64, N, G, L, seed=T + 3 * H)
+    o, grads = run_cuda(q, k, v, g, l, do)
+    want_o, want = orc.mamba2_grads(q, k, v, g, l, do, fn=orc.mamba2_chunkwise)
+    for got, ref, key in zip((o, *grads), (want_o, *want), ("o", "dq", "dk", "dv", "dg", "dl")):
+        assert_close(got, ref, key)
+
+
 @pytest.mark.parametrize("params", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("T,H", [(576, 9), (1024, 2)])
-def test_residual_of_a_layer(T, H, params):
+@pytest.mark.parametrize("T,H,heads", [(576, 9, 1), (1024, 2, 1), (2112, 18, 5)])      # (five heads: either team of warps takes a second and one a third)
+def test_residual_of_a_layer(T, H, heads, params):
     """y = bf16(o) + D x, in the parameters' dtype, leaves by way of the tile of x: every row of it, and nothing behind the sequence's end."""
     from hattention_b200.base import HStruct, HType
     from hattention_b200.mamba_apis import hmamba_chunk_scan_combined
-    dev, L = torch.device("cuda:0"), 12
+    dev, L = torch.device("cuda:0"), 12 if T <= 2048 else 13
+    assert heads_per_cta(2, T, H, 128, 1, L) == heads
     gen = torch.Generator().manual_seed(T + H)
     r = lambda *s: torch.randn(*s, generator=gen)
     x, Bm, Cm, dl = (t.bfloat16().to(dev) for t in (r(2, T, H, 64), r(2, T, 1, 128) / 128 ** 0.5, r(2, T, 1, 128) / 128 ** 0.5, r(2, T, H, L)))
