@@ -391,14 +391,16 @@ int llattn_gdn_grad_out(const void* q, const void* k, const float* dq, const flo
 /* Diagnostic: one 128 x N x kred bf16 tensor-core product (tcgen05.mma, accumulator in tensor
  * memory) per operand-layout combination used by the kernels: mode 0: D = A B^T with A [128][kred],
  * B [N][kred]; mode 1: D = A B with B [kred][N]; mode 2: D = A^T B with A [kred][128], B [kred][N].
- * D is [128][N] fp32.  Modes 10, 11, 12 are the same three products issued through the compile-time shaped
- * loops that the kernels use.  *err_flag is set to 1 if the tensor core did not signal completion within
+ * D is [128][N] fp32.  Modes 10, 11, 12 are the same three products issued through compile-time shaped
+ * loops in a branch of one lane; modes 20..23 by a converged warp with an elected lane leading (23: D = A^T B^T with
+ * A [kred][128], B [N][kred]), modes 30, 31 as 20, 21 with A in tensor memory.  *err_flag is set to 1 if the tensor core did not signal completion within
  * the kernel's bounded wait.  (No counterpart in the reference; used by the test-suite.) */
 int llattn_selftest_umma(const void* A, const void* B, float* D, int N, int kred, int mode, int* err_flag, void* stream);
 
 /* Diagnostic: SM clock cycles from the issue of `reps` back-to-back 128 x N x kred products of one layout
- * combination (modes as above, operands resident in shared memory, accumulator in tensor memory) to their
- * completion, written to *cycles (device memory); issuers = 2 lets two warps issue `reps` products each at the
+ * combination (operands resident in shared memory, accumulator in tensor memory; modes 0..2 as above, 3 and 4 with the
+ * 256-row operand of the Gated DeltaNet scans; issued by a converged warp: 20..24 the layouts of 0..4, 30, 31 those of
+ * 0, 1 with A in tensor memory) to their completion, written to *cycles (device memory); issuers = 2 lets two warps issue `reps` products each at the
  * same time into separate accumulators.  (No counterpart in the reference.) */
 int llattn_selftest_umma_cycles(int N, int kred, int mode, int reps, int issuers, long long* cycles, int* err_flag, void* stream);
 

@@ -15,7 +15,7 @@
 // The reader products qd H_lv (output) use the same bf16 copies; they are issued behind the transition products
 // and consumed one chunk later.  The bf16 copies are kept transposed ([V column][K]) so that they are K-major B
 // operands whose rows continue from level to level: a range of levels is read by ONE chain with N = 32 x (number
-// of levels) (an instruction costs the same for N = 32 as for N = 128; slots of levels inside the range that are
+// of levels) (an instruction takes 41 cycles for N = 32, 48 for 64, 64 for 128; slots of levels inside the range that are
 // not live receive products of stale copies and are never read).  The issuing warp stays converged and predicates
 // the instructions on an elected lane: the 20 instructions of a chunk are on its chain, and inside a branch of one
 // lane they took longer (B = 4, T = 8192, H = 16, forward that keeps its states: 778 -> 747 us).  What need not wait for

@@ -382,10 +382,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dq_tc_kernel(const __grid
             for (int j = 0; j < nlev; ++j) {
                 if (!(ok = wait(&st_full[st], phst) && wait(&dos_full[dos], phdos))) break;
                 umma::fence_after_sync();
-                const uint32_t db = umma::desc_lo_kmajor(aSt + st * tc::V_BYTES);
-#pragma unroll
-                for (int kk = 0; kk < tc::VD; kk += 16)
-                    umma::mma_ts_lead(lead, tbase + tcq::TM_DQ, tbase + tcq::TM_DOS + dos * 32 + kk / 2, db + ((kk * 2) >> 4), ID_KK_KD, started || kk > 0);
+                umma::gemm_tk_lead<KD, tc::VD>(lead, tbase + tcq::TM_DQ, tbase + tcq::TM_DOS + dos * 32, aSt + st * tc::V_BYTES, ID_KK_KD, started);
                 started = true;
                 umma::commit_lead(lead, &dos_empty[dos]);
                 umma::commit_lead(lead, &st_empty[st]);
@@ -844,10 +841,7 @@ __global__ void __launch_bounds__(tcg::NTHREADS, 1) m2_dkv_tc_kernel(const __gri
             if (read) {
                 if (!(ok = wait(vs_full, hh & 1))) break;
                 umma::fence_after_sync();
-                const uint32_t db = umma::desc_lo_kmajor(aA);
-#pragma unroll
-                for (int kk = 0; kk < tc::VD; kk += 16)
-                    umma::mma_ts_lead(lead, tbase + tck::TM_DK, tbase + tck::TM_U + kk / 2, db + ((kk * 2) >> 4), ID_KK_KD, started || kk > 0);
+                umma::gemm_tk_lead<KD, tc::VD>(lead, tbase + tck::TM_DK, tbase + tck::TM_U, aA, ID_KK_KD, started);
                 started = true;
                 umma::commit_lead(lead, a_read);
             }

@@ -142,9 +142,9 @@ __device__ __forceinline__ void gemm_mm(uint32_t d_tmem, uint32_t a_saddr, int a
     }
 }
 
-// ---- issue by a whole warp that stays converged, the instruction predicated on one elected lane (`lead`): the operands stay in uniform registers.  With
-// the loop inside a branch of one lane an instruction costs 45 cycles to issue whatever its shape; here N = 64 with A in tensor memory runs at 32 cycles,
-// the tensor core's own rate (A in shared memory: 48, the operand fetch).
+// ---- issue by a whole warp that stays converged, the instruction predicated on one elected lane (`lead`): the operands stay in uniform registers.
+// Cycles an instruction, back to back (llattn_selftest_umma_cycles, modes 0.. and 20..): inside a branch of one lane at least 55 whatever its shape; here N = 64
+// takes 32 with A in tensor memory, the tensor core's own rate, and 48 with A in shared memory, the operand fetch; N = 32 41; N = 128 is at 64 either way.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t r;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(r));
@@ -182,6 +182,16 @@ __device__ __forceinline__ void gemm_tm_lead(uint32_t lead, uint32_t d_tmem, uin
 #pragma unroll
     for (int kk = 0; kk < KRED; kk += 16)
         mma_ts_lead(lead, d_tmem, a_tmem + kk / 2, db + ((kk * ROW_BYTES) >> 4), idesc, accumulate || kk > 0);
+}
+// A in tensor memory, B a K-major tile (rows = N index)
+template <int B_ROWS, int KRED>
+__device__ __forceinline__ void gemm_tk_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_saddr, uint32_t idesc, bool accumulate) {
+    const uint32_t db = desc_lo_kmajor(b_saddr);
+#pragma unroll
+    for (int kk = 0; kk < KRED; kk += 16) {
+        const uint32_t kb = (kk >> 6) * B_ROWS * ROW_BYTES + (kk & 63) * 2;
+        mma_ts_lead(lead, d_tmem, a_tmem + kk / 2, db + (kb >> 4), idesc, accumulate || kk > 0);
+    }
 }
 template <int A_ROWS, int B_ROWS, int KRED>
 __device__ __forceinline__ void gemm_km_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_saddr, uint32_t b_saddr, uint32_t idesc, bool accumulate) {

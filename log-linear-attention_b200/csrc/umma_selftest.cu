@@ -11,22 +11,25 @@ namespace llattn {
 // mode 0: A [128][kred], B [N][kred]      -> D = A B^T   (both K-major)
 // mode 1: A [128][kred], B [kred][N]      -> D = A B     (A K-major, B MN-major)
 // mode 2: A [kred][128], B [kred][N]      -> D = A^T B   (both MN-major)
+// mode 3: A [kred][128], B [N][kred]      -> D = A^T B^T
+// mode + 10: the compile-time shaped issue loops inside a branch of one lane; mode + 20: issued by a converged warp, an elected lane leading
+// modes 30, 31: as 20, 21 with A in tensor memory (bf16 pairs along the reduction index)
 __global__ void __launch_bounds__(128, 1) umma_selftest_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B,
                                                                float* __restrict__ D, int N, int kred, int tmode,
                                                                int* __restrict__ err) {
-    const int mode = tmode >= 10 ? tmode - 10 + 100 : tmode;      // 100.. : no run-time shaped issue below
     const int lmode = tmode % 10;                                  // operand layout combination
+    const bool mn_a = lmode >= 2, mn_b = lmode == 1 || lmode == 2; // stored with the reduction index down the rows
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    // modes 10..12 place the tiles high in shared memory (the address range that the kernels' later tiles use)
+    // modes from 10 on place the tiles high in shared memory (the address range that the kernels' later tiles use)
     unsigned char* sA = smem + (tmode >= 10 ? 131072 : 0);              // up to 128 x 128 bf16 = 32 KB
     unsigned char* sB = smem + (tmode >= 10 ? 131072 + 49152 : 32768);  // up to 128 x 128 bf16
     __shared__ uint64_t bar;
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5;
 
-    const int a_rows = (lmode == 2) ? kred : 128, a_cols = (lmode == 2) ? 128 : kred;
-    const int b_rows = (lmode == 0) ? N : kred, b_cols = (lmode == 0) ? kred : N;
+    const int a_rows = mn_a ? kred : 128, a_cols = mn_a ? 128 : kred;
+    const int b_rows = mn_b ? kred : N, b_cols = mn_b ? N : kred;
     for (int e = tid; e < a_rows * a_cols; e += 128) {
         const int r = e / a_cols, c = e % a_cols;
         *reinterpret_cast<bf16*>(sA + umma::tile_offset(r, c, a_rows)) = A[e];
@@ -35,7 +38,7 @@ __global__ void __launch_bounds__(128, 1) umma_selftest_kernel(const bf16* __res
         const int r = e / b_cols, c = e % b_cols;
         *reinterpret_cast<bf16*>(sB + umma::tile_offset(r, c, b_rows)) = B[e];
     }
-    if (warp == 0) umma::tmem_alloc(&tmem_slot, 128);
+    if (warp == 0) umma::tmem_alloc(&tmem_slot, 256);
     if (tid == 0) {
         umma::mbar_init(&bar, 1);
         umma::fence_mbar_init();
@@ -44,8 +47,41 @@ __global__ void __launch_bounds__(128, 1) umma_selftest_kernel(const bf16* __res
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t tbase = tmem_slot;
-    if (tid == 0) {
+    const uint32_t tbase = tmem_slot, tA = tbase + 128;
+    if (tmode >= 30) {
+        // row `tid` of A, two values a column
+        for (int c = 0; c < kred / 2; c += 16) {
+            uint32_t x[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[i] = *reinterpret_cast<const uint32_t*>(A + tid * kred + 2 * (c + i));
+            umma::tmem_st16u(umma::tmem_addr(tA, warp, c), x);
+        }
+        umma::tmem_wait_st();
+        umma::fence_before_sync();
+        __syncthreads();
+        umma::fence_after_sync();
+    }
+    if (tmode >= 20) {
+        if (warp == 0) {
+            const uint32_t a = umma::smem_addr(sA), b = umma::smem_addr(sB), lead = umma::elect_one();
+#define LLATTN_ST_CASE(NN, KK)                                                                                                       \
+            if (N == NN && kred == KK) {                                                                                             \
+                if (tmode == 20) umma::gemm_kk_lead<128, NN, KK>(lead, tbase, a, b, umma::idesc_bf16(128, NN, false, false), false); \
+                if (tmode == 21) umma::gemm_km_lead<128, KK, KK>(lead, tbase, a, b, umma::idesc_bf16(128, NN, false, true), false);  \
+                if (tmode == 22) umma::gemm_mm_lead<KK, KK, KK>(lead, tbase, a, b, umma::idesc_bf16(128, NN, true, true), false);    \
+                if (tmode == 23) umma::gemm_mk_lead<KK, NN, KK>(lead, tbase, a, b, umma::idesc_bf16(128, NN, true, false), false);   \
+                if (tmode == 30) umma::gemm_tk_lead<NN, KK>(lead, tbase, tA, b, umma::idesc_bf16(128, NN, false, false), false);     \
+                if (tmode == 31) umma::gemm_tm_lead<KK, KK>(lead, tbase, tA, b, umma::idesc_bf16(128, NN, false, true), false);      \
+            }
+            LLATTN_ST_CASE(64, 64)
+            LLATTN_ST_CASE(64, 128)
+            LLATTN_ST_CASE(128, 64)
+            LLATTN_ST_CASE(128, 128)
+#undef LLATTN_ST_CASE
+            umma::commit_lead(lead, &bar);
+        }
+    } else if (tid == 0) {
+        const int mode = tmode;
         const uint32_t a = umma::smem_addr(sA), b = umma::smem_addr(sB);
         // mode + 10 selects the compile-time shaped issue loops that the kernels use
         if (mode == 0) umma::gemm_kk(tbase, a, a_rows, b, b_rows, kred, umma::idesc_bf16(128, N, false, false), false);
@@ -78,12 +114,28 @@ __global__ void __launch_bounds__(128, 1) umma_selftest_kernel(const bf16* __res
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tbase, 128);
+    if (warp == 0) umma::tmem_dealloc(tbase, 256);
+}
+
+template <int MODE, int KK>
+__device__ __forceinline__ void issue_converged(int reps, uint32_t lead, uint32_t d, uint32_t a, uint32_t tA, uint32_t b, int N) {
+    const uint32_t id = umma::idesc_bf16(128, N, MODE == 22 || MODE == 24, MODE == 21 || MODE == 22 || MODE == 31);
+    for (int r = 0; r < reps; ++r) {
+        if (MODE == 20) umma::gemm_kk_lead<128, 128, KK>(lead, d, a, b, id, r > 0);
+        if (MODE == 21) umma::gemm_km_lead<128, 128, KK>(lead, d, a, b, id, r > 0);
+        if (MODE == 22) umma::gemm_mm_lead<128, 128, KK>(lead, d, a, b, id, r > 0);
+        if (MODE == 23) umma::gemm_kk_lead<128, 256, KK>(lead, d, a, b, id, r > 0);
+        if (MODE == 24) umma::gemm_mk_lead<64, 256, KK>(lead, d, a, b, id, r > 0);
+        if (MODE == 30) umma::gemm_tk_lead<128, KK>(lead, d, tA, b, id, r > 0);
+        if (MODE == 31) umma::gemm_tm_lead<128, KK>(lead, d, tA, b, id, r > 0);
+    }
 }
 
 // Issue-to-completion time of `reps` back-to-back products of one layout combination (operands already in
 // shared memory, accumulators in tensor memory): the per-instruction cost that the kernel designs assume.
 // issuers = 2: warps 0 and 1 each issue `reps` products into their own accumulator at the same time.
+// Modes from 20 on: as the kernels issue them from a converged warp (see umma::elect_one); 20..22 the layouts of 0..2, 23, 24 those of 3, 4,
+// 30, 31 those of 0, 1 with A in tensor memory.
 // Dynamic shared memory: 64 KB of operands (modes 0..2) or 128 KB (modes 3, 4, whose B tile has 256-row panels:
 // the chain reads up to byte 32768 + 32768 + 128 * 128 of it).
 __global__ void __launch_bounds__(128, 1) umma_cycles_kernel(int N, int kred, int mode, int reps, int issuers, int smem_bytes,
@@ -96,7 +148,7 @@ __global__ void __launch_bounds__(128, 1) umma_cycles_kernel(int N, int kred, in
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int e = tid; e < smem_bytes / 4; e += 128) reinterpret_cast<uint32_t*>(smem)[e] = 0x3c003c00u;     // small finite bf16 pairs
-    if (warp == 0) umma::tmem_alloc(&tmem_slot, 256);
+    if (warp == 0) umma::tmem_alloc(&tmem_slot, 512);
     if (tid == 0) {
         umma::mbar_init(&bar[0], 1);
         umma::mbar_init(&bar[1], 1);
@@ -106,9 +158,35 @@ __global__ void __launch_bounds__(128, 1) umma_cycles_kernel(int N, int kred, in
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t tbase = tmem_slot + (warp == 1 ? 128 : 0);
+    const uint32_t tbase = tmem_slot + (warp == 1 ? 128 : 0), tA = tmem_slot + 256;
+    if (mode >= 30) {
+        uint32_t x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = 0x3c003c00u;
+        for (int c = 0; c < 64; c += 16) umma::tmem_st16u(umma::tmem_addr(tA, warp, c), x);
+        umma::tmem_wait_st();
+        umma::fence_before_sync();
+        __syncthreads();
+        umma::fence_after_sync();
+    }
     const long long t0 = clock64();
-    if (lane == 0 && warp < (issuers % 10)) {
+    if (mode >= 20) {
+        if (warp < (issuers % 10)) {
+            const uint32_t a = umma::smem_addr(sA), b = umma::smem_addr(sB), lead = umma::elect_one();
+            if (kred == 128) {
+                if (mode == 20) issue_converged<20, 128>(reps, lead, tbase, a, tA, b, N);
+                if (mode == 21) issue_converged<21, 128>(reps, lead, tbase, a, tA, b, N);
+                if (mode == 22) issue_converged<22, 128>(reps, lead, tbase, a, tA, b, N);
+                if (mode == 23) issue_converged<23, 128>(reps, lead, tbase, a, tA, b, N);
+                if (mode == 30) issue_converged<30, 128>(reps, lead, tbase, a, tA, b, N);
+                if (mode == 31) issue_converged<31, 128>(reps, lead, tbase, a, tA, b, N);
+            } else {
+                if (mode == 24) issue_converged<24, 64>(reps, lead, tbase, a, tA, b, N);
+                if (mode == 30) issue_converged<30, 64>(reps, lead, tbase, a, tA, b, N);
+            }
+            umma::commit_lead(lead, &bar[warp]);
+        }
+    } else if (lane == 0 && warp < (issuers % 10)) {
         const uint32_t a = umma::smem_addr(sA), b = umma::smem_addr(sB);
         const int a_rows = (mode == 2) ? kred : 128, b_rows = (mode == 0) ? N : kred;
         // the compile-time shaped issue loops of the kernels where one exists for the combination
@@ -160,7 +238,7 @@ __global__ void __launch_bounds__(128, 1) umma_cycles_kernel(int N, int kred, in
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem_slot, 256);
+    if (warp == 0) umma::tmem_dealloc(tmem_slot, 512);
 }
 
 }  // namespace llattn
@@ -181,11 +259,13 @@ __global__ void wait_timeout_kernel(uint32_t limit, int* status) {
 extern "C" int llattn_selftest_umma_cycles(int N, int kred, int mode, int reps, int issuers, long long* cycles, int* err_flag,
                                            void* stream) {
     if (!cycles || !err_flag) return LLATTN_ERR_NULL;
-    if (!(kred == 64 || kred == 128) || mode < 0 || mode > 4 || reps < 1 || reps > 4096 ||
-        !(issuers == 1 || issuers == 2 || issuers == 11 || issuers == 12))
+    if (!(kred == 64 || kred == 128) || reps < 1 || reps > 4096 || !(issuers == 1 || issuers == 2 || issuers == 11 || issuers == 12))
         return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    if (mode <= 2 ? !(N == 64 || N == 128) : !(N >= 32 && N <= 128 && N % 32 == 0)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
-    const int operand_bytes = mode >= 3 ? 131072 : 65536;
+    const bool known = (mode >= 0 && mode <= 4) || mode == 30 || (kred == 128 ? (mode >= 20 && mode <= 23) || mode == 31 : mode == 24);
+    if (!known) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    const bool scan = mode == 3 || mode == 4 || mode == 23 || mode == 24;
+    if (scan ? !(N >= 32 && N <= 128 && N % 32 == 0) : !(N == 64 || N == 128)) return LLATTN_ERR_UNSUPPORTED_SHAPE;
+    const int operand_bytes = scan ? 131072 : 65536;
     const size_t sm = (size_t)operand_bytes + 1024;
     cudaError_t e = cudaFuncSetAttribute(llattn::umma_cycles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return (int)e;
@@ -196,7 +276,8 @@ extern "C" int llattn_selftest_umma_cycles(int N, int kred, int mode, int reps, 
 extern "C" int llattn_selftest_umma(const void* A, const void* B, float* D, int N, int kred, int mode, int* err_flag,
                                     void* stream) {
     if (!A || !B || !D || !err_flag) return LLATTN_ERR_NULL;
-    if (!(N == 64 || N == 128) || !(kred == 64 || kred == 128) || !((mode >= 0 && mode <= 2) || (mode >= 10 && mode <= 12)))
+    if (!(N == 64 || N == 128) || !(kred == 64 || kred == 128) ||
+        !((mode >= 0 && mode <= 2) || (mode >= 10 && mode <= 12) || (mode >= 20 && mode <= 23) || mode == 30 || mode == 31))
         return LLATTN_ERR_UNSUPPORTED_SHAPE;
     const size_t sm = (mode >= 10 ? 131072 + 49152 + 32768 : 65536) + 1024;
     cudaError_t e = cudaFuncSetAttribute(llattn::umma_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -6,16 +6,17 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("mode", [0, 1, 2, 10, 11, 12])
+@pytest.mark.parametrize("mode", [0, 1, 2, 10, 11, 12, 20, 21, 22, 23, 30, 31])
 @pytest.mark.parametrize("N,kred", [(128, 128), (64, 128), (128, 64), (64, 64)])
 def test_umma_tile_product(mode, N, kred):
     from hattention_b200 import _lib
     lib = _lib.lib()
     dev = torch.device("cuda:0")
     gen = torch.Generator().manual_seed(mode * 10 + N + kred)
-    issue_mode, mode = mode, mode % 10        # 10..12: the compile-time shaped issue loops of the kernels
-    a_shape = (kred, 128) if mode == 2 else (128, kred)
-    b_shape = (N, kred) if mode == 0 else (kred, N)
+    # 10..12: compile-time shaped issue loops in a branch of one lane; 20..23: issued by a converged warp; 30, 31: so, with A in tensor memory
+    issue_mode, mode = mode, mode % 10
+    a_shape = (kred, 128) if mode >= 2 else (128, kred)
+    b_shape = (N, kred) if mode in (0, 3) else (kred, N)
     A = torch.randn(a_shape, generator=gen).bfloat16().to(dev)
     B = torch.randn(b_shape, generator=gen).bfloat16().to(dev)
     D = torch.zeros(128, N, device=dev)
@@ -26,7 +27,7 @@ def test_umma_tile_product(mode, N, kred):
     torch.cuda.synchronize()
     assert err.item() == 0, "tensor core completion was not signalled"
     Af, Bf = A.float(), B.float()
-    want = Af @ Bf.T if mode == 0 else (Af @ Bf if mode == 1 else Af.T @ Bf)
+    want = (Af.T if mode >= 2 else Af) @ (Bf.T if mode in (0, 3) else Bf)
     assert torch.allclose(D, want, rtol=1e-3, atol=1e-2), (D - want).abs().max().item()
 
 
@@ -40,6 +41,21 @@ def test_umma_tile_product(mode, N, kred):
     (3, 128, 128, 72.0),
     (4, 32, 64, 64.0),      # MN-major A (kd^T / qd^T), 64-token reduction
     (4, 96, 64, 64.0),
+    # the same layouts issued by a converged warp, an elected lane leading
+    (20, 128, 128, 72.0),
+    (22, 128, 128, 72.0),
+    (21, 64, 128, 52.0),    # N = 64: the operand fetch, 48
+    (22, 64, 128, 52.0),
+    (23, 32, 128, 46.0),    # N = 32: 41
+    (23, 64, 128, 52.0),
+    (23, 128, 128, 72.0),
+    (24, 32, 64, 46.0),
+    (24, 96, 64, 64.0),
+    (30, 128, 128, 72.0),   # A in tensor memory
+    (30, 64, 128, 36.0),    # ... where N = 64 takes the tensor core's own 32
+    (30, 128, 64, 72.0),
+    (31, 128, 128, 72.0),
+    (31, 64, 128, 36.0),
 ])
 def test_mma_issue_rate(mode, N, kred, bound):
     """Cycles per tcgen05.mma (M = 128, K = 16) of the compile-time shaped issue loops that the kernels use,
