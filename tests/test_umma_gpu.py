@@ -104,51 +104,6 @@ def test_wait_that_runs_out_sets_the_status_word():
     assert torch.ones(4, device=DEV).sum().item() == 4.0
 
 
-def test_phase_clock_stamps_of_one_pair():
-    """Only in a library built with `make -C log-linear-attention_b200/csrc clean all EXTRA=-DLLATTN_STAMPS`: prints the
-    clock64() stamps that three threads of one CTA take at fixed points of one chunk pair of the forward and the
-    forward-order / reverse-order backward kernels (run with -s).  Skipped for the normal build."""
-    import ctypes
-    from hattention_b200 import _lib
-    from hattention_b200.base import HType
-    from hattention_b200.chunkwise import chunkwise_bwd, chunkwise_fwd
-    from oracle import loglinear_oracle as orc
-    lib = _lib.lib()
-    if not hasattr(lib, "llattn_debug_read_stamps"):
-        pytest.skip("library built without -DLLATTN_STAMPS")
-    dev = torch.device("cuda:0")
-    q, k, v, g, l = orc.make_mamba2_inputs(1, 16384, 32, 64, 128, 1, 15, seed=0)
-    q, k, v, l = (x.bfloat16().to(dev) for x in (q, k, v, l))
-    g = g.float().to(dev)
-    do = torch.randn_like(v)
-    for _ in range(3):
-        kept = []
-        o, gc, _ = chunkwise_fwd(q, k, v, g, l, False, 2, HType.WEAK, 64, False, keep_workspace=kept)
-        chunkwise_bwd(q, k, v, gc, l, do, False, 2, HType.WEAK, 64, fwd_workspace=kept[0])
-    torch.cuda.synchronize()
-    if hasattr(lib, "llattn_debug_read_stamps_seg"):
-        # one CTA of the high-level backward kernel: entry, before / after the segment's cumulative decay, top of each pair,
-        # end of the pairs, reader summaries written, reduce-adds complete, exit
-        buf = (ctypes.c_longlong * 96)()
-        f = lib.llattn_debug_read_stamps_seg
-        f.argtypes = [ctypes.c_void_p]
-        assert f(buf) == 0
-        d = list(buf)[:16]
-        print("high-level backward, one CTA", [x - d[0] if x else None for x in d])
-    for name, fn in (("forward", "llattn_debug_read_stamps"), ("backward", "llattn_debug_read_stamps_bwd")):
-        buf = (ctypes.c_longlong * 96)()
-        f = getattr(lib, fn)
-        f.argtypes = [ctypes.c_void_p]
-        assert f(buf) == 0
-        d = list(buf)
-        for half, lo in (("forward-order / forward pass", 0), ("reverse-order pass", 16)):
-            if not d[lo]:
-                continue
-            for s_, who in enumerate(("thread 0", "thread 200", "thread 96")):
-                row = d[32 * s_ + lo: 32 * s_ + lo + 16]
-                print(name, half, who, [x - d[lo] if x else None for x in row])
-
-
 def test_phase_clock_stamps_of_one_gdn_scan_chunk():
     """Only in a library built with `make -C log-linear-attention_b200/csrc clean all EXTRA=-DLLATTN_STAMPS`: prints the
     clock64() stamps of one chunk (chunk 37 of CTA 5) of the Gated DeltaNet forward scan: an output thread, a staging
@@ -189,12 +144,11 @@ def test_phase_clock_stamps_of_one_gdn_scan_chunk():
         print(who, [x - t0 if x else None for x in d[32 * s_: 32 * s_ + 32]])
 
 
-def test_phase_clock_stamps_of_the_gdn_backward_kernels():
+def test_phase_clock_stamps_of_the_gdn_level_gradients():
     """Only in a library built with -DLLATTN_STAMPS (see above; LLATTN_LIB can name such a build): prints the clock64() stamps
     of one item of the level-gradient kernel (item 8 of CTA 5: per step, top / first batch complete / operands written for
     the element-wise threads 0 and 64, top / next first batch issued / operands ready / second batch issued for the MMA
-    thread, then the stages of the result write-out) and of one CTA of the chunk-local gradient kernel (lane 0 of warps 0,
-    7 and 2 after each barrier and between the products of the longer stages).  Run with -s."""
+    thread, then the stages of the result write-out).  Run with -s."""
     import ctypes
     from hattention_b200 import _lib
     from hattention_b200.gated_delta_rule_apis import chunk_h_gated_delta_rule
@@ -216,16 +170,14 @@ def test_phase_clock_stamps_of_the_gdn_backward_kernels():
         o = chunk_h_gated_delta_rule(*ins, use_qk_l2norm_in_kernel=True)[0]
         torch.autograd.grad(o, ins, do)
     torch.cuda.synchronize()
-    for fn, names in (("llattn_debug_read_stamps_gdn_levels", ("levels, thread 0 (q rows)", "levels, thread 64 (w rows)", "levels, MMA thread")),
-                      ("llattn_debug_read_stamps_gdn_chunk", ("chunk-local, warp 0", "chunk-local, warp 7", "chunk-local, warp 2"))):
-        buf = (ctypes.c_longlong * 96)()
-        f = getattr(lib, fn)
-        f.argtypes = [ctypes.c_void_p]
-        assert f(buf) == 0
-        d = list(buf)
-        t0 = min(x for x in d if x)
-        for s_, who in enumerate(names):
-            print(who, [x - t0 if x else None for x in d[32 * s_: 32 * s_ + 32]])
+    buf = (ctypes.c_longlong * 96)()
+    f = lib.llattn_debug_read_stamps_gdn_levels
+    f.argtypes = [ctypes.c_void_p]
+    assert f(buf) == 0
+    d = list(buf)
+    t0 = min(x for x in d if x)
+    for s_, who in enumerate(("levels, thread 0 (q rows)", "levels, thread 64 (w rows)", "levels, MMA thread")):
+        print(who, [x - t0 if x else None for x in d[32 * s_: 32 * s_ + 32]])
 
 
 def test_elementwise_phase_cycles():
