@@ -58,7 +58,7 @@ struct Mamba2Params {
     int B, T, H, G, K, V, L;
     int NT, NS, LH;
     int o_has_high;              // warp-level chunk kernel: o holds the partial output of the high levels
-    int hc;                      // heads per CTA of the output kernel
+    int hc;                      // heads per CTA of the output and gradient kernels
     int chunk_rounding;          // backward: a sequence of an odd number of chunks, or with K = 64, takes the chunk-by-chunk kernels
     // forward of a layer: y = o + D x takes the place of o (tensor-core kernels; res_D NULL: none)
     const __nv_bfloat16* res_x;  // (B,res_T,H,V)

@@ -567,9 +567,8 @@ std::atomic<int> g_use_tensor_core_path{1};
 
 // The tensor-core kernels take 64 or 128 state rows (K = 64 fills half of their tiles; the tensor maps supply zeros for the other half) and
 // any number of chunks (the second chunk of a last pair may lie beyond the sequence: zeros again, and nothing is written there).  They
-// hold 20 lambda levels.  Forward + backward of T = 57792 (903 chunks), 32 heads, took 10.8 ms on the warp-level kernels, which
-// sequences of an odd number of chunks and K = 64 went to before, and takes 3.8 ms here; T = 16384, 32 heads, K = 64: 1.98 -> 0.98 ms; a single
-// chunk, forward: 61 -> 18 us of which most is the host's.  More levels than 20 do not fit the tables in shared memory.
+// hold M2_MAX_L_TC lambda levels: more do not fit the tables in shared memory.  Forward + backward, warp-level kernels / these: T = 57792 (903 chunks), 32 heads
+// 10.6 / 2.7 ms; T = 16384, 32 heads, K = 64 1.94 / 0.64 ms; B = 2, T = 1984, 24 heads, K = 64, two groups 332 / 176 us.
 // o and dv leave them in 16-byte stores (the warp-level kernels write pairs of values).
 bool mamba2_uses_tc(const Mamba2Params& p) { return p.V == 64 && p.L <= M2_MAX_L_TC && !p.warp_level && !misaligned(16, {p.o, p.dv}) && g_use_tensor_core_path.load(); }
 

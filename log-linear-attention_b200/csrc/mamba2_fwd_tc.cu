@@ -33,7 +33,7 @@ constexpr int NSLOT = 2;                  // per team: tensor-memory slots of 64
 // Two teams, one CTA per SM.  A CTA of one head (one head a group, or a call too small to fill the chip with more) has work for one team only: with half of the
 // threads, of tensor memory (P in the place of S) and of shared memory two of them share an SM, which a chain of loads, S, P and two products leaves idle
 // for the most part.  B = 16, T = 1024, 24 heads and groups: 161 -> 92 us (with the kernels that walked segments 131 and 26 for the high levels); calls
-// of fewer CTAs than SMs take what they took.
+// of fewer CTAs than SMs, us of the whole forward: T = 128, 24 heads 20.5 -> 19.6, T = 640, 4 heads 25.6 -> 24.9, T = 2048, 8 heads 33.0 -> 33.0.
 template <int TEAMS>
 struct Teams {
     static constexpr int NST = TEAMS == 2 ? 3 : 2;                            // per team: stages of 16 KB
@@ -509,9 +509,12 @@ __global__ void __launch_bounds__(tco::Teams<TEAMS>::NTHREADS, TEAMS == 2 ? 1 : 
 }
 
 // ------------------------------------------------------------------------------------------
-// Sequences of two to four pairs (T <= 512), whose calls lend no scratch for level states: one CTA per (batch, head) walks its pairs in order and
-// keeps the states on chip, masters in registers in the tensor-memory readout layout (one state row per thread), bf16 copies as MN-major operands.
+// Sequences of two to four pairs (T <= 512), whose calls lend no scratch for level states (256 bytes of workspace): one CTA per (batch, head) walks its pairs in
+// order and keeps the states on chip, masters in registers in the tensor-memory readout layout (one state row per thread), bf16 copies as MN-major operands.
 //   S = q k^T, T = q H_level, O = P v, KV = k^T (v * decay) per pair
+// It stays for those calls: with scratch, states and outputs apart would be the faster way for most of them.  The forward call on this kernel / on those two, us
+// (sequences x tokens x heads): 1 x 192 x 8 26.7 / 29.0, 4 x 256 x 32 29.8 / 33.0, 1 x 256 x 48 29.8 / 29.9; 1 x 384 x 48 34.8 / 32.2, 1 x 512 x 48 41.0 / 35.2,
+// 8 x 512 x 24 62 / 45, 32 x 192 x 24 88 / 64, 32 x 512 x 24 158 / 114; with one head a group 16 x 512 x 24 94 / 94.
 // ------------------------------------------------------------------------------------------
 template <int MLOW>
 struct FwdTcSmem {
@@ -998,8 +1001,11 @@ int mamba2_fwd_one_segment_tc_launch(const Mamba2Params& p_in, cudaStream_t stre
     return p.res_round ? launch_one_segment<3>(p, stream) : launch_one_segment<1>(p, stream);
 }
 
-// Heads per CTA: the fewest rounds of CTAs over the SMs, a CTA counted as its heads and two more (q, k, S, tables).  Many heads share S and the loads of
-// q and k; few fill the chip when a call is small.
+// Heads per CTA of the output and gradient kernels: the fewest rounds of CTAs over the SMs, a CTA counted as its heads and two more (q, k, S, tables).  Many heads
+// share S and the loads of q and k; few fill the chip when a call is small.  Two lies between what the kernels show: at B = 2, T = 16384, 32 heads a CTA of
+// n heads takes 2.0 (n + 2.7) us of outputs (two teams), 5.0 (n + 1.3) of dq, 3.3 (n + 2.1) of dk and dv.  The rule against the best n of one to eight (outputs /
+// dq / dkv, us): 1 x 1024 x 48 (sequences, tokens, heads) 12/22/17, none better; 1 x 4096 x 32 23/51/34, none; 2 x 4096 x 24 32/72/56, none;
+// 4 x 2048 x 32, K = 64 36/83/63, none; 8 x 4096 x 24 six heads 109/244/188, eight 102/245/194; 1 x 65536 x 32, where L = 17 leaves six, 344/890/517.
 int mamba2_heads_per_cta(const Mamba2Params& p, int sms) {
     int reads = 1;                                   // levels that a pair reads at most
     while ((p.NT + 1) / 2 > 1 << reads) ++reads;
